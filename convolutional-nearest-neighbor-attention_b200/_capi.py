@@ -28,6 +28,28 @@ class ConvnnDesc(ctypes.Structure):
                                      "conv_type", "softmax", "coord", "seq_length", "reserved")]
 
 
+BLOCK_CONVNN, BLOCK_BRANCH_ATTENTION, BLOCK_BRANCH_CONV1D = 0, 1, 2
+
+
+class ConvnnBlock(ctypes.Structure):
+    """Mirror of ``struct convnn_block``."""
+    _fields_ = ([("layer", ConvnnDesc)] + [(n, c_i32) for n in ("kind", "d_mlp", "kernel_size", "fuse_mlp")] +
+                [(n, ctypes.c_float) for n in ("eps1", "eps2")] +
+                [(n, c_void) for n in ("norm1_w", "norm1_b", "norm2_w", "norm2_b", "w_qkv", "w_conv", "w_pw", "w_o", "cand",
+                                       "w_qkv_folded", "w_qkv_extra", "fc1_w", "fc1_b", "fc2_w", "fc2_b", "fc1_folded",
+                                       "fc1_extra", "branch_w_in", "branch_b_in", "branch_w_conv", "branch_b_conv",
+                                       "branch_w_out", "branch_b_out", "pointwise_w", "pointwise_b")])
+
+
+class ConvnnModel(ctypes.Structure):
+    """Mirror of ``struct convnn_model``."""
+    _fields_ = ([(n, c_i32) for n in ("dtype", "B", "T", "D", "n_blocks", "classes", "channels", "height", "width", "patch",
+                                      "images_u8")] + [("embed_eps", ctypes.c_float),
+                                                       ("blocks", ctypes.POINTER(ConvnnBlock))] +
+                [(n, c_void) for n in ("patch_w", "patch_b", "embed_norm_w", "embed_norm_b", "cls", "pe", "pixel_mean",
+                                       "pixel_inv_std", "head_w", "head_b")])
+
+
 # name -> (restype, argtypes); must list every symbol the header declares
 SIGNATURES = {
     "convnn_b200_abi_version": (ctypes.c_int, []),
@@ -90,6 +112,8 @@ SIGNATURES = {
     "convnn_b200_conv1d_attention": (ctypes.c_int, [ctypes.c_int, c_void, c_i64, c_void, c_void, c_void, c_void, c_void,
                                                     c_void, c_void, c_i64, c_i32, c_i32, c_i32, c_i32, c_i32, c_void,
                                                     c_size, c_void]),
+    "convnn_b200_model_workspace_bytes": (c_size, [ctypes.POINTER(ConvnnModel)]),
+    "convnn_b200_model_forward": (ctypes.c_int, [ctypes.POINTER(ConvnnModel), c_void, c_void, c_void, c_size, c_void]),
 }
 
 _lock = threading.Lock()

@@ -402,15 +402,12 @@ int launch_attention_tc(const void* q, const void* k, const void* v, void* o, in
     if (!encode_tensor_map_bf16(&tmK, k, 4, dims, str, boxK, pitch)) return CONVNN_E_CUDA;
     if (!encode_tensor_map_bf16(&tmV, v, 4, dims, str, boxV, 0)) return CONVNN_E_CUDA;
 
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = device_sms();
     const int per_sm = smem <= 113 * 1024 && p.BNpad <= 256 ? 2 : 1;
     const int ctas = sms * per_sm;
     const int grid = p.n_units < ctas ? p.n_units : ctas;
     auto kern = attention_tc_kernel;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    CONVNN_ENSURE_SMEM(kern, smem);
     kern<<<grid, NTHREADS, smem, st>>>(tmQ, tmK, tmV, p);
     CONVNN_CHECK_LAUNCH("attention_tc");
     return CONVNN_OK;
@@ -424,8 +421,7 @@ int launch_attention_simt_t(const void* q, const void* k, const void* v, void* o
     if (smem > 200 * 1024)
         return set_error(CONVNN_E_UNSUPPORTED, "softmax attention over %d tokens is outside this build", Tn);
     auto kern = attention_simt_kernel<T>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    CONVNN_ENSURE_SMEM(kern, smem);
     int gx = (Tn + nw - 1) / nw;
     if (gx > 64) gx = 64;
     kern<<<dim3(gx, B * H), nw * 32, smem, st>>>(static_cast<const T*>(q), static_cast<const T*>(k),

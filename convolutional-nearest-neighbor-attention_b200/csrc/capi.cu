@@ -1,6 +1,7 @@
 // extern "C" surface of libconvnn_b200: argument validation, workspace carving and the
 // chaining of the stage kernels on the caller's stream.
 #include <atomic>
+#include <mutex>
 #include <stdarg.h>
 #include <stdlib.h>
 #include <string.h>
@@ -26,6 +27,52 @@ bool force_simt() {
         return e && e[0] == '1';
     }();
     return v;
+}
+
+int device_sms() {
+    static std::atomic<int> sms[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    int n = sms[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 148;
+        sms[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+int SmemLimit::ensure(const void* kern, size_t smem) {
+    if (smem <= 32 * 1024) return CONVNN_OK;   // (48 KB with the static part needs no opt-in)
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const bool known = dev >= 0 && dev < 16;
+    if (known && bytes[dev].load(std::memory_order_acquire) >= (int)smem) return CONVNN_OK;
+    static std::mutex m;                     // sizes only grow: two threads must not set them in the wrong order
+    std::lock_guard<std::mutex> lock(m);
+    if (known && bytes[dev].load(std::memory_order_relaxed) >= (int)smem) return CONVNN_OK;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    if (known) bytes[dev].store((int)smem, std::memory_order_release);
+    return CONVNN_OK;
+}
+
+int ClusterLimit::query(const void* kern, const cudaLaunchConfig_t* cfg, int* clusters) {
+    const long long smem = (long long)cfg->dynamicSmemBytes;
+    for (auto& e : seen) {
+        const long long v = e.load(std::memory_order_relaxed);
+        if (v && (v >> 20) == smem) {
+            *clusters = (int)(v & 0xFFFFF);
+            return CONVNN_OK;
+        }
+    }
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(clusters, kern, cfg);
+    if (e != cudaSuccess || *clusters < 1)
+        return set_error(CONVNN_E_CUDA, "cudaOccupancyMaxActiveClusters: %s", cudaGetErrorString(e));
+    for (auto& slot : seen) {
+        long long expected = 0;
+        if (slot.compare_exchange_strong(expected, (smem << 20) | *clusters, std::memory_order_relaxed)) break;
+    }
+    return CONVNN_OK;
 }
 
 static std::atomic<unsigned long long> g_launches{0};

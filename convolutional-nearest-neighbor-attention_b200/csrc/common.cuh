@@ -6,6 +6,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #include "../../include/convnn_b200.h"
 
 namespace convnn {
@@ -23,6 +25,28 @@ void count_launch();
         if (e__ != cudaSuccess)                                                      \
             return ::convnn::set_error(CONVNN_E_CUDA, "%s: %s", what, cudaGetErrorString(e__)); \
     } while (0)
+
+// SM count of the current device, asked once per device.
+int device_sms();
+
+// Raises a kernel's dynamic shared-memory limit.  cudaFuncSetAttribute costs a launch about as much host time as
+// building a tensor map, so a call site keeps one of these per kernel and calls the runtime only when the size grows.
+struct SmemLimit {
+    std::atomic<int> bytes[16];
+    int ensure(const void* kern, size_t smem);
+};
+#define CONVNN_ENSURE_SMEM(kern, smem)                                                        \
+    do {                                                                                      \
+        static ::convnn::SmemLimit limit__{};                                                 \
+        const int rc__ = limit__.ensure(reinterpret_cast<const void*>(kern), smem);           \
+        if (rc__ != CONVNN_OK) return rc__;                                                   \
+    } while (0)
+
+// Clusters of a launch configuration that fit on the device at once, remembered per shared-memory size.
+struct ClusterLimit {
+    std::atomic<long long> seen[4];          // (shared-memory bytes << 20) | clusters; 0 = free
+    int query(const void* kern, const cudaLaunchConfig_t* cfg, int* clusters);
+};
 
 // ---- descriptor-derived quantities -------------------------------------------------
 struct Dims {

@@ -172,9 +172,7 @@ int try_launch_gather_conv_dw_stream(const convnn_desc* d, const Dims& dm, const
     const size_t nk = (size_t)dm.T * KT;
     const size_t smem = 2 * (size_t)p.slice_bytes + 2 * nk * 4 + 2 * nk * 4 + 8 + nk * 8 + 2 * 8;
 
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = device_sms();
     int per_chunk = (2 * sms) / p.nchunks;
     if (per_chunk < 1) per_chunk = 1;
     if (per_chunk > p.n_slices) per_chunk = p.n_slices;
@@ -187,8 +185,7 @@ int try_launch_gather_conv_dw_stream(const convnn_desc* d, const Dims& dm, const
     if (!encode_tensor_map_bf16(&tmV, v, 4, dims, strides, box, 0)) return CONVNN_E_CUDA;
 
     auto kern = gather_conv_dw_stream_kernel;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    CONVNN_ENSURE_SMEM(kern, smem);
     kern<<<per_chunk * p.nchunks, TPB, smem, st>>>(tmV, p);
     CONVNN_CHECK_LAUNCH("gather_conv_dw_stream");
     return CONVNN_OK;

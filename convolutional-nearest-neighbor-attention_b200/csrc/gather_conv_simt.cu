@@ -210,10 +210,7 @@ int launch_mat(const convnn_desc* d, const Dims& dm, const void* v, const int32_
     size_t smem = (size_t)TT * JC * dm.C * sizeof(float);
     if (smem > 200 * 1024) return set_error(CONVNN_E_UNSUPPORTED, "conv tile needs %zu bytes of shared memory", smem);
     auto kern = gather_conv_mat_kernel<T, ITEMS>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    }
+    CONVNN_ENSURE_SMEM(kern, smem);
     dim3 grid((dm.T + TT - 1) / TT, dm.B * dm.H);
     kern<<<grid, THREADS, smem, st>>>(static_cast<const T*>(v), idx, val, static_cast<const T*>(w_conv),
                                       static_cast<const T*>(w_pw), static_cast<T*>(o), dm.T, dm.H, dm.dk, dm.C,
@@ -305,9 +302,7 @@ int try_launch_gather_conv_tc(const convnn_desc* d, const Dims& dm, const void* 
         constexpr int TT = 64;
         const int BH = dm.B * dm.H;
         const int tiles_per_bh = (dm.T + TT - 1) / TT;
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const int sms = device_sms();
         long long grid = (long long)BH * tiles_per_bh;
         if (grid > sms * 8LL) grid = sms * 8LL;
         const int groups = dm.C / 8;
@@ -475,8 +470,7 @@ int launch_dw_smem(const convnn_desc* d, const Dims& dm, const void* v, const in
 #define CONVNN_DW_LAUNCH(KT)                                                                                 \
     do {                                                                                                     \
         auto kern = gather_conv_dw_smem_kernel<T, VEC, KT>;                                                  \
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
-        if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e)); \
+        CONVNN_ENSURE_SMEM(kern, smem);                                                            \
         kern<<<dm.B * dm.H, 256, smem, st>>>(static_cast<const T*>(v), idx, val, static_cast<const T*>(w_conv), \
                                              static_cast<T*>(o), dm.T, dm.H, dm.dk, dm.Cp, dm.K, maximum,    \
                                              d->softmax, groups, tpp);                                       \

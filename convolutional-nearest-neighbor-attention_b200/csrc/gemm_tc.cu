@@ -828,9 +828,7 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
     p.n_tiles = p.n_m_tiles * p.n_n_tiles;
 
     const int pitch = p.KCH * 2;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = device_sms();
     // W-resident mode when the whole BN x Kd tile of W fits beside a useful ring of A chunks and
     // a CTA sees several row tiles per W tile; otherwise both operands stream through the ring.
     const bool has_stat = p.stat[0] || p.stat[1] || p.stat[2];
@@ -955,22 +953,19 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
 #define CONVNN_GEMM_LAUNCH1(S, B, G, R, W)                                                                  \
     do {                                                                                                    \
         auto kern = gemm_tc_kernel<S, B, G, R, W, false>;                                                   \
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e)); \
+        CONVNN_ENSURE_SMEM(kern, smem);                                                            \
         kern<<<grid, W ? NTHREADS_WIDE : NTHREADS, smem, st>>>(tmA, tmW, tmX, tmM, p);                           \
     } while (0)
 #define CONVNN_GEMM_LAUNCH_X(S, G, R, W, LNFv, MOMv)                                                        \
     do {                                                                                                    \
         auto kern = gemm_tc_kernel<S, false, G, R, W, false, LNFv, MOMv>;                                   \
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e)); \
+        CONVNN_ENSURE_SMEM(kern, smem);                                                            \
         kern<<<grid, (W ? NTHREADS_WIDE : NTHREADS) + (LNFv ? 32 : 0), smem, st>>>(tmA, tmW, tmX, tmM, p);       \
     } while (0)
 #define CONVNN_GEMM_LAUNCH_PAIR(G, R, W)                                                                    \
     do {                                                                                                    \
         auto kern = gemm_tc_kernel<false, false, G, R, W, true>;                                            \
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e)); \
+        CONVNN_ENSURE_SMEM(kern, smem);                                                            \
         cudaLaunchConfig_t cfg{};                                                                           \
         cudaLaunchAttribute attr[1];                                                                        \
         attr[0].id = cudaLaunchAttributeClusterDimension;                                                   \
@@ -978,21 +973,12 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
         cfg.blockDim = dim3(W ? NTHREADS_WIDE : NTHREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;    \
         cfg.attrs = attr; cfg.numAttrs = 1;                                                                 \
         cfg.gridDim = dim3(2);                                                                              \
-        /* co-resident clusters for this kernel and shared-memory size, asked once per process */       \
-        static std::atomic<long long> occ_cache{-1};                                                        \
+        static ClusterLimit fit{};                                                                          \
         int max_clusters = 0;                                                                               \
-        const long long seen = occ_cache.load(std::memory_order_relaxed);                                   \
-        if (seen >= 0 && (size_t)(seen >> 20) == smem) {                                                    \
-            max_clusters = (int)(seen & 0xFFFFF);                                                           \
-        } else {                                                                                            \
-            e = cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg);                                  \
-            if (e != cudaSuccess || max_clusters < 1)                                                       \
-                return set_error(CONVNN_E_CUDA, "cudaOccupancyMaxActiveClusters: %s", cudaGetErrorString(e)); \
-            occ_cache.store(((long long)smem << 20) | max_clusters, std::memory_order_relaxed);             \
-        }                                                                                                   \
+        if (const int rc_ = fit.query(reinterpret_cast<const void*>(kern), &cfg, &max_clusters)) return rc_; \
         const int nc = p.n_tiles < max_clusters ? p.n_tiles : max_clusters;                                 \
         cfg.gridDim = dim3(2 * nc);                                                                         \
-        e = cudaLaunchKernelEx(&cfg, kern, tmA, tmW, tmX, tmM, p);                                                    \
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmW, tmX, tmM, p);                                                    \
         if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "gemm_tc pair launch: %s", cudaGetErrorString(e)); \
     } while (0)
 #define CONVNN_GEMM_LAUNCH(S, B, G, R)                          \

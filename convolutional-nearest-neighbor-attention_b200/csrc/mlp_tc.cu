@@ -748,8 +748,8 @@ int launch_mlp_tc(const void* x, long long ldx, const float* moments, int planes
     }
     const size_t smem = smem_plan(D).total + 1024;
     auto kern = w_o ? mlp_tc_kernel<true> : mlp_tc_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    static SmemLimit limits[2]{};
+    if (const int rc = limits[w_o ? 1 : 0].ensure(reinterpret_cast<const void*>(kern), smem)) return rc;
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -757,21 +757,12 @@ int launch_mlp_tc(const void* x, long long ldx, const float* moments, int planes
     cfg.blockDim = dim3(NT); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cfg.attrs = attr; cfg.numAttrs = 1;
     cfg.gridDim = dim3(2);
-    static std::atomic<long long> occ_caches[2] = {{-1}, {-1}};   // co-resident clusters per kernel and shared-memory size
-    std::atomic<long long>& occ_cache = occ_caches[w_o ? 1 : 0];
+    static ClusterLimit fit[2]{};
     int max_clusters = 0;
-    const long long seen = occ_cache.load(std::memory_order_relaxed);
-    if (seen >= 0 && (size_t)(seen >> 20) == smem) {
-        max_clusters = (int)(seen & 0xFFFFF);
-    } else {
-        e = cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg);
-        if (e != cudaSuccess || max_clusters < 1)
-            return set_error(CONVNN_E_CUDA, "cudaOccupancyMaxActiveClusters: %s", cudaGetErrorString(e));
-        occ_cache.store(((long long)smem << 20) | max_clusters, std::memory_order_relaxed);
-    }
+    if (const int rc = fit[w_o ? 1 : 0].query(reinterpret_cast<const void*>(kern), &cfg, &max_clusters)) return rc;
     const int nc = p.n_ptiles < max_clusters ? p.n_ptiles : max_clusters;
     cfg.gridDim = dim3(2 * nc);
-    e = cudaLaunchKernelEx(&cfg, kern, tmX, tmO, tmW1, tmWX, tmW2, tmWO, p);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmX, tmO, tmW1, tmWX, tmW2, tmWO, p);
     if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "mlp_tc launch: %s", cudaGetErrorString(e));
     CONVNN_CHECK_LAUNCH("mlp_tc");
     return CONVNN_OK;

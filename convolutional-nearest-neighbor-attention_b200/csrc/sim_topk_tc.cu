@@ -317,17 +317,14 @@ int launch_sim_topk_tc(const convnn_desc* d, const Dims& dm, const void* q, cons
     const int cw = small_cfg ? 16 : 32;
     const size_t smem = 1024 + (size_t)p.stages * (2 * BM + p.BN) * pitch + 2 * cw * GROUP * sizeof(float) +
                         8 * 128 * sizeof(float) + (2 * MAX_STAGES + 4) * 8 + 16;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = device_sms();
     const int ctas = sms * (small_cfg ? 2 : 1);
     const int grid = p.n_units < ctas ? p.n_units : ctas;
 
 #define CONVNN_TC_LAUNCH2(N, MINB, CWV)                                                                \
     do {                                                                                               \
         auto kern = sim_topk_tc_kernel<N, MINB, CWV>;                                                  \
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e)); \
+        CONVNN_ENSURE_SMEM(kern, smem);                                                            \
         kern<<<grid, NTHREADS, smem, st>>>(tmK, tmQ, p);                                               \
     } while (0)
 #define CONVNN_TC_LAUNCH(N)                            \

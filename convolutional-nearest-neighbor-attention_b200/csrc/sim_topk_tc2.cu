@@ -326,8 +326,7 @@ int launch_sim_topk_tc2(const convnn_desc* d, const Dims& dm, const void* q, con
         constexpr int NST = N > 24 ? STAGES - 1 : STAGES;                                                        \
         auto kern = sim_topk_tc2_kernel<N, NST>;                                                                 \
         const size_t smem = smem_fixed + (size_t)NST * STAGE_BYTES + 2 * N * kSelGroup * sizeof(float);          \
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
-        if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e)); \
+        CONVNN_ENSURE_SMEM(kern, smem);                                                            \
         cudaLaunchConfig_t cfg{};                                                                                \
         cudaLaunchAttribute attr[1];                                                                             \
         attr[0].id = cudaLaunchAttributeClusterDimension;                                                        \
@@ -335,21 +334,12 @@ int launch_sim_topk_tc2(const convnn_desc* d, const Dims& dm, const void* q, con
         cfg.blockDim = dim3(NTHREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;                             \
         cfg.attrs = attr; cfg.numAttrs = 1;                                                                      \
         cfg.gridDim = dim3(2);                                                                                   \
-        /* co-resident clusters for this kernel and shared-memory size, asked once per process */       \
-        static std::atomic<long long> occ_cache{-1};                                                        \
+        static ClusterLimit fit{};                                                                          \
         int max_clusters = 0;                                                                               \
-        const long long seen = occ_cache.load(std::memory_order_relaxed);                                   \
-        if (seen >= 0 && (size_t)(seen >> 20) == smem) {                                                    \
-            max_clusters = (int)(seen & 0xFFFFF);                                                           \
-        } else {                                                                                            \
-            e = cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg);                                  \
-            if (e != cudaSuccess || max_clusters < 1)                                                       \
-                return set_error(CONVNN_E_CUDA, "cudaOccupancyMaxActiveClusters: %s", cudaGetErrorString(e)); \
-            occ_cache.store(((long long)smem << 20) | max_clusters, std::memory_order_relaxed);             \
-        }                                                                                                   \
+        if (const int rc_ = fit.query(reinterpret_cast<const void*>(kern), &cfg, &max_clusters)) return rc_; \
         const int nc = p.n_units < max_clusters ? p.n_units : max_clusters;                                      \
         cfg.gridDim = dim3(2 * nc);                                                                              \
-        e = cudaLaunchKernelEx(&cfg, kern, tmK, tmQ, p);                                                         \
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmK, tmQ, p);                                                         \
         if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "sim_topk_tc2 launch: %s", cudaGetErrorString(e)); \
     } while (0)
     const int n = dm.nsel;

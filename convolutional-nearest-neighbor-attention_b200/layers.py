@@ -20,7 +20,75 @@ from . import ops
 from .ops import LayerSpec
 
 
-class MultiHeadConvNNAttention(nn.Module):
+_epoch = [0]
+
+
+def attribute_epoch() -> int:
+    """Counts the attribute assignments on this package's modules: whatever was prepared from their attributes
+    (a forward's host plan) is still valid while it stands still."""
+    return _epoch[0]
+
+
+class WatchedModule(nn.Module):
+    """``nn.Module`` whose public attribute assignments advance ``attribute_epoch()``."""
+
+    def __setattr__(self, name, value):
+        if name[0] != "_":
+            _epoch[0] += 1
+        super().__setattr__(name, value)
+
+    def __delattr__(self, name):
+        _epoch[0] += 1
+        super().__delattr__(name)
+
+
+class _NotCopied(dict):
+    """A cache that copies and pickles of its owner start without."""
+
+    def __deepcopy__(self, memo):
+        return _NotCopied()
+
+    def __reduce__(self):
+        return (_NotCopied, ())
+
+
+class _LayerCall:
+    """What one ConvNN layer call of a given input shape needs besides its tensors, prepared once: descriptor, packed
+    weights, candidate indices in the kernels' type, workspace size (27 us of host time per call before, 10 with it;
+    a small layer's kernels take 30)."""
+
+    def __init__(self, layer, x):
+        B, T, _ = x.shape
+        self.epoch = attribute_epoch()
+        mods = [m for m in layer.modules()]
+        self.slots = [(m._parameters, k) for m in mods for k in m._parameters]
+        params = [d[k] for d, k in self.slots]
+        self.ids = [id(p) for p in params]
+        self.cand, self.draw, spec = None, None, layer._spec()
+        if layer.sampling_type == "random" and layer.candidate_override is None:
+            self.draw, S = layer, len(range(T)[:layer.num_samples])     # drawn anew on every call
+        else:
+            self.cand, S = ops._cand_arg(spec, layer.candidates(T, x.device), T, x.device)
+        if layer.candidate_override is not None:
+            params.append(layer.candidate_override)
+        self.params = [p for p in params if p is not None]
+        self.versions = [p._version for p in self.params]
+        self.ptrs = [p.data_ptr() for p in self.params]
+        self.packed = layer.packed_weights(x.dtype, x.device)
+        self.call = ops.LayerForward(spec, B, T, S, x.dtype, x.device, self.packed)
+
+    def unchanged(self):
+        return (self.epoch == _epoch[0] and [id(d[k]) for d, k in self.slots if k in d] == self.ids and
+                [p._version for p in self.params] == self.versions and [p.data_ptr() for p in self.params] == self.ptrs)
+
+    def __call__(self, x, out, residual):
+        cand = self.cand
+        if self.draw is not None:
+            cand = self.draw.candidates(x.shape[1], x.device).to(torch.int32)
+        return self.call(x, cand, out, residual)
+
+
+class MultiHeadConvNNAttention(WatchedModule):
     def __init__(self, d_hidden, num_heads, attention_dropout, K, sampling_type, num_samples, sample_padding,
                  magnitude_type, seq_length=197, coordinate_encoding=False, convolution_type='depthwise',
                  softmax_topk_val=True):
@@ -70,6 +138,7 @@ class MultiHeadConvNNAttention(nn.Module):
         self._packed = None
         self._packed_key = None
         self._spatial_cache = {}
+        self._calls = _NotCopied()
 
     # -- host-side helpers --------------------------------------------------------------
     @property
@@ -139,12 +208,20 @@ class MultiHeadConvNNAttention(nn.Module):
         """``layer(x)``; with ``residual`` the caller's skip connection is folded into the last
         store (``residual + layer(x)``), with ``out`` the result is written in place."""
         self._check_mode(x)
-        B, T, D = x.shape
-        cand = self.candidates(T, x.device)
-        packed = self.packed_weights(x.dtype, x.device)
-        if self.stage_timer is not None:
-            return self._forward_staged(x, packed, cand, out, residual)
-        return ops.forward(self._spec(), x, packed, cand, out=out, residual=residual)
+        if self.stage_timer is not None or self._packed is None or x.dim() != 3:
+            B, T, D = x.shape
+            cand = self.candidates(T, x.device)
+            packed = self.packed_weights(x.dtype, x.device)
+            if self.stage_timer is not None:
+                return self._forward_staged(x, packed, cand, out, residual)
+            return ops.forward(self._spec(), x, packed, cand, out=out, residual=residual)
+        key = (x.shape, x.dtype, x.device)
+        call = self._calls.get(key)
+        if call is None or not call.unchanged():
+            if len(self._calls) >= 16:
+                self._calls.clear()
+            call = self._calls[key] = _LayerCall(self, x)
+        return call(x, out, residual)
 
     def prenorm_supported(self, x) -> bool:
         """Whether ``forward_prenorm`` takes this input (bfloat16, sampling 'all', a K/V/Q weight tile
@@ -163,15 +240,24 @@ class MultiHeadConvNNAttention(nn.Module):
         ``skip_out_proj`` (num_heads = 1) the result is the layer's output BEFORE ``W_o``, for a caller
         that fuses the projection into what follows (``ops.outproj_mlp`` with ``self.packed_w_o``)."""
         self._check_mode(x)
-        w_qkv, w_conv, w_pw, w_o = self.packed_weights(x.dtype, x.device)
-        if getattr(self, "_folded", None) is None:
-            self._folded = _PackedParams()
-        wf, wx = self._folded.get((w_qkv, norm.weight, norm.bias), x.dtype, x.device, lambda: ops.fold_layernorm(
-            w_qkv.view(-1, w_qkv.shape[-1]), None, norm.weight.detach().to(x.device, x.dtype),
-            norm.bias.detach().to(x.device, x.dtype)))
-        self.packed_w_o = w_o
+        _, w_conv, w_pw, w_o = self.packed_weights(x.dtype, x.device)
+        wf, wx = self.folded_qkv(norm, x.dtype, x.device)
         return ops.prenorm_forward(self._spec(), x, moments, norm.eps, (wf, wx, w_conv, w_pw, None if skip_out_proj else w_o),
                                    residual=residual, want_moments=want_moments)
+
+    @property
+    def packed_w_o(self):
+        """The output projection as last packed."""
+        return self._packed[3]
+
+    def folded_qkv(self, norm: nn.LayerNorm, dtype, device):
+        """The packed K/V/Q weight with ``norm`` folded in (``ops.fold_layernorm``)."""
+        w_qkv = self.packed_weights(dtype, device)[0]
+        if getattr(self, "_folded", None) is None:
+            self._folded = _PackedParams()
+        return self._folded.get((w_qkv, norm.weight, norm.bias), dtype, device, lambda: ops.fold_layernorm(
+            w_qkv.view(-1, w_qkv.shape[-1]), None, norm.weight.detach().to(device, dtype),
+            norm.bias.detach().to(device, dtype)))
 
     def _forward_staged(self, x, packed, cand, out, residual=None):
         """The same kernels in the same order as ``convnn_b200_forward``, issued through the
@@ -211,7 +297,7 @@ class _PackedParams:
         return self._val
 
 
-class MultiHeadAttention(nn.Module):
+class MultiHeadAttention(WatchedModule):
     """Softmax attention half of MultiHeadBranchingAttention (reference layers.py:90-130):
     bias-free W_q/W_k/W_v/W_o, softmax(QK^T / sqrt(d_k)) V.  The modules hold the parameters (same
     ``state_dict`` keys as the reference); the forward runs in libconvnn_b200: one packed
@@ -228,20 +314,23 @@ class MultiHeadAttention(nn.Module):
         self.W_o = nn.Linear(d_hidden, d_hidden, bias=False)
         self._packed = _PackedParams()
 
+    def packed_weights(self, dtype, device):
+        params = (self.W_q.weight, self.W_k.weight, self.W_v.weight, self.W_o.weight)
+        return self._packed.get(params, dtype, device, lambda: (
+            torch.stack([p.detach().to(device, dtype) for p in params[:3]]).contiguous(),
+            self.W_o.weight.detach().to(device, dtype).contiguous()))
+
     def forward(self, x, mask=None, out: Optional[torch.Tensor] = None):
         _library_call(x, "MultiHeadAttention")
         if mask is not None:
             raise RuntimeError("convnn_b200.MultiHeadAttention takes no mask (the reference's ViT never passes one)")
         if self.training and self.dropout.p > 0:
             raise RuntimeError("convnn_b200 is forward-only: dropout > 0 needs module.eval()")
-        params = (self.W_q.weight, self.W_k.weight, self.W_v.weight, self.W_o.weight)
-        w_qkv, w_o = self._packed.get(params, x.dtype, x.device, lambda: (
-            torch.stack([p.detach().to(x.device, x.dtype) for p in params[:3]]).contiguous(),
-            self.W_o.weight.detach().to(x.device, x.dtype).contiguous()))
+        w_qkv, w_o = self.packed_weights(x.dtype, x.device)
         return ops.softmax_attention(x, w_qkv, w_o, self.num_heads, out=out)
 
 
-class MultiHeadConv1dAttention(nn.Module):
+class MultiHeadConv1dAttention(WatchedModule):
     """Conv1d half of MultiHeadBranchingConv (reference layers.py:452-500): Linear, per-head
     Conv1d(d_k, d_k, kernel_size, padding='same'), the reference's flat head reinterpretation,
     Linear.  Parameters as in the reference; the forward runs in libconvnn_b200."""
@@ -257,20 +346,23 @@ class MultiHeadConv1dAttention(nn.Module):
         self.conv = nn.Conv1d(self.d_k, self.d_k, kernel_size=kernel_size, stride=1, padding="same")
         self._packed = _PackedParams()
 
-    def forward(self, x, out: Optional[torch.Tensor] = None):
-        _library_call(x, "MultiHeadConv1dAttention")
+    def packed_weights(self, dtype, device):
         params = (self.W_x.weight, self.W_x.bias, self.conv.weight, self.conv.bias, self.W_o.weight, self.W_o.bias)
 
         def build():
-            cvt = lambda t: t.detach().to(x.device, x.dtype).contiguous()
+            cvt = lambda t: t.detach().to(device, dtype).contiguous()
             # (d_k out, d_k in, kernel_size) -> (d_k out, kernel_size, d_k in): a (d_k, kernel_size * d_k) matrix
             return (cvt(self.W_x.weight), cvt(self.W_x.bias), cvt(self.conv.weight.permute(0, 2, 1)),
                     cvt(self.conv.bias), cvt(self.W_o.weight), cvt(self.W_o.bias))
-        w_x, b_x, w_c, b_c, w_o, b_o = self._packed.get(params, x.dtype, x.device, build)
+        return self._packed.get(params, dtype, device, build)
+
+    def forward(self, x, out: Optional[torch.Tensor] = None):
+        _library_call(x, "MultiHeadConv1dAttention")
+        w_x, b_x, w_c, b_c, w_o, b_o = self.packed_weights(x.dtype, x.device)
         return ops.conv1d_attention(x, w_x, b_x, w_c, b_c, w_o, b_o, self.num_heads, self.kernel_size, out=out)
 
 
-class _Branching(nn.Module):
+class _Branching(WatchedModule):
     def _init_common(self, d_hidden, num_heads, attention_dropout, K, sampling_type, num_samples,
                      sample_padding, magnitude_type, seq_length, coordinate_encoding, convolution_type,
                      softmax_topk_val, branch_ratio):
@@ -353,3 +445,7 @@ class MultiHeadBranchingConv(_Branching):
         else:
             return self._two_branches(x, self.conv1d, residual)
         return y if residual is None else residual + y
+
+
+OWN_MODULES = (MultiHeadConvNNAttention, MultiHeadAttention, MultiHeadConv1dAttention, MultiHeadBranchingAttention,
+               MultiHeadBranchingConv)

@@ -1,0 +1,234 @@
+"""Host plan of a ViT forward: everything ``convnn_b200_model_forward`` reads, prepared once.
+
+A ViT-Tiny forward is 52 launches; issued one binding call at a time they cost the host 1.14 ms (measured, one
+image), most of it argument handling and shape logic between the calls, so batches below ~100 images ran at the
+host's pace.  A plan holds the model's weight pointers, packed copies, layer descriptors and workspace size for
+one input shape; a forward then is a validity check, two allocations and one native call.
+
+A plan is used only while it describes the model: ``Watch.unchanged()`` compares the attribute epoch of this package's
+modules, the module tree, and identity, version counter and address of every parameter and buffer, and a call
+that finds a difference builds a new plan.  Anything a plan does not cover (training mode, hooks, a stage timer,
+parameters of another dtype or device) takes the op-by-op path in ``vit.py``.
+"""
+from __future__ import annotations
+
+import ctypes
+import threading
+import weakref
+from collections import OrderedDict
+
+import torch
+from torch.nn.modules import module as _nn_module
+
+from . import _capi, layers, ops
+from .layers import MultiHeadBranchingAttention, MultiHeadBranchingConv, MultiHeadConvNNAttention
+
+MAX_PLANS = 8                       # input shapes remembered per model
+_SEEN = object()                    # a shape that has been called once
+_plans: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
+
+
+class Watch:
+    """What a plan is valid for: one walk over the model's modules, taken before the plan is built."""
+
+    def __init__(self, model):
+        self.epoch = layers.attribute_epoch()
+        self.mods, self.trees, self.slots, self.tensors, self.hooks = [], [], [], [], []
+        todo, seen = [model], set()
+        while todo:
+            m = todo.pop()
+            if m is None or id(m) in seen:
+                continue
+            seen.add(id(m))
+            d = m.__dict__
+            self.mods.append(m)
+            children = d["_modules"]
+            if children:
+                self.trees.append((children, dict(children)))
+                todo.extend(children.values())
+            self.hooks += (d["_forward_hooks"], d["_forward_pre_hooks"])
+            for tensors in (d["_parameters"], d["_buffers"]):
+                for k, t in tensors.items():
+                    self.slots.append((tensors, k))
+                    if t is not None:
+                        self.tensors.append(t)
+        self.ids = [id(d[k]) for d, k in self.slots]
+        self.inputs = self.tensors + [m.candidate_override for m in self.mods if isinstance(m, MultiHeadConvNNAttention)
+                                      and m.candidate_override is not None]
+        self.versions = [t._version for t in self.inputs]
+        self.ptrs = [t.data_ptr() for t in self.inputs]
+
+    def unchanged(self) -> bool:
+        return (self.epoch == layers.attribute_epoch() and
+                [id(d[k]) for d, k in self.slots if k in d] == self.ids and
+                [t._version for t in self.inputs] == self.versions and
+                [t.data_ptr() for t in self.inputs] == self.ptrs and
+                all([d == c for d, c in self.trees]) and not any(self.hooks))
+
+
+class Plan:
+    def __init__(self, model, x: torch.Tensor, act: torch.dtype, watch: "Watch"):
+        a = model.args
+        B, C, Hh, Ww = x.shape
+        T, D = model.n_patches + 1, model.d_hidden
+        self.watch = watch
+        self.keep = []              # tensors whose addresses the structs hold
+        self.random = []            # (block index, attention layer): candidates drawn on every call
+        blocks = list(model.transformer_encoder)
+        self.blocks = (_capi.ConvnnBlock * max(1, len(blocks)))()
+        for i, blk in enumerate(blocks):
+            self._block(i, blk, B, T, D, act, x.device)
+        pe, pemb, cls = model.positional_encoding, model.patch_embedding, model.positional_encoding.cls_tokens
+        conv = pemb.linear_projection
+        m = self.model = _capi.ConvnnModel()
+        m.dtype, m.B, m.T, m.D = ops._dtype_code(act), B, T, D
+        m.n_blocks, m.classes = len(blocks), model.classifier.out_features
+        m.channels, m.height, m.width, m.patch = C, Hh, Ww, a.patch_size
+        m.embed_eps = pemb.norm.eps
+        m.blocks = ctypes.cast(self.blocks, ctypes.POINTER(_capi.ConvnnBlock))
+        m.patch_w, m.patch_b = self._ptr(conv.weight.view(D, -1)), self._ptr(conv.bias)
+        m.embed_norm_w, m.embed_norm_b = self._ptr(pemb.norm.weight), self._ptr(pemb.norm.bias)
+        m.cls, m.pe = self._ptr(cls.view(-1)), self._ptr(pe.pe.view(-1, D)[:T])
+        m.head_w, m.head_b = self._ptr(model.classifier.weight), self._ptr(model.classifier.bias)
+        m.images_u8 = int(x.dtype == torch.uint8)
+        if m.images_u8:
+            _, mean, inv_std = model.pixel_stats(x.device)
+            m.pixel_mean, m.pixel_inv_std = self._ptr(mean), self._ptr(inv_std)
+        self.act, self.out_shape, self.lock = act, (B, model.classifier.out_features), threading.Lock()
+        L = _capi.lib()
+        self.call, self.arg = L.convnn_b200_model_forward, ctypes.byref(m)
+        self.workspace_bytes = L.convnn_b200_model_workspace_bytes(self.arg)
+
+    # -- construction -------------------------------------------------------------------------------
+    def _ptr(self, t):
+        if t is None:
+            return None
+        if not t.is_contiguous():
+            t = t.contiguous()
+        self.keep.append(t)
+        return t.data_ptr()
+
+    def _folded(self, b, names, fold):
+        wf, wx = fold
+        setattr(b, names[0], self._ptr(wf))
+        setattr(b, names[1], self._ptr(wx))
+
+    def _layer(self, b, i, att, B, T, act, device):
+        """The ConvNN layer of a block: descriptor, packed weights, candidates."""
+        cand, S, spec = None, T, att._spec()
+        if att.sampling_type == "random" and att.candidate_override is None:
+            self.random.append((i, att))
+            S = len(range(T)[:att.num_samples])
+        else:
+            cand, S = ops._cand_arg(spec, att.candidates(T, device), T, device)
+        b.layer = ops.descriptor(spec, B, T, S, act)
+        b.cand = self._ptr(cand)
+        w_qkv, w_conv, w_pw, w_o = att.packed_weights(act, device)
+        b.w_qkv, b.w_conv, b.w_pw, b.w_o = (self._ptr(w) for w in (w_qkv, w_conv, w_pw, w_o))
+
+    def _block(self, i, blk, B, T, D, act, device):
+        b, att = self.blocks[i], blk.attention
+        n1, n2, fc1, fc2 = blk.norm1, blk.norm2, blk.mlp[0], blk.mlp[3]
+        branching = isinstance(att, (MultiHeadBranchingAttention, MultiHeadBranchingConv))
+        self._layer(b, i, att.convnn if branching else att, B, T, act, device)
+        b.d_mlp, b.eps1, b.eps2 = fc1.out_features, n1.eps, n2.eps
+        b.norm1_w, b.norm1_b, b.norm2_w, b.norm2_b = (self._ptr(t) for t in (n1.weight, n1.bias, n2.weight, n2.bias))
+        b.fc1_w, b.fc1_b, b.fc2_w, b.fc2_b = (self._ptr(t) for t in (fc1.weight, fc1.bias, fc2.weight, fc2.bias))
+        if not branching and blk.folds_norm1_shape(B, T, act):
+            self._folded(b, ("w_qkv_folded", "w_qkv_extra"), att.folded_qkv(n1, act, device))
+        if (blk.fold_layernorm and act == torch.bfloat16 and
+                ops.prenorm_linear_supported(fc1.out_features, fc1.in_features, True)):
+            self._folded(b, ("fc1_folded", "fc1_extra"), blk.folded_fc1(act, device))
+        b.fuse_mlp = int(blk.fuse_mlp)
+        if branching:
+            other = att.attention if isinstance(att, MultiHeadBranchingAttention) else att.conv1d
+            packed = [self._ptr(w) for w in other.packed_weights(act, device)]
+            if isinstance(att, MultiHeadBranchingAttention):
+                b.kind, (b.branch_w_in, b.branch_w_out) = _capi.BLOCK_BRANCH_ATTENTION, packed
+            else:
+                b.kind, b.kernel_size = _capi.BLOCK_BRANCH_CONV1D, other.kernel_size
+                (b.branch_w_in, b.branch_b_in, b.branch_w_conv, b.branch_b_conv, b.branch_w_out, b.branch_b_out) = packed
+            b.pointwise_w, b.pointwise_b = self._ptr(att.pointwise_linear.weight), self._ptr(att.pointwise_linear.bias)
+
+    # -- a forward ----------------------------------------------------------------------------------
+    def run(self, x: torch.Tensor) -> torch.Tensor:
+        if not x.is_contiguous():
+            x = x.contiguous()
+        dev = x.device
+        out = torch.empty(self.out_shape, dtype=self.act, device=dev)
+        ws = torch.empty(self.workspace_bytes, dtype=torch.uint8, device=dev)
+        args = (self.arg, x.data_ptr(), out.data_ptr(), ws.data_ptr(), self.workspace_bytes, ops._stream(x))
+        if self.random:
+            # drawn per layer and call, in the order of the layers; the lock keeps the structs this call's until it returns
+            drawn = [att.candidates(self.model.T, dev).to(torch.int32) for _, att in self.random]
+            with self.lock:
+                for (i, _), cand in zip(self.random, drawn):
+                    self.blocks[i].cand = cand.data_ptr()
+                rc = self.call(*args)
+        else:
+            rc = self.call(*args)
+        if rc:
+            _capi.check(rc)
+        return out
+
+
+class _Refused:
+    """A shape no plan covers, remembered until an attribute of the model changes."""
+
+    def __init__(self):
+        self.watch, self.epoch = self, layers.attribute_epoch()
+
+    def unchanged(self) -> bool:
+        return self.epoch == layers.attribute_epoch()
+
+
+def _covered(model, x: torch.Tensor, act: torch.dtype, watch: Watch) -> bool:
+    """Whether a plan can describe this call."""
+    from .vit import TransformerEncoder, ViT
+    if (type(model) is not ViT or x.dim() != 4 or x.shape[0] < 1 or act not in (torch.float32, torch.bfloat16) or
+            tuple(x.shape[1:]) != tuple(model.args.img_size) or not all(type(b) is TransformerEncoder
+                                                                        for b in model.transformer_encoder)):
+        return False
+    if any(watch.hooks):
+        return False
+    for m in watch.mods:
+        if isinstance(m, layers.WatchedModule) and (m.training or getattr(m, "stage_timer", None) is not None):
+            return False
+    for blk in model.transformer_encoder:
+        att = blk.attention
+        if blk.fuse_out_proj or type(att) not in layers.OWN_MODULES:
+            return False
+        if isinstance(att, (MultiHeadBranchingAttention, MultiHeadBranchingConv)) and not 0 < att.branch_ratio < 1:
+            return False
+    dev = x.device
+    return all([t.dtype == act and t.device == dev and t.is_contiguous() for t in watch.tensors])
+
+
+def run(model, x: torch.Tensor):
+    """The logits through a plan, or None where the op-by-op path has to be taken."""
+    per_model = _plans.get(model)
+    if per_model is None:
+        per_model = _plans.setdefault(model, OrderedDict())
+    if _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks:
+        return None
+    key = (x.shape, x.dtype, x.device)
+    plan = per_model.get(key)
+    if plan is not None and plan is not _SEEN and plan.watch.unchanged():
+        return plan.run(x) if type(plan) is Plan else None
+    # The first call of a shape, and the first after a change of the model, goes op by op: it packs weights while
+    # the GPU works, and a shape that never returns pays for no plan.  The second call builds the plan.
+    if plan is not _SEEN:
+        per_model[key] = _SEEN
+        while len(per_model) > MAX_PLANS:
+            per_model.popitem(last=False)
+        return None
+    act = model.patch_embedding.linear_projection.weight.dtype if x.dtype == torch.uint8 else x.dtype
+    watch = Watch(model)
+    if not _covered(model, x, act, watch):
+        per_model[key] = _Refused()
+        return None
+    plan = Plan(model, x, act, watch)
+    if plan.workspace_bytes == 0:           # a shape the library refuses: the op-by-op path raises its error
+        return None
+    per_model[key] = plan
+    return plan.run(x)

@@ -51,7 +51,14 @@ def _require_cuda(*tensors) -> None:
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _raw_stream(t.get_device())
+
+
+try:                                          # the stream's handle without a Python Stream object around it
+    _raw_stream = torch._C._cuda_getCurrentRawStream
+except AttributeError:
+    def _raw_stream(index: int) -> int:
+        return torch.cuda.current_stream(index).cuda_stream
 
 
 def descriptor(spec: LayerSpec, B: int, T: int, S: int, dtype: torch.dtype) -> _capi.ConvnnDesc:
@@ -233,6 +240,39 @@ def forward(spec: LayerSpec, x: torch.Tensor, packed, cand: Optional[torch.Tenso
                                       w_o.data_ptr(), _capi.ptr(cand), _capi.ptr(res), ldr, out.data_ptr(), ldo,
                                       workspace.data_ptr(), workspace.numel(), _stream(x)))
     return out
+
+
+class LayerForward:
+    """``forward`` for a fixed shape, its descriptor, weight addresses and workspace size looked up once.  The caller
+    keeps ``packed`` unchanged while it uses the object, and passes candidates as int32 on the device."""
+
+    def __init__(self, spec: LayerSpec, B: int, T: int, S: int, dtype, device, packed):
+        L = _capi.lib()
+        self.d = descriptor(spec, B, T, S, dtype)
+        self.need = L.convnn_b200_workspace_bytes(self.d)
+        if self.need == 0:
+            _capi.check(min(L.convnn_b200_head_channels(self.d), 0))
+        self.D, self.dtype, self.device, self.packed = spec.d_hidden, dtype, device, packed
+        self.w = [_capi.ptr(w) for w in packed]
+
+    def __call__(self, x: torch.Tensor, cand: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
+                 residual: Optional[torch.Tensor] = None) -> torch.Tensor:
+        x, ldx = _rows_view(x)
+        workspace = torch.empty(self.need, dtype=torch.uint8, device=self.device)
+        if out is None:
+            out, ldo = torch.empty(x.shape, dtype=self.dtype, device=self.device), self.D
+        else:
+            view, ldo = _rows_view(out)
+            if view is not out:
+                raise ValueError("out must have unit channel stride and evenly strided rows")
+        res, ldr = (None, 0) if residual is None else _residual_arg(residual, x)
+        w = self.w
+        rc = _capi.lib().convnn_b200_forward(
+            self.d, x.data_ptr(), ldx, w[0], w[1], w[2], w[3], None if cand is None else cand.data_ptr(),
+            None if res is None else res.data_ptr(), ldr, out.data_ptr(), ldo, workspace.data_ptr(), self.need, _stream(x))
+        if rc:
+            _capi.check(rc)
+        return out
 
 
 # ---- LayerNorm folded into the GEMM that consumes it (bfloat16) --------------------------------

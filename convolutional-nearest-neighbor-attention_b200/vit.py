@@ -17,8 +17,9 @@ from types import SimpleNamespace
 import torch
 import torch.nn as nn
 
-from . import ops
-from .layers import MultiHeadBranchingAttention, MultiHeadBranchingConv, MultiHeadConvNNAttention, _PackedParams
+from . import model_plan, ops
+from .layers import (MultiHeadBranchingAttention, MultiHeadBranchingConv, MultiHeadConvNNAttention, WatchedModule,
+                     _PackedParams)
 
 _DEFAULTS = dict(layer="ConvNNAttention", patch_size=16, num_layers=12, num_heads=3, d_hidden=192, d_mlp=768,
                  dropout=0.1, attention_dropout=0.1, convolution_type="depthwise", softmax_topk_val=True, K=9,
@@ -34,7 +35,7 @@ def make_args(**overrides) -> SimpleNamespace:
     return SimpleNamespace(**a)
 
 
-class PatchEmbedding(nn.Module):
+class PatchEmbedding(WatchedModule):
     def __init__(self, d_hidden, img_size, patch_size, n_channels=3):
         super().__init__()
         self.linear_projection = nn.Conv2d(n_channels, d_hidden, kernel_size=patch_size, stride=patch_size)
@@ -50,7 +51,7 @@ def _library_path(x: torch.Tensor) -> bool:
     return x.is_cuda and x.dtype in (torch.float32, torch.bfloat16, torch.uint8) and not torch.is_grad_enabled()
 
 
-class PositionalEncoding(nn.Module):
+class PositionalEncoding(WatchedModule):
     def __init__(self, d_hidden, max_seq_length):
         super().__init__()
         self.cls_tokens = nn.Parameter(torch.randn(1, 1, d_hidden))
@@ -66,7 +67,7 @@ class PositionalEncoding(nn.Module):
         return x + self.pe[:, :x.size(1)]
 
 
-class TransformerEncoder(nn.Module):
+class TransformerEncoder(WatchedModule):
     def __init__(self, args, d_hidden, d_mlp, num_heads, dropout, attention_dropout):
         super().__init__()
         common = dict(K=args.K, sampling_type=args.sampling_type, num_samples=args.num_samples,
@@ -117,6 +118,12 @@ class TransformerEncoder(nn.Module):
         return (self.fold_layernorm and isinstance(self.attention, MultiHeadConvNNAttention) and
                 self.attention.prenorm_supported_shape(B, T, dtype))
 
+    def folded_fc1(self, dtype, device):
+        """The first MLP weight with norm2 folded in (``ops.fold_layernorm``)."""
+        fc1, n2 = self.mlp[0], self.norm2
+        return self._fc1_folded.get((fc1.weight, fc1.bias, n2.weight, n2.bias), dtype, device,
+                                    lambda: ops.fold_layernorm(fc1.weight, fc1.bias, n2.weight, n2.bias))
+
     def _forward_library(self, x, moments=None, want_moments=False):
         """The same block in libconvnn_b200: both Linear layers (GELU and the skip connections folded
         into their stores), the attention layer with its output projection (+ skip), and the two
@@ -136,8 +143,7 @@ class TransformerEncoder(nn.Module):
                     ops.prenorm_mlp_supported(fc1.in_features, fc1.out_features, 1)):
                 # attention up to the gather / conv, then ONE kernel for W_o + skip + norm2 + mlp + skip
                 o, _ = self.attention.forward_prenorm(x, moments, n1, skip_out_proj=True)
-                wf, wx = self._fc1_folded.get((fc1.weight, fc1.bias, n2.weight, n2.bias), x.dtype, x.device,
-                                              lambda: ops.fold_layernorm(fc1.weight, fc1.bias, n2.weight, n2.bias))
+                wf, wx = self.folded_fc1(x.dtype, x.device)
                 return ops.outproj_mlp(o, self.attention.packed_w_o, x, n2.eps, wf, wx, fc2.weight, fc2.bias,
                                        want_moments=want_moments)
             x, m1 = self.attention.forward_prenorm(x, moments, n1, residual=x, want_moments=fold_mlp)
@@ -147,8 +153,7 @@ class TransformerEncoder(nn.Module):
         if fold_mlp:
             if m1 is None:
                 m1 = ops.row_moments(x)
-            wf, wx = self._fc1_folded.get((fc1.weight, fc1.bias, n2.weight, n2.bias), x.dtype, x.device,
-                                          lambda: ops.fold_layernorm(fc1.weight, fc1.bias, n2.weight, n2.bias))
+            wf, wx = self.folded_fc1(x.dtype, x.device)
             if self.fuse_mlp and ops.prenorm_mlp_supported(fc1.in_features, fc1.out_features, m1.shape[0]):
                 # the whole block in one kernel: the hidden activations never reach HBM
                 return ops.prenorm_mlp(x, m1, n2.eps, wf, wx, fc2.weight, fc2.bias, want_moments=want_moments)
@@ -161,7 +166,7 @@ class TransformerEncoder(nn.Module):
         return ops.linear(h, fc2.weight, fc2.bias, residual=x), None
 
 
-class ViT(nn.Module):
+class ViT(WatchedModule):
     def __init__(self, args):
         super().__init__()
         assert args.img_size[1] % args.patch_size == 0 and args.img_size[2] % args.patch_size == 0, \
@@ -189,14 +194,13 @@ class ViT(nn.Module):
 
     def forward(self, x):
         if _library_path(x):
+            y = model_plan.run(self, x)          # one native call; None: this call needs the op-by-op path
+            if y is not None:
+                return y
             pe_mod, pemb = self.positional_encoding, self.patch_embedding
             mean = inv_std = None
             if x.dtype == torch.uint8:
-                key = (tuple(self.pixel_mean), tuple(self.pixel_std), x.device)
-                if self._pixel_stats is None or self._pixel_stats[0] != key:
-                    self._pixel_stats = (key, torch.tensor(self.pixel_mean, dtype=torch.float32, device=x.device),
-                                         1.0 / torch.tensor(self.pixel_std, dtype=torch.float32, device=x.device))
-                _, mean, inv_std = self._pixel_stats
+                _, mean, inv_std = self.pixel_stats(x.device)
             blocks = list(self.transformer_encoder)
             act = pemb.linear_projection.weight.dtype if x.dtype == torch.uint8 else x.dtype
             T = self.n_patches + 1
@@ -220,6 +224,14 @@ class ViT(nn.Module):
         x = self.positional_encoding(self.patch_embedding(x))
         x = self.transformer_encoder(x)
         return self.classifier(x[:, 0])
+
+    def pixel_stats(self, device):
+        """(key, mean, 1 / std) of the normalisation of 8-bit images, on ``device``."""
+        key = (tuple(self.pixel_mean), tuple(self.pixel_std), device)
+        if self._pixel_stats is None or self._pixel_stats[0] != key:
+            self._pixel_stats = (key, torch.tensor(self.pixel_mean, dtype=torch.float32, device=device),
+                                 1.0 / torch.tensor(self.pixel_std, dtype=torch.float32, device=device))
+        return self._pixel_stats
 
     def set_candidates(self, cand):
         """Fix the candidate set of every sampled-mode ConvNN layer (the reference redraws a

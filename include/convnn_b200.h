@@ -338,6 +338,48 @@ int convnn_b200_conv1d_attention(int dtype, const void* x, int64_t ldx, const vo
                                  void* out, int64_t ldo, int32_t B, int32_t T, int32_t D, int32_t H,
                                  int32_t kernel_size, void* workspace, size_t workspace_bytes, void* stream);
 
+/* ---- the whole ViT forward as one call ----------------------------------------------------------
+ * The chain of the entry points above for a model whose weights, packed copies and candidate sets
+ * already exist: patch embedding, n_blocks encoder blocks, classifier (reference vit.py:71, 99-135,
+ * 247-270).  A forward is 50-170 launches; issuing them from one native call costs the host about
+ * two microseconds per launch instead of about twenty through one binding call each. */
+enum convnn_block_kind { CONVNN_BLOCK_CONVNN = 0, CONVNN_BLOCK_BRANCH_ATTENTION = 1, CONVNN_BLOCK_BRANCH_CONV1D = 2 };
+
+typedef struct convnn_block {
+    convnn_desc layer;          /* the ConvNN layer; layer.D < D of the model for the branching kinds */
+    int32_t kind;               /* enum convnn_block_kind */
+    int32_t d_mlp;
+    int32_t kernel_size;        /* BRANCH_CONV1D */
+    int32_t fuse_mlp;           /* with fc1_folded: MLP block as one kernel where it is built */
+    float eps1, eps2;
+    const void *norm1_w, *norm1_b, *norm2_w, *norm2_b;
+    const void *w_qkv, *w_conv, *w_pw, *w_o;
+    const int32_t* cand;        /* sampled layers: candidate tokens */
+    const void *w_qkv_folded, *w_qkv_extra;   /* norm1 folded (convnn_b200_fold_layernorm), or NULL */
+    const void *fc1_w, *fc1_b, *fc2_w, *fc2_b;
+    const void *fc1_folded, *fc1_extra;       /* norm2 folded, or NULL */
+    /* the other branch: [W_q; W_k; W_v] and W_o, or W_x, b_x, taps, tap bias, W_o, b_o; then pointwise_linear */
+    const void *branch_w_in, *branch_b_in, *branch_w_conv, *branch_b_conv, *branch_w_out, *branch_b_out;
+    const void *pointwise_w, *pointwise_b;
+} convnn_block;
+
+typedef struct convnn_model {
+    int32_t dtype, B, T, D;     /* T = patches + 1 */
+    int32_t n_blocks, classes;
+    int32_t channels, height, width, patch;
+    int32_t images_u8;          /* images are 8-bit, normalised with pixel_mean / pixel_inv_std */
+    float embed_eps;
+    const convnn_block* blocks; /* HOST array */
+    const void *patch_w, *patch_b, *embed_norm_w, *embed_norm_b, *cls, *pe;
+    const float *pixel_mean, *pixel_inv_std;
+    const void *head_w, *head_b;
+} convnn_model;
+
+size_t convnn_b200_model_workspace_bytes(const convnn_model* m);
+/* images (B, C, H, W) -> logits (B, classes).  The structs are read during the call only. */
+int convnn_b200_model_forward(const convnn_model* m, const void* images, void* logits, void* workspace,
+                              size_t workspace_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif
