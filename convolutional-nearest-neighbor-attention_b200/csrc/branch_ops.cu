@@ -4,7 +4,8 @@
 // Activations are token-major (B, T, H, d_k).  bfloat16 with d_k a multiple of 16: the taps are
 // unfolded, U[(b, h, t), j * d_k + c] = y[b, t + j - pad, h, c] (zero outside the sequence), and
 // the conv becomes U x W^T with W = (d_k, kernel_size * d_k) on the tensor-core GEMM, bias in its
-// epilogue.  Everything else (float32, odd head widths) takes a direct SIMT kernel.
+// epilogue.  Float32 takes the SIMT GEMM with the shifted rows as its implicit A operand; head widths that are no
+// multiple of four a direct SIMT kernel.
 #include "common.cuh"
 
 namespace convnn {
@@ -83,6 +84,13 @@ int launch_conv1d_heads(int dtype, const void* y, const void* w, const void* bia
         GemmTcOpts go;
         go.bias = bias;
         return launch_gemm_tc(unfold, (long long)ks * dk, w, (int)M, dk, ks * dk, 1, cs, dk, go, st);
+    }
+    if (dk % 4 == 0 && M < (1ll << 31)) {
+        GemmParams p{};
+        p.a = y; p.w = w; p.bias = bias; p.bias_first = 1; p.c = o; p.ldc = dk;
+        p.M = (int)M; p.N = dk; p.Kd = ks * dk; p.a_mode = A_CONV1D; p.c_mode = C_ROWS;
+        p.T = Tn; p.H = H; p.dk = dk; p.Cp = dk; p.C = dk; p.pad = pad;
+        return launch_gemm_simt(dtype, p, st);
     }
     const long long total = M * dk;
     int blocks = (int)((total + 255) / 256);

@@ -142,12 +142,13 @@ size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 // GEMM operand and for the head-merged (B, T, D) operand of the output projection.
 size_t stage_scratch(const Dims& dm, int conv_type) {
     size_t n = (size_t)dm.B * (dm.T > dm.S ? dm.T : dm.S) * dm.D;
-    if (conv_type == CONVNN_STANDARD) {          // weighted neighbour block (B, H, T, K*C) of the tensor-core conv
+    if (conv_type == CONVNN_STANDARD && dm.elt == 2 && dm.C == dm.dk) {          // weighted neighbour block (B, H, T, K*C) of the tensor-core conv
         const size_t m = (size_t)dm.B * dm.H * dm.T * dm.K * dm.C;
         if (m > n) n = m;
     } else if (conv_type == CONVNN_DEPTHWISE_SEPARABLE) {
-        const size_t m = (size_t)dm.B * dm.H * dm.T * dm.C;
-        if (m > n) n = m;
+        const size_t m = (size_t)dm.B * dm.H * dm.T * dm.Cp;     // (unrounded with the coordinate channel)
+        const size_t bytes = dm.C != dm.dk ? m * 4 : m * dm.elt;
+        if (bytes > n * dm.elt) return bytes;
     }
     return n * dm.elt;
 }
@@ -321,16 +322,16 @@ int qkv_proj_impl(const convnn_desc* d, const void* x, int64_t ldx, const void* 
     GemmParams p{};
     p.a = x; p.lda = ldx; p.bias = nullptr; p.N = dm.D; p.Kd = dm.D;
     p.a_mode = A_TOKENS; p.c_mode = C_HEADS; p.T = dm.T; p.H = dm.H; p.dk = dm.dk; p.Cp = dm.Cp; p.gelu = 0;
-    // keys and values: every token
-    p.cand = nullptr; p.rows_per_batch = dm.T; p.M = dm.B * dm.T;
-    p.w = static_cast<const char*>(w_qkv); p.c = k;
+    // keys and values: every token; queries: candidate tokens only (with sampling 'all' one launch makes all three)
+    const int parts = d->sampled ? 2 : 3;
+    p.rows_per_batch = dm.T; p.M = dm.B * dm.T; p.N = parts * dm.D; p.part_cols = dm.D;
+    p.w = w_qkv; p.c = k; p.c1 = v; p.c2 = d->sampled ? nullptr : q;
     if ((rc = launch_gemm_simt(d->dtype, p, st))) return rc;
-    p.w = static_cast<const char*>(w_qkv) + wsz; p.c = v;
-    if ((rc = launch_gemm_simt(d->dtype, p, st))) return rc;
-    // queries: candidate tokens only
-    p.cand = d->sampled ? cand : nullptr; p.rows_per_batch = dm.S; p.M = dm.B * dm.S;
-    p.w = static_cast<const char*>(w_qkv) + 2 * wsz; p.c = q;
-    if ((rc = launch_gemm_simt(d->dtype, p, st))) return rc;
+    if (d->sampled) {
+        p.cand = cand; p.rows_per_batch = dm.S; p.M = dm.B * dm.S; p.N = dm.D;
+        p.w = static_cast<const char*>(w_qkv) + 2 * wsz; p.c = q; p.c1 = nullptr;
+        if ((rc = launch_gemm_simt(d->dtype, p, st))) return rc;
+    }
     if ((rc = launch_head_fill_and_stats(d, dm, q, dm.S, stats ? qstat : nullptr, st))) return rc;
     if ((rc = launch_head_fill_and_stats(d, dm, k, dm.T, stats ? kstat : nullptr, st))) return rc;
     if ((rc = launch_head_fill_and_stats(d, dm, v, dm.T, nullptr, st))) return rc;
@@ -403,6 +404,10 @@ int out_proj_impl(const convnn_desc* d, const void* o, const void* w_o, const vo
     p.a = o; p.w = w_o; p.bias = nullptr; p.c = out; p.cand = nullptr;
     p.lda = dm.D; p.ldc = ldo; p.M = dm.B * dm.T; p.N = dm.D; p.Kd = dm.D;
     p.a_mode = dm.H == 1 ? A_ROWS : A_HEAD_QUIRK; p.c_mode = C_ROWS;
+    if (dm.H > 1 && scratch) {       // the head reinterpretation once, instead of a strided operand per column tile
+        if ((rc = launch_merge_heads(d->dtype, o, scratch, dm.B, dm.T, dm.H, dm.dk, static_cast<cudaStream_t>(stream)))) return rc;
+        p.a = scratch; p.a_mode = A_ROWS;
+    }
     p.rows_per_batch = dm.T; p.T = dm.T; p.H = dm.H; p.dk = dm.dk; p.Cp = dm.Cp; p.gelu = 0;
     p.residual = residual; p.ldr = ldr;
     return launch_gemm_simt(d->dtype, p, static_cast<cudaStream_t>(stream));

@@ -77,7 +77,9 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(flo
 enum AMode : int {
     A_ROWS = 0,       // A[m, kk] = a[m * lda + kk]
     A_TOKENS = 1,     // m = (b, r): token = cand ? cand[r] : r; a[(b*T + token) * lda + kk]
-    A_HEAD_QUIRK = 2  // m = (b, t'), kk = h*dk + c': a[((b*H + h) * T) * dk + c' * T + t']
+    A_HEAD_QUIRK = 2, // m = (b, t'), kk = h*dk + c': a[((b*H + h) * T) * dk + c' * T + t']
+    A_NEIGHBOURS = 3, // m = (b, h, t), kk = j*Cp + c: weight[m, j] * a[(b, neighbour[m, j], h, c)], a (B, T, H, Cp); Cp % 4 == 0
+    A_CONV1D = 4      // m = (b, h, t), kk = j*Cp + c: a[(b, t + j - pad, h, c)], zero outside the sequence; Cp % 4 == 0
 };
 // C placement of the SIMT GEMM.
 enum CMode : int {
@@ -99,6 +101,18 @@ struct GemmParams {
     int gelu;             // apply exact GELU after bias
     const void* residual; // (M, N) with row stride ldr, added after rounding to dtype; or nullptr
     long long ldr;
+    // the N columns may be split into up to three outputs of part_cols columns each (0: one output)
+    void *c1, *c2;
+    int part_cols;
+    long long ldw;        // row stride of w (0: Kd)
+    int bias_first;       // the sum starts from the bias instead of adding it at the end
+    int a_f32;            // bfloat16 weights and output, float32 A operand (A_ROWS)
+    // A_NEIGHBOURS: lists (M, taps) and how their values become weights; w rows hold taps x C values
+    const int32_t* nb_idx;
+    const float* nb_val;
+    int taps, C, nb_maximum, nb_softmax;
+    int pad;              // A_CONV1D
+    bool a_vec, w_vec, c_vec;   // set by the launcher
 };
 
 int launch_gemm_simt(int dtype, const GemmParams& p, cudaStream_t st);

@@ -13,7 +13,9 @@
 //   * bfloat16 standard / separable on the tensor cores: a gather kernel writes the GEMM's A
 //     operand (the weighted neighbour block, or the depthwise result) and gemm_tc multiplies it
 //     with the (d_k, K*C) tap matrix / the (d_k, C) pointwise matrix;
-//   * float32 (and fallback) standard / separable: shared-memory staged block times the weights.
+//   * float32, and the coordinate channel: the SIMT GEMM, standard with the neighbour block as its implicit A operand,
+//     separable over the depthwise result;
+//   * channel counts that are no multiple of four: shared-memory staged block times the weights.
 // The three K-times expanded copies of V that the reference builds never exist (the tensor-core
 // standard conv materialises the weighted block once, in bfloat16).
 #include "common.cuh"
@@ -179,6 +181,56 @@ __global__ void __launch_bounds__(THREADS) gather_conv_mat_kernel(
             }
         }
     }
+}
+
+// Depthwise stage of the separable conv with the coordinate channel: C = d_k + 1 taps per neighbour against rows of Cp
+// stored channels, result unrounded in float32 rows of Cp values (the padding comes out as zero).
+template <typename T, int TT>
+__global__ void __launch_bounds__(THREADS) gather_conv_dw_padded_kernel(
+    const T* __restrict__ v, const int32_t* __restrict__ idx, const float* __restrict__ val,
+    const T* __restrict__ wconv, float* __restrict__ o, int T_, int H, int C, int Cp, int K, int maximum, int softmax) {
+    __shared__ float ps[TT][kMaxK];
+    __shared__ int ns[TT][kMaxK];
+    const int bh = blockIdx.y, b = bh / H, h = bh - b * H;
+    const int t0 = blockIdx.x * TT, nt = min(TT, T_ - t0);
+    const long long nbase = ((long long)bh * T_ + t0) * K;
+    for (int e = threadIdx.x; e < nt * K; e += THREADS) ns[e / K][e % K] = idx[nbase + e] * (H * Cp);
+    if (threadIdx.x < nt) token_weights(val + nbase + (long long)threadIdx.x * K, ps[threadIdx.x], K, maximum, softmax);
+    __syncthreads();
+    const T* vb = v + ((long long)b * T_ * H + h) * Cp;
+    const int groups = Cp / 4;
+    for (int item = threadIdx.x; item < nt * groups; item += THREADS) {
+        const int tt = item / groups, c = (item - tt * groups) * 4;
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int j = 0; j < K; ++j) {
+            const T* src = vb + ns[tt][j] + c;
+            float x[4];
+            if (sizeof(T) == 4) {
+                const float4 q = *reinterpret_cast<const float4*>(src);
+                x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
+            } else {
+                const uint2 q = *reinterpret_cast<const uint2*>(src);
+                x[0] = __uint_as_float(q.x << 16); x[1] = __uint_as_float(q.x & 0xffff0000u);
+                x[2] = __uint_as_float(q.y << 16); x[3] = __uint_as_float(q.y & 0xffff0000u);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (c + e < C) acc[e] = fmaf(to_f32<T>(wconv[j * C + c + e]), ps[tt][j] * x[e], acc[e]);
+        }
+        *reinterpret_cast<float4*>(o + ((long long)bh * T_ + t0 + tt) * Cp + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    }
+}
+
+template <typename T>
+int launch_dw_padded(const convnn_desc* d, const Dims& dm, const void* v, const int32_t* idx, const float* val,
+                     const void* w_conv, void* o, cudaStream_t st) {
+    constexpr int TT = 8;
+    dim3 grid((dm.T + TT - 1) / TT, dm.B * dm.H);
+    gather_conv_dw_padded_kernel<T, TT><<<grid, THREADS, 0, st>>>(
+        static_cast<const T*>(v), idx, val, static_cast<const T*>(w_conv), static_cast<float*>(o), dm.T, dm.H, dm.C, dm.Cp,
+        dm.K, d->metric != CONVNN_EUCLIDEAN, d->softmax);
+    CONVNN_CHECK_LAUNCH("gather_conv_dw_padded");
+    return CONVNN_OK;
 }
 
 template <typename T, int VEC>
@@ -349,6 +401,31 @@ int launch_gather_conv_simt(const convnn_desc* d, const Dims& dm, const void* v,
                                : launch_dw<float, 1>(d, dm, v, idx, val, w_conv, o, st);
         return vec_ok ? launch_dw<__nv_bfloat16, 8>(d, dm, v, idx, val, w_conv, o, st)
                       : launch_dw<__nv_bfloat16, 1>(d, dm, v, idx, val, w_conv, o, st);
+    }
+    if (dm.Cp % 4 == 0 && aligned16(v)) {
+        GemmParams p{};
+        p.w = w_conv; p.c = o; p.ldc = dm.dk; p.M = dm.B * dm.H * dm.T; p.N = dm.dk; p.c_mode = C_ROWS;
+        p.T = dm.T; p.H = dm.H; p.dk = dm.dk; p.Cp = dm.Cp; p.C = dm.C;
+        if (d->conv_type == CONVNN_STANDARD) {
+            // implicit GEMM over the weighted neighbour block, gathered tile by tile as the A operand
+            p.a = v; p.a_mode = A_NEIGHBOURS; p.Kd = dm.K * dm.Cp; p.ldw = (long long)dm.K * dm.C;
+            p.nb_idx = idx; p.nb_val = val; p.taps = dm.K; p.nb_maximum = d->metric != CONVNN_EUCLIDEAN; p.nb_softmax = d->softmax;
+            return launch_gemm_simt(d->dtype, p, st);
+        }
+        if (scratch && aligned16(scratch) && (f32 || d->coord)) {
+            // depthwise stage into scratch (float32, padded to the stored channels where there are more), then the
+            // pointwise matrix
+            int rc = CONVNN_E_UNSUPPORTED;
+            if (!d->coord) {
+                rc = try_launch_gather_conv_dw_smem(d, dm, v, idx, val, w_conv, scratch, st);
+                if (rc == CONVNN_E_UNSUPPORTED && aligned16(w_conv)) rc = launch_dw<float, 4>(d, dm, v, idx, val, w_conv, scratch, st);
+            }
+            if (rc == CONVNN_E_UNSUPPORTED) rc = f32 ? launch_dw_padded<float>(d, dm, v, idx, val, w_conv, scratch, st)
+                                                     : launch_dw_padded<__nv_bfloat16>(d, dm, v, idx, val, w_conv, scratch, st);
+            if (rc) return rc;
+            p.a = scratch; p.lda = dm.Cp; p.a_mode = A_ROWS; p.a_f32 = 1; p.Kd = dm.C; p.w = w_pw; p.ldw = dm.C;
+            return launch_gemm_simt(d->dtype, p, st);
+        }
     }
     return f32 ? launch_mat<float>(d, dm, v, idx, val, w_conv, w_pw, o, st)
                : launch_mat<__nv_bfloat16>(d, dm, v, idx, val, w_conv, w_pw, o, st);

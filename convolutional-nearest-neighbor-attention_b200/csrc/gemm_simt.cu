@@ -1,118 +1,356 @@
-// FP32-accumulate SIMT GEMM  C = A * W^T (+ bias, + GELU)  with the operand addressing
-// modes the ConvNN path needs: token gather for the sampled-query projection, head-split
-// stores for q/k/v, and the reference's flat head reinterpretation as the A operand of
-// the output projection.  This is the float32 path (tensor cores would need a 3xTF32
-// split to keep the 1e-6 similarity accuracy the top-K parity asks for) and the
-// fallback for bfloat16 shapes the tcgen05 kernels do not cover.
+// FP32-accumulate SIMT GEMM  C = A * W^T (+ bias, + GELU)  with the operand addressing modes the ConvNN path needs:
+// token gather for the sampled-query projection, head-split stores for q / k / v (up to three outputs from one packed
+// weight), the reference's flat head reinterpretation, and two implicit operands that are never written to memory:
+// the weighted neighbour block of the standard conv and the shifted rows of the Conv1d branch.  This is the float32
+// path (tensor cores would need a split of every operand to keep the 1e-6 similarity accuracy the top-K parity asks
+// for) and the fallback for bfloat16 shapes the tcgen05 kernels do not cover.
+//
+// Bound by the fp32 pipes.  Each thread accumulates TM x TN outputs, k strictly ascending with one fused
+// multiply-add per term, so a result does not depend on the tile it was computed in.  Two columns share one packed
+// multiply-add instruction; operand tiles are transposed into shared memory ([k][row]) so that a warp (4 x 8 threads)
+// reads one 64-byte and one 128-byte span per k step without conflicts; the next tile's global loads are in flight
+// while the current one is multiplied, one barrier per 16 k.
 #include "common.cuh"
+#include "f32x2.cuh"
+#include "token_weights.cuh"
 
 namespace convnn {
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16;
-
-template <typename T>
-__device__ __forceinline__ const T* a_row_base(const GemmParams& p, int m) {
-    const T* a = static_cast<const T*>(p.a);
-    if (p.a_mode == A_ROWS) return a + (long long)m * p.lda;
-    if (p.a_mode == A_TOKENS) {
-        int b = m / p.rows_per_batch, r = m - b * p.rows_per_batch;
-        int tok = p.cand ? p.cand[r] : r;
-        return a + ((long long)b * p.T + tok) * p.lda;
-    }
-    return a;  // A_HEAD_QUIRK: resolved per element
-}
-
-template <typename T>
-__device__ __forceinline__ float a_load(const GemmParams& p, const T* base, int m, int kk) {
-    if (p.a_mode != A_HEAD_QUIRK) return to_f32<T>(base[kk]);
-    // y[b, t', h*dk + c'] = flat(o[b, h])[c' * T + t']   (reference layers.py:247-259)
-    int b = m / p.T, t = m - b * p.T;
-    int h = kk / p.dk, c = kk - h * p.dk;
-    return to_f32<T>(base[((long long)(b * p.H + h) * p.T) * p.dk + (long long)c * p.T + t]);
-}
+constexpr int BK = 16;
 
 __device__ __forceinline__ float gelu_exact(float x) {
     return 0.5f * x * (1.0f + erff(x * 0.70710678118654752440f));
 }
 
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                       __uint_as_float(v.y & 0xffff0000u));
+}
+__device__ __forceinline__ void store4(float* p, const float (&v)[4]) {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&v)[4]) {
+    __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+}
+// four consecutive values from p (or `n` of them, the rest zero)
 template <typename T>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmParams p) {
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Ws[BK][BN + 4];
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    const int lr = tid >> 2, lk = (tid & 3) * 4;
-    const int am = m0 + lr, wn = n0 + lr;
-    const T* abase = am < p.M ? a_row_base<T>(p, am) : nullptr;
-    const T* wbase = wn < p.N ? static_cast<const T*>(p.w) + (long long)wn * p.Kd : nullptr;
-    const int ty = tid >> 4, tx = tid & 15;
-
-    float acc[4][4];
+__device__ __forceinline__ float4 load_upto4(const T* p, int n, bool vec) {
+    if (vec && n >= 4) return load4(p);
+    float r[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+        if (i < n) r[i] = to_f32<T>(p[i]);
+    return make_float4(r[0], r[1], r[2], r[3]);
+}
 
-    for (int k0 = 0; k0 < p.Kd; k0 += BK) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            int kk = k0 + lk + i;
-            As[lk + i][lr] = (abase && kk < p.Kd) ? a_load<T>(p, abase, am, kk) : 0.f;
-            Ws[lk + i][lr] = (wbase && kk < p.Kd) ? to_f32<T>(wbase[kk]) : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < BK; ++k) {
-            float4 a4 = *reinterpret_cast<const float4*>(&As[k][ty * 4]);
-            float4 b4 = *reinterpret_cast<const float4*>(&Ws[k][tx * 4]);
-            float av[4] = {a4.x, a4.y, a4.z, a4.w};
-            float bv[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-        }
+// One operand row of this thread: where its values for the k range [kk, kk + 4) are.
+template <typename TA>
+struct ARow {
+    const TA* base;       // nullptr: a row past M
+    int m_local;          // row inside the tile (A_NEIGHBOURS)
+    int t;                // token (A_CONV1D)
+};
+
+// Tile BM x BN, NT = (BM / TM) * (BN / TN) threads in warps of 4 (rows) x 8 (columns).
+// TA: type of the A operand (float32 against bfloat16 weights for the separable conv's unrounded intermediate).
+template <typename TA, typename T, int MODE, int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const GemmParams p) {
+    constexpr int NT = (BM / TM) * (BN / TN);
+    constexpr int RG = TM / 4, CG = TN / 4;                 // groups of four rows / columns per thread
+    constexpr int WN = BN / TN / 8;                         // warps side by side along the columns
+    constexpr int LA = BM + 4, LB = BN + 4;
+    constexpr int NA = BM * (BK / 4) / NT, NB = BN * (BK / 4) / NT;     // four-value loads per thread and step
+    __shared__ __align__(16) float As[2][BK][LA];
+    __shared__ __align__(16) float Bs[2][BK][LB];
+    extern __shared__ __align__(16) unsigned char nb_smem[];            // A_NEIGHBOURS: weights, row offsets [BM][K]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    const int ty = (warp / WN) * 4 + (lane >> 3), tx = (warp % WN) * 8 + (lane & 7);
+
+    float* ps = reinterpret_cast<float*>(nb_smem);
+    int* ns = reinterpret_cast<int*>(ps + BM * p.taps);
+    if constexpr (MODE == A_NEIGHBOURS) {
+        const int nm = min(BM, p.M - m0);
+        for (int e = tid; e < nm * p.taps; e += NT) ns[e] = p.nb_idx[(long long)m0 * p.taps + e] * (p.H * p.Cp);
+        for (int r = tid; r < nm; r += NT)
+            token_weights(p.nb_val + (long long)(m0 + r) * p.taps, ps + r * p.taps, p.taps, p.nb_maximum, p.nb_softmax);
         __syncthreads();
     }
 
-    T* c = static_cast<T*>(p.c);
+    // Staging assignment: a warp takes 16 rows x two groups of four k (one full 32-byte sector per row in float32);
+    // the transposed stores of such a set fall into 32 different banks.
+    ARow<TA> ar[NA];
+    int akq[NA], arow[NA];
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+        const int c = (tid + i * NT) >> 5;
+        akq[i] = (lane & 1) + 2 * (c & 1);
+        arow[i] = (lane >> 1) + 16 * (c >> 1);
+        const int m = m0 + arow[i];
+        ar[i].base = nullptr;
+        if (m < p.M) {
+            const TA* a = static_cast<const TA*>(p.a);
+            if (MODE == A_ROWS) {
+                ar[i].base = a + (long long)m * p.lda;
+            } else if (MODE == A_TOKENS) {
+                const int b = m / p.rows_per_batch, r = m - b * p.rows_per_batch;
+                ar[i].base = a + ((long long)b * p.T + (p.cand ? p.cand[r] : r)) * p.lda;
+            } else if (MODE == A_HEAD_QUIRK) {
+                // y[b, t', h*dk + c'] = flat(o[b, h])[c' * T + t']   (reference layers.py:247-259)
+                const int b = m / p.T;
+                ar[i].base = a + (long long)b * p.H * p.T * p.dk + (m - b * p.T);
+            } else {
+                // m = (b, h, t): rows (b, token, h, :) of a (B, T, H, Cp) tensor
+                const int bh = m / p.T, b = bh / p.H, h = bh - b * p.H;
+                ar[i].t = m - bh * p.T;
+                ar[i].base = a + ((long long)b * p.T * p.H + h) * p.Cp;
+            }
+            ar[i].m_local = arow[i];
+        }
+    }
+    const T* wbase[NB];
+    int bkq[NB], brow[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+        const int c = (tid + i * NT) >> 5;
+        bkq[i] = (lane & 1) + 2 * (c & 1);
+        brow[i] = (lane >> 1) + 16 * (c >> 1);
+        const int n = n0 + brow[i];
+        wbase[i] = n < p.N ? static_cast<const T*>(p.w) + (long long)n * p.ldw : nullptr;
+    }
+    const bool avec = p.a_vec, wvec = p.w_vec;
+
+    float4 av[NA], bv[NB];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            const int kk = k0 + akq[i] * 4;
+            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (ar[i].base && kk < p.Kd) {
+                if (MODE == A_ROWS || MODE == A_TOKENS) {
+                    r = load_upto4<TA>(ar[i].base + kk, p.Kd - kk, avec);
+                } else if (MODE == A_HEAD_QUIRK) {
+                    float e[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (kk + j < p.Kd) {
+                            const int h = (kk + j) / p.dk, c = kk + j - h * p.dk;
+                            e[j] = to_f32<TA>(ar[i].base[((long long)h * p.dk + c) * p.T]);
+                        }
+                    r = make_float4(e[0], e[1], e[2], e[3]);
+                } else if (MODE == A_NEIGHBOURS) {
+                    // k = (tap, stored channel): Cp is a multiple of four, so the four values share a tap
+                    const int j = kk / p.Cp, c = kk - j * p.Cp;
+                    const int e = ar[i].m_local * p.taps + j;
+                    const float w = ps[e];
+                    r = load_upto4<TA>(ar[i].base + ns[e] + c, 4, avec);
+                    r.x *= w; r.y *= w; r.z *= w; r.w *= w;
+                } else {                                          // A_CONV1D: k = (tap, channel)
+                    const int j = kk / p.Cp, c = kk - j * p.Cp, tt = ar[i].t + j - p.pad;
+                    if (tt >= 0 && tt < p.T) r = load_upto4<TA>(ar[i].base + (long long)tt * p.H * p.Cp + c, 4, avec);
+                }
+            }
+            av[i] = r;
+        }
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            const int kk = k0 + bkq[i] * 4;
+            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (wbase[i] && kk < p.Kd) {
+                if (MODE == A_NEIGHBOURS && p.C != p.Cp) {        // taps of C values against C + padding stored channels
+                    const int j = kk / p.Cp, c = kk - j * p.Cp;
+                    r = load_upto4<T>(wbase[i] + (long long)j * p.C + c, p.C - c, false);
+                } else {
+                    r = load_upto4<T>(wbase[i] + kk, p.Kd - kk, wvec);
+                }
+            }
+            bv[i] = r;
+        }
+    };
+    auto stage = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            float* d = &As[buf][akq[i] * 4][arow[i]];
+            d[0] = av[i].x; d[LA] = av[i].y; d[2 * LA] = av[i].z; d[3 * LA] = av[i].w;
+        }
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            float* d = &Bs[buf][bkq[i] * 4][brow[i]];
+            d[0] = bv[i].x; d[LB] = bv[i].y; d[2 * LB] = bv[i].z; d[3 * LB] = bv[i].w;
+        }
+    };
+
+    f32x2 acc[TM][TN / 2];
     const T* bias = static_cast<const T*>(p.bias);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        int m = m0 + ty * 4 + i;
-        if (m >= p.M) continue;
+    for (int g = 0; g < CG; ++g)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int n = n0 + tx * 4 + j;
-            if (n >= p.N) continue;
-            float r = acc[i][j];
-            if (bias) r += to_f32<T>(bias[n]);
-            if (p.gelu) r = gelu_exact(r);
-            long long off;
-            if (p.c_mode == C_ROWS) {
-                off = (long long)m * p.ldc + n;
-            } else {
-                int h = n / p.dk, ch = n - h * p.dk;
-                off = (long long)m * p.H * p.Cp + (long long)h * p.Cp + ch;
+        for (int j = 0; j < 2; ++j) {
+            f32x2 init = 0ull;
+            if (p.bias_first && bias) {
+                const int n = n0 + g * (BN / CG) + tx * 4 + 2 * j;
+                init = pack2(n < p.N ? to_f32<T>(bias[n]) : 0.f, n + 1 < p.N ? to_f32<T>(bias[n + 1]) : 0.f);
             }
-            if (p.residual)
-                r = to_f32<T>(from_f32<T>(r)) + to_f32<T>(static_cast<const T*>(p.residual)[(long long)m * p.ldr + n]);
-            c[off] = from_f32<T>(r);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) acc[i][2 * g + j] = init;
         }
+
+    fetch(0);
+    stage(0);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = 0; k0 < p.Kd; k0 += BK, buf ^= 1) {
+        const bool more = k0 + BK < p.Kd;
+        if (more) fetch(k0 + BK);
+#pragma unroll
+        for (int k = 0; k < BK; ++k) {
+            float a[TM];
+            f32x2 b[TN / 2];
+#pragma unroll
+            for (int g = 0; g < RG; ++g) {
+                const float4 v = *reinterpret_cast<const float4*>(&As[buf][k][g * (BM / RG) + ty * 4]);
+                a[4 * g] = v.x; a[4 * g + 1] = v.y; a[4 * g + 2] = v.z; a[4 * g + 3] = v.w;
+            }
+#pragma unroll
+            for (int g = 0; g < CG; ++g) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&Bs[buf][k][g * (BN / CG) + tx * 4]);
+                b[2 * g] = v.x; b[2 * g + 1] = v.y;
+            }
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                const f32x2 aa = pack2(a[i], a[i]);
+#pragma unroll
+                for (int j = 0; j < TN / 2; ++j) acc[i][j] = fma2(aa, b[j], acc[i][j]);
+            }
+        }
+        if (more) {
+            stage(buf ^ 1);
+            __syncthreads();
+        }
+    }
+
+#pragma unroll
+    for (int g = 0; g < CG; ++g) {
+        const int n = n0 + g * (BN / CG) + tx * 4;
+        if (n >= p.N) continue;
+        const int nv = min(4, p.N - n);
+        const int part = n / p.part_cols, pn = n - part * p.part_cols;
+        T* c = static_cast<T*>(part == 0 ? p.c : (part == 1 ? p.c1 : p.c2));
+        int col = pn;
+        if (p.c_mode == C_HEADS) {
+            const int h = pn / p.dk;
+            col = h * p.Cp + (pn - h * p.dk);
+        }
+        const bool vec = p.c_vec && nv == 4;                    // the four columns are neighbours in one output row
+        float bb[4] = {0.f, 0.f, 0.f, 0.f};
+        if (bias && !p.bias_first)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j < nv) bb[j] = to_f32<T>(bias[n + j]);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int m = m0 + (i >> 2) * (BM / RG) + ty * 4 + (i & 3);
+            if (m >= p.M) continue;
+            float r[4];
+            unpack2(acc[i][2 * g], r[0], r[1]);
+            unpack2(acc[i][2 * g + 1], r[2], r[3]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (bias && !p.bias_first) r[j] += bb[j];
+                if (p.gelu) r[j] = gelu_exact(r[j]);
+            }
+            const long long row = p.c_mode == C_HEADS ? (long long)m * p.H * p.Cp : (long long)m * p.ldc;
+            if (vec) {
+                if (p.residual) {
+                    const float4 q = load4(static_cast<const T*>(p.residual) + (long long)m * p.ldr + n);
+                    const float rq[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) r[j] = to_f32<T>(from_f32<T>(r[j])) + rq[j];
+                }
+                store4(c + row + col, r);
+            } else {
+                for (int j = 0; j < nv; ++j) {
+                    float v = r[0];
+#pragma unroll
+                    for (int q = 1; q < 4; ++q)
+                        if (j == q) v = r[q];
+                    int nn = n + j, pp = nn / p.part_cols, cj = nn - pp * p.part_cols;
+                    T* cc = static_cast<T*>(pp == 0 ? p.c : (pp == 1 ? p.c1 : p.c2));
+                    if (p.c_mode == C_HEADS) {
+                        const int h = cj / p.dk;
+                        cj = h * p.Cp + (cj - h * p.dk);
+                    }
+                    if (p.residual)
+                        v = to_f32<T>(from_f32<T>(v)) + to_f32<T>(static_cast<const T*>(p.residual)[(long long)m * p.ldr + nn]);
+                    cc[row + cj] = from_f32<T>(v);
+                }
+            }
+        }
+    }
+}
+
+template <typename TA, typename T, int MODE, int BM, int BN, int TM, int TN>
+int launch_tile(const GemmParams& p, cudaStream_t st) {
+    const dim3 grid((p.M + BM - 1) / BM, (p.N + BN - 1) / BN);
+    const size_t smem = MODE == A_NEIGHBOURS ? (size_t)BM * p.taps * 8 : 0;
+    auto kern = gemm_simt_kernel<TA, T, MODE, BM, BN, TM, TN>;
+    if (smem) CONVNN_ENSURE_SMEM(kern, smem > 36 * 1024 ? smem : 36 * 1024);   // (beside up to 34 KB of static tiles)
+    kern<<<grid, (BM / TM) * (BN / TN), smem, st>>>(p);
+    return CONVNN_OK;
+}
+
+template <typename TA, typename T, int MODE>
+int launch_mode(const GemmParams& p, cudaStream_t st) {
+    // The tile with the least work on the busiest SM: rounds of tiles x outputs per tile, weighted by how well a
+    // tile's threads use the multiply-add pipes once it runs (measured ratios).
+    const long long sms = device_sms();
+    auto cost = [&](int bm, int bn, double eff) {
+        const long long tiles = (long long)((p.M + bm - 1) / bm) * ((p.N + bn - 1) / bn);
+        return (double)((tiles + sms - 1) / sms) * bm * bn / eff;
+    };
+    const double large = cost(128, 128, 1.0), mid = cost(64, 64, 0.8), small = cost(32, 64, 0.6);
+    if (large <= mid && large <= small) return launch_tile<TA, T, MODE, 128, 128, 8, 8>(p, st);
+    if (mid <= small) return launch_tile<TA, T, MODE, 64, 64, 8, 4>(p, st);
+    return launch_tile<TA, T, MODE, 32, 64, 4, 4>(p, st);
+}
+
+template <typename T>
+int launch_typed(const GemmParams& p, cudaStream_t st) {
+    switch (p.a_mode) {
+        case A_ROWS: return launch_mode<T, T, A_ROWS>(p, st);
+        case A_TOKENS: return launch_mode<T, T, A_TOKENS>(p, st);
+        case A_HEAD_QUIRK: return launch_mode<T, T, A_HEAD_QUIRK>(p, st);
+        case A_NEIGHBOURS: return launch_mode<T, T, A_NEIGHBOURS>(p, st);
+        default: return launch_mode<T, T, A_CONV1D>(p, st);
     }
 }
 
 }  // namespace
 
-int launch_gemm_simt(int dtype, const GemmParams& p, cudaStream_t st) {
+int launch_gemm_simt(int dtype, const GemmParams& params, cudaStream_t st) {
+    GemmParams p = params;
     if (p.M <= 0 || p.N <= 0) return CONVNN_OK;
-    dim3 grid((p.M + BM - 1) / BM, (p.N + BN - 1) / BN);
-    if (dtype == CONVNN_F32)
-        gemm_simt_kernel<float><<<grid, 256, 0, st>>>(p);
-    else
-        gemm_simt_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p);
+    const size_t v4 = dtype == CONVNN_F32 ? 16 : 8;
+    auto at4 = [&](const void* q) { return reinterpret_cast<uintptr_t>(q) % v4 == 0; };
+    if (p.part_cols <= 0) p.part_cols = p.N;
+    if (p.ldw <= 0) p.ldw = p.Kd;
+    // four-value accesses: operand rows, weight rows, output rows
+    p.a_vec = (p.a_f32 ? aligned16(p.a) : at4(p.a)) && (p.a_mode == A_NEIGHBOURS || p.a_mode == A_CONV1D ? p.Cp % 4 == 0 : p.lda % 4 == 0);
+    p.w_vec = at4(p.w) && p.ldw % 4 == 0;
+    p.c_vec = at4(p.c) && (!p.c1 || at4(p.c1)) && (!p.c2 || at4(p.c2)) && p.part_cols % 4 == 0 &&
+              (p.c_mode == C_ROWS ? p.ldc % 4 == 0 : (p.dk % 4 == 0 && p.Cp % 4 == 0)) &&
+              (!p.residual || (at4(p.residual) && p.ldr % 4 == 0));
+    if ((p.a_mode == A_NEIGHBOURS || p.a_mode == A_CONV1D) && p.Cp % 4 != 0)
+        return set_error(CONVNN_E_UNSUPPORTED, "gemm_simt: %d channels per head are not a multiple of four", p.Cp);
+    if (p.a_f32 && dtype == CONVNN_BF16 && p.a_mode != A_ROWS)
+        return set_error(CONVNN_E_UNSUPPORTED, "gemm_simt: a float32 operand against bfloat16 weights comes as plain rows");
+    const int rc = p.a_f32 && dtype == CONVNN_BF16 ? launch_mode<float, __nv_bfloat16, A_ROWS>(p, st) : dtype == CONVNN_F32 ? launch_typed<float>(p, st) : launch_typed<__nv_bfloat16>(p, st);
+    if (rc) return rc;
     CONVNN_CHECK_LAUNCH("gemm_simt");
     return CONVNN_OK;
 }

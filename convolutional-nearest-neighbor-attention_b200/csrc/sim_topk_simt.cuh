@@ -1,11 +1,15 @@
 // Similarity + streaming top-K on the FP32 SIMT pipes.
 //
-// One thread owns one key token (a row of the similarity matrix) of one (batch, head);
-// a CTA owns 128 consecutive rows.  Candidate columns are visited in increasing order in
-// tiles of 64; the 128x64 tile of dot products lives in registers (64 accumulators per
-// thread), is turned into a ranking key and is filtered against the thread's sorted
-// list, so the T x S matrix never exists in memory.  Strict comparisons while scanning
-// left to right make the lower candidate column win exact ties.
+// A CTA of 256 threads owns RB (128 or 64) consecutive key tokens (rows of the similarity matrix) of one
+// (batch, head) and visits the candidate columns in tiles of 64.  A tile's dot products are a register-blocked
+// matrix product (RB / 16 x 4 per thread, channels strictly ascending, two columns per packed multiply-add,
+// operands transposed through double-buffered shared memory, the loads of the next channel step in flight); they
+// become ranking keys in a shared-memory tile, which 256 / RB threads per row then scan, each with a sorted register
+// list of its own; the lists of a row are merged at the end under the full (key, column) order.  The T x S matrix
+// never exists in memory, and exact ties go to the lower candidate column.
+//
+// Bound by the fp32 pipes on long sequences (one thread per row with its 64 columns in registers, before, read every
+// operand value of a column from shared memory once per row: 97 us per layer at 32 x 65 tokens x 192 channels).
 //
 // Ranking keys (larger is better) and the values reported for the survivors:
 //   cosine     key = dot * qinv[j]            val = key * kinv[i]
@@ -21,113 +25,202 @@
 #include <math_constants.h>
 
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "toplist.cuh"
 
 namespace convnn {
 namespace simt_topk {
 
-constexpr int ROWS = 128;   // rows (key tokens) per CTA = threads per CTA
-constexpr int COLS = 64;    // candidate columns per register tile
-constexpr int CK = 32;      // channels staged per step
+constexpr int NT = 256;
+constexpr int CB = 64;      // candidate columns per tile
+constexpr int BK = 16;      // channels per step
+constexpr int LK = CB + 4;  // row stride of the key tile: 16-byte rows that fall into different banks
 
-template <typename T, int KCAP>
-__global__ void __launch_bounds__(ROWS) sim_topk_simt_kernel(
+__host__ __device__ constexpr int tile_floats(int rb) { return 2 * BK * (rb + 4) + 2 * BK * (CB + 4) + rb * LK; }
+__host__ __device__ constexpr int merge_floats(int rb, int kcap) { return 2 * kcap * rb * (NT / rb - 1); }
+__host__ __device__ constexpr int smem_bytes(int rb, int kcap) {
+    const int a = tile_floats(rb), b = merge_floats(rb, kcap);
+    return 4 * (a > b ? a : b);
+}
+
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                       __uint_as_float(v.y & 0xffff0000u));
+}
+template <typename T>
+__device__ __forceinline__ float4 load_upto4(const T* p, int n, bool vec) {
+    if (vec && n >= 4) return load4(p);
+    float r[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (i < n) r[i] = to_f32<T>(p[i]);
+    return make_float4(r[0], r[1], r[2], r[3]);
+}
+
+template <typename T, int KCAP, int RB>
+__global__ void __launch_bounds__(NT) sim_topk_simt_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const float* __restrict__ qstat,
     const float* __restrict__ kstat, const int32_t* __restrict__ cand, int32_t* __restrict__ idx,
     float* __restrict__ val, int T_, int S, int H, int Cp, int K, int nsel, int metric, int sampled,
-    float sqrt_dk) {
-    __shared__ float ks[CK][ROWS + 1];
-    __shared__ __align__(16) float qs[COLS][CK + 4];
-    __shared__ float qst[COLS];
-    __shared__ int cnd[COLS];
+    float sqrt_dk, int vec) {
+    constexpr int TM = RB / 16, RG = TM / 4;              // 16 x 16 threads, TM x 4 dot products each
+    constexpr int LA = RB + 4, LB = CB + 4;
+    constexpr int NA = RB * (BK / 4) / NT, TPR = NT / RB; // loads per thread and step; scanning threads per row
+    constexpr int CW = CB / TPR;                          // columns of a tile per scanning thread
+    extern __shared__ __align__(16) float sm[];
+    float* As = sm;                                       // [2][BK][LA]
+    float* Bs = As + 2 * BK * LA;                         // [2][BK][LB]
+    float* keys = Bs + 2 * BK * LB;                       // [RB][LK]
 
-    const int tid = threadIdx.x;
-    const int bh = blockIdx.y;
-    const int b = bh / H, h = bh - b * H;
-    const int row0 = blockIdx.x * ROWS;
-    const int row = row0 + tid;
-    const bool row_ok = row < T_;
-
-    const T* kb = k + ((long long)b * T_ * H + h) * Cp;   // + token * H*Cp + c
-    const T* qb = q + ((long long)b * S * H + h) * Cp;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int bh = blockIdx.y, b = bh / H, h = bh - b * H;
+    const int row0 = blockIdx.x * RB;
+    const int ty = (warp >> 1) * 4 + (lane >> 3), tx = (warp & 1) * 8 + (lane & 7);
     const long long tstride = (long long)H * Cp;
+    const T* kb = k + ((long long)b * T_ * H + h) * Cp;   // + token * tstride + c
+    const T* qb = q + ((long long)b * S * H + h) * Cp;
 
-    float kst = 0.f;
-    if (row_ok && metric != CONVNN_MATMUL) kst = kstat[((long long)b * H + h) * T_ + row];
-    float sentinel = -CUDART_INF_F;
-    if (sampled) {
-        if (metric == CONVNN_COSINE) sentinel = -0.1f / kst;
-        else if (metric == CONVNN_MATMUL) sentinel = -0.1f * sqrt_dk;
-        else sentinel = kst - 1.21f;
+    // staging: a warp takes 16 rows x two groups of four channels (conflict-free transposed stores)
+    const T* abase[NA];
+    int akq[NA], arow[NA];
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+        const int c = (tid + i * NT) >> 5;
+        akq[i] = (lane & 1) + 2 * (c & 1);
+        arow[i] = (lane >> 1) + 16 * (c >> 1);
+        abase[i] = row0 + arow[i] < T_ ? kb + (row0 + arow[i]) * tstride : nullptr;
     }
+    const int bkq = (lane & 1) + 2 * (warp & 1), brow = (lane >> 1) + 16 * (warp >> 1);
 
+    // this thread's row and column share when scanning
+    const int srow = tid % RB, sq = tid / RB;
+    const int row = row0 + srow;
+    const bool row_ok = row < T_;
+    const float* kst_row = metric != CONVNN_MATMUL ? kstat + ((long long)b * H + h) * T_ : nullptr;
+    const float* qst_row = metric != CONVNN_MATMUL ? qstat + ((long long)b * H + h) * S : nullptr;
     TopList<KCAP> top;
     top.init();
 
-    const int lc = tid & 31, lr = tid >> 5;   // staging: channel lc, rows / columns lr + 4*i
-
-    for (int c0 = 0; c0 < S; c0 += COLS) {
-        float acc[COLS];
+    const int ksteps = (Cp + BK - 1) / BK, ntiles = (S + CB - 1) / CB;
+    float4 av[NA], bv;
+    auto fetch = [&](int ct, int ks) {
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
-
-        if (tid < COLS) {
-            int col = c0 + tid;
-            qst[tid] = (col < S && metric != CONVNN_MATMUL) ? qstat[((long long)b * H + h) * S + col] : 0.f;
-            cnd[tid] = (sampled && col < S) ? cand[col] : -1;
+        for (int i = 0; i < NA; ++i) {
+            const int c = ks * BK + akq[i] * 4;
+            av[i] = abase[i] && c < Cp ? load_upto4<T>(abase[i] + c, Cp - c, vec) : z;
         }
+        const int c = ks * BK + bkq * 4, col = ct * CB + brow;
+        bv = col < S && c < Cp ? load_upto4<T>(qb + col * tstride + c, Cp - c, vec) : z;
+    };
+    auto stage = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            float* d = As + (buf * BK + akq[i] * 4) * LA + arow[i];
+            d[0] = av[i].x; d[LA] = av[i].y; d[2 * LA] = av[i].z; d[3 * LA] = av[i].w;
+        }
+        float* d = Bs + (buf * BK + bkq * 4) * LB + brow;
+        d[0] = bv.x; d[LB] = bv.y; d[2 * LB] = bv.z; d[3 * LB] = bv.w;
+    };
 
-        for (int ch0 = 0; ch0 < Cp; ch0 += CK) {
-            __syncthreads();   // previous chunk fully consumed
-            const bool ch_ok = ch0 + lc < Cp;
-#pragma unroll 4
-            for (int i = 0; i < ROWS / 4; ++i) {
-                int r = lr + 4 * i;
-                int tok = row0 + r;
-                ks[lc][r] = (ch_ok && tok < T_) ? to_f32<T>(kb[tok * tstride + ch0 + lc]) : 0.f;
-            }
-#pragma unroll 4
-            for (int i = 0; i < COLS / 4; ++i) {
-                int j = lr + 4 * i;
-                int col = c0 + j;
-                qs[j][lc] = (ch_ok && col < S) ? to_f32<T>(qb[col * tstride + ch0 + lc]) : 0.f;
-            }
-            __syncthreads();
+    fetch(0, 0);
+    stage(0);
+    __syncthreads();
+    int buf = 0;
+    for (int ct = 0; ct < ntiles; ++ct) {
+        f32x2 acc[TM][2];
 #pragma unroll
-            for (int c4 = 0; c4 < CK; c4 += 4) {
-                const float k0 = ks[c4 + 0][tid], k1 = ks[c4 + 1][tid];
-                const float k2 = ks[c4 + 2][tid], k3 = ks[c4 + 3][tid];
+        for (int i = 0; i < TM; ++i) acc[i][0] = acc[i][1] = 0ull;
+        for (int ks = 0; ks < ksteps; ++ks, buf ^= 1) {
+            const bool last = ks + 1 == ksteps, more = !last || ct + 1 < ntiles;
+            if (more) fetch(last ? ct + 1 : ct, last ? 0 : ks + 1);
 #pragma unroll
-                for (int j = 0; j < COLS; ++j) {
-                    const float4 q4 = *reinterpret_cast<const float4*>(&qs[j][c4]);
-                    float a = acc[j];
-                    a = fmaf(k0, q4.x, a);
-                    a = fmaf(k1, q4.y, a);
-                    a = fmaf(k2, q4.z, a);
-                    a = fmaf(k3, q4.w, a);
-                    acc[j] = a;
+            for (int kk = 0; kk < BK; ++kk) {
+                float a[TM];
+#pragma unroll
+                for (int g = 0; g < RG; ++g) {
+                    const float4 v = *reinterpret_cast<const float4*>(As + (buf * BK + kk) * LA + g * (RB / RG) + ty * 4);
+                    a[4 * g] = v.x; a[4 * g + 1] = v.y; a[4 * g + 2] = v.z; a[4 * g + 3] = v.w;
+                }
+                const ulonglong2 bb = *reinterpret_cast<const ulonglong2*>(Bs + (buf * BK + kk) * LB + tx * 4);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    const f32x2 aa = pack2(a[i], a[i]);
+                    acc[i][0] = fma2(aa, bb.x, acc[i][0]);
+                    acc[i][1] = fma2(aa, bb.y, acc[i][1]);
                 }
             }
-        }
-
-        if (row_ok) {
+            if (last) {
+                // keys of this tile (the previous tile's were scanned before the last barrier)
+                const int c0 = ct * CB + tx * 4;
+                float st[4];
+                int cd[4];
 #pragma unroll
-            for (int j = 0; j < COLS; ++j) {
-                const int col = c0 + j;
-                if (col < S) {
-                    float key;
-                    if (metric == CONVNN_COSINE) key = acc[j] * qst[j];
-                    else if (metric == CONVNN_MATMUL) key = acc[j];
-                    else key = fmaf(2.0f, acc[j], -qst[j]);
-                    if (sampled && cnd[j] == row) key = sentinel;
-                    if (key > top.worst()) top.insert(key, col);
+                for (int j = 0; j < 4; ++j) {
+                    const int col = min(c0 + j, S - 1);
+                    st[j] = qst_row ? qst_row[col] : 0.f;
+                    cd[j] = sampled ? cand[col] : -1;
+                }
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    const int r = (i >> 2) * (RB / RG) + ty * 4 + (i & 3);
+                    float d[4];
+                    unpack2(acc[i][0], d[0], d[1]);
+                    unpack2(acc[i][1], d[2], d[3]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (metric == CONVNN_COSINE) d[j] *= st[j];
+                        else if (metric == CONVNN_EUCLIDEAN) d[j] = fmaf(2.0f, d[j], -st[j]);
+                        if (sampled && cd[j] == row0 + r) {
+                            const float ks_ = kst_row ? kst_row[row0 + r] : 0.f;
+                            if (metric == CONVNN_COSINE) d[j] = -0.1f / ks_;
+                            else if (metric == CONVNN_MATMUL) d[j] = -0.1f * sqrt_dk;
+                            else d[j] = ks_ - 1.21f;
+                        }
+                    }
+                    *reinterpret_cast<float4*>(keys + r * LK + tx * 4) = make_float4(d[0], d[1], d[2], d[3]);
+                }
+                __syncthreads();
+                const int s0 = ct * CB + sq * CW;
+                if (row_ok) {
+#pragma unroll 4
+                    for (int j4 = 0; j4 < CW; j4 += 4) {
+                        const float4 v = *reinterpret_cast<const float4*>(keys + srow * LK + sq * CW + j4);
+                        const float kv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            if (s0 + j4 + j < S && kv[j] > top.worst()) top.insert_sorted(kv[j], s0 + j4 + j);
+                    }
                 }
             }
+            if (more) {
+                stage(buf ^ 1);
+                __syncthreads();
+            }
         }
-        __syncthreads();   // qst / cnd are rewritten by the next tile
     }
 
-    if (!row_ok) return;
+    // merge the lists of a row: lists 1 .. TPR - 1 through shared memory into list 0
+    __syncthreads();
+    float* mk = sm;                                       // [TPR - 1][KCAP][RB]
+    int* mc = reinterpret_cast<int*>(sm + (TPR - 1) * KCAP * RB);
+    if (sq > 0) {
+#pragma unroll
+        for (int s = 0; s < KCAP; ++s) {
+            mk[((sq - 1) * KCAP + s) * RB + srow] = top.v[s];
+            mc[((sq - 1) * KCAP + s) * RB + srow] = top.i[s];
+        }
+    }
+    __syncthreads();
+    if (sq > 0 || !row_ok) return;
+    for (int l = 0; l < (TPR - 1) * KCAP; ++l) {
+        const float key = mk[l * RB + srow];
+        if (key >= top.worst() && key > -CUDART_INF_F) top.insert_ordered(key, mc[l * RB + srow]);
+    }
+
+    const float kst = kst_row ? kst_row[row] : 0.f;
     const long long obase = (((long long)b * H + h) * T_ + row) * K;
     int off = 0;
     if (sampled) {
@@ -155,23 +248,37 @@ __global__ void __launch_bounds__(ROWS) sim_topk_simt_kernel(
     }
 }
 
+template <typename T, int KCAP, int RB>
+int launch(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
+           const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st) {
+    const size_t smem = smem_bytes(RB, KCAP);
+    auto kern = sim_topk_simt_kernel<T, KCAP, RB>;
+    CONVNN_ENSURE_SMEM(kern, smem);
+    const int vec = dm.Cp % 4 == 0 && aligned16(q) && aligned16(k);
+    kern<<<dim3((dm.T + RB - 1) / RB, dm.B * dm.H), NT, smem, st>>>(
+        static_cast<const T*>(q), static_cast<const T*>(k), qstat, kstat, cand, idx, val, dm.T, dm.S, dm.H, dm.Cp, dm.K,
+        dm.nsel, d->metric, d->sampled, (float)sqrt((double)dm.dk), vec);
+    CONVNN_CHECK_LAUNCH("sim_topk_simt");
+    return CONVNN_OK;
+}
+
 template <typename T>
 int dispatch(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
              const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st) {
-    dim3 grid((dm.T + ROWS - 1) / ROWS, dm.B * dm.H);
-    const float sq = (float)sqrt((double)dm.dk);
-#define CONVNN_LAUNCH(KC)                                                                           \
-    sim_topk_simt_kernel<T, KC><<<grid, ROWS, 0, st>>>(static_cast<const T*>(q), static_cast<const T*>(k), \
-        qstat, kstat, cand, idx, val, dm.T, dm.S, dm.H, dm.Cp, dm.K, dm.nsel, d->metric, d->sampled, sq)
+    // 128 rows per CTA use the pipes better (8 x 4 dot products per thread instead of 4 x 4); 64 where the 128-row grid
+    // leaves SMs without work or most of a tile is padding.
+    const long long wide = (long long)((dm.T + 127) / 128) * dm.B * dm.H;
+    const bool rows128 = wide >= device_sms() && ((dm.T + 127) / 128) * 128 <= ((dm.T + 63) / 64) * 64 * 5 / 4;
+#define CONVNN_LAUNCH(KC)                                                                                     \
+    return rows128 ? launch<T, KC, 128>(d, dm, q, k, qstat, kstat, cand, idx, val, st)                        \
+                   : launch<T, KC, 64>(d, dm, q, k, qstat, kstat, cand, idx, val, st)
     const int n = dm.nsel;
     if (n <= 4) CONVNN_LAUNCH(4);
-    else if (n <= 8) CONVNN_LAUNCH(8);
-    else if (n <= 12) CONVNN_LAUNCH(12);
-    else if (n <= 16) CONVNN_LAUNCH(16);
-    else CONVNN_LAUNCH(32);
+    if (n <= 9) CONVNN_LAUNCH(9);
+    if (n <= 16) CONVNN_LAUNCH(16);
+    if (n <= 25) CONVNN_LAUNCH(25);
+    CONVNN_LAUNCH(32);
 #undef CONVNN_LAUNCH
-    CONVNN_CHECK_LAUNCH("sim_topk_simt");
-    return CONVNN_OK;
 }
 
 }  // namespace simt_topk

@@ -1,0 +1,132 @@
+"""The fp32-pipe kernels at the edges of their tiles: plain, three-output, neighbour and Conv1d operands of the SIMT
+GEMM, and the register-blocked similarity / top-K kernel."""
+import pytest
+import torch
+
+from convnn_b200 import ops
+from gpu_util import DEV
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -24
+
+
+def _bound(a, w, terms):
+    """|computed - exact| of a sum of `terms` fp32 products in any order: terms * eps * sum |a||w| (first order)."""
+    return (terms + 2) * EPS * (a.double().abs() @ w.double().abs().T) + 1e-30
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (31, 33, 15), (32, 64, 16), (65, 63, 17), (128, 128, 32), (129, 257, 100),
+                                   (3000, 192, 192), (4097, 130, 36), (20000, 768, 20)])
+def test_linear_float32(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(M * 7 + N)
+    a = torch.randn(M, K, device=DEV, generator=g)
+    w = torch.randn(N, K, device=DEV, generator=g)
+    b = torch.randn(N, device=DEV, generator=g)
+    r = torch.randn(M, N, device=DEV, generator=g)
+    got = ops.linear(a, w, b, residual=r)
+    want = a.double() @ w.double().T + b.double() + r.double()
+    err = (got.double() - want).abs()
+    assert bool((err <= _bound(a, w, K) + 4 * EPS * (b.abs() + r.abs() + want.abs())).all())
+
+
+@pytest.mark.parametrize("H,dk,T,coord", [(1, 20, 70, True), (3, 12, 197, False), (1, 193, 130, True), (1, 132, 257, False)])
+@pytest.mark.parametrize("conv", ["standard", "depthwise-separable"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_matrix_convs_against_float64(H, dk, T, coord, conv, dtype):
+    if conv == "standard" and dk % 4:
+        pytest.skip("head widths that are no multiple of four take another kernel")
+    B, K = 2, 5
+    g = torch.Generator(device=DEV).manual_seed(dk + T)
+    spec = ops.LayerSpec(H * dk, H, K, "all", "cosine", conv, True, coord, T)
+    C = dk + int(coord)
+    Cp = (C + 7) // 8 * 8 if coord else dk
+    v = torch.zeros(B, T, H, Cp, device=DEV)
+    v[..., :C] = torch.randn(B, T, H, C, device=DEV, generator=g)
+    v = v.to(dtype)
+    idx = torch.randint(0, T, (B, H, T, K), device=DEV, generator=g, dtype=torch.int32)
+    val = torch.randn(B, H, T, K, device=DEV, generator=g)
+    p = torch.softmax(val.double(), -1)
+    rows = v.double().permute(0, 2, 1, 3)[..., :C]                        # (B, H, T, C)
+    nb = torch.gather(rows.unsqueeze(3).expand(B, H, T, K, C), 2, idx.long().unsqueeze(-1).expand(B, H, T, K, C))
+    nb = nb * p.unsqueeze(-1)
+    if conv == "standard":
+        w = (torch.randn(dk, K, C, device=DEV, generator=g) / (K * C) ** 0.5).to(dtype)
+        got = ops.gather_conv(spec, v, idx, val, w)
+        want = torch.einsum("bhtjc,ojc->bhto", nb, w.double())
+        mass = torch.einsum("bhtjc,ojc->bhto", nb.abs(), w.double().abs())
+        terms = K * C
+    else:
+        w = torch.randn(K, C, device=DEV, generator=g).to(dtype)
+        pw = (torch.randn(dk, C, device=DEV, generator=g) / C ** 0.5).to(dtype)
+        got = ops.gather_conv(spec, v, idx, val, w, pw)
+        mid = torch.einsum("bhtjc,jc->bhtc", nb, w.double())
+        want = torch.einsum("bhtc,oc->bhto", mid, pw.double())
+        mass = torch.einsum("bhtc,oc->bhto", torch.einsum("bhtjc,jc->bhtc", nb.abs(), w.double().abs()), pw.double().abs())
+        terms = K + C
+    # fp32 sums (and softmax weights within a few eps) plus, in bfloat16, one rounding of the result; without the
+    # coordinate channel the tensor-core route also rounds its operand once
+    rel = (terms + 16) * EPS + (0 if dtype == torch.float32 else 2.0 ** -9 * (1 if coord else 2))
+    assert bool(((got.double() - want).abs() <= rel * mass + (0 if dtype == torch.float32 else 2.0 ** -8) * want.abs() + 1e-30).all())
+
+
+@pytest.mark.parametrize("ks", [1, 4, 9])
+@pytest.mark.parametrize("T,dk", [(3, 4), (65, 12), (130, 36)])
+def test_conv1d_branch_float32(T, dk, ks):
+    g = torch.Generator(device=DEV).manual_seed(T)
+    B, H, D = 2, 2, 2 * dk
+    eye, zero = torch.eye(D, device=DEV), torch.zeros(D, device=DEV)
+    x = torch.randn(B, T, D, device=DEV, generator=g)
+    w = torch.randn(dk, ks, dk, device=DEV, generator=g)
+    b = torch.randn(dk, device=DEV, generator=g)
+    got = ops.conv1d_attention(x, eye, zero, w, b, eye, zero, H, ks)
+    y = x.double().view(B, T, H, dk).permute(0, 2, 3, 1).reshape(B * H, dk, T)
+    left = (ks - 1) // 2
+    z = torch.nn.functional.conv1d(torch.nn.functional.pad(y, (left, ks - 1 - left)), w.double().permute(0, 2, 1), b.double())
+    flat = z.permute(0, 2, 1).reshape(B, H, T * dk)                       # (t, c) rows read back as (c, t)
+    want = flat.view(B, H, dk, T).permute(0, 3, 1, 2).reshape(B, T, D)
+    scale = float(w.abs().sum(dim=(1, 2)).max()) * float(x.abs().max()) + float(b.abs().max())
+    assert float((got.double() - want).abs().max()) <= (ks * dk + D + 4) * EPS * scale
+
+
+@pytest.mark.parametrize("T,S,C,K", [(1, 1, 4, 1), (63, 64, 20, 9), (65, 65, 16, 25), (129, 200, 33, 32), (257, 63, 48, 4),
+                                     (300, 300, 8, 16), (2500, 65, 36, 9)])
+@pytest.mark.parametrize("metric", ["cosine", "matmul", "euclidean"])
+def test_similarity_lists_float32(T, S, C, K, metric):
+    g = torch.Generator(device=DEV).manual_seed(T + S)
+    B = 2 if T < 2000 else 8
+    spec = ops.LayerSpec(C, 1, K, "random", metric, "depthwise", True, False, T) if S != T else \
+        ops.LayerSpec(C, 1, K, "all", metric, "depthwise", True, False, T)
+    cand = torch.randint(0, T, (S,), device=DEV, generator=g, dtype=torch.int32) if S != T else None
+    q = torch.randn(B, S, 1, C, device=DEV, generator=g)
+    k = torch.randn(B, T, 1, C, device=DEV, generator=g)
+    q[:, S // 2] = q[:, 0]                                                # an exact tie: the lower column goes first
+    qs, ks = q.double().square().sum(-1).view(B, 1, S), k.double().square().sum(-1).view(B, 1, T)
+    if metric == "cosine":
+        qs, ks = 1 / qs.sqrt(), 1 / ks.sqrt()
+    idx, val = ops.sim_topk(spec, q, k, qs.float(), ks.float(), cand)
+    sim = torch.einsum("btc,bsc->bts", k[:, :, 0].double(), q[:, :, 0].double())
+    if metric == "cosine":
+        sim = sim * ks.view(B, T, 1) * qs.view(B, 1, S)
+    elif metric == "matmul":
+        sim = sim / C ** 0.5
+    else:
+        sim = -(ks.view(B, T, 1) + qs.view(B, 1, S) - 2 * sim).clamp_min(0).sqrt()
+    if cand is not None:
+        own = cand.view(1, 1, S).long() == torch.arange(T, device=DEV).view(1, T, 1)
+        sim = sim.masked_fill(own, -1.1 if metric == "euclidean" else -0.1)
+    n = K if cand is None else K - 1
+    got = idx[:, 0, :, K - n:].long()
+    if n == 0:
+        return
+    want = sim.topk(n, -1).values
+    chosen = val[:, 0, :, K - n:].double() * (-1 if metric == "euclidean" else 1)
+    # every reported value is the n-th best one up to the rounding of a C-term dot product (euclidean: a root of a
+    # difference, absolute 1e-3 at distances near zero)
+    tol = 1e-3 if metric == "euclidean" else (C + 8) * EPS * 64
+    assert float((chosen - want).abs().max()) <= tol
+    if cand is None:
+        assert all(len(set(r.tolist())) == n for r in got.view(-1, n)[:200])
+        first = (got == 0).int().argmax(-1)
+        tied = (got == S // 2).int().argmax(-1)
+        both = (got == 0).any(-1) & (got == S // 2).any(-1)
+        assert S < 2 or bool((first[both] < tied[both]).all())
