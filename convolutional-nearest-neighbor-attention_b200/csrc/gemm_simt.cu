@@ -5,11 +5,11 @@
 // path (tensor cores would need a split of every operand to keep the 1e-6 similarity accuracy the top-K parity asks
 // for) and the fallback for bfloat16 shapes the tcgen05 kernels do not cover.
 //
-// Bound by the fp32 pipes.  Each thread accumulates TM x TN outputs, k strictly ascending with one fused
+// Bound by the fp32 pipes and the shared-memory reads that feed them.  Each thread accumulates TM x TN outputs, k strictly ascending with one fused
 // multiply-add per term, so a result does not depend on the tile it was computed in.  Two columns share one packed
 // multiply-add instruction; operand tiles are transposed into shared memory ([k][row]) so that a warp (4 x 8 threads)
 // reads one 64-byte and one 128-byte span per k step without conflicts; the next tile's global loads are in flight
-// while the current one is multiplied, one barrier per 16 k.
+// while the current one is multiplied.
 #include "common.cuh"
 #include "f32x2.cuh"
 #include "token_weights.cuh"
@@ -17,8 +17,6 @@
 namespace convnn {
 
 namespace {
-
-constexpr int BK = 16;
 
 __device__ __forceinline__ float gelu_exact(float x) {
     return 0.5f * x * (1.0f + erff(x * 0.70710678118654752440f));
@@ -58,21 +56,22 @@ struct ARow {
 
 // Tile BM x BN, NT = (BM / TM) * (BN / TN) threads in warps of 4 (rows) x 8 (columns).
 // TA: type of the A operand (float32 against bfloat16 weights for the separable conv's unrounded intermediate).
-template <typename TA, typename T, int MODE, int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const GemmParams p) {
+template <typename TA, typename T, int MODE, int BM, int BN, int BK, int TM, int TN, int MINB>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_kernel(const GemmParams p) {
     constexpr int NT = (BM / TM) * (BN / TN);
-    constexpr int RG = TM / 4, CG = TN / 4;                 // groups of four rows / columns per thread
+    constexpr int VM = TM < 4 ? TM : 4, VN = TN < 4 ? TN : 4;   // rows / columns read with one instruction
+    constexpr int RG = TM / VM, CG = TN / VN;               // groups of them per thread
     constexpr int WN = BN / TN / 8;                         // warps side by side along the columns
     constexpr int LA = BM + 4, LB = BN + 4;
     constexpr int NA = BM * (BK / 4) / NT, NB = BN * (BK / 4) / NT;     // four-value loads per thread and step
-    __shared__ __align__(16) float As[2][BK][LA];
-    __shared__ __align__(16) float Bs[2][BK][LB];
-    extern __shared__ __align__(16) unsigned char nb_smem[];            // A_NEIGHBOURS: weights, row offsets [BM][K]
+    extern __shared__ __align__(16) float gs[];
+    float* As = gs;                                         // [2][BK][LA]
+    float* Bs = As + 2 * BK * LA;                           // [2][BK][LB]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
     const int ty = (warp / WN) * 4 + (lane >> 3), tx = (warp % WN) * 8 + (lane & 7);
 
-    float* ps = reinterpret_cast<float*>(nb_smem);
+    float* ps = Bs + 2 * BK * LB;                           // A_NEIGHBOURS: weights, row offsets [BM][taps]
     int* ns = reinterpret_cast<int*>(ps + BM * p.taps);
     if constexpr (MODE == A_NEIGHBOURS) {
         const int nm = min(BM, p.M - m0);
@@ -89,8 +88,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
 #pragma unroll
     for (int i = 0; i < NA; ++i) {
         const int c = (tid + i * NT) >> 5;
-        akq[i] = (lane & 1) + 2 * (c & 1);
-        arow[i] = (lane >> 1) + 16 * (c >> 1);
+        akq[i] = (lane & 1) + 2 * (c % (BK / 8));
+        arow[i] = (lane >> 1) + 16 * (c / (BK / 8));
         const int m = m0 + arow[i];
         ar[i].base = nullptr;
         if (m < p.M) {
@@ -118,8 +117,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
         const int c = (tid + i * NT) >> 5;
-        bkq[i] = (lane & 1) + 2 * (c & 1);
-        brow[i] = (lane >> 1) + 16 * (c >> 1);
+        bkq[i] = (lane & 1) + 2 * (c % (BK / 8));
+        brow[i] = (lane >> 1) + 16 * (c / (BK / 8));
         const int n = n0 + brow[i];
         wbase[i] = n < p.N ? static_cast<const T*>(p.w) + (long long)n * p.ldw : nullptr;
     }
@@ -175,12 +174,12 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
     auto stage = [&](int buf) {
 #pragma unroll
         for (int i = 0; i < NA; ++i) {
-            float* d = &As[buf][akq[i] * 4][arow[i]];
+            float* d = As + (buf * BK + akq[i] * 4) * LA + arow[i];
             d[0] = av[i].x; d[LA] = av[i].y; d[2 * LA] = av[i].z; d[3 * LA] = av[i].w;
         }
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
-            float* d = &Bs[buf][bkq[i] * 4][brow[i]];
+            float* d = Bs + (buf * BK + bkq[i] * 4) * LB + brow[i];
             d[0] = bv[i].x; d[LB] = bv[i].y; d[2 * LB] = bv[i].z; d[3 * LB] = bv[i].w;
         }
     };
@@ -188,17 +187,15 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
     f32x2 acc[TM][TN / 2];
     const T* bias = static_cast<const T*>(p.bias);
 #pragma unroll
-    for (int g = 0; g < CG; ++g)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            f32x2 init = 0ull;
-            if (p.bias_first && bias) {
-                const int n = n0 + g * (BN / CG) + tx * 4 + 2 * j;
-                init = pack2(n < p.N ? to_f32<T>(bias[n]) : 0.f, n + 1 < p.N ? to_f32<T>(bias[n + 1]) : 0.f);
-            }
-#pragma unroll
-            for (int i = 0; i < TM; ++i) acc[i][2 * g + j] = init;
+    for (int j = 0; j < TN / 2; ++j) {
+        f32x2 init = 0ull;
+        if (p.bias_first && bias) {
+            const int n = n0 + (2 * j / VN) * (BN / CG) + tx * VN + 2 * j % VN;
+            init = pack2(n < p.N ? to_f32<T>(bias[n]) : 0.f, n + 1 < p.N ? to_f32<T>(bias[n + 1]) : 0.f);
         }
+#pragma unroll
+        for (int i = 0; i < TM; ++i) acc[i][j] = init;
+    }
 
     fetch(0);
     stage(0);
@@ -213,13 +210,24 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
             f32x2 b[TN / 2];
 #pragma unroll
             for (int g = 0; g < RG; ++g) {
-                const float4 v = *reinterpret_cast<const float4*>(&As[buf][k][g * (BM / RG) + ty * 4]);
-                a[4 * g] = v.x; a[4 * g + 1] = v.y; a[4 * g + 2] = v.z; a[4 * g + 3] = v.w;
+                const float* src = As + (buf * BK + k) * LA + g * (BM / RG) + ty * VM;
+                if (VM == 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(src);
+                    a[4 * g] = v.x; a[4 * g + 1] = v.y; a[(4 * g + 2) % TM] = v.z; a[(4 * g + 3) % TM] = v.w;
+                } else {
+                    const float2 v = *reinterpret_cast<const float2*>(src);
+                    a[2 * g] = v.x; a[2 * g + 1] = v.y;
+                }
             }
 #pragma unroll
             for (int g = 0; g < CG; ++g) {
-                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&Bs[buf][k][g * (BN / CG) + tx * 4]);
-                b[2 * g] = v.x; b[2 * g + 1] = v.y;
+                const float* src = Bs + (buf * BK + k) * LB + g * (BN / CG) + tx * VN;
+                if (VN == 4) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(src);
+                    b[2 * g] = v.x; b[(2 * g + 1) % (TN / 2)] = v.y;
+                } else {
+                    b[g] = *reinterpret_cast<const f32x2*>(src);
+                }
             }
 #pragma unroll
             for (int i = 0; i < TM; ++i) {
@@ -236,9 +244,9 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
 
 #pragma unroll
     for (int g = 0; g < CG; ++g) {
-        const int n = n0 + g * (BN / CG) + tx * 4;
+        const int n = n0 + g * (BN / CG) + tx * VN;
         if (n >= p.N) continue;
-        const int nv = min(4, p.N - n);
+        const int nv = min(VN, p.N - n);
         const int part = n / p.part_cols, pn = n - part * p.part_cols;
         T* c = static_cast<T*>(part == 0 ? p.c : (part == 1 ? p.c1 : p.c2));
         int col = pn;
@@ -246,77 +254,85 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
             const int h = pn / p.dk;
             col = h * p.Cp + (pn - h * p.dk);
         }
-        const bool vec = p.c_vec && nv == 4;                    // the four columns are neighbours in one output row
-        float bb[4] = {0.f, 0.f, 0.f, 0.f};
+        const bool vec = VN == 4 && p.c_vec && nv == 4;         // the four columns are neighbours in one output row
+        float bb[VN] = {};
         if (bias && !p.bias_first)
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int j = 0; j < VN; ++j)
                 if (j < nv) bb[j] = to_f32<T>(bias[n + j]);
 #pragma unroll
         for (int i = 0; i < TM; ++i) {
-            const int m = m0 + (i >> 2) * (BM / RG) + ty * 4 + (i & 3);
+            const int m = m0 + (i / VM) * (BM / RG) + ty * VM + i % VM;
             if (m >= p.M) continue;
-            float r[4];
-            unpack2(acc[i][2 * g], r[0], r[1]);
-            unpack2(acc[i][2 * g + 1], r[2], r[3]);
+            float r[VN];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < VN / 2; ++j) unpack2(acc[i][g * (VN / 2) + j], r[2 * j], r[2 * j + 1]);
+#pragma unroll
+            for (int j = 0; j < VN; ++j) {
                 if (bias && !p.bias_first) r[j] += bb[j];
                 if (p.gelu) r[j] = gelu_exact(r[j]);
             }
             const long long row = p.c_mode == C_HEADS ? (long long)m * p.H * p.Cp : (long long)m * p.ldc;
-            if (vec) {
-                if (p.residual) {
-                    const float4 q = load4(static_cast<const T*>(p.residual) + (long long)m * p.ldr + n);
-                    const float rq[4] = {q.x, q.y, q.z, q.w};
+            if constexpr (VN == 4) {
+                if (vec) {
+                    if (p.residual) {
+                        const float4 q = load4(static_cast<const T*>(p.residual) + (long long)m * p.ldr + n);
+                        const float rq[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) r[j] = to_f32<T>(from_f32<T>(r[j])) + rq[j];
-                }
-                store4(c + row + col, r);
-            } else {
-                for (int j = 0; j < nv; ++j) {
-                    float v = r[0];
-#pragma unroll
-                    for (int q = 1; q < 4; ++q)
-                        if (j == q) v = r[q];
-                    int nn = n + j, pp = nn / p.part_cols, cj = nn - pp * p.part_cols;
-                    T* cc = static_cast<T*>(pp == 0 ? p.c : (pp == 1 ? p.c1 : p.c2));
-                    if (p.c_mode == C_HEADS) {
-                        const int h = cj / p.dk;
-                        cj = h * p.Cp + (cj - h * p.dk);
+                        for (int j = 0; j < 4; ++j) r[j] = to_f32<T>(from_f32<T>(r[j])) + rq[j];
                     }
-                    if (p.residual)
-                        v = to_f32<T>(from_f32<T>(v)) + to_f32<T>(static_cast<const T*>(p.residual)[(long long)m * p.ldr + nn]);
-                    cc[row + cj] = from_f32<T>(v);
+                    store4(c + row + col, r);
+                    continue;
                 }
+            }
+#pragma unroll
+            for (int j = 0; j < VN; ++j) {
+                if (j >= nv) continue;
+                float v = r[j];
+                const int nn = n + j, pp = nn / p.part_cols;
+                int cj = nn - pp * p.part_cols;
+                T* cc = static_cast<T*>(pp == 0 ? p.c : (pp == 1 ? p.c1 : p.c2));
+                if (p.c_mode == C_HEADS) {
+                    const int h = cj / p.dk;
+                    cj = h * p.Cp + (cj - h * p.dk);
+                }
+                if (p.residual)
+                    v = to_f32<T>(from_f32<T>(v)) + to_f32<T>(static_cast<const T*>(p.residual)[(long long)m * p.ldr + nn]);
+                cc[row + cj] = from_f32<T>(v);
             }
         }
     }
 }
 
-template <typename TA, typename T, int MODE, int BM, int BN, int TM, int TN>
+template <typename TA, typename T, int MODE, int BM, int BN, int BK, int TM, int TN, int MINB>
 int launch_tile(const GemmParams& p, cudaStream_t st) {
     const dim3 grid((p.M + BM - 1) / BM, (p.N + BN - 1) / BN);
-    const size_t smem = MODE == A_NEIGHBOURS ? (size_t)BM * p.taps * 8 : 0;
-    auto kern = gemm_simt_kernel<TA, T, MODE, BM, BN, TM, TN>;
-    if (smem) CONVNN_ENSURE_SMEM(kern, smem > 36 * 1024 ? smem : 36 * 1024);   // (beside up to 34 KB of static tiles)
+    const size_t smem = (size_t)2 * BK * (BM + 4 + BN + 4) * 4 + (MODE == A_NEIGHBOURS ? (size_t)BM * p.taps * 8 : 0);
+    auto kern = gemm_simt_kernel<TA, T, MODE, BM, BN, BK, TM, TN, MINB>;
+    CONVNN_ENSURE_SMEM(kern, smem);
     kern<<<grid, (BM / TM) * (BN / TN), smem, st>>>(p);
     return CONVNN_OK;
 }
 
 template <typename TA, typename T, int MODE>
 int launch_mode(const GemmParams& p, cudaStream_t st) {
-    // The tile with the least work on the busiest SM: rounds of tiles x outputs per tile, weighted by how well a
-    // tile's threads use the multiply-add pipes once it runs (measured ratios).
+    // The tile with the least work on the busiest SM: rounds of tiles x outputs per tile over the rate of the tile's
+    // threads.  That rate is set by shared memory: a k step reads TM + TN values per thread for TM * TN multiply-adds
+    // (45, 40, 29 and 26 TFLOP/s at 16384 x 768 x 768; 25 before).  2080 x 192 x 768: 33 us, 50 before; 50432 x 192 x
+    // 192: 89 us, 150 before.
     const long long sms = device_sms();
-    auto cost = [&](int bm, int bn, double eff) {
+    auto cost = [&](int bm, int bn, double rate) {
         const long long tiles = (long long)((p.M + bm - 1) / bm) * ((p.N + bn - 1) / bn);
-        return (double)((tiles + sms - 1) / sms) * bm * bn / eff;
+        return (double)((tiles + sms - 1) / sms) * bm * bn / rate;
     };
-    const double large = cost(128, 128, 1.0), mid = cost(64, 64, 0.8), small = cost(32, 64, 0.6);
-    if (large <= mid && large <= small) return launch_tile<TA, T, MODE, 128, 128, 8, 8>(p, st);
-    if (mid <= small) return launch_tile<TA, T, MODE, 64, 64, 8, 4>(p, st);
-    return launch_tile<TA, T, MODE, 32, 64, 4, 4>(p, st);
+    const double c[4] = {cost(128, 64, 45), cost(64, 64, 40), cost(32, 64, 29), cost(32, 32, 26)};
+    int best = 0;
+    for (int i = 1; i < 4; ++i)
+        if (c[i] < c[best]) best = i;
+    if (best == 0) return launch_tile<TA, T, MODE, 128, 64, 16, 8, 8, 3>(p, st);
+    if (best == 1) return launch_tile<TA, T, MODE, 64, 64, 32, 8, 4, 3>(p, st);
+    if (best == 2) return launch_tile<TA, T, MODE, 32, 64, 64, 4, 4, 2>(p, st);
+    return launch_tile<TA, T, MODE, 32, 32, 32, 4, 4, 4>(p, st);
 }
 
 template <typename T>
