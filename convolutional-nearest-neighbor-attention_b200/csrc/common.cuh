@@ -135,6 +135,10 @@ int read_sim_topk_status(int* out);
 int read_sim_topk2_status(int* out);
 int try_launch_gather_conv_dw_stream(const convnn_desc* d, const Dims& dm, const void* v, const int32_t* idx,
                                      const float* val, const void* w_conv, void* o, cudaStream_t st);
+int try_launch_gather_conv_dw(const convnn_desc* d, const Dims& dm, const void* v, const int32_t* idx, const float* val,
+                              const void* w_conv, void* o, bool out_f32, cudaStream_t st);
+int launch_gather_weighted(const convnn_desc* d, const Dims& dm, const void* v, const int32_t* idx, const float* val, void* P,
+                           cudaStream_t st);
 int read_dw_stream_status(int* out);
 int read_gemm_tc_status(int* out);
 // bfloat16 tensor-core GEMM C = A W^T (+bias, +GELU); `parts` outputs share M and split N evenly.

@@ -1,0 +1,55 @@
+"""Depthwise gather / conv at the edges of its tiles (tokens per CTA, tokens per thread, channel groups, weights that are
+not 16-byte rows) and the weighted neighbour block, against float64."""
+import pytest
+import torch
+
+from convnn_b200 import ops
+from gpu_util import DEV
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -24
+
+
+@pytest.mark.parametrize("B,T,H,dk,K", [(1, 1, 1, 8, 1), (1, 65, 1, 768, 16), (3, 197, 3, 32, 9), (2, 300, 1, 40, 32), (9, 513, 2, 64, 5),
+                                        (40, 1025, 1, 64, 9), (33, 1024, 4, 16, 25), (1, 13, 1, 264, 7)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("metric,softmax", [("cosine", True), ("euclidean", True), ("euclidean", False), ("matmul", False)])
+def test_depthwise_against_float64(B, T, H, dk, K, dtype, metric, softmax):
+    g = torch.Generator(device=DEV).manual_seed(B * T + K)
+    spec = ops.LayerSpec(H * dk, H, K, "all", metric, "depthwise", softmax, False, T)
+    v = torch.randn(B, T, H, dk, device=DEV, generator=g).to(dtype)
+    idx = torch.randint(0, T, (B, H, T, K), device=DEV, generator=g, dtype=torch.int32)
+    val = torch.rand(B, H, T, K, device=DEV, generator=g) + 0.25
+    w = torch.randn(K, dk, device=DEV, generator=g).to(dtype)
+    got = ops.gather_conv(spec, v, idx, val, w)
+    x = val.double() * (1 if metric != "euclidean" else -1)
+    p = torch.softmax(x, -1) if softmax else (val.double() if metric != "euclidean" else 1 / (val.double() + 1e-8))
+    rows = v.double().permute(0, 2, 1, 3)
+    want, mass = torch.zeros(B, H, T, dk, device=DEV, dtype=torch.double), torch.zeros(B, H, T, dk, device=DEV, dtype=torch.double)
+    for j in range(K):
+        term = p[..., j:j + 1] * torch.gather(rows, 2, idx[..., j:j + 1].long().expand(B, H, T, dk)) * w[j].double()
+        want += term
+        mass += term.abs()
+    bound = (2 * K + 24) * EPS * mass + (0 if dtype == torch.float32 else 2.0 ** -8) * want.abs() + 1e-30
+    assert bool(((got.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("B,T,H,dk,K", [(2, 65, 1, 768, 25), (1, 3, 1, 16, 1), (5, 197, 12, 32, 9), (2, 1030, 1, 192, 5)])
+def test_standard_conv_bfloat16_against_float64(B, T, H, dk, K):
+    g = torch.Generator(device=DEV).manual_seed(T)
+    spec = ops.LayerSpec(H * dk, H, K, "all", "cosine", "standard", True, False, T)
+    v = torch.randn(B, T, H, dk, device=DEV, generator=g).to(torch.bfloat16)
+    idx = torch.randint(0, T, (B, H, T, K), device=DEV, generator=g, dtype=torch.int32)
+    val = torch.randn(B, H, T, K, device=DEV, generator=g)
+    w = (torch.randn(dk, K, dk, device=DEV, generator=g) / (K * dk) ** 0.5).to(torch.bfloat16)
+    got = ops.gather_conv(spec, v, idx, val, w)
+    p = torch.softmax(val.double(), -1)
+    rows = v.double().permute(0, 2, 1, 3)
+    want, mass = torch.zeros(B, H, T, dk, device=DEV, dtype=torch.double), torch.zeros(B, H, T, dk, device=DEV, dtype=torch.double)
+    for j in range(K):
+        nb = p[..., j:j + 1] * torch.gather(rows, 2, idx[..., j:j + 1].long().expand(B, H, T, dk))
+        want += nb @ w[:, j].double().T
+        mass += nb.abs() @ w[:, j].double().abs().T
+    # the weighted block is rounded to bfloat16 once, the result once; fp32 sums of K * dk terms
+    bound = (2.0 ** -9 + (K * dk + 16) * EPS) * mass + 2.0 ** -8 * want.abs() + 1e-30
+    assert bool(((got.double() - want).abs() <= bound).all())
