@@ -50,7 +50,7 @@ struct TcParams {
     float* val;
     int T, S, H, K, nsel, metric, sampled;
     int KCH;          // channels per shared-memory chunk (64, 32 or 16)
-    int KC;           // chunks per tile = C / KCH
+    int KC;           // chunks per tile = ceil(C / KCH)
     int BN;           // candidate columns per MMA (multiple of 16, <= 128)
     int BNpad;        // TMEM columns per accumulator (power of two >= BN)
     int stages;       // shared-memory ring depth (<= MAX_STAGES)
@@ -279,7 +279,7 @@ int pow2_at_least(int v, int lo) {
 }  // namespace
 
 bool sim_topk_tc_supported(const convnn_desc* d, const Dims& dm, const void* q, const void* k) {
-    return d->dtype == CONVNN_BF16 && dm.Cp % 16 == 0 && aligned16(q) && aligned16(k);
+    return d->dtype == CONVNN_BF16 && dm.Cp % 8 == 0 && aligned16(q) && aligned16(k);
 }
 
 int launch_sim_topk_tc(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
@@ -288,8 +288,11 @@ int launch_sim_topk_tc(const convnn_desc* d, const Dims& dm, const void* q, cons
     TcParams p{};
     p.qstat = qstat; p.kstat = kstat; p.cand = cand; p.idx = idx; p.val = val;
     p.T = dm.T; p.S = dm.S; p.H = dm.H; p.K = dm.K; p.nsel = dm.nsel; p.metric = d->metric; p.sampled = d->sampled;
-    p.KCH = dm.Cp % 64 == 0 ? 64 : (dm.Cp % 32 == 0 ? 32 : 16);
-    p.KC = dm.Cp / p.KCH;
+    // 64-channel chunks whatever the head width: the copies fill what lies past a head's last channel with zeros, which
+    // add nothing to a dot product (three 16-channel chunks of a 48-channel head cost three stages, one padded one costs
+    // one; the coordinate channel's 392 stored channels are seven chunks).
+    p.KCH = dm.Cp <= 16 ? 16 : (dm.Cp <= 32 ? 32 : 64);
+    p.KC = (dm.Cp + p.KCH - 1) / p.KCH;
     // (heads of 257-512 channels on short sequences: 19.3 against 22.8 us at B=256, T=197, S=64, d_k=384;
     // with 768 channels the small shape measured slower)
     const bool small_cfg = dm.nsel <= 12 && (dm.Cp <= 256 || (dm.Cp <= 512 && dm.T <= 512));

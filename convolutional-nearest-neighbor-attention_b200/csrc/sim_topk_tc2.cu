@@ -286,11 +286,11 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 }  // namespace
 
 // The pair kernel pays off where the tensor pipe is the limiter: long key and candidate
-// lists, full 64-channel chunks.
+// lists, mostly full 64-channel chunks.
 bool sim_topk_tc2_wanted(const convnn_desc* d, const Dims& dm) {
     static const int env = [] { const char* e = getenv("CONVNN_B200_SIM_PAIR"); return e ? atoi(e) : -1; }();
     if (env == 0) return false;
-    if (d->dtype != CONVNN_BF16 || dm.Cp % 64 != 0) return false;
+    if (d->dtype != CONVNN_BF16 || dm.Cp % 8 != 0 || dm.Cp < 96) return false;   // (a last chunk is zero-filled past the head)
     // Lists longer than 16 double the cost of keeping two lists per row; measured break-even
     // is at many units per cluster and a few thousand candidates.
     if (dm.nsel > 16) return dm.T >= 8192 && dm.S >= 4096;
@@ -302,7 +302,7 @@ int launch_sim_topk_tc2(const convnn_desc* d, const Dims& dm, const void* q, con
     Tc2Params p{};
     p.qstat = qstat; p.kstat = kstat; p.cand = cand; p.idx = idx; p.val = val;
     p.T = dm.T; p.S = dm.S; p.H = dm.H; p.K = dm.K; p.nsel = dm.nsel; p.metric = d->metric; p.sampled = d->sampled;
-    p.KC = dm.Cp / KCH;
+    p.KC = (dm.Cp + KCH - 1) / KCH;
     p.n_row_units = (dm.T + 2 * BM - 1) / (2 * BM);
     p.n_col_tiles = (dm.S + BN - 1) / BN;
     p.n_units = dm.B * dm.H * p.n_row_units;
