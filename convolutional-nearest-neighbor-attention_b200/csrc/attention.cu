@@ -112,6 +112,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    chain_begin();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -320,6 +321,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 template <typename T>
 __global__ void attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                                       T* __restrict__ o, int Tn, int H, int dk, float scale) {
+    chain_begin();
     extern __shared__ float sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     float* prob = sm + warp * (Tn + dk);
@@ -408,7 +410,7 @@ int launch_attention_tc(const void* q, const void* k, const void* v, void* o, in
     const int grid = p.n_units < ctas ? p.n_units : ctas;
     auto kern = attention_tc_kernel;
     CONVNN_ENSURE_SMEM(kern, smem);
-    kern<<<grid, NTHREADS, smem, st>>>(tmQ, tmK, tmV, p);
+    launch_chained(kern, grid, NTHREADS, smem, st, tmQ, tmK, tmV, p);
     CONVNN_CHECK_LAUNCH("attention_tc");
     return CONVNN_OK;
 }
@@ -424,7 +426,7 @@ int launch_attention_simt_t(const void* q, const void* k, const void* v, void* o
     CONVNN_ENSURE_SMEM(kern, smem);
     int gx = (Tn + nw - 1) / nw;
     if (gx > 64) gx = 64;
-    kern<<<dim3(gx, B * H), nw * 32, smem, st>>>(static_cast<const T*>(q), static_cast<const T*>(k),
+    launch_chained(kern, dim3(gx, B * H), nw * 32, smem, st, static_cast<const T*>(q), static_cast<const T*>(k),
                                                  static_cast<const T*>(v), static_cast<T*>(o), Tn, H, dk,
                                                  (float)(1.0 / sqrt((double)dk)));
     CONVNN_CHECK_LAUNCH("attention_simt");

@@ -14,6 +14,7 @@ namespace {
 template <typename T>
 __global__ void conv1d_unfold_kernel(const T* __restrict__ y, T* __restrict__ u, int Tn, int H, int dk, int ks, int pad,
                                      long long total_vec, int vec) {
+    chain_begin();
     const int per_tap = dk / vec;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total_vec;
          i += (long long)gridDim.x * blockDim.x) {
@@ -42,6 +43,7 @@ __global__ void conv1d_unfold_kernel(const T* __restrict__ y, T* __restrict__ u,
 template <typename T>
 __global__ void conv1d_simt_kernel(const T* __restrict__ y, const T* __restrict__ w, const T* __restrict__ bias,
                                    T* __restrict__ o, int Tn, int H, int dk, int ks, int pad, long long total) {
+    chain_begin();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
         const int oc = (int)(i % dk);
@@ -77,7 +79,7 @@ int launch_conv1d_heads(int dtype, const void* y, const void* w, const void* bia
         const long long total = M * ks * (dk / vec);
         int blocks = (int)((total + 255) / 256);
         if (blocks > 148 * 16) blocks = 148 * 16;
-        conv1d_unfold_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(y),
+        launch_chained(conv1d_unfold_kernel<__nv_bfloat16>, blocks, 256, 0, st, static_cast<const __nv_bfloat16*>(y),
                                                                    static_cast<__nv_bfloat16*>(unfold), Tn, H, dk, ks, pad,
                                                                    total, vec);
         CONVNN_CHECK_LAUNCH("conv1d_unfold");
@@ -96,11 +98,11 @@ int launch_conv1d_heads(int dtype, const void* y, const void* w, const void* bia
     int blocks = (int)((total + 255) / 256);
     if (blocks > 148 * 16) blocks = 148 * 16;
     if (dtype == CONVNN_F32)
-        conv1d_simt_kernel<float><<<blocks, 256, 0, st>>>(static_cast<const float*>(y), static_cast<const float*>(w),
+        launch_chained(conv1d_simt_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(y), static_cast<const float*>(w),
                                                          static_cast<const float*>(bias), static_cast<float*>(o), Tn, H, dk,
                                                          ks, pad, total);
     else
-        conv1d_simt_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(
+        launch_chained(conv1d_simt_kernel<__nv_bfloat16>, blocks, 256, 0, st, 
             static_cast<const __nv_bfloat16*>(y), static_cast<const __nv_bfloat16*>(w),
             static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(o), Tn, H, dk, ks, pad, total);
     CONVNN_CHECK_LAUNCH("conv1d_simt");

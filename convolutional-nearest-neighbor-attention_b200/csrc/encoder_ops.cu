@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const T* __restrict__ x,
                                                         float eps, T* __restrict__ y, long long ldy, long long rows,
                                                         int D, const T* __restrict__ pe, const T* __restrict__ cls,
                                                         int Np, long long cls_rows, float2* __restrict__ moments) {
+    chain_begin();
     // moments (or nullptr): (sum, sum of squares) of every STORED output row, indexed by output row: what the
     // pre-norm fold of the first GEMM behind the embedding needs
     constexpr int V = Vec16<T>::N;
@@ -156,6 +157,7 @@ __global__ void __launch_bounds__(256, MINB) layernorm_bf16_row256_kernel(
     const __nv_bfloat16* __restrict__ beta, float eps, __nv_bfloat16* __restrict__ y, long long ldy, long long rows,
     int D, const __nv_bfloat16* __restrict__ pe, const __nv_bfloat16* __restrict__ cls, int Np, long long cls_rows,
     float2* __restrict__ moments) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long wpb = blockDim.x >> 5;
     const bool act = lane < D / 8;
@@ -295,6 +297,7 @@ __global__ void __launch_bounds__(256, MINB) layernorm_bf16_row256_kernel(
 template <typename T, typename VT>
 __global__ void __launch_bounds__(256) patchify_kernel(const T* __restrict__ img, T* __restrict__ out, int C, int Hh,
                                                        int Ww, int P) {
+    chain_begin();
     // One CTA per (image, row of patches): C * P image rows of Ww elements, read in image order
     // (whole rows, coalesced) and stored as the P-element runs of the patches' rows.  The index
     // arithmetic is 32-bit inside the strip; four vectors per thread are in flight.
@@ -337,6 +340,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(256) patchify_u8_kernel(const uint8_t* __restrict__ img, const float* __restrict__ mean,
                                                           const float* __restrict__ inv_std, T* __restrict__ out, int C,
                                                           int Hh, int Ww, int P) {
+    chain_begin();
     constexpr int U = VEC == 8 ? 4 : 8;
     const int Hp = Hh / P, Wp = Ww / P;
     const int b = blockIdx.x / Hp, py = blockIdx.x - b * Hp;
@@ -383,7 +387,7 @@ __global__ void __launch_bounds__(256) patchify_u8_kernel(const uint8_t* __restr
 
 template <typename T, typename VT>
 void patchify_launch(const void* img, void* out, int B, int C, int Hh, int Ww, int P, cudaStream_t st) {
-    patchify_kernel<T, VT><<<B * (Hh / P), 256, 0, st>>>(static_cast<const T*>(img), static_cast<T*>(out), C, Hh, Ww, P);
+    launch_chained(patchify_kernel<T, VT>, B * (Hh / P), 256, 0, st, static_cast<const T*>(img), static_cast<T*>(out), C, Hh, Ww, P);
 }
 
 template <typename T>
@@ -402,11 +406,11 @@ int ln_dispatch(const void* x, long long ldx, const void* gamma, const void* bet
 #define CONVNN_LN(NVV)                                                                                          \
     do {                                                                                                        \
         if (pe)                                                                                                 \
-            layernorm_kernel<T, NVV, true><<<blocks, 256, 0, st>>>(static_cast<const T*>(x), ldx,              \
+            launch_chained(layernorm_kernel<T, NVV, true>, blocks, 256, 0, st, static_cast<const T*>(x), ldx,              \
                 static_cast<const T*>(gamma), static_cast<const T*>(beta), eps, static_cast<T*>(y), ldy, rows, D, \
                 static_cast<const T*>(pe), static_cast<const T*>(cls), Np, cls_rows, reinterpret_cast<float2*>(moments)); \
         else                                                                                                    \
-            layernorm_kernel<T, NVV, false><<<blocks, 256, 0, st>>>(static_cast<const T*>(x), ldx,             \
+            launch_chained(layernorm_kernel<T, NVV, false>, blocks, 256, 0, st, static_cast<const T*>(x), ldx,             \
                 static_cast<const T*>(gamma), static_cast<const T*>(beta), eps, static_cast<T*>(y), ldy, rows, D, \
                 nullptr, nullptr, 0, 0, nullptr);                                                               \
     } while (0)
@@ -441,11 +445,11 @@ int launch_layernorm(int dtype, const void* x, long long ldx, const void* gamma,
         const auto* xb = static_cast<const __nv_bfloat16*>(x);
         const auto *gb = static_cast<const __nv_bfloat16*>(gamma), *bb = static_cast<const __nv_bfloat16*>(beta);
         if (pe)
-            layernorm_bf16_row256_kernel<R, MINB, true><<<blocks, 256, 0, st>>>(
+            launch_chained(layernorm_bf16_row256_kernel<R, MINB, true>, blocks, 256, 0, st, 
                 xb, ldx, gb, bb, eps, static_cast<__nv_bfloat16*>(y), ldy, rows, D, static_cast<const __nv_bfloat16*>(pe),
                 static_cast<const __nv_bfloat16*>(cls), Np, cls_rows, reinterpret_cast<float2*>(moments));
         else
-            layernorm_bf16_row256_kernel<R, MINB, false><<<blocks, 256, 0, st>>>(
+            launch_chained(layernorm_bf16_row256_kernel<R, MINB, false>, blocks, 256, 0, st, 
                 xb, ldx, gb, bb, eps, static_cast<__nv_bfloat16*>(y), ldy, rows, D, nullptr, nullptr, 0, 0, nullptr);
         CONVNN_CHECK_LAUNCH("layernorm_bf16_row256");
         return CONVNN_OK;
@@ -461,6 +465,7 @@ namespace {
 // later set of moments comes out of a GEMM epilogue.
 __global__ void __launch_bounds__(256) row_moments_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
                                                           long long rows, int D, float2* __restrict__ out) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (r >= rows) return;
@@ -519,7 +524,7 @@ __global__ void __launch_bounds__(256) fold_layernorm_kernel(const __nv_bfloat16
 int launch_row_moments(const void* x, long long ldx, long long rows, int D, float* moments, cudaStream_t st) {
     if (D % 8 != 0 || ldx % 8 != 0 || !aligned16(x) || (reinterpret_cast<uintptr_t>(moments) & 7u))
         return set_error(CONVNN_E_ALIGN, "row_moments: D and ldx must be multiples of 8 elements, x 16-byte aligned");
-    row_moments_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), ldx, rows, D,
+    launch_chained(row_moments_kernel, (unsigned)((rows + 7) / 8), 256, 0, st, static_cast<const __nv_bfloat16*>(x), ldx, rows, D,
                                                                   reinterpret_cast<float2*>(moments));
     CONVNN_CHECK_LAUNCH("row_moments");
     return CONVNN_OK;
@@ -539,7 +544,7 @@ int launch_patchify_u8(int dtype, const uint8_t* img, const float* mean, const f
                        int Hh, int Ww, int P, cudaStream_t st) {
     if (Hh % P != 0 || Ww % P != 0) return set_error(CONVNN_E_INVALID, "patchify: image not divisible into patches");
     const bool v8 = P % 8 == 0 && Ww % 8 == 0 && (reinterpret_cast<uintptr_t>(img) & 7u) == 0 && aligned16(out);
-#define CONVNN_PU8(T, V) patchify_u8_kernel<T, V><<<B * (Hh / P), 256, 0, st>>>(img, mean, inv_std, static_cast<T*>(out), C, Hh, Ww, P)
+#define CONVNN_PU8(T, V) launch_chained(patchify_u8_kernel<T, V>, B * (Hh / P), 256, 0, st, img, mean, inv_std, static_cast<T*>(out), C, Hh, Ww, P)
     if (dtype == CONVNN_F32) { if (v8) CONVNN_PU8(float, 8); else CONVNN_PU8(float, 1); }
     else { if (v8) CONVNN_PU8(__nv_bfloat16, 8); else CONVNN_PU8(__nv_bfloat16, 1); }
 #undef CONVNN_PU8

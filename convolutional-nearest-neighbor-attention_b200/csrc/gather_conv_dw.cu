@@ -87,6 +87,7 @@ __device__ __forceinline__ void token_pairs(const DwParams& p, int m0, int nt, i
 
 template <typename T, typename TO, int VEC, int TPT>
 __global__ void __launch_bounds__(THREADS) gather_conv_dw_kernel(const DwParams p, const int TT) {
+    chain_begin();
     typedef Channels<T, VEC> Ch;
     extern __shared__ __align__(16) unsigned char dw_smem[];
     int2* pairs = reinterpret_cast<int2*>(dw_smem);           // [TT][K]
@@ -147,6 +148,7 @@ __global__ void __launch_bounds__(THREADS) gather_conv_dw_kernel(const DwParams 
 // Weighted neighbour block of the tensor-core standard conv: P[m, j * C + c] = bf16(weight(m, j) * v[neighbour(m, j), c]),
 // the A operand of a GEMM with the (d_k, K * C) tap weights; four independent rows in flight per thread.
 __global__ void __launch_bounds__(THREADS) gather_weighted_kernel(const DwParams p, const int TT) {
+    chain_begin();
     constexpr int U = 4;
     extern __shared__ __align__(16) unsigned char dw_smem[];
     int2* pairs = reinterpret_cast<int2*>(dw_smem);
@@ -200,8 +202,8 @@ int launch(const DwParams& p, cudaStream_t st) {
     if (TT < tpt) TT = tpt;
     const size_t smem = (size_t)TT * p.K * 8 + TT * 4;
     const int grid = (p.M + TT - 1) / TT;
-    if (tpt == 4) gather_conv_dw_kernel<T, TO, VEC, 4><<<grid, THREADS, smem, st>>>(p, TT);
-    else gather_conv_dw_kernel<T, TO, VEC, 1><<<grid, THREADS, smem, st>>>(p, TT);
+    if (tpt == 4) launch_chained(gather_conv_dw_kernel<T, TO, VEC, 4>, grid, THREADS, smem, st, p, TT);
+    else launch_chained(gather_conv_dw_kernel<T, TO, VEC, 1>, grid, THREADS, smem, st, p, TT);
     CONVNN_CHECK_LAUNCH("gather_conv_dw");
     return CONVNN_OK;
 }
@@ -226,7 +228,7 @@ int launch_gather_weighted(const convnn_desc* d, const Dims& dm, const void* v, 
     // images of 65 tokens, 768 channels, 25 taps on four CTAs: 245 us)
     int TT = 8 * THREADS / (p.K * p.groups);
     TT = TT < 1 ? 1 : (TT > 64 ? 64 : TT);
-    gather_weighted_kernel<<<(p.M + TT - 1) / TT, THREADS, (size_t)TT * p.K * 8 + TT * 4, st>>>(p, TT);
+    launch_chained(gather_weighted_kernel, (p.M + TT - 1) / TT, THREADS, (size_t)TT * p.K * 8 + TT * 4, st, p, TT);
     CONVNN_CHECK_LAUNCH("gather_weighted");
     return CONVNN_OK;
 }

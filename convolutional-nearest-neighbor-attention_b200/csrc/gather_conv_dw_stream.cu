@@ -75,6 +75,7 @@ gather_conv_dw_stream_kernel(const __grid_constant__ CUtensorMap tmV, const DwsP
         prefetch_tensormap(&tmV);
     }
     __syncthreads();
+    chain_begin();
 
     // tap weights of this thread's 8 channels, as packed pairs
     f32x2 w2[KT][4];
@@ -186,7 +187,7 @@ int try_launch_gather_conv_dw_stream(const convnn_desc* d, const Dims& dm, const
 
     auto kern = gather_conv_dw_stream_kernel;
     CONVNN_ENSURE_SMEM(kern, smem);
-    kern<<<per_chunk * p.nchunks, TPB, smem, st>>>(tmV, p);
+    launch_chained(kern, per_chunk * p.nchunks, TPB, smem, st, tmV, p);
     CONVNN_CHECK_LAUNCH("gather_conv_dw_stream");
     return CONVNN_OK;
 }

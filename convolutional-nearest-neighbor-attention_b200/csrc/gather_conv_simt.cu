@@ -30,6 +30,7 @@ __global__ void __launch_bounds__(THREADS) gather_conv_dw_scalar_kernel(
     const T* __restrict__ v, const int32_t* __restrict__ idx, const float* __restrict__ val,
     const T* __restrict__ wconv, T* __restrict__ o, int T_, int H, int dk, int Cp, int K, int maximum,
     int softmax) {
+    chain_begin();
     __shared__ float ps[TT][kMaxK];
     __shared__ int ns[TT][kMaxK];
     const int bh = blockIdx.y;
@@ -59,6 +60,7 @@ __global__ void __launch_bounds__(THREADS) gather_conv_mat_kernel(
     const T* __restrict__ v, const int32_t* __restrict__ idx, const float* __restrict__ val,
     const T* __restrict__ wconv, const T* __restrict__ wpw, T* __restrict__ o, int T_, int H, int dk,
     int C, int Cp, int K, int maximum, int softmax, int separable, int TT, int JC) {
+    chain_begin();
     extern __shared__ __align__(16) float P[];
     __shared__ float ps[32][kMaxK];
     __shared__ int ns[32][kMaxK];
@@ -142,7 +144,7 @@ int launch_dw_scalar(const convnn_desc* d, const Dims& dm, const void* v, const 
                      const void* w_conv, void* o, cudaStream_t st) {
     constexpr int TT = 16;
     dim3 grid((dm.T + TT - 1) / TT, dm.B * dm.H);
-    gather_conv_dw_scalar_kernel<T, TT><<<grid, THREADS, 0, st>>>(
+    launch_chained(gather_conv_dw_scalar_kernel<T, TT>, grid, THREADS, 0, st, 
         static_cast<const T*>(v), idx, val, static_cast<const T*>(w_conv), static_cast<T*>(o), dm.T, dm.H,
         dm.dk, dm.Cp, dm.K, d->metric != CONVNN_EUCLIDEAN, d->softmax);
     CONVNN_CHECK_LAUNCH("gather_conv_dw_scalar");
@@ -176,7 +178,7 @@ int launch_mat(const convnn_desc* d, const Dims& dm, const void* v, const int32_
     auto kern = gather_conv_mat_kernel<T, ITEMS>;
     CONVNN_ENSURE_SMEM(kern, smem);
     dim3 grid((dm.T + TT - 1) / TT, dm.B * dm.H);
-    kern<<<grid, THREADS, smem, st>>>(static_cast<const T*>(v), idx, val, static_cast<const T*>(w_conv),
+    launch_chained(kern, grid, THREADS, smem, st, static_cast<const T*>(v), idx, val, static_cast<const T*>(w_conv),
                                       static_cast<const T*>(w_pw), static_cast<T*>(o), dm.T, dm.H, dm.dk, dm.C,
                                       dm.Cp, dm.K, d->metric != CONVNN_EUCLIDEAN, d->softmax, separable, TT, JC);
     CONVNN_CHECK_LAUNCH("gather_conv_mat");

@@ -239,6 +239,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (PAIR) { tmem_alloc_pair(tmem_slot, ncols); tmem_relinquish_pair(); }
         else { tmem_alloc(tmem_slot, ncols); tmem_relinquish(); }
     }
+    chain_wait();
     if (p.mma_bias) {
         // D = ones * btile^T = bias[n] in every row.  Both 16-byte halves of a row of `ones`
         // start with 1.0 and a btile row holds its bias in exactly one half, so the product
@@ -261,6 +262,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (PAIR) cluster_sync_all();               // both CTAs' barriers exist before any remote signal
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    chain_next();
     const uint32_t peer_abort = PAIR ? map_to_cta(smem_u32(const_cast<int*>(abort_flag)), rank ^ 1u) : 0u;
     auto give_up = [&](int code) {
         if (PAIR) fail_pair(abort_flag, peer_abort, code);
@@ -777,6 +779,7 @@ namespace {
 // out[i] = f(sum over pieces of partial[piece][i]): the statistic of heads that span several tiles
 __global__ void stat_combine_kernel(const float* __restrict__ partial, long long plane, int pieces, long long n,
                                     int cosine, float* __restrict__ out) {
+    chain_begin();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float s = 0.f;
@@ -954,20 +957,20 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
     do {                                                                                                    \
         auto kern = gemm_tc_kernel<S, B, G, R, W, false>;                                                   \
         CONVNN_ENSURE_SMEM(kern, smem);                                                            \
-        kern<<<grid, W ? NTHREADS_WIDE : NTHREADS, smem, st>>>(tmA, tmW, tmX, tmM, p);                           \
+        launch_chained(kern, grid, W ? NTHREADS_WIDE : NTHREADS, smem, st, tmA, tmW, tmX, tmM, p);                           \
     } while (0)
 #define CONVNN_GEMM_LAUNCH_X(S, G, R, W, LNFv, MOMv)                                                        \
     do {                                                                                                    \
         auto kern = gemm_tc_kernel<S, false, G, R, W, false, LNFv, MOMv>;                                   \
         CONVNN_ENSURE_SMEM(kern, smem);                                                            \
-        kern<<<grid, (W ? NTHREADS_WIDE : NTHREADS) + (LNFv ? 32 : 0), smem, st>>>(tmA, tmW, tmX, tmM, p);       \
+        launch_chained(kern, grid, (W ? NTHREADS_WIDE : NTHREADS) + (LNFv ? 32 : 0), smem, st, tmA, tmW, tmX, tmM, p);       \
     } while (0)
 #define CONVNN_GEMM_LAUNCH_PAIR(G, R, W)                                                                    \
     do {                                                                                                    \
         auto kern = gemm_tc_kernel<false, false, G, R, W, true>;                                            \
         CONVNN_ENSURE_SMEM(kern, smem);                                                            \
         cudaLaunchConfig_t cfg{};                                                                           \
-        cudaLaunchAttribute attr[1];                                                                        \
+        cudaLaunchAttribute attr[2];                                                                        \
         attr[0].id = cudaLaunchAttributeClusterDimension;                                                   \
         attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;           \
         cfg.blockDim = dim3(W ? NTHREADS_WIDE : NTHREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;    \
@@ -978,6 +981,7 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
         if (const int rc_ = fit.query(reinterpret_cast<const void*>(kern), &cfg, &max_clusters)) return rc_; \
         const int nc = p.n_tiles < max_clusters ? p.n_tiles : max_clusters;                                 \
         cfg.gridDim = dim3(2 * nc);                                                                         \
+        attr[1] = chained_attribute(st); cfg.numAttrs = 2;                                                  \
         const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmW, tmX, tmM, p);                                                    \
         if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "gemm_tc pair launch: %s", cudaGetErrorString(e)); \
     } while (0)
@@ -1014,7 +1018,7 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
         for (int i = 0; i < parts; ++i) {
             if (!stat_final[i]) continue;
             const long long n = p.stat_plane;
-            stat_combine_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p.stat[i], p.stat_plane, p.stat_pieces, n,
+            launch_chained(stat_combine_kernel, (unsigned)((n + 255) / 256), 256, 0, st, p.stat[i], p.stat_plane, p.stat_pieces, n,
                                                                             p.stat_mode == CONVNN_COSINE, stat_final[i]);
             CONVNN_CHECK_LAUNCH("stat_combine");
         }

@@ -20,6 +20,7 @@ __device__ __forceinline__ float linspace_pm1(int i, int steps) {
 template <typename T>
 __global__ void head_stats_kernel(T* t, float* stat, int B, int rows, int H, int dk, int C, int Cp,
                                   int coord, int metric) {
+    chain_begin();
     const int warps_per_block = blockDim.x >> 5;
     const long long total = (long long)B * rows * H;
     const int lane = threadIdx.x & 31;
@@ -74,10 +75,10 @@ int launch_head_fill_and_stats(const convnn_desc* d, const Dims& dm, void* t, in
     if (blocks > 148 * 16) blocks = 148 * 16;
     if (blocks < 1) blocks = 1;
     if (d->dtype == CONVNN_F32)
-        head_stats_kernel<float><<<blocks, 256, 0, st>>>(static_cast<float*>(t), stat, dm.B, rows, dm.H,
+        launch_chained(head_stats_kernel<float>, blocks, 256, 0, st, static_cast<float*>(t), stat, dm.B, rows, dm.H,
                                                         dm.dk, dm.C, dm.Cp, d->coord, d->metric);
     else
-        head_stats_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(static_cast<__nv_bfloat16*>(t), stat, dm.B,
+        launch_chained(head_stats_kernel<__nv_bfloat16>, blocks, 256, 0, st, static_cast<__nv_bfloat16*>(t), stat, dm.B,
                                                                 rows, dm.H, dm.dk, dm.C, dm.Cp, d->coord,
                                                                 d->metric);
     CONVNN_CHECK_LAUNCH("head_stats");

@@ -13,6 +13,7 @@ namespace {
 template <typename T>
 __global__ void gather_rows_kernel(const T* __restrict__ x, long long ldx, const int32_t* __restrict__ cand,
                                    T* __restrict__ xq, int Tn, int S, int D, long long total_vec, int vec) {
+    chain_begin();
     const int per_row = D / vec;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total_vec;
          i += (long long)gridDim.x * blockDim.x) {
@@ -33,6 +34,7 @@ __global__ void gather_rows_kernel(const T* __restrict__ x, long long ldx, const
 // Sequences of which eight channels exceed shared memory: 32 x 32 tiles.
 template <typename T>
 __global__ void merge_heads_tile_kernel(const T* __restrict__ o, T* __restrict__ y, int Tn, int H, int dk, int D) {
+    chain_begin();
     __shared__ T tile[32][33];
     const int bh = blockIdx.z;
     const int b = bh / H, h = bh - b * H;
@@ -55,6 +57,7 @@ __global__ void merge_heads_tile_kernel(const T* __restrict__ o, T* __restrict__
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) merge_heads_kernel(const T* __restrict__ o, T* __restrict__ y, int Tn, int H, int dk,
                                                           int D, int CB) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char mh_smem[];
     T* s = reinterpret_cast<T*>(mh_smem);                 // [CB][Tn]
     constexpr int PER = 16 / sizeof(T);
@@ -95,7 +98,7 @@ int merge_heads(const void* o, void* y, int B, int Tn, int H, int dk, cudaStream
     if (CB > dk) CB = dk;
     const size_t smem = (size_t)CB * Tn * sizeof(T);
     if (smem > 200 * 1024) {
-        merge_heads_tile_kernel<T><<<dim3((Tn + 31) / 32, (dk + 31) / 32, B * H), dim3(32, 8), 0, st>>>(
+        launch_chained(merge_heads_tile_kernel<T>, dim3((Tn + 31) / 32, (dk + 31) / 32, B * H), dim3(32, 8), 0, st, 
             static_cast<const T*>(o), static_cast<T*>(y), Tn, H, dk, H * dk);
         CONVNN_CHECK_LAUNCH("merge_heads");
         return CONVNN_OK;
@@ -104,11 +107,11 @@ int merge_heads(const void* o, void* y, int B, int Tn, int H, int dk, cudaStream
     if (vec) {
         auto kern = merge_heads_kernel<T, V>;
         CONVNN_ENSURE_SMEM(kern, smem);
-        kern<<<grid, 256, smem, st>>>(static_cast<const T*>(o), static_cast<T*>(y), Tn, H, dk, H * dk, CB);
+        launch_chained(kern, grid, 256, smem, st, static_cast<const T*>(o), static_cast<T*>(y), Tn, H, dk, H * dk, CB);
     } else {
         auto kern = merge_heads_kernel<T, 1>;
         CONVNN_ENSURE_SMEM(kern, smem);
-        kern<<<grid, 256, smem, st>>>(static_cast<const T*>(o), static_cast<T*>(y), Tn, H, dk, H * dk, CB);
+        launch_chained(kern, grid, 256, smem, st, static_cast<const T*>(o), static_cast<T*>(y), Tn, H, dk, H * dk, CB);
     }
     CONVNN_CHECK_LAUNCH("merge_heads");
     return CONVNN_OK;
@@ -125,10 +128,10 @@ int launch_gather_rows(int dtype, const void* x, long long ldx, const int32_t* c
     int blocks = (int)((total + 255) / 256);
     if (blocks > 148 * 8) blocks = 148 * 8;
     if (dtype == CONVNN_F32)
-        gather_rows_kernel<float><<<blocks, 256, 0, st>>>(static_cast<const float*>(x), ldx, cand,
+        launch_chained(gather_rows_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(x), ldx, cand,
                                                          static_cast<float*>(xq), Tn, S, D, total, vec);
     else
-        gather_rows_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), ldx, cand,
+        launch_chained(gather_rows_kernel<__nv_bfloat16>, blocks, 256, 0, st, static_cast<const __nv_bfloat16*>(x), ldx, cand,
                                                                  static_cast<__nv_bfloat16*>(xq), Tn, S, D, total, vec);
     CONVNN_CHECK_LAUNCH("gather_rows");
     return CONVNN_OK;

@@ -190,6 +190,7 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
     }
     __syncthreads();
     if (warp == 1) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
+    chain_wait();
     for (int i = threadIdx.x; i < p.D / 2; i += blockDim.x)         // b2 (or zeros) for the final epilogue
         reinterpret_cast<uint32_t*>(smem + L.bias)[i] = p.bias2 ? reinterpret_cast<const uint32_t*>(p.bias2)[i] : 0u;
     tc_fence_before_sync();
@@ -197,6 +198,7 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
     cluster_sync_all();                          // both CTAs' barriers exist before any remote signal
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    chain_next();
     const uint32_t peer_abort = map_to_cta(smem_u32(const_cast<int*>(abort_flag)), rank ^ 1u);
     auto give_up = [&](int code) {
         st_cluster_u32(peer_abort, 1u);
@@ -751,7 +753,7 @@ int launch_mlp_tc(const void* x, long long ldx, const float* moments, int planes
     static SmemLimit limits[2]{};
     if (const int rc = limits[w_o ? 1 : 0].ensure(reinterpret_cast<const void*>(kern), smem)) return rc;
     cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.blockDim = dim3(NT); cfg.dynamicSmemBytes = smem; cfg.stream = st;
@@ -762,6 +764,7 @@ int launch_mlp_tc(const void* x, long long ldx, const float* moments, int planes
     if (const int rc = fit[w_o ? 1 : 0].query(reinterpret_cast<const void*>(kern), &cfg, &max_clusters)) return rc;
     const int nc = p.n_ptiles < max_clusters ? p.n_ptiles : max_clusters;
     cfg.gridDim = dim3(2 * nc);
+    attr[1] = chained_attribute(st); cfg.numAttrs = 2;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmX, tmO, tmW1, tmWX, tmW2, tmWO, p);
     if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "mlp_tc launch: %s", cudaGetErrorString(e));
     CONVNN_CHECK_LAUNCH("mlp_tc");

@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(NT) sim_topk_simt_kernel(
     const float* __restrict__ kstat, const int32_t* __restrict__ cand, int32_t* __restrict__ idx,
     float* __restrict__ val, int T_, int S, int H, int Cp, int K, int nsel, int metric, int sampled,
     float sqrt_dk, int vec) {
+    chain_begin();
     constexpr int TM = RB / 16, RG = TM / 4;              // 16 x 16 threads, TM x 4 dot products each
     constexpr int LA = RB + 4, LB = CB + 4;
     constexpr int NA = RB * (BK / 4) / NT, TPR = NT / RB; // loads per thread and step; scanning threads per row

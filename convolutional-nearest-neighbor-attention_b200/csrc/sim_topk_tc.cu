@@ -109,6 +109,7 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    chain_begin();
 
     const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty);
     const uint32_t st0 = smem_u32(stages);
@@ -328,7 +329,7 @@ int launch_sim_topk_tc(const convnn_desc* d, const Dims& dm, const void* q, cons
     do {                                                                                               \
         auto kern = sim_topk_tc_kernel<N, MINB, CWV>;                                                  \
         CONVNN_ENSURE_SMEM(kern, smem);                                                            \
-        kern<<<grid, NTHREADS, smem, st>>>(tmK, tmQ, p);                                               \
+        launch_chained(kern, grid, NTHREADS, smem, st, tmK, tmQ, p);                                               \
     } while (0)
 #define CONVNN_TC_LAUNCH(N)                            \
     do {                                               \

@@ -114,6 +114,7 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     cluster_sync_all();                         // both CTAs' barriers exist before any remote signal
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    chain_begin();
 
     const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty);
     const uint32_t tfull0 = smem_u32(tfull), tempty0 = smem_u32(tempty);
@@ -328,7 +329,7 @@ int launch_sim_topk_tc2(const convnn_desc* d, const Dims& dm, const void* q, con
         const size_t smem = smem_fixed + (size_t)NST * STAGE_BYTES + 2 * N * kSelGroup * sizeof(float);          \
         CONVNN_ENSURE_SMEM(kern, smem);                                                            \
         cudaLaunchConfig_t cfg{};                                                                                \
-        cudaLaunchAttribute attr[1];                                                                             \
+        cudaLaunchAttribute attr[2];                                                                             \
         attr[0].id = cudaLaunchAttributeClusterDimension;                                                        \
         attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;                \
         cfg.blockDim = dim3(NTHREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;                             \
@@ -339,6 +340,7 @@ int launch_sim_topk_tc2(const convnn_desc* d, const Dims& dm, const void* q, con
         if (const int rc_ = fit.query(reinterpret_cast<const void*>(kern), &cfg, &max_clusters)) return rc_; \
         const int nc = p.n_units < max_clusters ? p.n_units : max_clusters;                                      \
         cfg.gridDim = dim3(2 * nc);                                                                              \
+        attr[1] = chained_attribute(st); cfg.numAttrs = 2;                                                       \
         const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmK, tmQ, p);                                                         \
         if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "sim_topk_tc2 launch: %s", cudaGetErrorString(e)); \
     } while (0)
