@@ -1,0 +1,487 @@
+// Similarity + top-K for short candidate lists (S <= 256): a row's whole similarity vector is one accumulator in tensor
+// memory, so the selection can read it twice.
+//
+//   pass 1  values only: a sorted list of the best NSEL keys, two columns at a time.  With a >= b the merged list is
+//           v'[s] = max(v[s], min(v[s-1], a), min(v[s-2], b)): three instructions per slot and PAIR of columns, no
+//           branches, no indices, every slot computed from old values.
+//   pass 2  the nsel-th value is now the exact threshold: columns whose key reaches it (nsel of them unless keys tie there)
+//           are appended, in column order, to the row's entries in shared memory.
+//   rank    all pairs of entries are compared once; the earlier column wins ties.
+//
+// A row with ties at the threshold or too few keys above -inf (NaN inputs) makes its warp repeat the selection with the
+// ordered insertion of the streaming kernels, so results are the same bit for bit.
+//
+// A persistent CTA per SM: warp 0 TMA producer (128 key rows + all candidate rows of one (batch, head), 64-channel chunks,
+// ring), warp 1 MMA issuer (M = 128, N = S rounded to 16), then selection warps (thread = row).  G accumulators of 512 / G
+// columns, G = 4 for S <= 128, else 2, so the next units' MMAs run under the selection.  With NH = 2 two warps share a row
+// block of an accumulator, a column half each: the threshold follows from their two sorted lists (the n-th largest of
+// a and b is the largest min(a[i], b[n-2-i])), their entries grow towards each other, and they take turns at ranking.
+// (Eight selection warps, G = 2 and NH = 1, left each scheduler with two: 41 us at 256 images of 197 tokens, now 35.)
+#include "common.cuh"
+#include "sm100.cuh"
+#include "toplist.cuh"
+#include "sim_topk_select.cuh"
+
+namespace convnn {
+
+__device__ int g_sim_short_status = 0;
+
+namespace {
+
+using namespace sm100;
+
+constexpr int BM = 128;
+constexpr int MAX_STAGES = 6;
+
+struct ShortParams {
+    const float* qstat;
+    const float* kstat;
+    const int32_t* cand;
+    int32_t* idx;
+    float* val;
+    int T, S, H, K, nsel, metric, sampled;
+    int KCH, KC;      // channels per shared-memory chunk, chunks per unit
+    int BN;           // S rounded up to 16
+    int stages, n_row_tiles, n_units;
+    float sqrt_dk;
+};
+
+__device__ __forceinline__ void fail(volatile int* abort_flag, int code) {
+    *abort_flag = 1;
+    atomicCAS(&g_sim_short_status, 0, code);
+}
+
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld_x32(taddr, r); }
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld_x16(taddr, r); }
+
+// (NaN stays out of the list: min propagates it, max drops it)
+__device__ __forceinline__ float min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+template <int NSEL>
+__device__ __forceinline__ void merge_pair(float (&v)[NSEL], float k0, float k1) {
+    const float a = fmaxf(k0, k1), b = min_nan(k0, k1);
+#pragma unroll
+    for (int s = NSEL - 1; s >= 2; --s) v[s] = max3(v[s], min_nan(v[s - 1], a), min_nan(v[s - 2], b));
+    if (NSEL > 1) v[1] = max3(v[1], min_nan(v[0], a), b);
+    v[0] = fmaxf(v[0], a);
+}
+
+// Ranking keys of W accumulator columns from `col0` on; -inf past the last candidate.
+template <int W>
+__device__ __forceinline__ void make_keys(float (&key)[W], const uint32_t (&acc)[W], const float* qs, const int* cs, int col0,
+                                          const ShortParams& p, int row, float sentinel) {
+    if (p.metric != CONVNN_MATMUL) {
+        const f32x2 two = pack2(2.0f, 2.0f);
+#pragma unroll
+        for (int j4 = 0; j4 < W / 4; ++j4) {
+            const float4 s4 = *reinterpret_cast<const float4*>(qs + col0 + 4 * j4);
+            const f32x2 d01 = pack2(__uint_as_float(acc[4 * j4]), __uint_as_float(acc[4 * j4 + 1]));
+            const f32x2 d23 = pack2(__uint_as_float(acc[4 * j4 + 2]), __uint_as_float(acc[4 * j4 + 3]));
+            f32x2 k01, k23;
+            if (p.metric == CONVNN_COSINE) {
+                k01 = mul2(d01, pack2(s4.x, s4.y));
+                k23 = mul2(d23, pack2(s4.z, s4.w));
+            } else {
+                k01 = fma2(two, d01, pack2(-s4.x, -s4.y));
+                k23 = fma2(two, d23, pack2(-s4.z, -s4.w));
+            }
+            unpack2(k01, key[4 * j4], key[4 * j4 + 1]);
+            unpack2(k23, key[4 * j4 + 2], key[4 * j4 + 3]);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < W; ++j) key[j] = __uint_as_float(acc[j]);
+    }
+    if (p.sampled) {
+#pragma unroll
+        for (int j4 = 0; j4 < W / 4; ++j4) {
+            const int4 c4 = *reinterpret_cast<const int4*>(cs + col0 + 4 * j4);
+            if (c4.x == row) key[4 * j4] = sentinel;
+            if (c4.y == row) key[4 * j4 + 1] = sentinel;
+            if (c4.z == row) key[4 * j4 + 2] = sentinel;
+            if (c4.w == row) key[4 * j4 + 3] = sentinel;
+        }
+    }
+    const int left = p.S - col0;
+    if (left < W) {
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+            if (j >= left) key[j] = -CUDART_INF_F;
+    }
+}
+
+template <int NSEL, int G, int NH>
+__global__ void __launch_bounds__(64 + 128 * G * NH, 1)
+sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const ShortParams p) {
+    constexpr int MAXC = 512 / G;                  // tensor-memory columns of one accumulator
+    constexpr int W = G * NH == 4 ? 16 : 32;       // columns per read (18 warps leave 96 registers per thread)
+    constexpr int NT = 128 * G * NH;               // selection threads
+    constexpr uint32_t ENTRY = 128 * G * 8;        // bytes between a row's successive entries
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const uint32_t pitch = p.KCH * 2;
+    const uint32_t a_bytes = BM * pitch, b_bytes = p.BN * pitch, stage_bytes = a_bytes + b_bytes;
+    const uint32_t STAGES = p.stages;
+    float2* hits = reinterpret_cast<float2*>(smem + STAGES * stage_bytes);       // [NSEL + 2][128 * G] (key, column)
+    float* statbuf = reinterpret_cast<float*>(hits + (NSEL + 2) * 128 * G);      // [warps][MAXC] column statistics
+    int* cs = reinterpret_cast<int*>(statbuf + NT / 32 * MAXC);                  // [MAXC] candidate tokens
+    float* lists = reinterpret_cast<float*>(cs + MAXC);                          // NH = 2: [NSEL][NT] sorted keys
+    int* counts = reinterpret_cast<int*>(lists + (NH == 2 ? NSEL * NT : 0));     //         [NT] entries
+    uint64_t* full = reinterpret_cast<uint64_t*>(counts + (NH == 2 ? NT : 0));
+    uint64_t* empty = full + MAX_STAGES;
+    uint64_t* tfull = empty + MAX_STAGES;
+    uint64_t* tempty = tfull + G;
+    uint64_t* xlist = tempty + G;                  // NH = 2, per (accumulator, lane quarter): both lists written
+    uint64_t* xhits = xlist + 4 * G;               //                                          both sets of entries written
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xhits + 4 * G);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < MAX_STAGES; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < G; ++b) {
+            mbar_init(&tfull[b], 1);
+            mbar_init(&tempty[b], 4 * NH);
+        }
+        for (int b = 0; b < 4 * G; ++b) {
+            mbar_init(&xlist[b], 2);
+            mbar_init(&xhits[b], 2);
+        }
+        *abort_flag = 0;
+        fence_barrier_init();
+        prefetch_tensormap(&tmK);
+        prefetch_tensormap(&tmQ);
+    }
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+    chain_begin();
+
+    const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty), st0 = smem_u32(smem);
+    if (warp == 0) {
+        if (lane < 2) {                              // lane 0: key rows, lane 1: candidate rows (their copies overlap)
+            uint32_t s = 0, ph = 0;
+            bool ok = true;
+            for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x) {
+                const int bh = unit / p.n_row_tiles, rt = unit - bh * p.n_row_tiles;
+                const int b = bh / p.H, h = bh - b * p.H;
+                for (int kc = 0; kc < p.KC; ++kc) {
+                    ok = mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag);
+                    ok = __all_sync(0x3u, ok);
+                    if (!ok) { if (lane == 0) fail(abort_flag, 71); break; }
+                    const uint32_t st = st0 + s * stage_bytes, fb = full0 + 8 * s;
+                    if (lane == 0) mbar_expect_tx_a(fb, stage_bytes);
+                    __syncwarp(0x3u);
+                    if (lane == 0) tma_load_4d_a(st, &tmK, fb, kc * p.KCH, h, rt * BM, b);
+                    else tma_load_4d_a(st + a_bytes, &tmQ, fb, kc * p.KCH, h, 0, b);
+                    if (++s == STAGES) { s = 0; ph ^= 1u; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = make_idesc_bf16_f32(BM, p.BN);
+            const uint64_t dhi = kmajor_desc_hi(pitch);
+            const int nk16 = p.KCH / 16;
+            const uint32_t tfull0 = smem_u32(tfull), tempty0 = smem_u32(tempty);
+            uint32_t s = 0, ph = 0, buf = 0, use = 0;
+            bool ok = true;
+            for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x) {
+                if (!mbar_wait_a(tempty0 + 8 * buf, (use & 1u) ^ 1u, abort_flag)) { fail(abort_flag, 72); break; }
+                tc_fence_after_sync();
+                for (int kc = 0; kc < p.KC; ++kc) {
+                    if (!mbar_wait_a(full0 + 8 * s, ph, abort_flag)) { fail(abort_flag, 73); ok = false; break; }
+                    tc_fence_after_sync();
+                    const uint32_t sa = st0 + s * stage_bytes;
+                    mma_chunk(tmem_base + buf * MAXC, dhi | (uint64_t)(sa >> 4), dhi | (uint64_t)((sa + a_bytes) >> 4), idesc, nk16,
+                              kc != 0);
+                    mma_commit_a(empty0 + 8 * s);
+                    if (++s == STAGES) { s = 0; ph ^= 1u; }
+                }
+                if (ok) mma_commit_a(tfull0 + 8 * buf);
+                if (++buf == G) { buf = 0; ++use; }
+            }
+        }
+    } else {
+        const int g = (warp - 2) / (4 * NH);         // accumulator this warp serves
+        const int half = NH == 2 ? ((warp - 2) >> 2) & 1 : 0;
+        const int lq = warp & 3;                     // TMEM lane quarter it may read
+        const int r = lq * 32 + lane;
+        const int tid = threadIdx.x - 64, peer = NH == 2 ? (tid ^ 128) : tid;   // the other half's thread of this row
+        const int xb = g * 4 + lq;
+        float* qs = statbuf + (warp - 2) * MAXC;
+        // entries of a row: the lower half's upwards from slot 0, the upper half's downwards from slot NSEL + 1; a count
+        // stops at nsel + 1 (more than nsel in all is repeated below, whatever the slots hold then)
+        const uint32_t hit0 = smem_u32(hits) + (uint32_t)(g * 128 + r) * 8u;
+        const int c_begin = half ? ((p.S + 1) / 2 + 15) / 16 * 16 : 0;
+        const int c_end = NH == 2 && !half ? min(((p.S + 1) / 2 + 15) / 16 * 16, p.S) : p.S;
+        const uint32_t taddr = tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)g * MAXC;
+        if (p.sampled)                               // (every warp writes the same values)
+            for (int c = lane; c < MAXC; c += 32) cs[c] = c < p.S ? p.cand[c] : -1;
+        uint32_t use = 0, use_of_pair = 0;           // (a row block past the sequence takes no part in an exchange)
+        bool ok = true;
+        for (int unit = blockIdx.x + g * gridDim.x; unit < p.n_units && ok; unit += G * gridDim.x, ++use) {
+            const int bh = unit / p.n_row_tiles, rt = unit - bh * p.n_row_tiles;
+            const int row = rt * BM + r;
+            const bool row_ok = row < p.T;
+            const bool warp_live = rt * BM + lq * 32 < p.T;
+            const bool ranks = NH == 1 || (int)(use & 1u) == half;
+            float kst = 1.0f;
+            if (row_ok && p.metric != CONVNN_MATMUL) kst = p.kstat[(long long)bh * p.T + row];
+            const float sentinel = p.sampled ? self_sentinel(p.metric, kst, p.sqrt_dk) : 0.f;
+            __syncwarp();
+            if (p.metric != CONVNN_MATMUL) {
+                const float* qrow = p.qstat + (long long)bh * p.S;
+#pragma unroll
+                for (int c = 0; c < MAXC; c += 32) qs[c + lane] = c + lane < p.S ? qrow[c + lane] : 0.f;
+            }
+            __syncwarp();
+            ok = mbar_wait(&tfull[g], use & 1u, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) { if (lane == 0) fail(abort_flag, 74); break; }
+            tc_fence_after_sync();
+            bool exact = true;
+            int n_low = 0;
+            if (warp_live) {
+                float v[NSEL];
+#pragma unroll
+                for (int s = 0; s < NSEL; ++s) v[s] = -CUDART_INF_F;
+#pragma unroll 1
+                for (int c = c_begin; c < c_end; c += W) {
+                    uint32_t acc[W];
+                    tmem_ld(taddr + c, acc);
+                    tmem_ld_wait();
+                    float key[W];
+                    make_keys<W>(key, acc, qs, cs, c, p, row, sentinel);
+#pragma unroll
+                    for (int j = 0; j < W; j += 2) merge_pair<NSEL>(v, key[j], key[j + 1]);
+                }
+                float thr = v[0];                    // v[nsel - 1] = the smallest of the first nsel
+#pragma unroll
+                for (int s = 1; s < NSEL; ++s) thr = fminf(thr, s < p.nsel ? v[s] : CUDART_INF_F);
+                if (NH == 2) {
+#pragma unroll
+                    for (int s = 0; s < NSEL; ++s) lists[s * NT + tid] = v[s];
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&xlist[xb]);
+                    ok = mbar_wait(&xlist[xb], use_of_pair & 1u, abort_flag);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) { if (lane == 0) fail(abort_flag, 75); break; }
+                    thr = fmaxf(thr, lists[(p.nsel - 1) * NT + peer]);
+#pragma unroll
+                    for (int i = 0; i < NSEL - 1; ++i)
+                        if (i < p.nsel - 1) thr = fmaxf(thr, fminf(v[i], lists[(p.nsel - 2 - i) * NT + peer]));
+                }
+                int cnt = 0;
+                const uint32_t first = half ? hit0 + (NSEL + 1) * ENTRY : hit0;
+                uint32_t at = first;
+#pragma unroll 1
+                for (int c = c_begin; c < c_end; c += W) {
+                    uint32_t acc[W];
+                    tmem_ld(taddr + c, acc);
+                    tmem_ld_wait();
+                    float key[W];
+                    make_keys<W>(key, acc, qs, cs, c, p, row, sentinel);
+#pragma unroll
+                    for (int j = 0; j < W; ++j) {
+                        if (key[j] >= thr) {
+                            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(__float_as_uint(key[j])), "r"(c + j)
+                                         : "memory");
+                            at = half ? max(at - ENTRY, hit0 + (uint32_t)(NSEL - p.nsel) * ENTRY)
+                                      : min(at + ENTRY, hit0 + (uint32_t)(p.nsel + 1) * ENTRY);
+                        }
+                    }
+                }
+                cnt = (int)((half ? first - at : at - first) / ENTRY);
+                n_low = cnt;
+                if (NH == 2) {
+                    counts[tid] = cnt;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&xhits[xb]);
+                    if (ranks) {
+                        ok = mbar_wait(&xhits[xb], use_of_pair & 1u, abort_flag);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) { if (lane == 0) fail(abort_flag, 76); break; }
+                        const int other = counts[peer];
+                        n_low = half ? other : cnt;
+                        cnt += other;
+                    }
+                    ++use_of_pair;
+                }
+                if (ranks) {
+                    exact = !row_ok || (cnt == p.nsel && thr > -CUDART_INF_F);
+                    if (!__all_sync(0xffffffffu, exact)) {
+                        TopList<NSEL> top;
+                        top.init();
+#pragma unroll 1
+                        for (int c = 0; c < p.S; c += 16) {
+                            uint32_t acc[16];
+                            tmem_ld_x16(taddr + c, acc);
+                            tmem_ld_wait();
+                            float key[16];
+                            make_keys<16>(key, acc, qs, cs, c, p, row, sentinel);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) top.insert_sorted(key[j], c + j);
+                        }
+                        if (row_ok && !exact)
+                            write_selection<NSEL>(top, p, ((long long)bh * p.T + row) * p.K, row, kst);
+                    }
+                }
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty[g]);
+            if (ranks && row_ok && exact) {
+                const float2* e = hits + g * 128 + r;
+                // n-th entry in column order
+                auto entry = [&](int n) { return (NH == 1 || n < n_low ? n : NSEL + 1 + n_low - n) * 128 * G; };
+                float key[NSEL];
+                int slot[NSEL];
+#pragma unroll
+                for (int n = 0; n < NSEL; ++n) {
+                    key[n] = n < p.nsel ? e[entry(n)].x : -CUDART_INF_F;
+                    slot[n] = 0;
+                }
+#pragma unroll
+                for (int n = 1; n < NSEL; ++n)
+#pragma unroll
+                    for (int m = 0; m < n; ++m) {
+                        const int first = key[m] >= key[n] ? 1 : 0;
+                        slot[n] += first;
+                        slot[m] += 1 - first;
+                    }
+                long long obase = ((long long)bh * p.T + row) * p.K;
+                if (p.sampled) {
+                    p.idx[obase] = row;
+                    p.val[obase] = 1.0f;
+                    ++obase;
+                }
+#pragma unroll
+                for (int n = 0; n < NSEL; ++n) {
+                    if (n < p.nsel) {
+                        int tok = __float_as_int(e[entry(n)].y);
+                        float s;
+                        if (p.metric == CONVNN_COSINE) s = key[n] * kst;
+                        else if (p.metric == CONVNN_MATMUL) s = key[n] / p.sqrt_dk;
+                        else s = sqrtf(fmaxf(kst - key[n], 0.f));
+                        if (p.sampled) {
+                            tok = cs[tok];
+                            if (tok == row) s = (p.metric == CONVNN_EUCLIDEAN) ? 1.1f : -0.1f;
+                        }
+                        p.idx[obase + slot[n]] = tok;
+                        p.val[obase + slot[n]] = s;
+                    }
+                }
+            }
+        }
+    }
+
+    tc_fence_before_sync();
+    __syncthreads();
+    if (*abort_flag) {
+        // a wait expired: give copies still in flight time to land before the CTA's shared memory is released
+        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+        __syncthreads();
+    }
+    if (warp == 1) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem_base, 512);
+    }
+}
+
+template <int NSEL, int G, int NH>
+int launch_short(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const CUtensorMap& tmQ, cudaStream_t st) {
+    constexpr int MAXC = 512 / G;
+    const size_t stage = (size_t)(BM + p.BN) * p.KCH * 2;
+    constexpr int NT = 128 * G * NH;
+    const size_t fixed = 1024 + (size_t)(NSEL + 2) * 128 * G * 8 + (size_t)(NT / 32 + 1) * MAXC * 4 +
+                         (NH == 2 ? (size_t)(NSEL + 1) * NT * 4 : 0) + (2 * MAX_STAGES + 10 * G) * 8 + 16;
+    p.stages = (int)((226 * 1024 - fixed) / stage);
+    if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
+    if (p.stages > 2 * p.KC) p.stages = 2 * p.KC;            // deeper than two units' chunks serves nothing
+    size_t smem = fixed + p.stages * stage;
+    if (smem < 116 * 1024) smem = 116 * 1024;                // a CTA takes all of an SM's TMEM: never two on one SM
+    const int sms = device_sms();
+    auto kern = sim_topk_short_kernel<NSEL, G, NH>;
+    CONVNN_ENSURE_SMEM(kern, smem);
+    launch_chained(kern, p.n_units < sms ? p.n_units : sms, 64 + NT, smem, st, tmK, tmQ, p);
+    CONVNN_CHECK_LAUNCH("sim_topk_short");
+    return CONVNN_OK;
+}
+
+}  // namespace
+
+// Where the streaming kernel leaves most of the chip idle: up to one unit per SM.  B x 197 tokens of 192 channels, K = 9:
+// 15.4 us for 1 to 74 images, streaming 21.6; 256 images (3.5 units per SM) 34.6 against 30.8, where eight to sixteen
+// streaming warps per SM hide each other's latency.  Lists of 13 to 16 always: their streaming variant runs one CTA per SM
+// (577 tokens, 150 candidates, K = 16: 1 image 26.4 -> 18.5 us, 74 images 49.9 -> 39.8, 256 images 132 -> 107).
+bool sim_topk_short_wanted(const Dims& dm) {
+    const long long units = (long long)dm.B * dm.H * ((dm.T + BM - 1) / BM);
+    return dm.S <= 256 && (units <= device_sms() || (dm.nsel > 12 && dm.nsel <= 16));
+}
+
+int launch_sim_topk_short(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
+                          const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st) {
+    ShortParams p{};
+    p.qstat = qstat; p.kstat = kstat; p.cand = cand; p.idx = idx; p.val = val;
+    p.T = dm.T; p.S = dm.S; p.H = dm.H; p.K = dm.K; p.nsel = dm.nsel; p.metric = d->metric; p.sampled = d->sampled;
+    p.KCH = dm.Cp <= 16 ? 16 : (dm.Cp <= 32 ? 32 : 64);      // (the copies fill what lies past a head with zeros)
+    p.KC = (dm.Cp + p.KCH - 1) / p.KCH;
+    p.BN = (dm.S + 15) / 16 * 16;
+    p.n_row_tiles = (dm.T + BM - 1) / BM;
+    p.n_units = dm.B * dm.H * p.n_row_tiles;
+    p.sqrt_dk = (float)sqrt((double)dm.dk);
+
+    CUtensorMap tmK, tmQ;
+    const uint64_t dimsK[4] = {(uint64_t)dm.Cp, (uint64_t)dm.H, (uint64_t)dm.T, (uint64_t)dm.B};
+    const uint64_t dimsQ[4] = {(uint64_t)dm.Cp, (uint64_t)dm.H, (uint64_t)dm.S, (uint64_t)dm.B};
+    const uint64_t strK[3] = {(uint64_t)dm.Cp * 2, (uint64_t)dm.H * dm.Cp * 2, (uint64_t)dm.T * dm.H * dm.Cp * 2};
+    const uint64_t strQ[3] = {(uint64_t)dm.Cp * 2, (uint64_t)dm.H * dm.Cp * 2, (uint64_t)dm.S * dm.H * dm.Cp * 2};
+    const uint32_t boxK[4] = {(uint32_t)p.KCH, 1, (uint32_t)BM, 1};
+    const uint32_t boxQ[4] = {(uint32_t)p.KCH, 1, (uint32_t)p.BN, 1};
+    if (!encode_tensor_map_bf16(&tmK, k, 4, dimsK, strK, boxK, p.KCH * 2)) return CONVNN_E_CUDA;
+    if (!encode_tensor_map_bf16(&tmQ, q, 4, dimsQ, strQ, boxQ, p.KCH * 2)) return CONVNN_E_CUDA;
+
+    const int n = dm.nsel;
+#define CONVNN_SHORT(N)                                                     \
+    do {                                                                    \
+        if (dm.S <= 128) return launch_short<N, 4, 1>(dm, p, tmK, tmQ, st);    \
+        return launch_short<N, 2, 2>(dm, p, tmK, tmQ, st);                     \
+    } while (0)
+    if (n <= 4) CONVNN_SHORT(4);
+    if (n <= 8) CONVNN_SHORT(8);
+    if (n == 9) CONVNN_SHORT(9);
+    if (n <= 12) CONVNN_SHORT(12);
+    if (n <= 16) CONVNN_SHORT(16);
+    // (longer lists: their exchange buffers would take the ring's shared memory)
+    if (n <= 25) return launch_short<25, 2, 1>(dm, p, tmK, tmQ, st);
+    return launch_short<32, 2, 1>(dm, p, tmK, tmQ, st);
+#undef CONVNN_SHORT
+}
+
+int read_sim_short_status(int* out) {
+    int v = 0;
+    cudaError_t e = cudaMemcpyFromSymbol(&v, g_sim_short_status, sizeof(int));
+    if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaMemcpyFromSymbol: %s", cudaGetErrorString(e));
+    *out = v;
+    return CONVNN_OK;
+}
+
+}  // namespace convnn

@@ -1,0 +1,79 @@
+"""Two-pass selection over at most 256 candidates: integer-valued q and k make every similarity exact in float32, so lists,
+their order and the tie rule (lower column first) are compared exactly with a stable sort, ties and NaN included."""
+import math
+
+import pytest
+import torch
+
+from convnn_b200 import ops
+from gpu_util import DEV
+
+pytestmark = pytest.mark.gpu
+
+
+def expect(key, n):
+    """(rows, S) float32 keys -> the n best columns, ties by column; NaN and -inf are never picked, empty slots hold 0 / -inf."""
+    usable = ~key.isnan() & (key > -math.inf)
+    ranked = torch.where(usable, key, torch.full_like(key, -math.inf))
+    order = torch.sort(ranked, dim=-1, descending=True, stable=True)
+    idx = torch.where(order.values[..., :n] > -math.inf, order.indices[..., :n], torch.zeros_like(order.indices[..., :n]))
+    return idx, order.values[..., :n]
+
+
+@pytest.mark.parametrize("T,S,H,dk", [(1, 1, 1, 8), (5, 5, 2, 16), (33, 17, 1, 32), (129, 32, 3, 24), (65, 65, 1, 64), (97, 96, 1, 200),
+                                      (300, 127, 1, 64), (128, 128, 2, 32), (129, 129, 1, 64), (197, 197, 3, 64), (197, 197, 1, 192),
+                                      (577, 150, 1, 384), (255, 255, 1, 48), (256, 256, 1, 768), (700, 256, 2, 32)])
+@pytest.mark.parametrize("K", [1, 4, 5, 9, 11, 16, 24, 25, 32])
+@pytest.mark.parametrize("values", ["few", "many", "nan"])
+def test_exact_lists(T, S, H, dk, K, values):
+    sampled = S != T
+    n = K - 1 if sampled else K
+    if n < 1 or n > S:
+        pytest.skip("list longer than the candidates")
+    g = torch.Generator().manual_seed(T * 1000 + S + K)
+    B = 3
+    top = 1 if values == "few" else 11               # products and sums stay far below 2^24
+    q, k = (torch.randint(-top, top + 1, (B, r, H, dk), generator=g).float() for r in (S, T))
+    if values == "nan":
+        q[:, ::3] = math.nan                          # a third of the candidates
+        q[1, 2:] = math.nan                           # one image with two candidates left
+    spec = ops.LayerSpec(H * dk, H, K, "spatial" if sampled else "all", "matmul", "depthwise", True, False, T)
+    cand = torch.randperm(T, generator=g)[:S].to(torch.int32) if sampled else None
+    idx, val = ops.sim_topk(spec, q.bfloat16().to(DEV), k.bfloat16().to(DEV), None, None, None if cand is None else cand.to(DEV))
+    key = torch.einsum("bthc,bshc->bhts", k, q)
+    if sampled:
+        own = cand.view(1, 1, 1, S).long() == torch.arange(T).view(1, 1, T, 1)
+        key = torch.where(own, torch.full_like(key, -0.1) * torch.tensor(math.sqrt(dk), dtype=torch.float32), key)
+    want_idx, want_key = expect(key, n)
+    want_tok = want_idx if cand is None else cand.long()[want_idx]
+    got_idx, got_val = idx.long().cpu()[..., K - n:], val.cpu()[..., K - n:]
+    assert torch.equal(got_idx, want_tok)
+    real = want_key > -math.inf
+    if sampled:
+        assert torch.equal(idx.long().cpu()[..., 0], torch.arange(T).expand(B, H, T))
+        assert bool((got_val[(want_tok == torch.arange(T).view(1, 1, T, 1)) & real] == -0.1).all())
+        real &= want_tok != torch.arange(T).view(1, 1, T, 1)
+    want_val = want_key / torch.tensor(math.sqrt(dk), dtype=torch.float32)
+    # one division: equal up to its rounding
+    assert float(((got_val - want_val)[real].abs() / want_val[real].abs().clamp_min(1e-30)).max() if real.any() else 0.0) <= 2.0 ** -22
+
+
+@pytest.mark.parametrize("metric", ["cosine", "euclidean"])
+def test_metrics_at_the_ends(metric):
+    B, T, dk = 2, 197, 192
+    g = torch.Generator(device=DEV).manual_seed(3)
+    q, k = (torch.randn(B, T, 1, dk, device=DEV, generator=g).bfloat16() for _ in range(2))
+    n2 = [t.float().pow(2).sum(-1).permute(0, 2, 1).contiguous() for t in (q, k)]
+    qs, ks = [t.rsqrt() for t in n2] if metric == "cosine" else n2
+    spec = ops.LayerSpec(dk, 1, 9, "all", metric, "depthwise", True, False, T)
+    idx, val = ops.sim_topk(spec, q, k, qs, ks)
+    dot = torch.einsum("bthc,bshc->bhts", k.double(), q.double())
+    if metric == "cosine":
+        sim, sign = dot * ks.double().unsqueeze(-1) * qs.double().unsqueeze(2), 1.0
+    else:
+        sim, sign = (ks.double().unsqueeze(-1) + qs.double().unsqueeze(2) - 2 * dot).clamp_min(0).sqrt(), -1.0
+    want = sign * (sign * sim).topk(9, -1).values
+    # a dk-term fp32 sum of values whose squares add up to ~dk, relative to the distance / to 1
+    bound = (dk + 16) * 2.0 ** -24 * (1.0 if metric == "cosine" else 4.0 * math.sqrt(dk))
+    assert float((val.double() - want).abs().max()) <= bound
+    assert float((torch.gather(sim, -1, idx.long()) - val.double()).abs().max()) <= bound
