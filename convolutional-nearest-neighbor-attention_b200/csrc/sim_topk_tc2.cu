@@ -291,7 +291,7 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 bool sim_topk_tc2_wanted(const convnn_desc* d, const Dims& dm) {
     static const int env = [] { const char* e = getenv("CONVNN_B200_SIM_PAIR"); return e ? atoi(e) : -1; }();
     if (env == 0) return false;
-    if (d->dtype != CONVNN_BF16 || dm.Cp % 8 != 0 || dm.Cp < 96) return false;   // (a last chunk is zero-filled past the head)
+    if (d->dtype != CONVNN_BF16 || dm.Cp % 16 != 0 || dm.Cp < 96) return false;   // (a last chunk is zero-filled past the head)
     // Lists longer than 16 double the cost of keeping two lists per row; measured break-even
     // is at many units per cluster and a few thousand candidates.
     if (dm.nsel > 16) return dm.T >= 8192 && dm.S >= 4096;

@@ -1,5 +1,5 @@
-"""Tensor-core similarity at head widths that do not fill their 64-channel chunks (zero-filled by the copies), with and
-without the coordinate channel's padding: lists against float64 on the same bfloat16 q and k."""
+"""Similarity of bfloat16 heads at widths that do not fill the tensor-core kernels' 64-channel chunks (zero-filled by the
+copies) or are no multiple of sixteen (fp32 pipes): lists against float64 on the same bfloat16 q and k."""
 import pytest
 import torch
 
@@ -40,3 +40,22 @@ def test_lists(T, S, H, dk, coord, K):
     col = got if cand is None else got // (T // S)
     picked = torch.gather(sim, -1, col)
     assert float((picked - val[..., K - n:].double()).abs().max()) <= (C + 16) * EPS      # values belong to their indices
+
+
+@pytest.mark.parametrize("T,S,H,dk", [(577, 150, 1, 384), (197, 197, 3, 64), (130, 33, 1, 768), (1100, 1100, 1, 192), (65, 65, 2, 16)])
+@pytest.mark.parametrize("metric", ["cosine", "matmul", "euclidean"])
+def test_coordinate_channel_keeps_the_fp32_sums(T, S, H, dk, metric):
+    """Products of bfloat16 values are exact in float32, so the sums over the stored channels have to be those of the
+    float32 path on the same values, bit for bit."""
+    g = torch.Generator(device=DEV).manual_seed(T + dk)
+    K, C = 9, dk + 1
+    spec = ops.LayerSpec(H * dk, H, K, "all" if S == T else "spatial", metric, "standard", True, True, T)
+    q, k = (torch.zeros(2, n, H, (C + 7) // 8 * 8, device=DEV) for n in (S, T))
+    q[..., :C] = torch.randn(2, S, H, C, device=DEV, generator=g)
+    k[..., :C] = torch.randn(2, T, H, C, device=DEV, generator=g)
+    q, k = q.to(torch.bfloat16), k.to(torch.bfloat16)
+    n2 = [t.float().pow(2).sum(-1).permute(0, 2, 1).contiguous() for t in (q, k)]
+    qs, ks = [t.rsqrt() for t in n2] if metric == "cosine" else n2
+    cand = None if S == T else torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32)
+    got, want = (ops.sim_topk(spec, a, b, qs, ks, cand) for a, b in ((q, k), (q.float(), k.float())))
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
