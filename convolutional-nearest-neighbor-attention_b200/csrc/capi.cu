@@ -320,29 +320,17 @@ int qkv_proj_impl(const convnn_desc* d, const void* x, int64_t ldx, const void* 
         }
     }
     if (pn) return set_error(CONVNN_E_UNSUPPORTED, "prenorm_forward: this descriptor takes the unfused path");
-    // bfloat16 with the coordinate channel: v comes from the tensor cores, stored into rows of padded heads.  k and q decide
-    // the neighbour order, and a value that rounds the other way under another order of summation can swap two of them
-    // (up to 2e-2 of the output norm at 197 tokens x 64 channels), so they keep the order of the SIMT kernel.
-    // Layer of 7 x 577 x 384, 150 candidates: 250 -> 223 us (all three on the tensor cores: 146).
-    const bool v_tc = d->dtype == CONVNN_BF16 && d->coord && dm.dk % 8 == 0 && !force_simt() &&
-                      gemm_tc_supported(x, ldx, static_cast<const char*>(w_qkv) + wsz, dm.D, dm.D, 1, &v, (int64_t)dm.H * dm.Cp);
     GemmParams p{};
     p.a = x; p.lda = ldx; p.bias = nullptr; p.N = dm.D; p.Kd = dm.D;
     p.a_mode = A_TOKENS; p.c_mode = C_HEADS; p.T = dm.T; p.H = dm.H; p.dk = dm.dk; p.Cp = dm.Cp; p.gelu = 0;
     // keys and values: every token; queries: candidate tokens only (with sampling 'all' one launch makes all three)
-    const int parts = v_tc ? 1 : (d->sampled ? 2 : 3);
+    const int parts = d->sampled ? 2 : 3;
     p.rows_per_batch = dm.T; p.M = dm.B * dm.T; p.N = parts * dm.D; p.part_cols = dm.D;
-    p.w = w_qkv; p.c = k; p.c1 = v_tc ? nullptr : v; p.c2 = parts == 3 ? q : nullptr;
+    p.w = w_qkv; p.c = k; p.c1 = v; p.c2 = d->sampled ? nullptr : q;
     if ((rc = launch_gemm_simt(d->dtype, p, st))) return rc;
-    if (v_tc) {
-        GemmTcOpts o;
-        o.dk = dm.dk; o.heads = dm.H; o.head_pad = dm.Cp - dm.dk;
-        if ((rc = launch_gemm_tc(x, ldx, static_cast<const char*>(w_qkv) + wsz, dm.B * dm.T, dm.D, dm.D, 1, &v,
-                                 (int64_t)dm.H * dm.Cp, o, st))) return rc;
-    }
-    if (parts != 3) {
-        if (d->sampled) { p.cand = cand; p.rows_per_batch = dm.S; p.M = dm.B * dm.S; }
-        p.N = dm.D; p.w = static_cast<const char*>(w_qkv) + 2 * wsz; p.c = q; p.c1 = nullptr;
+    if (d->sampled) {
+        p.cand = cand; p.rows_per_batch = dm.S; p.M = dm.B * dm.S; p.N = dm.D;
+        p.w = static_cast<const char*>(w_qkv) + 2 * wsz; p.c = q; p.c1 = nullptr;
         if ((rc = launch_gemm_simt(d->dtype, p, st))) return rc;
     }
     if ((rc = launch_head_fill_and_stats(d, dm, q, dm.S, stats ? qstat : nullptr, st))) return rc;

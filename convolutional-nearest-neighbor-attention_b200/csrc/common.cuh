@@ -190,7 +190,6 @@ struct GemmTcOpts {
     long long ldr = 0;
     int gelu = 0;
     float* stat[3] = {nullptr, nullptr, nullptr};   // per part: fused per-(row, head) statistic
-    int head_pad = 0;   // elements between the heads of an output row (ldc counts them; dk and head_pad multiples of eight)
     int stat_mode = 0, dk = 0, heads = 1, rows_per_batch = 1;
     // heads wider than a tile: room for gemm_tc_stat_pieces() x M x heads floats per part with a
     // statistic (the tiles' partial sums, combined by a second small kernel)

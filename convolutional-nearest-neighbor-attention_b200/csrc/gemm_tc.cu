@@ -84,7 +84,6 @@ struct GemmTcParams {
     int ln_planes;
     float ln_eps, ln_inv_k;
     float2* moments_out;   // MOM: [2 * n_n_tiles][mom_ld] partial moments of the stored rows
-    int head_pad;          // unused elements between the heads of an output row (dk % 8 == 0)
     long long mom_ld;      // plane stride of moments_out (M rounded up to an even count)
 };
 
@@ -585,9 +584,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
                 __syncwarp();
                 // phase B: 8 rows x 64 bytes per instruction, coalesced
-                int cpos = c;
-                if constexpr (!RES && !LNF)
-                    if (p.head_pad) cpos += (pc0 + (lane & 3) * 8 + c) / p.dk * p.head_pad;
                 const bool cok = c + (lane & 3) * 8 < ncol;
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {
@@ -614,7 +610,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                 mo2[g] = fmaf(hi, hi, fmaf(lo, lo, mo2[g]));
                             }
                         }
-                        *reinterpret_cast<uint4*>(optr[g] + cpos) = v;
+                        *reinterpret_cast<uint4*>(optr[g] + c) = v;
                     }
                 }
                 __syncwarp();
@@ -806,9 +802,6 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
     p.stat_mode = o.stat_mode; p.dk = o.dk > 0 ? o.dk : 32; p.heads = o.heads; p.rows_per_batch = o.rows_per_batch > 0 ? o.rows_per_batch : 1;
     p.M = M; p.N = N;
     p.part_cols = N / parts;
-    p.head_pad = o.head_pad;
-    if (o.head_pad && (o.residual || o.ln_moments || o.moments_out || p.dk % 8 != 0 || o.head_pad % 8 != 0))
-        return set_error(CONVNN_E_UNSUPPORTED, "gemm_tc: padded heads come from the plain epilogue, eight channels at a time");
     p.KCH = Kd % 64 == 0 ? 64 : (Kd % 32 == 0 ? 32 : 16);
     p.KC = Kd / p.KCH;
     p.BN = tile_width(N, parts, o.stat[0] != nullptr);

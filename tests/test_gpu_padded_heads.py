@@ -1,4 +1,4 @@
-"""Values stored into rows of padded heads by the tensor-core GEMM (bfloat16, coordinate channel)."""
+"""Values stored into rows of padded heads (bfloat16, coordinate channel)."""
 import pytest
 import torch
 
@@ -26,3 +26,17 @@ def test_values(H, dk, B, T):
     assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + D * 2.0 ** -24 * s).all())
     line = torch.linspace(-1, 1, T).bfloat16().to(DEV).view(1, T, 1).expand(B, T, H)
     assert torch.equal(v[..., dk], line) and not bool(v[..., dk + 1:].any())
+
+
+@pytest.mark.parametrize("H,dk", [(1, 384), (3, 64), (2, 24), (1, 768)])
+def test_projections_keep_the_fp32_sums(H, dk):
+    """Products of bfloat16 values are exact in float32: k, v and q are the float32 path's sums, rounded once."""
+    g = torch.Generator(device=DEV).manual_seed(H * 100 + dk)
+    D, T = H * dk, 577
+    w = [(torch.randn(D, D, device=DEV, generator=g) / D ** 0.5).bfloat16() for _ in range(4)]
+    x = torch.randn(4, T, D, device=DEV, generator=g).bfloat16()
+    spec = ops.LayerSpec(D, H, 1, "all", "matmul", "standard", True, True, T)
+    packed = ops.pack_weights(spec, *w, (torch.zeros(dk, dk + 1, 1, device=DEV),), torch.bfloat16, torch.device(DEV))[0]
+    got, want = ops.qkv_proj(spec, x, packed)[:3], ops.qkv_proj(spec, x.float(), packed.float())[:3]
+    for a, b in zip(got, want):
+        assert torch.equal(a[..., :dk], b[..., :dk].bfloat16())
