@@ -54,8 +54,8 @@ class _NotCopied(dict):
 
 class _LayerCall:
     """What one ConvNN layer call of a given input shape needs besides its tensors, prepared once: descriptor, packed
-    weights, candidate indices in the kernels' type, workspace size (27 us of host time per call before, 10 with it;
-    a small layer's kernels take 30)."""
+    weights, workspace size (27 us of host time per call before, 10 with it; a small layer's kernels take 30).
+    Candidates are not part of it (``kernel_candidates``): a captured graph would read them after this object is gone."""
 
     def __init__(self, layer, x):
         B, T, _ = x.shape
@@ -64,27 +64,22 @@ class _LayerCall:
         self.slots = [(m._parameters, k) for m in mods for k in m._parameters]
         params = [d[k] for d, k in self.slots]
         self.ids = [id(p) for p in params]
-        self.cand, self.draw, spec = None, None, layer._spec()
-        if layer.sampling_type == "random" and layer.candidate_override is None:
-            self.draw, S = layer, len(range(T)[:layer.num_samples])     # drawn anew on every call
-        else:
-            self.cand, S = ops._cand_arg(spec, layer.candidates(T, x.device), T, x.device)
-        if layer.candidate_override is not None:
-            params.append(layer.candidate_override)
+        self.S = layer.candidate_count(T, x.device)
         self.params = [p for p in params if p is not None]
         self.versions = [p._version for p in self.params]
         self.ptrs = [p.data_ptr() for p in self.params]
         self.packed = layer.packed_weights(x.dtype, x.device)
-        self.call = ops.LayerForward(spec, B, T, S, x.dtype, x.device, self.packed)
+        self.call = ops.LayerForward(layer._spec(), B, T, self.S, x.dtype, x.device, self.packed)
 
     def unchanged(self):
         return (self.epoch == _epoch[0] and [id(d[k]) for d, k in self.slots if k in d] == self.ids and
                 [p._version for p in self.params] == self.versions and [p.data_ptr() for p in self.params] == self.ptrs)
 
-    def __call__(self, x, out, residual):
-        cand = self.cand
-        if self.draw is not None:
-            cand = self.draw.candidates(x.shape[1], x.device).to(torch.int32)
+    def __call__(self, layer, x, out, residual):
+        """``layer(x)``; None: the candidate set has another size now."""
+        cand = layer.kernel_candidates(x.shape[1], x.device)
+        if cand is not None and cand.numel() != self.S:
+            return None
         return self.call(x, cand, out, residual)
 
 
@@ -192,6 +187,34 @@ class MultiHeadConvNNAttention(WatchedModule):
             return self._spatial_cache[key]
         raise ValueError("Invalid sampling_type. Must be one of ['all', 'random', 'spatial']")
 
+    def kernel_candidates(self, T: int, device) -> Optional[torch.Tensor]:
+        """``candidates`` as the kernels read them (int32), converted by every call on its own stream: a set that is
+        changed in place is followed, and a captured graph holds the conversion and its memory.  The set of 'spatial' never
+        changes: it is converted once, kept as long as the layer, and complete before any stream can see it."""
+        cand = self.candidates(T, device)
+        if cand is None:
+            return None
+        key = (T, str(device))
+        if cand is not self._spatial_cache.get(key):
+            return cand.to(device=device, dtype=torch.int32).contiguous()
+        key += (torch.int32,)
+        kept = self._spatial_cache.get(key)
+        if kept is None:
+            kept = cand.to(torch.int32)
+            if kept.is_cuda:
+                if torch.cuda.is_current_stream_capturing():
+                    return kept                       # (recorded, not written yet)
+                torch.cuda.current_stream(kept.device).synchronize()
+            self._spatial_cache[key] = kept
+        return kept
+
+    def candidate_count(self, T: int, device) -> int:
+        """S of a call over T tokens (without a draw)."""
+        if self.sampling_type == 'random' and self._candidate_override is None:
+            return len(range(T)[:self.num_samples])
+        cand = self.candidates(T, device)
+        return T if cand is None else cand.numel()
+
     def _check_mode(self, x):
         if not x.is_cuda:
             raise RuntimeError("convnn_b200.MultiHeadConvNNAttention runs on CUDA (sm_100a) only; "
@@ -217,11 +240,14 @@ class MultiHeadConvNNAttention(WatchedModule):
             return ops.forward(self._spec(), x, packed, cand, out=out, residual=residual)
         key = (x.shape, x.dtype, x.device)
         call = self._calls.get(key)
-        if call is None or not call.unchanged():
-            if len(self._calls) >= 16:
-                self._calls.clear()
-            call = self._calls[key] = _LayerCall(self, x)
-        return call(x, out, residual)
+        if call is not None and call.unchanged():
+            y = call(self, x, out, residual)
+            if y is not None:
+                return y
+        if len(self._calls) >= 16:
+            self._calls.clear()
+        call = self._calls[key] = _LayerCall(self, x)
+        return call(self, x, out, residual)
 
     def prenorm_supported(self, x) -> bool:
         """Whether ``forward_prenorm`` takes this input (bfloat16, sampling 'all', a K/V/Q weight tile

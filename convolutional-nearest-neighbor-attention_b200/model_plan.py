@@ -3,7 +3,8 @@
 A ViT-Tiny forward is 52 launches; issued one binding call at a time they cost the host 1.14 ms (measured, one
 image), most of it argument handling and shape logic between the calls, so batches below ~100 images ran at the
 host's pace.  A plan holds the model's weight pointers, packed copies, layer descriptors and workspace size for
-one input shape; a forward then is a validity check, two allocations and one native call.
+one input shape; a forward then is a validity check, two allocations and one native call.  Candidate sets are not
+part of it but taken from the layers on every call: a captured graph would read a plan's copy after the plan is gone.
 
 A plan is used only while it describes the model: ``Watch.unchanged()`` compares the attribute epoch of this package's
 modules, the module tree, and identity, version counter and address of every parameter and buffer, and a call
@@ -53,16 +54,14 @@ class Watch:
                     if t is not None:
                         self.tensors.append(t)
         self.ids = [id(d[k]) for d, k in self.slots]
-        self.inputs = self.tensors + [m.candidate_override for m in self.mods if isinstance(m, MultiHeadConvNNAttention)
-                                      and m.candidate_override is not None]
-        self.versions = [t._version for t in self.inputs]
-        self.ptrs = [t.data_ptr() for t in self.inputs]
+        self.versions = [t._version for t in self.tensors]
+        self.ptrs = [t.data_ptr() for t in self.tensors]
 
     def unchanged(self) -> bool:
         return (self.epoch == layers.attribute_epoch() and
                 [id(d[k]) for d, k in self.slots if k in d] == self.ids and
-                [t._version for t in self.inputs] == self.versions and
-                [t.data_ptr() for t in self.inputs] == self.ptrs and
+                [t._version for t in self.tensors] == self.versions and
+                [t.data_ptr() for t in self.tensors] == self.ptrs and
                 all([d == c for d, c in self.trees]) and not any(self.hooks))
 
 
@@ -73,7 +72,7 @@ class Plan:
         T, D = model.n_patches + 1, model.d_hidden
         self.watch = watch
         self.keep = []              # tensors whose addresses the structs hold
-        self.random = []            # (block index, attention layer): candidates drawn on every call
+        self.sampled = []           # (block index, attention layer, candidates the plan was made for)
         blocks = list(model.transformer_encoder)
         self.blocks = (_capi.ConvnnBlock * max(1, len(blocks)))()
         for i, blk in enumerate(blocks):
@@ -114,15 +113,11 @@ class Plan:
         setattr(b, names[1], self._ptr(wx))
 
     def _layer(self, b, i, att, B, T, act, device):
-        """The ConvNN layer of a block: descriptor, packed weights, candidates."""
-        cand, S, spec = None, T, att._spec()
-        if att.sampling_type == "random" and att.candidate_override is None:
-            self.random.append((i, att))
-            S = len(range(T)[:att.num_samples])
-        else:
-            cand, S = ops._cand_arg(spec, att.candidates(T, device), T, device)
-        b.layer = ops.descriptor(spec, B, T, S, act)
-        b.cand = self._ptr(cand)
+        """The ConvNN layer of a block: descriptor, packed weights."""
+        S = att.candidate_count(T, device)
+        if att.sampling_type != "all":
+            self.sampled.append((i, att, S))
+        b.layer = ops.descriptor(att._spec(), B, T, S, act)
         w_qkv, w_conv, w_pw, w_o = att.packed_weights(act, device)
         b.w_qkv, b.w_conv, b.w_pw, b.w_o = (self._ptr(w) for w in (w_qkv, w_conv, w_pw, w_o))
 
@@ -151,18 +146,35 @@ class Plan:
             b.pointwise_w, b.pointwise_b = self._ptr(att.pointwise_linear.weight), self._ptr(att.pointwise_linear.bias)
 
     # -- a forward ----------------------------------------------------------------------------------
-    def run(self, x: torch.Tensor) -> torch.Tensor:
+    def _candidates(self, device):
+        """This call's candidate sets, one per sampled layer in the order of the layers (a set that several layers share
+        is converted once); None: one has another size now."""
+        shared, sets = {}, []
+        for _, att, S in self.sampled:
+            override = att.candidate_override
+            cand = None if override is None else shared.get(id(override))
+            if cand is None:
+                cand = att.kernel_candidates(self.model.T, device)
+                shared[id(override)] = cand
+            if cand.numel() != S:
+                return None
+            sets.append(cand)
+        return sets
+
+    def run(self, x: torch.Tensor):
+        """The logits; None where the plan does not describe the call any more."""
         if not x.is_contiguous():
             x = x.contiguous()
         dev = x.device
         out = torch.empty(self.out_shape, dtype=self.act, device=dev)
         ws = torch.empty(self.workspace_bytes, dtype=torch.uint8, device=dev)
         args = (self.arg, x.data_ptr(), out.data_ptr(), ws.data_ptr(), self.workspace_bytes, ops._stream(x))
-        if self.random:
-            # drawn per layer and call, in the order of the layers; the lock keeps the structs this call's until it returns
-            drawn = [att.candidates(self.model.T, dev).to(torch.int32) for _, att in self.random]
-            with self.lock:
-                for (i, _), cand in zip(self.random, drawn):
+        if self.sampled:
+            sets = self._candidates(dev)
+            if sets is None:
+                return None
+            with self.lock:          # the structs are this call's until it returns
+                for (i, _, _), cand in zip(self.sampled, sets):
                     self.blocks[i].cand = cand.data_ptr()
                 rc = self.call(*args)
         else:
@@ -214,7 +226,9 @@ def run(model, x: torch.Tensor):
     key = (x.shape, x.dtype, x.device)
     plan = per_model.get(key)
     if plan is not None and plan is not _SEEN and plan.watch.unchanged():
-        return plan.run(x) if type(plan) is Plan else None
+        y = plan.run(x) if type(plan) is Plan else None
+        if y is not None or type(plan) is not Plan:
+            return y
     # The first call of a shape, and the first after a change of the model, goes op by op: it packs weights while
     # the GPU works, and a shape that never returns pays for no plan.  The second call builds the plan.
     if plan is not _SEEN:

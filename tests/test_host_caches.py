@@ -1,0 +1,116 @@
+"""What the host side keeps between forwards (the ViT's host plan, the layers' prepared calls), on CPU tensors: the
+native entry points are replaced by recorders of what they are handed."""
+import ctypes
+import types
+
+import numpy as np
+import pytest
+import torch
+
+import convnn_b200
+from convnn_b200 import _capi, layers, model_plan, ops
+
+
+def _ints(pointer, n):
+    return list((ctypes.c_int32 * n).from_address(pointer)) if pointer else None
+
+
+@pytest.fixture
+def host(monkeypatch):
+    """The host path on CPU; ``host.models`` / ``host.layers`` list the recorded native calls."""
+    rec = types.SimpleNamespace(models=[], layers=[], general=[])
+    lib = _capi.lib()
+
+    def model_forward(arg, images, logits, workspace, nbytes, stream):
+        m = arg._obj
+        rec.models.append(types.SimpleNamespace(
+            embed_eps=m.embed_eps, eps=[(b.eps1, b.eps2) for b in m.blocks[:m.n_blocks]],
+            cand=[_ints(b.cand, b.layer.S) if b.layer.sampled else None for b in m.blocks[:m.n_blocks]],
+            cand_ptr=[b.cand for b in m.blocks[:m.n_blocks]], pixel_mean=m.pixel_mean))
+        return 0
+
+    def layer_forward(d, x, ldx, w_qkv, w_conv, w_pw, w_o, cand, *rest):
+        rec.layers.append(types.SimpleNamespace(cand=_ints(cand, d.S) if d.sampled else None, w_pw=w_pw, w_conv=w_conv,
+                                                ldo=rest[3], K=d.K))
+        return 0
+    monkeypatch.setattr(lib, "convnn_b200_model_forward", model_forward)
+    monkeypatch.setattr(lib, "convnn_b200_forward", layer_forward)
+    monkeypatch.setattr(ops, "_stream", lambda t: 0)
+    monkeypatch.setattr(ops, "_require_cuda", lambda *t: None)
+    monkeypatch.setattr(layers.MultiHeadConvNNAttention, "_check_mode", lambda self, x: None)
+    return rec
+
+
+def _vit(**kw):
+    args = dict(img_size=(3, 32, 32), patch_size=8, num_layers=2, num_heads=1, d_hidden=16, d_mlp=32, num_classes=5, K=3,
+                magnitude_type="cosine", dropout=0.0, attention_dropout=0.0, device="cpu")
+    args.update(kw)
+    return convnn_b200.ViT(convnn_b200.make_args(**args)).eval()
+
+
+def _layer(*, K=3, conv="depthwise", sampling="all", samples=-1):
+    return convnn_b200.MultiHeadConvNNAttention(16, 1, 0.0, K, sampling, samples, 0, "cosine", convolution_type=conv).eval()
+
+
+def _images(B=2):
+    return torch.randn(B, 3, 32, 32)
+
+
+@torch.no_grad()
+def test_plan_takes_the_candidates_of_each_call(host):
+    m, x = _vit(sampling_type="random", num_samples=6), _images()
+    numbers = np.arange(6)
+    m.set_candidates(torch.from_numpy(numbers))
+    for _ in range(3):
+        model_plan.run(m, x)
+    assert host.models[-1].cand == [list(range(6))] * 2
+    numbers += 7                                  # in place, where no version counter sees it
+    model_plan.run(m, x)
+    assert host.models[-1].cand == [list(range(7, 13))] * 2
+
+
+@torch.no_grad()
+def test_layer_call_takes_the_candidates_of_each_call(host):
+    m, x = _layer(sampling="random", samples=6), torch.randn(2, 17, 16)
+    numbers = np.arange(6)
+    m.candidate_override = torch.from_numpy(numbers)
+    for _ in range(3):
+        m(x)
+    numbers += 7
+    m(x)
+    assert host.layers[-1].cand == list(range(7, 13))
+
+
+@torch.no_grad()
+def test_candidates_of_another_size(host):
+    m, x = _vit(sampling_type="random", num_samples=6), _images()
+    cand = torch.arange(6)
+    m.set_candidates(cand)
+    for _ in range(2):
+        model_plan.run(m, x)
+    cand.set_(torch.arange(9))
+    for _ in range(3):                            # op by op, noticed, planned again
+        model_plan.run(m, x)
+    assert host.models[-1].cand == [list(range(9))] * 2
+    lay = _layer(sampling="random", samples=6)
+    lay.candidate_override = cand = torch.arange(6)
+    lx = torch.randn(2, 17, 16)
+    for _ in range(2):
+        lay(lx)
+    cand.set_(torch.arange(9))
+    lay(lx)
+    assert host.layers[-1].cand == list(range(9))
+
+
+@torch.no_grad()
+def test_spatial_candidates_belong_to_the_layer(host):
+    m, x = _vit(sampling_type="spatial", num_samples=5), _images()
+    for _ in range(2):
+        model_plan.run(m, x)
+    want = torch.linspace(0, 16, 5).long().tolist()
+    assert host.models[-1].cand == [want] * 2
+    before = host.models[-1].cand_ptr
+    model_plan._plans.pop(m)                       # a captured graph outlives the plan it was captured with
+    for _ in range(2):
+        model_plan.run(m, x)
+    assert host.models[-1].cand_ptr == before
