@@ -42,6 +42,12 @@ class WatchedModule(nn.Module):
         super().__delattr__(name)
 
 
+def capturing(device) -> bool:
+    """Whether work on a CUDA ``device`` is being recorded into a graph.  What such work writes does not exist before the
+    first replay, so nothing prepared in it is kept for later calls."""
+    return device.type == "cuda" and torch.cuda.is_current_stream_capturing()
+
+
 class _NotCopied(dict):
     """A cache that copies and pickles of its owner start without."""
 
@@ -181,10 +187,13 @@ class MultiHeadConvNNAttention(WatchedModule):
             return torch.randperm(T, device=device)[:self.num_samples]
         if self.sampling_type == 'spatial':
             key = (T, str(device))
-            if key not in self._spatial_cache:
-                self._spatial_cache[key] = torch.linspace(
-                    0 + self.sample_padding, T - self.sample_padding - 1, self.num_samples, device=device).long()
-            return self._spatial_cache[key]
+            kept = self._spatial_cache.get(key)
+            if kept is None:
+                kept = torch.linspace(0 + self.sample_padding, T - self.sample_padding - 1, self.num_samples,
+                                      device=device).long()
+                if not capturing(kept.device):
+                    self._spatial_cache[key] = kept
+            return kept
         raise ValueError("Invalid sampling_type. Must be one of ['all', 'random', 'spatial']")
 
     def kernel_candidates(self, T: int, device) -> Optional[torch.Tensor]:
@@ -201,9 +210,9 @@ class MultiHeadConvNNAttention(WatchedModule):
         kept = self._spatial_cache.get(key)
         if kept is None:
             kept = cand.to(torch.int32)
+            if capturing(kept.device):
+                return kept
             if kept.is_cuda:
-                if torch.cuda.is_current_stream_capturing():
-                    return kept                       # (recorded, not written yet)
                 torch.cuda.current_stream(kept.device).synchronize()
             self._spatial_cache[key] = kept
         return kept
@@ -232,22 +241,28 @@ class MultiHeadConvNNAttention(WatchedModule):
         store (``residual + layer(x)``), with ``out`` the result is written in place."""
         self._check_mode(x)
         if self.stage_timer is not None or self._packed is None or x.dim() != 3:
-            B, T, D = x.shape
-            cand = self.candidates(T, x.device)
-            packed = self.packed_weights(x.dtype, x.device)
-            if self.stage_timer is not None:
-                return self._forward_staged(x, packed, cand, out, residual)
-            return ops.forward(self._spec(), x, packed, cand, out=out, residual=residual)
+            return self._forward_general(x, out, residual)
         key = (x.shape, x.dtype, x.device)
         call = self._calls.get(key)
         if call is not None and call.unchanged():
             y = call(self, x, out, residual)
             if y is not None:
                 return y
+        if capturing(x.device):
+            return self._forward_general(x, out, residual)
         if len(self._calls) >= 16:
             self._calls.clear()
         call = self._calls[key] = _LayerCall(self, x)
         return call(self, x, out, residual)
+
+    def _forward_general(self, x, out, residual):
+        """The call with nothing prepared for it."""
+        B, T, D = x.shape
+        cand = self.candidates(T, x.device)
+        packed = self.packed_weights(x.dtype, x.device)
+        if self.stage_timer is not None:
+            return self._forward_staged(x, packed, cand, out, residual)
+        return ops.forward(self._spec(), x, packed, cand, out=out, residual=residual)
 
     def prenorm_supported(self, x) -> bool:
         """Whether ``forward_prenorm`` takes this input (bfloat16, sampling 'all', a K/V/Q weight tile

@@ -229,6 +229,8 @@ def run(model, x: torch.Tensor):
         y = plan.run(x) if type(plan) is Plan else None
         if y is not None or type(plan) is not Plan:
             return y
+    if layers.capturing(x.device):
+        return None
     # The first call of a shape, and the first after a change of the model, goes op by op: it packs weights while
     # the GPU works, and a shape that never returns pays for no plan.  The second call builds the plan.
     if plan is not _SEEN:

@@ -92,3 +92,19 @@ def test_another_stream_reads_nothing_unfinished(which, kind):
     other.synchronize()
     assert torch.equal(y, want)
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("kind", SETS)
+@pytest.mark.parametrize("which", ["vit", "layer"])
+@torch.no_grad()
+def test_one_warm_up_then_capture_then_an_eager_call(which, kind):
+    m, shape = _case(which, kind)
+    x = torch.randn(shape, device=DEV).bfloat16()
+    want = m(x)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        y = m(x)
+    for _ in range(3):                            # before any replay: nothing recorded has run
+        assert torch.equal(m(x), want)
+    g.replay()
+    assert torch.equal(y, want)

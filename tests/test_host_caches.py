@@ -114,3 +114,29 @@ def test_spatial_candidates_belong_to_the_layer(host):
     for _ in range(2):
         model_plan.run(m, x)
     assert host.models[-1].cand_ptr == before
+
+
+@torch.no_grad()
+def test_nothing_is_prepared_while_a_graph_is_captured(host, monkeypatch):
+    m, x = _vit(sampling_type="spatial", num_samples=5), _images()
+    lay, lx = _layer(sampling="spatial", samples=5), torch.randn(2, 17, 16)
+    model_plan.run(m, x), lay(lx)
+    monkeypatch.setattr(layers, "capturing", lambda device: True)
+    assert model_plan.run(m, x) is None and not host.models
+    lay(lx)
+    assert len(host.layers) == 2 and not lay._calls
+    monkeypatch.setattr(layers, "capturing", lambda device: False)
+    model_plan.run(m, x), lay(lx)
+    assert len(host.models) == 1 and len(lay._calls) == 1
+    monkeypatch.setattr(layers, "capturing", lambda device: True)
+    model_plan.run(m, x), lay(lx)                  # what is there already serves a capture too
+    assert len(host.models) == 2 and len(host.layers) == 4
+
+
+def test_spatial_set_of_a_capture_is_not_kept(monkeypatch):
+    lay = _layer(sampling="spatial", samples=5)
+    monkeypatch.setattr(layers, "capturing", lambda device: True)
+    assert lay.candidates(17, torch.device("cpu")).tolist() == [0, 4, 8, 12, 16] and not lay._spatial_cache
+    assert lay.kernel_candidates(17, torch.device("cpu")).tolist() == [0, 4, 8, 12, 16] and not lay._spatial_cache
+    monkeypatch.setattr(layers, "capturing", lambda device: False)
+    assert lay.kernel_candidates(17, torch.device("cpu")).tolist() == [0, 4, 8, 12, 16] and len(lay._spatial_cache) == 2
