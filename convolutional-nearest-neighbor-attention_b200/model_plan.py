@@ -30,7 +30,8 @@ _plans: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
 
 
 class Watch:
-    """What a plan is valid for: one walk over the model's modules, taken before the plan is built."""
+    """What a plan is valid for: one walk over the model's modules, taken before the plan is built.  It holds the modules
+    below ``model`` but not ``model`` itself: ``_plans`` is keyed by the model and must not keep it alive."""
 
     def __init__(self, model):
         self.epoch = layers.attribute_epoch()
@@ -42,7 +43,8 @@ class Watch:
                 continue
             seen.add(id(m))
             d = m.__dict__
-            self.mods.append(m)
+            if m is not model:
+                self.mods.append(m)
             children = d["_modules"]
             if children:
                 self.trees.append((children, dict(children)))
@@ -203,7 +205,7 @@ def _covered(model, x: torch.Tensor, act: torch.dtype, watch: Watch) -> bool:
         return False
     if any(watch.hooks):
         return False
-    for m in watch.mods:
+    for m in [model] + watch.mods:
         if isinstance(m, layers.WatchedModule) and (m.training or getattr(m, "stage_timer", None) is not None):
             return False
     for blk in model.transformer_encoder:

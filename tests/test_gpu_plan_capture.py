@@ -108,3 +108,17 @@ def test_one_warm_up_then_capture_then_an_eager_call(which, kind):
         assert torch.equal(m(x), want)
     g.replay()
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("which", ["vit", "layer"])
+@torch.no_grad()
+def test_deleted_model_gives_its_memory_back(which):
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    m, shape = _case(which, "spatial")
+    x = torch.randn(shape, device=DEV).bfloat16()
+    for _ in range(3):
+        m(x)
+    torch.cuda.synchronize()
+    del m, x
+    assert torch.cuda.memory_allocated() == before

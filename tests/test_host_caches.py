@@ -1,7 +1,9 @@
 """What the host side keeps between forwards (the ViT's host plan, the layers' prepared calls), on CPU tensors: the
 native entry points are replaced by recorders of what they are handed."""
 import ctypes
+import gc
 import types
+import weakref
 
 import numpy as np
 import pytest
@@ -140,3 +142,23 @@ def test_spatial_set_of_a_capture_is_not_kept(monkeypatch):
     assert lay.kernel_candidates(17, torch.device("cpu")).tolist() == [0, 4, 8, 12, 16] and not lay._spatial_cache
     monkeypatch.setattr(layers, "capturing", lambda device: False)
     assert lay.kernel_candidates(17, torch.device("cpu")).tolist() == [0, 4, 8, 12, 16] and len(lay._spatial_cache) == 2
+
+
+@torch.no_grad()
+def test_models_and_layers_are_freed(host):
+    """By their last reference, not by a later collection: their weights are GPU memory."""
+    m, x = _vit(sampling_type="random", num_samples=6), _images()
+    for _ in range(3):
+        model_plan.run(m, x)
+    lay, lx = _layer(sampling="random", samples=6), torch.randn(2, 17, 16)
+    for _ in range(3):
+        lay(lx)
+    assert len(host.models) == 2 and len(lay._calls) == 1
+    dead = [weakref.ref(o) for o in (m, m.classifier.weight, lay, lay.W_v.weight)]
+    plans = len(model_plan._plans)
+    gc.disable()
+    try:
+        del m, lay
+        assert [r() for r in dead] == [None] * 4 and len(model_plan._plans) == plans - 1
+    finally:
+        gc.enable()
