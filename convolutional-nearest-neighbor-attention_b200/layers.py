@@ -244,10 +244,11 @@ class MultiHeadConvNNAttention(WatchedModule):
             return self._forward_general(x, out, residual)
         key = (x.shape, x.dtype, x.device)
         call = self._calls.get(key)
-        if call is not None and call.unchanged():
-            y = call(self, x, out, residual)
+        if call is not None:
+            y = call(self, x, out, residual) if call.unchanged() else None
             if y is not None:
                 return y
+            self._calls.clear()       # those of other shapes hold the same weights as they were
         if capturing(x.device):
             return self._forward_general(x, out, residual)
         if len(self._calls) >= 16:

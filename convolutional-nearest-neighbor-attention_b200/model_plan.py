@@ -227,10 +227,13 @@ def run(model, x: torch.Tensor):
         return None
     key = (x.shape, x.dtype, x.device)
     plan = per_model.get(key)
-    if plan is not None and plan is not _SEEN and plan.watch.unchanged():
-        y = plan.run(x) if type(plan) is Plan else None
-        if y is not None or type(plan) is not Plan:
-            return y
+    if plan is not None and plan is not _SEEN:
+        if plan.watch.unchanged():
+            y = plan.run(x) if type(plan) is Plan else None
+            if y is not None or type(plan) is not Plan:
+                return y
+        per_model.clear()               # those of other shapes hold the same weights as they were
+        plan = None
     if layers.capturing(x.device):
         return None
     # The first call of a shape, and the first after a change of the model, goes op by op: it packs weights while

@@ -162,3 +162,19 @@ def test_models_and_layers_are_freed(host):
         assert [r() for r in dead] == [None] * 4 and len(model_plan._plans) == plans - 1
     finally:
         gc.enable()
+
+
+@torch.no_grad()
+def test_packed_weights_of_another_parameter_version_are_given_back(host):
+    lay, m = _layer(), _vit()
+    for B in (1, 2, 3):
+        for _ in range(2):
+            lay(torch.randn(B, 17, 16)), model_plan.run(m, _images(B))
+    att = m.transformer_encoder[0].attention
+    old = [weakref.ref(w) for w in lay._packed + att._packed if w is not None]
+    for layer in (lay, att):
+        layer.W_v.weight.mul_(2.0)
+    for _ in range(2):
+        lay(torch.randn(2, 17, 16)), model_plan.run(m, _images(2))
+    gc.collect()
+    assert all(r() is None for r in old)
