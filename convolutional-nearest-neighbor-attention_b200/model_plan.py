@@ -7,8 +7,9 @@ one input shape; a forward then is a validity check, two allocations and one nat
 part of it but taken from the layers on every call: a captured graph would read a plan's copy after the plan is gone.
 
 A plan is used only while it describes the model: ``Watch.unchanged()`` compares the attribute epoch of this package's
-modules, the module tree, and identity, version counter and address of every parameter and buffer, and a call
-that finds a difference builds a new plan.  Anything a plan does not cover (training mode, hooks, a stage timer,
+modules, the module tree, and identity, version counter and address of every parameter and buffer, ``Plan.unchanged()``
+also the numbers read from other objects (``eps`` of the norms, the patch size), and a call that finds a difference builds
+a new plan.  Anything a plan does not cover (training mode, hooks, a stage timer,
 parameters of another dtype or device) takes the op-by-op path in ``vit.py``.
 """
 from __future__ import annotations
@@ -74,6 +75,7 @@ class Plan:
         T, D = model.n_patches + 1, model.d_hidden
         self.watch = watch
         self.keep = []              # tensors whose addresses the structs hold
+        self.read = []              # (object, attribute, value) of what the structs hold of objects outside this package
         self.sampled = []           # (block index, attention layer, candidates the plan was made for)
         blocks = list(model.transformer_encoder)
         self.blocks = (_capi.ConvnnBlock * max(1, len(blocks)))()
@@ -83,9 +85,9 @@ class Plan:
         conv = pemb.linear_projection
         m = self.model = _capi.ConvnnModel()
         m.dtype, m.B, m.T, m.D = ops._dtype_code(act), B, T, D
-        m.n_blocks, m.classes = len(blocks), model.classifier.out_features
-        m.channels, m.height, m.width, m.patch = C, Hh, Ww, a.patch_size
-        m.embed_eps = pemb.norm.eps
+        m.n_blocks, m.classes = len(blocks), model.classifier.weight.shape[0]
+        m.channels, m.height, m.width, m.patch = C, Hh, Ww, self._attr(a, "patch_size")
+        m.embed_eps = self._attr(pemb.norm, "eps")
         m.blocks = ctypes.cast(self.blocks, ctypes.POINTER(_capi.ConvnnBlock))
         m.patch_w, m.patch_b = self._ptr(conv.weight.view(D, -1)), self._ptr(conv.bias)
         m.embed_norm_w, m.embed_norm_b = self._ptr(pemb.norm.weight), self._ptr(pemb.norm.bias)
@@ -95,12 +97,20 @@ class Plan:
         if m.images_u8:
             _, mean, inv_std = model.pixel_stats(x.device)
             m.pixel_mean, m.pixel_inv_std = self._ptr(mean), self._ptr(inv_std)
-        self.act, self.out_shape, self.lock = act, (B, model.classifier.out_features), threading.Lock()
+        self.act, self.out_shape, self.lock = act, (B, m.classes), threading.Lock()
         L = _capi.lib()
         self.call, self.arg = L.convnn_b200_model_forward, ctypes.byref(m)
         self.workspace_bytes = L.convnn_b200_model_workspace_bytes(self.arg)
 
+    def unchanged(self) -> bool:
+        return self.watch.unchanged() and all([getattr(o, name) == value for o, name, value in self.read])
+
     # -- construction -------------------------------------------------------------------------------
+    def _attr(self, o, name):
+        value = getattr(o, name)
+        self.read.append((o, name, value))
+        return value
+
     def _ptr(self, t):
         if t is None:
             return None
@@ -128,13 +138,13 @@ class Plan:
         n1, n2, fc1, fc2 = blk.norm1, blk.norm2, blk.mlp[0], blk.mlp[3]
         branching = isinstance(att, (MultiHeadBranchingAttention, MultiHeadBranchingConv))
         self._layer(b, i, att.convnn if branching else att, B, T, act, device)
-        b.d_mlp, b.eps1, b.eps2 = fc1.out_features, n1.eps, n2.eps
+        b.d_mlp, b.eps1, b.eps2 = fc1.weight.shape[0], self._attr(n1, "eps"), self._attr(n2, "eps")
         b.norm1_w, b.norm1_b, b.norm2_w, b.norm2_b = (self._ptr(t) for t in (n1.weight, n1.bias, n2.weight, n2.bias))
         b.fc1_w, b.fc1_b, b.fc2_w, b.fc2_b = (self._ptr(t) for t in (fc1.weight, fc1.bias, fc2.weight, fc2.bias))
         if not branching and blk.folds_norm1_shape(B, T, act):
             self._folded(b, ("w_qkv_folded", "w_qkv_extra"), att.folded_qkv(n1, act, device))
         if (blk.fold_layernorm and act == torch.bfloat16 and
-                ops.prenorm_linear_supported(fc1.out_features, fc1.in_features, True)):
+                ops.prenorm_linear_supported(*fc1.weight.shape, True)):
             self._folded(b, ("fc1_folded", "fc1_extra"), blk.folded_fc1(act, device))
         b.fuse_mlp = int(blk.fuse_mlp)
         if branching:
@@ -190,7 +200,7 @@ class _Refused:
     """A shape no plan covers, remembered until an attribute of the model changes."""
 
     def __init__(self):
-        self.watch, self.epoch = self, layers.attribute_epoch()
+        self.epoch = layers.attribute_epoch()
 
     def unchanged(self) -> bool:
         return self.epoch == layers.attribute_epoch()
@@ -228,7 +238,7 @@ def run(model, x: torch.Tensor):
     key = (x.shape, x.dtype, x.device)
     plan = per_model.get(key)
     if plan is not None and plan is not _SEEN:
-        if plan.watch.unchanged():
+        if plan.unchanged():
             y = plan.run(x) if type(plan) is Plan else None
             if y is not None or type(plan) is not Plan:
                 return y

@@ -178,3 +178,26 @@ def test_packed_weights_of_another_parameter_version_are_given_back(host):
         lay(torch.randn(2, 17, 16)), model_plan.run(m, _images(2))
     gc.collect()
     assert all(r() is None for r in old)
+
+
+@torch.no_grad()
+def test_plan_follows_the_eps_of_the_norms(host):
+    m, x = _vit(), _images()
+    for _ in range(2):
+        model_plan.run(m, x)
+    m.transformer_encoder[0].norm1.eps = 0.5
+    m.transformer_encoder[1].norm2.eps = 0.25
+    m.patch_embedding.norm.eps = 0.125
+    for _ in range(2):
+        model_plan.run(m, x)
+    last = host.models[-1]
+    assert last.eps[0][0] == 0.5 and last.eps[1][1] == 0.25 and last.embed_eps == 0.125
+
+
+@torch.no_grad()
+def test_plan_follows_the_patch_size_it_was_given(host):
+    m, x = _vit(), _images()
+    for _ in range(2):
+        model_plan.run(m, x)
+    m.args.patch_size = 4                          # no longer what the weights are for: the op-by-op path refuses it
+    assert model_plan.run(m, x) is None
