@@ -58,6 +58,45 @@ class _NotCopied(dict):
         return (_NotCopied, ())
 
 
+class Watch:
+    """The state of ``root`` and the modules below it that something prepared is valid for: one walk, taken before the
+    preparation.  It holds the modules below ``root`` but not ``root``, which owns what was prepared and must not be kept
+    alive by it."""
+
+    def __init__(self, root):
+        self.epoch = attribute_epoch()
+        self.mods, self.trees, self.slots, self.tensors, self.hooks = [], [], [], [], []
+        todo, seen = [root], set()
+        while todo:
+            m = todo.pop()
+            if m is None or id(m) in seen:
+                continue
+            seen.add(id(m))
+            d = m.__dict__
+            if m is not root:
+                self.mods.append(m)
+            children = d["_modules"]
+            if children:
+                self.trees.append((children, dict(children)))
+                todo.extend(children.values())
+            self.hooks += (d["_forward_hooks"], d["_forward_pre_hooks"])
+            for tensors in (d["_parameters"], d["_buffers"]):
+                for k, t in tensors.items():
+                    self.slots.append((tensors, k))
+                    if t is not None:
+                        self.tensors.append(t)
+        self.ids = [id(d[k]) for d, k in self.slots]
+        self.versions = [t._version for t in self.tensors]
+        self.ptrs = [t.data_ptr() for t in self.tensors]
+
+    def unchanged(self) -> bool:
+        return (self.epoch == _epoch[0] and
+                [id(d[k]) for d, k in self.slots if k in d] == self.ids and
+                [t._version for t in self.tensors] == self.versions and
+                [t.data_ptr() for t in self.tensors] == self.ptrs and
+                all([d == c for d, c in self.trees]))
+
+
 class _LayerCall:
     """What one ConvNN layer call of a given input shape needs besides its tensors, prepared once: descriptor, packed
     weights, workspace size (27 us of host time per call before, 10 with it; a small layer's kernels take 30).
@@ -65,21 +104,10 @@ class _LayerCall:
 
     def __init__(self, layer, x):
         B, T, _ = x.shape
-        self.epoch = attribute_epoch()
-        mods = [m for m in layer.modules()]
-        self.slots = [(m._parameters, k) for m in mods for k in m._parameters]
-        params = [d[k] for d, k in self.slots]
-        self.ids = [id(p) for p in params]
+        self.watch = Watch(layer)
         self.S = layer.candidate_count(T, x.device)
-        self.params = [p for p in params if p is not None]
-        self.versions = [p._version for p in self.params]
-        self.ptrs = [p.data_ptr() for p in self.params]
         self.packed = layer.packed_weights(x.dtype, x.device)
         self.call = ops.LayerForward(layer._spec(), B, T, self.S, x.dtype, x.device, self.packed)
-
-    def unchanged(self):
-        return (self.epoch == _epoch[0] and [id(d[k]) for d, k in self.slots if k in d] == self.ids and
-                [p._version for p in self.params] == self.versions and [p.data_ptr() for p in self.params] == self.ptrs)
 
     def __call__(self, layer, x, out, residual):
         """``layer(x)``; None: the candidate set has another size now."""
@@ -245,7 +273,7 @@ class MultiHeadConvNNAttention(WatchedModule):
         key = (x.shape, x.dtype, x.device)
         call = self._calls.get(key)
         if call is not None:
-            y = call(self, x, out, residual) if call.unchanged() else None
+            y = call(self, x, out, residual) if call.watch.unchanged() else None
             if y is not None:
                 return y
             self._calls.clear()       # those of other shapes hold the same weights as they were

@@ -23,53 +23,15 @@ import torch
 from torch.nn.modules import module as _nn_module
 
 from . import _capi, layers, ops
-from .layers import MultiHeadBranchingAttention, MultiHeadBranchingConv, MultiHeadConvNNAttention
+from .layers import MultiHeadBranchingAttention, MultiHeadBranchingConv, Watch
 
 MAX_PLANS = 8                       # input shapes remembered per model
 _SEEN = object()                    # a shape that has been called once
 _plans: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
 
 
-class Watch:
-    """What a plan is valid for: one walk over the model's modules, taken before the plan is built.  It holds the modules
-    below ``model`` but not ``model`` itself: ``_plans`` is keyed by the model and must not keep it alive."""
-
-    def __init__(self, model):
-        self.epoch = layers.attribute_epoch()
-        self.mods, self.trees, self.slots, self.tensors, self.hooks = [], [], [], [], []
-        todo, seen = [model], set()
-        while todo:
-            m = todo.pop()
-            if m is None or id(m) in seen:
-                continue
-            seen.add(id(m))
-            d = m.__dict__
-            if m is not model:
-                self.mods.append(m)
-            children = d["_modules"]
-            if children:
-                self.trees.append((children, dict(children)))
-                todo.extend(children.values())
-            self.hooks += (d["_forward_hooks"], d["_forward_pre_hooks"])
-            for tensors in (d["_parameters"], d["_buffers"]):
-                for k, t in tensors.items():
-                    self.slots.append((tensors, k))
-                    if t is not None:
-                        self.tensors.append(t)
-        self.ids = [id(d[k]) for d, k in self.slots]
-        self.versions = [t._version for t in self.tensors]
-        self.ptrs = [t.data_ptr() for t in self.tensors]
-
-    def unchanged(self) -> bool:
-        return (self.epoch == layers.attribute_epoch() and
-                [id(d[k]) for d, k in self.slots if k in d] == self.ids and
-                [t._version for t in self.tensors] == self.versions and
-                [t.data_ptr() for t in self.tensors] == self.ptrs and
-                all([d == c for d, c in self.trees]) and not any(self.hooks))
-
-
 class Plan:
-    def __init__(self, model, x: torch.Tensor, act: torch.dtype, watch: "Watch"):
+    def __init__(self, model, x: torch.Tensor, act: torch.dtype, watch: Watch):
         a = model.args
         B, C, Hh, Ww = x.shape
         T, D = model.n_patches + 1, model.d_hidden
@@ -103,7 +65,8 @@ class Plan:
         self.workspace_bytes = L.convnn_b200_model_workspace_bytes(self.arg)
 
     def unchanged(self) -> bool:
-        return self.watch.unchanged() and all([getattr(o, name) == value for o, name, value in self.read])
+        return (self.watch.unchanged() and not any(self.watch.hooks) and
+                all([getattr(o, name) == value for o, name, value in self.read]))
 
     # -- construction -------------------------------------------------------------------------------
     def _attr(self, o, name):

@@ -201,3 +201,16 @@ def test_plan_follows_the_patch_size_it_was_given(host):
         model_plan.run(m, x)
     m.args.patch_size = 4                          # no longer what the weights are for: the op-by-op path refuses it
     assert model_plan.run(m, x) is None
+
+
+@torch.no_grad()
+def test_layer_call_follows_its_modules(host):
+    lay, x = _layer(conv="depthwise-separable"), torch.randn(2, 17, 16)
+    for _ in range(3):
+        lay(x)
+    old = host.layers[-1]
+    lay.conv[1] = torch.nn.Conv1d(16, 16, 1, bias=False)
+    lay(x)
+    torch.testing.assert_close(lay._packed[2], lay.conv[1].weight[:, :, 0])
+    new = host.layers[-1]
+    assert new.w_pw == lay._packed[2].data_ptr() and new.w_pw != old.w_pw
