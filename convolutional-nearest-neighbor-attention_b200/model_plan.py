@@ -55,9 +55,10 @@ class Plan:
         m.embed_norm_w, m.embed_norm_b = self._ptr(pemb.norm.weight), self._ptr(pemb.norm.bias)
         m.cls, m.pe = self._ptr(cls.view(-1)), self._ptr(pe.pe.view(-1, D)[:T])
         m.head_w, m.head_b = self._ptr(model.classifier.weight), self._ptr(model.classifier.bias)
-        m.images_u8 = int(x.dtype == torch.uint8)
+        m.images_u8, self.mean = int(x.dtype == torch.uint8), None
         if m.images_u8:
             _, mean, inv_std = model.pixel_stats(x.device)
+            self.mean = mean
             m.pixel_mean, m.pixel_inv_std = self._ptr(mean), self._ptr(inv_std)
         self.act, self.out_shape, self.lock = act, (B, m.classes), threading.Lock()
         L = _capi.lib()
@@ -136,8 +137,10 @@ class Plan:
             sets.append(cand)
         return sets
 
-    def run(self, x: torch.Tensor):
+    def run(self, model, x: torch.Tensor):
         """The logits; None where the plan does not describe the call any more."""
+        if self.mean is not None and model.pixel_stats(x.device)[1] is not self.mean:
+            return None
         if not x.is_contiguous():
             x = x.contiguous()
         dev = x.device
@@ -202,7 +205,7 @@ def run(model, x: torch.Tensor):
     plan = per_model.get(key)
     if plan is not None and plan is not _SEEN:
         if plan.unchanged():
-            y = plan.run(x) if type(plan) is Plan else None
+            y = plan.run(model, x) if type(plan) is Plan else None
             if y is not None or type(plan) is not Plan:
                 return y
         per_model.clear()               # those of other shapes hold the same weights as they were
@@ -225,4 +228,4 @@ def run(model, x: torch.Tensor):
     if plan.workspace_bytes == 0:           # a shape the library refuses: the op-by-op path raises its error
         return None
     per_model[key] = plan
-    return plan.run(x)
+    return plan.run(model, x)

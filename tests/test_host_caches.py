@@ -214,3 +214,17 @@ def test_layer_call_follows_its_modules(host):
     torch.testing.assert_close(lay._packed[2], lay.conv[1].weight[:, :, 0])
     new = host.layers[-1]
     assert new.w_pw == lay._packed[2].data_ptr() and new.w_pw != old.w_pw
+
+
+@torch.no_grad()
+def test_plan_follows_the_pixel_statistics(host):
+    m, x = _vit(), torch.randint(0, 256, (2, 3, 32, 32), dtype=torch.uint8)
+    m.pixel_mean = [0.5, 0.5, 0.5]
+    for _ in range(3):
+        model_plan.run(m, x)
+    assert host.models[-1].pixel_mean == m.pixel_stats(x.device)[1].data_ptr()
+    m.pixel_mean[1] = 0.25                         # in place: no assignment to count
+    for _ in range(2):
+        model_plan.run(m, x)
+    now = m.pixel_stats(x.device)[1]
+    assert now.tolist() == [0.5, 0.25, 0.5] and host.models[-1].pixel_mean == now.data_ptr()
