@@ -58,6 +58,14 @@ class _NotCopied(dict):
         return (_NotCopied, ())
 
 
+def _counts_versions(t) -> bool:
+    """False for tensors made under ``torch.inference_mode()``."""
+    try:
+        return t._version >= 0
+    except RuntimeError:
+        return False
+
+
 class Watch:
     """The state of ``root`` and the modules below it that something prepared is valid for: one walk, taken before the
     preparation.  It holds the modules below ``root`` but not ``root``, which owns what was prepared and must not be kept
@@ -86,13 +94,15 @@ class Watch:
                     if t is not None:
                         self.tensors.append(t)
         self.ids = [id(d[k]) for d, k in self.slots]
-        self.versions = [t._version for t in self.tensors]
+        # (what is packed from a tensor without a version counter is refused where it is packed; others are read in place)
+        self.versioned = [t for t in self.tensors if _counts_versions(t)]
+        self.versions = [t._version for t in self.versioned]
         self.ptrs = [t.data_ptr() for t in self.tensors]
 
     def unchanged(self) -> bool:
         return (self.epoch == _epoch[0] and
                 [id(d[k]) for d, k in self.slots if k in d] == self.ids and
-                [t._version for t in self.tensors] == self.versions and
+                [t._version for t in self.versioned] == self.versions and
                 [t.data_ptr() for t in self.tensors] == self.ptrs and
                 all([d == c for d, c in self.trees]))
 

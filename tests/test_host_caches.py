@@ -228,3 +228,21 @@ def test_plan_follows_the_pixel_statistics(host):
         model_plan.run(m, x)
     now = m.pixel_stats(x.device)[1]
     assert now.tolist() == [0.5, 0.25, 0.5] and host.models[-1].pixel_mean == now.data_ptr()
+
+
+def test_tensors_made_under_inference_mode(host):
+    """They have no version counter: a converted model's buffers, a candidate set."""
+    m, x = _vit(sampling_type="random", num_samples=6), _images()
+    with torch.inference_mode():
+        m = m.double().float()
+        m.set_candidates(torch.randperm(17)[:6])
+    lay, lx = _layer(sampling="random", samples=6), torch.randn(2, 17, 16)
+    with torch.inference_mode():
+        lay.candidate_override = torch.arange(6)
+    with pytest.raises(RuntimeError):
+        m.positional_encoding.pe._version
+    for mode in (torch.no_grad, torch.inference_mode):
+        with mode():
+            for _ in range(3):
+                model_plan.run(m, x), lay(lx)
+    assert len(host.models) == 5 and len(host.layers) == 6
