@@ -11,6 +11,7 @@ library; their modules only hold the parameters under the reference's names.
 """
 from __future__ import annotations
 
+import itertools
 from typing import Optional
 
 import torch
@@ -20,26 +21,25 @@ from . import ops
 from .ops import LayerSpec
 
 
-_epoch = [0]
-
-
-def attribute_epoch() -> int:
-    """Counts the attribute assignments on this package's modules: whatever was prepared from their attributes
-    (a forward's host plan) is still valid while it stands still."""
-    return _epoch[0]
+_stamps = itertools.count(1)
+_ABSENT = object()
+_PLAIN = (bool, int, float, str, tuple, type(None))
 
 
 class WatchedModule(nn.Module):
-    """``nn.Module`` whose public attribute assignments advance ``attribute_epoch()``."""
+    """``nn.Module`` that gets a new ``_stamp`` whenever a public attribute is given another value: whatever was prepared
+    from its attributes (a forward's host plan) is valid while the stamp stands.  The stamp comes after the assignment, so
+    what another thread prepares in between is at worst prepared again."""
 
     def __setattr__(self, name, value):
-        if name[0] != "_":
-            _epoch[0] += 1
+        old = self.__dict__.get(name, _ABSENT)
         super().__setattr__(name, value)
+        if name[0] != "_" and not (old is value and type(value) in _PLAIN):
+            self.__dict__["_stamp"] = next(_stamps)
 
     def __delattr__(self, name):
-        _epoch[0] += 1
         super().__delattr__(name)
+        self.__dict__["_stamp"] = next(_stamps)
 
 
 def capturing(device) -> bool:
@@ -72,7 +72,6 @@ class Watch:
     alive by it."""
 
     def __init__(self, root):
-        self.epoch = attribute_epoch()
         self.mods, self.trees, self.slots, self.tensors, self.hooks = [], [], [], [], []
         todo, seen = [root], set()
         while todo:
@@ -93,14 +92,22 @@ class Watch:
                     self.slots.append((tensors, k))
                     if t is not None:
                         self.tensors.append(t)
+        self.dicts = [m.__dict__ for m in self.mods if isinstance(m, WatchedModule)]
+        self.stamps = self._stamps(root)
         self.ids = [id(d[k]) for d, k in self.slots]
         # (what is packed from a tensor without a version counter is refused where it is packed; others are read in place)
         self.versioned = [t for t in self.tensors if _counts_versions(t)]
         self.versions = [t._version for t in self.versioned]
         self.ptrs = [t.data_ptr() for t in self.tensors]
 
-    def unchanged(self) -> bool:
-        return (self.epoch == _epoch[0] and
+    def _stamps(self, root):
+        return [d.get("_stamp") for d in self.dicts] + [root.__dict__.get("_stamp")]
+
+    def options_unchanged(self, root) -> bool:
+        return self._stamps(root) == self.stamps
+
+    def unchanged(self, root) -> bool:
+        return (self._stamps(root) == self.stamps and
                 [id(d[k]) for d, k in self.slots if k in d] == self.ids and
                 [t._version for t in self.versioned] == self.versions and
                 [t.data_ptr() for t in self.tensors] == self.ptrs and
@@ -283,7 +290,7 @@ class MultiHeadConvNNAttention(WatchedModule):
         key = (x.shape, x.dtype, x.device)
         call = self._calls.get(key)
         if call is not None:
-            y = call(self, x, out, residual) if call.watch.unchanged() else None
+            y = call(self, x, out, residual) if call.watch.unchanged(self) else None
             if y is not None:
                 return y
             self._calls.clear()       # those of other shapes hold the same weights as they were

@@ -6,7 +6,7 @@ host's pace.  A plan holds the model's weight pointers, packed copies, layer des
 one input shape; a forward then is a validity check, two allocations and one native call.  Candidate sets are not
 part of it but taken from the layers on every call: a captured graph would read a plan's copy after the plan is gone.
 
-A plan is used only while it describes the model: ``Watch.unchanged()`` compares the attribute epoch of this package's
+A plan is used only while it describes the model: ``Watch.unchanged()`` compares the attribute stamps of this package's
 modules, the module tree, and identity, version counter and address of every parameter and buffer, ``Plan.unchanged()``
 also the numbers read from other objects (``eps`` of the norms, the patch size), and a call that finds a difference builds
 a new plan.  Anything a plan does not cover (training mode, hooks, a stage timer,
@@ -65,8 +65,8 @@ class Plan:
         self.call, self.arg = L.convnn_b200_model_forward, ctypes.byref(m)
         self.workspace_bytes = L.convnn_b200_model_workspace_bytes(self.arg)
 
-    def unchanged(self) -> bool:
-        return (self.watch.unchanged() and not any(self.watch.hooks) and
+    def unchanged(self, model) -> bool:
+        return (self.watch.unchanged(model) and not any(self.watch.hooks) and
                 all([getattr(o, name) == value for o, name, value in self.read]))
 
     # -- construction -------------------------------------------------------------------------------
@@ -163,13 +163,13 @@ class Plan:
 
 
 class _Refused:
-    """A shape no plan covers, remembered until an attribute of the model changes."""
+    """A shape no plan covers, remembered until an attribute of the model or its hooks change."""
 
-    def __init__(self):
-        self.epoch = layers.attribute_epoch()
+    def __init__(self, watch: Watch):
+        self.watch, self.hooked = watch, any(watch.hooks)
 
-    def unchanged(self) -> bool:
-        return self.epoch == layers.attribute_epoch()
+    def unchanged(self, model) -> bool:
+        return self.watch.options_unchanged(model) and any(self.watch.hooks) == self.hooked
 
 
 def _covered(model, x: torch.Tensor, act: torch.dtype, watch: Watch) -> bool:
@@ -204,7 +204,7 @@ def run(model, x: torch.Tensor):
     key = (x.shape, x.dtype, x.device)
     plan = per_model.get(key)
     if plan is not None and plan is not _SEEN:
-        if plan.unchanged():
+        if plan.unchanged(model):
             y = plan.run(model, x) if type(plan) is Plan else None
             if y is not None or type(plan) is not Plan:
                 return y
@@ -222,7 +222,7 @@ def run(model, x: torch.Tensor):
     act = model.patch_embedding.linear_projection.weight.dtype if x.dtype == torch.uint8 else x.dtype
     watch = Watch(model)
     if not _covered(model, x, act, watch):
-        per_model[key] = _Refused()
+        per_model[key] = _Refused(watch)
         return None
     plan = Plan(model, x, act, watch)
     if plan.workspace_bytes == 0:           # a shape the library refuses: the op-by-op path raises its error

@@ -246,3 +246,24 @@ def test_tensors_made_under_inference_mode(host):
             for _ in range(3):
                 model_plan.run(m, x), lay(lx)
     assert len(host.models) == 5 and len(host.layers) == 6
+
+
+@torch.no_grad()
+def test_plans_outlive_assignments_that_do_not_concern_them(host):
+    m, x = _vit(), _images()
+    lay, lx = _layer(), torch.randn(2, 17, 16)
+    for _ in range(2):
+        model_plan.run(m, x), lay(lx)
+    plan, call = next(iter(model_plan._plans[m].values())), next(iter(lay._calls.values()))
+    _vit().classifier.bias.zero_()                 # another model is built
+    _layer().K = 2                                 # and changed
+    for _ in range(3):
+        m.eval(), lay.eval()                       # nothing changes
+        assert model_plan.run(m, x) is not None and lay(lx) is not None
+    assert next(iter(model_plan._plans[m].values())) is plan and next(iter(lay._calls.values())) is call
+    lay.train()
+    lay.softmax_topk_val = False
+    lay.eval(), lay(lx)
+    assert next(iter(lay._calls.values())) is not call
+    m.transformer_encoder[1].attention.softmax_topk_val = False
+    assert model_plan.run(m, x) is None
