@@ -25,9 +25,18 @@ from torch.nn.modules import module as _nn_module
 from . import _capi, layers, ops
 from .layers import MultiHeadBranchingAttention, MultiHeadBranchingConv, Watch
 
-MAX_PLANS = 8                       # input shapes remembered per model
+MAX_PLANS = 32                      # input shapes remembered per model, the latest used ones (host memory only)
 _SEEN = object()                    # a shape that has been called once
 _plans: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
+_lock = threading.Lock()            # the order of a model's entries
+
+
+def _remember(per_model, key, entry):
+    with _lock:
+        per_model[key] = entry
+        per_model.move_to_end(key)
+        while len(per_model) > MAX_PLANS:
+            per_model.popitem(last=False)
 
 
 class Plan:
@@ -207,25 +216,27 @@ def run(model, x: torch.Tensor):
         if plan.unchanged(model):
             y = plan.run(model, x) if type(plan) is Plan else None
             if y is not None or type(plan) is not Plan:
+                _remember(per_model, key, plan)
                 return y
-        per_model.clear()               # those of other shapes hold the same weights as they were
+        with _lock:
+            per_model.clear()           # those of other shapes hold the same weights as they were
         plan = None
     if layers.capturing(x.device):
         return None
     # The first call of a shape, and the first after a change of the model, goes op by op: it packs weights while
     # the GPU works, and a shape that never returns pays for no plan.  The second call builds the plan.
     if plan is not _SEEN:
-        per_model[key] = _SEEN
-        while len(per_model) > MAX_PLANS:
-            per_model.popitem(last=False)
+        _remember(per_model, key, _SEEN)
         return None
     act = model.patch_embedding.linear_projection.weight.dtype if x.dtype == torch.uint8 else x.dtype
     watch = Watch(model)
     if not _covered(model, x, act, watch):
-        per_model[key] = _Refused(watch)
+        _remember(per_model, key, _Refused(watch))
         return None
     plan = Plan(model, x, act, watch)
     if plan.workspace_bytes == 0:           # a shape the library refuses: the op-by-op path raises its error
         return None
-    per_model[key] = plan
-    return plan.run(model, x)
+    y = plan.run(model, x)
+    if y is not None:
+        _remember(per_model, key, plan)
+    return y

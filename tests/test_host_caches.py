@@ -2,6 +2,7 @@
 native entry points are replaced by recorders of what they are handed."""
 import ctypes
 import gc
+import threading
 import types
 import weakref
 
@@ -267,3 +268,32 @@ def test_plans_outlive_assignments_that_do_not_concern_them(host):
     assert next(iter(lay._calls.values())) is not call
     m.transformer_encoder[1].attention.softmax_topk_val = False
     assert model_plan.run(m, x) is None
+
+
+@torch.no_grad()
+def test_twenty_batch_sizes_keep_their_plans(host):
+    m = _vit()
+    for turn in range(4):
+        for B in range(1, 21):
+            assert (model_plan.run(m, _images(B)) is not None) == (turn > 0)
+    assert len(model_plan._plans[m]) == 20
+    for B in range(21, 21 + model_plan.MAX_PLANS):  # bounded, and those in use stay
+        model_plan.run(m, _images(1)), model_plan.run(m, _images(B))
+    assert len(model_plan._plans[m]) == model_plan.MAX_PLANS and model_plan.run(m, _images(1)) is not None
+
+
+@torch.no_grad()
+def test_plans_of_a_model_from_many_threads(host, monkeypatch):
+    m, failures = _vit(), []
+    monkeypatch.setattr(model_plan, "MAX_PLANS", 3)
+
+    def work(seed):
+        try:
+            for i in range(60):
+                model_plan.run(m, _images(1 + (i * seed) % 7))
+        except Exception as e:                     # noqa: BLE001
+            failures.append(e)
+    with torch.no_grad():
+        threads = [threading.Thread(target=torch.no_grad()(work), args=(s,)) for s in (1, 2, 3, 5)]
+        [t.start() for t in threads], [t.join() for t in threads]
+    assert not failures and len(model_plan._plans[m]) <= 3
