@@ -114,6 +114,12 @@ class Watch:
                 all([d == c for d, c in self.trees]))
 
 
+def registered(*modules) -> bool:
+    """Whether the weights and biases of ``modules`` are parameters, which a ``Watch`` sees (and no attributes or
+    parametrizations)."""
+    return all(m._parameters.keys() >= {"weight", "bias"} for m in modules)
+
+
 class _LayerCall:
     """What one ConvNN layer call of a given input shape needs besides its tensors, prepared once: descriptor, packed
     weights, workspace size (27 us of host time per call before, 10 with it; a small layer's kernels take 30).
@@ -209,6 +215,10 @@ class MultiHeadConvNNAttention(WatchedModule):
             return (self.conv[0].weight, self.conv[1].weight)
         return (self.conv.weight,)
 
+    def _weight_modules(self):
+        conv = self.conv if self.convolution_type == 'depthwise-separable' else (self.conv,)
+        return (self.W_q, self.W_k, self.W_v, self.W_o, *conv)
+
     def packed_weights(self, dtype, device):
         params = (self.W_q.weight, self.W_k.weight, self.W_v.weight, self.W_o.weight) + self._conv_params()
         key = (dtype, device) + tuple((p.data_ptr(), p._version) for p in params)
@@ -294,7 +304,7 @@ class MultiHeadConvNNAttention(WatchedModule):
             if y is not None:
                 return y
             self._calls.clear()       # those of other shapes hold the same weights as they were
-        if capturing(x.device):
+        if capturing(x.device) or not registered(*self._weight_modules()):
             return self._forward_general(x, out, residual)
         if len(self._calls) >= 16:
             self._calls.clear()
@@ -401,6 +411,9 @@ class MultiHeadAttention(WatchedModule):
         self.W_o = nn.Linear(d_hidden, d_hidden, bias=False)
         self._packed = _PackedParams()
 
+    def _weight_modules(self):
+        return self.W_q, self.W_k, self.W_v, self.W_o
+
     def packed_weights(self, dtype, device):
         params = (self.W_q.weight, self.W_k.weight, self.W_v.weight, self.W_o.weight)
         return self._packed.get(params, dtype, device, lambda: (
@@ -432,6 +445,9 @@ class MultiHeadConv1dAttention(WatchedModule):
         self.in_channels = self.out_channels = self.d_k
         self.conv = nn.Conv1d(self.d_k, self.d_k, kernel_size=kernel_size, stride=1, padding="same")
         self._packed = _PackedParams()
+
+    def _weight_modules(self):
+        return self.W_x, self.conv, self.W_o
 
     def packed_weights(self, dtype, device):
         params = (self.W_x.weight, self.W_x.bias, self.conv.weight, self.conv.bias, self.W_o.weight, self.W_o.bias)
@@ -532,7 +548,3 @@ class MultiHeadBranchingConv(_Branching):
         else:
             return self._two_branches(x, self.conv1d, residual)
         return y if residual is None else residual + y
-
-
-OWN_MODULES = (MultiHeadConvNNAttention, MultiHeadAttention, MultiHeadConv1dAttention, MultiHeadBranchingAttention,
-               MultiHeadBranchingConv)

@@ -23,7 +23,8 @@ import torch
 from torch.nn.modules import module as _nn_module
 
 from . import _capi, layers, ops
-from .layers import MultiHeadBranchingAttention, MultiHeadBranchingConv, Watch
+from .layers import (MultiHeadAttention, MultiHeadBranchingAttention, MultiHeadBranchingConv, MultiHeadConv1dAttention,
+                     MultiHeadConvNNAttention, Watch, registered)
 
 MAX_PLANS = 32                      # input shapes remembered per model, the latest used ones (host memory only)
 _SEEN = object()                    # a shape that has been called once
@@ -181,6 +182,24 @@ class _Refused:
         return self.watch.options_unchanged(model) and any(self.watch.hooks) == self.hooked
 
 
+def _own(m, cls) -> bool:
+    return type(m) is cls and "forward" not in m.__dict__
+
+
+def _own_attention(att) -> bool:
+    """Whether calling the module would run this package's code, on registered weights."""
+    if _own(att, MultiHeadConvNNAttention):
+        return registered(*att._weight_modules())
+    if _own(att, MultiHeadBranchingAttention):
+        halves = ("convnn", MultiHeadConvNNAttention), ("attention", MultiHeadAttention)
+    elif _own(att, MultiHeadBranchingConv):
+        halves = ("convnn", MultiHeadConvNNAttention), ("conv1d", MultiHeadConv1dAttention)
+    else:
+        return False
+    return (0 < att.branch_ratio < 1 and registered(att.pointwise_linear) and
+            all(_own(getattr(att, name), cls) and registered(*getattr(att, name)._weight_modules()) for name, cls in halves))
+
+
 def _covered(model, x: torch.Tensor, act: torch.dtype, watch: Watch) -> bool:
     """Whether a plan can describe this call."""
     from .vit import TransformerEncoder, ViT
@@ -193,11 +212,14 @@ def _covered(model, x: torch.Tensor, act: torch.dtype, watch: Watch) -> bool:
     for m in [model] + watch.mods:
         if isinstance(m, layers.WatchedModule) and (m.training or getattr(m, "stage_timer", None) is not None):
             return False
+    pe, pemb = model.positional_encoding, model.patch_embedding
+    if ("cls_tokens" not in pe._parameters or "pe" not in pe._buffers or
+            not registered(pemb.linear_projection, pemb.norm, model.classifier)):
+        return False
     for blk in model.transformer_encoder:
-        att = blk.attention
-        if blk.fuse_out_proj or type(att) not in layers.OWN_MODULES:
+        if blk.fuse_out_proj or not _own_attention(blk.attention):
             return False
-        if isinstance(att, (MultiHeadBranchingAttention, MultiHeadBranchingConv)) and not 0 < att.branch_ratio < 1:
+        if not registered(blk.norm1, blk.norm2, blk.mlp[0], blk.mlp[3]):
             return False
     dev = x.device
     return all([t.dtype == act and t.device == dev and t.is_contiguous() for t in watch.tensors])

@@ -297,3 +297,51 @@ def test_plans_of_a_model_from_many_threads(host, monkeypatch):
         threads = [threading.Thread(target=torch.no_grad()(work), args=(s,)) for s in (1, 2, 3, 5)]
         [t.start() for t in threads], [t.join() for t in threads]
     assert not failures and len(model_plan._plans[m]) <= 3
+
+
+@torch.no_grad()
+def test_calls_that_run_somebody_elses_code_are_not_planned(host):
+    """The op-by-op path calls a block's attention, and the halves of a branching one, as modules; they may be a subclass or
+    have a forward of their own.  Weights that are no registered parameters cannot be watched."""
+    class Mine(layers.MultiHeadAttention):
+        pass
+
+    def own_forward(m):
+        m.transformer_encoder[1].attention.forward = lambda x, residual=None: residual
+
+    def own_half(m):
+        att = m.transformer_encoder[0].attention
+        att.attention = Mine(att.d_hidden_attention, att.num_heads, 0.0).eval()
+
+    def own_forward_of_a_half(m):
+        m.transformer_encoder[0].attention.convnn.forward = lambda x, out=None: out
+
+    def plain_weight(m):
+        lin = m.transformer_encoder[1].mlp[0]
+        w = lin.weight.detach().clone()
+        del lin.weight
+        lin.weight = w
+
+    def plain_packed_weight(m):
+        lin = m.transformer_encoder[1].attention.convnn.W_v
+        w = lin.weight.detach().clone()
+        del lin.weight
+        lin.weight = w
+
+    x = _images()
+    for change in (own_forward, own_half, own_forward_of_a_half, plain_weight, plain_packed_weight):
+        m = _vit(layer="BranchAttention", d_hidden=32)
+        for _ in range(2):
+            model_plan.run(m, x)
+        assert host.models
+        host.models.clear()
+        change(m)
+        assert [model_plan.run(m, x) for _ in range(4)] == [None] * 4 and not host.models, change.__name__
+    lay, lx = _layer(), torch.randn(2, 17, 16)
+    w = lay.W_v.weight.detach().clone()
+    del lay.W_v.weight
+    lay.W_v.weight = w
+    lay(lx), lay(lx)
+    lay.W_v.weight = w * 2
+    lay(lx)
+    torch.testing.assert_close(lay._packed[0][1], w * 2)
