@@ -252,7 +252,7 @@ class LayerForward:
         self.need = L.convnn_b200_workspace_bytes(self.d)
         if self.need == 0:
             _capi.check(min(L.convnn_b200_head_channels(self.d), 0))
-        self.D, self.dtype, self.device, self.packed = spec.d_hidden, dtype, device, packed
+        self.dtype, self.device, self.packed = dtype, device, packed
         self.w = [_capi.ptr(w) for w in packed]
 
     def __call__(self, x: torch.Tensor, cand: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
@@ -260,7 +260,8 @@ class LayerForward:
         x, ldx = _rows_view(x)
         workspace = torch.empty(self.need, dtype=torch.uint8, device=self.device)
         if out is None:
-            out, ldo = torch.empty(x.shape, dtype=self.dtype, device=self.device), self.D
+            # (rows as wide as the input's, whatever the layer's width: the library refuses narrower ones)
+            out, ldo = torch.empty(x.shape, dtype=self.dtype, device=self.device), x.shape[2]
         else:
             view, ldo = _rows_view(out)
             if view is not out:

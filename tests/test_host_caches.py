@@ -345,3 +345,13 @@ def test_calls_that_run_somebody_elses_code_are_not_planned(host):
     lay.W_v.weight = w * 2
     lay(lx)
     torch.testing.assert_close(lay._packed[0][1], w * 2)
+
+
+@torch.no_grad()
+def test_input_of_another_width_than_the_layer(host):
+    """The result has rows as wide as the input's, and the library is told so (it refuses rows narrower than the layer:
+    a channel slice that is too narrow must not be written past its rows)."""
+    for x in (torch.randn(2, 17, 24), torch.randn(2, 17, 24)[:, :, :8]):
+        lay = _layer()
+        seen = [(lay(x).shape, host.layers[-1].ldo) for _ in range(3)]
+        assert seen == [(x.shape, x.shape[2])] * 3
