@@ -298,18 +298,22 @@ class MultiHeadConvNNAttention(WatchedModule):
         if self.stage_timer is not None or self._packed is None or x.dim() != 3:
             return self._forward_general(x, out, residual)
         key = (x.shape, x.dtype, x.device)
-        call = self._calls.get(key)
+        calls = self.__dict__.get("_calls")
+        if calls is None:             # saved as a whole before there were any
+            calls = self._calls = _NotCopied()
+        call = calls.get(key)
         if call is not None:
             y = call(self, x, out, residual) if call.watch.unchanged(self) else None
             if y is not None:
                 return y
-            self._calls.clear()       # those of other shapes hold the same weights as they were
+            calls.clear()             # those of other shapes hold the same weights as they were
         if capturing(x.device) or not registered(*self._weight_modules()):
             return self._forward_general(x, out, residual)
-        if len(self._calls) >= 16:
-            self._calls.clear()
-        call = self._calls[key] = _LayerCall(self, x)
-        return call(self, x, out, residual)
+        if len(calls) >= 16:
+            calls.clear()
+        call = calls[key] = _LayerCall(self, x)
+        y = call(self, x, out, residual)
+        return self._forward_general(x, out, residual) if y is None else y
 
     def _forward_general(self, x, out, residual):
         """The call with nothing prepared for it."""

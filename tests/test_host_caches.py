@@ -1,7 +1,9 @@
 """What the host side keeps between forwards (the ViT's host plan, the layers' prepared calls), on CPU tensors: the
 native entry points are replaced by recorders of what they are handed."""
+import copy
 import ctypes
 import gc
+import pickle
 import threading
 import types
 import weakref
@@ -355,3 +357,19 @@ def test_input_of_another_width_than_the_layer(host):
         lay = _layer()
         seen = [(lay(x).shape, host.layers[-1].ldo) for _ in range(3)]
         assert seen == [(x.shape, x.shape[2])] * 3
+
+
+@torch.no_grad()
+def test_modules_saved_before_they_kept_prepared_calls(host):
+    lay, x = _layer(), torch.randn(2, 17, 16)
+    old = copy.deepcopy(lay)
+    old(x)
+    for name in ("_calls", "_stamp"):
+        old.__dict__.pop(name)
+    old = pickle.loads(pickle.dumps(old))
+    for _ in range(3):
+        old(x)
+    assert len(host.layers) == 4
+    new = pickle.loads(pickle.dumps(lay))
+    new(x), new(x)
+    assert len(new._calls) == 1
