@@ -130,7 +130,7 @@ int check_device() {
 }
 
 struct Workspace {
-    char *q, *k, *v, *o, *scratch;
+    char *q, *k, *v, *o, *scratch, *conv_scratch;
     float *qstat, *kstat, *val;
     int32_t* idx;
     size_t total;
@@ -153,11 +153,26 @@ size_t stage_scratch(const Dims& dm, int conv_type) {
     return n * dm.elt;
 }
 
+// The whole layer's buffers.  The separable conv's unrounded intermediate of the coordinate channel (bfloat16: twice the
+// bytes of its other scratch) lies over the stage scratch, q and k, which the conv no longer needs, so that a forward asks
+// for no more than its other stages do.  Where candidates are so few that q leaves no room for the padding channels, the
+// conv runs without scratch (same sums, in one kernel; it takes heads of up to 1024 channels).
 Workspace carve(const Dims& dm, int conv_type, void* base) {
     Workspace w;
     char* p = static_cast<char*>(base);
     size_t off = 0;
     auto take = [&](size_t bytes) { char* r = p ? p + off : nullptr; off += up256(bytes); return r; };
+    const size_t need = stage_scratch(dm, conv_type);
+    const size_t q_k = up256((size_t)dm.B * dm.S * dm.H * dm.Cp * dm.elt) + up256((size_t)dm.B * dm.T * dm.H * dm.Cp * dm.elt);
+    size_t own = need;
+    if (conv_type == CONVNN_DEPTHWISE_SEPARABLE && dm.C != dm.dk) {
+        own = (size_t)dm.B * (dm.T > dm.S ? dm.T : dm.S) * dm.D * dm.elt;
+        const size_t rounded = (size_t)dm.B * dm.H * dm.T * dm.C * dm.elt;
+        if (rounded > own) own = rounded;
+        if (dm.dk > 1024 && own + q_k < need) own = need - q_k;
+    }
+    w.scratch = take(own);
+    w.conv_scratch = up256(own) + q_k >= need ? w.scratch : nullptr;
     w.q = take((size_t)dm.B * dm.S * dm.H * dm.Cp * dm.elt);
     w.k = take((size_t)dm.B * dm.T * dm.H * dm.Cp * dm.elt);
     w.v = take((size_t)dm.B * dm.T * dm.H * dm.Cp * dm.elt);
@@ -166,7 +181,6 @@ Workspace carve(const Dims& dm, int conv_type, void* base) {
     w.kstat = reinterpret_cast<float*>(take((size_t)dm.B * dm.H * dm.T * 4));
     w.val = reinterpret_cast<float*>(take((size_t)dm.B * dm.H * dm.T * dm.K * 4));
     w.idx = reinterpret_cast<int32_t*>(take((size_t)dm.B * dm.H * dm.T * dm.K * 4));
-    w.scratch = take(stage_scratch(dm, conv_type));
     w.total = off;
     return w;
 }
@@ -436,7 +450,7 @@ int convnn_b200_forward(const convnn_desc* d, const void* x, int64_t ldx, const 
         return set_error(CONVNN_E_WORKSPACE, "workspace has %zu bytes, %zu needed", workspace_bytes, w.total);
     if ((rc = convnn_b200_qkv_proj(d, x, ldx, w_qkv, cand, w.q, w.k, w.v, w.qstat, w.kstat, w.scratch, stream))) return rc;
     if ((rc = convnn_b200_sim_topk(d, w.q, w.k, w.qstat, w.kstat, cand, w.idx, w.val, stream))) return rc;
-    if ((rc = convnn_b200_gather_conv(d, w.v, w.idx, w.val, w_conv, w_pw, w.o, w.scratch, stream))) return rc;
+    if ((rc = convnn_b200_gather_conv(d, w.v, w.idx, w.val, w_conv, w_pw, w.o, w.conv_scratch, stream))) return rc;
     return convnn_b200_out_proj(d, w.o, w_o, residual, ldr, out, ldo, w.scratch, stream);
 }
 

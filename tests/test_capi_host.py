@@ -179,3 +179,20 @@ def test_candidate_indices_are_range_checked_on_the_host():
     spec = ops.LayerSpec(48, 1, 5, "random")
     with pytest.raises(IndexError):
         ops._cand_arg(spec, torch.tensor([1, 99]), 65, torch.device("cpu"))
+
+
+@pytest.mark.parametrize("dtype,elt", [(_capi.BF16, 2), (_capi.F32, 4)])
+@pytest.mark.parametrize("B,T,S,D,H", [(83, 197, 197, 192, 1), (14, 577, 577, 384, 1), (8, 4096, 33, 64, 1), (3, 65, 20, 2080, 1),
+                                       (9, 197, 49, 96, 3)])
+def test_separable_workspace_with_the_coordinate_channel(B, T, S, D, H, dtype, elt):
+    """No more than the buffers of the other stages and one (B, H, T, C) operand: what fits a fixed workspace (the
+    built-in one holds 83 images of 197 x 192) is not to depend on how the conv keeps its intermediate."""
+    dk = D // H
+    C, Cp, up = dk + 1, (dk + 8) // 8 * 8, lambda n: (n + 255) // 256 * 256
+    total = (up(B * S * H * Cp * elt) + 2 * up(B * T * H * Cp * elt) + up(B * T * D * elt) + up(B * H * S * 4) + up(B * H * T * 4) +
+             2 * up(B * H * T * 9 * 4) + up(max(B * max(T, S) * D, B * H * T * C) * elt))
+    got = _capi.lib().convnn_b200_workspace_bytes(desc(B=B, T=T, S=S, D=D, H=H, sampled=S != T, conv_type="depthwise-separable",
+                                                       coord=True, dtype=dtype))
+    assert 0 < got <= total or dk > 1024
+    if (B, dtype) == (83, _capi.BF16):
+        assert got <= 32 << 20

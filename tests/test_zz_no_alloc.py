@@ -97,3 +97,24 @@ def test_noalloc_forward_refuses_shapes_beyond_its_capacity():
     rc, _ = _call_noalloc(spec, x, packed)
     assert rc == _capi.E_WORKSPACE
     assert "built-in workspace" in L.convnn_b200_last_error().decode()
+
+
+@pytest.mark.parametrize("B,T,S,D", [(83, 197, 197, 192), (4, 4096, 33, 64), (2, 300, 50, 1032)])
+def test_separable_conv_of_the_coordinate_channel_shares_buffers(B, T, S, D):
+    """The intermediate over q and k, or without scratch where they leave no room for it, and the stage calls with scratch
+    of their own: the same bits.  (83, 197, 197, 192) is the largest batch of its shape that fits the built-in array."""
+    cfg = ConvNNConfig(d_hidden=D, num_heads=1, K=9, magnitude_type="cosine", sampling_type="all" if S == T else "spatial",
+                       num_samples=S, convolution_type="depthwise-separable", coordinate_encoding=True)
+    w = {n: bf16_round(t) for n, t in make_layer_weights(cfg, seed=5).items()}
+    spec, packed = spec_of(cfg), pack(cfg, w, torch.bfloat16)
+    cand = None if S == T else torch.linspace(0, T - 1, S).to(DEV, torch.int32)
+    x = make_input(B, T, D, seed=3).to(DEV, torch.bfloat16)
+    w_qkv, w_conv, w_pw, w_o = packed
+    q, k, v, qs, ks = ops.qkv_proj(spec, x, w_qkv, cand)
+    idx, val = ops.sim_topk(spec, q, k, qs, ks, cand)
+    want = ops.out_proj(spec, ops.gather_conv(spec, v, idx, val, w_conv, w_pw, S=S), w_o, S=S)
+    assert torch.equal(ops.forward(spec, x, packed, cand), want)
+    if (B, T) == (83, 197):
+        rc, got = _call_noalloc(spec, x, packed)
+        _capi.check(rc)
+        assert torch.equal(got, want)
