@@ -286,16 +286,30 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
 
 }  // namespace
 
-// The pair kernel pays off where the tensor pipe is the limiter: long key and candidate
-// lists, mostly full 64-channel chunks.
+// The pair kernel pays off where the tensor pipe is the limiter: long key and candidate lists, heads of several full
+// 64-channel chunks.  Lists longer than 16 double the cost of keeping two lists per row; measured break-even is at many
+// units per cluster and a few thousand candidates.
+//
+// Heads of 64 channels, and widths whose last chunk is partly zeros, are closer to the selection's limit, and there the
+// rounds of 256-row units decide: one per pair of SMs here, two per SM (lists up to 12, up to 256 channels) or one per SM in
+// the other kernel, whose round takes about three (short lists), two or one and a half times as long.  Both kernels give the
+// same bits.  us, pair against single kernel, 1024 x 1024 per image: 8 images of 64 channels, K = 9: 37 / 65, K = 16: 51 / 62;
+// 32 images: 68 / 66, 97 / 64; 64 images of 112 channels: 129 / 96, 193 / 129.  4096 x 4096: 8 images of 64 channels 166 / 203,
+// 206 / 170; 96 images 1658 / 1465, 2054 / 1796.  K = 25 at 16384 x 16384, 4 images of 64 channels: 1379 / 1195.
 bool sim_topk_tc2_wanted(const convnn_desc* d, const Dims& dm) {
     static const int env = [] { const char* e = getenv("CONVNN_B200_SIM_PAIR"); return e ? atoi(e) : -1; }();
     if (env == 0) return false;
-    if (d->dtype != CONVNN_BF16 || dm.Cp % 16 != 0 || dm.Cp < 96) return false;   // (a last chunk is zero-filled past the head)
-    // Lists longer than 16 double the cost of keeping two lists per row; measured break-even
-    // is at many units per cluster and a few thousand candidates.
-    if (dm.nsel > 16) return dm.T >= 8192 && dm.S >= 4096;
-    return dm.T >= 1024 && dm.S >= 1024;
+    if (d->dtype != CONVNN_BF16 || dm.Cp % 16 != 0 || (dm.Cp != 64 && dm.Cp < 96)) return false;
+    if (dm.T < 1024 || dm.S < 1024) return false;
+    if (dm.Cp > 64 && dm.Cp % 64 == 0) return dm.nsel <= 16 || (dm.T >= 8192 && dm.S >= 4096);
+    if (dm.nsel > 16) return false;
+    const long long units = (long long)dm.B * dm.H * ((dm.T + 2 * BM - 1) / (2 * BM)), sms = device_sms();
+    auto rounds = [&](long long at_once) { return (units + at_once - 1) / at_once; };
+    const long long pair = rounds(sms / 2 > 0 ? sms / 2 : 1);
+    if (dm.nsel > 12) return 20 * pair <= 29 * rounds(sms);
+    if (dm.Cp <= 256) return pair <= 3 * rounds(2 * sms);
+    const bool fills = dm.Cp >= 320 && dm.S >= 4096;      // (400 channels: 320 / 348 at 4096 x 4096, 68 / 60 at 1024 x 1024)
+    return fills ? pair <= 2 * rounds(sms) : pair < 2 * rounds(sms);
 }
 
 int launch_sim_topk_tc2(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,

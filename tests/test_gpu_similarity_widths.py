@@ -59,3 +59,18 @@ def test_coordinate_channel_keeps_the_fp32_sums(T, S, H, dk, metric):
     cand = None if S == T else torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32)
     got, want = (ops.sim_topk(spec, a, b, qs, ks, cand) for a, b in ((q, k), (q.float(), k.float())))
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("C", [64, 96, 144, 272])
+@pytest.mark.parametrize("K", [9, 16, 17])
+def test_long_sequences_give_the_same_lists_in_batches_of_any_size(C, K):
+    """Which of the two long-sequence kernels runs depends on the number of rows: one, two, five and nine rounds of it."""
+    g = torch.Generator(device=DEV).manual_seed(C)
+    T = 1024
+    spec = ops.LayerSpec(C, 1, K, "all", "cosine", "depthwise", True, False, T)
+    q, k = (torch.randn(160, T, 1, C, device=DEV, generator=g).bfloat16() for _ in range(2))
+    qs, ks = (1 / t.float().norm(dim=-1).permute(0, 2, 1).contiguous() for t in (q, k))
+    want = ops.sim_topk(spec, q, k, qs, ks)
+    for B in (1, 33, 80):
+        got = ops.sim_topk(spec, q[:B], k[:B], qs[:B].contiguous(), ks[:B].contiguous())
+        assert torch.equal(got[0], want[0][:B]) and torch.equal(got[1], want[1][:B])
