@@ -89,7 +89,8 @@ def test_conv1d_branch_float32(T, dk, ks):
 
 
 @pytest.mark.parametrize("T,S,C,K", [(1, 1, 4, 1), (63, 64, 20, 9), (65, 65, 16, 25), (129, 200, 33, 32), (257, 63, 48, 4),
-                                     (300, 300, 8, 16), (2500, 65, 36, 9)])
+                                     (300, 300, 8, 16), (2500, 65, 36, 9), (65, 65, 24, 8), (130, 130, 20, 12),
+                                     (197, 70, 36, 11)])
 @pytest.mark.parametrize("metric", ["cosine", "matmul", "euclidean"])
 def test_similarity_lists_float32(T, S, C, K, metric):
     g = torch.Generator(device=DEV).manual_seed(T + S)
