@@ -76,9 +76,11 @@ def test_plan_follows_changes_of_the_model():
             assert torch.equal(got, want) and not torch.equal(got, before)
             before = _planned(m, x)
             assert torch.equal(before, want)
-        m.transformer_encoder[0].attention.register_forward_hook(lambda *a: None)
-        m(x)
-        assert torch.equal(m(x), before)          # (hooks take the op-by-op path)
+        seen = []                                 # (hooks of the modules that are called take the op-by-op path)
+        m.transformer_encoder[0].fold_layernorm = False
+        m.transformer_encoder[0].attention.register_forward_hook(lambda *a: seen.append(len(a)))
+        outs = [m(x) for _ in range(4)]
+        assert len(seen) == 4 and all(torch.equal(y, _op_by_op(m, x)) for y in outs)
 
 
 def test_random_candidates_are_drawn_per_call_as_before():
@@ -106,8 +108,11 @@ def test_layer_call_follows_changes_and_options():
         assert not torch.equal(m(x), first)
         fresh = copy.deepcopy(m)
         assert len(fresh._calls) == 0 and torch.equal(fresh(x), m(x))
-        m.K = 5
-        with pytest.raises(Exception):
-            m.conv.weight.data = m.conv.weight.data[:, :, :5].contiguous()
-            m.magnitude_type = "unknown"
+        m.K = 5                                   # an option of the layer, with taps cut to it
+        m.conv.weight.data = m.conv.weight.data[:, :, :5].contiguous()
+        short = convnn_b200.MultiHeadConvNNAttention(96, 3, 0.0, 5, "spatial", 50, 0, "cosine").to(DEV, torch.bfloat16).eval()
+        short.load_state_dict(m.state_dict())
+        assert torch.equal(m(x), short(x)) and not torch.equal(m(x), fresh(x))
+        m.magnitude_type = "unknown"
+        with pytest.raises(ValueError, match="magnitude_type"):
             m(x)
