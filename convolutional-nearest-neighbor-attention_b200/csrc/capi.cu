@@ -163,16 +163,16 @@ Workspace carve(const Dims& dm, int conv_type, void* base) {
     size_t off = 0;
     auto take = [&](size_t bytes) { char* r = p ? p + off : nullptr; off += up256(bytes); return r; };
     const size_t need = stage_scratch(dm, conv_type);
-    const size_t q_k = up256((size_t)dm.B * dm.S * dm.H * dm.Cp * dm.elt) + up256((size_t)dm.B * dm.T * dm.H * dm.Cp * dm.elt);
-    size_t own = need;
-    if (conv_type == CONVNN_DEPTHWISE_SEPARABLE && dm.C != dm.dk) {
-        own = (size_t)dm.B * (dm.T > dm.S ? dm.T : dm.S) * dm.D * dm.elt;
+    const bool overlaid = conv_type == CONVNN_DEPTHWISE_SEPARABLE && dm.C != dm.dk;
+    if (overlaid) {
+        const size_t q_k = up256((size_t)dm.B * dm.S * dm.H * dm.Cp * dm.elt) + up256((size_t)dm.B * dm.T * dm.H * dm.Cp * dm.elt);
+        size_t own = (size_t)dm.B * (dm.T > dm.S ? dm.T : dm.S) * dm.D * dm.elt;
         const size_t rounded = (size_t)dm.B * dm.H * dm.T * dm.C * dm.elt;
         if (rounded > own) own = rounded;
         if (dm.dk > 1024 && own + q_k < need) own = need - q_k;
+        w.scratch = take(own);
+        w.conv_scratch = up256(own) + q_k >= need ? w.scratch : nullptr;
     }
-    w.scratch = take(own);
-    w.conv_scratch = up256(own) + q_k >= need ? w.scratch : nullptr;
     w.q = take((size_t)dm.B * dm.S * dm.H * dm.Cp * dm.elt);
     w.k = take((size_t)dm.B * dm.T * dm.H * dm.Cp * dm.elt);
     w.v = take((size_t)dm.B * dm.T * dm.H * dm.Cp * dm.elt);
@@ -181,6 +181,7 @@ Workspace carve(const Dims& dm, int conv_type, void* base) {
     w.kstat = reinterpret_cast<float*>(take((size_t)dm.B * dm.H * dm.T * 4));
     w.val = reinterpret_cast<float*>(take((size_t)dm.B * dm.H * dm.T * dm.K * 4));
     w.idx = reinterpret_cast<int32_t*>(take((size_t)dm.B * dm.H * dm.T * dm.K * 4));
+    if (!overlaid) w.scratch = w.conv_scratch = take(need);
     w.total = off;
     return w;
 }
