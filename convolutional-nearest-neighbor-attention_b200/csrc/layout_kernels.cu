@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(256) merge_heads_kernel(const T* __restrict__ 
         const int l = i & 31, blk = i >> 5;
         const int cv = (blk % (g4 / 4)) * 4 + (l & 3), t = blk / (g4 / 4) * 8 + (l >> 2);
         if (cv >= nv || t >= Tn) continue;
-        T v[VEC];
+        __align__(16) T v[VEC];
 #pragma unroll
         for (int e = 0; e < VEC; ++e) v[e] = s[(cv * VEC + e) * Tn + t];
         T* d = dst + (long long)t * D + cv * VEC;
