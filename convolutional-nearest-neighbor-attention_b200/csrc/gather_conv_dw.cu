@@ -6,8 +6,8 @@
 // 16-byte channel group of TPT tokens at a time: a tap's weights are loaded and unpacked once for the TPT tokens,
 // whose neighbour rows are TPT independent 16-byte loads in flight.
 //
-// Bound by the neighbour reads, K x the size of V out of L2 (and L1 where an image's tokens share an SM): at 131072
-// tokens of 768 channels and 25 taps 5.0 GB.  Before, one thread per output group issued its taps one after another,
+// Reads K x the size of V, most of it from L2 and L1: at 131072 tokens of 768 channels and 25 taps 5.0 GB against
+// 0.2 GB of values.  Before, one thread per output group issued its taps one after another,
 // and shapes whose V slice fits in shared memory were tied to one CTA per slice: 144 us for one image of 65 tokens,
 // 768 channels and 16 taps.
 #include "common.cuh"
@@ -191,7 +191,7 @@ int launch(const DwParams& p, cudaStream_t st) {
     // Four tokens per thread where that still leaves every SM two CTAs' worth of threads, else one.  Tokens per CTA: one
     // item (token set, channel group) per thread on small grids; on large ones up to eight, as long as six CTAs per SM
     // remain, so that a CTA's prologue (its tokens' weights) is spread over more rows: 131072 x 768, 25 taps 641 us
-    // with one item per thread, 501 with eight (10 TB/s of neighbour rows, what L2 delivers; 772 before).
+    // with one item per thread, 501 with eight (5.0 GB of neighbour rows, 10 TB/s; 772 before).
     const long long items = (long long)p.M * p.groups;
     const int tpt = items >= 4LL * device_sms() * 512 ? 4 : 1;
     int TT = (THREADS * tpt + p.groups - 1) / p.groups;

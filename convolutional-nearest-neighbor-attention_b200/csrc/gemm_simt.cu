@@ -5,9 +5,9 @@
 // path (tensor cores would need a split of every operand to keep the 1e-6 similarity accuracy the top-K parity asks
 // for) and the fallback for bfloat16 shapes the tcgen05 kernels do not cover.
 //
-// Bound by the fp32 pipes and the shared-memory reads that feed them.  Each thread accumulates TM x TN outputs, k strictly ascending with one fused
-// multiply-add per term, so a result does not depend on the tile it was computed in.  Two columns share one packed
-// multiply-add instruction; operand tiles are transposed into shared memory ([k][row]) so that a warp (4 x 8 threads)
+// Bound by the fp32 pipes and the shared-memory reads that feed them.  Each thread accumulates TM x TN outputs, k strictly
+// ascending with one fused multiply-add per term, so a result does not depend on the tile it was computed in.  Two columns
+// share one packed multiply-add instruction; operand tiles are transposed into shared memory ([k][row]) so that a warp (4 x 8 threads)
 // reads one 64-byte and one 128-byte span per k step without conflicts; the next tile's global loads are in flight
 // while the current one is multiplied.
 #include "common.cuh"
@@ -368,7 +368,9 @@ int launch_gemm_simt(int dtype, const GemmParams& params, cudaStream_t st) {
         return set_error(CONVNN_E_UNSUPPORTED, "gemm_simt: %d channels per head are not a multiple of four", p.Cp);
     if (p.a_f32 && dtype == CONVNN_BF16 && p.a_mode != A_ROWS)
         return set_error(CONVNN_E_UNSUPPORTED, "gemm_simt: a float32 operand against bfloat16 weights comes as plain rows");
-    const int rc = p.a_f32 && dtype == CONVNN_BF16 ? launch_mode<float, __nv_bfloat16, A_ROWS>(p, st) : dtype == CONVNN_F32 ? launch_typed<float>(p, st) : launch_typed<__nv_bfloat16>(p, st);
+    const int rc = dtype == CONVNN_F32 ? launch_typed<float>(p, st)
+                   : p.a_f32           ? launch_mode<float, __nv_bfloat16, A_ROWS>(p, st)
+                                       : launch_typed<__nv_bfloat16>(p, st);
     if (rc) return rc;
     CONVNN_CHECK_LAUNCH("gemm_simt");
     return CONVNN_OK;

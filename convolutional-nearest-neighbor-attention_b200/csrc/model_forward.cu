@@ -1,7 +1,7 @@
 // The whole ViT forward as one native call: the chain of entry points that vit.py issues one binding call at a
 // time, over one workspace.  No kernel of its own.
 //
-// Why: at batch sizes up to ~100 images a ViT-Tiny forward was bound by the host, 1.14 ms per forward for 52
+// Why: at batch sizes up to ~100 images a ViT-Tiny forward was bound by the host, 1.14 ms per forward for 64
 // launches, of which the library's own share was a fifth; the rest was argument handling, allocation of the
 // intermediates and shape logic in Python between them.
 #include "common.cuh"

@@ -1,6 +1,6 @@
 """Host plan of a ViT forward: everything ``convnn_b200_model_forward`` reads, prepared once.
 
-A ViT-Tiny forward is 52 launches; issued one binding call at a time they cost the host 1.14 ms (measured, one
+A ViT-Tiny forward is 64 launches; issued one binding call at a time they cost the host 1.14 ms (measured, one
 image), most of it argument handling and shape logic between the calls, so batches below ~100 images ran at the
 host's pace.  A plan holds the model's weight pointers, packed copies, layer descriptors and workspace size for
 one input shape; a forward then is a validity check, two allocations and one native call.  Candidate sets are not
