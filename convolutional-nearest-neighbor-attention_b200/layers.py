@@ -255,9 +255,12 @@ class MultiHeadConvNNAttention(WatchedModule):
         """``candidates`` as the kernels read them (int32), converted by every call on its own stream: a set that is
         changed in place is followed, and a captured graph holds the conversion and its memory.  The set of 'spatial' never
         changes: it is converted once, kept as long as the layer, and complete before any stream can see it."""
-        cand = self.candidates(T, device)
+        override = self._candidate_override
+        cand = self.candidates(T, device if override is None else override.device)
         if cand is None:
             return None
+        if cand.device.type == "cpu" and device.type == "cuda":
+            return self._device_copy(cand, device)
         key = (T, str(device))
         if cand is not self._spatial_cache.get(key):
             return cand.to(device=device, dtype=torch.int32).contiguous()
@@ -272,10 +275,30 @@ class MultiHeadConvNNAttention(WatchedModule):
             self._spatial_cache[key] = kept
         return kept
 
+    def _device_copy(self, cand, device) -> torch.Tensor:
+        """A set in host memory on ``device``, copied again when its values change (the copy has arrived when the call
+        returns, and cannot be made while a graph is captured).  A copy that a graph was captured with is kept as long as the
+        layer."""
+        copies = self.__dict__.get("_copies")
+        if copies is None:
+            copies = self._copies = _NotCopied()
+        now = cand.to(torch.int32)
+        values, kept = copies.get(device, (None, None))
+        if kept is None or not torch.equal(values, now):
+            kept = now.to(device)
+            copies[device] = (now.clone(), kept)
+        if capturing(device):
+            copies.setdefault("captured", []).append(kept)
+        else:
+            kept.record_stream(torch.cuda.current_stream(device))
+        return kept
+
     def candidate_count(self, T: int, device) -> int:
         """S of a call over T tokens (without a draw)."""
         if self.sampling_type == 'random' and self._candidate_override is None:
             return len(range(T)[:self.num_samples])
+        if self._candidate_override is not None and self.sampling_type != 'all':
+            return self._candidate_override.numel()
         cand = self.candidates(T, device)
         return T if cand is None else cand.numel()
 
@@ -318,7 +341,7 @@ class MultiHeadConvNNAttention(WatchedModule):
     def _forward_general(self, x, out, residual):
         """The call with nothing prepared for it."""
         B, T, D = x.shape
-        cand = self.candidates(T, x.device)
+        cand = self.kernel_candidates(T, x.device)
         packed = self.packed_weights(x.dtype, x.device)
         if self.stage_timer is not None:
             return self._forward_staged(x, packed, cand, out, residual)

@@ -8,26 +8,26 @@ from convnn_b200 import model_plan
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
-SETS = ["override", "spatial"]
+SETS = ["override", "host", "spatial"]
 
 
 def _model(kind):
     torch.manual_seed(0)
     m = convnn_b200.ViT(convnn_b200.make_args(
         num_layers=2, num_heads=1, d_hidden=64, d_mlp=128, num_classes=24, device=DEV, dropout=0.0, attention_dropout=0.0,
-        magnitude_type="cosine", sampling_type="random" if kind == "override" else "spatial", num_samples=40))
+        magnitude_type="cosine", sampling_type="spatial" if kind == "spatial" else "random", num_samples=40))
     m = m.to(torch.bfloat16).eval()
-    if kind == "override":
-        m.set_candidates(torch.randperm(197, device=DEV)[:40])
+    if kind != "spatial":
+        m.set_candidates(torch.randperm(197, device=DEV if kind == "override" else "cpu")[:40])
     return m
 
 
 def _layer(kind):
     torch.manual_seed(0)
-    m = convnn_b200.MultiHeadConvNNAttention(64, 1, 0.0, 9, "random" if kind == "override" else "spatial", 40, 0, "cosine")
+    m = convnn_b200.MultiHeadConvNNAttention(64, 1, 0.0, 9, "spatial" if kind == "spatial" else "random", 40, 0, "cosine")
     m = m.to(DEV, torch.bfloat16).eval()
-    if kind == "override":
-        m.candidate_override = torch.randperm(197, device=DEV)[:40]
+    if kind != "spatial":
+        m.candidate_override = torch.randperm(197, device=DEV if kind == "override" else "cpu")[:40]
     return m
 
 
@@ -122,3 +122,25 @@ def test_deleted_model_gives_its_memory_back(which):
     torch.cuda.synchronize()
     del m, x
     assert torch.cuda.memory_allocated() == before
+
+
+@pytest.mark.parametrize("which", ["vit", "layer"])
+@torch.no_grad()
+def test_host_set_changed_in_place(which):
+    """Followed by later calls; a graph keeps what it was captured with, also when its copy has been replaced."""
+    m, shape = _case(which, "host")
+    x = torch.randn(shape, device=DEV).bfloat16()
+    cand = m.candidate_override if which == "layer" else m.transformer_encoder[0].attention.candidate_override
+    for _ in range(3):
+        first = m(x)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        y = m(x)
+    for seed in (1, 2):
+        cand.copy_(torch.randperm(197, generator=torch.Generator().manual_seed(seed))[:40])
+        got = [m(x) for _ in range(3)]
+        _drop(m)
+        assert all(torch.equal(a, m(x)) for a in got) and not torch.equal(got[0], first)
+    keep = [torch.zeros(n, dtype=torch.int32, device=DEV) for n in [40, 64, 128, 256] * 200]
+    g.replay()
+    assert torch.equal(y, first) and len(keep) == 800
