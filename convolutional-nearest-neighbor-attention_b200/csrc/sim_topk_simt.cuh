@@ -8,8 +8,9 @@
 // list of its own; the lists of a row are merged at the end under the full (key, column) order.  The T x S matrix
 // never exists in memory, and exact ties go to the lower candidate column.
 //
-// Bound by the fp32 pipes on long sequences (one thread per row with its 64 columns in registers, before, read every
-// operand value of a column from shared memory once per row: 97 us per layer at 32 x 65 tokens x 192 channels).
+// Bound by the shared-memory reads that feed the fp32 pipes (64 images of 197 x 192: L1 68 % busy, warps wait for shared
+// memory most).  One thread per row with its 64 columns in registers, before, read every operand value of a column from
+// shared memory once per row: 97 us per layer at 32 x 65 tokens x 192 channels.
 //
 // Ranking keys (larger is better) and the values reported for the survivors:
 //   cosine     key = dot * qinv[j]            val = key * kinv[i]
