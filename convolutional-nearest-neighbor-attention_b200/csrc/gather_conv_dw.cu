@@ -7,9 +7,9 @@
 // whose neighbour rows are TPT independent 16-byte loads in flight.
 //
 // Reads K x the size of V, most of it from L2 and L1: at 131072 tokens of 768 channels and 25 taps 5.0 GB against
-// 0.2 GB of values.  There L2 is 42 % busy and the ALU, which unpacks, 50 %: bound by the latency of the neighbour rows.  Before, one thread per output group issued its taps one after another,
-// and shapes whose V slice fits in shared memory were tied to one CTA per slice: 144 us for one image of 65 tokens,
-// 768 channels and 16 taps.
+// 0.2 GB of values.  There L2 is 42 % busy and the ALU, which unpacks, 50 %: bound by the latency of the neighbour rows.
+// Before, one thread per output group issued its taps one after another, and shapes whose V slice fits in shared memory
+// were tied to one CTA per slice: 144 us for one image of 65 tokens, 768 channels and 16 taps.
 #include "common.cuh"
 #include "f32x2.cuh"
 
