@@ -228,6 +228,7 @@ int convnn_b200_device_status(int* code) {
     if ((rc = read_gemm_tc_status(&b))) return rc;
     if ((rc = read_sim_topk2_status(&c))) return rc;
     if (!c && (rc = read_sim_short_status(&c))) return rc;
+    if (!c && (rc = read_sim_rows_status(&c))) return rc;
     if (!c && (rc = read_dw_stream_status(&c))) return rc;
     if (!c && (rc = read_attention_status(&c))) return rc;
     if (!c && (rc = read_mlp_tc_status(&c))) return rc;

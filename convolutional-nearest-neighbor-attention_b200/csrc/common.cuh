@@ -167,10 +167,14 @@ bool sim_topk_tc2_wanted(const convnn_desc* d, const Dims& dm);
 int launch_sim_topk_tc2(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
                         const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st);
 // Candidate lists that fit one accumulator (S <= 256): bfloat16 operands, same rules as launch_sim_topk_tc.
+bool sim_topk_rows_wanted(const Dims& dm);
+int launch_sim_topk_rows(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
+                         const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st);
 bool sim_topk_short_wanted(const Dims& dm);
 int launch_sim_topk_short(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
                           const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st);
 int read_sim_short_status(int* out);
+int read_sim_rows_status(int* out);
 int read_sim_topk_status(int* out);
 int read_sim_topk2_status(int* out);
 int try_launch_gather_conv_dw_stream(const convnn_desc* d, const Dims& dm, const void* v, const int32_t* idx,

@@ -1,0 +1,636 @@
+// Similarity + top-K for candidate lists that fit one accumulator (S <= 256), a WARP per key row.
+//
+// A thread per row (the TMEM layout) leaves at most 256 rows in flight per SM and chains of dependent comparisons.  Here the
+// accumulator is copied once to shared memory as ranking keys, row by row, and sixteen warps take rows from there: lane l
+// holds columns l, l + 32, ..., two rows are interleaved, nothing diverges and no lane idles on a ragged sequence end.
+//
+//   bound      the nsel-th largest of the 32 lane maxima (nsel warp-wide maxima): at least nsel keys reach it
+//   survivors  the keys that reach it (9 of 197: ~10.5) are packed into shared memory
+//   rank       every survivor counts the survivors above it: its slot of the list
+//
+// Lists are collected in shared memory as (key, column) and written out a warp's rows at a time.  A row with equal keys among
+// its best, with more survivors than the buffer holds, or with fewer than nsel keys above -inf (NaN inputs) takes its list one
+// (key, column) maximum at a time instead; the lists are the streaming kernels' bit for bit.
+//
+// A persistent CTA per SM owns an equal share of the flattened (batch, head, row) range, in segments of up to 128 rows of
+// one (batch, head), wherever they start.  Warp 0: TMA producer (128 key rows from the segment's first, all
+// candidate rows, 64-channel chunks, ring); warp 1: MMA issuer (M = 128, N = S rounded to 16), two accumulators; warps 2-17:
+// copy and selection.
+#include <limits.h>
+
+#include <type_traits>
+
+#include "common.cuh"
+#include "f32x2.cuh"
+#include "sim_topk_select.cuh"
+#include "sm100.cuh"
+
+namespace convnn {
+
+__device__ int g_sim_rows_status = 0;
+
+namespace {
+
+using namespace sm100;
+
+constexpr int BM = 128;
+constexpr int MAX_STAGES = 6;
+constexpr int NW = 16;                  // selection warps
+constexpr int R = 2;                    // rows a warp interleaves
+constexpr int WR = BM / NW;             // most rows of a segment per warp
+constexpr int NT = 64 + 32 * NW;
+
+struct RowsParams {
+    const float *qstat, *kstat;
+    const int32_t* cand;
+    int32_t* idx;
+    float* val;
+    int T, S, H, K, nsel, metric, sampled;
+    int KCH, KC;        // channels per shared-memory chunk, chunks per segment
+    int BN, pitch;      // S rounded up to 16; words between the rows of the key buffer (4 mod 8: 16-byte stores of eight
+                        // consecutive rows fall into different banks)
+    int acc_cols;       // TMEM columns of one accumulator
+    int seg_rows;       // most rows of a segment (rows of the key buffer)
+    int list_len, inv_K;
+    int stages;
+    int rows_total, rows_per_cta, per_head;
+    float sqrt_dk;
+};
+
+__device__ __forceinline__ void fail(volatile int* abort_flag, int code) {
+    *abort_flag = 1;
+    atomicCAS(&g_sim_rows_status, 0, code);
+}
+
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// Largest value of the warp (NaN only if every lane holds NaN).
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+template <int N>
+__device__ __forceinline__ float max_of(const float (&v)[N], int first, int step) {
+    float m = v[first];
+    int j = first + step;
+#pragma unroll
+    for (; j + step < N; j += 2 * step) m = max3(m, v[j], v[j + step]);
+    if (j < N) m = fmaxf(m, v[j]);
+    return m;
+}
+
+// A CTA's range of flattened rows, cut into segments of one (batch, head).  Ranges follow each other; with `per_head` set they
+// start anew in every (batch, head), `per_head` of them.
+struct Segment {
+    int g, end;          // first flattened row, end of the CTA's range
+    int bh, row, n;
+    __device__ __forceinline__ Segment(const RowsParams& p) {
+        if (p.per_head) {
+            bh = blockIdx.x / p.per_head;
+            row = (blockIdx.x - bh * p.per_head) * p.rows_per_cta;
+            g = bh * p.T + row;
+            end = g + min(p.rows_per_cta, p.T - row);
+        } else {
+            g = blockIdx.x * p.rows_per_cta;
+            end = min(g + p.rows_per_cta, p.rows_total);
+            bh = g / p.T;
+            row = g - bh * p.T;
+        }
+        n = min(min(p.T - row, end - g), p.seg_rows);
+    }
+    __device__ __forceinline__ bool valid() const { return g < end; }
+    __device__ __forceinline__ void next(const RowsParams& p) {
+        g += n;
+        row += n;
+        if (row == p.T) { row = 0; ++bh; }
+        n = min(min(p.T - row, end - g), p.seg_rows);
+    }
+};
+
+__device__ __forceinline__ void sts_entry(uint32_t at, float key, int col) {
+    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(__float_as_uint(key)), "r"(col) : "memory");
+}
+
+// Exact list of one row under the full (key, column) order, one maximum at a time; keys of -inf and NaN never enter.
+template <int J>
+__device__ __noinline__ void select_ordered(const float* keys, int BN, int nsel, uint32_t list) {
+    const int lane = threadIdx.x & 31;
+    float v[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) v[j] = 32 * j + lane < BN ? keys[32 * j + lane] : -CUDART_INF_F;
+    float last = CUDART_INF_F;
+    int last_col = -1;
+    for (int s = 0; s < nsel; ++s) {
+        float best = -CUDART_INF_F;
+        int col = INT_MAX;
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int c = 32 * j + lane;
+            if ((v[j] < last || (v[j] == last && c > last_col)) && v[j] > best) { best = v[j]; col = c; }
+        }
+        last = warp_max(best);
+        last_col = __reduce_min_sync(0xffffffffu, best == last ? col : INT_MAX);
+        if (!(last > -CUDART_INF_F)) last_col = 0;
+        if (lane == 0) sts_entry(list + s * 8, last, last_col);
+    }
+}
+
+// Keys that reach the bound: (key, column) pairs at `at`, which moves on.
+__device__ __forceinline__ void store_if_reached(float key, float bound, int col, uint32_t& at) {
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "setp.ge.f32 p, %1, %2;\n\t"
+                 "@p st.shared.v2.b32 [%0], {%3, %4};\n\t"
+                 "@p add.u32 %0, %0, 8;\n\t}"
+                 : "+r"(at) : "f"(key), "f"(bound), "r"(__float_as_uint(key)), "r"(col) : "memory");
+}
+__device__ __forceinline__ float4 lds_v4(uint32_t at) {
+    float4 r;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(at) : "memory");
+    return r;
+}
+
+// R rows of the key buffer at once (rows at, at + NW, ...): J columns per lane, GR groups of them per lane whose maxima give
+// the bound, room for 32 E survivors per row at `found`.  Returns the rows (bit r) that need select_ordered().
+template <int J, int GR, int E, int NS, int R>
+__device__ __forceinline__ uint32_t select_rows(const RowsParams& p, const float* keybuf, uint32_t found, uint32_t list,
+                                                     uint32_t list_stride, int at) {
+    constexpr int CAP = 32 * E;
+    const int lane = threadIdx.x & 31;
+    const uint32_t below = (1u << lane) - 1u;
+    const int nsel = NS ? NS : p.nsel;
+    float v[R][J];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const float* kr = keybuf + (at + r * NW) * p.pitch + lane;
+#pragma unroll
+        for (int j = 0; j < J - 1; ++j) v[r][j] = kr[32 * j];
+        v[r][J - 1] = -CUDART_INF_F;
+        if (32 * (J - 1) + lane < p.BN) v[r][J - 1] = kr[32 * (J - 1)];
+    }
+    float m[R][GR], bound[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int q = 0; q < GR; ++q) m[r][q] = max_of<J>(v[r], q < J ? q : 0, GR);
+#pragma unroll
+    for (int r = 0; r < R; ++r) bound[r] = warp_max(GR == 2 ? fmaxf(m[r][0], m[r][GR - 1]) : m[r][0]);
+    auto lower = [&] {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+#pragma unroll
+            for (int q = 0; q < GR; ++q) m[r][q] = m[r][q] == bound[r] ? -CUDART_INF_F : m[r][q];
+            bound[r] = warp_max(GR == 2 ? fmaxf(m[r][0], m[r][GR - 1]) : m[r][0]);
+        }
+    };
+    if (NS) {
+#pragma unroll
+        for (int s = 1; s < NS; ++s) lower();
+    } else {
+#pragma unroll 1
+        for (int s = 1; s < nsel; ++s) lower();
+    }
+    // where each lane's survivors go: exclusive prefix of the lanes' counts, bit by bit
+    int mine[R], before[R], n[R], most = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        mine[r] = 0;
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+            if (v[r][j] >= bound[r]) ++mine[r];
+        before[r] = __popc(__ballot_sync(0xffffffffu, mine[r] & 1) & below);
+        if (J >= 2) before[r] += 2 * __popc(__ballot_sync(0xffffffffu, mine[r] & 2) & below);
+        most = max(most, mine[r]);
+    }
+    if (J >= 4 && __any_sync(0xffffffffu, most >= 4)) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            before[r] += 4 * __popc(__ballot_sync(0xffffffffu, mine[r] & 4) & below);
+            if (J >= 8) before[r] += 8 * __popc(__ballot_sync(0xffffffffu, mine[r] & 8) & below);
+        }
+    }
+    uint32_t redo = 0;
+    int n_max = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) n[r] = __shfl_sync(0xffffffffu, before[r] + mine[r], 31);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (n[r] > CAP || !(bound[r] > -CUDART_INF_F)) {
+            redo |= 1u << r;                     // (keys of +inf may still be stored: a lane's J from slot 0 on)
+            n[r] = 0;
+            bound[r] = CUDART_INF_F;
+            before[r] = 0;
+        }
+        n_max = max(n_max, n[r]);
+        uint32_t to = found + (r * CAP + before[r]) * 8;
+#pragma unroll
+        for (int j = 0; j < J; ++j) store_if_reached(v[r][j], bound[r], 32 * j + lane, to);
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            if (lane + 32 * e >= n[r])
+                asm volatile("st.shared.b32 [%0], %1;" ::"r"(found + (r * CAP + lane + 32 * e) * 8), "r"(0xff800000u) : "memory");
+    }
+    __syncwarp();
+    float key[R][E];
+    int col[R][E], rank[R][E];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=f"(key[r][e]), "=r"(col[r][e])
+                         : "r"(found + (r * CAP + lane + 32 * e) * 8) : "memory");
+            rank[r][e] = 0;
+        }
+    }
+    auto count_above = [&](int i) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float4 a = lds_v4(found + (r * CAP + i) * 8), b = lds_v4(found + (r * CAP + i) * 8 + 16);
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                if (a.x > key[r][e]) ++rank[r][e];
+                if (a.z > key[r][e]) ++rank[r][e];
+                if (b.x > key[r][e]) ++rank[r][e];
+                if (b.z > key[r][e]) ++rank[r][e];
+            }
+        }
+    };
+    constexpr int FIRST = NS ? (NS + 3) / 4 * 4 : 0;    // (9 of 197 columns: 12 survivors suffice for nine rows in ten)
+#pragma unroll
+    for (int i = 0; i < FIRST; i += 4) count_above(i);
+#pragma unroll 1
+    for (int i = FIRST; i < n_max; i += 4) count_above(i);
+    __syncwarp();
+    // A lane past the survivors holds -inf and rank n.  Equal keys share a rank and leave a later one out: the list is right
+    // if the ranks below nsel all occur and are nsel in number.
+    const uint32_t all = nsel == 32 ? 0xffffffffu : (1u << nsel) - 1u;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        uint32_t bits = 0;
+        int listed = 0;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const bool in = rank[r][e] < nsel;
+            listed += __popc(__ballot_sync(0xffffffffu, in));
+            if (in) bits |= 1u << rank[r][e];
+        }
+        const bool good = __reduce_or_sync(0xffffffffu, bits) == all && listed == nsel && !(redo >> r & 1u);
+        if (!good) redo |= 1u << r;
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            if (good && rank[r][e] < nsel) sts_entry(list + r * list_stride + rank[r][e] * 8, key[r][e], col[r][e]);
+    }
+    return redo;
+}
+
+__device__ __forceinline__ void selection_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory"); }
+
+// NS: number of neighbours where it is fixed, 0: any up to 16, -1: up to 25, -2: up to 32.
+template <int J, int NS>
+__global__ void __launch_bounds__(NT, 1)
+sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ,
+                     const __grid_constant__ RowsParams p) {
+    constexpr int E = NS < 0 ? 2 : 1, GR = NS == -2 && J > 1 ? 2 : 1;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const uint32_t pitch = p.KCH * 2;
+    const uint32_t a_bytes = BM * pitch, b_bytes = p.BN * pitch, stage_bytes = a_bytes + b_bytes;
+    const uint32_t STAGES = p.stages;
+    float* keybuf = reinterpret_cast<float*>(smem + STAGES * stage_bytes);      // [seg_rows][pitch]
+    float2* lists = reinterpret_cast<float2*>(keybuf + p.seg_rows * p.pitch);   // [NW][WR][nsel] key, column
+    float2* found = lists + NW * WR * p.list_len;                               // [NW][R][32 E] survivors: key, column
+    float* qs = reinterpret_cast<float*>(found + NW * R * 32 * E);              // [BN] column statistics
+    int* cs = reinterpret_cast<int*>(qs + p.BN);                                // [BN] candidate tokens
+    float* kst_s = reinterpret_cast<float*>(cs + p.BN);                         // [BM] row statistics
+    uint64_t* full = reinterpret_cast<uint64_t*>(kst_s + BM);
+    uint64_t* empty = full + MAX_STAGES;
+    uint64_t* tfull = empty + MAX_STAGES;
+    uint64_t* tempty = tfull + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < MAX_STAGES; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&tfull[b], 1);
+            mbar_init(&tempty[b], NW);
+        }
+        *abort_flag = 0;
+        fence_barrier_init();
+        prefetch_tensormap(&tmK);
+        prefetch_tensormap(&tmQ);
+    }
+    const uint32_t ncols = 2u * p.acc_cols;
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, ncols);
+        tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+    chain_begin();
+
+    const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty), st0 = smem_u32(smem);
+    if (warp == 0) {
+        if (lane < 2) {                              // lane 0: key rows, lane 1: candidate rows (their copies overlap)
+            uint32_t s = 0, ph = 0;
+            bool ok = true;
+            for (Segment sg(p); sg.valid() && ok; sg.next(p)) {
+                const int b = sg.bh / p.H, h = sg.bh - b * p.H;
+                for (int kc = 0; kc < p.KC; ++kc) {
+                    ok = mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag);
+                    ok = __all_sync(0x3u, ok);
+                    if (!ok) { if (lane == 0) fail(abort_flag, 81); break; }
+                    const uint32_t st = st0 + s * stage_bytes, fb = full0 + 8 * s;
+                    if (lane == 0) mbar_expect_tx_a(fb, stage_bytes);
+                    __syncwarp(0x3u);
+                    if (lane == 0) tma_load_4d_a(st, &tmK, fb, kc * p.KCH, h, sg.row, b);
+                    else tma_load_4d_a(st + a_bytes, &tmQ, fb, kc * p.KCH, h, 0, b);
+                    if (++s == STAGES) { s = 0; ph ^= 1u; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = make_idesc_bf16_f32(BM, p.BN);
+            const uint64_t dhi = kmajor_desc_hi(pitch);
+            const int nk16 = p.KCH / 16;
+            const uint32_t tfull0 = smem_u32(tfull), tempty0 = smem_u32(tempty);
+            uint32_t s = 0, ph = 0, buf = 0, use = 0;
+            bool ok = true;
+            for (Segment sg(p); sg.valid() && ok; sg.next(p)) {
+                if (!mbar_wait_a(tempty0 + 8 * buf, (use & 1u) ^ 1u, abort_flag)) { fail(abort_flag, 82); break; }
+                tc_fence_after_sync();
+                for (int kc = 0; kc < p.KC; ++kc) {
+                    if (!mbar_wait_a(full0 + 8 * s, ph, abort_flag)) { fail(abort_flag, 83); ok = false; break; }
+                    tc_fence_after_sync();
+                    const uint32_t sa = st0 + s * stage_bytes;
+                    mma_chunk(tmem_base + buf * p.acc_cols, dhi | (uint64_t)(sa >> 4),
+                              dhi | (uint64_t)((sa + a_bytes) >> 4), idesc, nk16, kc != 0);
+                    mma_commit_a(empty0 + 8 * s);
+                    if (++s == STAGES) { s = 0; ph ^= 1u; }
+                }
+                if (ok) mma_commit_a(tfull0 + 8 * buf);
+                if (++buf == 2) { buf = 0; ++use; }
+            }
+        }
+    } else {
+        const int w = warp - 2;
+        const int tid = threadIdx.x - 64;
+        const int lq = warp & 3;                     // TMEM lane quarter it may read
+        const int sub = w >> 2;                      // its share of that quarter's columns
+        const int r = lq * 32 + lane;
+        float2* list = lists + w * WR * p.list_len;
+        const uint32_t list0 = smem_u32(list), list_stride = p.list_len * 8, found0 = smem_u32(found + w * R * 32 * E);
+        const bool stats = p.metric != CONVNN_MATMUL;
+        if (p.sampled)
+            for (int c = tid; c < p.BN; c += 32 * NW) cs[c] = c < p.S ? p.cand[c] : -1;
+        uint32_t buf = 0, use = 0;
+        const float none = __int_as_float(0x7fffffff);           // columns past the last candidate: their keys become NaN
+        // Every selection warp makes the same number of passes and meets every barrier, also after a wait has expired
+        // anywhere in the CTA (it then skips the work): none is left waiting for another.
+        Segment sg(p);
+        float q_next = none, kst_next = 1.f;
+        auto fetch = [&] {
+            if (tid < p.S) q_next = stats ? p.qstat[(long long)sg.bh * p.S + tid] : 1.f;
+            if (stats && r < sg.n) kst_next = p.kstat[sg.g + r];
+        };
+        if (sg.valid()) fetch();
+        while (sg.valid()) {
+            const float kst = kst_next;
+            if (tid < p.BN) qs[tid] = q_next;
+            const Segment cur = sg;
+            sg.next(p);
+            if (sg.valid()) fetch();
+            bool ok = mbar_wait(&tfull[buf], use & 1u, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok && lane == 0) fail(abort_flag, 84);
+            selection_barrier();                     // the key buffer is free, the column statistics are there
+            if (ok && lq * 32 < cur.n) {
+                tc_fence_after_sync();
+                if (sub == 0) kst_s[r] = kst;
+                const int row = cur.row + r;
+                const float sentinel = p.sampled ? self_sentinel(p.metric, kst, p.sqrt_dk) : 0.f;
+                float* out = keybuf + (r < p.seg_rows ? r : 0) * p.pitch;
+                const bool mine = r < cur.n;
+                const uint32_t taddr = tmem_base + ((uint32_t)(lq * 32) << 16) + buf * p.acc_cols;
+                auto store_keys = [&](const uint32_t (&acc)[16], int c) {
+#pragma unroll
+                    for (int j4 = 0; j4 < 4; ++j4) {
+                        const float4 s4 = *reinterpret_cast<const float4*>(qs + c + 4 * j4);
+                        const f32x2 d01 = pack2(__uint_as_float(acc[4 * j4]), __uint_as_float(acc[4 * j4 + 1]));
+                        const f32x2 d23 = pack2(__uint_as_float(acc[4 * j4 + 2]), __uint_as_float(acc[4 * j4 + 3]));
+                        f32x2 k01, k23;
+                        if (p.metric != CONVNN_EUCLIDEAN) {      // (matmul: statistics of 1)
+                            k01 = mul2(d01, pack2(s4.x, s4.y));
+                            k23 = mul2(d23, pack2(s4.z, s4.w));
+                        } else {
+                            const f32x2 two = pack2(2.0f, 2.0f);
+                            k01 = fma2(two, d01, pack2(-s4.x, -s4.y));
+                            k23 = fma2(two, d23, pack2(-s4.z, -s4.w));
+                        }
+                        float4 k;
+                        unpack2(k01, k.x, k.y);
+                        unpack2(k23, k.z, k.w);
+                        if (p.sampled) {
+                            const int4 c4 = *reinterpret_cast<const int4*>(cs + c + 4 * j4);
+                            if (c4.x == row) k.x = sentinel;
+                            if (c4.y == row) k.y = sentinel;
+                            if (c4.z == row) k.z = sentinel;
+                            if (c4.w == row) k.w = sentinel;
+                        }
+                        if (mine) *reinterpret_cast<float4*>(out + c + 4 * j4) = k;
+                    }
+                };
+                for (int c = sub * 16; c < p.BN; c += 128) {     // two blocks in flight
+                    uint32_t a0[16], a1[16];
+                    const bool two = c + 64 < p.BN;
+                    tmem_ld_x16(taddr + c, a0);
+                    if (two) tmem_ld_x16(taddr + c + 64, a1);
+                    tmem_ld_wait();
+                    store_keys(a0, c);
+                    if (two) store_keys(a1, c + 64);
+                }
+                tc_fence_before_sync();
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty[buf]);
+            selection_barrier();                     // the keys are there
+            if (!*abort_flag) {
+                uint32_t redo = 0;                   // bit n: row w + n NW
+                int n = 0;
+                auto select = [&](auto rows) {
+                    constexpr int RR = decltype(rows)::value;
+                    const uint32_t to = list0 + n * list_stride;
+                    redo |= select_rows<J, GR, E, (NS > 0 ? NS : 0), RR>(p, keybuf, found0, to, list_stride, w + n * NW) << n;
+                    n += RR;
+                };
+                while (w + (n + R - 1) * NW < cur.n) select(std::integral_constant<int, R>{});
+                if (w + n * NW < cur.n) select(std::integral_constant<int, 1>{});
+                for (; redo; redo &= redo - 1) {
+                    const int m = __ffs(redo) - 1;
+                    __syncwarp();
+                    select_ordered<J>(keybuf + (w + m * NW) * p.pitch, p.BN, p.nsel, list0 + m * list_stride);
+                }
+                __syncwarp();
+                // keys back to similarity values, columns back to tokens, the row itself first in the sampled modes
+                for (int e = lane; e < n * p.K; e += 32) {
+                    const int m = (int)((uint32_t)e * p.inv_K >> 16), slot = e - m * p.K;
+                    const int rw = w + m * NW, row = cur.row + rw;
+                    int tok = row;
+                    float s = 1.0f;
+                    if (!p.sampled || slot) {
+                        const float2 f = list[m * p.list_len + slot - p.sampled];
+                        const float kst_row = kst_s[rw];
+                        tok = __float_as_int(f.y);
+                        if (p.metric == CONVNN_COSINE) s = f.x * kst_row;
+                        else if (p.metric == CONVNN_MATMUL) s = f.x / p.sqrt_dk;
+                        else s = sqrtf(fmaxf(kst_row - f.x, 0.f));
+                        if (p.sampled) {
+                            tok = cs[tok];
+                            if (tok == row) s = (p.metric == CONVNN_EUCLIDEAN) ? 1.1f : -0.1f;
+                        }
+                    }
+                    const int to = (cur.g + rw) * p.K + slot;    // (B H T K < 2^31)
+                    p.idx[to] = tok;
+                    p.val[to] = s;
+                }
+            }
+            if (++buf == 2) { buf = 0; ++use; }
+        }
+    }
+
+    tc_fence_before_sync();
+    __syncthreads();
+    if (*abort_flag) {
+        // a wait expired: give copies still in flight time to land before the CTA's shared memory is released
+        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+        __syncthreads();
+    }
+    if (warp == 1) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem_base, ncols);
+    }
+}
+
+template <int J, int NS>
+int launch_rows(RowsParams& p, size_t smem, int grid, const CUtensorMap& tmK, const CUtensorMap& tmQ, cudaStream_t st) {
+    auto kern = sim_topk_rows_kernel<J, NS>;
+    CONVNN_ENSURE_SMEM(kern, smem);
+    launch_chained(kern, grid, NT, smem, st, tmK, tmQ, p);
+    CONVNN_CHECK_LAUNCH("sim_topk_rows");
+    return CONVNN_OK;
+}
+
+template <int J>
+int launch_rows_j(RowsParams& p, size_t smem, int grid, const CUtensorMap& tmK, const CUtensorMap& tmQ, cudaStream_t st) {
+    if (p.nsel == 8) return launch_rows<J, 8>(p, smem, grid, tmK, tmQ, st);
+    if (p.nsel == 9) return launch_rows<J, 9>(p, smem, grid, tmK, tmQ, st);
+    if (p.nsel <= 16) return launch_rows<J, 0>(p, smem, grid, tmK, tmQ, st);
+    if (p.nsel <= 25) return launch_rows<J, -1>(p, smem, grid, tmK, tmQ, st);
+    return launch_rows<J, -2>(p, smem, grid, tmK, tmQ, st);
+}
+
+}  // namespace
+
+static int rows_per_sm(const Dims& dm) {
+    const int sms = device_sms();
+    return (int)(((long long)dm.B * dm.H * dm.T + sms - 1) / sms + NW - 1) / NW * NW;
+}
+
+// What bounds it: warp instructions, ~300 per row of 197 keys with the copy, at 0.5 to 0.8 per cycle and scheduler.  A row
+// costs about the same wherever it runs, while the two-pass kernel works in whole 128-row units and the streaming kernel
+// needs many rows per SM to hide its chains.  us, others -> this kernel, 192 channels unless noted:
+//   197 x 197, K = 9         1 image 14.9 -> 6.5    37: 15.2 -> 8.8    148: 21.9 -> 17.1    220: 30.4 -> 26.2    256: 30.4 -> 30.2 (not taken)
+//   12 heads of 64           1 image 14.8 -> 6.6    16: 27.5 -> 22.3    32: 40.4 -> 37.8 (not taken)
+//   197 x 64 x 384, K = 9    1 image 9.2 -> 6.5     16: 9.5 -> 7.1      74: 9.8 -> 12.2 (not taken)
+//   197 x 197, K = 25        1 image 23.5 -> 8.2    16: 24.1 -> 21.0    48: 24.4 -> 28.3 (not taken)
+//   (two batches in flight lose 0.6 % with it at 256 images: a CTA of this kernel fills its SM)
+//   1000 x 256 x 768, K = 5  1 image 18.0 -> 9.9    4: 18.2 -> 11.1     16: 18.9 -> 21.5 (not taken)
+bool sim_topk_rows_wanted(const Dims& dm) {
+    if (dm.S > 256) return false;
+    const int rows = rows_per_sm(dm);
+    if (dm.nsel > 16) return rows <= 32;
+    return rows <= 48 || (dm.S > 128 && dm.Cp <= 384 && rows <= 304);
+}
+
+int launch_sim_topk_rows(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
+                         const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st) {
+    RowsParams p{};
+    p.qstat = qstat; p.kstat = kstat; p.cand = cand; p.idx = idx; p.val = val;
+    p.T = dm.T; p.S = dm.S; p.H = dm.H; p.K = dm.K; p.nsel = dm.nsel; p.metric = d->metric; p.sampled = d->sampled ? 1 : 0;
+    p.BN = (dm.S + 15) / 16 * 16;
+    p.pitch = p.BN + 4;
+    p.acc_cols = 32;
+    while (p.acc_cols < p.BN) p.acc_cols *= 2;
+    p.sqrt_dk = (float)sqrt((double)dm.dk);
+    p.rows_total = dm.B * dm.H * dm.T;
+    p.rows_per_cta = rows_per_sm(dm);
+    int grid = (int)(((long long)p.rows_total + p.rows_per_cta - 1) / p.rows_per_cta);
+    // ranges that do not cross from one (batch, head) to the next, where they need be no longer: a segment less each
+    const int parts = device_sms() / (dm.B * dm.H);
+    if (parts > 0) {
+        const int rows = ((dm.T + parts - 1) / parts + NW - 1) / NW * NW;
+        if (rows <= p.rows_per_cta + NW) {
+            p.rows_per_cta = rows;
+            p.per_head = (dm.T + rows - 1) / rows;
+            grid = dm.B * dm.H * p.per_head;
+        }
+    }
+    p.seg_rows = p.rows_per_cta < BM ? p.rows_per_cta : BM;
+    p.list_len = dm.nsel;
+    p.inv_K = (65536 + dm.K - 1) / dm.K;             // e / K = e * inv_K >> 16 for e < WR * K
+    const size_t fixed = 1024 + (size_t)p.seg_rows * p.pitch * 4 + (size_t)NW * WR * dm.nsel * 8 +
+                         (size_t)NW * R * (dm.nsel > 16 ? 64 : 32) * 8 + (size_t)p.BN * 8 + BM * 4 +
+                         (2 * MAX_STAGES + 4) * 8 + 16;
+    const size_t room = 226 * 1024 - fixed;
+    // (the copies fill what lies past a head with zeros; 32-channel chunks where only one of 64 would fit)
+    p.KCH = dm.Cp <= 16 ? 16 : (dm.Cp <= 32 ? 32 : 64);
+    if (p.KCH == 64 && room / ((size_t)(BM + p.BN) * 128) < 2) p.KCH = 32;
+    p.KC = (dm.Cp + p.KCH - 1) / p.KCH;
+    const size_t stage = (size_t)(BM + p.BN) * p.KCH * 2;
+    p.stages = (int)(room / stage);
+    if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
+    if (p.stages > 2 * p.KC) p.stages = 2 * p.KC;            // deeper than two segments' chunks serves nothing
+    size_t smem = fixed + p.stages * stage;
+    if (smem < 116 * 1024) smem = 116 * 1024;                // a CTA may take all of an SM's TMEM: never two on one SM
+
+    CUtensorMap tmK, tmQ;
+    const uint64_t dimsK[4] = {(uint64_t)dm.Cp, (uint64_t)dm.H, (uint64_t)dm.T, (uint64_t)dm.B};
+    const uint64_t dimsQ[4] = {(uint64_t)dm.Cp, (uint64_t)dm.H, (uint64_t)dm.S, (uint64_t)dm.B};
+    const uint64_t strK[3] = {(uint64_t)dm.Cp * 2, (uint64_t)dm.H * dm.Cp * 2, (uint64_t)dm.T * dm.H * dm.Cp * 2};
+    const uint64_t strQ[3] = {(uint64_t)dm.Cp * 2, (uint64_t)dm.H * dm.Cp * 2, (uint64_t)dm.S * dm.H * dm.Cp * 2};
+    const uint32_t boxK[4] = {(uint32_t)p.KCH, 1, (uint32_t)BM, 1};
+    const uint32_t boxQ[4] = {(uint32_t)p.KCH, 1, (uint32_t)p.BN, 1};
+    if (!encode_tensor_map_bf16(&tmK, k, 4, dimsK, strK, boxK, p.KCH * 2)) return CONVNN_E_CUDA;
+    if (!encode_tensor_map_bf16(&tmQ, q, 4, dimsQ, strQ, boxQ, p.KCH * 2)) return CONVNN_E_CUDA;
+
+    switch ((p.BN + 31) / 32) {
+        case 1: return launch_rows_j<1>(p, smem, grid, tmK, tmQ, st);
+        case 2: return launch_rows_j<2>(p, smem, grid, tmK, tmQ, st);
+        case 3: return launch_rows_j<3>(p, smem, grid, tmK, tmQ, st);
+        case 4: return launch_rows_j<4>(p, smem, grid, tmK, tmQ, st);
+        case 5: return launch_rows_j<5>(p, smem, grid, tmK, tmQ, st);
+        case 6: return launch_rows_j<6>(p, smem, grid, tmK, tmQ, st);
+        case 7: return launch_rows_j<7>(p, smem, grid, tmK, tmQ, st);
+        default: return launch_rows_j<8>(p, smem, grid, tmK, tmQ, st);
+    }
+}
+
+int read_sim_rows_status(int* out) {
+    int v = 0;
+    cudaError_t e = cudaMemcpyFromSymbol(&v, g_sim_rows_status, sizeof(int));
+    if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "cudaMemcpyFromSymbol: %s", cudaGetErrorString(e));
+    *out = v;
+    return CONVNN_OK;
+}
+
+}  // namespace convnn

@@ -428,8 +428,8 @@ int launch_short(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const C
 
 }  // namespace
 
-// Where the streaming kernel leaves most of the chip idle: up to one unit per SM.  B x 197 tokens of 192 channels, K = 9:
-// 15.4 us for 1 to 74 images, streaming 21.6; 256 images (3.5 units per SM) 34.6 against 30.8, where eight to sixteen
+// What the warp-per-row kernel leaves to it where the streaming kernel would leave most of the chip idle: up to one unit per
+// SM.  B x 197 tokens of 192 channels, K = 9: 15.4 us for 1 to 74 images, streaming 21.6; 256 images (3.5 units per SM) 34.6 against 30.8, where eight to sixteen
 // streaming warps per SM hide each other's latency.  Lists of 13 to 16 always: their streaming variant runs one CTA per SM
 // (577 tokens, 150 candidates, K = 16: 1 image 26.4 -> 18.5 us, 74 images 49.9 -> 39.8, 256 images 132 -> 107).
 bool sim_topk_short_wanted(const Dims& dm) {

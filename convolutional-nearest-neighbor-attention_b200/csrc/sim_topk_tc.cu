@@ -289,6 +289,7 @@ bool sim_topk_tc_supported(const convnn_desc* d, const Dims& dm, const void* q, 
 
 int launch_sim_topk_tc(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
                        const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st) {
+    if (sim_topk_rows_wanted(dm)) return launch_sim_topk_rows(d, dm, q, k, qstat, kstat, cand, idx, val, st);
     if (sim_topk_short_wanted(dm)) return launch_sim_topk_short(d, dm, q, k, qstat, kstat, cand, idx, val, st);
     if (sim_topk_tc2_wanted(d, dm)) return launch_sim_topk_tc2(d, dm, q, k, qstat, kstat, cand, idx, val, st);
     TcParams p{};

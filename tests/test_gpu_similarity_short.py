@@ -77,3 +77,37 @@ def test_metrics_at_the_ends(metric):
     bound = (dk + 16) * 2.0 ** -24 * (1.0 if metric == "cosine" else 4.0 * math.sqrt(dk))
     assert float((val.double() - want).abs().max()) <= bound
     assert float((torch.gather(sim, -1, idx.long()) - val.double()).abs().max()) <= bound
+
+
+# Batches at which a CTA of the warp-per-row kernel has several segments (whole sequences, ends, ranges across heads), and
+# the first ones that go to the two-pass and the streaming kernel instead.
+@pytest.mark.parametrize("T,S,H,dk,K,B", [(197, 197, 1, 64, 9, 90), (197, 197, 3, 32, 9, 64), (197, 197, 1, 32, 9, 300),
+                                          (150, 150, 1, 16, 16, 152), (1, 1, 1, 16, 1, 3000), (33, 17, 1, 32, 9, 150),
+                                          (130, 130, 2, 64, 5, 74), (300, 200, 1, 48, 12, 149), (65, 65, 1, 64, 25, 60),
+                                          (197, 64, 1, 64, 9, 74), (197, 197, 1, 64, 25, 60), (197, 64, 1, 64, 9, 200)])
+@pytest.mark.parametrize("values", ["few", "many", "nan"])
+def test_exact_lists_of_many_rows(T, S, H, dk, K, B, values):
+    sampled = S != T
+    n = K - 1 if sampled else K
+    g = torch.Generator(device=DEV).manual_seed(T + S + K + B)
+    top = 1 if values == "few" else 40               # products and sums stay below 2^24
+    q, k = (torch.randint(-top, top + 1, (B, r, H, dk), device=DEV, generator=g).float() for r in (S, T))
+    if values == "nan":
+        q[1::2, ::2] = math.nan
+        q[2::3, 2:] = math.nan
+    spec = ops.LayerSpec(H * dk, H, K, "spatial" if sampled else "all", "matmul", "depthwise", True, False, T)
+    cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if sampled else None
+    idx, val = ops.sim_topk(spec, q.bfloat16(), k.bfloat16(), None, None, cand)
+    key = torch.einsum("bthc,bshc->bhts", k.double(), q.double()).float()        # whole numbers: exact
+    if sampled:
+        own = cand.view(1, 1, 1, S).long() == torch.arange(T, device=DEV).view(1, 1, T, 1)
+        key = torch.where(own, torch.full_like(key, -0.1) * torch.tensor(math.sqrt(dk), dtype=torch.float32, device=DEV), key)
+    want_idx, want_key = expect(key, n)
+    want_tok = want_idx if cand is None else cand.long()[want_idx]
+    assert torch.equal(idx.long()[..., K - n:], want_tok)
+    if sampled:
+        assert torch.equal(idx.long()[..., 0], torch.arange(T, device=DEV).expand(B, H, T))
+    real = (want_key > -math.inf) & (want_tok != torch.arange(T, device=DEV).view(1, 1, T, 1) if sampled else want_key > -math.inf)
+    want_val = want_key / torch.tensor(math.sqrt(dk), dtype=torch.float32, device=DEV)
+    # one division: equal up to its rounding
+    assert bool(((val[..., K - n:] - want_val).abs()[real] <= 2.0 ** -22 * want_val.abs()[real]).all())
