@@ -2,28 +2,17 @@
 //
 // A thread per row (the TMEM layout) leaves at most 256 rows in flight per SM and chains of dependent comparisons.  Here the
 // accumulator is copied once to shared memory as ranking keys, row by row, and sixteen warps take rows from there: lane l
-// holds columns l, l + 32, ..., two rows are interleaved, nothing diverges and no lane idles on a ragged sequence end.
-//
-//   bound      the nsel-th largest of the 32 lane maxima (nsel warp-wide maxima): at least nsel keys reach it
-//   survivors  the keys that reach it (9 of 197: ~10.5) are packed into shared memory
-//   rank       every survivor counts the survivors above it: its slot of the list
-//
-// Lists are collected in shared memory as (key, column) and written out a warp's rows at a time.  A row with equal keys among
-// its best, with more survivors than the buffer holds, or with fewer than nsel keys above -inf (NaN inputs) takes its list one
-// (key, column) maximum at a time instead; the lists are the streaming kernels' bit for bit.
+// holds columns l, l + 32, ..., two rows are interleaved, nothing diverges and no lane idles on a ragged sequence end (topk_rows.cuh).
 //
 // A persistent CTA per SM owns an equal share of the flattened (batch, head, row) range, in segments of up to 128 rows of
 // one (batch, head), wherever they start.  Warp 0: TMA producer (128 key rows from the segment's first, all
 // candidate rows, 64-channel chunks, ring); warp 1: MMA issuer (M = 128, N = S rounded to 16), two accumulators; warps 2-17:
 // copy and selection.
-#include <limits.h>
-
-#include <type_traits>
-
 #include "common.cuh"
 #include "f32x2.cuh"
 #include "sim_topk_select.cuh"
 #include "sm100.cuh"
+#include "topk_rows.cuh"
 
 namespace convnn {
 
@@ -32,11 +21,11 @@ __device__ int g_sim_rows_status = 0;
 namespace {
 
 using namespace sm100;
+using namespace topk_rows;
 
 constexpr int BM = 128;
 constexpr int MAX_STAGES = 6;
 constexpr int NW = 16;                  // selection warps
-constexpr int R = 2;                    // rows a warp interleaves
 constexpr int WR = BM / NW;             // most rows of a segment per warp
 constexpr int NT = 64 + 32 * NW;
 
@@ -51,7 +40,7 @@ struct RowsParams {
                         // consecutive rows fall into different banks)
     int acc_cols;       // TMEM columns of one accumulator
     int seg_rows;       // most rows of a segment (rows of the key buffer)
-    int list_len, inv_K;
+    int inv_K;
     int stages;
     int rows_total, rows_per_cta, per_head;
     float sqrt_dk;
@@ -60,27 +49,6 @@ struct RowsParams {
 __device__ __forceinline__ void fail(volatile int* abort_flag, int code) {
     *abort_flag = 1;
     atomicCAS(&g_sim_rows_status, 0, code);
-}
-
-__device__ __forceinline__ float max3(float a, float b, float c) {
-    float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-// Largest value of the warp (NaN only if every lane holds NaN).
-__device__ __forceinline__ float warp_max(float v) {
-    float r;
-    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
-}
-template <int N>
-__device__ __forceinline__ float max_of(const float (&v)[N], int first, int step) {
-    float m = v[first];
-    int j = first + step;
-#pragma unroll
-    for (; j + step < N; j += 2 * step) m = max3(m, v[j], v[j + step]);
-    if (j < N) m = fmaxf(m, v[j]);
-    return m;
 }
 
 // A CTA's range of flattened rows, cut into segments of one (batch, head).  Ranges follow each other; with `per_head` set they
@@ -111,189 +79,12 @@ struct Segment {
     }
 };
 
-__device__ __forceinline__ void sts_entry(uint32_t at, float key, int col) {
-    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(__float_as_uint(key)), "r"(col) : "memory");
-}
-
-// Exact list of one row under the full (key, column) order, one maximum at a time; keys of -inf and NaN never enter.
-template <int J>
-__device__ __noinline__ void select_ordered(const float* keys, int BN, int nsel, uint32_t list) {
-    const int lane = threadIdx.x & 31;
-    float v[J];
-#pragma unroll
-    for (int j = 0; j < J; ++j) v[j] = 32 * j + lane < BN ? keys[32 * j + lane] : -CUDART_INF_F;
-    float last = CUDART_INF_F;
-    int last_col = -1;
-    for (int s = 0; s < nsel; ++s) {
-        float best = -CUDART_INF_F;
-        int col = INT_MAX;
-#pragma unroll
-        for (int j = 0; j < J; ++j) {
-            const int c = 32 * j + lane;
-            if ((v[j] < last || (v[j] == last && c > last_col)) && v[j] > best) { best = v[j]; col = c; }
-        }
-        last = warp_max(best);
-        last_col = __reduce_min_sync(0xffffffffu, best == last ? col : INT_MAX);
-        if (!(last > -CUDART_INF_F)) last_col = 0;
-        if (lane == 0) sts_entry(list + s * 8, last, last_col);
-    }
-}
-
-// Keys that reach the bound: (key, column) pairs at `at`, which moves on.
-__device__ __forceinline__ void store_if_reached(float key, float bound, int col, uint32_t& at) {
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "setp.ge.f32 p, %1, %2;\n\t"
-                 "@p st.shared.v2.b32 [%0], {%3, %4};\n\t"
-                 "@p add.u32 %0, %0, 8;\n\t}"
-                 : "+r"(at) : "f"(key), "f"(bound), "r"(__float_as_uint(key)), "r"(col) : "memory");
-}
-__device__ __forceinline__ float4 lds_v4(uint32_t at) {
-    float4 r;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(at) : "memory");
-    return r;
-}
-
-// R rows of the key buffer at once (rows at, at + NW, ...): J columns per lane, GR groups of them per lane whose maxima give
-// the bound, room for 32 E survivors per row at `found`.  Returns the rows (bit r) that need select_ordered().
-template <int J, int GR, int E, int NS, int R>
-__device__ __forceinline__ uint32_t select_rows(const RowsParams& p, const float* keybuf, uint32_t found, uint32_t list,
-                                                     uint32_t list_stride, int at) {
-    constexpr int CAP = 32 * E;
-    const int lane = threadIdx.x & 31;
-    const uint32_t below = (1u << lane) - 1u;
-    const int nsel = NS ? NS : p.nsel;
-    float v[R][J];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const float* kr = keybuf + (at + r * NW) * p.pitch + lane;
-#pragma unroll
-        for (int j = 0; j < J - 1; ++j) v[r][j] = kr[32 * j];
-        v[r][J - 1] = -CUDART_INF_F;
-        if (32 * (J - 1) + lane < p.BN) v[r][J - 1] = kr[32 * (J - 1)];
-    }
-    float m[R][GR], bound[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int q = 0; q < GR; ++q) m[r][q] = max_of<J>(v[r], q < J ? q : 0, GR);
-#pragma unroll
-    for (int r = 0; r < R; ++r) bound[r] = warp_max(GR == 2 ? fmaxf(m[r][0], m[r][GR - 1]) : m[r][0]);
-    auto lower = [&] {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-#pragma unroll
-            for (int q = 0; q < GR; ++q) m[r][q] = m[r][q] == bound[r] ? -CUDART_INF_F : m[r][q];
-            bound[r] = warp_max(GR == 2 ? fmaxf(m[r][0], m[r][GR - 1]) : m[r][0]);
-        }
-    };
-    if (NS) {
-#pragma unroll
-        for (int s = 1; s < NS; ++s) lower();
-    } else {
-#pragma unroll 1
-        for (int s = 1; s < nsel; ++s) lower();
-    }
-    // where each lane's survivors go: exclusive prefix of the lanes' counts, bit by bit
-    int mine[R], before[R], n[R], most = 0;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        mine[r] = 0;
-#pragma unroll
-        for (int j = 0; j < J; ++j)
-            if (v[r][j] >= bound[r]) ++mine[r];
-        before[r] = __popc(__ballot_sync(0xffffffffu, mine[r] & 1) & below);
-        if (J >= 2) before[r] += 2 * __popc(__ballot_sync(0xffffffffu, mine[r] & 2) & below);
-        most = max(most, mine[r]);
-    }
-    if (J >= 4 && __any_sync(0xffffffffu, most >= 4)) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            before[r] += 4 * __popc(__ballot_sync(0xffffffffu, mine[r] & 4) & below);
-            if (J >= 8) before[r] += 8 * __popc(__ballot_sync(0xffffffffu, mine[r] & 8) & below);
-        }
-    }
-    uint32_t redo = 0;
-    int n_max = 0;
-#pragma unroll
-    for (int r = 0; r < R; ++r) n[r] = __shfl_sync(0xffffffffu, before[r] + mine[r], 31);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        if (n[r] > CAP || !(bound[r] > -CUDART_INF_F)) {
-            redo |= 1u << r;                     // (keys of +inf may still be stored: a lane's J from slot 0 on)
-            n[r] = 0;
-            bound[r] = CUDART_INF_F;
-            before[r] = 0;
-        }
-        n_max = max(n_max, n[r]);
-        uint32_t to = found + (r * CAP + before[r]) * 8;
-#pragma unroll
-        for (int j = 0; j < J; ++j) store_if_reached(v[r][j], bound[r], 32 * j + lane, to);
-#pragma unroll
-        for (int e = 0; e < E; ++e)
-            if (lane + 32 * e >= n[r])
-                asm volatile("st.shared.b32 [%0], %1;" ::"r"(found + (r * CAP + lane + 32 * e) * 8), "r"(0xff800000u) : "memory");
-    }
-    __syncwarp();
-    float key[R][E];
-    int col[R][E], rank[R][E];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=f"(key[r][e]), "=r"(col[r][e])
-                         : "r"(found + (r * CAP + lane + 32 * e) * 8) : "memory");
-            rank[r][e] = 0;
-        }
-    }
-    auto count_above = [&](int i) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const float4 a = lds_v4(found + (r * CAP + i) * 8), b = lds_v4(found + (r * CAP + i) * 8 + 16);
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                if (a.x > key[r][e]) ++rank[r][e];
-                if (a.z > key[r][e]) ++rank[r][e];
-                if (b.x > key[r][e]) ++rank[r][e];
-                if (b.z > key[r][e]) ++rank[r][e];
-            }
-        }
-    };
-    constexpr int FIRST = NS ? (NS + 3) / 4 * 4 : 0;    // (9 of 197 columns: 12 survivors suffice for nine rows in ten)
-#pragma unroll
-    for (int i = 0; i < FIRST; i += 4) count_above(i);
-#pragma unroll 1
-    for (int i = FIRST; i < n_max; i += 4) count_above(i);
-    __syncwarp();
-    // A lane past the survivors holds -inf and rank n.  Equal keys share a rank and leave a later one out: the list is right
-    // if the ranks below nsel all occur and are nsel in number.
-    const uint32_t all = nsel == 32 ? 0xffffffffu : (1u << nsel) - 1u;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        uint32_t bits = 0;
-        int listed = 0;
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const bool in = rank[r][e] < nsel;
-            listed += __popc(__ballot_sync(0xffffffffu, in));
-            if (in) bits |= 1u << rank[r][e];
-        }
-        const bool good = __reduce_or_sync(0xffffffffu, bits) == all && listed == nsel && !(redo >> r & 1u);
-        if (!good) redo |= 1u << r;
-#pragma unroll
-        for (int e = 0; e < E; ++e)
-            if (good && rank[r][e] < nsel) sts_entry(list + r * list_stride + rank[r][e] * 8, key[r][e], col[r][e]);
-    }
-    return redo;
-}
-
 __device__ __forceinline__ void selection_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory"); }
 
-// NS: number of neighbours where it is fixed, 0: any up to 16, -1: up to 25, -2: up to 32.
-template <int J, int NS>
+template <int J, int NS>          // as in select_and_write()
 __global__ void __launch_bounds__(NT, 1)
 sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ,
                      const __grid_constant__ RowsParams p) {
-    constexpr int E = NS < 0 ? 2 : 1, GR = NS == -2 && J > 1 ? 2 : 1;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t pitch = p.KCH * 2;
@@ -301,8 +92,8 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     const uint32_t STAGES = p.stages;
     float* keybuf = reinterpret_cast<float*>(smem + STAGES * stage_bytes);      // [seg_rows][pitch]
     float2* lists = reinterpret_cast<float2*>(keybuf + p.seg_rows * p.pitch);   // [NW][WR][nsel] key, column
-    float2* found = lists + NW * WR * p.list_len;                               // [NW][R][32 E] survivors: key, column
-    float* qs = reinterpret_cast<float*>(found + NW * R * 32 * E);              // [BN] column statistics
+    float2* found = lists + NW * WR * p.nsel;                                   // [NW][found_pairs] survivors: key, column
+    float* qs = reinterpret_cast<float*>(found + NW * found_pairs(NS));         // [BN] column statistics
     int* cs = reinterpret_cast<int*>(qs + p.BN);                                // [BN] candidate tokens
     float* kst_s = reinterpret_cast<float*>(cs + p.BN);                         // [BM] row statistics
     uint64_t* full = reinterpret_cast<uint64_t*>(kst_s + BM);
@@ -388,8 +179,9 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         const int lq = warp & 3;                     // TMEM lane quarter it may read
         const int sub = w >> 2;                      // its share of that quarter's columns
         const int r = lq * 32 + lane;
-        float2* list = lists + w * WR * p.list_len;
-        const uint32_t list0 = smem_u32(list), list_stride = p.list_len * 8, found0 = smem_u32(found + w * R * 32 * E);
+        float2* list = lists + w * WR * p.nsel;
+        const uint32_t found0 = smem_u32(found + w * found_pairs(NS));
+        const RowsTask task{kst_s, cs, p.idx, p.val, p.pitch, p.BN, p.nsel, p.K, p.inv_K, p.metric, p.sampled, p.sqrt_dk};
         const bool stats = p.metric != CONVNN_MATMUL;
         if (p.sampled)
             for (int c = tid; c < p.BN; c += 32 * NW) cs[c] = c < p.S ? p.cand[c] : -1;
@@ -465,44 +257,7 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             if (lane == 0) mbar_arrive(&tempty[buf]);
             selection_barrier();                     // the keys are there
             if (!*abort_flag) {
-                uint32_t redo = 0;                   // bit n: row w + n NW
-                int n = 0;
-                auto select = [&](auto rows) {
-                    constexpr int RR = decltype(rows)::value;
-                    const uint32_t to = list0 + n * list_stride;
-                    redo |= select_rows<J, GR, E, (NS > 0 ? NS : 0), RR>(p, keybuf, found0, to, list_stride, w + n * NW) << n;
-                    n += RR;
-                };
-                while (w + (n + R - 1) * NW < cur.n) select(std::integral_constant<int, R>{});
-                if (w + n * NW < cur.n) select(std::integral_constant<int, 1>{});
-                for (; redo; redo &= redo - 1) {
-                    const int m = __ffs(redo) - 1;
-                    __syncwarp();
-                    select_ordered<J>(keybuf + (w + m * NW) * p.pitch, p.BN, p.nsel, list0 + m * list_stride);
-                }
-                __syncwarp();
-                // keys back to similarity values, columns back to tokens, the row itself first in the sampled modes
-                for (int e = lane; e < n * p.K; e += 32) {
-                    const int m = (int)((uint32_t)e * p.inv_K >> 16), slot = e - m * p.K;
-                    const int rw = w + m * NW, row = cur.row + rw;
-                    int tok = row;
-                    float s = 1.0f;
-                    if (!p.sampled || slot) {
-                        const float2 f = list[m * p.list_len + slot - p.sampled];
-                        const float kst_row = kst_s[rw];
-                        tok = __float_as_int(f.y);
-                        if (p.metric == CONVNN_COSINE) s = f.x * kst_row;
-                        else if (p.metric == CONVNN_MATMUL) s = f.x / p.sqrt_dk;
-                        else s = sqrtf(fmaxf(kst_row - f.x, 0.f));
-                        if (p.sampled) {
-                            tok = cs[tok];
-                            if (tok == row) s = (p.metric == CONVNN_EUCLIDEAN) ? 1.1f : -0.1f;
-                        }
-                    }
-                    const int to = (cur.g + rw) * p.K + slot;    // (B H T K < 2^31)
-                    p.idx[to] = tok;
-                    p.val[to] = s;
-                }
+                select_and_write<J, NS, NW>(task, keybuf, list, found0, w, cur.n, cur.g, cur.row);
             }
             if (++buf == 2) { buf = 0; ++use; }
         }
@@ -586,10 +341,9 @@ int launch_sim_topk_rows(const convnn_desc* d, const Dims& dm, const void* q, co
         }
     }
     p.seg_rows = p.rows_per_cta < BM ? p.rows_per_cta : BM;
-    p.list_len = dm.nsel;
-    p.inv_K = (65536 + dm.K - 1) / dm.K;             // e / K = e * inv_K >> 16 for e < WR * K
+    p.inv_K = inverse_of(dm.K);
     const size_t fixed = 1024 + (size_t)p.seg_rows * p.pitch * 4 + (size_t)NW * WR * dm.nsel * 8 +
-                         (size_t)NW * R * (dm.nsel > 16 ? 64 : 32) * 8 + (size_t)p.BN * 8 + BM * 4 +
+                         (size_t)NW * found_pairs(dm.nsel > 16 ? -1 : 0) * 8 + (size_t)p.BN * 8 + BM * 4 +
                          (2 * MAX_STAGES + 4) * 8 + 16;
     const size_t room = 226 * 1024 - fixed;
     // (the copies fill what lies past a head with zeros; 32-channel chunks where only one of 64 would fit)

@@ -1,10 +1,13 @@
 // bfloat16 instantiations of the SIMT similarity + top-K kernel.
 #include "sim_topk_simt.cuh"
+#include "sim_topk_simt_rows.cuh"
 
 namespace convnn {
 int launch_sim_topk_simt_bf16(const convnn_desc* d, const Dims& dm, const void* q, const void* k,
                               const float* qstat, const float* kstat, const int32_t* cand, int32_t* idx,
                               float* val, cudaStream_t st) {
+    if (simt_topk_rows::wanted(dm))
+        return simt_topk_rows::dispatch<__nv_bfloat16>(d, dm, q, k, qstat, kstat, cand, idx, val, st);
     return simt_topk::dispatch<__nv_bfloat16>(d, dm, q, k, qstat, kstat, cand, idx, val, st);
 }
 }  // namespace convnn

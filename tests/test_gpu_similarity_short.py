@@ -111,3 +111,30 @@ def test_exact_lists_of_many_rows(T, S, H, dk, K, B, values):
     want_val = want_key / torch.tensor(math.sqrt(dk), dtype=torch.float32, device=DEV)
     # one division: equal up to its rounding
     assert bool(((val[..., K - n:] - want_val).abs()[real] <= 2.0 ** -22 * want_val.abs()[real]).all())
+
+
+# float32 through the kernel that takes the whole candidate list at once: edges of its 32-row blocks, 32-column groups and
+# 32-channel steps, and the last shape goes to the streaming kernel.
+@pytest.mark.parametrize("T,S,H,dk,K,B", [(1, 1, 1, 3, 1, 1), (31, 31, 1, 32, 9, 2), (33, 33, 2, 33, 5, 2), (65, 65, 1, 192, 9, 3),
+                                          (40, 32, 3, 20, 16, 2), (70, 64, 1, 31, 9, 2), (100, 97, 1, 64, 25, 2), (96, 96, 1, 65, 32, 2),
+                                          (129, 129, 1, 16, 9, 2), (300, 150, 1, 48, 16, 2), (197, 197, 3, 64, 9, 4),
+                                          (256, 256, 1, 7, 12, 2), (257, 225, 1, 40, 26, 2), (64, 40, 1, 8, 9, 500)])
+@pytest.mark.parametrize("values", ["few", "many", "nan"])
+def test_exact_lists_float32(T, S, H, dk, K, B, values):
+    sampled = S != T
+    n = K - 1 if sampled else K
+    g = torch.Generator(device=DEV).manual_seed(T + S + K + dk)
+    top = 1 if values == "few" else 50               # products and sums stay below 2^24
+    q, k = (torch.randint(-top, top + 1, (B, r, H, dk), device=DEV, generator=g).float() for r in (S, T))
+    if values == "nan":
+        q[:, ::3] = math.nan
+        q[:1, 2:] = math.nan
+    spec = ops.LayerSpec(H * dk, H, K, "spatial" if sampled else "all", "matmul", "depthwise", True, False, T)
+    cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if sampled else None
+    idx, _ = ops.sim_topk(spec, q, k, None, None, cand)
+    key = torch.einsum("bthc,bshc->bhts", k.double(), q.double()).float()        # whole numbers: exact
+    if sampled:
+        own = cand.view(1, 1, 1, S).long() == torch.arange(T, device=DEV).view(1, 1, T, 1)
+        key = torch.where(own, torch.full_like(key, -0.1) * torch.tensor(math.sqrt(dk), dtype=torch.float32, device=DEV), key)
+    want_idx, _ = expect(key, n)
+    assert torch.equal(idx.long()[..., K - n:], want_idx if cand is None else cand.long()[want_idx])
