@@ -331,8 +331,7 @@ int qkv_proj_impl(const convnn_desc* d, const void* x, int64_t ldx, const void* 
         }
         if (done) {
             if (fuse || !stats) return CONVNN_OK;
-            if ((rc = launch_head_fill_and_stats(d, dm, q, dm.S, qstat, st))) return rc;
-            return launch_head_fill_and_stats(d, dm, k, dm.T, kstat, st);
+            return launch_head_fill_and_stats(d, dm, q, qstat, k, kstat, nullptr, st);
         }
     }
     if (pn) return set_error(CONVNN_E_UNSUPPORTED, "prenorm_forward: this descriptor takes the unfused path");
@@ -349,10 +348,7 @@ int qkv_proj_impl(const convnn_desc* d, const void* x, int64_t ldx, const void* 
         p.w = static_cast<const char*>(w_qkv) + 2 * wsz; p.c = q; p.c1 = nullptr;
         if ((rc = launch_gemm_simt(d->dtype, p, st))) return rc;
     }
-    if ((rc = launch_head_fill_and_stats(d, dm, q, dm.S, stats ? qstat : nullptr, st))) return rc;
-    if ((rc = launch_head_fill_and_stats(d, dm, k, dm.T, stats ? kstat : nullptr, st))) return rc;
-    if ((rc = launch_head_fill_and_stats(d, dm, v, dm.T, nullptr, st))) return rc;
-    return CONVNN_OK;
+    return launch_head_fill_and_stats(d, dm, q, stats ? qstat : nullptr, k, stats ? kstat : nullptr, v, st);
 }
 }  // namespace
 

@@ -152,7 +152,9 @@ struct GemmParams {
 
 int launch_gemm_simt(int dtype, const GemmParams& p, cudaStream_t st);
 
-int launch_head_fill_and_stats(const convnn_desc* d, const Dims& dm, void* t, int rows, float* stat,
+// Coordinate and padding channels and / or the similarity's statistic of stored q, k, v (nullptr: not this tensor / no
+// statistic), in one launch.
+int launch_head_fill_and_stats(const convnn_desc* d, const Dims& dm, void* q, float* qstat, void* k, float* kstat, void* v,
                                cudaStream_t st);
 int launch_sim_topk_simt_f32(const convnn_desc* d, const Dims& dm, const void* q, const void* k,
                              const float* qstat, const float* kstat, const int32_t* cand,

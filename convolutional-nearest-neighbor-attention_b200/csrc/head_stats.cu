@@ -17,10 +17,20 @@ __device__ __forceinline__ float linspace_pm1(int i, int steps) {
     return (i < steps / 2) ? (-1.0f + step * (float)i) : (1.0f - step * (float)(steps - 1 - i));
 }
 
+// Up to three tensors of one layer in a launch, one per grid row (a launch each, before: 2.5 us per tensor at 2080 rows of
+// 192 float32 channels, all of it latency).
+struct HeadTensors {
+    void* t[3];
+    float* stat[3];
+    int rows[3];
+};
+
 template <typename T>
-__global__ void head_stats_kernel(T* t, float* stat, int B, int rows, int H, int dk, int C, int Cp,
-                                  int coord, int metric) {
+__global__ void head_stats_kernel(const HeadTensors in, int B, int H, int dk, int C, int Cp, int coord, int metric) {
     chain_begin();
+    T* t = static_cast<T*>(in.t[blockIdx.y]);
+    float* stat = in.stat[blockIdx.y];
+    const int rows = in.rows[blockIdx.y];
     const int warps_per_block = blockDim.x >> 5;
     const long long total = (long long)B * rows * H;
     const int lane = threadIdx.x & 31;
@@ -67,20 +77,27 @@ __global__ void head_stats_kernel(T* t, float* stat, int B, int rows, int H, int
 
 }  // namespace
 
-int launch_head_fill_and_stats(const convnn_desc* d, const Dims& dm, void* t, int rows, float* stat,
+int launch_head_fill_and_stats(const convnn_desc* d, const Dims& dm, void* q, float* qstat, void* k, float* kstat, void* v,
                                cudaStream_t st) {
-    if (!d->coord && !stat) return CONVNN_OK;
-    long long total = (long long)dm.B * rows * dm.H;
-    int blocks = (int)((total + 7) / 8);
-    if (blocks > 148 * 16) blocks = 148 * 16;
+    HeadTensors in{};
+    int n = 0, most = 0;
+    auto add = [&](void* t, int rows, float* stat) {
+        if (!t || (!d->coord && !stat)) return;
+        in.t[n] = t; in.stat[n] = stat; in.rows[n++] = rows;
+        if (rows > most) most = rows;
+    };
+    add(q, dm.S, qstat);
+    add(k, dm.T, kstat);
+    add(v, dm.T, nullptr);
+    if (n == 0) return CONVNN_OK;
+    const long long total = (long long)dm.B * most * dm.H;
+    int blocks = (int)((total + 7) / 8 < 148 * 16 ? (total + 7) / 8 : 148 * 16);
     if (blocks < 1) blocks = 1;
     if (d->dtype == CONVNN_F32)
-        launch_chained(head_stats_kernel<float>, blocks, 256, 0, st, static_cast<float*>(t), stat, dm.B, rows, dm.H,
-                                                        dm.dk, dm.C, dm.Cp, d->coord, d->metric);
+        launch_chained(head_stats_kernel<float>, dim3(blocks, n), 256, 0, st, in, dm.B, dm.H, dm.dk, dm.C, dm.Cp, d->coord, d->metric);
     else
-        launch_chained(head_stats_kernel<__nv_bfloat16>, blocks, 256, 0, st, static_cast<__nv_bfloat16*>(t), stat, dm.B,
-                                                                rows, dm.H, dm.dk, dm.C, dm.Cp, d->coord,
-                                                                d->metric);
+        launch_chained(head_stats_kernel<__nv_bfloat16>, dim3(blocks, n), 256, 0, st, in, dm.B, dm.H, dm.dk, dm.C, dm.Cp, d->coord,
+                       d->metric);
     CONVNN_CHECK_LAUNCH("head_stats");
     return CONVNN_OK;
 }
