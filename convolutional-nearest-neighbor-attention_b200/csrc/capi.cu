@@ -232,6 +232,7 @@ int convnn_b200_device_status(int* code) {
     if (!c && (rc = read_dw_stream_status(&c))) return rc;
     if (!c && (rc = read_attention_status(&c))) return rc;
     if (!c && (rc = read_mlp_tc_status(&c))) return rc;
+    if (!c && (rc = read_conv1d_tc_status(&c))) return rc;
     *code = a ? a : (b ? b : c);
     return CONVNN_OK;
 }
@@ -739,9 +740,14 @@ int convnn_b200_conv1d_attention(int dtype, const void* x, int64_t ldx, const vo
     void *y = ws, *o = ws + part, *merged = ws + 2 * part, *unfold = ws + 3 * part;
     const long long M = (long long)B * T;
     if ((rc = convnn_b200_linear(dtype, x, ldx, w_x, b_x, nullptr, 0, y, D, M, D, D, 0, stream))) return rc;
-    if ((rc = launch_conv1d_heads(dtype, y, w_conv, b_conv, o, unfold, B, T, H, D / H, kernel_size, st))) return rc;
     // the reference reads the per-head (T, d_k) block back as (d_k, T) for every H (layers.py:487-489, 499)
-    if ((rc = launch_merge_heads(dtype, o, merged, B, T, H, D / H, st))) return rc;
+    rc = dtype == CONVNN_BF16 && !force_simt() ? try_launch_conv1d_tc(y, w_conv, b_conv, merged, B, T, H, D / H, kernel_size, st)
+                                               : (int)CONVNN_E_UNSUPPORTED;
+    if (rc == CONVNN_E_UNSUPPORTED) {
+        if ((rc = launch_conv1d_heads(dtype, y, w_conv, b_conv, o, unfold, B, T, H, D / H, kernel_size, st))) return rc;
+        rc = launch_merge_heads(dtype, o, merged, B, T, H, D / H, st);
+    }
+    if (rc) return rc;
     return convnn_b200_linear(dtype, merged, D, w_o, b_o, nullptr, 0, out, ldo, M, D, D, 0, stream);
 }
 

@@ -243,6 +243,10 @@ int launch_attention(int dtype, const void* q, const void* k, const void* v, voi
 int read_attention_status(int* out);
 int launch_conv1d_heads(int dtype, const void* y, const void* w, const void* bias, void* o, void* unfold, int B,
                         int Tn, int H, int dk, int ks, cudaStream_t st);
+// Conv1d half and its flat reinterpretation in one kernel (heads of 16, 32 or 64 channels).
+int try_launch_conv1d_tc(const void* y, const void* w, const void* bias, void* out, int B, int Tn, int H, int dk, int ks,
+                         cudaStream_t st);
+int read_conv1d_tc_status(int* out);
 bool force_simt();   // debugging switch: environment variable CONVNN_B200_FORCE_SIMT=1
 int launch_gather_conv_simt(const convnn_desc* d, const Dims& dm, const void* v, const int32_t* idx,
                             const float* val, const void* w_conv, const void* w_pw, void* o, void* scratch,

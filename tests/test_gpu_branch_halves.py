@@ -97,6 +97,14 @@ def test_conv1d_attention_matches_oracle(B, T, D, H, ks, dtype):
     assert rel_err(y, want) < (1e-4 if dtype == torch.float32 else 2e-2)
 
 
+# The fused convolution: one token, whole and ragged 128-row tiles, even kernels, several slices per CTA, heads of 64, one set
+# of taps in flight (25 taps), and a kernel too long for it.
+@pytest.mark.parametrize("B,T,D,H,ks", [(2, 1, 32, 1, 3), (1, 128, 64, 2, 8), (1, 257, 64, 1, 5), (60, 129, 96, 3, 9),
+                                        (200, 65, 32, 2, 4), (2, 300, 32, 1, 25), (2, 50, 128, 2, 1), (1, 60, 64, 1, 25)])
+def test_fused_conv1d_attention_matches_oracle(B, T, D, H, ks):
+    test_conv1d_attention_matches_oracle(B, T, D, H, ks, torch.bfloat16)
+
+
 def test_branching_modules_fold_the_skip_connection():
     """residual + layer(x) from one call equals the two-step result bit for bit."""
     g = torch.Generator().manual_seed(5)
