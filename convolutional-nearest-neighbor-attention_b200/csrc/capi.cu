@@ -391,6 +391,19 @@ int convnn_b200_gather_conv(const convnn_desc* d, const void* v, const int32_t* 
 }  // extern "C"
 
 namespace {
+// Neighbours of the workspace's q and k and the conv over its v: in one kernel where that takes the shape (the lists are then
+// not written), else stage by stage.
+int select_and_conv(const convnn_desc* d, const Dims& dm, const Workspace& w, const int32_t* cand, const void* w_conv,
+                    const void* w_pw, void* o, void* stream) {
+    REQUIRE_PTR(w_conv); REQUIRE_PTR(o);
+    int rc = CONVNN_E_UNSUPPORTED;
+    if (d->conv_type == CONVNN_DEPTHWISE && !force_simt())
+        rc = try_launch_sim_gather(d, dm, w.q, w.k, w.v, w.qstat, w.kstat, cand, w_conv, o, static_cast<cudaStream_t>(stream));
+    if (rc != CONVNN_E_UNSUPPORTED) return rc;
+    if ((rc = convnn_b200_sim_topk(d, w.q, w.k, w.qstat, w.kstat, cand, w.idx, w.val, stream))) return rc;
+    return convnn_b200_gather_conv(d, w.v, w.idx, w.val, w_conv, w_pw, o, w.conv_scratch, stream);
+}
+
 int out_proj_impl(const convnn_desc* d, const void* o, const void* w_o, const void* residual, int64_t ldr,
                   void* out, int64_t ldo, void* scratch, void* stream, float* moments_out) {
     Dims dm;
@@ -448,8 +461,7 @@ int convnn_b200_forward(const convnn_desc* d, const void* x, int64_t ldx, const 
     if (workspace_bytes < w.total)
         return set_error(CONVNN_E_WORKSPACE, "workspace has %zu bytes, %zu needed", workspace_bytes, w.total);
     if ((rc = convnn_b200_qkv_proj(d, x, ldx, w_qkv, cand, w.q, w.k, w.v, w.qstat, w.kstat, w.scratch, stream))) return rc;
-    if ((rc = convnn_b200_sim_topk(d, w.q, w.k, w.qstat, w.kstat, cand, w.idx, w.val, stream))) return rc;
-    if ((rc = convnn_b200_gather_conv(d, w.v, w.idx, w.val, w_conv, w_pw, w.o, w.conv_scratch, stream))) return rc;
+    if ((rc = select_and_conv(d, dm, w, cand, w_conv, w_pw, w.o, stream))) return rc;
     return convnn_b200_out_proj(d, w.o, w_o, residual, ldr, out, ldo, w.scratch, stream);
 }
 
@@ -626,10 +638,8 @@ int convnn_b200_prenorm_forward(const convnn_desc* d, const void* x, int64_t ldx
                                            "contiguous `out` (num_heads = 1, ldo = D, no residual, no moments)");
     const PreNorm pn{moments, planes, eps, w_qkv_extra};
     if ((rc = qkv_proj_impl(d, x, ldx, w_qkv_folded, nullptr, w.q, w.k, w.v, w.qstat, w.kstat, w.scratch, stream, &pn))) return rc;
-    if ((rc = convnn_b200_sim_topk(d, w.q, w.k, w.qstat, w.kstat, nullptr, w.idx, w.val, stream))) return rc;
-    if (!w_o)      // the caller fuses the output projection into what follows (convnn_b200_outproj_mlp)
-        return convnn_b200_gather_conv(d, w.v, w.idx, w.val, w_conv, w_pw, out, w.scratch, stream);
-    if ((rc = convnn_b200_gather_conv(d, w.v, w.idx, w.val, w_conv, w_pw, w.o, w.scratch, stream))) return rc;
+    // (without w_o the caller fuses the output projection into what follows: convnn_b200_outproj_mlp)
+    if ((rc = select_and_conv(d, dm, w, nullptr, w_conv, w_pw, w_o ? w.o : out, stream)) || !w_o) return rc;
     return out_proj_impl(d, w.o, w_o, residual, ldr, out, ldo, w.scratch, stream, moments_out);
 }
 

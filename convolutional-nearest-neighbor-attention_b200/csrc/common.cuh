@@ -176,6 +176,10 @@ bool sim_topk_short_wanted(const Dims& dm);
 int launch_sim_topk_short(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
                           const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st);
 int read_sim_short_status(int* out);
+// The same kernel with the depthwise conv over the neighbours in it (o (B, H, T, d_k), no lists); CONVNN_E_UNSUPPORTED
+// (last_error untouched) where it does not take the shape.
+int try_launch_sim_gather(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const void* v, const float* qstat,
+                          const float* kstat, const int32_t* cand, const void* w_conv, void* o, cudaStream_t st);
 int read_sim_rows_status(int* out);
 int read_sim_topk_status(int* out);
 int read_sim_topk2_status(int* out);

@@ -35,6 +35,11 @@ struct RowsParams {
     int32_t* idx;
     float* val;
     int T, S, H, K, nsel, metric, sampled;
+    // GATHER: the depthwise conv over the neighbours instead of their lists (reference layers.py:345-406)
+    const uint4* v;     // (B, T, H, 8 groups)
+    const uint4* w;     // taps (K, 8 groups)
+    uint4* o;           // (B, H, T, 8 groups)
+    int groups, softmax;
     int KCH, KC;        // channels per shared-memory chunk, chunks per segment
     int BN, pitch;      // S rounded up to 16; words between the rows of the key buffer (4 mod 8: 16-byte stores of eight
                         // consecutive rows fall into different banks)
@@ -81,7 +86,66 @@ struct Segment {
 
 __device__ __forceinline__ void selection_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory"); }
 
-template <int J, int NS>          // as in select_and_write()
+// Depthwise conv of the warp's rows, whose (value, token) lists lie in `list` (pairs: .x value, .y token): weights over the
+// values as in token_weights.cuh (sums in tap order), then a 16-byte channel group of a row per lane.
+constexpr int TAPS = 5;                 // neighbour rows in flight per lane (nine spill: 504 -> 496 us per ViT-Tiny image)
+__device__ __forceinline__ void conv_rows(const RowsParams& p, float2* list, const uint4* taps, int w, int n, int g, int bh) {
+    const int lane = threadIdx.x & 31, b = bh / p.H, h = bh - b * p.H;
+    const bool maximum = p.metric != CONVNN_EUCLIDEAN;
+    const int vbase = (b * p.T * p.H + h) * p.groups, vstride = p.H * p.groups;      // (B T D < 2^31)
+    for (int m0 = 0; m0 < n; m0 += 2) {             // two rows, sixteen lanes each (K <= 17: a lane more holds the last)
+        const int j = lane & 15, m = m0 + (lane >> 4);
+        const bool in = m < n && j < p.K, last = p.K > 16 && m < n && j == 15;
+        float2* e0 = list + m * p.K;
+        float x = in ? e0[j].x : 0.f, x16 = last ? e0[16].x : 0.f;
+        float wt, wt16 = 0.f;
+        if (p.softmax) {
+            if (!maximum) { x = -x; x16 = -x16; }
+            float mx = in ? fmaxf(x, -3.402823466e38f) : -3.402823466e38f;
+            if (last) mx = fmaxf(mx, x16);
+#pragma unroll
+            for (int d = 8; d >= 1; d /= 2) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+            const float ex = in ? expf(x - mx) : 0.f, ex16 = last ? expf(x16 - mx) : 0.f;
+            float s = 0.f;
+            for (int i = 0; i < min(p.K, 16); ++i) s += __shfl_sync(0xffffffffu, ex, i, 16);
+            if (p.K > 16) s += __shfl_sync(0xffffffffu, ex16, 15, 16);
+            wt = ex / s;
+            wt16 = ex16 / s;
+        } else {
+            wt = maximum ? x : 1.0f / (x + 1e-8f);
+            wt16 = maximum ? x16 : 1.0f / (x16 + 1e-8f);
+        }
+        if (in) e0[j] = make_float2(wt, __int_as_float(vbase + __float_as_int(e0[j].y) * vstride));
+        if (last) e0[16] = make_float2(wt16, __int_as_float(vbase + __float_as_int(e0[16].y) * vstride));
+    }
+    __syncwarp();
+    for (int e = lane; e < n * p.groups; e += 32) {
+        const int m = e / p.groups, cg = e - m * p.groups;
+        const float2* l = list + m * p.K;
+        f32x2 acc[4] = {0ull, 0ull, 0ull, 0ull};
+        for (int j0 = 0; j0 < p.K; j0 += TAPS) {
+            uint4 raw[TAPS];
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j)
+                if (j0 + j < p.K) raw[j] = __ldg(p.v + __float_as_int(l[j0 + j].y) + cg);
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j)
+                if (j0 + j < p.K) {
+                    f32x2 x[4], tw[4];
+                    bf16x8_to_f32x2(raw[j], x);
+                    bf16x8_to_f32x2(taps[(j0 + j) * p.groups + cg], tw);
+                    const float pj = l[j0 + j].x;
+                    const f32x2 p2 = pack2(pj, pj);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) acc[q] = fma2(tw[q], mul2(p2, x[q]), acc[q]);
+                }
+        }
+        p.o[(long long)(g + w + m * NW) * p.groups + cg] = f32x2_to_bf16x8(acc);
+    }
+    __syncwarp();
+}
+
+template <int J, int NS, bool GATHER>          // NS as in select_lists()
 __global__ void __launch_bounds__(NT, 1)
 sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ,
                      const __grid_constant__ RowsParams p) {
@@ -91,8 +155,8 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     const uint32_t a_bytes = BM * pitch, b_bytes = p.BN * pitch, stage_bytes = a_bytes + b_bytes;
     const uint32_t STAGES = p.stages;
     float* keybuf = reinterpret_cast<float*>(smem + STAGES * stage_bytes);      // [seg_rows][pitch]
-    float2* lists = reinterpret_cast<float2*>(keybuf + p.seg_rows * p.pitch);   // [NW][WR][nsel] key, column
-    float2* found = lists + NW * WR * p.nsel;                                   // [NW][found_pairs] survivors: key, column
+    float2* lists = reinterpret_cast<float2*>(keybuf + p.seg_rows * p.pitch);   // [NW][WR][K] key, column
+    float2* found = lists + NW * WR * p.K;                                      // [NW][found_pairs] survivors: key, column
     float* qs = reinterpret_cast<float*>(found + NW * found_pairs(NS));         // [BN] column statistics
     int* cs = reinterpret_cast<int*>(qs + p.BN);                                // [BN] candidate tokens
     float* kst_s = reinterpret_cast<float*>(cs + p.BN);                         // [BM] row statistics
@@ -102,6 +166,7 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     uint64_t* tempty = tfull + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    uint4* taps = reinterpret_cast<uint4*>(tempty + 4);                         // GATHER: [K][groups]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -179,12 +244,14 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         const int lq = warp & 3;                     // TMEM lane quarter it may read
         const int sub = w >> 2;                      // its share of that quarter's columns
         const int r = lq * 32 + lane;
-        float2* list = lists + w * WR * p.nsel;
+        float2* list = lists + w * WR * p.K;
         const uint32_t found0 = smem_u32(found + w * found_pairs(NS));
         const RowsTask task{kst_s, cs, p.idx, p.val, p.pitch, p.BN, p.nsel, p.K, p.inv_K, p.metric, p.sampled, p.sqrt_dk};
         const bool stats = p.metric != CONVNN_MATMUL;
         if (p.sampled)
             for (int c = tid; c < p.BN; c += 32 * NW) cs[c] = c < p.S ? p.cand[c] : -1;
+        if (GATHER)                                  // (read behind the barriers of the first segment)
+            for (int c = tid; c < p.K * p.groups; c += 32 * NW) taps[c] = p.w[c];
         uint32_t buf = 0, use = 0;
         const float none = __int_as_float(0x7fffffff);           // columns past the last candidate: their keys become NaN
         // Every selection warp makes the same number of passes and meets every barrier, also after a wait has expired
@@ -257,7 +324,13 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             if (lane == 0) mbar_arrive(&tempty[buf]);
             selection_barrier();                     // the keys are there
             if (!*abort_flag) {
-                select_and_write<J, NS, NW>(task, keybuf, list, found0, w, cur.n, cur.g, cur.row);
+                if constexpr (GATHER) {
+                    const int n = select_lists<J, NS, NW>(task, keybuf, list, found0, w, cur.n, cur.row,
+                        [&](int m, int slot, int tok, float s) { list[m * p.K + slot] = make_float2(s, __int_as_float(tok)); });
+                    conv_rows(p, list, taps, w, n, cur.g, cur.bh);
+                } else {
+                    select_and_write<J, NS, NW>(task, keybuf, list, found0, w, cur.n, cur.g, cur.row);
+                }
             }
             if (++buf == 2) { buf = 0; ++use; }
         }
@@ -276,9 +349,9 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     }
 }
 
-template <int J, int NS>
+template <int J, int NS, bool GATHER>
 int launch_rows(RowsParams& p, size_t smem, int grid, const CUtensorMap& tmK, const CUtensorMap& tmQ, cudaStream_t st) {
-    auto kern = sim_topk_rows_kernel<J, NS>;
+    auto kern = sim_topk_rows_kernel<J, NS, GATHER>;
     CONVNN_ENSURE_SMEM(kern, smem);
     launch_chained(kern, grid, NT, smem, st, tmK, tmQ, p);
     CONVNN_CHECK_LAUNCH("sim_topk_rows");
@@ -287,11 +360,15 @@ int launch_rows(RowsParams& p, size_t smem, int grid, const CUtensorMap& tmK, co
 
 template <int J>
 int launch_rows_j(RowsParams& p, size_t smem, int grid, const CUtensorMap& tmK, const CUtensorMap& tmQ, cudaStream_t st) {
-    if (p.nsel == 8) return launch_rows<J, 8>(p, smem, grid, tmK, tmQ, st);
-    if (p.nsel == 9) return launch_rows<J, 9>(p, smem, grid, tmK, tmQ, st);
-    if (p.nsel <= 16) return launch_rows<J, 0>(p, smem, grid, tmK, tmQ, st);
-    if (p.nsel <= 25) return launch_rows<J, -1>(p, smem, grid, tmK, tmQ, st);
-    return launch_rows<J, -2>(p, smem, grid, tmK, tmQ, st);
+    if (p.o) {
+        if (p.nsel == 9) return launch_rows<J, 9, true>(p, smem, grid, tmK, tmQ, st);
+        return launch_rows<J, 0, true>(p, smem, grid, tmK, tmQ, st);
+    }
+    if (p.nsel == 8) return launch_rows<J, 8, false>(p, smem, grid, tmK, tmQ, st);
+    if (p.nsel == 9) return launch_rows<J, 9, false>(p, smem, grid, tmK, tmQ, st);
+    if (p.nsel <= 16) return launch_rows<J, 0, false>(p, smem, grid, tmK, tmQ, st);
+    if (p.nsel <= 25) return launch_rows<J, -1, false>(p, smem, grid, tmK, tmQ, st);
+    return launch_rows<J, -2, false>(p, smem, grid, tmK, tmQ, st);
 }
 
 }  // namespace
@@ -299,6 +376,25 @@ int launch_rows_j(RowsParams& p, size_t smem, int grid, const CUtensorMap& tmK, 
 static int rows_per_sm(const Dims& dm) {
     const int sms = device_sms();
     return (int)(((long long)dm.B * dm.H * dm.T + sms - 1) / sms + NW - 1) / NW * NW;
+}
+
+// Rows per CTA; ranges that do not cross from one (batch, head) to the next, where they need be no longer: a segment less each.
+struct Ranges {
+    int rows, per_head, grid;
+};
+static Ranges ranges_of(const Dims& dm) {
+    const long long total = (long long)dm.B * dm.H * dm.T;
+    Ranges r{rows_per_sm(dm), 0, 0};
+    const int parts = device_sms() / (dm.B * dm.H);
+    if (parts > 0) {
+        const int rows = ((dm.T + parts - 1) / parts + NW - 1) / NW * NW;
+        if (rows <= r.rows + NW) {
+            r.rows = rows;
+            r.per_head = (dm.T + rows - 1) / rows;
+        }
+    }
+    r.grid = r.per_head ? dm.B * dm.H * r.per_head : (int)((total + r.rows - 1) / r.rows);
+    return r;
 }
 
 // What bounds it: warp instructions, ~300 per row of 197 keys with the copy, at 0.5 to 0.8 per cycle and scheduler.  A row
@@ -317,8 +413,9 @@ bool sim_topk_rows_wanted(const Dims& dm) {
     return rows <= 48 || (dm.S > 128 && dm.Cp <= 384 && rows <= 304);
 }
 
-int launch_sim_topk_rows(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
-                         const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st) {
+static int launch_impl(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
+                       const float* kstat, const int32_t* cand, int32_t* idx, float* val, const void* v, const void* w_conv,
+                       void* o, cudaStream_t st) {
     RowsParams p{};
     p.qstat = qstat; p.kstat = kstat; p.cand = cand; p.idx = idx; p.val = val;
     p.T = dm.T; p.S = dm.S; p.H = dm.H; p.K = dm.K; p.nsel = dm.nsel; p.metric = d->metric; p.sampled = d->sampled ? 1 : 0;
@@ -328,23 +425,17 @@ int launch_sim_topk_rows(const convnn_desc* d, const Dims& dm, const void* q, co
     while (p.acc_cols < p.BN) p.acc_cols *= 2;
     p.sqrt_dk = (float)sqrt((double)dm.dk);
     p.rows_total = dm.B * dm.H * dm.T;
-    p.rows_per_cta = rows_per_sm(dm);
-    int grid = (int)(((long long)p.rows_total + p.rows_per_cta - 1) / p.rows_per_cta);
-    // ranges that do not cross from one (batch, head) to the next, where they need be no longer: a segment less each
-    const int parts = device_sms() / (dm.B * dm.H);
-    if (parts > 0) {
-        const int rows = ((dm.T + parts - 1) / parts + NW - 1) / NW * NW;
-        if (rows <= p.rows_per_cta + NW) {
-            p.rows_per_cta = rows;
-            p.per_head = (dm.T + rows - 1) / rows;
-            grid = dm.B * dm.H * p.per_head;
-        }
-    }
+    const Ranges ranges = ranges_of(dm);
+    p.rows_per_cta = ranges.rows; p.per_head = ranges.per_head;
+    const int grid = ranges.grid;
     p.seg_rows = p.rows_per_cta < BM ? p.rows_per_cta : BM;
     p.inv_K = inverse_of(dm.K);
-    const size_t fixed = 1024 + (size_t)p.seg_rows * p.pitch * 4 + (size_t)NW * WR * dm.nsel * 8 +
+    p.v = static_cast<const uint4*>(v); p.w = static_cast<const uint4*>(w_conv); p.o = static_cast<uint4*>(o);
+    p.groups = dm.dk / 8; p.softmax = d->softmax;
+    const size_t fixed = 1024 + (size_t)p.seg_rows * p.pitch * 4 + (size_t)NW * WR * dm.K * 8 +
+                         (o ? (size_t)dm.K * dm.dk * 2 : 0) +
                          (size_t)NW * found_pairs(dm.nsel > 16 ? -1 : 0) * 8 + (size_t)p.BN * 8 + BM * 4 +
-                         (2 * MAX_STAGES + 4) * 8 + 16;
+                         (2 * MAX_STAGES + 6) * 8;
     const size_t room = 226 * 1024 - fixed;
     // (the copies fill what lies past a head with zeros; 32-channel chunks where only one of 64 would fit)
     p.KCH = dm.Cp <= 16 ? 16 : (dm.Cp <= 32 ? 32 : 64);
@@ -377,6 +468,22 @@ int launch_sim_topk_rows(const convnn_desc* d, const Dims& dm, const void* q, co
         case 7: return launch_rows_j<7>(p, smem, grid, tmK, tmQ, st);
         default: return launch_rows_j<8>(p, smem, grid, tmK, tmQ, st);
     }
+}
+
+int launch_sim_topk_rows(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
+                         const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st) {
+    return launch_impl(d, dm, q, k, qstat, kstat, cand, idx, val, nullptr, nullptr, nullptr, st);
+}
+
+// Where a CTA has at most 32 rows, two per warp: the conv's neighbour rows come from L2 a few at a time, which costs less than
+// another kernel then, and more from four rows per warp on.  ViT-Tiny forward, us, lists and conv in two kernels -> in one:
+// 1 image 527 -> 496, 16 images 605 -> 572 (32 rows per CTA), 37: 656 -> 655 (64), 64: 739 -> 817 (96).
+int try_launch_sim_gather(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const void* v, const float* qstat,
+                          const float* kstat, const int32_t* cand, const void* w_conv, void* o, cudaStream_t st) {
+    if (!sim_topk_tc_supported(d, dm, q, k) || !sim_topk_rows_wanted(dm) || dm.nsel > 16 || ranges_of(dm).rows > 32 || dm.C != dm.dk || dm.dk % 8 != 0 ||
+        (size_t)dm.K * dm.dk * 2 > 16 * 1024 || !aligned16(v) || !aligned16(w_conv) || !aligned16(o))
+        return CONVNN_E_UNSUPPORTED;
+    return launch_impl(d, dm, q, k, qstat, kstat, cand, nullptr, nullptr, v, w_conv, o, st);
 }
 
 int read_sim_rows_status(int* out) {

@@ -33,8 +33,8 @@ __global__ void __launch_bounds__(NT) sim_topk_simt_rows_kernel(
     float* Bs = As + 2 * BK * LA;                         // [2][BK][LB]
     float* keys = Bs + 2 * BK * LB;                       // [RB][LB]
     float2* found = reinterpret_cast<float2*>(keys + RB * LB);                 // [NW][found_pairs]
-    float2* lists = found + NW * found_pairs(NS);                              // [NW][RB / NW][nsel]
-    float* kst_s = reinterpret_cast<float*>(lists + RB * nsel);                // [RB]
+    float2* lists = found + NW * found_pairs(NS);                              // [NW][RB / NW][K]
+    float* kst_s = reinterpret_cast<float*>(lists + RB * K);                   // [RB]
     int* cs = reinterpret_cast<int*>(kst_s + RB);                              // [NB]
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(NT) sim_topk_simt_rows_kernel(
     }
     __syncthreads();
     const RowsTask task{kst_s, cs, idx, val, LB, ncg * 4, nsel, K, inverse_of(K), metric, sampled, sqrt_dk};
-    select_and_write<J, NS, NW>(task, keys, lists + warp * (RB / NW) * nsel,
+    select_and_write<J, NS, NW>(task, keys, lists + warp * (RB / NW) * K,
                                 static_cast<uint32_t>(__cvta_generic_to_shared(found + warp * found_pairs(NS))), warp,
                                 min(RB, T_ - row0), bh * T_ + row0, row0);
 }
@@ -149,7 +149,7 @@ int launch(const convnn_desc* d, const Dims& dm, const void* q, const void* k, c
            const int32_t* cand, int32_t* idx, float* val, cudaStream_t st) {
     constexpr int LB = 32 * J + 4;
     const size_t smem = (size_t)(2 * BK * LA + 2 * BK * LB + RB * LB + RB + 32 * J) * 4 +
-                        (size_t)(NW * found_pairs(NS) + RB * dm.nsel) * 8;
+                        (size_t)(NW * found_pairs(NS) + RB * dm.K) * 8;
     auto kern = sim_topk_simt_rows_kernel<T, J, NS>;
     CONVNN_ENSURE_SMEM(kern, smem);
     const int vec = dm.Cp % 4 == 0 && aligned16(q) && aligned16(k);

@@ -232,15 +232,15 @@ __device__ __forceinline__ uint32_t select_rows(const RowsTask& p, const float* 
     return redo;
 }
 
-// The rows w, w + NW, ... below n_rows of a key buffer: lists through `list` (room for nsel pairs per row of the warp) to
-// global memory, as rows g + r of the flattened (batch, head, row) order, tokens row0 + r.  NS: number of neighbours where it
-// is fixed, 0: any up to 16, -1: up to 25, -2: up to 32.
-template <int J, int NS, int NW>
-__device__ __forceinline__ void select_and_write(const RowsTask& p, const float* keybuf, float2* list, uint32_t found0, int w,
-                                                 int n_rows, int g, int row0) {
+// The rows w, w + NW, ... below n_rows of a key buffer (tokens row0 + r of their sequence): lists through `list` (room for K
+// pairs per row of the warp), then sink(row of the warp, slot, token, value) for every entry.  Returns the rows of the warp.
+// NS: number of neighbours where it is fixed, 0: any up to 16, -1: up to 25, -2: up to 32.
+template <int J, int NS, int NW, class Sink>
+__device__ __forceinline__ int select_lists(const RowsTask& p, const float* keybuf, float2* list, uint32_t found0, int w,
+                                            int n_rows, int row0, Sink sink) {
     constexpr int E = NS < 0 ? 2 : 1, GR = NS == -2 && J > 1 ? 2 : 1;
     const int lane = threadIdx.x & 31;
-    const uint32_t list0 = static_cast<uint32_t>(__cvta_generic_to_shared(list)), list_stride = p.nsel * 8;
+    const uint32_t list0 = static_cast<uint32_t>(__cvta_generic_to_shared(list + p.sampled)), list_stride = p.K * 8;
     uint32_t redo = 0;                       // bit n: row w + n NW
     int n = 0;
     auto select = [&](auto rows) {
@@ -264,7 +264,7 @@ __device__ __forceinline__ void select_and_write(const RowsTask& p, const float*
         int tok = row;
         float s = 1.0f;
         if (!p.sampled || slot) {
-            const float2 f = list[m * p.nsel + slot - p.sampled];
+            const float2 f = list[e];
             const float kst = p.kst[rw];
             tok = __float_as_int(f.y);
             if (p.metric == CONVNN_COSINE) s = f.x * kst;
@@ -275,11 +275,21 @@ __device__ __forceinline__ void select_and_write(const RowsTask& p, const float*
                 if (tok == row) s = (p.metric == CONVNN_EUCLIDEAN) ? 1.1f : -0.1f;
             }
         }
-        const int to = (g + rw) * p.K + slot;            // (B H T K < 2^31)
-        p.idx[to] = tok;
-        p.val[to] = s;
+        sink(m, slot, tok, s);
     }
     __syncwarp();
+    return n;
+}
+
+// The same with the lists written to global memory, as rows g + r of the flattened (batch, head, row) order.
+template <int J, int NS, int NW>
+__device__ __forceinline__ void select_and_write(const RowsTask& p, const float* keybuf, float2* list, uint32_t found0, int w,
+                                                 int n_rows, int g, int row0) {
+    select_lists<J, NS, NW>(p, keybuf, list, found0, w, n_rows, row0, [&](int m, int slot, int tok, float s) {
+        const int to = (g + w + m * NW) * p.K + slot;    // (B H T K < 2^31)
+        p.idx[to] = tok;
+        p.val[to] = s;
+    });
 }
 
 }  // namespace topk_rows

@@ -53,3 +53,24 @@ def test_standard_conv_bfloat16_against_float64(B, T, H, dk, K):
     # the weighted block is rounded to bfloat16 once, the result once; fp32 sums of K * dk terms
     bound = (2.0 ** -9 + (K * dk + 16) * EPS) * mass + 2.0 ** -8 * want.abs() + 1e-30
     assert bool(((got.double() - want).abs() <= bound).all())
+
+
+# Selection and depthwise conv in one kernel (few rows per SM, at most 17 neighbours) against the two stages, whose lists and
+# sums are the same: bit for bit.  One row, ragged sequences, sixteen and seventeen neighbours, one channel group, the widest
+# taps, several heads, every way of weighting; the last shape has too many rows for it.
+@pytest.mark.parametrize("B,T,S,H,dk,K", [(1, 1, 1, 1, 16, 1), (3, 197, 197, 1, 192, 9), (1, 197, 197, 3, 64, 9), (2, 65, 40, 1, 48, 17),
+                                          (5, 130, 100, 1, 16, 16), (2, 257, 225, 1, 384, 5), (1, 33, 33, 2, 80, 12),
+                                          (1, 500, 256, 1, 768, 10), (40, 197, 197, 1, 64, 9)])
+@pytest.mark.parametrize("metric,softmax", [("cosine", True), ("matmul", False), ("euclidean", True), ("euclidean", False)])
+def test_selection_with_conv_equals_the_stages(B, T, S, H, dk, K, metric, softmax):
+    D = H * dk
+    g = torch.Generator(device=DEV).manual_seed(T + S + K)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+    spec = ops.LayerSpec(D, H, K, "spatial" if S != T else "all", metric, "depthwise", softmax, False, T)
+    x, w_qkv, w_o, taps = rnd(B, T, D), rnd(3, D, D) * D ** -0.5, rnd(D, D) * D ** -0.5, rnd(K, dk)
+    cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if S != T else None
+    whole = ops.forward(spec, x, (w_qkv, taps, None, w_o), cand)
+    q, k, v, qs, ks = ops.qkv_proj(spec, x, w_qkv, cand)
+    idx, val = ops.sim_topk(spec, q, k, qs, ks, cand)
+    out = ops.out_proj(spec, ops.gather_conv(spec, v, idx, val, taps, None, S=S), w_o, S=S)
+    assert torch.equal(whole.isnan(), out.isnan()) and torch.equal(whole.nan_to_num(), out.nan_to_num())
