@@ -232,6 +232,7 @@ int convnn_b200_device_status(int* code) {
     if (!c && (rc = read_dw_stream_status(&c))) return rc;
     if (!c && (rc = read_attention_status(&c))) return rc;
     if (!c && (rc = read_mlp_tc_status(&c))) return rc;
+    if (!c && (rc = read_conv_std_status(&c))) return rc;
     if (!c && (rc = read_conv1d_tc_status(&c))) return rc;
     *code = a ? a : (b ? b : c);
     return CONVNN_OK;
@@ -392,20 +393,27 @@ int convnn_b200_gather_conv(const convnn_desc* d, const void* v, const int32_t* 
 
 namespace {
 // Neighbours of the workspace's q and k and the conv over its v: in one kernel where that takes the shape (the lists are then
-// not written), else stage by stage.
+// not written), else stage by stage.  *merged: o has several heads already in the flat reinterpretation (B, T, D).
 int select_and_conv(const convnn_desc* d, const Dims& dm, const Workspace& w, const int32_t* cand, const void* w_conv,
-                    const void* w_pw, void* o, void* stream) {
+                    const void* w_pw, void* o, bool* merged, void* stream) {
     REQUIRE_PTR(w_conv); REQUIRE_PTR(o);
     int rc = CONVNN_E_UNSUPPORTED;
+    *merged = false;
     if (d->conv_type == CONVNN_DEPTHWISE && !force_simt())
         rc = try_launch_sim_gather(d, dm, w.q, w.k, w.v, w.qstat, w.kstat, cand, w_conv, o, static_cast<cudaStream_t>(stream));
     if (rc != CONVNN_E_UNSUPPORTED) return rc;
     if ((rc = convnn_b200_sim_topk(d, w.q, w.k, w.qstat, w.kstat, cand, w.idx, w.val, stream))) return rc;
+    if (dm.H > 1) {
+        rc = try_launch_conv_std_tc(d, dm, w.v, w.idx, w.val, w_conv, o, true, static_cast<cudaStream_t>(stream));
+        *merged = rc == CONVNN_OK;
+        if (rc != CONVNN_E_UNSUPPORTED) return rc;
+    }
     return convnn_b200_gather_conv(d, w.v, w.idx, w.val, w_conv, w_pw, o, w.conv_scratch, stream);
 }
 
+// merged: o is (B, T, D), heads in the flat reinterpretation.
 int out_proj_impl(const convnn_desc* d, const void* o, const void* w_o, const void* residual, int64_t ldr,
-                  void* out, int64_t ldo, void* scratch, void* stream, float* moments_out) {
+                  void* out, int64_t ldo, void* scratch, void* stream, float* moments_out, bool merged) {
     Dims dm;
     int rc = validate(d, &dm);
     if (rc) return rc;
@@ -419,9 +427,9 @@ int out_proj_impl(const convnn_desc* d, const void* o, const void* w_o, const vo
         GemmTcOpts go;
         go.residual = residual; go.ldr = ldr; go.moments_out = moments_out;
         const bool res_ok = !residual || (ldr % 8 == 0 && aligned16(residual));
-        if (res_ok && dm.H == 1 && gemm_tc_supported(o, dm.D, w_o, dm.D, dm.D, 1, cs, ldo))
+        if (res_ok && (dm.H == 1 || merged) && gemm_tc_supported(o, dm.D, w_o, dm.D, dm.D, 1, cs, ldo))
             return launch_gemm_tc(o, dm.D, w_o, dm.B * dm.T, dm.D, dm.D, 1, cs, ldo, go, st);
-        if (res_ok && dm.H > 1 && scratch && gemm_tc_supported(scratch, dm.D, w_o, dm.D, dm.D, 1, cs, ldo)) {
+        if (res_ok && dm.H > 1 && !merged && scratch && gemm_tc_supported(scratch, dm.D, w_o, dm.D, dm.D, 1, cs, ldo)) {
             if ((rc = launch_merge_heads(d->dtype, o, scratch, dm.B, dm.T, dm.H, dm.dk, st))) return rc;
             return launch_gemm_tc(scratch, dm.D, w_o, dm.B * dm.T, dm.D, dm.D, 1, cs, ldo, go, st);
         }
@@ -430,8 +438,8 @@ int out_proj_impl(const convnn_desc* d, const void* o, const void* w_o, const vo
     GemmParams p{};
     p.a = o; p.w = w_o; p.bias = nullptr; p.c = out; p.cand = nullptr;
     p.lda = dm.D; p.ldc = ldo; p.M = dm.B * dm.T; p.N = dm.D; p.Kd = dm.D;
-    p.a_mode = dm.H == 1 ? A_ROWS : A_HEAD_QUIRK; p.c_mode = C_ROWS;
-    if (dm.H > 1 && scratch) {       // the head reinterpretation once, instead of a strided operand per column tile
+    p.a_mode = dm.H == 1 || merged ? A_ROWS : A_HEAD_QUIRK; p.c_mode = C_ROWS;
+    if (dm.H > 1 && !merged && scratch) {       // the head reinterpretation once, instead of a strided operand per column tile
         if ((rc = launch_merge_heads(d->dtype, o, scratch, dm.B, dm.T, dm.H, dm.dk, static_cast<cudaStream_t>(stream)))) return rc;
         p.a = scratch; p.a_mode = A_ROWS;
     }
@@ -445,7 +453,7 @@ extern "C" {
 
 int convnn_b200_out_proj(const convnn_desc* d, const void* o, const void* w_o, const void* residual, int64_t ldr,
                          void* out, int64_t ldo, void* scratch, void* stream) {
-    return out_proj_impl(d, o, w_o, residual, ldr, out, ldo, scratch, stream, nullptr);
+    return out_proj_impl(d, o, w_o, residual, ldr, out, ldo, scratch, stream, nullptr, false);
 }
 
 int convnn_b200_forward(const convnn_desc* d, const void* x, int64_t ldx, const void* w_qkv,
@@ -461,8 +469,9 @@ int convnn_b200_forward(const convnn_desc* d, const void* x, int64_t ldx, const 
     if (workspace_bytes < w.total)
         return set_error(CONVNN_E_WORKSPACE, "workspace has %zu bytes, %zu needed", workspace_bytes, w.total);
     if ((rc = convnn_b200_qkv_proj(d, x, ldx, w_qkv, cand, w.q, w.k, w.v, w.qstat, w.kstat, w.scratch, stream))) return rc;
-    if ((rc = select_and_conv(d, dm, w, cand, w_conv, w_pw, w.o, stream))) return rc;
-    return convnn_b200_out_proj(d, w.o, w_o, residual, ldr, out, ldo, w.scratch, stream);
+    bool merged;
+    if ((rc = select_and_conv(d, dm, w, cand, w_conv, w_pw, w.o, &merged, stream))) return rc;
+    return out_proj_impl(d, w.o, w_o, residual, ldr, out, ldo, w.scratch, stream, nullptr, merged);
 }
 
 int convnn_b200_layernorm(int dtype, const void* x, int64_t ldx, const void* gamma, const void* beta, float eps,
@@ -639,8 +648,9 @@ int convnn_b200_prenorm_forward(const convnn_desc* d, const void* x, int64_t ldx
     const PreNorm pn{moments, planes, eps, w_qkv_extra};
     if ((rc = qkv_proj_impl(d, x, ldx, w_qkv_folded, nullptr, w.q, w.k, w.v, w.qstat, w.kstat, w.scratch, stream, &pn))) return rc;
     // (without w_o the caller fuses the output projection into what follows: convnn_b200_outproj_mlp)
-    if ((rc = select_and_conv(d, dm, w, nullptr, w_conv, w_pw, w_o ? w.o : out, stream)) || !w_o) return rc;
-    return out_proj_impl(d, w.o, w_o, residual, ldr, out, ldo, w.scratch, stream, moments_out);
+    bool merged;
+    if ((rc = select_and_conv(d, dm, w, nullptr, w_conv, w_pw, w_o ? w.o : out, &merged, stream)) || !w_o) return rc;
+    return out_proj_impl(d, w.o, w_o, residual, ldr, out, ldo, w.scratch, stream, moments_out, merged);
 }
 
 int convnn_b200_prenorm_mlp_supported(int32_t D, int32_t DM, int32_t planes) {

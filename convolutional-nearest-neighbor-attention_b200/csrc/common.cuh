@@ -251,6 +251,11 @@ int launch_conv1d_heads(int dtype, const void* y, const void* w, const void* bia
 int try_launch_conv1d_tc(const void* y, const void* w, const void* bias, void* out, int B, int Tn, int H, int dk, int ks,
                          cudaStream_t st);
 int read_conv1d_tc_status(int* out);
+// Standard conv with its weighted neighbour block kept on the SM (bfloat16 heads of 16, 32 or 64 channels); merged: o is
+// (B, T, D) in the flat reinterpretation.
+int try_launch_conv_std_tc(const convnn_desc* d, const Dims& dm, const void* v, const int32_t* idx, const float* val,
+                           const void* w_conv, void* o, bool merged, cudaStream_t st);
+int read_conv_std_status(int* out);
 bool force_simt();   // debugging switch: environment variable CONVNN_B200_FORCE_SIMT=1
 int launch_gather_conv_simt(const convnn_desc* d, const Dims& dm, const void* v, const int32_t* idx,
                             const float* val, const void* w_conv, const void* w_pw, void* o, void* scratch,

@@ -200,6 +200,7 @@ int try_launch_gather_conv_tc(const convnn_desc* d, const Dims& dm, const void* 
     void* cs[1] = {o};
     int rc;
     if (d->conv_type == CONVNN_STANDARD) {
+        if ((rc = try_launch_conv_std_tc(d, dm, v, idx, val, w_conv, o, false, st)) != CONVNN_E_UNSUPPORTED) return rc;
         const int Kd = dm.K * dm.C;
         if (!gemm_tc_supported(scratch, Kd, w_conv, Kd, dm.dk, 1, cs, dm.dk)) return CONVNN_E_UNSUPPORTED;
         if ((rc = launch_gather_weighted(d, dm, v, idx, val, scratch, st))) return rc;

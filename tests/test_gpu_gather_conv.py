@@ -74,3 +74,27 @@ def test_selection_with_conv_equals_the_stages(B, T, S, H, dk, K, metric, softma
     idx, val = ops.sim_topk(spec, q, k, qs, ks, cand)
     out = ops.out_proj(spec, ops.gather_conv(spec, v, idx, val, taps, None, S=S), w_o, S=S)
     assert torch.equal(whole.isnan(), out.isnan()) and torch.equal(whole.nan_to_num(), out.nan_to_num())
+
+
+# The standard conv whose neighbour block stays on the SM: edges of its 128-token tiles, of a producer warp's eight tokens and of
+# its groups of taps, the longest lists, several slices per CTA; then heads narrower and wider than it takes.
+@pytest.mark.parametrize("B,T,H,dk,K", [(1, 127, 2, 16, 5), (2, 128, 1, 32, 6), (1, 129, 3, 64, 3), (3, 9, 2, 64, 4), (2, 256, 1, 32, 32),
+                                        (60, 137, 3, 32, 9), (80, 300, 2, 16, 17), (2, 300, 1, 32, 9), (1, 40, 2, 64, 25), (2, 50, 2, 24, 9)])
+def test_standard_conv_tiles(B, T, H, dk, K):
+    test_standard_conv_bfloat16_against_float64(B, T, H, dk, K)
+
+
+@pytest.mark.parametrize("B,T,H,dk,K", [(2, 197, 3, 32, 9), (3, 65, 2, 64, 16), (1, 130, 4, 16, 5)])
+@pytest.mark.parametrize("metric,softmax", [("cosine", True), ("matmul", False), ("euclidean", True), ("euclidean", False)])
+def test_standard_conv_in_the_flat_reinterpretation(B, T, H, dk, K, metric, softmax):
+    """The layer's call, whose conv stores the reinterpreted rows, against the stages, which store them as they are."""
+    D = H * dk
+    g = torch.Generator(device=DEV).manual_seed(T + K)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+    spec = ops.LayerSpec(D, H, K, "all", metric, "standard", softmax, False, T)
+    x, w_qkv, w_o, taps = rnd(B, T, D), rnd(3, D, D) * D ** -0.5, rnd(D, D) * D ** -0.5, rnd(dk, K, dk) * (K * dk) ** -0.5
+    whole = ops.forward(spec, x, (w_qkv, taps, None, w_o), None)
+    q, k, v, qs, ks = ops.qkv_proj(spec, x, w_qkv, None)
+    idx, val = ops.sim_topk(spec, q, k, qs, ks, None)
+    out = ops.out_proj(spec, ops.gather_conv(spec, v, idx, val, taps), w_o, S=T)
+    assert torch.equal(whole.isnan(), out.isnan()) and torch.equal(whole.nan_to_num(), out.nan_to_num())
