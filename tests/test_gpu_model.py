@@ -211,6 +211,20 @@ def test_layernorm_widths(D, dtype):
     assert rel_err(ops.layernorm(part, w, b, 1e-5), want) < tol
 
 
+@pytest.mark.parametrize("rows,D", [(1, 264), (15, 504), (17, 512), (4739, 384), (9, 520), (2371, 768), (4737, 640), (30011, 272)])
+def test_layernorm_rows_ahead(rows, D):
+    """bfloat16 rows of 257 to 768 channels at the ends of a CTA's rows and of its passes, strided rows among them."""
+    g = torch.Generator(device=DEV).manual_seed(rows + D)
+    wide = (torch.randn(rows, D + 24, device=DEV, generator=g) * 3 + 1).bfloat16()
+    w, b = (torch.randn(D, device=DEV, generator=g).bfloat16() for _ in range(2))
+    for x in (wide[:, :D].contiguous(), wide[:, 8:D + 8]):
+        want = torch.nn.functional.layer_norm(x.double(), (D,), w.double(), b.double(), 1e-5)
+        got = ops.layernorm(x, w, b, 1e-5).double()
+        # one rounding of the result, fp32 sums of D terms before it
+        assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + (D + 16) * 2.0 ** -24 * (1 + want.abs())).all())
+
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_uint8_images_are_normalised_in_the_unfold(dtype):
     """8-bit images through convnn_b200_patchify_u8 equal the float path fed with the loader's
