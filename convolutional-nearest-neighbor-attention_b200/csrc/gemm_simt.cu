@@ -332,6 +332,15 @@ int launch_mode(const GemmParams& p, cudaStream_t st) {
     int best = 0;
     for (int i = 1; i < 4; ++i)
         if (c[i] < c[best]) best = i;
+    // An implicit operand is fetched with divisions and dependent reads per value, and that, not the products, is what a step
+    // waits for: twice the threads per tile.  float32 standard conv, 9 taps, us: 8 x 197 tokens x 3 heads of 64 32.4 -> 27.5 (32 x
+    // 64 tiles), 192 channels 133 -> 103 (64 x 64), 1 x 197 x 3 heads of 64 38.8 -> 26.5 (32 x 32).  Plain rows lose up to 20 %.
+    if constexpr (MODE == A_NEIGHBOURS || MODE == A_CONV1D) {
+        if (best == 0) return launch_tile<TA, T, MODE, 128, 64, 16, 8, 4, 2>(p, st);
+        if (best == 1) return launch_tile<TA, T, MODE, 64, 64, 32, 4, 4, 2>(p, st);
+        if (best == 2) return launch_tile<TA, T, MODE, 32, 64, 64, 4, 2, 2>(p, st);
+        return launch_tile<TA, T, MODE, 32, 32, 32, 4, 2, 4>(p, st);
+    }
     if (best == 0) return launch_tile<TA, T, MODE, 128, 64, 16, 8, 8, 3>(p, st);
     if (best == 1) return launch_tile<TA, T, MODE, 64, 64, 32, 8, 4, 3>(p, st);
     if (best == 2) return launch_tile<TA, T, MODE, 32, 64, 64, 4, 4, 2>(p, st);
