@@ -324,22 +324,43 @@ int launch_mode(const GemmParams& p, cudaStream_t st) {
     // (45, 40, 29 and 26 TFLOP/s at 16384 x 768 x 768; 25 before).  2080 x 192 x 768: 33 us, 50 before; 50432 x 192 x
     // 192: 89 us, 150 before.
     const long long sms = device_sms();
-    auto cost = [&](int bm, int bn, double rate) {
-        const long long tiles = (long long)((p.M + bm - 1) / bm) * ((p.N + bn - 1) / bn);
-        return (double)((tiles + sms - 1) / sms) * bm * bn / rate;
+    long long tiles_of[4];
+    auto cost = [&](int i, int bm, int bn, double rate) {
+        tiles_of[i] = (long long)((p.M + bm - 1) / bm) * ((p.N + bn - 1) / bn);
+        return (double)((tiles_of[i] + sms - 1) / sms) * bm * bn / rate;
     };
-    const double c[4] = {cost(128, 64, 45), cost(64, 64, 40), cost(32, 64, 29), cost(32, 32, 26)};
+    const double c[4] = {cost(0, 128, 64, 45), cost(1, 64, 64, 40), cost(2, 32, 64, 29), cost(3, 32, 32, 26)};
     int best = 0;
     for (int i = 1; i < 4; ++i)
         if (c[i] < c[best]) best = i;
-    // An implicit operand is fetched with divisions and dependent reads per value, and that, not the products, is what a step
-    // waits for: twice the threads per tile.  float32 standard conv, 9 taps, us: 8 x 197 tokens x 3 heads of 64 32.4 -> 27.5 (32 x
-    // 64 tiles), 192 channels 133 -> 103 (64 x 64), 1 x 197 x 3 heads of 64 38.8 -> 26.5 (32 x 32).  Plain rows lose up to 20 %.
+    // An implicit operand is fetched with divisions and dependent reads per value.  While an SM has few tiles that, not the
+    // products, is what a step waits for, and a tile with twice the threads wins; with more of them the tiles hide each other's
+    // waits, and its extra shared-memory reads per product lose.  It keeps two tiles on an SM (four of the smallest) where
+    // the other form keeps three (seven), so it is taken where that takes no more passes.  Weighted neighbours, us, other form -> twice the
+    // threads, float32, 9 taps unless noted; rounds of tiles per SM first:
+    //   128 x 64   1: 32 x 197 x 3 heads of 64 84.9 -> 60.0   2: 64 x 197 x 3 x 64 107 -> 87   3: 256 x 65 x 192 380 -> 388 (not taken)   4: 128 x 197 x 3 x 64 194 -> 170
+    //   64 x 64    1: 8 x 197 x 192 133 -> 103   3: 20 x 577 x 100 113 -> 128 (not taken)   4: 64 x 197 x 192 314 -> 301   5: 32 x 197 x 384 675 -> 706 (not taken)
+    //   32 x 64    1: 8 x 197 x 3 x 64 32.4 -> 27.7   4: 32 x 197 x 192 206 -> 212
+    //   32 x 32    1: 1 x 65 x 192 104 -> 67   6: 64 x 197 x 2 heads of 20 21.9 -> 28.1 (not taken)
+    // Shifted rows cost one division less and gain less: 16 x 197 x 192 209 -> 177 (1), 64 x 197 x 192 312 -> 342 (4, not taken).
+    // Tap rows of C values against more stored channels come value by value: in bfloat16 they gain longest (coordinate channel,
+    // 64 x 197 x 192, 64 x 64 tiles, 4: 617 -> 375; 24 x 577 x 96, 16 taps, 3: 240 -> 303, not taken).  Plain rows lose up to 20 %.
     if constexpr (MODE == A_NEIGHBOURS || MODE == A_CONV1D) {
-        if (best == 0) return launch_tile<TA, T, MODE, 128, 64, 16, 8, 4, 2>(p, st);
-        if (best == 1) return launch_tile<TA, T, MODE, 64, 64, 32, 4, 4, 2>(p, st);
-        if (best == 2) return launch_tile<TA, T, MODE, 32, 64, 64, 4, 2, 2>(p, st);
-        return launch_tile<TA, T, MODE, 32, 32, 32, 4, 2, 4>(p, st);
+        const long long per_sm = (tiles_of[best] + sms - 1) / sms, here = best == 3 ? 4 : 2, other = best == 3 ? 7 : 3;
+        bool twice = (per_sm + here - 1) / here <= (per_sm + other - 1) / other;
+        if (MODE == A_CONV1D) {
+            twice = 2 * per_sm <= here;
+        } else {
+            const bool by_value = p.C != p.Cp && sizeof(T) == 2;
+            if (per_sm > other && (best == 0 || by_value)) twice = true;
+            if (by_value && best < 3 && p.taps < 16) twice = true;
+        }
+        if (twice) {
+            if (best == 0) return launch_tile<TA, T, MODE, 128, 64, 16, 8, 4, 2>(p, st);
+            if (best == 1) return launch_tile<TA, T, MODE, 64, 64, 32, 4, 4, 2>(p, st);
+            if (best == 2) return launch_tile<TA, T, MODE, 32, 64, 64, 4, 2, 2>(p, st);
+            return launch_tile<TA, T, MODE, 32, 32, 32, 4, 2, 4>(p, st);
+        }
     }
     if (best == 0) return launch_tile<TA, T, MODE, 128, 64, 16, 8, 8, 3>(p, st);
     if (best == 1) return launch_tile<TA, T, MODE, 64, 64, 32, 8, 4, 3>(p, st);

@@ -1,5 +1,6 @@
 """Helpers shared by the GPU parity tests: every CUDA result is obtained through the C ABI
 (convnn_b200.ops / the nn.Modules) and compared with the CPU oracle."""
+import pytest
 import torch
 
 import convnn_b200
@@ -7,6 +8,10 @@ from convnn_b200 import ops
 from oracle.convnn_oracle import ConvNNConfig
 
 DEV = "cuda"
+
+# tests of a dispatch that goes by the number of SMs
+on_148_sms = pytest.mark.skipif(torch.cuda.is_available() and torch.cuda.get_device_properties(0).multi_processor_count != 148,
+                                reason="the lines of this rule are tested for 148 SMs")
 
 
 def spec_of(cfg: ConvNNConfig) -> ops.LayerSpec:
@@ -41,3 +46,29 @@ def heads_to_oracle(t, C):
 def rel_err(a, b):
     a, b = a.double().cpu(), b.double().cpu()
     return float((a - b).norm() / b.norm().clamp_min(1e-30))
+
+
+def launches(fn):
+    """{kernel name (mangled): threads per block} of what fn() launches, read from a captured graph."""
+    from cuda.bindings import driver
+
+    def ok(r):
+        assert int(r[0]) == 0, r[0]
+        return r[1:]
+
+    fn()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fn()
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    count = ok(driver.cuGraphGetNodes(raw, 0))[-1]
+    found = {}
+    for node in ok(driver.cuGraphGetNodes(raw, count))[0][:count]:
+        if ok(driver.cuGraphNodeGetType(node))[0] != driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            continue
+        p = ok(driver.cuGraphKernelNodeGetParams(node))[0]
+        name = ok(driver.cuFuncGetName(p.func) if int(p.func) else driver.cuKernelGetName(p.kern))[0]
+        found[name.decode()] = p.blockDimX
+    graph.reset()
+    return found

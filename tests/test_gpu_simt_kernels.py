@@ -1,10 +1,12 @@
 """The fp32-pipe kernels at the edges of their tiles: plain, three-output, neighbour and Conv1d operands of the SIMT
 GEMM, and the register-blocked similarity / top-K kernel."""
+import re
+
 import pytest
 import torch
 
 from convnn_b200 import ops
-from gpu_util import DEV
+from gpu_util import DEV, launches, on_148_sms
 
 pytestmark = pytest.mark.gpu
 EPS = 2.0 ** -24
@@ -86,6 +88,71 @@ def test_conv1d_branch_float32(T, dk, ks):
     want = flat.view(B, H, dk, T).permute(0, 3, 1, 2).reshape(B, T, D)
     scale = float(w.abs().sum(dim=(1, 2)).max()) * float(x.abs().max()) + float(b.abs().max())
     assert float((got.double() - want).abs().max()) <= (ks * dk + D + 4) * EPS * scale
+
+
+# Every tile of the implicit operands in both its forms (outputs per thread), at the rounds of tiles per SM where the rule
+# changes its mind; standard conv (coord: one channel more, in bfloat16), then the shifted rows of the Conv1d branch.
+@on_148_sms
+@pytest.mark.parametrize("B,T,H,dk,K,coord,tile", [
+    (32, 197, 3, 64, 9, False, "128x64 8x4"), (256, 65, 1, 192, 9, False, "128x64 8x8"), (128, 197, 3, 64, 9, False, "128x64 8x4"),
+    (8, 197, 1, 192, 9, False, "64x64 4x4"), (20, 577, 1, 100, 9, False, "64x64 8x4"), (64, 197, 1, 192, 9, False, "64x64 4x4"),
+    (32, 197, 1, 384, 2, False, "64x64 8x4"), (8, 197, 3, 64, 9, False, "32x64 4x2"), (1, 197, 3, 64, 9, False, "32x32 4x2"),
+    (64, 197, 2, 20, 9, False, "32x32 4x4"), (16, 197, 1, 192, 9, True, "128x64 8x4"), (24, 577, 1, 96, 16, True, "64x64 8x4"),
+    (64, 197, 1, 192, 5, True, "64x64 4x4")])
+def test_standard_conv_tiles_of_the_simt_gemm(B, T, H, dk, K, coord, tile):
+    dtype = torch.bfloat16 if coord else torch.float32
+    C = dk + int(coord)
+    Cp = (C + 7) // 8 * 8 if coord else dk
+    g = torch.Generator(device=DEV).manual_seed(B + T + dk)
+    spec = ops.LayerSpec(H * dk, H, K, "all", "cosine", "standard", True, coord, T)
+    v = torch.zeros(B, T, H, Cp, device=DEV)
+    v[..., :C] = torch.randn(B, T, H, C, device=DEV, generator=g)
+    v = v.to(dtype)
+    idx = torch.randint(0, T, (B, H, T, K), device=DEV, generator=g, dtype=torch.int32)
+    val = torch.randn(B, H, T, K, device=DEV, generator=g)
+    w = (torch.randn(dk, K, C, device=DEV, generator=g) / (K * C) ** 0.5).to(dtype)
+    assert _tiles(lambda: ops.gather_conv(spec, v, idx, val, w)) == {tile}
+    got = ops.gather_conv(spec, v, idx, val, w)
+    p = torch.softmax(val.double(), -1)
+    rows = v.double().permute(0, 2, 1, 3)[..., :C]
+    want, mass = torch.zeros(B, H, T, dk, device=DEV, dtype=torch.double), torch.zeros(B, H, T, dk, device=DEV, dtype=torch.double)
+    for j in range(K):
+        nb = p[..., j:j + 1] * torch.gather(rows, 2, idx[..., j:j + 1].long().expand(B, H, T, C))
+        want += nb @ w[:, j].double().T
+        mass += nb.abs() @ w[:, j].double().abs().T
+    # fp32 sums of K * C terms, softmax weights within a few eps; in bfloat16 one rounding of the result
+    bound = (K * C + 16) * EPS * mass + (2.0 ** -8 * want.abs() if coord else 0) + 1e-30
+    assert bool(((got.double() - want).abs() <= bound).all())
+
+
+def _tiles(fn):
+    names = [re.search(r"gemm_simt_kernelI.*?Li[34]ELi(\d+)ELi(\d+)ELi\d+ELi(\d+)ELi(\d+)E", n) for n in launches(fn)]
+    return {"{}x{} {}x{}".format(*m.groups()) for m in names if m}
+
+
+@on_148_sms
+@pytest.mark.parametrize("B,T,H,dk,ks,tile", [(16, 197, 1, 192, 9, "128x64 8x4"), (64, 197, 1, 192, 3, "64x64 8x4"),
+                                              (8, 197, 1, 192, 4, "64x64 4x4"), (32, 197, 1, 192, 3, "32x64 4x4"),
+                                              (8, 197, 1, 96, 9, "32x64 4x2"), (1, 197, 3, 32, 9, "32x32 4x2"), (64, 197, 2, 20, 9, "32x32 4x4")])
+def test_conv1d_tiles_of_the_simt_gemm(B, T, H, dk, ks, tile):
+    D = H * dk
+    g = torch.Generator(device=DEV).manual_seed(B + T + dk)
+    eye, zero = torch.eye(D, device=DEV), torch.zeros(D, device=DEV)
+    x = torch.randn(B, T, D, device=DEV, generator=g)
+    w = torch.randn(dk, ks, dk, device=DEV, generator=g)
+    b = torch.randn(dk, device=DEV, generator=g)
+    call = lambda: ops.conv1d_attention(x, eye, zero, w, b, eye, zero, H, ks)
+    assert _tiles(call) == {tile}
+    left = (ks - 1) // 2
+    y = torch.nn.functional.pad(x.double().view(B, T, H, dk).permute(0, 2, 1, 3), (0, 0, left, ks - 1 - left))
+    z = b.double().expand(B, H, T, dk).clone()
+    mass = b.double().abs().expand(B, H, T, dk).clone()
+    for j in range(ks):
+        z += y[:, :, j:j + T] @ w[:, j].double().T
+        mass += y[:, :, j:j + T].abs() @ w[:, j].double().abs().T
+    flat = lambda t: t.reshape(B, H, dk, T).permute(0, 3, 1, 2).reshape(B, T, D)       # (t, c) rows read back as (c, t)
+    # fp32 sums of ks * dk terms between two products with the identity
+    assert bool(((call().double() - flat(z)).abs() <= (ks * dk + 8) * EPS * flat(mass) + 1e-30).all())
 
 
 @pytest.mark.parametrize("T,S,C,K", [(1, 1, 4, 1), (63, 64, 20, 9), (65, 65, 16, 25), (129, 200, 33, 32), (257, 63, 48, 4),
