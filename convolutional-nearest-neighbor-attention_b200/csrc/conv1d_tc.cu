@@ -213,11 +213,29 @@ conv1d_tc_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant_
 
 }  // namespace
 
+// Where this kernel is faster than unfold + GEMM + merge_heads, which spread a long slice over the chip while one CTA walks its
+// tiles here (0.4 to 5 us each, by taps and channels), and which waste no tile on sequences of a few tokens.  us for the whole
+// branch (two more GEMMs on both sides), others -> this kernel:
+//   slices of up to 256 tokens           8 x 197 x 32, 9 taps 18.9 -> 15.7     300 x 256 x 64, 5 taps 59.7 -> 35.7
+//   longer, few slices                   1 x 600 x 32, 9 taps 19.3 -> 20.4, 1 x 1000 20.9 -> 30.8, 1 x 4096 x 16 29.4 -> 47.1 (not taken)
+//                                        1 x 300 x 32, 9 taps 17.9 -> 16.9     8 x 1000 x 16, 5 taps 21.2 -> 19.1
+//   from a fifth / 0.3 of the SMs        32 x 1000 x 64, 3 taps 30.8 -> 35.0, 25 x 600 x 16, 25 taps 28.3 -> 31.9 (not taken)
+//                                        32 x 1000 x 32, 9 taps 34.2 -> 33.2     48 x 2000 x 32, 9 taps 70.5 -> 57.9
+//   fewer than 32 tokens, many slices    1536 x 9 x 32, 9 taps 23.3 -> 29.1, 300 x 17 x 32, 15 taps 21.1 -> 21.7 (not taken)
+static bool conv1d_tc_wanted(int B, int Tn, int H, int dk, int ks) {
+    const int sms = device_sms();
+    const long long units = (long long)B * H, tiles = (Tn + BM - 1) / BM, n = (units + sms - 1) / sms * tiles;
+    if (Tn < 32) return n == 1 || (n <= 5 && n * ks * dk <= 1100);
+    if (tiles <= 2 || units * 10 >= sms * 3) return true;
+    return tiles * (ks + 4) * dk <= (units * 5 < sms ? 1250 : dk == 64 ? 2400 : 3500);
+}
+
 // y (B, T, H, dk) bfloat16, w (dk, ks, dk), bias (dk) or nullptr -> out (B, T, H dk).  CONVNN_E_UNSUPPORTED (last_error
-// untouched) where the heads are of another width, the slice does not fit beside the taps, or pointers are unaligned.
+// untouched) where the heads are of another width, the other kernels are faster (above), pointers are unaligned, or a slice
+// does not fit beside the taps and one set of boxes (nine taps: 64 channels up to 21 tokens).
 int try_launch_conv1d_tc(const void* y, const void* w, const void* bias, void* out, int B, int Tn, int H, int dk, int ks,
                          cudaStream_t st) {
-    if ((dk != 16 && dk != 32 && dk != 64) || ks > 32 || !aligned16(y) || !aligned16(w) || !aligned16(out)) return CONVNN_E_UNSUPPORTED;
+    if ((dk != 16 && dk != 32 && dk != 64) || ks > 32 || !conv1d_tc_wanted(B, Tn, H, dk, ks) || !aligned16(y) || !aligned16(w) || !aligned16(out)) return CONVNN_E_UNSUPPORTED;
     Conv1dParams p{};
     p.bias = static_cast<const __nv_bfloat16*>(bias); p.out = static_cast<__nv_bfloat16*>(out);
     p.T = Tn; p.H = H; p.dk = dk; p.ks = ks; p.pad = (ks - 1) / 2; p.D = H * dk;

@@ -10,9 +10,9 @@ import pytest
 import torch
 
 import convnn_b200
-from convnn_b200 import _capi
+from convnn_b200 import _capi, ops
 from oracle.convnn_oracle import bf16_round, conv1d_attention, softmax_attention
-from gpu_util import DEV, rel_err
+from gpu_util import DEV, launches, on_148_sms, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -63,7 +63,7 @@ def test_softmax_attention_matches_oracle(B, T, D, H, dtype):
 
 CONV_CASES = [
     # B, T, D, H, kernel_size, dtype
-    (2, 197, 96, 3, 9, torch.bfloat16),     # d_k = 32: unfold + tensor-core GEMM
+    (2, 197, 96, 3, 9, torch.bfloat16),     # d_k = 32: the fused convolution
     (2, 197, 48, 3, 5, torch.bfloat16),     # d_k = 16
     (2, 197, 384, 12, 9, torch.bfloat16),
     (2, 65, 40, 1, 4, torch.bfloat16),      # d_k = 40 (SIMT kernel), even kernel size
@@ -98,11 +98,44 @@ def test_conv1d_attention_matches_oracle(B, T, D, H, ks, dtype):
 
 
 # The fused convolution: one token, whole and ragged 128-row tiles, even kernels, several slices per CTA, heads of 64, one set
-# of taps in flight (25 taps), and a kernel too long for it.
-@pytest.mark.parametrize("B,T,D,H,ks", [(2, 1, 32, 1, 3), (1, 128, 64, 2, 8), (1, 257, 64, 1, 5), (60, 129, 96, 3, 9),
-                                        (200, 65, 32, 2, 4), (2, 300, 32, 1, 25), (2, 50, 128, 2, 1), (1, 60, 64, 1, 25)])
+# of taps in flight (250 tokens); then three that are unfolded (257 tokens: another tile; 25 taps: they do not fit).
+@pytest.mark.parametrize("B,T,D,H,ks", [(2, 1, 32, 1, 3), (1, 128, 64, 2, 8), (60, 129, 96, 3, 9), (200, 65, 32, 2, 4),
+                                        (2, 50, 128, 2, 1), (2, 250, 64, 1, 5), (1, 257, 64, 1, 5), (2, 300, 32, 1, 25), (1, 60, 64, 1, 25)])
 def test_fused_conv1d_attention_matches_oracle(B, T, D, H, ks):
     test_conv1d_attention_matches_oracle(B, T, D, H, ks, torch.bfloat16)
+
+
+# Which shapes the fused convolution takes (slices of at most two tiles, few tiles, or many slices; not many tiny sequences) and
+# its result there and beside them: y = x and out = (conv, reinterpreted) by products with the identity, every element
+# bounded.  Kernels of 16 channels up to 32 taps (the widest mask), one set of taps in flight (250 x 64 x 5, 130 x 32 x 15),
+# whole and ragged tiles, ends of the sequence with even kernels.
+@on_148_sms
+@pytest.mark.parametrize("B,T,H,dk,ks,fused", [
+    (1, 1000, 1, 32, 9, False), (1, 4096, 1, 16, 9, False), (1, 600, 1, 64, 1, False), (25, 600, 1, 16, 25, False),
+    (32, 1000, 1, 64, 3, False), (400, 9, 3, 32, 9, False), (300, 17, 1, 32, 15, False), (2, 300, 1, 32, 25, False),
+    (2, 300, 1, 16, 25, False), (2, 257, 1, 64, 5, False), (1, 300, 1, 32, 9, True), (8, 1000, 1, 16, 5, True), (16, 1000, 2, 32, 9, True), (25, 300, 6, 32, 9, True),
+    (2, 128, 1, 16, 32, True), (2, 130, 2, 32, 15, True), (3, 256, 1, 16, 17, True), (2, 250, 1, 64, 5, True), (1, 127, 2, 64, 4, True),
+    (60, 129, 5, 32, 8, True), (148, 9, 1, 64, 9, True)])
+def test_fused_conv1d_every_element(B, T, H, dk, ks, fused):
+    D, left = H * dk, (ks - 1) // 2
+    g = torch.Generator(device=DEV).manual_seed(T + ks)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+    eye, zero = torch.eye(D, device=DEV).bfloat16(), torch.zeros(D, device=DEV).bfloat16()
+    x, w, b = rnd(B, T, D), rnd(dk, ks, dk), rnd(dk)
+    call = lambda: ops.conv1d_attention(x, eye, zero, w, b, eye, zero, H, ks)
+    assert any("conv1d_tc_kernel" in n for n in launches(call)) == fused
+    got = call().double()
+    torch.cuda.synchronize()
+    assert _capi.device_status() == 0
+    y = torch.nn.functional.pad(x.double().view(B, T, H, dk).permute(0, 2, 1, 3), (0, 0, left, ks - 1 - left))
+    z, mass = [t.expand(B, H, T, dk).clone() for t in (b.double(), b.double().abs())]
+    for j in range(ks):
+        z += y[:, :, j:j + T] @ w[:, j].double().T
+        mass += y[:, :, j:j + T].abs() @ w[:, j].double().abs().T
+    flat = lambda t: t.reshape(B, H, dk, T).permute(0, 3, 1, 2).reshape(B, T, D)       # (t, c) rows read back as (c, t)
+    # fp32 sums of ks * dk terms, one rounding of the result (the products with the identity are exact)
+    bound = (ks * dk + 8) * 2.0 ** -24 * flat(mass) + 2.0 ** -8 * flat(z).abs() + 1e-30
+    assert bool(((got - flat(z)).abs() <= bound).all())
 
 
 def test_branching_modules_fold_the_skip_connection():
