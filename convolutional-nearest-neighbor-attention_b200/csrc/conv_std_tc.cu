@@ -334,14 +334,48 @@ int launch(const ConvStdParams& p, size_t smem, const CUtensorMap& tmW, cudaStre
 
 }  // namespace
 
+// Where this kernel is faster than gather_weighted_kernel + gemm_tc (+ merge_heads).  Its time goes by the 128-token tiles of the
+// busiest CTA (3.6 us and 2.5 to 6.5 a tile), the others' by rows (0.1 to 0.5 ns) from a floor of 7 to 16 us.  One tile per
+// CTA always wins.  Beyond that `fill` counts, the share of those tiles that holds rows: short sequences and ragged ends
+// waste tiles, many taps make the others write more.  us, others -> this kernel, slices x tokens x channels, nine taps unless noted:
+//   1 tile     8 x 65 x 32 10.2 -> 6.9     148 x 100 x 64 13.5 -> 9.5
+//   one slice  8 x 197 x 64 11.0 -> 14.5, 74 x 256 x 64, 5 taps 11.3 -> 12.9 (not taken)     148 x 197 x 64 20.9 -> 15.0, 148 x 2000 x 16 81.8 -> 59.0
+//   several    600 x 17 x 32 11.1 -> 17.9, 600 x 197 x 64, 5 taps 40.7 -> 45.2, 300 x 1000 x 16, 5 taps 53.2 -> 65.2 (not taken)
+//              600 x 197 x 32 44.5 -> 37.5     600 x 256 x 64 85.3 -> 60.5     1536 x 256 x 16 104.7 -> 79.5
+// Merged, the reinterpretation's own kernel (2.5 us and more) is saved as well.  Whole layers of two or four heads, us:
+//   148 slices x 197 x 64 54.3 -> 45.1, 600 x 197 x 32 127.7 -> 117.4     8 x 256 x 64 31.1 -> 34.0, 600 x 17 x 16 43.5 -> 49.9 (not taken)
+// (captured; call by call the saved launches count too: ViT-Tiny of three heads, 16 images 749 -> 719)
+static bool conv_std_wanted(const Dims& dm, bool merged) {
+    const int sms = device_sms();
+    const long long units = (long long)dm.B * dm.H, tiles = (units + sms - 1) / sms * ((dm.T + BM - 1) / BM);
+    if (dm.T > 2 * BM && units < sms) return false;      // (one slice of 600 tokens: 10 us before, 21 here)
+    if (tiles == 1) return true;
+    const double fill = (double)units * dm.T / ((double)tiles * BM * sms), taps = dm.K;
+    if (merged) {
+        // (tokens a multiple of 32 apart lie in one bank for the reinterpreted store: 2 x 256 x 64 30.4 -> 33.2, 2 x 197 x 64 29.7 -> 30.6)
+        if (tiles == 2 && (fill >= 0.4 || dm.K * dm.dk <= 288 || dm.T % 32 != 0)) return true;
+    } else if (units <= sms) {
+        if ((tiles == 2 || dm.K >= 5) && (dm.dk == 32 ? units * 3 >= sms * 2 : units * 5 >= sms * 4)) return true;
+    } else if (tiles == 2 && fill >= 0.5) {
+        return true;
+    }
+    double need;
+    if (dm.dk == 16) need = merged ? 0.45 + 1.25 / taps : dm.K > 16 ? 0.34 : 0.42 + 2.25 / taps;
+    else if (dm.dk == 32) need = (merged ? 0.1 : 0.21) + 2. / taps;
+    else need = 0.25 + (merged ? 1.5 : 2.25) / taps;
+    // sixteen taps of sixteen channels: the weights that a warp's tokens read lie in the same banks (300 x 2000: 226 -> 253)
+    if (dm.dk == 16 && dm.K == 16 && !merged) need += 0.12;
+    return fill >= need;
+}
+
 // merged: o is (B, T, H d_k) in the flat reinterpretation, else (B, H, T, d_k).  CONVNN_E_UNSUPPORTED (last_error untouched)
-// where heads are of another width, where few long slices would leave SMs idle (one of 600 tokens: 10 us before, 21 here), or
-// where the tap weights, two slots and a slice do not fit in shared memory.
+// where heads are of another width, where the other kernels are faster (above), or where the tap weights, two slots and a
+// slice do not fit in shared memory (64 channels: from 14 taps on).
 int try_launch_conv_std_tc(const convnn_desc* d, const Dims& dm, const void* v, const int32_t* idx, const float* val,
                            const void* w_conv, void* o, bool merged, cudaStream_t st) {
     if (d->dtype != CONVNN_BF16 || d->conv_type != CONVNN_STANDARD || d->coord || force_simt() ||
         (dm.dk != 16 && dm.dk != 32 && dm.dk != 64) ||
-        (dm.T > 2 * BM && dm.B * dm.H < device_sms()) || !aligned16(v) || !aligned16(w_conv) || !aligned16(o))
+        !conv_std_wanted(dm, merged) || !aligned16(v) || !aligned16(w_conv) || !aligned16(o))
         return CONVNN_E_UNSUPPORTED;
     ConvStdParams p{};
     p.v = static_cast<const uint4*>(v); p.idx = idx; p.val = val; p.o = static_cast<__nv_bfloat16*>(o);

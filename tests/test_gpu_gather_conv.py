@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from convnn_b200 import ops
-from gpu_util import DEV
+from gpu_util import DEV, launches, on_148_sms
 
 pytestmark = pytest.mark.gpu
 EPS = 2.0 ** -24
@@ -77,22 +77,48 @@ def test_selection_with_conv_equals_the_stages(B, T, S, H, dk, K, metric, softma
 
 
 # The standard conv whose neighbour block stays on the SM: edges of its 128-token tiles, of a producer warp's eight tokens and of
-# its groups of taps, the longest lists, several slices per CTA; then heads narrower and wider than it takes.
-@pytest.mark.parametrize("B,T,H,dk,K", [(1, 127, 2, 16, 5), (2, 128, 1, 32, 6), (1, 129, 3, 64, 3), (3, 9, 2, 64, 4), (2, 256, 1, 32, 32),
-                                        (60, 137, 3, 32, 9), (80, 300, 2, 16, 17), (2, 300, 1, 32, 9), (1, 40, 2, 64, 25), (2, 50, 2, 24, 9)])
+# its groups of taps, the longest lists, several slices per CTA; from the eleventh on shapes
+# that others take: few or sparse tiles, taps that do not fit, 24 channels.
+@pytest.mark.parametrize("B,T,H,dk,K", [(1, 127, 2, 16, 5), (2, 128, 1, 32, 6), (148, 129, 1, 64, 3), (3, 9, 2, 64, 4), (120, 256, 1, 32, 32),
+                                        (100, 197, 3, 32, 9), (74, 300, 2, 16, 17), (148, 250, 4, 16, 17), (148, 300, 1, 32, 9), (148, 256, 1, 64, 9),
+                                        (1, 129, 3, 64, 3), (2, 256, 1, 32, 32), (60, 137, 3, 32, 9), (80, 300, 2, 16, 17), (2, 300, 1, 32, 9),
+                                        (1, 40, 2, 64, 25), (2, 50, 2, 24, 9)])
 def test_standard_conv_tiles(B, T, H, dk, K):
     test_standard_conv_bfloat16_against_float64(B, T, H, dk, K)
 
 
-@pytest.mark.parametrize("B,T,H,dk,K", [(2, 197, 3, 32, 9), (3, 65, 2, 64, 16), (1, 130, 4, 16, 5)])
+# Which shapes it takes, one head (the stage) and several (a layer's reinterpreted store): one tile per CTA, two, several; full
+# and sparse tiles; few and many taps.
+@on_148_sms
+@pytest.mark.parametrize("B,T,H,dk,K,fused", [
+    (8, 65, 1, 32, 9, True), (148, 100, 1, 64, 9, True), (1, 128, 1, 16, 32, True), (8, 197, 1, 64, 9, False), (74, 256, 1, 64, 5, False),
+    (32, 256, 1, 32, 16, False), (148, 130, 1, 64, 3, True), (100, 197, 1, 32, 3, True), (148, 600, 1, 16, 5, True), (200, 100, 1, 16, 9, True),
+    (600, 17, 1, 32, 9, False), (600, 197, 1, 64, 5, False), (600, 197, 1, 32, 9, True), (300, 256, 1, 16, 16, False), (200, 65, 1, 16, 25, True),
+    (1, 600, 1, 32, 9, False), (1, 40, 1, 64, 25, False), (1, 40, 1, 24, 9, False)])
+def test_standard_conv_routes(B, T, H, dk, K, fused):
+    g = torch.Generator(device=DEV).manual_seed(T)
+    spec = ops.LayerSpec(H * dk, H, K, "all", "cosine", "standard", True, False, T)
+    v = torch.randn(B, T, H, dk, device=DEV, generator=g).bfloat16()
+    idx = torch.randint(0, T, (B, H, T, K), device=DEV, generator=g, dtype=torch.int32)
+    val, w = torch.randn(B, H, T, K, device=DEV, generator=g), torch.randn(dk, K, dk, device=DEV, generator=g).bfloat16()
+    assert any("conv_std_tc_kernel" in n for n in launches(lambda: ops.gather_conv(spec, v, idx, val, w))) == fused
+    test_standard_conv_bfloat16_against_float64(B, T, H, dk, K)
+
+
+@on_148_sms
+@pytest.mark.parametrize("B,T,H,dk,K,fused", [(2, 197, 3, 32, 9, True), (2, 65, 2, 64, 9, True), (1, 130, 4, 16, 5, True), (1, 197, 3, 64, 3, True),
+                                              (60, 137, 3, 32, 9, True), (74, 197, 2, 64, 9, True), (40, 300, 4, 32, 9, True),
+                                              (3, 65, 2, 64, 16, False), (4, 256, 2, 64, 9, False), (300, 17, 2, 16, 9, False)])
 @pytest.mark.parametrize("metric,softmax", [("cosine", True), ("matmul", False), ("euclidean", True), ("euclidean", False)])
-def test_standard_conv_in_the_flat_reinterpretation(B, T, H, dk, K, metric, softmax):
+def test_standard_conv_in_the_flat_reinterpretation(B, T, H, dk, K, fused, metric, softmax):
     """The layer's call, whose conv stores the reinterpreted rows, against the stages, which store them as they are."""
     D = H * dk
     g = torch.Generator(device=DEV).manual_seed(T + K)
     rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
     spec = ops.LayerSpec(D, H, K, "all", metric, "standard", softmax, False, T)
     x, w_qkv, w_o, taps = rnd(B, T, D), rnd(3, D, D) * D ** -0.5, rnd(D, D) * D ** -0.5, rnd(dk, K, dk) * (K * dk) ** -0.5
+    names = launches(lambda: ops.forward(spec, x, (w_qkv, taps, None, w_o), None))
+    assert [any(k in n for n in names) for k in ("conv_std_tc_kernel", "merge_heads_kernel")] == [fused, not fused]
     whole = ops.forward(spec, x, (w_qkv, taps, None, w_o), None)
     q, k, v, qs, ks = ops.qkv_proj(spec, x, w_qkv, None)
     idx, val = ops.sim_topk(spec, q, k, qs, ks, None)
