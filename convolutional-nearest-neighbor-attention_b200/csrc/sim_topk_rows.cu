@@ -406,11 +406,28 @@ static Ranges ranges_of(const Dims& dm) {
 //   197 x 197, K = 25        1 image 23.5 -> 8.2    16: 24.1 -> 21.0    48: 24.4 -> 28.3 (not taken)
 //   (two batches in flight lose 0.6 % with it at 256 images: a CTA of this kernel fills its SM)
 //   1000 x 256 x 768, K = 5  1 image 18.0 -> 9.9    4: 18.2 -> 11.1     16: 18.9 -> 21.5 (not taken)
+// Where others win, and the lines of the rule (R rows per SM, rounds u of 256-row units per SM, w the share of their warps that
+// has rows: two units of the streaming kernel share an SM and slow each other down by about w / 2):
+//   * up to 128 candidates, and heads above 384 channels, only ranges that stay inside a head: a range across heads is cut into
+//     segments with a product each (278 x 17 x 17 x 384, K = 9 9.2 -> 11.2; 109 x 65 x 40 x 768 10.9 -> 13.7)
+//   * lists of up to four are cheap elsewhere (256 x 130 x 130 x 16, K = 3 12.9 -> 17.3; 192 x 197 x 197 x 192, K = 3 1.08 times)
+//   * up to 175 candidates the streaming kernel's 64-column tiles fit better (236 x 130 x 130 x 16, K = 5 1.08 times)
+//   * many wide candidates are fetched again for every segment (30 x 1000 x 250 x 384, K = 9 1.13 times; 120 x 256 x 256 x 384 0.91)
+//   * sixteen: in most batches a row or two overflow the survivors' buffer, which adds 6 us (64 x 197 x 197 x 192 14.4 without, 19.5 to
+//     20.7 with, two-pass 19.7; room for 64 costs every batch 5 to 8 %); the two-pass kernel's own slow path, a tie at its threshold, costs
+//     15 us (74 x 224 x 224 x 16 20 or 35).  More candidates or longer sequences lose more (37 x 1000 x 250 x 192 33.7 -> 36.9)
 bool sim_topk_rows_wanted(const Dims& dm) {
     if (dm.S > 256) return false;
-    const int rows = rows_per_sm(dm);
-    if (dm.nsel > 16) return rows <= 32;
-    return rows <= 48 || (dm.S > 128 && dm.Cp <= 384 && rows <= 304);
+    const int R = rows_per_sm(dm);
+    if (dm.nsel > 16) return R <= 32;
+    if (dm.S <= 128 || dm.Cp > 384) return R <= 48 && ranges_of(dm).per_head;
+    if (dm.nsel == 16) return R <= (dm.S <= 208 && dm.T <= 256 ? 304 : 64);
+    if (dm.Cp > 192 && dm.S > 208 && (dm.T > 256 || dm.nsel > 12)) return R <= 96;
+    if (dm.nsel > 12 || (dm.nsel > 4 && dm.S >= 176)) return R <= 304;
+    const int units_of = (dm.T + 255) / 256;
+    const double u = (double)dm.B * dm.H * units_of / device_sms(), w = (double)((dm.T + 31) / 32) / (8 * units_of);
+    if (dm.nsel <= 4) return R <= (dm.S < 144 ? 110 : dm.S < 176 ? 150 : 165) * (u <= 1 ? 1 : u <= 2 ? 1 + 0.4 * w : 2);
+    return R <= (dm.S < 144 ? 128 : 190) * (u <= 1 ? 1 : u <= 2 ? 1 + 0.5 * w : 2);
 }
 
 static int launch_impl(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
@@ -477,11 +494,13 @@ int launch_sim_topk_rows(const convnn_desc* d, const Dims& dm, const void* q, co
 
 // Where a CTA has at most 32 rows, two per warp: the conv's neighbour rows come from L2 a few at a time, which costs less than
 // another kernel then, and more from four rows per warp on.  ViT-Tiny forward, us, lists and conv in two kernels -> in one:
-// 1 image 527 -> 496, 16 images 605 -> 572 (32 rows per CTA), 37: 656 -> 655 (64), 64: 739 -> 817 (96).
+// 1 image 527 -> 496, 16 images 605 -> 572 (32 rows per CTA), 37: 656 -> 655 (64), 64: 739 -> 817 (96).  Not for ranges across
+// heads, whose segments are served one after the other (whole layers: 278 x 17 tokens x 64, K = 9 19.3 -> 24.9), nor for more
+// than 12 KB of taps over short lists, where the conv is the longer part (23 x 100 x 768, K = 9 46.2 -> 48.7, but 3 x 197 44.9 -> 37.7).
 int try_launch_sim_gather(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const void* v, const float* qstat,
                           const float* kstat, const int32_t* cand, const void* w_conv, void* o, cudaStream_t st) {
-    if (!sim_topk_tc_supported(d, dm, q, k) || !sim_topk_rows_wanted(dm) || dm.nsel > 16 || ranges_of(dm).rows > 32 || dm.C != dm.dk || dm.dk % 8 != 0 ||
-        (size_t)dm.K * dm.dk * 2 > 16 * 1024 || !aligned16(v) || !aligned16(w_conv) || !aligned16(o))
+    if (!sim_topk_tc_supported(d, dm, q, k) || dm.S > 256 || dm.nsel > 16 || ranges_of(dm).rows > 32 || !ranges_of(dm).per_head ||
+        dm.C != dm.dk || dm.dk % 8 != 0 || dm.K * dm.dk > (dm.S <= 128 ? 6144 : 8192) || !aligned16(v) || !aligned16(w_conv) || !aligned16(o))
         return CONVNN_E_UNSUPPORTED;
     return launch_impl(d, dm, q, k, qstat, kstat, cand, nullptr, nullptr, v, w_conv, o, st);
 }

@@ -57,18 +57,25 @@ def test_standard_conv_bfloat16_against_float64(B, T, H, dk, K):
 
 # Selection and depthwise conv in one kernel (few rows per SM, at most 17 neighbours) against the two stages, whose lists and
 # sums are the same: bit for bit.  One row, ragged sequences, sixteen and seventeen neighbours, one channel group, the widest
-# taps, several heads, every way of weighting; the last shape has too many rows for it.
-@pytest.mark.parametrize("B,T,S,H,dk,K", [(1, 1, 1, 1, 16, 1), (3, 197, 197, 1, 192, 9), (1, 197, 197, 3, 64, 9), (2, 65, 40, 1, 48, 17),
-                                          (5, 130, 100, 1, 16, 16), (2, 257, 225, 1, 384, 5), (1, 33, 33, 2, 80, 12),
-                                          (1, 500, 256, 1, 768, 10), (40, 197, 197, 1, 64, 9)])
+# taps, several heads, every way of weighting; then two rows per warp (32 rows per CTA), odd ends and seventeen neighbours among
+# them.  The last four do not go to it: too many rows per CTA, ranges across heads, and long taps over short lists.
+@on_148_sms
+@pytest.mark.parametrize("B,T,S,H,dk,K,fused", [
+    (1, 1, 1, 1, 16, 1, True), (3, 197, 197, 1, 192, 9, True), (1, 197, 197, 3, 64, 9, True), (2, 65, 40, 1, 48, 17, True),
+    (5, 130, 100, 1, 16, 16, True), (2, 257, 225, 1, 384, 5, True), (1, 33, 33, 2, 80, 12, True), (1, 500, 256, 1, 768, 10, True),
+    (16, 197, 197, 1, 64, 9, True), (20, 197, 197, 1, 192, 9, True), (10, 200, 150, 2, 32, 17, True), (40, 83, 60, 1, 16, 17, True),
+    (139, 17, 17, 1, 32, 9, True), (6, 250, 250, 3, 32, 16, True),
+    (40, 197, 197, 1, 64, 9, False), (200, 17, 17, 1, 32, 9, False), (300, 9, 9, 1, 16, 9, False), (23, 100, 100, 1, 768, 9, False)])
 @pytest.mark.parametrize("metric,softmax", [("cosine", True), ("matmul", False), ("euclidean", True), ("euclidean", False)])
-def test_selection_with_conv_equals_the_stages(B, T, S, H, dk, K, metric, softmax):
+def test_selection_with_conv_equals_the_stages(B, T, S, H, dk, K, fused, metric, softmax):
     D = H * dk
     g = torch.Generator(device=DEV).manual_seed(T + S + K)
     rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
     spec = ops.LayerSpec(D, H, K, "spatial" if S != T else "all", metric, "depthwise", softmax, False, T)
     x, w_qkv, w_o, taps = rnd(B, T, D), rnd(3, D, D) * D ** -0.5, rnd(D, D) * D ** -0.5, rnd(K, dk)
     cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if S != T else None
+    names = launches(lambda: ops.forward(spec, x, (w_qkv, taps, None, w_o), cand))
+    assert any("sim_topk_rows_kernel" in n and "Lb1E" in n for n in names) == fused
     whole = ops.forward(spec, x, (w_qkv, taps, None, w_o), cand)
     q, k, v, qs, ks = ops.qkv_proj(spec, x, w_qkv, cand)
     idx, val = ops.sim_topk(spec, q, k, qs, ks, cand)

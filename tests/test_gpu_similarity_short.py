@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from convnn_b200 import ops
-from gpu_util import DEV
+from gpu_util import DEV, launches, on_148_sms
 
 pytestmark = pytest.mark.gpu
 
@@ -80,11 +80,12 @@ def test_metrics_at_the_ends(metric):
 
 
 # Batches at which a CTA of the warp-per-row kernel has several segments (whole sequences, ends, ranges across heads), and
-# the first ones that go to the two-pass and the streaming kernel instead.
+# some beside them that go to the two-pass and the streaming kernel (test_warp_per_row_routes has the lines).
 @pytest.mark.parametrize("T,S,H,dk,K,B", [(197, 197, 1, 64, 9, 90), (197, 197, 3, 32, 9, 64), (197, 197, 1, 32, 9, 300),
                                           (150, 150, 1, 16, 16, 152), (1, 1, 1, 16, 1, 3000), (33, 17, 1, 32, 9, 150),
                                           (130, 130, 2, 64, 5, 74), (300, 200, 1, 48, 12, 149), (65, 65, 1, 64, 25, 60),
-                                          (197, 64, 1, 64, 9, 74), (197, 197, 1, 64, 25, 60), (197, 64, 1, 64, 9, 200)])
+                                          (197, 64, 1, 64, 9, 74), (197, 197, 1, 64, 25, 60), (197, 64, 1, 64, 9, 200), (17, 17, 1, 32, 17, 278),
+                                          (256, 256, 1, 64, 3, 55)])
 @pytest.mark.parametrize("values", ["few", "many", "nan"])
 def test_exact_lists_of_many_rows(T, S, H, dk, K, B, values):
     sampled = S != T
@@ -138,3 +139,24 @@ def test_exact_lists_float32(T, S, H, dk, K, B, values):
         key = torch.where(own, torch.full_like(key, -0.1) * torch.tensor(math.sqrt(dk), dtype=torch.float32, device=DEV), key)
     want_idx, _ = expect(key, n)
     assert torch.equal(idx.long()[..., K - n:], want_idx if cand is None else cand.long()[want_idx])
+
+
+# Lines of the rule: which kernel takes a batch just inside and just outside of each.
+@on_148_sms
+@pytest.mark.parametrize("B,T,S,H,dk,K,dtype,rows", [
+    # bfloat16: at most 128 candidates and wide heads: 48 rows per SM, inside a head
+    (139, 17, 17, 1, 384, 9, torch.bfloat16, True), (278, 17, 17, 1, 384, 9, torch.bfloat16, False), (109, 65, 40, 1, 768, 9, torch.bfloat16, False),
+    (71, 100, 100, 1, 64, 9, torch.bfloat16, True), (74, 100, 100, 1, 64, 9, torch.bfloat16, False), (5, 197, 197, 1, 768, 9, torch.bfloat16, True),
+    # more candidates, by the length of the list
+    (37, 197, 197, 2, 32, 3, torch.bfloat16, True), (256, 130, 130, 1, 16, 3, torch.bfloat16, False), (192, 197, 197, 1, 192, 3, torch.bfloat16, False),
+    (236, 130, 130, 1, 16, 5, torch.bfloat16, False), (140, 130, 130, 1, 16, 5, torch.bfloat16, True), (220, 197, 197, 1, 192, 9, torch.bfloat16, True),
+    (256, 197, 197, 1, 192, 9, torch.bfloat16, False), (30, 1000, 250, 1, 384, 9, torch.bfloat16, False), (120, 256, 256, 1, 384, 9, torch.bfloat16, True),
+    (64, 197, 197, 1, 192, 16, torch.bfloat16, True), (37, 1000, 250, 1, 192, 17, torch.bfloat16, False), (64, 197, 197, 1, 192, 13, torch.bfloat16, True),
+    (16, 197, 197, 1, 192, 25, torch.bfloat16, True), (48, 197, 197, 1, 192, 25, torch.bfloat16, False)])
+def test_warp_per_row_routes(B, T, S, H, dk, K, dtype, rows):
+    g = torch.Generator(device=DEV).manual_seed(1)
+    spec = ops.LayerSpec(H * dk, H, K, "spatial" if S != T else "all", "matmul", "depthwise", True, False, T)
+    q, k = (torch.randn(B, r, H, dk, device=DEV, generator=g).to(dtype) for r in (S, T))
+    cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if S != T else None
+    names = launches(lambda: ops.sim_topk(spec, q, k, None, None, cand))
+    assert len(names) == 1 and any(n in next(iter(names)) for n in ("sim_topk_rows_kernel", "sim_topk_simt_rows_kernel")) == rows
