@@ -264,13 +264,22 @@ int launch(const convnn_desc* d, const Dims& dm, const void* q, const void* k, c
     return CONVNN_OK;
 }
 
+// Rows per CTA and CTAs.  128 rows per CTA use the pipes better (8 x 4 dot products per thread instead of 4 x 4); 64 where the
+// 128-row grid leaves SMs without work or most of a tile is padding.
+struct Blocks {
+    int rows;
+    long long ctas;
+};
+inline Blocks blocks_of(const Dims& dm) {
+    const long long bh = (long long)dm.B * dm.H, wide = (dm.T + 127) / 128 * bh;
+    if (wide >= device_sms() && ((dm.T + 127) / 128) * 128 <= ((dm.T + 63) / 64) * 64 * 5 / 4) return {128, wide};
+    return {64, (dm.T + 63) / 64 * bh};
+}
+
 template <typename T>
 int dispatch(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
              const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st) {
-    // 128 rows per CTA use the pipes better (8 x 4 dot products per thread instead of 4 x 4); 64 where the 128-row grid
-    // leaves SMs without work or most of a tile is padding.
-    const long long wide = (long long)((dm.T + 127) / 128) * dm.B * dm.H;
-    const bool rows128 = wide >= device_sms() && ((dm.T + 127) / 128) * 128 <= ((dm.T + 63) / 64) * 64 * 5 / 4;
+    const bool rows128 = blocks_of(dm).rows == 128;
 #define CONVNN_LAUNCH(KC)                                                                                     \
     return rows128 ? launch<T, KC, 128>(d, dm, q, k, qstat, kstat, cand, idx, val, st)                        \
                    : launch<T, KC, 64>(d, dm, q, k, qstat, kstat, cand, idx, val, st)

@@ -161,18 +161,34 @@ int launch(const convnn_desc* d, const Dims& dm, const void* q, const void* k, c
 }
 
 // What bounds it: shared-memory reads of the product (12 values per 32 multiply-adds), with one or two CTAs per SM; the
-// streaming kernel reads less per multiply-add in its 128-row CTAs and catches up once every SM has several of them.
-// us, streaming -> this kernel (float32, K = 9, one head, unless noted):
+// streaming kernel reads less per multiply-add in its 128-row CTAs and catches up once every SM has several of them.  From
+// 8/3 CTAs per SM on the padded work of its busiest SM (rounds x rows x 64-column tiles) is therefore weighed against this
+// kernel's, a 32-row CTA of which costs as much as 32 (a S + b).  Long lists cost the streaming kernel more: from 10 on up
+// to 25/6 CTAs per SM, above 16 always.  us, streaming -> this kernel (float32, K = 9, one head, unless noted):
 //   65 x 65 x 192       1 to 32 images 29 -> 13       256: 52.8 -> 41.9
 //   197 x 197 x 192     1: 50.1 -> 19.2    64: 76.3 -> 58.5    256: 209 -> 199 (not taken)
 //   577 x 150 x 385 bfloat16, K = 16    7: 101 -> 42    32: 187 -> 134        65 x 65 x 192, K = 25    300: 157 -> 59
 //   197 x 64 x 384      16: 30.0 -> 23.5   64: 43.3 -> 51.4 (not taken)       197 x 49, 3 heads of 64  16: 15.7 -> 10.9
-//   2000 x 100 x 256    32: 145 -> 156 (not taken)                            256 x 256 x 256, K = 16  128: 175 -> 191 (not taken)
+//   100 x 100 x 192     150: 0.87 of the time   230: 57.4 -> 64.1 (not taken)   130 x 130 x 400, K = 16  152: 232 -> 123
+//   1000 x 100 x 192    18: 43.8 -> 49.6 (not taken)   16 channels, K = 16  18: 34.4 -> 17.8
+//   256 x 256 x 400     75: 0.81 of the time   115: 1.25 times (not taken)      100 x 100 x 16, K = 1  230: 11.8 -> 17.3 (not taken)
 static bool wanted(const Dims& dm) {
-    const long long ctas = (long long)((dm.T + RB - 1) / RB) * dm.B * dm.H, sms = device_sms();
+    const long long bh = (long long)dm.B * dm.H, ctas = (dm.T + RB - 1) / RB * bh, sms = device_sms();
     if (dm.S > 256) return false;
-    if (dm.S <= 64) return ctas <= sms * 8 / 3;
-    return dm.nsel > 16 || ctas <= sms * 25 / 4;
+    if (dm.nsel > 16 && dm.S > 64) return true;
+    const bool light = dm.nsel <= 4 && dm.Cp <= 64;                   // little to select, little to multiply: mostly fixed costs
+    if (light && dm.Cp <= 32 && dm.S > 32) return ctas <= 2 * sms;    // (109 x 65 x 40 x 16, K = 1 6.9 -> 7.4 from there on)
+    if (ctas <= sms * 8 / 3) return true;
+    if (dm.S <= 64 || ctas > sms * 25 / 4) return false;
+    const bool few = ctas <= sms * 25 / 6;
+    if (dm.nsel >= 10 && few) return true;
+    double a = 1.0, b = 50;
+    if (dm.Cp > 256) { a = 1.3; b = 40; }
+    else if (dm.nsel >= 10) { a = 1.1; b = 20; }
+    else if (light) { a = 0.9; b = few ? 110 : 130; }
+    const simt_topk::Blocks other = simt_topk::blocks_of(dm);
+    const long long streamed = (other.ctas + sms - 1) / sms * other.rows * ((dm.S + 63) / 64 * 64);
+    return (double)((ctas + sms - 1) / sms) * RB * (a * dm.S + b) < (double)streamed;
 }
 
 template <typename T, int J>

@@ -119,7 +119,8 @@ def test_exact_lists_of_many_rows(T, S, H, dk, K, B, values):
 @pytest.mark.parametrize("T,S,H,dk,K,B", [(1, 1, 1, 3, 1, 1), (31, 31, 1, 32, 9, 2), (33, 33, 2, 33, 5, 2), (65, 65, 1, 192, 9, 3),
                                           (40, 32, 3, 20, 16, 2), (70, 64, 1, 31, 9, 2), (100, 97, 1, 64, 25, 2), (96, 96, 1, 65, 32, 2),
                                           (129, 129, 1, 16, 9, 2), (300, 150, 1, 48, 16, 2), (197, 197, 3, 64, 9, 4),
-                                          (256, 256, 1, 7, 12, 2), (257, 225, 1, 40, 26, 2), (64, 40, 1, 8, 9, 500)])
+                                          (256, 256, 1, 7, 12, 2), (257, 225, 1, 40, 26, 2), (64, 40, 1, 8, 9, 500), (165, 165, 1, 33, 9, 2),
+                                          (192, 192, 2, 16, 12, 2)])
 @pytest.mark.parametrize("values", ["few", "many", "nan"])
 def test_exact_lists_float32(T, S, H, dk, K, B, values):
     sampled = S != T
@@ -141,7 +142,7 @@ def test_exact_lists_float32(T, S, H, dk, K, B, values):
     assert torch.equal(idx.long()[..., K - n:], want_idx if cand is None else cand.long()[want_idx])
 
 
-# Lines of the rule: which kernel takes a batch just inside and just outside of each.
+# Lines of the two rules: which kernel takes a batch just inside and just outside of each.
 @on_148_sms
 @pytest.mark.parametrize("B,T,S,H,dk,K,dtype,rows", [
     # bfloat16: at most 128 candidates and wide heads: 48 rows per SM, inside a head
@@ -152,7 +153,13 @@ def test_exact_lists_float32(T, S, H, dk, K, B, values):
     (236, 130, 130, 1, 16, 5, torch.bfloat16, False), (140, 130, 130, 1, 16, 5, torch.bfloat16, True), (220, 197, 197, 1, 192, 9, torch.bfloat16, True),
     (256, 197, 197, 1, 192, 9, torch.bfloat16, False), (30, 1000, 250, 1, 384, 9, torch.bfloat16, False), (120, 256, 256, 1, 384, 9, torch.bfloat16, True),
     (64, 197, 197, 1, 192, 16, torch.bfloat16, True), (37, 1000, 250, 1, 192, 17, torch.bfloat16, False), (64, 197, 197, 1, 192, 13, torch.bfloat16, True),
-    (16, 197, 197, 1, 192, 25, torch.bfloat16, True), (48, 197, 197, 1, 192, 25, torch.bfloat16, False)])
+    (16, 197, 197, 1, 192, 25, torch.bfloat16, True), (48, 197, 197, 1, 192, 25, torch.bfloat16, False),
+    # float32: 8/3 CTAs per SM, then by the streaming kernel's work
+    (32, 65, 65, 1, 192, 9, torch.float32, True), (64, 197, 197, 1, 192, 9, torch.float32, True), (150, 100, 100, 1, 192, 9, torch.float32, True),
+    (230, 100, 100, 1, 192, 9, torch.float32, False), (18, 1000, 100, 1, 192, 9, torch.float32, False), (18, 1000, 100, 1, 16, 16, torch.float32, True),
+    (75, 256, 256, 1, 400, 9, torch.float32, True), (115, 256, 256, 1, 400, 9, torch.float32, False), (152, 130, 130, 1, 400, 16, torch.float32, True),
+    (230, 100, 100, 1, 16, 1, torch.float32, False), (109, 65, 40, 1, 16, 1, torch.float32, False), (64, 197, 64, 1, 384, 9, torch.float32, False),
+    (300, 65, 65, 1, 192, 25, torch.float32, True), (131, 256, 256, 1, 33, 12, torch.float32, False)])
 def test_warp_per_row_routes(B, T, S, H, dk, K, dtype, rows):
     g = torch.Generator(device=DEV).manual_seed(1)
     spec = ops.LayerSpec(H * dk, H, K, "spatial" if S != T else "all", "matmul", "depthwise", True, False, T)
