@@ -1,11 +1,10 @@
 // The Conv1d half of the reference's MultiHeadBranchingConv (MultiHeadConv1dAttention.forward,
 // layers.py:477-500): per-head Conv1d(d_k, d_k, kernel_size, padding='same') over the tokens.
 //
-// Activations are token-major (B, T, H, d_k).  What conv1d_tc.cu does not take comes here.  bfloat16 with d_k a multiple of 16:
-// the taps are
-// unfolded, U[(b, h, t), j * d_k + c] = y[b, t + j - pad, h, c] (zero outside the sequence), and
-// the conv becomes U x W^T with W = (d_k, kernel_size * d_k) on the tensor-core GEMM, bias in its
-// epilogue.  Float32 takes the SIMT GEMM with the shifted rows as its implicit A operand; head widths that are no
+// Activations are token-major (B, T, H, d_k).  What conv1d_tc.cu does not take comes here: other head widths, heads of 64
+// channels with the default nine taps from 22 tokens on, few long slices.  bfloat16 with d_k a multiple of 16: the taps are unfolded,
+// U[(b, h, t), j * d_k + c] = y[b, t + j - pad, h, c] (zero outside the sequence), and the conv becomes U x W^T with
+// W = (d_k, kernel_size * d_k) on the tensor-core GEMM, bias in its epilogue.  Float32 takes the SIMT GEMM with the shifted rows as its implicit A operand; head widths that are no
 // multiple of four a direct SIMT kernel.
 #include "common.cuh"
 

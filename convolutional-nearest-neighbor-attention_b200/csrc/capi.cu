@@ -142,7 +142,9 @@ size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 // GEMM operand and for the head-merged (B, T, D) operand of the output projection.
 size_t stage_scratch(const Dims& dm, int conv_type) {
     size_t n = (size_t)dm.B * (dm.T > dm.S ? dm.T : dm.S) * dm.D;
-    if (conv_type == CONVNN_STANDARD && dm.elt == 2 && dm.C == dm.dk) {          // weighted neighbour block (B, H, T, K*C) of the tensor-core conv
+    // Weighted neighbour block (B, H, T, K*C) of the tensor-core conv.  Shapes whose block stays on the SM leave it unused unless v or
+    // the taps are unaligned; sizes do not depend on pointers, and buffers of this size stay valid.
+    if (conv_type == CONVNN_STANDARD && dm.elt == 2 && dm.C == dm.dk) {
         const size_t m = (size_t)dm.B * dm.H * dm.T * dm.K * dm.C;
         if (m > n) n = m;
     } else if (conv_type == CONVNN_DEPTHWISE_SEPARABLE) {
@@ -738,6 +740,7 @@ int convnn_b200_softmax_attention(int dtype, const void* x, int64_t ldx, const v
 size_t convnn_b200_conv1d_attention_workspace_bytes(int dtype, int32_t B, int32_t T, int32_t D, int32_t kernel_size) {
     if ((dtype != CONVNN_F32 && dtype != CONVNN_BF16) || B < 1 || T < 1 || D < 1 || kernel_size < 1) return 0;
     const size_t elt = dtype == CONVNN_F32 ? 4 : 2, part = up256((size_t)B * T * D * elt);
+    // (the unfolded operand also for shapes that only unfold where the taps are unaligned)
     return 3 * part + up256((size_t)B * T * D * kernel_size * elt);
 }
 

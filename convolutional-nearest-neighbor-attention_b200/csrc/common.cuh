@@ -33,7 +33,7 @@ void count_launch();
 // predecessor has waited likewise, so completion is transitive along the stream.  chain_next() lets the successor start;
 // it comes after the wait (nothing older than the predecessor can still run when a successor starts) and, in kernels that
 // allocate TMEM, after the allocation (a successor's CTA may take only what is left, and gives it back).
-// A ViT-Tiny forward is 64 kernels with gaps of ~1.9 us and prologues of ~2 us.  One image 827 -> 712 us, 37 images
+// A ViT-Tiny forward is 64 kernels (52 up to 21 images) with gaps of ~1.9 us and prologues of ~2 us.  One image 827 -> 712 us, 37 images
 // 923 -> 808 us, 256 images 1757 -> 1673 us, BranchConv 64 images 1788 -> 1500 us, ViT-Small 256 images 4588 -> 4441 us.
 __device__ __forceinline__ void chain_wait() { cudaGridDependencySynchronize(); }
 __device__ __forceinline__ void chain_next() { cudaTriggerProgrammaticLaunchCompletion(); }
@@ -247,12 +247,13 @@ int launch_attention(int dtype, const void* q, const void* k, const void* v, voi
 int read_attention_status(int* out);
 int launch_conv1d_heads(int dtype, const void* y, const void* w, const void* bias, void* o, void* unfold, int B,
                         int Tn, int H, int dk, int ks, cudaStream_t st);
-// Conv1d half and its flat reinterpretation in one kernel (heads of 16, 32 or 64 channels).
+// Conv1d half and its flat reinterpretation in one kernel (heads of 16, 32 or 64 channels whose taps fit in shared memory, by a rule
+// on the number and length of the slices).
 int try_launch_conv1d_tc(const void* y, const void* w, const void* bias, void* out, int B, int Tn, int H, int dk, int ks,
                          cudaStream_t st);
 int read_conv1d_tc_status(int* out);
-// Standard conv with its weighted neighbour block kept on the SM (bfloat16 heads of 16, 32 or 64 channels); merged: o is
-// (B, T, D) in the flat reinterpretation.
+// Standard conv with its weighted neighbour block kept on the SM (bfloat16 heads of 16, 32 or 64 channels whose taps fit, by a rule on
+// tiles per SM and taps); merged: o is (B, T, D) in the flat reinterpretation.
 int try_launch_conv_std_tc(const convnn_desc* d, const Dims& dm, const void* v, const int32_t* idx, const float* val,
                            const void* w_conv, void* o, bool merged, cudaStream_t st);
 int read_conv_std_status(int* out);

@@ -1,5 +1,6 @@
-// The Conv1d half of MultiHeadBranchingConv on the tensor cores, heads of 16, 32 or 64 channels: convolution and the flat
-// reinterpretation of its result in one kernel (reference layers.py:477-500).
+// The Conv1d half of MultiHeadBranchingConv on the tensor cores: convolution and the flat reinterpretation of its result in one
+// kernel (reference layers.py:477-500), for heads of 16, 32 or 64 channels whose taps and one set of boxes fit beside a
+// slice (nine taps: 32 channels up to 2074 tokens, 64 channels up to 21) and where conv1d_tc_wanted() finds it the faster way.
 //
 //   o[b, h, t, oc] = bias[oc] + sum_{j, c} w[oc, j, c] * y[b, t + j - pad, h, c]          (zero outside the sequence)
 //   out[b, t', h * dk + c'] = flat(o[b, h])[c' * T + t']
@@ -10,8 +11,9 @@
 // the copy and the second kernel that the reinterpretation cost.  Terms are added in the order of the unfolded GEMM (bias,
 // then taps and channels ascending in steps of 16): the same bits.
 //
-// Bound by latency (a handful of tiles per SM): 64 images x 197 tokens x 3 heads of 32, 9 taps: 11 us, 24 as
-// unfold (11), GEMM (8.6) and reinterpretation (4.6) in kernels of their own.
+// Bound by latency (a handful of tiles per SM; 0.12 instructions per cycle and scheduler, the warps wait for boxes and for one
+// another): 64 images x 197 tokens x 3 heads of 32, 9 taps: 11 us, 24 as unfold (11), GEMM (8.6) and reinterpretation (4.6) in
+// kernels of their own.
 //
 // Warps: 0 TMA (lane j loads tap j), 1 MMA issuer, 2-9 epilogue: two sets of four (lane quarters), one per accumulator.
 #include "common.cuh"

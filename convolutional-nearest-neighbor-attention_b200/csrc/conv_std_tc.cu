@@ -8,7 +8,8 @@
 // v went through memory twice.  A CTA owns whole (batch, head) slices, so with several heads the result can leave in the
 // flat reinterpretation the output projection reads (layers.py:247-259), without a kernel of its own.
 //
-// Bound by the latency of a tile's weights and neighbour rows on sixteen warps.  128 images x 197 tokens x 12 heads of 32, 9
+// Bound by the instructions that fetch, weigh and store the neighbour rows (0.57 per cycle and scheduler, shared-memory wavefronts 51 %)
+// and their latency on sixteen warps.  128 images x 197 tokens x 12 heads of 32, 9
 // taps: 78 us, with the reinterpretation; 98 + 11 us before (block 174 MB written and read).  64 images, 3 heads: 17 (17.5 + 4).
 //
 // Warps: 0 MMA issuer and TMA of the taps, 1-16 producers, 17-20 epilogue (lane quarters).

@@ -8,7 +8,7 @@
 // Kernels, in the order the dispatcher tries them:
 //   * depthwise with 16-byte rows: gather_conv_dw_stream.cu (short bfloat16 sequences, V through shared memory) and
 //     gather_conv_dw.cu; other channel counts: a scalar kernel here;
-//   * bfloat16 standard, heads of 16, 32 or 64 channels: conv_std_tc.cu, whose neighbour block stays on the SM;
+//   * bfloat16 standard, heads of 16, 32 or 64 channels, where it is faster: conv_std_tc.cu, whose neighbour block stays on the SM;
 //   * bfloat16 standard / separable on the tensor cores: a gather kernel writes the GEMM's A
 //     operand (the weighted neighbour block, or the depthwise result) and gemm_tc multiplies it
 //     with the (d_k, K*C) tap matrix / the (d_k, C) pointwise matrix;
@@ -16,7 +16,7 @@
 //     separable over the depthwise result;
 //   * channel counts that are no multiple of four: shared-memory staged block times the weights.
 // The three K-times expanded copies of V that the reference builds never exist (the tensor-core
-// standard conv of other head widths materialises the weighted block once, in bfloat16).
+// standard conv of the other shapes materialises the weighted block once, in bfloat16).
 #include "common.cuh"
 #include "token_weights.cuh"
 

@@ -397,8 +397,8 @@ static Ranges ranges_of(const Dims& dm) {
     return r;
 }
 
-// What bounds it: warp instructions, ~300 per row of 197 keys with the copy, at 0.5 to 0.8 per cycle and scheduler.  A row
-// costs about the same wherever it runs, while the two-pass kernel works in whole 128-row units and the streaming kernel
+// What bounds it: warp instructions, ~310 per row of 197 keys with the copy, at 0.44 per cycle and scheduler (148 images; copying
+// the accumulator and selecting do not overlap).  A row costs about the same wherever it runs, while the two-pass kernel works in whole 128-row units and the streaming kernel
 // needs many rows per SM to hide its chains.  us, others -> this kernel, 192 channels unless noted:
 //   197 x 197, K = 9         1 image 14.9 -> 6.5    37: 15.2 -> 8.8    148: 21.9 -> 17.1    220: 30.4 -> 26.2    256: 30.4 -> 30.2 (not taken)
 //   12 heads of 64           1 image 14.8 -> 6.6    16: 27.5 -> 22.3    32: 40.4 -> 37.8 (not taken)

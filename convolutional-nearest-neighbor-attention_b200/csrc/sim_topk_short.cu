@@ -428,10 +428,11 @@ int launch_short(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const C
 
 }  // namespace
 
-// What the warp-per-row kernel leaves to it where the streaming kernel would leave most of the chip idle: up to one unit per
-// SM.  B x 197 tokens of 192 channels, K = 9: 15.4 us for 1 to 74 images, streaming 21.6; 256 images (3.5 units per SM) 34.6 against 30.8, where eight to sixteen
-// streaming warps per SM hide each other's latency.  Lists of 13 to 16 always: their streaming variant runs one CTA per SM
-// (577 tokens, 150 candidates, K = 16: 1 image 26.4 -> 18.5 us, 74 images 49.9 -> 39.8, 256 images 132 -> 107).
+// What the warp-per-row kernel leaves to it where the streaming kernel would leave most of the chip idle: up to one unit per SM.  us,
+// streaming -> this kernel: 148 x 100 x 100 x 64, K = 9 11.5 -> 9.5, 74 x 197 x 64 x 384 12.9 -> 9.3, 37 x 197 x 197 x 768 22.8 -> 18.0, 48 x
+// 197 x 197 x 192, K = 25 33.8 -> 23.0.  With several units per SM eight to sixteen streaming warps hide each other's latency (256 images
+// of 197 x 192, K = 9: 30.8, 34.6 here).  Lists of 13 to 16 always: their streaming variant runs one CTA per SM (256 x 577 x 150 x 384,
+// K = 16 129 -> 110; 256 x 197 x 197 x 192 47.0 -> 49.0).
 bool sim_topk_short_wanted(const Dims& dm) {
     const long long units = (long long)dm.B * dm.H * ((dm.T + BM - 1) / BM);
     return dm.S <= 256 && (units <= device_sms() || (dm.nsel > 12 && dm.nsel <= 16));
