@@ -17,8 +17,10 @@ __device__ __forceinline__ float linspace_pm1(int i, int steps) {
     return (i < steps / 2) ? (-1.0f + step * (float)i) : (1.0f - step * (float)(steps - 1 - i));
 }
 
-// Up to three tensors of one layer in a launch, one per grid row (a launch each, before: 2.5 us per tensor at 2080 rows of
-// 192 float32 channels, all of it latency).
+// Up to three tensors of one layer in a launch, one per grid row: bound by the latency of a row's loads and shuffles, so six CTAs per SM
+// (40 registers), and nothing in local memory: the tensor is picked by comparisons, since an index that is no constant would put the
+// struct on the stack.  Projections with statistics, us, a launch per tensor -> one: 1 x 197 x 2 heads of 16 7.3 -> 5.5, 32 x 65 x 192
+// float32 26.1 -> 23.9, 128 x 197 x 3 heads of 64 float32 174.6 -> 168.2 (with the stack: 4 CTAs, 176.2; 100 x 197 x 2 heads of 16 31.1 for 26.1).
 struct HeadTensors {
     void* t[3];
     float* stat[3];
@@ -26,11 +28,12 @@ struct HeadTensors {
 };
 
 template <typename T>
-__global__ void head_stats_kernel(const HeadTensors in, int B, int H, int dk, int C, int Cp, int coord, int metric) {
+__global__ void __launch_bounds__(256, 6) head_stats_kernel(const HeadTensors in, int B, int H, int dk, int C, int Cp, int coord, int metric) {
     chain_begin();
-    T* t = static_cast<T*>(in.t[blockIdx.y]);
-    float* stat = in.stat[blockIdx.y];
-    const int rows = in.rows[blockIdx.y];
+    const int which = blockIdx.y;
+    T* t = static_cast<T*>(which == 0 ? in.t[0] : which == 1 ? in.t[1] : in.t[2]);
+    float* stat = which == 0 ? in.stat[0] : which == 1 ? in.stat[1] : in.stat[2];
+    const int rows = which == 0 ? in.rows[0] : which == 1 ? in.rows[1] : in.rows[2];
     const int warps_per_block = blockDim.x >> 5;
     const long long total = (long long)B * rows * H;
     const int lane = threadIdx.x & 31;

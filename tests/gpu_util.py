@@ -49,7 +49,7 @@ def rel_err(a, b):
 
 
 def launches(fn):
-    """{kernel name (mangled): threads per block} of what fn() launches, read from a captured graph."""
+    """{kernel name (mangled): bytes of local memory per thread} of what fn() launches, read from a captured graph."""
     from cuda.bindings import driver
 
     def ok(r):
@@ -68,7 +68,8 @@ def launches(fn):
         if ok(driver.cuGraphNodeGetType(node))[0] != driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
             continue
         p = ok(driver.cuGraphKernelNodeGetParams(node))[0]
-        name = ok(driver.cuFuncGetName(p.func) if int(p.func) else driver.cuKernelGetName(p.kern))[0]
-        found[name.decode()] = p.blockDimX
+        func = p.func if int(p.func) else ok(driver.cuKernelGetFunction(p.kern))[0]
+        found[ok(driver.cuFuncGetName(func))[0].decode()] = ok(driver.cuFuncGetAttribute(
+            driver.CUfunction_attribute.CU_FUNC_ATTRIBUTE_LOCAL_SIZE_BYTES, func))[0]
     graph.reset()
     return found

@@ -210,3 +210,28 @@ def test_similarity_lists_float32(T, S, C, K, metric):
         tied = (got == S // 2).int().argmax(-1)
         both = (got == 0).any(-1) & (got == S // 2).any(-1)
         assert S < 2 or bool((first[both] < tied[both]).all())
+
+
+@pytest.mark.parametrize("B,T,S,H,dk,coord,dtype", [(3, 65, 65, 2, 16, False, torch.bfloat16), (2, 100, 40, 1, 20, True, torch.bfloat16),
+                                                    (2, 50, 50, 3, 12, False, torch.float32), (1, 33, 20, 1, 24, True, torch.float32)])
+@pytest.mark.parametrize("metric", ["cosine", "euclidean"])
+def test_statistics_of_all_tensors_in_one_launch(B, T, S, H, dk, coord, dtype, metric):
+    """Norms of the stored q and k, the coordinate channel of all three, and a kernel without local memory."""
+    D, C = H * dk, dk + int(coord)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    spec = ops.LayerSpec(D, H, 5, "spatial" if S != T else "all", metric, "standard", True, coord, T)
+    x, w = (torch.randn(*s, device=DEV, generator=g).to(dtype) for s in ((B, T, D), (3, D, D)))
+    cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if S != T else None
+    names = {n: local for n, local in launches(lambda: ops.qkv_proj(spec, x, w, cand)).items() if "head_stats_kernel" in n}
+    assert list(names.values()) == [0]
+    q, k, v, qs, ks = ops.qkv_proj(spec, x, w, cand)
+    for t, stat, rows in ((q, qs, S), (k, ks, T), (v, None, T)):
+        if coord:
+            ramp = torch.linspace(-1, 1, rows, device=DEV).to(dtype).view(1, rows, 1)
+            assert bool(((t[..., dk] - ramp).abs() <= 2.0 ** -8).all()) and not bool(t[..., C:].any())
+        if stat is None:
+            continue
+        want = t[..., :C].double().square().sum(-1).permute(0, 2, 1)
+        want = 1 / want.sqrt().clamp_min(1e-12) if metric == "cosine" else want
+        # a C-term fp32 sum of squares, a root and a division
+        assert bool(((stat.view(B, H, rows).double() - want).abs() <= (C + 8) * EPS * want.abs() + 1e-30).all())
