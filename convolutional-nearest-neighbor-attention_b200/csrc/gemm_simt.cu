@@ -342,18 +342,21 @@ int launch_mode(const GemmParams& p, cudaStream_t st) {
     //   64 x 64    1: 8 x 197 x 192 133 -> 103   3: 20 x 577 x 100 113 -> 128 (not taken)   4: 64 x 197 x 192 314 -> 301   5: 32 x 197 x 384 675 -> 706 (not taken)
     //   32 x 64    1: 8 x 197 x 3 x 64 32.4 -> 27.7   4: 32 x 197 x 192 206 -> 212
     //   32 x 32    1: 1 x 65 x 192 104 -> 67   6: 64 x 197 x 2 heads of 20 21.9 -> 28.1 (not taken)
-    // Shifted rows cost one division less and gain less: 16 x 197 x 192 209 -> 177 (1), 64 x 197 x 192 312 -> 342 (4, not taken).
-    // Tap rows of C values against more stored channels come value by value: in bfloat16 they gain longest (coordinate channel,
-    // 64 x 197 x 192, 64 x 64 tiles, 4: 617 -> 375; 24 x 577 x 96, 16 taps, 3: 240 -> 303, not taken).  Plain rows lose up to 20 %.
+    // Shifted rows cost one division less and gain less: 16 x 197 x 192 209 -> 177 (1), 64 x 197 x 192 312 -> 342 (4, not taken), 32 x 197 x 72
+    // bfloat16 32 x 32 tiles 0.83 of the time (4).
+    // Tap rows of C values against more stored channels (the coordinate channel) come value by value: in bfloat16 they gain longest, longer
+    // still where an odd number of taps leaves every other row of them at an odd address.  64 x 64, 4: 64 x 197 x 192 617 -> 375; 3: 24 x 197 x
+    // 384, 9 taps 726 -> 615, 24 x 577 x 96, 8 taps 123 -> 151 (not taken); 32 x 32, 7: 159 x 65 x 96, 25 taps 741 -> 391, 6 and one column
+    // of tiles: 48 x 577 x 20, 16 taps 58 -> 63 (not taken).  Plain rows lose up to 20 %.
     if constexpr (MODE == A_NEIGHBOURS || MODE == A_CONV1D) {
         const long long per_sm = (tiles_of[best] + sms - 1) / sms, here = best == 3 ? 4 : 2, other = best == 3 ? 7 : 3;
         bool twice = (per_sm + here - 1) / here <= (per_sm + other - 1) / other;
         if (MODE == A_CONV1D) {
-            twice = 2 * per_sm <= here;
+            twice = best == 3 ? per_sm <= (sizeof(T) == 2 ? 4 : 3) : per_sm == 1;
         } else {
             const bool by_value = p.C != p.Cp && sizeof(T) == 2;
             if (per_sm > other && (best == 0 || by_value)) twice = true;
-            if (by_value && best < 3 && p.taps < 16) twice = true;
+            if (by_value && (best < 3 ? p.taps % 2 != 0 : p.N > 32)) twice = true;
         }
         if (twice) {
             if (best == 0) return launch_tile<TA, T, MODE, 128, 64, 16, 8, 4, 2>(p, st);

@@ -98,7 +98,8 @@ def test_conv1d_branch_float32(T, dk, ks):
     (8, 197, 1, 192, 9, False, "64x64 4x4"), (20, 577, 1, 100, 9, False, "64x64 8x4"), (64, 197, 1, 192, 9, False, "64x64 4x4"),
     (32, 197, 1, 384, 2, False, "64x64 8x4"), (8, 197, 3, 64, 9, False, "32x64 4x2"), (1, 197, 3, 64, 9, False, "32x32 4x2"),
     (64, 197, 2, 20, 9, False, "32x32 4x4"), (16, 197, 1, 192, 9, True, "128x64 8x4"), (24, 577, 1, 96, 16, True, "64x64 8x4"),
-    (64, 197, 1, 192, 5, True, "64x64 4x4")])
+    (64, 197, 1, 192, 5, True, "64x64 4x4"), (24, 577, 1, 96, 8, True, "64x64 8x4"), (24, 197, 1, 384, 3, True, "64x64 4x4"),
+    (159, 65, 1, 96, 25, True, "32x32 4x2"), (48, 577, 1, 20, 16, True, "32x32 4x4")])
 def test_standard_conv_tiles_of_the_simt_gemm(B, T, H, dk, K, coord, tile):
     dtype = torch.bfloat16 if coord else torch.float32
     C = dk + int(coord)
