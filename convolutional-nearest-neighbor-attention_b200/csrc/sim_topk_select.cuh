@@ -24,10 +24,11 @@ __device__ __forceinline__ void prefix_insert(TopList<NSEL>& top, const float (&
 // qs points at the W column statistics of this chunk in shared memory (16-byte aligned, the same
 // for every lane: broadcast loads); cv holds the candidate token of column (32-aligned base +
 // lane).  P needs the fields metric, sampled and S (number of candidate columns).
-template <int NSEL, int W, class P>
+// FLOOR: keys at or below `floor` are known to lie outside the row's final list.
+template <int NSEL, int W, bool FLOOR = false, class P>
 __device__ __forceinline__ void consume(TopList<NSEL>& top, const uint32_t (&acc)[W], int col0, int lane_off,
                                         const float* qs, int cv, const P& p, int row, bool row_ok, float sentinel,
-                                        float* ks) {
+                                        float* ks, float floor = 0.f) {
     float key[W];
     if (p.metric != CONVNN_MATMUL) {
         const f32x2 two = pack2(2.0f, 2.0f);
@@ -69,7 +70,7 @@ __device__ __forceinline__ void consume(TopList<NSEL>& top, const uint32_t (&acc
         }
         return;
     }
-    const float thr = top.worst();
+    const float thr = FLOOR ? fmaxf(top.worst(), floor) : top.worst();
     uint32_t mask = 0;
 #pragma unroll
     for (int j = 0; j < W; ++j) mask |= (key[j] > thr) ? (1u << j) : 0u;
@@ -94,6 +95,13 @@ __device__ __forceinline__ void consume(TopList<NSEL>& top, const uint32_t (&acc
             if (live && kc > top.worst()) top.insert_sorted(kc, col0 + jc);
         }
     }
+}
+
+// The largest float below x (x itself for -inf): key > just_below(x) holds exactly where key >= x does.
+__device__ __forceinline__ float just_below(float x) {
+    const int b = __float_as_int(x);
+    const int down = b > 0 ? b - 1 : (b == 0 ? (int)0x80000001 : b + 1);
+    return x == -CUDART_INF_F ? x : __int_as_float(down);
 }
 
 // Ranking key of a sampled row's own column: the finite stand-in the reference uses

@@ -71,7 +71,9 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     float* keybuf = reinterpret_cast<float*>(smem + NST * STAGE_BYTES);       // [2 column halves][CW][128]
     float* mbuf = keybuf + 2 * CW * kSelGroup;                                // [2 * NSEL][128] merge hand-over
     float* statbuf = mbuf + 2 * NSEL * kSelGroup;                             // [8 warps][128] column statistics of the tile
-    uint64_t* bars = reinterpret_cast<uint64_t*>(statbuf + 8 * 128);
+    // [2 column halves][128 rows]: (rank value, unit number) of a row's list so far, see `floor` below
+    volatile unsigned long long* ranks = reinterpret_cast<volatile unsigned long long*>(statbuf + 8 * 128);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(statbuf + 8 * 128) + 2 * kSelGroup;
     uint64_t* full = bars;                      // used in the leader only
     uint64_t* empty = bars + STAGES;
     uint64_t* tfull = bars + 2 * STAGES;
@@ -104,6 +106,7 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         prefetch_tensormap(&tmK);
         prefetch_tensormap(&tmQ);
     }
+    if (threadIdx.x < 2 * kSelGroup) ranks[threadIdx.x] = 0ull;      // (unit numbers start at one)
     __syncthreads();
     if (warp == 1) {
         tmem_alloc_pair(tmem_slot, 512);
@@ -184,6 +187,16 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         float* ks = keybuf + chalf * CW * kSelGroup + r;
         float* sq = statbuf + (warp - 2) * 128;
         uint32_t it = 0;                         // units done by this CTA (phase of the merge barriers)
+        // A list alone only learns the NSEL-th largest key of its own half of the columns, which is about the 2 NSEL-th of
+        // the row.  The R0-th key of the lower half's list and the R1-th of the upper half's, R0 + R1 = NSEL, are NSEL keys
+        // that are no smaller than the smaller of the two: a key below that is in no final list.  Each warp publishes its
+        // value after every 32 columns, with the number of its unit, and reads the other's, which may be older (a rank's
+        // value only grows within a unit) or of another unit (then it is not used).  Equal keys stay: the order among them
+        // goes by column, and the other half may hold the higher ones.  768 channels: 16384 x 4096, K = 25 1184 -> 1119 us; 4096 x
+        // 4096, K = 9 198.4 -> 196.5 (the products bound it); 384 channels, K = 16 204 -> 197; 3000 x 1500 x 128, K = 12 104 -> 98.
+        constexpr int R0 = (NSEL + 1) / 2, R1 = NSEL / 2;
+        volatile unsigned long long* own_rank = ranks + chalf * kSelGroup + r;
+        volatile unsigned long long* their_rank = ranks + (chalf ^ 1) * kSelGroup + r;
         const uint32_t lead_tempty0 = map_to_cta(tempty0, 0);
         uint32_t tile = 0;
         bool ok = true;
@@ -197,6 +210,7 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
             const float sentinel = p.sampled ? self_sentinel(p.metric, kst, p.sqrt_dk) : 0.f;
             TopList<NSEL> top;
             top.init();
+            float my_rank = -CUDART_INF_F;
             float qv[4], qn[4];
             int cv[4], cn[4];
             auto fetch = [&](int ct, float (&fq)[4], int (&fc)[4]) {
@@ -230,8 +244,15 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
                         if (cbase + c4 * 32 < p.S) {             // otherwise the rest of the tile is padding
                             uint32_t acc[32];
                             tmem_ld_x32(taddr + c4 * 32, acc);
+                            const unsigned long long other = *their_rank;
+                            const float floor = (uint32_t)(other >> 32) == it + 1
+                                                    ? just_below(fminf(my_rank, __uint_as_float((uint32_t)other)))
+                                                    : -CUDART_INF_F;
                             tmem_ld_wait();
-                            consume<NSEL, 32>(top, acc, cbase + c4 * 32, 0, sq + c4 * 32, cv[c4], p, row, row_ok, sentinel, ks);
+                            consume<NSEL, 32, true>(top, acc, cbase + c4 * 32, 0, sq + c4 * 32, cv[c4], p, row, row_ok,
+                                                    sentinel, ks, floor);
+                            my_rank = chalf == 0 ? top.v[R0 - 1] : top.v[R1 - 1];
+                            *own_rank = ((unsigned long long)(it + 1) << 32) | __float_as_uint(my_rank);
                         }
                     }
                 }
@@ -333,7 +354,7 @@ int launch_sim_topk_tc2(const convnn_desc* d, const Dims& dm, const void* q, con
     if (!encode_tensor_map_bf16(&tmK, k, 4, dimsK, strK, boxK, KCH * 2)) return CONVNN_E_CUDA;
     if (!encode_tensor_map_bf16(&tmQ, q, 4, dimsQ, strQ, boxQ, KCH * 2)) return CONVNN_E_CUDA;
 
-    const size_t smem_fixed = 1024 + 2 * CW * kSelGroup * sizeof(float) + 8 * 128 * sizeof(float) +
+    const size_t smem_fixed = 1024 + 2 * CW * kSelGroup * sizeof(float) + 8 * 128 * sizeof(float) + 2 * kSelGroup * 8 +
                               (2 * STAGES + 12) * 8 + 16;
 
 #define CONVNN_TC2_LAUNCH(N)                                                                                     \

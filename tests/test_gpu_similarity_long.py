@@ -1,0 +1,43 @@
+"""The pair kernel's selection under ties: small whole numbers, whose products and sums are exact, so that every list is known."""
+import pytest
+import torch
+
+from convnn_b200 import ops
+from gpu_util import DEV, launches
+
+pytestmark = pytest.mark.gpu
+
+
+# Whole tiles of 256 columns and a ragged end; an upper half of the last tile that is padding; even and odd lists (the two
+# halves' shares differ); rows that are all ties, and keys that grow or fall with the column, so that one half of a tile always
+# sees the better ones first.
+@pytest.mark.parametrize("T,S,dk,K", [(1100, 1100, 128, 9), (1024, 1024, 128, 5), (1030, 1153, 192, 16), (1281, 1040, 128, 12),
+                                      (8192, 4096, 128, 25), (8200, 4225, 128, 26), (8192, 4100, 128, 32)])
+@pytest.mark.parametrize("order", ["mixed", "rising", "falling"])
+def test_ties_go_to_the_lower_column(T, S, dk, K, order):
+    T = max(T, S)
+    g = torch.Generator(device=DEV).manual_seed(T + S + K)
+    spec = ops.LayerSpec(dk, 1, K, "all" if S == T else "spatial", "matmul", "depthwise", True, False, T)
+    q = torch.randint(-1, 2, (1, S, 1, dk), device=DEV, generator=g).float()
+    k = torch.randint(-1, 2, (1, T, 1, dk), device=DEV, generator=g).float()
+    k[:, 5] = 0                                                # every key of this row is the same
+    if order != "mixed":                                       # steps of 64 columns, more than the rest of a product reaches
+        step = (torch.arange(S, device=DEV) // 64).float()
+        q[0, :, 0, 0] = step if order == "rising" else step.flip(0)
+        k[..., 0] = 4.0
+        k[:, 5] = 0
+    cand = None if S == T else torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32)
+    qb, kb = q.bfloat16(), k.bfloat16()
+    call = lambda: ops.sim_topk(spec, qb, kb, None, None, cand)
+    assert any("sim_topk_tc2_kernel" in n for n in launches(call))
+    idx, val = call()
+    key = k[0, :, 0] @ q[0, :, 0].T                            # exact: whole numbers below 2^24
+    n, first = K, 0
+    if cand is not None:
+        own = cand.view(1, S).long() == torch.arange(T, device=DEV).view(T, 1)
+        key = key.masked_fill(own, -0.1 * dk ** 0.5)
+        n, first = K - 1, 1
+        assert torch.equal(idx[0, 0, :, 0].long(), torch.arange(T, device=DEV))
+    col = key.sort(dim=1, descending=True, stable=True).indices[:, :n]
+    want = col if cand is None else cand.long()[col]
+    assert torch.equal(idx[0, 0, :, first:].long(), want)
