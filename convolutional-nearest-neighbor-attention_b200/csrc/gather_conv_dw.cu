@@ -7,9 +7,10 @@
 // whose neighbour rows are TPT independent 16-byte loads in flight.
 //
 // Reads K x the size of V, most of it from L2 and L1: at 131072 tokens of 768 channels and 25 taps 5.0 GB against
-// 0.2 GB of values.  There L2 is 42 % busy and the ALU, which unpacks, 50 %: bound by the latency of the neighbour rows.
-// Before, one thread per output group issued its taps one after another, and shapes whose V slice fits in shared memory
-// were tied to one CTA per slice: 144 us for one image of 65 tokens, 768 channels and 16 taps.
+// 0.2 GB of values.  There L2 is 42 % busy and the ALU, which unpacks, 50 %: bound by the latency of the neighbour rows, so
+// what counts is how many of them an SM has in flight: four tokens side by side, one tap at a time and three CTAs (80
+// registers), whose (row, weight) pairs of a tap lie together: 131072 x 768 x 25 501 -> 477 us (two taps and two CTAs, 104
+// registers, before), 32768 x 768 x 9 66.2 -> 58.4, 32768 x 384 x 9 35.4 -> 32.6; one token: four taps, four CTAs.
 #include "common.cuh"
 #include "f32x2.cuh"
 
@@ -50,50 +51,69 @@ __device__ __forceinline__ void store_group(float* o, const f32x2 (&a)[N]) {
     for (int q = 0; q < N; q += 2) *reinterpret_cast<ulonglong2*>(o + 2 * q) = make_ulonglong2(a[q], a[q + 1]);
 }
 
-// (neighbour row in units of VEC channels, weight) pairs of tokens m0 ... m0 + nt - 1 into shared memory.  The exponentials
-// are taken by all threads; a token's maximum and its sum in tap order by one, so the weights are those of a serial loop.
-template <int VEC>
+// (neighbour row in units of VEC channels, weight) pairs of tokens m0 ... m0 + nt - 1 into shared memory, the TPT tokens of
+// a set side by side per tap.  The exponentials are taken by all threads; a token's maximum and its sum in tap order by
+// one, so the weights are those of a serial loop.  The places behind the last token hold its rows again.
+template <int VEC, int TPT>
 __device__ __forceinline__ void token_pairs(const DwParams& p, int m0, int nt, int2* pairs, float* red) {
-    const int n = nt * p.K;
+    const int n = nt * p.K, n_up = (nt + TPT - 1) / TPT * TPT * p.K;
     const long long nbase = (long long)m0 * p.K;
-    for (int e = threadIdx.x; e < n; e += THREADS) {
-        const int bh = (m0 + e / p.K) / p.T, b = bh / p.H, h = bh - b * p.H;
-        const float x = p.val[nbase + e];
-        pairs[e] = make_int2(((b * p.T + p.idx[nbase + e]) * p.H + h) * (p.Cp / VEC), __float_as_int(p.maximum ? x : -x));
+    auto at = [&](int t, int j) { return TPT == 1 ? t * p.K + j : ((t / TPT) * p.K + j) * TPT + t % TPT; };
+    for (int e = threadIdx.x; e < n_up; e += THREADS) {
+        const int slot = e / p.K, t = TPT == 1 ? slot : min(slot, nt - 1);
+        const long long ne = nbase + (e - (slot - t) * p.K);
+        const int bh = (m0 + t) / p.T, b = bh / p.H, h = bh - b * p.H;
+        const float x = p.val[ne];
+        pairs[TPT == 1 ? e : at(slot, e - slot * p.K)] =
+            make_int2(((b * p.T + p.idx[ne]) * p.H + h) * (p.Cp / VEC), __float_as_int(p.maximum ? x : -x));
     }
     __syncthreads();
+    // f(weight, token) over all of them
+    auto each = [&](auto f) {
+        for (int e = threadIdx.x; e < n; e += THREADS) {
+            const int t = e / p.K;
+            int& y = pairs[TPT == 1 ? e : at(t, e - t * p.K)].y;
+            y = __float_as_int(f(__int_as_float(y), t));
+        }
+    };
     if (p.softmax) {
         for (int t = threadIdx.x; t < nt; t += THREADS) {
             float m = -3.402823466e38f;
-            for (int j = 0; j < p.K; ++j) m = fmaxf(m, __int_as_float(pairs[t * p.K + j].y));
+            for (int j = 0; j < p.K; ++j) m = fmaxf(m, __int_as_float(pairs[at(t, j)].y));
             red[t] = m;
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < n; e += THREADS)
-            pairs[e].y = __float_as_int(expf(__int_as_float(pairs[e].y) - red[e / p.K]));
+        each([&](float x, int t) { return expf(x - red[t]); });
         __syncthreads();
         for (int t = threadIdx.x; t < nt; t += THREADS) {
             float s = 0.f;
-            for (int j = 0; j < p.K; ++j) s += __int_as_float(pairs[t * p.K + j].y);
+            for (int j = 0; j < p.K; ++j) s += __int_as_float(pairs[at(t, j)].y);
             red[t] = s;
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < n; e += THREADS) pairs[e].y = __float_as_int(__int_as_float(pairs[e].y) / red[e / p.K]);
+        each([&](float x, int t) { return x / red[t]; });
     } else if (!p.maximum) {
-        for (int e = threadIdx.x; e < n; e += THREADS) pairs[e].y = __float_as_int(1.0f / (-__int_as_float(pairs[e].y) + 1e-8f));
+        each([](float x, int) { return 1.0f / (-x + 1e-8f); });
     }
     __syncthreads();
 }
 
+// Rows in flight: TPT tokens side by side per tap, UNROLL taps; more of either leaves fewer warps (MINB CTAs per SM).
+template <typename T, typename TO, int TPT> struct DwShape {
+    static constexpr bool wider = sizeof(TO) > sizeof(T);
+    static constexpr int UNROLL = TPT == 4 ? 1 : (wider ? 2 : 4), MINB = TPT == 4 ? 3 : (wider ? 5 : 4);
+};
+
 template <typename T, typename TO, int VEC, int TPT>
-__global__ void __launch_bounds__(THREADS) gather_conv_dw_kernel(const DwParams p, const int TT) {
+__global__ void __launch_bounds__(THREADS, DwShape<T, TO, TPT>::MINB) gather_conv_dw_kernel(const DwParams p, const int TT) {
     chain_begin();
     typedef Channels<T, VEC> Ch;
+    constexpr int UNROLL = DwShape<T, TO, TPT>::UNROLL;
     extern __shared__ __align__(16) unsigned char dw_smem[];
-    int2* pairs = reinterpret_cast<int2*>(dw_smem);           // [TT][K]
+    int2* pairs = reinterpret_cast<int2*>(dw_smem);           // [TT / TPT][K][TPT]
     float* red = reinterpret_cast<float*>(pairs + TT * p.K);  // [TT]
     const int m0 = blockIdx.x * TT, nt = min(TT, p.M - m0);
-    token_pairs<VEC>(p, m0, nt, pairs, red);
+    token_pairs<VEC, TPT>(p, m0, nt, pairs, red);
 
     const typename Ch::raw* v = static_cast<const typename Ch::raw*>(p.v);
     const T* w = static_cast<const T*>(p.w);
@@ -101,23 +121,29 @@ __global__ void __launch_bounds__(THREADS) gather_conv_dw_kernel(const DwParams 
     for (int item = threadIdx.x; item < sets * p.groups; item += THREADS) {
         const int set = item / p.groups, cg = item - set * p.groups, c = cg * VEC;
         const typename Ch::raw* vc = v + cg;
-        const int2* pr[TPT];
-#pragma unroll
-        for (int q = 0; q < TPT; ++q) pr[q] = pairs + min(set * TPT + q, nt - 1) * p.K;
+        const int2* pr = pairs + set * p.K * TPT;
         f32x2 acc[TPT][VEC / 2];
 #pragma unroll
         for (int q = 0; q < TPT; ++q)
 #pragma unroll
             for (int e = 0; e < VEC / 2; ++e) acc[q][e] = 0ull;
-#pragma unroll 2
+#pragma unroll UNROLL
         for (int j = 0; j < p.K; ++j) {
             typename Ch::raw raw[TPT];
             float pj[TPT];
+            if constexpr (TPT == 1) {
+                const int2 e = pr[j];
+                raw[0] = vc[e.x];
+                pj[0] = __int_as_float(e.y);
+            } else {
 #pragma unroll
-            for (int q = 0; q < TPT; ++q) {
-                const int2 e = pr[q][j];
-                raw[q] = vc[e.x];
-                pj[q] = __int_as_float(e.y);
+                for (int q = 0; q < TPT; q += 2) {
+                    const int4 e = *reinterpret_cast<const int4*>(pr + j * TPT + q);
+                    raw[q] = vc[e.x];
+                    raw[q + 1] = vc[e.z];
+                    pj[q] = __int_as_float(e.y);
+                    pj[q + 1] = __int_as_float(e.w);
+                }
             }
             f32x2 w2[VEC / 2];
             if (p.wvec) {
@@ -154,7 +180,7 @@ __global__ void __launch_bounds__(THREADS) gather_weighted_kernel(const DwParams
     int2* pairs = reinterpret_cast<int2*>(dw_smem);
     float* red = reinterpret_cast<float*>(pairs + TT * p.K);
     const int m0 = blockIdx.x * TT, nt = min(TT, p.M - m0);
-    token_pairs<8>(p, m0, nt, pairs, red);
+    token_pairs<8, 1>(p, m0, nt, pairs, red);
     const uint4* v = static_cast<const uint4*>(p.v);
     uint4* o = static_cast<uint4*>(p.o) + (long long)m0 * p.K * p.groups;
     const int n = nt * p.K * p.groups;                        // output vectors, consecutive in memory
@@ -190,8 +216,8 @@ template <typename T, typename TO, int VEC>
 int launch(const DwParams& p, cudaStream_t st) {
     // Four tokens per thread where that still leaves every SM two CTAs' worth of threads, else one.  Tokens per CTA: one
     // item (token set, channel group) per thread on small grids; on large ones up to eight, as long as six CTAs per SM
-    // remain, so that a CTA's prologue (its tokens' weights) is spread over more rows: 131072 x 768, 25 taps 641 us
-    // with one item per thread, 501 with eight (5.0 GB of neighbour rows, 10 TB/s; 772 before).
+    // remain, so that a CTA's prologue (its tokens' weights) is spread over more rows (131072 x 768, 25 taps: 641 us
+    // with one item per thread where eight took 501).
     const long long items = (long long)p.M * p.groups;
     const int tpt = items >= 4LL * device_sms() * 512 ? 4 : 1;
     int TT = (THREADS * tpt + p.groups - 1) / p.groups;

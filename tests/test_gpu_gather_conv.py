@@ -131,3 +131,11 @@ def test_standard_conv_in_the_flat_reinterpretation(B, T, H, dk, K, fused, metri
     idx, val = ops.sim_topk(spec, q, k, qs, ks, None)
     out = ops.out_proj(spec, ops.gather_conv(spec, v, idx, val, taps), w_o, S=T)
     assert torch.equal(whole.isnan(), out.isnan()) and torch.equal(whole.nan_to_num(), out.nan_to_num())
+
+
+# Four tokens per thread: a last set of one, two, three tokens, one tap and many, taps and rows of one vector less than a warp's.
+@pytest.mark.parametrize("B,T,H,dk,K", [(1, 6401, 1, 384, 9), (2, 3203, 1, 384, 1), (5, 1283, 1, 384, 25), (3, 1024, 2, 248, 5), (1, 40001, 1, 72, 32)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_sets_of_four_tokens(B, T, H, dk, K, dtype):
+    test_depthwise_against_float64(B, T, H, dk, K, dtype, "cosine", True)
+    test_depthwise_against_float64(B, T, H, dk, K, dtype, "euclidean", False)
