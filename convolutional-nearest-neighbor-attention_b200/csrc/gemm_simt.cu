@@ -54,6 +54,72 @@ struct ARow {
     int t;                // token (A_CONV1D)
 };
 
+// Bias, GELU, skip connection and store of a thread's outputs: TM rows row_of(i) by CG groups of VN neighbouring columns, the
+// first of group g being n0 + g * step; value(i, g, r) reads a group's sums.
+template <typename T, int TM, int CG, int VN, class Row, class Value>
+__device__ __forceinline__ void store_outputs(const GemmParams& p, int n0, int step, Row row_of, Value value) {
+    const T* bias = static_cast<const T*>(p.bias);
+#pragma unroll
+    for (int g = 0; g < CG; ++g) {
+        const int n = n0 + g * step;
+        if (n >= p.N) continue;
+        const int nv = min(VN, p.N - n);
+        const int part = n / p.part_cols, pn = n - part * p.part_cols;
+        T* c = static_cast<T*>(part == 0 ? p.c : (part == 1 ? p.c1 : p.c2));
+        int col = pn;
+        if (p.c_mode == C_HEADS) {
+            const int h = pn / p.dk;
+            col = h * p.Cp + (pn - h * p.dk);
+        }
+        const bool vec = VN == 4 && p.c_vec && nv == 4;         // the four columns are neighbours in one output row
+        float bb[VN] = {};
+        if (bias && !p.bias_first)
+#pragma unroll
+            for (int j = 0; j < VN; ++j)
+                if (j < nv) bb[j] = to_f32<T>(bias[n + j]);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int m = row_of(i);
+            if (m >= p.M) continue;
+            float r[VN];
+            value(i, g, r);
+#pragma unroll
+            for (int j = 0; j < VN; ++j) {
+                if (bias && !p.bias_first) r[j] += bb[j];
+                if (p.gelu) r[j] = gelu_exact(r[j]);
+            }
+            const long long row = p.c_mode == C_HEADS ? (long long)m * p.H * p.Cp : (long long)m * p.ldc;
+            if constexpr (VN == 4) {
+                if (vec) {
+                    if (p.residual) {
+                        const float4 q = load4(static_cast<const T*>(p.residual) + (long long)m * p.ldr + n);
+                        const float rq[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) r[j] = to_f32<T>(from_f32<T>(r[j])) + rq[j];
+                    }
+                    store4(c + row + col, r);
+                    continue;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < VN; ++j) {
+                if (j >= nv) continue;
+                float v = r[j];
+                const int nn = n + j, pp = nn / p.part_cols;
+                int cj = nn - pp * p.part_cols;
+                T* cc = static_cast<T*>(pp == 0 ? p.c : (pp == 1 ? p.c1 : p.c2));
+                if (p.c_mode == C_HEADS) {
+                    const int h = cj / p.dk;
+                    cj = h * p.Cp + (cj - h * p.dk);
+                }
+                if (p.residual)
+                    v = to_f32<T>(from_f32<T>(v)) + to_f32<T>(static_cast<const T*>(p.residual)[(long long)m * p.ldr + nn]);
+                cc[row + cj] = from_f32<T>(v);
+            }
+        }
+    }
+}
+
 // Tile BM x BN, NT = (BM / TM) * (BN / TN) threads in warps of 4 (rows) x 8 (columns).
 // TA: type of the A operand (float32 against bfloat16 weights for the separable conv's unrounded intermediate).
 template <typename TA, typename T, int MODE, int BM, int BN, int BK, int TM, int TN, int MINB>
@@ -243,66 +309,128 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_kernel(
         }
     }
 
-#pragma unroll
-    for (int g = 0; g < CG; ++g) {
-        const int n = n0 + g * (BN / CG) + tx * VN;
-        if (n >= p.N) continue;
-        const int nv = min(VN, p.N - n);
-        const int part = n / p.part_cols, pn = n - part * p.part_cols;
-        T* c = static_cast<T*>(part == 0 ? p.c : (part == 1 ? p.c1 : p.c2));
-        int col = pn;
-        if (p.c_mode == C_HEADS) {
-            const int h = pn / p.dk;
-            col = h * p.Cp + (pn - h * p.dk);
-        }
-        const bool vec = VN == 4 && p.c_vec && nv == 4;         // the four columns are neighbours in one output row
-        float bb[VN] = {};
-        if (bias && !p.bias_first)
-#pragma unroll
-            for (int j = 0; j < VN; ++j)
-                if (j < nv) bb[j] = to_f32<T>(bias[n + j]);
-#pragma unroll
-        for (int i = 0; i < TM; ++i) {
-            const int m = m0 + (i / VM) * (BM / RG) + ty * VM + i % VM;
-            if (m >= p.M) continue;
-            float r[VN];
+    store_outputs<T, TM, CG, VN>(
+        p, n0 + tx * VN, BN / CG, [&](int i) { return m0 + (i / VM) * (BM / RG) + ty * VM + i % VM; },
+        [&](int i, int g, float (&r)[VN]) {
 #pragma unroll
             for (int j = 0; j < VN / 2; ++j) unpack2(acc[i][g * (VN / 2) + j], r[2 * j], r[2 * j + 1]);
+        });
+}
+
+// float32 rows that can be copied 16 bytes at a time: steps of 32 k values land by asynchronous copies, three ahead, in the
+// order they have in memory (a row is 128 bytes, its 16-byte pieces exchanged, so that the lanes of a warp read their rows
+// without conflicts and nothing is transposed); a thread reads four k values of its rows at once, the next four while
+// these are multiplied.  Plain multiply-adds: they run at the rate of the packed ones (70 against 67 TFLOP/s with four
+// warps per scheduler) and need no pairs.  Same sums as above, k strictly ascending.  A tile is two warps, so that its
+// steps wait for no others and small outputs spread evenly over the SMs; the shared-memory port, TM + TN cycles per
+// warp and k value, and the latency of a lone warp per scheduler bound it.
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+template <int MODE, int BM, int BN, int TM, int TN, int MINB>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_copy_kernel(const GemmParams p) {
+    static_assert(MODE == A_ROWS || MODE == A_TOKENS, "plain rows");
+    chain_begin();
+    constexpr int NT = (BM / TM) * (BN / TN), BK = 32, ST = 4, PIECES = BK / 4;
+    constexpr int WN = BN / TN / 8;
+    constexpr int NL = (BM + BN) * PIECES / NT;                 // copies per thread and step
+    static_assert((BM + BN) * PIECES % NT == 0 && NT % 32 == 0 && (BN / TN) % 8 == 0 && TN == 4, "tile");
+    extern __shared__ __align__(128) float gs[];               // [ST][BM + BN][BK]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    const int ty = (warp / WN) * 4 + (lane >> 3), tx = (warp % WN) * 8 + (lane & 7);
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(gs);
+    // Where a piece of a tile row lies, in floats: rows that a warp's lanes read side by side differ in the exchange.
+    auto place = [](int row, int piece) {
+        const int x = row < BM ? row / TM : (row - BM) / 4;
+        return row * BK + ((piece ^ (x & 7)) << 2);
+    };
+
+    const int piece = tid % PIECES;                             // (NT is a multiple of the pieces of a row)
+    const float* src[NL];
 #pragma unroll
-            for (int j = 0; j < VN; ++j) {
-                if (bias && !p.bias_first) r[j] += bb[j];
-                if (p.gelu) r[j] = gelu_exact(r[j]);
-            }
-            const long long row = p.c_mode == C_HEADS ? (long long)m * p.H * p.Cp : (long long)m * p.ldc;
-            if constexpr (VN == 4) {
-                if (vec) {
-                    if (p.residual) {
-                        const float4 q = load4(static_cast<const T*>(p.residual) + (long long)m * p.ldr + n);
-                        const float rq[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) r[j] = to_f32<T>(from_f32<T>(r[j])) + rq[j];
-                    }
-                    store4(c + row + col, r);
-                    continue;
+    for (int i = 0; i < NL; ++i) {
+        const int row = (tid + i * NT) / PIECES;
+        src[i] = nullptr;
+        if (row < BM) {
+            const int m = m0 + row;
+            if (m < p.M) {
+                long long r = m;
+                if (MODE == A_TOKENS) {
+                    const int b = m / p.rows_per_batch, t = m - b * p.rows_per_batch;
+                    r = (long long)b * p.T + (p.cand ? p.cand[t] : t);
                 }
+                src[i] = static_cast<const float*>(p.a) + r * p.lda + piece * 4;
             }
-#pragma unroll
-            for (int j = 0; j < VN; ++j) {
-                if (j >= nv) continue;
-                float v = r[j];
-                const int nn = n + j, pp = nn / p.part_cols;
-                int cj = nn - pp * p.part_cols;
-                T* cc = static_cast<T*>(pp == 0 ? p.c : (pp == 1 ? p.c1 : p.c2));
-                if (p.c_mode == C_HEADS) {
-                    const int h = cj / p.dk;
-                    cj = h * p.Cp + (cj - h * p.dk);
-                }
-                if (p.residual)
-                    v = to_f32<T>(from_f32<T>(v)) + to_f32<T>(static_cast<const T*>(p.residual)[(long long)m * p.ldr + nn]);
-                cc[row + cj] = from_f32<T>(v);
-            }
+        } else if (n0 + row - BM < p.N) {
+            src[i] = static_cast<const float*>(p.w) + (long long)(n0 + row - BM) * p.ldw + piece * 4;
         }
     }
+    auto request = [&](int slot, int k0) {
+        const int left = (p.Kd - k0 - piece * 4) * 4;           // bytes of this piece inside the row; the rest is zeros
+        const int bytes = left >= 16 ? 16 : (left > 0 ? left : 0);
+#pragma unroll
+        for (int i = 0; i < NL; ++i) {
+            const int row = (tid + i * NT) / PIECES;
+            const bool on = src[i] && bytes > 0;
+            copy16(base + 4u * (uint32_t)(slot * (BM + BN) * BK + place(row, piece)), on ? src[i] + k0 : p.a, on ? bytes : 0);
+        }
+    };
+
+    float acc[TM][TN];
+    const float* bias = static_cast<const float*>(p.bias);
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+        const int n = n0 + tx * 4 + j;
+        const float init = p.bias_first && bias && n < p.N ? bias[n] : 0.f;
+#pragma unroll
+        for (int i = 0; i < TM; ++i) acc[i][j] = init;
+    }
+
+    const int steps = (p.Kd + BK - 1) / BK;
+#pragma unroll
+    for (int s = 0; s < ST - 1; ++s) {
+        if (s < steps) request(s, s * BK);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    int slot = 0, next = ST - 1;
+    for (int step = 0; step < steps; ++step) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+        __syncthreads();                                        // everyone's copies of this step; the slot of the last one is free
+        if (step + ST - 1 < steps) request(next, (step + ST - 1) * BK);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float* pa = gs + slot * (BM + BN) * BK + ty * TM * BK;
+        const float* pb = gs + slot * (BM + BN) * BK + (BM + tx * 4) * BK;
+        slot = slot + 1 == ST ? 0 : slot + 1;
+        next = next + 1 == ST ? 0 : next + 1;
+        float4 a[2][TM], b[2][TN];
+        auto read = [&](int q, int u) {
+#pragma unroll
+            for (int i = 0; i < TM; ++i) a[u][i] = *reinterpret_cast<const float4*>(pa + i * BK + ((q ^ (ty & 7)) << 2));
+#pragma unroll
+            for (int j = 0; j < TN; ++j) b[u][j] = *reinterpret_cast<const float4*>(pb + j * BK + ((q ^ (tx & 7)) << 2));
+        };
+        read(0, 0);
+#pragma unroll
+        for (int q = 0; q < PIECES; ++q) {
+            const int u = q & 1;
+            if (q + 1 < PIECES) read(q + 1, u ^ 1);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) acc[i][j] = fmaf((&a[u][i].x)[e], (&b[u][j].x)[e], acc[i][j]);
+        }
+    }
+
+    store_outputs<float, TM, 1, 4>(
+        p, n0 + tx * 4, 0, [&](int i) { return m0 + ty * TM + i; },
+        [&](int i, int, float (&r)[4]) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) r[j] = acc[i][j];
+        });
 }
 
 template <typename TA, typename T, int MODE, int BM, int BN, int BK, int TM, int TN, int MINB>
@@ -317,12 +445,67 @@ int launch_tile(const GemmParams& p, cudaStream_t st) {
     return CONVNN_OK;
 }
 
+template <int MODE, int BM, int BN, int TM, int TN, int MINB>
+int launch_copy_tile(const GemmParams& p, cudaStream_t st) {
+    const dim3 grid((p.M + BM - 1) / BM, (p.N + BN - 1) / BN);
+    const size_t smem = (size_t)4 * (BM + BN) * 32 * 4;
+    auto kern = gemm_simt_copy_kernel<MODE, BM, BN, TM, TN, MINB>;
+    CONVNN_ENSURE_SMEM(kern, smem);
+    kern<<<grid, (BM / TM) * (BN / TN), smem, st>>>(p);
+    return CONVNN_OK;
+}
+
+// float32 plain rows: the tile with the shortest time on the busiest SM, which runs `fit` tiles at a time.  `step` is
+// what a k step takes there with 1, 2, ... tiles side by side, ns: a tile of two warps leaves two of the four schedulers
+// idle, so tiles come in pairs.  Fitted to 396 shapes (65 to 25216 rows, 10 to 2304 columns, 64 to 1536 values of k; rms 3 to 7 %);
+// the choice is within 0.6 % of the best of twelve tiles on average, 12 % at worst.  With the first two tiles alone
+// (and smaller transposed ones, since gone) 2080 rows took 33.0 us at 192 x 768, now 25.8; 20.6 at 576 x 192, now 17.8;
+// 1576 x 384 x 192 15.5, now 11.5; 1050 x 384 x 384 18.7, now 15.6.
+template <int MODE>
+int launch_plain_f32(const GemmParams& p, cudaStream_t st) {
+    struct Tile {
+        int bm, bn, fit;
+        double launch, round, step[6];        // us per launch and per round of tiles
+    };
+    static const Tile tiles[6] = {
+        {128, 64, 3, 5.4, 0.5, {65.4, 107.1, 153.3}},
+        {64, 64, 3, 3.2, 0.7, {38.2, 62.3, 88.9}},
+        {32, 32, 6, 1.7, 1.5, {19.6, 20.9, 33.3, 35.3, 51.4, 48.7}},
+        {40, 32, 6, 2.2, 1.6, {23.5, 25.2, 38.8, 39.7, 61.1, 58.2}},
+        {48, 32, 5, 2.2, 2.3, {26.3, 28.8, 42.9, 46.8, 60.0}},
+        {56, 32, 5, 1.9, 3.1, {30.2, 32.5, 50.4, 53.8, 72.0}},
+    };
+    const long long sms = device_sms();
+    int best = 0;
+    double least = 0;
+    for (int i = 0; i < 6; ++i) {
+        const Tile& t = tiles[i];
+        if (i > 1 && (p.N + t.bn - 1) / t.bn > 65535) continue;      // (grid rows)
+        const long long n = (long long)((p.M + t.bm - 1) / t.bm) * ((p.N + t.bn - 1) / t.bn), per_sm = (n + sms - 1) / sms;
+        const long long full = per_sm / t.fit, rest = per_sm % t.fit;
+        double cost = t.launch + (full + (rest ? 1 : 0)) * t.round + 1e-3 * p.Kd * full * t.step[t.fit - 1];
+        if (rest) cost += 1e-3 * p.Kd * t.step[rest - 1];
+        if (i == 0 || cost < least) { least = cost; best = i; }
+    }
+    switch (best) {
+        case 0: return launch_tile<float, float, MODE, 128, 64, 16, 8, 8, 3>(p, st);
+        case 1: return launch_tile<float, float, MODE, 64, 64, 32, 8, 4, 3>(p, st);
+        case 2: return launch_copy_tile<MODE, 32, 32, 4, 4, 6>(p, st);
+        case 3: return launch_copy_tile<MODE, 40, 32, 5, 4, 6>(p, st);
+        case 4: return launch_copy_tile<MODE, 48, 32, 6, 4, 5>(p, st);
+        default: return launch_copy_tile<MODE, 56, 32, 7, 4, 5>(p, st);
+    }
+}
+
 template <typename TA, typename T, int MODE>
 int launch_mode(const GemmParams& p, cudaStream_t st) {
     // The tile with the least work on the busiest SM: rounds of tiles x outputs per tile over the rate of the tile's
     // threads.  That rate is set by shared memory: a k step reads TM + TN values per thread for TM * TN multiply-adds
     // (45, 40, 29 and 26 TFLOP/s at 16384 x 768 x 768; 25 before).  2080 x 192 x 768: 33 us, 50 before; 50432 x 192 x
     // 192: 89 us, 150 before.
+    if constexpr (sizeof(TA) == 4 && sizeof(T) == 4 && (MODE == A_ROWS || MODE == A_TOKENS)) {
+        if (p.a_vec && p.w_vec) return launch_plain_f32<MODE>(p, st);
+    }
     const long long sms = device_sms();
     long long tiles_of[4];
     auto cost = [&](int i, int bm, int bn, double rate) {

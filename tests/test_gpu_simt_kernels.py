@@ -236,3 +236,36 @@ def test_statistics_of_all_tensors_in_one_launch(B, T, S, H, dk, coord, dtype, m
         want = 1 / want.sqrt().clamp_min(1e-12) if metric == "cosine" else want
         # a C-term fp32 sum of squares, a root and a division
         assert bool(((stat.view(B, H, rows).double() - want).abs() <= (C + 8) * EPS * want.abs() + 1e-30).all())
+
+
+# Every tile of the float32 rows (columns of a tile x outputs per thread; "transposed": those that are), with ragged rows,
+# columns and k; a sum is the same whichever tile it was computed in.
+@on_148_sms
+@pytest.mark.parametrize("M,N,K,tile", [
+    (2081, 190, 100, "32x32 4x4"), (1, 1, 4, "32x32 4x4"), (33, 65, 768, "32x32 4x4"), (3121, 190, 764, "32x32 4x4"),
+    (5003, 193, 36, "40x32 5x4"), (1576, 385, 100, "40x32 5x4"), (1001, 1003, 192, "40x32 5x4"), (2081, 190, 768, "48x32 6x4"),
+    (1050, 383, 388, "48x32 6x4"), (5203, 190, 768, "56x32 7x4"), (2081, 577, 32, "transposed"), (50432, 190, 8, "transposed")])
+def test_tiles_of_float32_rows(M, N, K, tile):
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    a, w, b, r = (torch.randn(*s, device=DEV, generator=g) for s in ((M, K + 4), (N, K), (N,), (M, N)))
+    a = a[:, :K]                                                     # rows K + 4 values apart
+    call = lambda: ops.linear(a, w, b, residual=r)
+    names = [re.search(r"gemm_simt_copy_kernelILi\dELi(\d+)ELi(\d+)ELi(\d+)ELi(\d+)E", n) for n in launches(call)]
+    assert [("{}x{} {}x{}".format(*m.groups()) if m else "transposed") for m in names] == [tile]
+    got = call()
+    want = a.double() @ w.double().T + b.double() + r.double()
+    assert bool(((got.double() - want).abs() <= _bound(a, w, K) + 4 * EPS * (b.abs() + r.abs() + want.abs())).all())
+    some = torch.randperm(M, device=DEV, generator=g)[:20]
+    assert torch.equal(ops.linear(a[some], w, b, residual=r[some]), got[some])
+
+
+@pytest.mark.parametrize("B,T,S,D,H", [(8, 197, 49, 192, 3), (2, 50, 50, 96, 1), (33, 65, 65, 192, 1)])
+def test_three_outputs_of_float32_rows(B, T, S, D, H):
+    g = torch.Generator(device=DEV).manual_seed(T)
+    spec = ops.LayerSpec(D, H, 9, "all" if S == T else "spatial", "matmul", "depthwise", True, False, T)
+    x, w = torch.randn(B, T, D, device=DEV, generator=g), torch.randn(3, D, D, device=DEV, generator=g)
+    cand = None if S == T else torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32)
+    q, k, v = ops.qkv_proj(spec, x, w, cand)[:3]
+    xq = x if cand is None else x[:, cand.long()]
+    for got, rows, part in ((k, x, 0), (v, x, 1), (q, xq, 2)):
+        assert torch.equal(got.reshape(-1, D), ops.linear(rows.reshape(-1, D), w[part]))
