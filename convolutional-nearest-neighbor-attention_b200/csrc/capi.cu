@@ -280,7 +280,7 @@ bool qkv_fold_supported(const convnn_desc* d, const Dims& dm) {
 
 int qkv_proj_impl(const convnn_desc* d, const void* x, int64_t ldx, const void* w_qkv,
                   const int32_t* cand, void* q, void* k, void* v, float* qstat, float* kstat,
-                  void* scratch, void* stream, const PreNorm* pn) {
+                  void* scratch, void* stream, const PreNorm* pn, bool at_rest) {
     Dims dm;
     int rc = validate(d, &dm);
     if (rc) return rc;
@@ -309,7 +309,7 @@ int qkv_proj_impl(const convnn_desc* d, const void* x, int64_t ldx, const void* 
         float* sc_k = pieces > 1 && fuse ? reinterpret_cast<float*>(static_cast<char*>(scratch) + gathered) : nullptr;
         float* sc_q = sc_k ? reinterpret_cast<float*>(static_cast<char*>(scratch) + gathered + part_k) : nullptr;
         GemmTcOpts o;
-        o.stat_mode = d->metric; o.dk = dm.dk; o.heads = dm.H;
+        o.stat_mode = d->metric; o.dk = dm.dk; o.heads = dm.H; o.w_at_rest = at_rest;
         bool done = false;
         if (pn) {
             if (!qkv_fold_supported(d, dm) || !gemm_tc_supported(x, ldx, w_qkv, dm.D, 3 * dm.D, 3, kvq, dm.D))
@@ -327,7 +327,7 @@ int qkv_proj_impl(const convnn_desc* d, const void* x, int64_t ldx, const void* 
             if ((rc = launch_gemm_tc(x, ldx, w_qkv, dm.B * dm.T, 2 * dm.D, dm.D, 2, kvq, dm.D, o, st))) return rc;
             if ((rc = launch_gather_rows(d->dtype, x, ldx, cand, scratch, dm.B, dm.T, dm.S, dm.D, st))) return rc;
             GemmTcOpts oq;
-            oq.stat_mode = d->metric; oq.dk = dm.dk; oq.heads = dm.H;
+            oq.stat_mode = d->metric; oq.dk = dm.dk; oq.heads = dm.H; oq.w_at_rest = true;
             if (fuse) { oq.stat[0] = qstat; oq.rows_per_batch = dm.S; oq.stat_scratch = sc_q; }
             if ((rc = launch_gemm_tc(scratch, dm.D, wb + 2 * wsz, dm.B * dm.S, dm.D, dm.D, 1, &kvq[2], dm.D, oq, st)))
                 return rc;
@@ -361,7 +361,7 @@ extern "C" {
 int convnn_b200_qkv_proj(const convnn_desc* d, const void* x, int64_t ldx, const void* w_qkv,
                          const int32_t* cand, void* q, void* k, void* v, float* qstat, float* kstat,
                          void* scratch, void* stream) {
-    return qkv_proj_impl(d, x, ldx, w_qkv, cand, q, k, v, qstat, kstat, scratch, stream, nullptr);
+    return qkv_proj_impl(d, x, ldx, w_qkv, cand, q, k, v, qstat, kstat, scratch, stream, nullptr, false);
 }
 
 int convnn_b200_sim_topk(const convnn_desc* d, const void* q, const void* k, const float* qstat,
@@ -415,7 +415,7 @@ int select_and_conv(const convnn_desc* d, const Dims& dm, const Workspace& w, co
 
 // merged: o is (B, T, D), heads in the flat reinterpretation.
 int out_proj_impl(const convnn_desc* d, const void* o, const void* w_o, const void* residual, int64_t ldr,
-                  void* out, int64_t ldo, void* scratch, void* stream, float* moments_out, bool merged) {
+                  void* out, int64_t ldo, void* scratch, void* stream, float* moments_out, bool merged, bool at_rest) {
     Dims dm;
     int rc = validate(d, &dm);
     if (rc) return rc;
@@ -427,12 +427,13 @@ int out_proj_impl(const convnn_desc* d, const void* o, const void* w_o, const vo
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         void* cs[1] = {out};
         GemmTcOpts go;
-        go.residual = residual; go.ldr = ldr; go.moments_out = moments_out;
+        go.residual = residual; go.ldr = ldr; go.moments_out = moments_out; go.w_at_rest = at_rest;
         const bool res_ok = !residual || (ldr % 8 == 0 && aligned16(residual));
         if (res_ok && (dm.H == 1 || merged) && gemm_tc_supported(o, dm.D, w_o, dm.D, dm.D, 1, cs, ldo))
             return launch_gemm_tc(o, dm.D, w_o, dm.B * dm.T, dm.D, dm.D, 1, cs, ldo, go, st);
         if (res_ok && dm.H > 1 && !merged && scratch && gemm_tc_supported(scratch, dm.D, w_o, dm.D, dm.D, 1, cs, ldo)) {
             if ((rc = launch_merge_heads(d->dtype, o, scratch, dm.B, dm.T, dm.H, dm.dk, st))) return rc;
+            go.w_at_rest = true;
             return launch_gemm_tc(scratch, dm.D, w_o, dm.B * dm.T, dm.D, dm.D, 1, cs, ldo, go, st);
         }
     }
@@ -455,25 +456,14 @@ extern "C" {
 
 int convnn_b200_out_proj(const convnn_desc* d, const void* o, const void* w_o, const void* residual, int64_t ldr,
                          void* out, int64_t ldo, void* scratch, void* stream) {
-    return out_proj_impl(d, o, w_o, residual, ldr, out, ldo, scratch, stream, nullptr, false);
+    return out_proj_impl(d, o, w_o, residual, ldr, out, ldo, scratch, stream, nullptr, false, false);
 }
 
 int convnn_b200_forward(const convnn_desc* d, const void* x, int64_t ldx, const void* w_qkv,
                         const void* w_conv, const void* w_pw, const void* w_o, const int32_t* cand,
                         const void* residual, int64_t ldr, void* out, int64_t ldo, void* workspace,
                         size_t workspace_bytes, void* stream) {
-    Dims dm;
-    int rc = validate(d, &dm);
-    if (rc) return rc;
-    REQUIRE_PTR(workspace);
-    if (!aligned16(workspace)) return set_error(CONVNN_E_ALIGN, "workspace must be 16-byte aligned");
-    Workspace w = carve(dm, d->conv_type, workspace);
-    if (workspace_bytes < w.total)
-        return set_error(CONVNN_E_WORKSPACE, "workspace has %zu bytes, %zu needed", workspace_bytes, w.total);
-    if ((rc = convnn_b200_qkv_proj(d, x, ldx, w_qkv, cand, w.q, w.k, w.v, w.qstat, w.kstat, w.scratch, stream))) return rc;
-    bool merged;
-    if ((rc = select_and_conv(d, dm, w, cand, w_conv, w_pw, w.o, &merged, stream))) return rc;
-    return out_proj_impl(d, w.o, w_o, residual, ldr, out, ldo, w.scratch, stream, nullptr, merged);
+    return layer_forward(d, x, ldx, w_qkv, w_conv, w_pw, w_o, cand, residual, ldr, out, ldo, workspace, workspace_bytes, false, stream);
 }
 
 int convnn_b200_layernorm(int dtype, const void* x, int64_t ldx, const void* gamma, const void* beta, float eps,
@@ -531,29 +521,7 @@ int convnn_b200_patchify_u8(int dtype, const uint8_t* img, const float* mean, co
 int convnn_b200_linear(int dtype, const void* a, int64_t lda, const void* w, const void* bias, const void* residual,
                        int64_t ldr, void* out, int64_t ldo, int64_t M, int32_t N, int32_t K, int32_t gelu,
                        void* stream) {
-    if (dtype != CONVNN_F32 && dtype != CONVNN_BF16) return set_error(CONVNN_E_INVALID, "unknown dtype %d", dtype);
-    REQUIRE_PTR(a); REQUIRE_PTR(w); REQUIRE_PTR(out);
-    if (M < 0 || N < 1 || K < 1 || lda < K || ldo < N || (residual && ldr < N) || M >= (1ll << 31))
-        return set_error(CONVNN_E_INVALID, "linear: bad shape (M=%lld N=%d K=%d)", (long long)M, N, K);
-    int rc = check_device();
-    if (rc) return rc;
-    if (M == 0) return CONVNN_OK;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (dtype == CONVNN_BF16 && !force_simt()) {
-        void* cs[1] = {out};
-        const bool extra_ok = (!bias || aligned16(bias)) && (!residual || (aligned16(residual) && ldr % 8 == 0));
-        if (extra_ok && gemm_tc_supported(a, lda, w, K, N, 1, cs, ldo)) {
-            GemmTcOpts o;
-            o.bias = bias; o.residual = residual; o.ldr = ldr; o.gelu = gelu;
-            return launch_gemm_tc(a, lda, w, (int)M, N, K, 1, cs, ldo, o, st);
-        }
-    }
-    GemmParams p{};
-    p.a = a; p.w = w; p.bias = bias; p.c = out; p.cand = nullptr;
-    p.lda = lda; p.ldc = ldo; p.M = (int)M; p.N = N; p.Kd = K;
-    p.a_mode = A_ROWS; p.c_mode = C_ROWS; p.rows_per_batch = 1; p.T = 1; p.H = 1; p.dk = N; p.Cp = N;
-    p.gelu = gelu; p.residual = residual; p.ldr = ldr;
-    return launch_gemm_simt(dtype, p, st);
+    return linear(dtype, a, lda, w, bias, residual, ldr, out, ldo, M, N, K, gelu, false, stream);
 }
 
 // ---- LayerNorm folded into the GEMM that consumes it ----------------------------------------------
@@ -592,40 +560,13 @@ int convnn_b200_fold_layernorm(const void* w, const void* bias, const void* gamm
 int convnn_b200_prenorm_linear(const void* a, int64_t lda, const float* moments, int32_t planes, float eps,
                                const void* w_folded, const void* w_extra, void* out, int64_t ldo, int64_t M,
                                int32_t N, int32_t K, int32_t gelu, void* stream) {
-    REQUIRE_PTR(a); REQUIRE_PTR(moments); REQUIRE_PTR(w_folded); REQUIRE_PTR(w_extra); REQUIRE_PTR(out);
-    if (M < 0 || N < 1 || K < 1 || lda < K || ldo < N || planes < 1 || M >= (1ll << 31))
-        return set_error(CONVNN_E_INVALID, "prenorm_linear: bad shape (M=%lld N=%d K=%d planes=%d)", (long long)M, N, K, planes);
-    int rc = check_device();
-    if (rc) return rc;
-    if (M == 0) return CONVNN_OK;
-    void* cs[1] = {out};
-    if (force_simt() || !gemm_tc_supported(a, lda, w_folded, K, N, 1, cs, ldo) ||
-        !gemm_tc_prenorm_supported(N, K, 1, false, gelu != 0))
-        return set_error(CONVNN_E_UNSUPPORTED, "prenorm_linear: N=%d K=%d takes the unfused path "
-                                               "(see convnn_b200_prenorm_linear_supported)", N, K);
-    GemmTcOpts o;
-    o.gelu = gelu;
-    o.ln_moments = moments; o.ln_planes = planes; o.ln_eps = eps; o.ln_wextra = w_extra;
-    return launch_gemm_tc(a, lda, w_folded, (int)M, N, K, 1, cs, ldo, o, static_cast<cudaStream_t>(stream));
+    return prenorm_linear(a, lda, moments, planes, eps, w_folded, w_extra, out, ldo, M, N, K, gelu, false, stream);
 }
 
 int convnn_b200_linear_moments(const void* a, int64_t lda, const void* w, const void* bias, const void* residual,
                                int64_t ldr, void* out, int64_t ldo, int64_t M, int32_t N, int32_t K,
                                float* moments_out, void* stream) {
-    REQUIRE_PTR(a); REQUIRE_PTR(w); REQUIRE_PTR(residual); REQUIRE_PTR(out); REQUIRE_PTR(moments_out);
-    if (M < 0 || N < 1 || K < 1 || lda < K || ldo < N || ldr < N || M >= (1ll << 31))
-        return set_error(CONVNN_E_INVALID, "linear_moments: bad shape (M=%lld N=%d K=%d)", (long long)M, N, K);
-    int rc = check_device();
-    if (rc) return rc;
-    if (M == 0) return CONVNN_OK;
-    void* cs[1] = {out};
-    const bool extra_ok = (!bias || aligned16(bias)) && aligned16(residual) && ldr % 8 == 0 &&
-                          (reinterpret_cast<uintptr_t>(moments_out) & 7u) == 0;
-    if (force_simt() || !extra_ok || !gemm_tc_supported(a, lda, w, K, N, 1, cs, ldo))
-        return set_error(CONVNN_E_UNSUPPORTED, "linear_moments: needs the bfloat16 tensor-core path");
-    GemmTcOpts o;
-    o.bias = bias; o.residual = residual; o.ldr = ldr; o.moments_out = moments_out;
-    return launch_gemm_tc(a, lda, w, (int)M, N, K, 1, cs, ldo, o, static_cast<cudaStream_t>(stream));
+    return linear_moments(a, lda, w, bias, residual, ldr, out, ldo, M, N, K, moments_out, false, stream);
 }
 
 int convnn_b200_prenorm_forward(const convnn_desc* d, const void* x, int64_t ldx, const float* moments,
@@ -633,26 +574,8 @@ int convnn_b200_prenorm_forward(const convnn_desc* d, const void* x, int64_t ldx
                                 const void* w_conv, const void* w_pw, const void* w_o, const void* residual,
                                 int64_t ldr, void* out, int64_t ldo, float* moments_out, void* workspace,
                                 size_t workspace_bytes, void* stream) {
-    Dims dm;
-    int rc = validate(d, &dm);
-    if (rc) return rc;
-    REQUIRE_PTR(workspace); REQUIRE_PTR(moments); REQUIRE_PTR(w_qkv_extra);
-    if (planes < 1) return set_error(CONVNN_E_INVALID, "prenorm_forward: planes must be positive");
-    if (moments_out && !residual)
-        return set_error(CONVNN_E_UNSUPPORTED, "prenorm_forward: row moments come with the skip connection");
-    if (!aligned16(workspace)) return set_error(CONVNN_E_ALIGN, "workspace must be 16-byte aligned");
-    Workspace w = carve(dm, d->conv_type, workspace);
-    if (workspace_bytes < w.total)
-        return set_error(CONVNN_E_WORKSPACE, "workspace has %zu bytes, %zu needed", workspace_bytes, w.total);
-    if (!w_o && (dm.H != 1 || ldo != dm.D || residual || moments_out))
-        return set_error(CONVNN_E_INVALID, "prenorm_forward: without w_o the layer's pre-projection output is written to a "
-                                           "contiguous `out` (num_heads = 1, ldo = D, no residual, no moments)");
-    const PreNorm pn{moments, planes, eps, w_qkv_extra};
-    if ((rc = qkv_proj_impl(d, x, ldx, w_qkv_folded, nullptr, w.q, w.k, w.v, w.qstat, w.kstat, w.scratch, stream, &pn))) return rc;
-    // (without w_o the caller fuses the output projection into what follows: convnn_b200_outproj_mlp)
-    bool merged;
-    if ((rc = select_and_conv(d, dm, w, nullptr, w_conv, w_pw, w_o ? w.o : out, &merged, stream)) || !w_o) return rc;
-    return out_proj_impl(d, w.o, w_o, residual, ldr, out, ldo, w.scratch, stream, moments_out, merged);
+    return prenorm_forward(d, x, ldx, moments, planes, eps, w_qkv_folded, w_qkv_extra, w_conv, w_pw, w_o, residual, ldr, out,
+                           ldo, moments_out, workspace, workspace_bytes, false, stream);
 }
 
 int convnn_b200_prenorm_mlp_supported(int32_t D, int32_t DM, int32_t planes) {
@@ -664,15 +587,7 @@ int convnn_b200_prenorm_mlp_moment_planes(void) { return mlp_tc_moment_planes();
 int convnn_b200_prenorm_mlp(const void* x, int64_t ldx, const float* moments, int32_t planes, float eps,
                             const void* w1_folded, const void* w1_extra, const void* w2, const void* b2, void* out,
                             int64_t ldo, int64_t M, int32_t D, int32_t DM, float* moments_out, void* stream) {
-    REQUIRE_PTR(x); REQUIRE_PTR(moments); REQUIRE_PTR(w1_folded); REQUIRE_PTR(w1_extra); REQUIRE_PTR(w2); REQUIRE_PTR(out);
-    if (M < 0 || D < 1 || DM < 1 || ldx < D || ldo < D || planes < 1 || M >= (1ll << 31))
-        return set_error(CONVNN_E_INVALID, "prenorm_mlp: bad shape (M=%lld D=%d d_mlp=%d planes=%d)", (long long)M, D, DM, planes);
-    int rc = check_device();
-    if (rc) return rc;
-    if (M == 0) return CONVNN_OK;
-    if (force_simt()) return set_error(CONVNN_E_UNSUPPORTED, "prenorm_mlp: needs the tensor-core path");
-    return launch_mlp_tc(x, ldx, moments, planes, eps, w1_folded, w1_extra, w2, b2, out, ldo, (int)M, D, DM, moments_out,
-                         nullptr, nullptr, 0, static_cast<cudaStream_t>(stream));
+    return prenorm_mlp(x, ldx, moments, planes, eps, w1_folded, w1_extra, w2, b2, out, ldo, M, D, DM, moments_out, false, stream);
 }
 
 int convnn_b200_outproj_mlp(const void* o, int64_t ld_o, const void* w_o, const void* x, int64_t ldx, float eps,
@@ -687,7 +602,7 @@ int convnn_b200_outproj_mlp(const void* o, int64_t ld_o, const void* w_o, const 
     if (M == 0) return CONVNN_OK;
     if (force_simt()) return set_error(CONVNN_E_UNSUPPORTED, "outproj_mlp: needs the tensor-core path");
     return launch_mlp_tc(o, ld_o, nullptr, 1, eps, w1_folded, w1_extra, w2, b2, out, ldo, (int)M, D, DM, moments_out, w_o, x,
-                         ldx, static_cast<cudaStream_t>(stream));
+                         ldx, false, static_cast<cudaStream_t>(stream));
 }
 
 // ---- the other halves of the branching wrappers ------------------------------------------------
@@ -709,6 +624,157 @@ size_t convnn_b200_attention_workspace_bytes(int dtype, int32_t B, int32_t T, in
 int convnn_b200_softmax_attention(int dtype, const void* x, int64_t ldx, const void* w_qkv, const void* w_o, void* out,
                                   int64_t ldo, int32_t B, int32_t T, int32_t D, int32_t H, void* workspace,
                                   size_t workspace_bytes, void* stream) {
+    return softmax_attention(dtype, x, ldx, w_qkv, w_o, out, ldo, B, T, D, H, workspace, workspace_bytes, false, stream);
+}
+
+size_t convnn_b200_conv1d_attention_workspace_bytes(int dtype, int32_t B, int32_t T, int32_t D, int32_t kernel_size) {
+    if ((dtype != CONVNN_F32 && dtype != CONVNN_BF16) || B < 1 || T < 1 || D < 1 || kernel_size < 1) return 0;
+    const size_t elt = dtype == CONVNN_F32 ? 4 : 2, part = up256((size_t)B * T * D * elt);
+    // (the unfolded operand also for shapes that only unfold where the taps are unaligned)
+    return 3 * part + up256((size_t)B * T * D * kernel_size * elt);
+}
+
+int convnn_b200_conv1d_attention(int dtype, const void* x, int64_t ldx, const void* w_x, const void* b_x,
+                                 const void* w_conv, const void* b_conv, const void* w_o, const void* b_o, void* out,
+                                 int64_t ldo, int32_t B, int32_t T, int32_t D, int32_t H, int32_t kernel_size,
+                                 void* workspace, size_t workspace_bytes, void* stream) {
+    return conv1d_attention(dtype, x, ldx, w_x, b_x, w_conv, b_conv, w_o, b_o, out, ldo, B, T, D, H, kernel_size, workspace, workspace_bytes, false,
+                            stream);
+}
+
+}  // extern "C"
+
+// ---- the entry points above; at_rest: the call's first weights may be read before the previous launch has ended ----
+
+int convnn::prenorm_forward(const convnn_desc* d, const void* x, int64_t ldx, const float* moments,
+                                int32_t planes, float eps, const void* w_qkv_folded, const void* w_qkv_extra,
+                                const void* w_conv, const void* w_pw, const void* w_o, const void* residual,
+                                int64_t ldr, void* out, int64_t ldo, float* moments_out, void* workspace,
+                                size_t workspace_bytes, bool at_rest, void* stream) {
+    Dims dm;
+    int rc = validate(d, &dm);
+    if (rc) return rc;
+    REQUIRE_PTR(workspace); REQUIRE_PTR(moments); REQUIRE_PTR(w_qkv_extra);
+    if (planes < 1) return set_error(CONVNN_E_INVALID, "prenorm_forward: planes must be positive");
+    if (moments_out && !residual)
+        return set_error(CONVNN_E_UNSUPPORTED, "prenorm_forward: row moments come with the skip connection");
+    if (!aligned16(workspace)) return set_error(CONVNN_E_ALIGN, "workspace must be 16-byte aligned");
+    Workspace w = carve(dm, d->conv_type, workspace);
+    if (workspace_bytes < w.total)
+        return set_error(CONVNN_E_WORKSPACE, "workspace has %zu bytes, %zu needed", workspace_bytes, w.total);
+    if (!w_o && (dm.H != 1 || ldo != dm.D || residual || moments_out))
+        return set_error(CONVNN_E_INVALID, "prenorm_forward: without w_o the layer's pre-projection output is written to a "
+                                           "contiguous `out` (num_heads = 1, ldo = D, no residual, no moments)");
+    const PreNorm pn{moments, planes, eps, w_qkv_extra};
+    if ((rc = qkv_proj_impl(d, x, ldx, w_qkv_folded, nullptr, w.q, w.k, w.v, w.qstat, w.kstat, w.scratch, stream, &pn, at_rest))) return rc;
+    // (without w_o the caller fuses the output projection into what follows: convnn_b200_outproj_mlp)
+    bool merged;
+    if ((rc = select_and_conv(d, dm, w, nullptr, w_conv, w_pw, w_o ? w.o : out, &merged, stream)) || !w_o) return rc;
+    return out_proj_impl(d, w.o, w_o, residual, ldr, out, ldo, w.scratch, stream, moments_out, merged, true);
+}
+
+int convnn::prenorm_mlp(const void* x, int64_t ldx, const float* moments, int32_t planes, float eps,
+                            const void* w1_folded, const void* w1_extra, const void* w2, const void* b2, void* out,
+                            int64_t ldo, int64_t M, int32_t D, int32_t DM, float* moments_out, bool at_rest, void* stream) {
+    REQUIRE_PTR(x); REQUIRE_PTR(moments); REQUIRE_PTR(w1_folded); REQUIRE_PTR(w1_extra); REQUIRE_PTR(w2); REQUIRE_PTR(out);
+    if (M < 0 || D < 1 || DM < 1 || ldx < D || ldo < D || planes < 1 || M >= (1ll << 31))
+        return set_error(CONVNN_E_INVALID, "prenorm_mlp: bad shape (M=%lld D=%d d_mlp=%d planes=%d)", (long long)M, D, DM, planes);
+    int rc = check_device();
+    if (rc) return rc;
+    if (M == 0) return CONVNN_OK;
+    if (force_simt()) return set_error(CONVNN_E_UNSUPPORTED, "prenorm_mlp: needs the tensor-core path");
+    return launch_mlp_tc(x, ldx, moments, planes, eps, w1_folded, w1_extra, w2, b2, out, ldo, (int)M, D, DM, moments_out,
+                         nullptr, nullptr, 0, at_rest, static_cast<cudaStream_t>(stream));
+}
+
+int convnn::layer_forward(const convnn_desc* d, const void* x, int64_t ldx, const void* w_qkv,
+                        const void* w_conv, const void* w_pw, const void* w_o, const int32_t* cand,
+                        const void* residual, int64_t ldr, void* out, int64_t ldo, void* workspace,
+                        size_t workspace_bytes, bool at_rest, void* stream) {
+    Dims dm;
+    int rc = validate(d, &dm);
+    if (rc) return rc;
+    REQUIRE_PTR(workspace);
+    if (!aligned16(workspace)) return set_error(CONVNN_E_ALIGN, "workspace must be 16-byte aligned");
+    Workspace w = carve(dm, d->conv_type, workspace);
+    if (workspace_bytes < w.total)
+        return set_error(CONVNN_E_WORKSPACE, "workspace has %zu bytes, %zu needed", workspace_bytes, w.total);
+    if ((rc = qkv_proj_impl(d, x, ldx, w_qkv, cand, w.q, w.k, w.v, w.qstat, w.kstat, w.scratch, stream, nullptr, at_rest))) return rc;
+    bool merged;
+    if ((rc = select_and_conv(d, dm, w, cand, w_conv, w_pw, w.o, &merged, stream))) return rc;
+    return out_proj_impl(d, w.o, w_o, residual, ldr, out, ldo, w.scratch, stream, nullptr, merged, true);
+}
+
+int convnn::linear(int dtype, const void* a, int64_t lda, const void* w, const void* bias, const void* residual,
+                       int64_t ldr, void* out, int64_t ldo, int64_t M, int32_t N, int32_t K, int32_t gelu,
+                       bool at_rest, void* stream) {
+    if (dtype != CONVNN_F32 && dtype != CONVNN_BF16) return set_error(CONVNN_E_INVALID, "unknown dtype %d", dtype);
+    REQUIRE_PTR(a); REQUIRE_PTR(w); REQUIRE_PTR(out);
+    if (M < 0 || N < 1 || K < 1 || lda < K || ldo < N || (residual && ldr < N) || M >= (1ll << 31))
+        return set_error(CONVNN_E_INVALID, "linear: bad shape (M=%lld N=%d K=%d)", (long long)M, N, K);
+    int rc = check_device();
+    if (rc) return rc;
+    if (M == 0) return CONVNN_OK;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (dtype == CONVNN_BF16 && !force_simt()) {
+        void* cs[1] = {out};
+        const bool extra_ok = (!bias || aligned16(bias)) && (!residual || (aligned16(residual) && ldr % 8 == 0));
+        if (extra_ok && gemm_tc_supported(a, lda, w, K, N, 1, cs, ldo)) {
+            GemmTcOpts o;
+            o.bias = bias; o.residual = residual; o.ldr = ldr; o.gelu = gelu; o.w_at_rest = at_rest;
+            return launch_gemm_tc(a, lda, w, (int)M, N, K, 1, cs, ldo, o, st);
+        }
+    }
+    GemmParams p{};
+    p.a = a; p.w = w; p.bias = bias; p.c = out; p.cand = nullptr;
+    p.lda = lda; p.ldc = ldo; p.M = (int)M; p.N = N; p.Kd = K;
+    p.a_mode = A_ROWS; p.c_mode = C_ROWS; p.rows_per_batch = 1; p.T = 1; p.H = 1; p.dk = N; p.Cp = N;
+    p.gelu = gelu; p.residual = residual; p.ldr = ldr;
+    return launch_gemm_simt(dtype, p, st);
+}
+
+int convnn::prenorm_linear(const void* a, int64_t lda, const float* moments, int32_t planes, float eps,
+                               const void* w_folded, const void* w_extra, void* out, int64_t ldo, int64_t M,
+                               int32_t N, int32_t K, int32_t gelu, bool at_rest, void* stream) {
+    REQUIRE_PTR(a); REQUIRE_PTR(moments); REQUIRE_PTR(w_folded); REQUIRE_PTR(w_extra); REQUIRE_PTR(out);
+    if (M < 0 || N < 1 || K < 1 || lda < K || ldo < N || planes < 1 || M >= (1ll << 31))
+        return set_error(CONVNN_E_INVALID, "prenorm_linear: bad shape (M=%lld N=%d K=%d planes=%d)", (long long)M, N, K, planes);
+    int rc = check_device();
+    if (rc) return rc;
+    if (M == 0) return CONVNN_OK;
+    void* cs[1] = {out};
+    if (force_simt() || !gemm_tc_supported(a, lda, w_folded, K, N, 1, cs, ldo) ||
+        !gemm_tc_prenorm_supported(N, K, 1, false, gelu != 0))
+        return set_error(CONVNN_E_UNSUPPORTED, "prenorm_linear: N=%d K=%d takes the unfused path "
+                                               "(see convnn_b200_prenorm_linear_supported)", N, K);
+    GemmTcOpts o;
+    o.gelu = gelu; o.w_at_rest = at_rest;
+    o.ln_moments = moments; o.ln_planes = planes; o.ln_eps = eps; o.ln_wextra = w_extra;
+    return launch_gemm_tc(a, lda, w_folded, (int)M, N, K, 1, cs, ldo, o, static_cast<cudaStream_t>(stream));
+}
+
+int convnn::linear_moments(const void* a, int64_t lda, const void* w, const void* bias, const void* residual,
+                               int64_t ldr, void* out, int64_t ldo, int64_t M, int32_t N, int32_t K,
+                               float* moments_out, bool at_rest, void* stream) {
+    REQUIRE_PTR(a); REQUIRE_PTR(w); REQUIRE_PTR(residual); REQUIRE_PTR(out); REQUIRE_PTR(moments_out);
+    if (M < 0 || N < 1 || K < 1 || lda < K || ldo < N || ldr < N || M >= (1ll << 31))
+        return set_error(CONVNN_E_INVALID, "linear_moments: bad shape (M=%lld N=%d K=%d)", (long long)M, N, K);
+    int rc = check_device();
+    if (rc) return rc;
+    if (M == 0) return CONVNN_OK;
+    void* cs[1] = {out};
+    const bool extra_ok = (!bias || aligned16(bias)) && aligned16(residual) && ldr % 8 == 0 &&
+                          (reinterpret_cast<uintptr_t>(moments_out) & 7u) == 0;
+    if (force_simt() || !extra_ok || !gemm_tc_supported(a, lda, w, K, N, 1, cs, ldo))
+        return set_error(CONVNN_E_UNSUPPORTED, "linear_moments: needs the bfloat16 tensor-core path");
+    GemmTcOpts o;
+    o.bias = bias; o.residual = residual; o.ldr = ldr; o.moments_out = moments_out; o.w_at_rest = at_rest;
+    return launch_gemm_tc(a, lda, w, (int)M, N, K, 1, cs, ldo, o, static_cast<cudaStream_t>(stream));
+}
+
+int convnn::softmax_attention(int dtype, const void* x, int64_t ldx, const void* w_qkv, const void* w_o, void* out,
+                                  int64_t ldo, int32_t B, int32_t T, int32_t D, int32_t H, void* workspace,
+                                  size_t workspace_bytes, bool at_rest, void* stream) {
     int rc = branch_args_ok("softmax_attention", dtype, B, T, D, H, ldx, ldo);
     if (rc) return rc;
     REQUIRE_PTR(x); REQUIRE_PTR(w_qkv); REQUIRE_PTR(w_o); REQUIRE_PTR(out); REQUIRE_PTR(workspace);
@@ -726,6 +792,7 @@ int convnn_b200_softmax_attention(int dtype, const void* x, int64_t ldx, const v
     // q, k, v: one launch over the packed weight where the tensor-core GEMM takes the shape
     if (dtype == CONVNN_BF16 && !force_simt() && gemm_tc_supported(x, ldx, w_qkv, D, 3 * D, 3, qkv, D)) {
         GemmTcOpts go;
+        go.w_at_rest = at_rest;
         if ((rc = launch_gemm_tc(x, ldx, w_qkv, (int)M, 3 * D, D, 3, qkv, D, go, st))) return rc;
     } else {
         for (int i = 0; i < 3; ++i)
@@ -734,20 +801,13 @@ int convnn_b200_softmax_attention(int dtype, const void* x, int64_t ldx, const v
                 return rc;
     }
     if ((rc = launch_attention(dtype, qkv[0], qkv[1], qkv[2], o, B, T, D, H, st))) return rc;
-    return convnn_b200_linear(dtype, o, D, w_o, nullptr, nullptr, 0, out, ldo, M, D, D, 0, stream);
+    return linear(dtype, o, D, w_o, nullptr, nullptr, 0, out, ldo, M, D, D, 0, true, stream);
 }
 
-size_t convnn_b200_conv1d_attention_workspace_bytes(int dtype, int32_t B, int32_t T, int32_t D, int32_t kernel_size) {
-    if ((dtype != CONVNN_F32 && dtype != CONVNN_BF16) || B < 1 || T < 1 || D < 1 || kernel_size < 1) return 0;
-    const size_t elt = dtype == CONVNN_F32 ? 4 : 2, part = up256((size_t)B * T * D * elt);
-    // (the unfolded operand also for shapes that only unfold where the taps are unaligned)
-    return 3 * part + up256((size_t)B * T * D * kernel_size * elt);
-}
-
-int convnn_b200_conv1d_attention(int dtype, const void* x, int64_t ldx, const void* w_x, const void* b_x,
+int convnn::conv1d_attention(int dtype, const void* x, int64_t ldx, const void* w_x, const void* b_x,
                                  const void* w_conv, const void* b_conv, const void* w_o, const void* b_o, void* out,
                                  int64_t ldo, int32_t B, int32_t T, int32_t D, int32_t H, int32_t kernel_size,
-                                 void* workspace, size_t workspace_bytes, void* stream) {
+                                 void* workspace, size_t workspace_bytes, bool at_rest, void* stream) {
     int rc = branch_args_ok("conv1d_attention", dtype, B, T, D, H, ldx, ldo);
     if (rc) return rc;
     if (kernel_size < 1) return set_error(CONVNN_E_INVALID, "conv1d_attention: kernel_size must be positive");
@@ -762,7 +822,7 @@ int convnn_b200_conv1d_attention(int dtype, const void* x, int64_t ldx, const vo
     char* ws = static_cast<char*>(workspace);
     void *y = ws, *o = ws + part, *merged = ws + 2 * part, *unfold = ws + 3 * part;
     const long long M = (long long)B * T;
-    if ((rc = convnn_b200_linear(dtype, x, ldx, w_x, b_x, nullptr, 0, y, D, M, D, D, 0, stream))) return rc;
+    if ((rc = linear(dtype, x, ldx, w_x, b_x, nullptr, 0, y, D, M, D, D, 0, at_rest, stream))) return rc;
     // the reference reads the per-head (T, d_k) block back as (d_k, T) for every H (layers.py:487-489, 499)
     rc = dtype == CONVNN_BF16 && !force_simt() ? try_launch_conv1d_tc(y, w_conv, b_conv, merged, B, T, H, D / H, kernel_size, st)
                                                : (int)CONVNN_E_UNSUPPORTED;
@@ -771,7 +831,5 @@ int convnn_b200_conv1d_attention(int dtype, const void* x, int64_t ldx, const vo
         rc = launch_merge_heads(dtype, o, merged, B, T, H, D / H, st);
     }
     if (rc) return rc;
-    return convnn_b200_linear(dtype, merged, D, w_o, b_o, nullptr, 0, out, ldo, M, D, D, 0, stream);
+    return linear(dtype, merged, D, w_o, b_o, nullptr, 0, out, ldo, M, D, D, 0, true, stream);
 }
-
-}  // extern "C"

@@ -29,12 +29,18 @@ void count_launch();
 // Kernels of a chain: each is launched while its predecessor on the stream still runs (programmatic stream
 // serialization), so that its launch, barrier set-up and TMEM allocation overlap the predecessor's tail.  The rule that
 // makes this safe: EVERY thread of a kernel launched with launch_chained() calls chain_wait() before its first access to
-// global memory, read or write.  The wait ends when the predecessor has completed and its writes are visible; the
+// global memory, read or write (one exception below).  The wait ends when the predecessor has completed and its writes are visible; the
 // predecessor has waited likewise, so completion is transitive along the stream.  chain_next() lets the successor start;
 // it comes after the wait (nothing older than the predecessor can still run when a successor starts) and, in kernels that
 // allocate TMEM, after the allocation (a successor's CTA may take only what is left, and gives it back).
+// The exception: weights, where the predecessor is a kernel of this library that the same call has launched and that does not write
+// them ("at rest").  That kernel let this one start only after its own wait, so all that came before it on the stream, a
+// kernel of the caller's that wrote the weights included, has ended.  The first kernel of a call never does this.
 // A ViT-Tiny forward is 64 kernels (52 up to 21 images) with gaps of ~1.9 us and prologues of ~2 us.  One image 827 -> 712 us, 37 images
 // 923 -> 808 us, 256 images 1757 -> 1673 us, BranchConv 64 images 1788 -> 1500 us, ViT-Small 256 images 4588 -> 4441 us.
+// The GEMM and MLP kernels' roles each wait for themselves, after their set-up (in the MLP block of one image 4.7 us passed
+// between the wait and the first product, 0.9 of them barriers, 1.7 the first instructions and copies of the roles, 1.9 moments
+// read a row at a time), and load weights at rest meanwhile: one image 483 -> 436 us, 37 images 655 -> 609 us, 256 1659 -> 1587 us.
 __device__ __forceinline__ void chain_wait() { cudaGridDependencySynchronize(); }
 __device__ __forceinline__ void chain_next() { cudaTriggerProgrammaticLaunchCompletion(); }
 __device__ __forceinline__ void chain_begin() {
@@ -211,6 +217,9 @@ struct GemmTcOpts {
     int ln_planes = 0;
     float ln_eps = 0.f;
     const void* ln_wextra = nullptr;
+    // The launch before this one on the stream is this library's own, made by the same call, and does not write W, its
+    // extra rows or the bias: they may be read before it has ended (see chain_wait()).
+    bool w_at_rest = false;
     // Row moments of the stored rows, [gemm_tc_moment_planes(N)][gemm_tc_moment_stride(M)][2]; needs a skip connection.
     float* moments_out = nullptr;
 };
@@ -231,8 +240,32 @@ bool mlp_tc_supported(int D, int DM, int planes);
 int mlp_tc_moment_planes();
 int launch_mlp_tc(const void* x, long long ldx, const float* moments, int planes, float eps, const void* w1_folded,
                   const void* w1_extra, const void* w2, const void* b2, void* out, long long ldo, int M, int D, int DM,
-                  float* moments_out, const void* w_o, const void* resid, long long ldr, cudaStream_t st);
+                  float* moments_out, const void* w_o, const void* resid, long long ldr, bool weights_at_rest, cudaStream_t st);
 int read_mlp_tc_status(int* out);
+// The entry points of these names; at_rest: as GemmTcOpts::w_at_rest, for the call's first weights.
+int prenorm_mlp(const void* x, int64_t ldx, const float* moments, int32_t planes, float eps, const void* w1_folded,
+                const void* w1_extra, const void* w2, const void* b2, void* out, int64_t ldo, int64_t M, int32_t D, int32_t DM,
+                float* moments_out, bool at_rest, void* stream);
+int prenorm_forward(const convnn_desc* d, const void* x, int64_t ldx, const float* moments, int32_t planes, float eps,
+                    const void* w_qkv_folded, const void* w_qkv_extra, const void* w_conv, const void* w_pw, const void* w_o,
+                    const void* residual, int64_t ldr, void* out, int64_t ldo, float* moments_out, void* workspace,
+                    size_t workspace_bytes, bool at_rest, void* stream);
+int layer_forward(const convnn_desc* d, const void* x, int64_t ldx, const void* w_qkv, const void* w_conv, const void* w_pw,
+                  const void* w_o, const int32_t* cand, const void* residual, int64_t ldr, void* out, int64_t ldo, void*
+                  workspace, size_t workspace_bytes, bool at_rest, void* stream);
+int linear(int dtype, const void* a, int64_t lda, const void* w, const void* bias, const void* residual, int64_t ldr, void*
+           out, int64_t ldo, int64_t M, int32_t N, int32_t K, int32_t gelu, bool at_rest, void* stream);
+int prenorm_linear(const void* a, int64_t lda, const float* moments, int32_t planes, float eps, const void* w_folded, const
+                   void* w_extra, void* out, int64_t ldo, int64_t M, int32_t N, int32_t K, int32_t gelu, bool at_rest, void*
+                   stream);
+int linear_moments(const void* a, int64_t lda, const void* w, const void* bias, const void* residual, int64_t ldr, void* out,
+                   int64_t ldo, int64_t M, int32_t N, int32_t K, float* moments_out, bool at_rest, void* stream);
+int softmax_attention(int dtype, const void* x, int64_t ldx, const void* w_qkv, const void* w_o, void* out, int64_t ldo,
+                      int32_t B, int32_t T, int32_t D, int32_t H, void* workspace, size_t workspace_bytes, bool at_rest, void*
+                      stream);
+int conv1d_attention(int dtype, const void* x, int64_t ldx, const void* w_x, const void* b_x, const void* w_conv, const void*
+                     b_conv, const void* w_o, const void* b_o, void* out, int64_t ldo, int32_t B, int32_t T, int32_t D,
+                     int32_t H, int32_t kernel_size, void* workspace, size_t workspace_bytes, bool at_rest, void* stream);
 int launch_row_moments(const void* x, long long ldx, long long rows, int D, float* moments, cudaStream_t st);
 int launch_fold_layernorm(const void* w, const void* bias, const void* gamma, const void* beta, int N, int K,
                           void* w_folded, void* w_extra, cudaStream_t st);

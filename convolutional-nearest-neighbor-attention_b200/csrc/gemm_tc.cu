@@ -79,6 +79,7 @@ struct GemmTcParams {
     int stages;            // depth of the shared-memory ring
     int wstat;             // 1: the whole W tile (BN x Kd) stays in shared memory; the ring holds A only
     int tiles_per_cta;     // wstat: each CTA owns a contiguous range of the n-major tile list
+    int w_at_rest;         // nothing that may still run on the stream writes W, its extra rows or the bias
     // pre-norm fold: the moments of the A rows, [ln_planes][mom_ld] (sum, sum of squares) partial sums,
     // arrive through the tensor map tmM
     int ln_planes;
@@ -239,8 +240,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (PAIR) { tmem_alloc_pair(tmem_slot, ncols); tmem_relinquish_pair(); }
         else { tmem_alloc(tmem_slot, ncols); tmem_relinquish(); }
     }
-    chain_wait();
     if (p.mma_bias) {
+        if (!p.w_at_rest) chain_wait();
         // D = ones * btile^T = bias[n] in every row.  Both 16-byte halves of a row of `ones`
         // start with 1.0 and a btile row holds its bias in exactly one half, so the product
         // does not depend on how the 32-byte swizzle orders the halves.
@@ -262,7 +263,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (PAIR) cluster_sync_all();               // both CTAs' barriers exist before any remote signal
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_next();
+    // From here on every role waits for the predecessor (chain_wait) before its own first access to global memory; what
+    // comes before that, and with p.w_at_rest the loads of W, is done when the predecessor ends.
     const uint32_t peer_abort = PAIR ? map_to_cta(smem_u32(const_cast<int*>(abort_flag)), rank ^ 1u) : 0u;
     auto give_up = [&](int code) {
         if (PAIR) fail_pair(abort_flag, peer_abort, code);
@@ -295,6 +297,34 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             trace(tr, 0, tn);
             const uint32_t tx = (a_bytes + (p.wstat ? 0u : b_bytes)) * (PAIR ? 2u : 1u);
             const uint32_t lead_full0 = PAIR ? map_to_cta(full0, 0) : full0;
+            auto load_w_tile = [&](int nt) {
+                mbar_expect_tx_a(wfull_a, p.KC * b_bytes + (LNF ? (uint32_t)bn_cta * 32u : 0u));
+                for (int kc = 0; kc < p.KC; ++kc)
+                    tma_load_2d_a(sB0 + kc * b_bytes, &tmW, wfull_a, kc * p.KCH, nt * p.BN);
+                if (LNF) tma_load_2d_a(smem_u32(xb), &tmX, wfull_a, 0, nt * p.BN);
+                cur_nt = nt;
+                ++wloads;
+            };
+            auto load_w_chunk = [&](uint32_t slot, int kc, int n0) {
+                if (PAIR) tma_load_2d_pair(sB0 + slot * b_bytes, &tmW, lead_full0 + 8 * slot, kc * p.KCH, n0);
+                else if (!p.wstat) tma_load_2d_a(sB0 + slot * b_bytes, &tmW, full0 + 8 * slot, kc * p.KCH, n0);
+            };
+            // W of the first tile, or as many of its chunks as the ring holds, before the predecessor has ended
+            int w_ahead = 0;
+            if (p.w_at_rest && first < last) {
+                int mt, nt;
+                tile_mn(first, mt, nt);
+                if (p.wstat) {
+                    load_w_tile(nt);
+                } else {
+                    w_ahead = min(p.KC, (int)STAGES);
+                    for (int kc = 0; kc < w_ahead; ++kc) {
+                        if (!PAIR || rank == 0) mbar_expect_tx_a(full0 + 8 * kc, tx);
+                        load_w_chunk((uint32_t)kc, kc, nt * p.BN + (int)rank * bn_cta);
+                    }
+                }
+            }
+            chain_wait();
             for (int t = first; t < last && ok; t += step) {
                 int mt, nt;
                 tile_mn(t, mt, nt);
@@ -302,26 +332,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     // every MMA that reads the old W tile has completed once the most recently
                     // filled ring stage has been released
                     if (any && !mbar_wait_a(empty0 + 8 * last_s, last_ph, abort_flag)) { give_up(15); ok = false; break; }
-                    mbar_expect_tx_a(wfull_a, p.KC * b_bytes + (LNF ? (uint32_t)bn_cta * 32u : 0u));
-                    for (int kc = 0; kc < p.KC; ++kc)
-                        tma_load_2d_a(sB0 + kc * b_bytes, &tmW, wfull_a, kc * p.KCH, nt * p.BN);
-                    if (LNF) tma_load_2d_a(smem_u32(xb), &tmX, wfull_a, 0, nt * p.BN);
-                    cur_nt = nt;
-                    ++wloads;
+                    load_w_tile(nt);
                 }
                 trace(tr, 0, tn);
                 const int m0 = mt * TM + (int)rank * BM, n0 = nt * p.BN + (int)rank * bn_cta;
                 for (int kc = 0; kc < p.KC; ++kc) {
                     if (!mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag)) { give_up(11); ok = false; break; }
-                    if (PAIR) {
-                        if (rank == 0) mbar_expect_tx_a(full0 + 8 * s, tx);
-                        tma_load_2d_pair(sA0 + s * a_bytes, &tmA, lead_full0 + 8 * s, kc * p.KCH, m0);
-                        tma_load_2d_pair(sB0 + s * b_bytes, &tmW, lead_full0 + 8 * s, kc * p.KCH, n0);
-                    } else {
-                        mbar_expect_tx_a(full0 + 8 * s, tx);
-                        tma_load_2d_a(sA0 + s * a_bytes, &tmA, full0 + 8 * s, kc * p.KCH, m0);
-                        if (!p.wstat) tma_load_2d_a(sB0 + s * b_bytes, &tmW, full0 + 8 * s, kc * p.KCH, n0);
-                    }
+                    const bool whole = w_ahead == 0;            // (otherwise its W chunk is on the way)
+                    if (whole && (!PAIR || rank == 0)) mbar_expect_tx_a(full0 + 8 * s, tx);
+                    if (PAIR) tma_load_2d_pair(sA0 + s * a_bytes, &tmA, lead_full0 + 8 * s, kc * p.KCH, m0);
+                    else tma_load_2d_a(sA0 + s * a_bytes, &tmA, full0 + 8 * s, kc * p.KCH, m0);
+                    if (whole) load_w_chunk(s, kc, n0);
+                    else --w_ahead;
                     last_s = s; last_ph = ph; any = true;
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
@@ -412,6 +434,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             mbar_expect_tx(&mfull[slot], slot_bytes);
             tma_load_2d(mring + slot * slot_bytes, &tmM, &mfull[slot], mt * BM * 2, 0);
         };
+        chain_wait();
         if (lane == 0)
             for (int k = 0; k < MOM_AHEAD; ++k)
                 if (first + k * step < last) fetch((uint32_t)k, first + k * step);
@@ -486,6 +509,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const bool tr = !PAIR && trace_enabled() && blockIdx.x == 0 && lq == 0 && lane == 0 && chalf == 0;
         const uint32_t lead_tempty0 = PAIR ? map_to_cta(smem_u32(tempty), 0) : 0u;
         int tn = 0;
+        chain_wait();
+        chain_next();
         for (int t = first + half * step; t < last && ok; t += 2 * step, tile += 2) {
             int mt, nt;
             tile_mn(t, mt, nt);
@@ -797,6 +822,7 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
     }
     p.ldc = ldc; p.bias = static_cast<const __nv_bfloat16*>(o.bias); p.gelu = o.gelu;
     p.mma_bias = nullptr;
+    p.w_at_rest = o.w_at_rest;
     p.residual = static_cast<const __nv_bfloat16*>(o.residual); p.ldr = o.ldr;
     p.stat_pieces = 1; p.stat_plane = 0;
     p.stat_mode = o.stat_mode; p.dk = o.dk > 0 ? o.dk : 32; p.heads = o.heads; p.rows_per_batch = o.rows_per_batch > 0 ? o.rows_per_batch : 1;

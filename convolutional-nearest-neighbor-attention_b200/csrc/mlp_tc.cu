@@ -96,6 +96,7 @@ struct MlpParams {
     int planes;         // planes of the incoming moments
     long long mom_ld_in, mom_ld_out;
     float eps, inv_d;
+    int weights_at_rest;   // nothing that may still run on the stream writes the weights: their first chunks need not wait
     const float2* moments;
     const __nv_bfloat16* resid;   // OP: the rows x of the skip connection x + o W_o^T, stride ldr
     long long ldr;
@@ -190,15 +191,14 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
     }
     __syncthreads();
     if (warp == 1) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
-    chain_wait();
-    for (int i = threadIdx.x; i < p.D / 2; i += blockDim.x)         // b2 (or zeros) for the final epilogue
-        reinterpret_cast<uint32_t*>(smem + L.bias)[i] = p.bias2 ? reinterpret_cast<const uint32_t*>(p.bias2)[i] : 0u;
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync_all();                          // both CTAs' barriers exist before any remote signal
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_next();
+    // From here on the roles go their own ways; each waits for the predecessor (chain_wait) before its own first access to
+    // global memory, so that all of this, the first instructions of every role and, with p.weights_at_rest, the first
+    // weight chunks are done when the predecessor ends.
     const uint32_t peer_abort = map_to_cta(smem_u32(const_cast<int*>(abort_flag)), rank ^ 1u);
     auto give_up = [&](int code) {
         st_cluster_u32(peer_abort, 1u);
@@ -225,6 +225,21 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         // the x tiles) with one instruction of the warp; lane KC + 2 stores finished tiles and refills their
         // buffers.  The W2 stream, whose slots are released by MMA 2, has warp 20.
         const uint32_t w1_mask = (2u << p.KC) - 1u;              // lanes 0 .. KC
+        // one W1 super-chunk into slot b
+        auto load_w1 = [&](uint32_t b, int sc) {
+            if (rank == 0 && lane == 0) mbar_expect_tx_a(lbar(W1FULL + b), 2u * L.w1_slot);
+            __syncwarp(w1_mask);
+            const uint32_t w1s = base + L.w1 + b * L.w1_slot;
+            if (lane < p.KC)
+                tma_load_2d_pair(w1s + lane * 8192u, &tmW1, leadbar(W1FULL + b), lane * 64, sc * SC + (int)rank * 64);
+            else
+                tma_load_2d_pair(w1s + p.KC * 8192u, &tmWX, leadbar(W1FULL + b), 0, sc * SC + (int)rank * 64);
+        };
+        const int w1_ahead = !OP && p.weights_at_rest && my_tiles > 0 ? min(nsc, 2) : 0;
+        if (lane <= p.KC)
+            for (int sc = 0; sc < w1_ahead; ++sc) load_w1((uint32_t)sc, sc);
+        __syncwarp();
+        chain_wait();
         if (lane <= p.KC) {
             bool ok = true;
             auto load_x = [&](int it) {
@@ -259,38 +274,37 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
                 for (int sc = 0; sc < nsc && ok; ++sc, ++n) {
                     if (OP && sc == kp && it + 1 < my_tiles) { load_wo(); if (!ok) break; }
                     const uint32_t b = n & 1u;
+                    if ((int)n < w1_ahead) continue;
                     // the slot's previous item (n - 2) has been multiplied
                     ok = mbar_wait(&bars[A1FULL + b], ((n >> 1) & 1u) ^ 1u, abort_flag);
                     ok = __all_sync(w1_mask, ok);
                     if (!ok) { if (lane == 0) give_up(52); break; }
                     mtrace(cluster_id == 0 && rank == 0 && lane == 0, 1, n);
-                    if (rank == 0 && lane == 0) mbar_expect_tx_a(lbar(W1FULL + b), 2u * L.w1_slot);
-                    __syncwarp(w1_mask);
-                    const uint32_t w1s = base + L.w1 + b * L.w1_slot;
-                    if (lane < p.KC)
-                        tma_load_2d_pair(w1s + lane * 8192u, &tmW1, leadbar(W1FULL + b), lane * 64, sc * SC + (int)rank * 64);
-                    else
-                        tma_load_2d_pair(w1s + p.KC * 8192u, &tmWX, leadbar(W1FULL + b), 0, sc * SC + (int)rank * 64);
+                    load_w1(b, sc);
                 }
             }
-        } else if (lane == p.KC + 2) {
-            // the finished rows of a tile leave through a TMA store of the x buffer they were written into;
-            // the buffer is refilled at once with the tile after the next (tile 1 is requested up front)
+        } else if (lane >= 8 && lane < 8 + p.KC) {
+            // the finished rows of a tile leave through TMA stores of the x buffer they were written into, a sub-chunk per
+            // lane; the buffer is refilled at once with the tile after the next (tile 1 is requested up front)
+            const uint32_t st_mask = ((1u << p.KC) - 1u) << 8;
+            const int kc = lane - 8;
             auto load_next = [&](int it) {
                 const uint32_t xb = (uint32_t)it & 1u;
-                if (rank == 0) mbar_expect_tx_a(lbar(XFULL + xb), 2u * x_tile_bytes);
-                for (int kc = 0; kc < p.KC; ++kc)
-                    tma_load_2d_pair(base + L.x + xb * x_tile_bytes + kc * 16384u, &tmX, leadbar(XFULL + xb), kc * 64, row0_of(it));
+                if (rank == 0 && kc == 0) mbar_expect_tx_a(lbar(XFULL + xb), 2u * x_tile_bytes);
+                __syncwarp(st_mask);
+                tma_load_2d_pair(base + L.x + xb * x_tile_bytes + kc * 16384u, &tmX, leadbar(XFULL + xb), kc * 64, row0_of(it));
             };
             if (my_tiles > 1) load_next(1);
             for (int it = 0; it < my_tiles; ++it) {
                 const uint32_t xb = (uint32_t)it & 1u;
-                if (!mbar_wait_a(lbar(OUTREADY + xb), (uint32_t)(it >> 1) & 1u, abort_flag)) { give_up(66); break; }
-                for (int kc = 0; kc < p.KC; ++kc)
-                    tma_store_2d(&tmO, smem + L.x + xb * x_tile_bytes + kc * 16384u, kc * 64, row0_of(it));
+                bool ok = mbar_wait_a(lbar(OUTREADY + xb), (uint32_t)(it >> 1) & 1u, abort_flag);
+                ok = __all_sync(st_mask, ok);
+                if (!ok) { if (kc == 0) give_up(66); break; }
+                tma_store_2d(&tmO, smem + L.x + xb * x_tile_bytes + kc * 16384u, kc * 64, row0_of(it));
                 tma_store_commit();
                 tma_store_wait_read<0>();
-                mbar_arrive(&bars[XFREE + xb]);                   // the buffer's contents are no longer needed
+                __syncwarp(st_mask);
+                if (kc == 0) mbar_arrive(&bars[XFREE + xb]);      // the buffer's contents are no longer needed
                 if (it + 2 < my_tiles) load_next(it + 2);
             }
             tma_store_wait<0>();
@@ -392,6 +406,7 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
             uint32_t s = 0, ph = 0;
             int c = 0;
             const int nch = nsc * 2;
+            if (!p.weights_at_rest) chain_wait();
             for (uint32_t g = 0; g < total; ++g) {
                 if (!mbar_wait_a(lbar(W2EMPTY + s), ph ^ 1u, abort_flag)) { give_up(53); break; }
                 mtrace(cluster_id == 0 && rank == 0, 0, g);
@@ -404,6 +419,8 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
     } else if (warp == 2) {
         // ---- extra operand chunk of every tile (as in gemm_tc.cu): lane l prepares rows l, l + 32, ...
         // The moments of tile it are read with plain loads while tile it - 1 is still being worked on.
+        chain_wait();
+        chain_next();
         bool ok = true;
         for (int it = 0; it < my_tiles && ok; ++it) {
             const uint32_t xb = (uint32_t)it & 1u;
@@ -416,28 +433,36 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) { if (lane == 0) give_up(61); break; }
             }
+            float s1[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};
+            if (OP) {
+                const float2* part = reinterpret_cast<const float2*>(smem + L.xa + xb * 4096u);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int row = row0_of(it) + j * 32 + lane;
-                float s1 = 0.f, s2 = 0.f;
-                if (OP) {
-                    const float2* part = reinterpret_cast<const float2*>(smem + L.xa + xb * 4096u);
+                for (int j = 0; j < 4; ++j)
                     for (int gq = 0; gq < p.D / 64; ++gq) {
                         const float2 m = part[gq * BM + j * 32 + lane];
-                        s1 += m.x; s2 += m.y;
+                        s1[j] += m.x; s2[j] += m.y;
                     }
-                } else if (row < p.M)
-                    for (int pl0 = 0; pl0 < p.planes; pl0 += 4) {      // four independent loads in flight per row
-                        float2 m[4];
+            } else {
+                for (int pl0 = 0; pl0 < p.planes; pl0 += 4) {      // sixteen independent loads in flight
+                    float2 m[4][4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int row = row0_of(it) + j * 32 + lane;
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
-                            m[k] = pl0 + k < p.planes ? __ldg(p.moments + (long long)(pl0 + k) * p.mom_ld_in + row)
-                                                      : make_float2(0.f, 0.f);
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) { s1 += m[k].x; s2 += m[k].y; }
+                            m[j][k] = pl0 + k < p.planes && row < p.M
+                                          ? __ldg(p.moments + (long long)(pl0 + k) * p.mom_ld_in + row) : make_float2(0.f, 0.f);
                     }
-                const float mean = s1 * p.inv_d;
-                const float var = fmaxf(fmaf(-mean, mean, s2 * p.inv_d), 0.f) + p.eps;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) { s1[j] += m[j][k].x; s2[j] += m[j][k].y; }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float mean = s1[j] * p.inv_d;
+                const float var = fmaxf(fmaf(-mean, mean, s2[j] * p.inv_d), 0.f) + p.eps;
                 const float rstd = rsqrtf(var), sigma = var * rstd;
                 rs[j] = rstd;
                 const __nv_bfloat16 mh = __float2bfloat16_rn(-mean), sh = __float2bfloat16_rn(sigma);
@@ -474,6 +499,10 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         // back to tensor memory (16 columns of this warp's rows) and MMA 2 reads them there, so h never
         // passes through shared memory.  (Two groups of eight warps that alternated over the super-chunks
         // were measured too: the same time.)
+        chain_wait();
+        for (int i = threadIdx.x - 3 * 32; i < p.D / 2; i += 16 * 32)   // b2 (or zeros) for the final epilogue
+            reinterpret_cast<uint32_t*>(smem + L.bias)[i] = p.bias2 ? reinterpret_cast<const uint32_t*>(p.bias2)[i] : 0u;
+        asm volatile("bar.sync 1, 512;" ::: "memory");
         const int ew = warp - 3;
         const int cg = ew >> 2, lq = warp & 3;                    // column group, TMEM lane quarter
         const int hb = cg >> 1;                                   // h chunk this warp writes into
@@ -703,7 +732,7 @@ int mlp_tc_moment_planes() { return 4; }
 
 int launch_mlp_tc(const void* x, long long ldx, const float* moments, int planes, float eps, const void* w1_folded,
                   const void* w1_extra, const void* w2, const void* b2, void* out, long long ldo, int M, int D, int DM,
-                  float* moments_out, const void* w_o, const void* resid, long long ldr, cudaStream_t st) {
+                  float* moments_out, const void* w_o, const void* resid, long long ldr, bool weights_at_rest, cudaStream_t st) {
     if (!mlp_tc_supported(D, DM, planes))
         return set_error(CONVNN_E_UNSUPPORTED, "mlp_tc: D=%d d_mlp=%d planes=%d is outside the fused kernel's shapes", D, DM, planes);
     if (!aligned16(x) || !aligned16(out) || !aligned16(w1_folded) || !aligned16(w1_extra) || !aligned16(w2) ||
@@ -719,6 +748,7 @@ int launch_mlp_tc(const void* x, long long ldx, const float* moments, int planes
     p.planes = planes; p.eps = eps; p.inv_d = 1.0f / (float)D;
     p.bias2 = static_cast<const __nv_bfloat16*>(b2);
     p.resid = static_cast<const __nv_bfloat16*>(resid); p.ldr = ldr;
+    p.weights_at_rest = weights_at_rest;
     p.moments_out = reinterpret_cast<float2*>(moments_out);
     CUtensorMap tmX, tmO, tmW1, tmWX, tmW2, tmWO;
     {

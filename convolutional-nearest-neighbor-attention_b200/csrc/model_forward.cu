@@ -80,35 +80,34 @@ int block_forward(const convnn_model* m, const convnn_block& b, char* ws, const 
             if ((rc = convnn_b200_row_moments(x, D, rows, (int32_t)D, mom, stream))) return rc;
             *planes = 1;
         }
-        if ((rc = convnn_b200_prenorm_forward(&b.layer, x, D, mom, *planes, b.eps1, b.w_qkv_folded, b.w_qkv_extra, b.w_conv,
-                                              b.w_pw, b.w_o, x, D, x1, D, fold_mlp ? mom1 : nullptr, layer_ws,
-                                              layer_bytes, stream)))
+        if ((rc = prenorm_forward(&b.layer, x, D, mom, *planes, b.eps1, b.w_qkv_folded, b.w_qkv_extra, b.w_conv, b.w_pw, b.w_o, x,
+                                  D, x1, D, fold_mlp ? mom1 : nullptr, layer_ws, layer_bytes, true, stream)))
             return rc;
         if (fold_mlp) planes1 = convnn_b200_moment_planes((int32_t)D);
     } else {
         if ((rc = convnn_b200_layernorm(m->dtype, x, D, b.norm1_w, b.norm1_b, b.eps1, xn, D, rows, (int32_t)D, stream))) return rc;
         if (b.kind == CONVNN_BLOCK_CONVNN) {
-            if ((rc = convnn_b200_forward(&b.layer, xn, D, b.w_qkv, b.w_conv, b.w_pw, b.w_o, b.cand, x, D, x1, D, layer_ws,
-                                          layer_bytes, stream)))
+            if ((rc = layer_forward(&b.layer, xn, D, b.w_qkv, b.w_conv, b.w_pw, b.w_o, b.cand, x, D, x1, D, layer_ws, layer_bytes,
+                                    true, stream)))
                 return rc;
         } else {
             // both branches read their channel slice of xn and write theirs of the concat buffer
             const int64_t dc = b.layer.D, rest = D - dc;
             char* cat = scratch + p.cat;
-            if ((rc = convnn_b200_forward(&b.layer, xn, D, b.w_qkv, b.w_conv, b.w_pw, b.w_o, b.cand, nullptr, 0, cat, D,
-                                          layer_ws, layer_bytes, stream)))
+            if ((rc = layer_forward(&b.layer, xn, D, b.w_qkv, b.w_conv, b.w_pw, b.w_o, b.cand, nullptr, 0, cat, D, layer_ws,
+                                    layer_bytes, true, stream)))
                 return rc;
             const char* xr = xn + dc * elt;
             char* cr = cat + dc * elt;
             rc = b.kind == CONVNN_BLOCK_BRANCH_ATTENTION
-                     ? convnn_b200_softmax_attention(m->dtype, xr, D, b.branch_w_in, b.branch_w_out, cr, D, m->B, m->T,
-                                                     (int32_t)rest, b.layer.H, layer_ws, layer_bytes, stream)
-                     : convnn_b200_conv1d_attention(m->dtype, xr, D, b.branch_w_in, b.branch_b_in, b.branch_w_conv,
-                                                    b.branch_b_conv, b.branch_w_out, b.branch_b_out, cr, D, m->B, m->T,
-                                                    (int32_t)rest, b.layer.H, b.kernel_size, layer_ws, layer_bytes, stream);
+                     ? softmax_attention(m->dtype, xr, D, b.branch_w_in, b.branch_w_out, cr, D, m->B, m->T, (int32_t)rest,
+                                         b.layer.H, layer_ws, layer_bytes, true, stream)
+                     : conv1d_attention(m->dtype, xr, D, b.branch_w_in, b.branch_b_in, b.branch_w_conv, b.branch_b_conv,
+                                        b.branch_w_out, b.branch_b_out, cr, D, m->B, m->T, (int32_t)rest, b.layer.H,
+                                        b.kernel_size, layer_ws, layer_bytes, true, stream);
             if (rc) return rc;
-            if ((rc = convnn_b200_linear(m->dtype, cat, D, b.pointwise_w, b.pointwise_b, x, D, x1, D, rows, (int32_t)D,
-                                         (int32_t)D, 0, stream)))
+            if ((rc = linear(m->dtype, cat, D, b.pointwise_w, b.pointwise_b, x, D, x1, D, rows, (int32_t)D, (int32_t)D, 0, true,
+                             stream)))
                 return rc;
         }
     }
@@ -122,21 +121,21 @@ int block_forward(const convnn_model* m, const convnn_block& b, char* ws, const 
         }
         if (b.fuse_mlp && convnn_b200_prenorm_mlp_supported((int32_t)D, dm, planes1)) {
             if (want_moments) *planes = convnn_b200_prenorm_mlp_moment_planes();
-            return convnn_b200_prenorm_mlp(x1, D, mom1, planes1, b.eps2, b.fc1_folded, b.fc1_extra, b.fc2_w, b.fc2_b, x, D,
-                                           rows, (int32_t)D, dm, want_moments ? mom : nullptr, stream);
+            return prenorm_mlp(x1, D, mom1, planes1, b.eps2, b.fc1_folded, b.fc1_extra, b.fc2_w, b.fc2_b, x, D, rows, (int32_t)D,
+                               dm, want_moments ? mom : nullptr, true, stream);
         }
-        if ((rc = convnn_b200_prenorm_linear(x1, D, mom1, planes1, b.eps2, b.fc1_folded, b.fc1_extra, h, dm, rows, dm,
-                                             (int32_t)D, 1, stream)))
+        if ((rc = prenorm_linear(x1, D, mom1, planes1, b.eps2, b.fc1_folded, b.fc1_extra, h, dm, rows, dm, (int32_t)D, 1, true,
+                                 stream)))
             return rc;
     } else {
         if ((rc = convnn_b200_layernorm(m->dtype, x1, D, b.norm2_w, b.norm2_b, b.eps2, xn, D, rows, (int32_t)D, stream))) return rc;
-        if ((rc = convnn_b200_linear(m->dtype, xn, D, b.fc1_w, b.fc1_b, nullptr, 0, h, dm, rows, dm, (int32_t)D, 1, stream))) return rc;
+        if ((rc = linear(m->dtype, xn, D, b.fc1_w, b.fc1_b, nullptr, 0, h, dm, rows, dm, (int32_t)D, 1, true, stream))) return rc;
     }
     if (want_moments && m->dtype == CONVNN_BF16) {
         *planes = convnn_b200_moment_planes((int32_t)D);
-        return convnn_b200_linear_moments(h, dm, b.fc2_w, b.fc2_b, x1, D, x, D, rows, (int32_t)D, dm, mom, stream);
+        return linear_moments(h, dm, b.fc2_w, b.fc2_b, x1, D, x, D, rows, (int32_t)D, dm, mom, true, stream);
     }
-    return convnn_b200_linear(m->dtype, h, dm, b.fc2_w, b.fc2_b, x1, D, x, D, rows, (int32_t)D, dm, 0, stream);
+    return linear(m->dtype, h, dm, b.fc2_w, b.fc2_b, x1, D, x, D, rows, (int32_t)D, dm, 0, true, stream);
 }
 
 int check(const convnn_model* m) {
@@ -185,8 +184,8 @@ int convnn_b200_model_forward(const convnn_model* m, const void* images, void* l
     else
         rc = convnn_b200_patchify(m->dtype, images, cols, m->B, m->channels, m->height, m->width, m->patch, stream);
     if (rc) return rc;
-    if ((rc = convnn_b200_linear(m->dtype, cols, pix, m->patch_w, m->patch_b, nullptr, 0, proj, m->D, (int64_t)m->B * np, m->D,
-                                 pix, 0, stream)))
+    if ((rc = linear(m->dtype, cols, pix, m->patch_w, m->patch_b, nullptr, 0, proj, m->D, (int64_t)m->B * np, m->D, pix, 0, true,
+                     stream)))
         return rc;
     const bool first_folds = m->n_blocks > 0 && m->blocks[0].w_qkv_folded;
     if ((rc = convnn_b200_embed_tokens_moments(m->dtype, proj, m->embed_norm_w, m->embed_norm_b, m->embed_eps, m->cls, m->pe,
@@ -198,8 +197,8 @@ int convnn_b200_model_forward(const convnn_model* m, const void* images, void* l
         const bool want = i + 1 < m->n_blocks && m->blocks[i + 1].w_qkv_folded;
         if ((rc = block_forward(m, m->blocks[i], ws, p, &planes, want, stream))) return rc;
     }
-    return convnn_b200_linear(m->dtype, ws + p.x, (int64_t)m->T * m->D, m->head_w, m->head_b, nullptr, 0, logits, m->classes,
-                              m->B, m->classes, m->D, 0, stream);
+    return linear(m->dtype, ws + p.x, (int64_t)m->T * m->D, m->head_w, m->head_b, nullptr, 0, logits, m->classes, m->B,
+                  m->classes, m->D, 0, true, stream);
 }
 
 }  // extern "C"

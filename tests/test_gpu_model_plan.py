@@ -116,3 +116,24 @@ def test_layer_call_follows_changes_and_options():
         m.magnitude_type = "unknown"
         with pytest.raises(ValueError, match="magnitude_type"):
             m(x)
+
+
+@pytest.mark.parametrize("cfg", sorted(CONFIGS))
+def test_weights_written_by_the_launch_before_a_forward(cfg):
+    """A forward's kernels may fetch weights early, but never ahead of what the stream did before the call."""
+    m = _model(cfg, torch.bfloat16)
+    x = torch.randn(3, 3, 224, 224, device=DEV).bfloat16()
+    kept = [{n: p.detach() * f for n, p in m.named_parameters()} for f in (0.5, 1.5, 1.0)]
+    with torch.no_grad():
+        want = []
+        for w in kept:
+            for n, p in m.named_parameters():
+                p.copy_(w[n])
+            torch.cuda.synchronize()
+            want.append(_op_by_op(m, x))
+        for _ in range(2):
+            m(x)
+        for turn in range(12):
+            for n, p in m.named_parameters():
+                p.copy_(kept[turn % 3][n])                      # the last of these is the launch before the forward's
+            assert torch.equal(m(x), want[turn % 3])
