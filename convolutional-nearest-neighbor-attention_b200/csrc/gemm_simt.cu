@@ -328,6 +328,41 @@ __device__ __forceinline__ void copy16(uint32_t dst, const void* src, int bytes)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
+// Where a 16-byte piece of a tile row (32 k values; rows of A, then of W) lies, in floats: rows that the lanes of a warp
+// read side by side differ in the exchange.
+template <int BM, int TM>
+__device__ __forceinline__ int place_piece(int row, int piece) {
+    const int x = row < BM ? row / TM : (row - BM) / 4;
+    return row * 32 + ((piece ^ (x & 7)) << 2);
+}
+// The products of one step of 32 k values, ascending; the next four values of every row are read while four are multiplied.
+// (Eight columns per thread leave no registers for that: 128 x 64 tiles of this kind 110 us where 64 x 64 take 86.)
+template <int BM, int TM, int TN>
+__device__ __forceinline__ void multiply_step(const float* tile, int ty, int tx, float (&acc)[TM][TN]) {
+    static_assert(TN == 4, "four columns per thread");
+    const float* pa = tile + ty * TM * 32;
+    const float* pb = tile + (BM + tx * 4) * 32;
+    float4 a[2][TM], b[2][TN];
+    auto read = [&](int q, int u) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i) a[u][i] = *reinterpret_cast<const float4*>(pa + i * 32 + ((q ^ (ty & 7)) << 2));
+#pragma unroll
+        for (int j = 0; j < TN; ++j) b[u][j] = *reinterpret_cast<const float4*>(pb + j * 32 + ((q ^ (tx & 7)) << 2));
+    };
+    read(0, 0);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int u = q & 1;
+        if (q + 1 < 8) read(q + 1, u ^ 1);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf((&a[u][i].x)[e], (&b[u][j].x)[e], acc[i][j]);
+    }
+}
+
 template <int MODE, int BM, int BN, int TM, int TN, int MINB>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_copy_kernel(const GemmParams p) {
     static_assert(MODE == A_ROWS || MODE == A_TOKENS, "plain rows");
@@ -341,12 +376,6 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_copy_ke
     const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
     const int ty = (warp / WN) * 4 + (lane >> 3), tx = (warp % WN) * 8 + (lane & 7);
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(gs);
-    // Where a piece of a tile row lies, in floats: rows that a warp's lanes read side by side differ in the exchange.
-    auto place = [](int row, int piece) {
-        const int x = row < BM ? row / TM : (row - BM) / 4;
-        return row * BK + ((piece ^ (x & 7)) << 2);
-    };
-
     const int piece = tid % PIECES;                             // (NT is a multiple of the pieces of a row)
     const float* src[NL];
 #pragma unroll
@@ -374,7 +403,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_copy_ke
         for (int i = 0; i < NL; ++i) {
             const int row = (tid + i * NT) / PIECES;
             const bool on = src[i] && bytes > 0;
-            copy16(base + 4u * (uint32_t)(slot * (BM + BN) * BK + place(row, piece)), on ? src[i] + k0 : p.a, on ? bytes : 0);
+            copy16(base + 4u * (uint32_t)(slot * (BM + BN) * BK + place_piece<BM, TM>(row, piece)), on ? src[i] + k0 : p.a, on ? bytes : 0);
         }
     };
 
@@ -400,32 +429,140 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_copy_ke
         __syncthreads();                                        // everyone's copies of this step; the slot of the last one is free
         if (step + ST - 1 < steps) request(next, (step + ST - 1) * BK);
         asm volatile("cp.async.commit_group;" ::: "memory");
-        const float* pa = gs + slot * (BM + BN) * BK + ty * TM * BK;
-        const float* pb = gs + slot * (BM + BN) * BK + (BM + tx * 4) * BK;
+        multiply_step<BM, TM, TN>(gs + slot * (BM + BN) * BK, ty, tx, acc);
         slot = slot + 1 == ST ? 0 : slot + 1;
         next = next + 1 == ST ? 0 : next + 1;
-        float4 a[2][TM], b[2][TN];
-        auto read = [&](int q, int u) {
-#pragma unroll
-            for (int i = 0; i < TM; ++i) a[u][i] = *reinterpret_cast<const float4*>(pa + i * BK + ((q ^ (ty & 7)) << 2));
-#pragma unroll
-            for (int j = 0; j < TN; ++j) b[u][j] = *reinterpret_cast<const float4*>(pb + j * BK + ((q ^ (tx & 7)) << 2));
-        };
-        read(0, 0);
-#pragma unroll
-        for (int q = 0; q < PIECES; ++q) {
-            const int u = q & 1;
-            if (q + 1 < PIECES) read(q + 1, u ^ 1);
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-#pragma unroll
-                for (int i = 0; i < TM; ++i)
-#pragma unroll
-                    for (int j = 0; j < TN; ++j) acc[i][j] = fmaf((&a[u][i].x)[e], (&b[u][j].x)[e], acc[i][j]);
-        }
     }
 
     store_outputs<float, TM, 1, 4>(
+        p, n0 + tx * 4, 0, [&](int i) { return m0 + ty * TM + i; },
+        [&](int i, int, float (&r)[4]) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) r[j] = acc[i][j];
+        });
+}
+
+// Four values of an operand row as they came from memory, made float32 when they are stored to shared memory, a step later.
+template <typename T> struct Four;
+template <> struct Four<float> {
+    float4 v;
+    __device__ __forceinline__ void none() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ __forceinline__ void load(const float* p, int n, bool vec) { v = load_upto4(p, n, vec); }
+    __device__ __forceinline__ float4 get() const { return v; }
+};
+template <> struct Four<__nv_bfloat16> {
+    uint32_t r[4];             // two pairs, or four values one by one (`vec` tells)
+    bool pairs;
+    __device__ __forceinline__ void none() {
+        pairs = true;
+        r[0] = r[1] = 0u;
+    }
+    __device__ __forceinline__ void load(const __nv_bfloat16* p, int n, bool vec) {
+        pairs = vec && n >= 4;
+        if (pairs) {
+            const uint2 w = *reinterpret_cast<const uint2*>(p);
+            r[0] = w.x;
+            r[1] = w.y;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r[i] = i < n ? reinterpret_cast<const unsigned short*>(p)[i] : 0u;
+        }
+    }
+    __device__ __forceinline__ float4 get() const {
+        if (pairs)
+            return make_float4(__uint_as_float(r[0] << 16), __uint_as_float(r[0] & 0xffff0000u), __uint_as_float(r[1] << 16),
+                               __uint_as_float(r[1] & 0xffff0000u));
+        return make_float4(__uint_as_float(r[0] << 16), __uint_as_float(r[1] << 16), __uint_as_float(r[2] << 16),
+                           __uint_as_float(r[3] << 16));
+    }
+};
+
+// The same tiles for rows that have to be converted, or that cannot be copied 16 bytes at a time: they come through
+// registers, a step ahead.
+template <typename TA, typename T, int MODE, int BM, int BN, int TM, int TN, int MINB>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_stage_kernel(const GemmParams p) {
+    static_assert(MODE == A_ROWS || MODE == A_TOKENS, "plain rows");
+    chain_begin();
+    constexpr int NT = (BM / TM) * (BN / TN), BK = 32, PIECES = BK / 4, STEP = NT / PIECES;   // rows per pass
+    constexpr int WN = BN / TN / 8, NA = BM / STEP, NB = BN / STEP;
+    static_assert(BM % STEP == 0 && BN % STEP == 0 && NT % 32 == 0 && (BN / TN) % 8 == 0, "tile");
+    extern __shared__ __align__(128) float gs[];                // [2][BM + BN][BK]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    const int ty = (warp / WN) * 4 + (lane >> 3), tx = (warp % WN) * 8 + (lane & 7);
+    const int piece = tid % PIECES, row0 = tid / PIECES;
+
+    const TA* ab[NA];
+    const T* wb[NB];
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+        const int m = m0 + row0 + i * STEP;
+        ab[i] = nullptr;
+        if (m < p.M) {
+            const TA* a = static_cast<const TA*>(p.a);
+            if (MODE == A_ROWS) {
+                ab[i] = a + (long long)m * p.lda;
+            } else {
+                const int b = m / p.rows_per_batch, r = m - b * p.rows_per_batch;
+                ab[i] = a + ((long long)b * p.T + (p.cand ? p.cand[r] : r)) * p.lda;
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+        const int n = n0 + row0 + i * STEP;
+        wb[i] = n < p.N ? static_cast<const T*>(p.w) + (long long)n * p.ldw : nullptr;
+    }
+    const bool avec = p.a_vec, wvec = p.w_vec;
+
+    Four<TA> fa[NA];
+    Four<T> fb[NB];
+    auto fetch = [&](int step) {
+        const int kk = step * BK + piece * 4, left = p.Kd - kk;
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            fa[i].none();
+            if (ab[i] && left > 0) fa[i].load(ab[i] + kk, left, avec);
+        }
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            fb[i].none();
+            if (wb[i] && left > 0) fb[i].load(wb[i] + kk, left, wvec);
+        }
+    };
+    auto stage = [&](int slot) {
+        float* t = gs + slot * (BM + BN) * BK;
+#pragma unroll
+        for (int i = 0; i < NA; ++i)
+            *reinterpret_cast<float4*>(t + place_piece<BM, TM>(row0 + i * STEP, piece)) = fa[i].get();
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+            *reinterpret_cast<float4*>(t + place_piece<BM, TM>(BM + row0 + i * STEP, piece)) = fb[i].get();
+    };
+
+    float acc[TM][TN];
+    const T* bias = static_cast<const T*>(p.bias);
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+        const int n = n0 + tx * 4 + j;
+        const float init = p.bias_first && bias && n < p.N ? to_f32<T>(bias[n]) : 0.f;
+#pragma unroll
+        for (int i = 0; i < TM; ++i) acc[i][j] = init;
+    }
+    const int steps = (p.Kd + BK - 1) / BK;
+    fetch(0);
+    stage(0);
+    __syncthreads();
+    for (int step = 0; step < steps; ++step) {
+        const bool more = step + 1 < steps;
+        if (more) fetch(step + 1);
+        multiply_step<BM, TM, TN>(gs + (step & 1) * (BM + BN) * BK, ty, tx, acc);
+        if (more) {
+            stage((step + 1) & 1);
+            __syncthreads();
+        }
+    }
+    store_outputs<T, TM, 1, 4>(
         p, n0 + tx * 4, 0, [&](int i) { return m0 + ty * TM + i; },
         [&](int i, int, float (&r)[4]) {
 #pragma unroll
@@ -445,6 +582,16 @@ int launch_tile(const GemmParams& p, cudaStream_t st) {
     return CONVNN_OK;
 }
 
+template <typename TA, typename T, int MODE, int BM, int BN, int TM, int TN, int MINB>
+int launch_stage_tile(const GemmParams& p, cudaStream_t st) {
+    const dim3 grid((p.M + BM - 1) / BM, (p.N + BN - 1) / BN);
+    const size_t smem = (size_t)2 * (BM + BN) * 32 * 4;
+    auto kern = gemm_simt_stage_kernel<TA, T, MODE, BM, BN, TM, TN, MINB>;
+    CONVNN_ENSURE_SMEM(kern, smem);
+    kern<<<grid, (BM / TM) * (BN / TN), smem, st>>>(p);
+    return CONVNN_OK;
+}
+
 template <int MODE, int BM, int BN, int TM, int TN, int MINB>
 int launch_copy_tile(const GemmParams& p, cudaStream_t st) {
     const dim3 grid((p.M + BM - 1) / BM, (p.N + BN - 1) / BN);
@@ -455,18 +602,36 @@ int launch_copy_tile(const GemmParams& p, cudaStream_t st) {
     return CONVNN_OK;
 }
 
-// float32 plain rows: the tile with the shortest time on the busiest SM, which runs `fit` tiles at a time.  `step` is
-// what a k step takes there with 1, 2, ... tiles side by side, ns: a tile of two warps leaves two of the four schedulers
-// idle, so tiles come in pairs.  Fitted to 396 shapes (65 to 25216 rows, 10 to 2304 columns, 64 to 1536 values of k; rms 3 to 7 %);
-// the choice is within 0.6 % of the best of twelve tiles on average, 12 % at worst.  With the first two tiles alone
-// (and smaller transposed ones, since gone) 2080 rows took 33.0 us at 192 x 768, now 25.8; 20.6 at 576 x 192, now 17.8;
-// 1576 x 384 x 192 15.5, now 11.5; 1050 x 384 x 384 18.7, now 15.6.
+// Plain rows: the tile with the shortest time on the busiest SM, which runs `fit` tiles at a time.  `step` is what a k
+// step takes there with 1, 2, ... tiles side by side, ns.  The numbers are fits to measured times (rms 3 to 7 %).
+struct Tile {
+    int bm, bn, fit;
+    double launch, round, step[6];        // us per launch and per round of tiles
+};
+template <int COUNT>
+int cheapest_tile(const Tile (&tiles)[COUNT], const GemmParams& p, int first = 0) {
+    const long long sms = device_sms();
+    int best = first;
+    double least = 0;
+    for (int i = first; i < COUNT; ++i) {
+        const Tile& t = tiles[i];
+        if (t.bn < 64 && (p.N + t.bn - 1) / t.bn > 65535) continue;      // (grid rows)
+        const long long n = (long long)((p.M + t.bm - 1) / t.bm) * ((p.N + t.bn - 1) / t.bn), per_sm = (n + sms - 1) / sms;
+        const long long full = per_sm / t.fit, rest = per_sm % t.fit;
+        double cost = t.launch + (full + (rest ? 1 : 0)) * t.round + 1e-3 * p.Kd * full * t.step[t.fit - 1];
+        if (rest) cost += 1e-3 * p.Kd * t.step[rest - 1];
+        if (i == first || cost < least) { least = cost; best = i; }
+    }
+    return best;
+}
+
+// float32 rows that can be copied.  A tile of two warps leaves two of the four schedulers idle, so tiles come in pairs.
+// Over 396 shapes (65 to 25216 rows, 10 to 2304 columns, 64 to 1536 values of k) the choice is within 0.6 % of the
+// best of twelve tiles on average, 12 % at worst.  With the first two tiles alone (and smaller transposed ones, since
+// gone) 2080 rows took 33.0 us at 192 x 768, now 25.8; 20.6 at 576 x 192, now 17.8; 1576 x 384 x 192 15.5, now 11.5; 1050
+// x 384 x 384 18.7, now 15.6.
 template <int MODE>
 int launch_plain_f32(const GemmParams& p, cudaStream_t st) {
-    struct Tile {
-        int bm, bn, fit;
-        double launch, round, step[6];        // us per launch and per round of tiles
-    };
     static const Tile tiles[6] = {
         {128, 64, 3, 5.4, 0.5, {65.4, 107.1, 153.3}},
         {64, 64, 3, 3.2, 0.7, {38.2, 62.3, 88.9}},
@@ -475,19 +640,7 @@ int launch_plain_f32(const GemmParams& p, cudaStream_t st) {
         {48, 32, 5, 2.2, 2.3, {26.3, 28.8, 42.9, 46.8, 60.0}},
         {56, 32, 5, 1.9, 3.1, {30.2, 32.5, 50.4, 53.8, 72.0}},
     };
-    const long long sms = device_sms();
-    int best = 0;
-    double least = 0;
-    for (int i = 0; i < 6; ++i) {
-        const Tile& t = tiles[i];
-        if (i > 1 && (p.N + t.bn - 1) / t.bn > 65535) continue;      // (grid rows)
-        const long long n = (long long)((p.M + t.bm - 1) / t.bm) * ((p.N + t.bn - 1) / t.bn), per_sm = (n + sms - 1) / sms;
-        const long long full = per_sm / t.fit, rest = per_sm % t.fit;
-        double cost = t.launch + (full + (rest ? 1 : 0)) * t.round + 1e-3 * p.Kd * full * t.step[t.fit - 1];
-        if (rest) cost += 1e-3 * p.Kd * t.step[rest - 1];
-        if (i == 0 || cost < least) { least = cost; best = i; }
-    }
-    switch (best) {
+    switch (cheapest_tile(tiles, p)) {
         case 0: return launch_tile<float, float, MODE, 128, 64, 16, 8, 8, 3>(p, st);
         case 1: return launch_tile<float, float, MODE, 64, 64, 32, 8, 4, 3>(p, st);
         case 2: return launch_copy_tile<MODE, 32, 32, 4, 4, 6>(p, st);
@@ -497,15 +650,32 @@ int launch_plain_f32(const GemmParams& p, cudaStream_t st) {
     }
 }
 
+// Other plain rows (bfloat16, float32 against bfloat16 weights, rows of any alignment).  Over 146 bfloat16 shapes within 1 % of the best
+// of nine tiles on average, 18 % at worst, and 0.71 of the time of the transposed tiles that were here (which waited for
+// their operands to be converted and stored value by value), the first tile only where rows are read four values at a time (4039
+// x 768 x 385 135 us, the second 93); us: 2080 x 384 x 388 57.9, now 27.8; 4039 x 384 x 388 51.9, now 44.3; the separable conv with the coordinate channel (rows of d_k + 1 values) of 7 x 577 tokens, 384 channels 89.8, now 68.1; 4 x 197 x 768
+// 130 -> 55; 197 x 192 29.0 -> 16.3.
 template <typename TA, typename T, int MODE>
-int launch_mode(const GemmParams& p, cudaStream_t st) {
-    // The tile with the least work on the busiest SM: rounds of tiles x outputs per tile over the rate of the tile's
-    // threads.  That rate is set by shared memory: a k step reads TM + TN values per thread for TM * TN multiply-adds
-    // (45, 40, 29 and 26 TFLOP/s at 16384 x 768 x 768; 25 before).  2080 x 192 x 768: 33 us, 50 before; 50432 x 192 x
-    // 192: 89 us, 150 before.
-    if constexpr (sizeof(TA) == 4 && sizeof(T) == 4 && (MODE == A_ROWS || MODE == A_TOKENS)) {
-        if (p.a_vec && p.w_vec) return launch_plain_f32<MODE>(p, st);
+int launch_plain_staged(const GemmParams& p, cudaStream_t st) {
+    static const Tile tiles[4] = {
+        {128, 64, 3, 6.4, 0.0, {124.7, 163.2, 198.0}},
+        {64, 64, 3, 0.8, 5.4, {40.2, 64.4, 95.6}},
+        {32, 64, 4, 0.3, 3.6, {26.9, 45.3, 61.7, 77.4}},
+        {40, 32, 6, 0.0, 5.0, {31.9, 33.6, 49.2, 52.1, 70.4, 70.8}},
+    };
+    switch (cheapest_tile(tiles, p, p.a_vec && p.w_vec ? 0 : 1)) {
+        case 0: return launch_tile<TA, T, MODE, 128, 64, 16, 8, 8, 3>(p, st);
+        case 1: return launch_stage_tile<TA, T, MODE, 64, 64, 8, 4, 3>(p, st);
+        case 2: return launch_stage_tile<TA, T, MODE, 32, 64, 4, 4, 4>(p, st);
+        default: return launch_stage_tile<TA, T, MODE, 40, 32, 5, 4, 6>(p, st);
     }
+}
+
+template <typename TA, typename T, int MODE>
+int launch_other_mode(const GemmParams& p, cudaStream_t st) {
+    // Implicit operands and the flat head reinterpretation: the tile with the least work on the busiest SM, rounds of tiles x
+    // outputs per tile over the rate of the tile's threads.  That rate is set by shared memory: a k step reads TM + TN values per
+    // thread for TM * TN multiply-adds (45, 40, 29 and 26 TFLOP/s with plain rows at 16384 x 768 x 768).
     const long long sms = device_sms();
     long long tiles_of[4];
     auto cost = [&](int i, int bm, int bn, double rate) {
@@ -530,7 +700,7 @@ int launch_mode(const GemmParams& p, cudaStream_t st) {
     // Tap rows of C values against more stored channels (the coordinate channel) come value by value: in bfloat16 they gain longest, longer
     // still where an odd number of taps leaves every other row of them at an odd address.  64 x 64, 4: 64 x 197 x 192 617 -> 375; 3: 24 x 197 x
     // 384, 9 taps 726 -> 615, 24 x 577 x 96, 8 taps 123 -> 151 (not taken); 32 x 32, 7: 159 x 65 x 96, 25 taps 741 -> 391, 6 and one column
-    // of tiles: 48 x 577 x 20, 16 taps 58 -> 63 (not taken).  Plain rows lose up to 20 %.
+    // of tiles: 48 x 577 x 20, 16 taps 58 -> 63 (not taken).
     if constexpr (MODE == A_NEIGHBOURS || MODE == A_CONV1D) {
         const long long per_sm = (tiles_of[best] + sms - 1) / sms, here = best == 3 ? 4 : 2, other = best == 3 ? 7 : 3;
         bool twice = (per_sm + here - 1) / here <= (per_sm + other - 1) / other;
@@ -552,6 +722,18 @@ int launch_mode(const GemmParams& p, cudaStream_t st) {
     if (best == 1) return launch_tile<TA, T, MODE, 64, 64, 32, 8, 4, 3>(p, st);
     if (best == 2) return launch_tile<TA, T, MODE, 32, 64, 64, 4, 4, 2>(p, st);
     return launch_tile<TA, T, MODE, 32, 32, 32, 4, 4, 4>(p, st);
+}
+
+template <typename TA, typename T, int MODE>
+int launch_mode(const GemmParams& p, cudaStream_t st) {
+    if constexpr (MODE == A_ROWS || MODE == A_TOKENS) {
+        if constexpr (sizeof(TA) == 4 && sizeof(T) == 4) {
+            if (p.a_vec && p.w_vec) return launch_plain_f32<MODE>(p, st);
+        }
+        return launch_plain_staged<TA, T, MODE>(p, st);
+    } else {
+        return launch_other_mode<TA, T, MODE>(p, st);
+    }
 }
 
 template <typename T>

@@ -269,3 +269,30 @@ def test_three_outputs_of_float32_rows(B, T, S, D, H):
     xq = x if cand is None else x[:, cand.long()]
     for got, rows, part in ((k, x, 0), (v, x, 1), (q, xq, 2)):
         assert torch.equal(got.reshape(-1, D), ops.linear(rows.reshape(-1, D), w[part]))
+
+
+# Every tile of the rows that come through registers: bfloat16 with k a multiple of four (read four at a time) and not, and
+# float32 rows that are not 16-byte aligned; a sum is the same whichever tile it was computed in.
+@on_148_sms
+@pytest.mark.parametrize("M,N,K,tile", [
+    (1, 1, 1, "32x64 4x4"), (65, 193, 385, "32x64 4x4"), (1050, 384, 388, "32x64 4x4"), (788, 768, 772, "40x32 5x4"),
+    (1576, 191, 196, "40x32 5x4"), (4039, 384, 385, "64x64 8x4"), (12001, 384, 197, "64x64 8x4"), (50433, 66, 65, "64x64 8x4"),
+    (50433, 66, 68, "transposed")])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_tiles_of_staged_rows(M, N, K, tile, dtype):
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    ld = K + (1 if dtype == torch.float32 or K % 4 else 4)           # (odd row strides keep float32 off the copies)
+    a, w, b, r = (torch.randn(*s, device=DEV, generator=g).to(dtype) for s in ((M, ld), (N, K), (N,), (M, N)))
+    a = a[:, :K]
+    call = lambda: ops.linear(a, w, b, residual=r)
+    names = [re.search(r"gemm_simt_stage_kernelI.*?Li\dELi(\d+)ELi(\d+)ELi(\d+)ELi(\d+)E", n) for n in launches(call)]
+    if dtype == torch.float32 and tile == "transposed":
+        tile = "64x64 8x4"
+    assert [("{}x{} {}x{}".format(*m.groups()) if m else "transposed") for m in names] == [tile]
+    got = call()
+    want = a.double() @ w.double().T + b.double()
+    step = 2.0 ** -8 if dtype == torch.bfloat16 else 2 * EPS         # the sum is rounded, then the skip connection added
+    bound = _bound(a, w, K) + 2 * EPS * b.abs() + step * (want.abs() + (want + r.double()).abs())
+    assert bool(((got.double() - want - r.double()).abs() <= bound).all())
+    some = torch.randperm(M, device=DEV, generator=g)[:20]
+    assert torch.equal(ops.linear(a[some], w, b, residual=r[some]), got[some])
