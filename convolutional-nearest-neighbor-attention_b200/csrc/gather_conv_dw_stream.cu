@@ -77,12 +77,6 @@ gather_conv_dw_stream_kernel(const __grid_constant__ CUtensorMap tmV, const DwsP
     __syncthreads();
     chain_begin();
 
-    // tap weights of this thread's 8 channels, as packed pairs
-    f32x2 w2[KT][4];
-#pragma unroll
-    for (int j = 0; j < KT; ++j)
-        bf16x8_to_f32x2(*reinterpret_cast<const uint4*>(p.wconv + j * p.dk + c0 + cg * 8), w2[j]);
-
     auto issue = [&](int slice, int buf) {
         const int b = slice / p.H, h = slice - b * p.H;
         if (threadIdx.x == 0) {
@@ -100,6 +94,13 @@ gather_conv_dw_stream_kernel(const __grid_constant__ CUtensorMap tmV, const DwsP
 
     int slice = lane_cta;
     if (slice < p.n_slices) issue(slice, 0);
+
+    // tap weights of this thread's 8 channels, as packed pairs
+    f32x2 w2[KT][4];
+#pragma unroll
+    for (int j = 0; j < KT; ++j)
+        bf16x8_to_f32x2(*reinterpret_cast<const uint4*>(p.wconv + j * p.dk + c0 + cg * 8), w2[j]);
+
     for (uint32_t it = 0; slice < p.n_slices; slice += p.ctas_per_chunk, ++it) {
         const uint32_t buf = it & 1u;
         const int next = slice + p.ctas_per_chunk;

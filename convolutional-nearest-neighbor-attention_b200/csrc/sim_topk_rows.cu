@@ -49,6 +49,7 @@ struct RowsParams {
     int stages;
     int rows_total, rows_per_cta, per_head;
     float sqrt_dk;
+    int box_rows;                  // key rows fetched per segment
 };
 
 __device__ __forceinline__ void fail(volatile int* abort_flag, int code) {
@@ -153,6 +154,7 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t pitch = p.KCH * 2;
     const uint32_t a_bytes = BM * pitch, b_bytes = p.BN * pitch, stage_bytes = a_bytes + b_bytes;
+    const uint32_t landing = p.box_rows * pitch + b_bytes;    // (rows past the CTA's range stay whatever they were: no sum uses them)
     const uint32_t STAGES = p.stages;
     float* keybuf = reinterpret_cast<float*>(smem + STAGES * stage_bytes);      // [seg_rows][pitch]
     float2* lists = reinterpret_cast<float2*>(keybuf + p.seg_rows * p.pitch);   // [NW][WR][K] key, column
@@ -192,13 +194,14 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_begin();
+    // (every role waits for the predecessor before its own first access to global memory)
 
     const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty), st0 = smem_u32(smem);
     if (warp == 0) {
         if (lane < 2) {                              // lane 0: key rows, lane 1: candidate rows (their copies overlap)
             uint32_t s = 0, ph = 0;
             bool ok = true;
+            chain_wait();
             for (Segment sg(p); sg.valid() && ok; sg.next(p)) {
                 const int b = sg.bh / p.H, h = sg.bh - b * p.H;
                 for (int kc = 0; kc < p.KC; ++kc) {
@@ -206,7 +209,7 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
                     ok = __all_sync(0x3u, ok);
                     if (!ok) { if (lane == 0) fail(abort_flag, 81); break; }
                     const uint32_t st = st0 + s * stage_bytes, fb = full0 + 8 * s;
-                    if (lane == 0) mbar_expect_tx_a(fb, stage_bytes);
+                    if (lane == 0) mbar_expect_tx_a(fb, landing);
                     __syncwarp(0x3u);
                     if (lane == 0) tma_load_4d_a(st, &tmK, fb, kc * p.KCH, h, sg.row, b);
                     else tma_load_4d_a(st + a_bytes, &tmQ, fb, kc * p.KCH, h, 0, b);
@@ -248,10 +251,6 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         const uint32_t found0 = smem_u32(found + w * found_pairs(NS));
         const RowsTask task{kst_s, cs, p.idx, p.val, p.pitch, p.BN, p.nsel, p.K, p.inv_K, p.metric, p.sampled, p.sqrt_dk};
         const bool stats = p.metric != CONVNN_MATMUL;
-        if (p.sampled)
-            for (int c = tid; c < p.BN; c += 32 * NW) cs[c] = c < p.S ? p.cand[c] : -1;
-        if (GATHER)                                  // (read behind the barriers of the first segment)
-            for (int c = tid; c < p.K * p.groups; c += 32 * NW) taps[c] = p.w[c];
         uint32_t buf = 0, use = 0;
         const float none = __int_as_float(0x7fffffff);           // columns past the last candidate: their keys become NaN
         // Every selection warp makes the same number of passes and meets every barrier, also after a wait has expired
@@ -262,7 +261,13 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             if (tid < p.S) q_next = stats ? p.qstat[(long long)sg.bh * p.S + tid] : 1.f;
             if (stats && r < sg.n) kst_next = p.kstat[sg.g + r];
         };
+        chain_wait();
+        chain_next();
         if (sg.valid()) fetch();
+        if (p.sampled)                               // (this and the taps are read behind the barriers of the first segment)
+            for (int c = tid; c < p.BN; c += 32 * NW) cs[c] = c < p.S ? p.cand[c] : -1;
+        if (GATHER)
+            for (int c = tid; c < p.K * p.groups; c += 32 * NW) taps[c] = p.w[c];
         while (sg.valid()) {
             const float kst = kst_next;
             if (tid < p.BN) qs[tid] = q_next;
@@ -470,7 +475,9 @@ static int launch_impl(const convnn_desc* d, const Dims& dm, const void* q, cons
     const uint64_t dimsQ[4] = {(uint64_t)dm.Cp, (uint64_t)dm.H, (uint64_t)dm.S, (uint64_t)dm.B};
     const uint64_t strK[3] = {(uint64_t)dm.Cp * 2, (uint64_t)dm.H * dm.Cp * 2, (uint64_t)dm.T * dm.H * dm.Cp * 2};
     const uint64_t strQ[3] = {(uint64_t)dm.Cp * 2, (uint64_t)dm.H * dm.Cp * 2, (uint64_t)dm.S * dm.H * dm.Cp * 2};
-    const uint32_t boxK[4] = {(uint32_t)p.KCH, 1, (uint32_t)BM, 1};
+    // (a box of the CTA's rows alone: with 16 of them 86 KB land where 128 did)
+    p.box_rows = (p.seg_rows + 7) / 8 * 8;
+    const uint32_t boxK[4] = {(uint32_t)p.KCH, 1, (uint32_t)p.box_rows, 1};
     const uint32_t boxQ[4] = {(uint32_t)p.KCH, 1, (uint32_t)p.BN, 1};
     if (!encode_tensor_map_bf16(&tmK, k, 4, dimsK, strK, boxK, p.KCH * 2)) return CONVNN_E_CUDA;
     if (!encode_tensor_map_bf16(&tmQ, q, 4, dimsQ, strQ, boxQ, p.KCH * 2)) return CONVNN_E_CUDA;

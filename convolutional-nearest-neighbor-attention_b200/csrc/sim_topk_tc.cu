@@ -109,7 +109,7 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_begin();
+    // (every role waits for the predecessor before its own first access to global memory)
 
     const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty);
     const uint32_t st0 = smem_u32(stages);
@@ -122,6 +122,7 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
             const uint32_t m3 = 0x7u;
             uint32_t s = 0, ph = 0;                  // ring slot and phase, advanced incrementally
             bool ok = true;
+            chain_wait();
             for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x) {
                 const int bh = unit / p.n_pairs, pp = unit - bh * p.n_pairs;
                 const int b = bh / p.H, h = bh - b * p.H;
@@ -186,6 +187,8 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         float* sq = statbuf + (warp - 2) * 128;
         uint32_t tile = 0;
         bool ok = true;
+        chain_wait();
+        chain_next();
         for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x) {
             const int bh = unit / p.n_pairs, pp = unit - bh * p.n_pairs;
             const int row = pp * 2 * BM + grp * BM + r;
