@@ -286,45 +286,73 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t sA0 = smem_u32(sA), sB0 = smem_u32(sB);
 
     if (warp == 0) {
+        // One thread can start a TMA operation only every ~0.3 us, while operations started by different lanes overlap: a first
+        // tile of few chunks, all of which its products wait for, is requested by as many lanes (a small GEMM is little more
+        // than that), the rest by lane 0.  With more chunks the first would land later (K = 384 0.6 us per launch).
+        const uint32_t tx = (a_bytes + (p.wstat ? 0u : b_bytes)) * (PAIR ? 2u : 1u);
+        const uint32_t lead_full0 = PAIR ? map_to_cta(full0, 0) : full0;
+        auto load_a = [&](uint32_t slot, int kc, int m0) {
+            if (PAIR) tma_load_2d_pair(sA0 + slot * a_bytes, &tmA, lead_full0 + 8 * slot, kc * p.KCH, m0);
+            else tma_load_2d_a(sA0 + slot * a_bytes, &tmA, full0 + 8 * slot, kc * p.KCH, m0);
+        };
+        auto load_w_chunk = [&](uint32_t slot, int kc, int n0) {
+            if (PAIR) tma_load_2d_pair(sB0 + slot * b_bytes, &tmW, lead_full0 + 8 * slot, kc * p.KCH, n0);
+            else if (!p.wstat) tma_load_2d_a(sB0 + slot * b_bytes, &tmW, full0 + 8 * slot, kc * p.KCH, n0);
+        };
+        int cur_nt = -1;
+        const int lead = first < last && p.KC <= 4 ? min(p.KC, (int)STAGES) : 0;     // chunks of the first tile requested at once
+        int w_ahead = 0;                                                // chunks of W alone that lane 0 requests early
+        if (lead > 0) {
+            int mt, nt;
+            tile_mn(first, mt, nt);
+            const int m0 = mt * TM + (int)rank * BM, n0 = nt * p.BN + (int)rank * bn_cta;
+            auto request_w = [&]() {                                     // W of the first tile, or its chunks in the ring
+                if (p.wstat) {
+                    if (lane == 0) mbar_expect_tx_a(wfull_a, p.KC * b_bytes + (LNF ? (uint32_t)bn_cta * 32u : 0u));
+                    __syncwarp();
+                    if (lane < p.KC) tma_load_2d_a(sB0 + lane * b_bytes, &tmW, wfull_a, lane * p.KCH, nt * p.BN);
+                    if (LNF && lane == 31) tma_load_2d_a(smem_u32(xb), &tmX, wfull_a, 0, nt * p.BN);
+                    cur_nt = nt;
+                } else if (lane < lead) {
+                    load_w_chunk((uint32_t)lane, lane, n0);
+                }
+                __syncwarp();
+            };
+            if (lane < lead && (!PAIR || rank == 0)) mbar_expect_tx_a(full0 + 8 * lane, tx);
+            if (p.w_at_rest) request_w();                                // before the predecessor has ended
+            chain_wait();
+            if (!p.w_at_rest) request_w();
+            if (lane < lead) load_a((uint32_t)lane, lane, m0);
+            __syncwarp();
+        }
         if (lane == 0) {
-            uint32_t s = 0, ph = 0, wloads = 0;      // ring slot and its phase, advanced incrementally
-            uint32_t last_s = 0, last_ph = 0;
-            bool any = false;
-            int cur_nt = -1;
+            uint32_t s = lead == (int)STAGES ? 0u : (uint32_t)lead, ph = lead == (int)STAGES ? 1u : 0u;   // ring slot and its phase
+            uint32_t last_s = lead > 0 ? (uint32_t)lead - 1u : 0u, last_ph = 0;
+            int skip = lead;                                             // chunks of the first tile that are on the way
             bool ok = true;
             const bool tr = !PAIR && trace_enabled() && blockIdx.x == 0;
             int tn = 0;
             trace(tr, 0, tn);
-            const uint32_t tx = (a_bytes + (p.wstat ? 0u : b_bytes)) * (PAIR ? 2u : 1u);
-            const uint32_t lead_full0 = PAIR ? map_to_cta(full0, 0) : full0;
             auto load_w_tile = [&](int nt) {
                 mbar_expect_tx_a(wfull_a, p.KC * b_bytes + (LNF ? (uint32_t)bn_cta * 32u : 0u));
-                for (int kc = 0; kc < p.KC; ++kc)
-                    tma_load_2d_a(sB0 + kc * b_bytes, &tmW, wfull_a, kc * p.KCH, nt * p.BN);
+                for (int kc = 0; kc < p.KC; ++kc) tma_load_2d_a(sB0 + kc * b_bytes, &tmW, wfull_a, kc * p.KCH, nt * p.BN);
                 if (LNF) tma_load_2d_a(smem_u32(xb), &tmX, wfull_a, 0, nt * p.BN);
                 cur_nt = nt;
-                ++wloads;
             };
-            auto load_w_chunk = [&](uint32_t slot, int kc, int n0) {
-                if (PAIR) tma_load_2d_pair(sB0 + slot * b_bytes, &tmW, lead_full0 + 8 * slot, kc * p.KCH, n0);
-                else if (!p.wstat) tma_load_2d_a(sB0 + slot * b_bytes, &tmW, full0 + 8 * slot, kc * p.KCH, n0);
-            };
-            // W of the first tile, or as many of its chunks as the ring holds, before the predecessor has ended
-            int w_ahead = 0;
-            if (p.w_at_rest && first < last) {
-                int mt, nt;
-                tile_mn(first, mt, nt);
-                if (p.wstat) {
-                    load_w_tile(nt);
-                } else {
-                    w_ahead = min(p.KC, (int)STAGES);
-                    for (int kc = 0; kc < w_ahead; ++kc) {
-                        if (!PAIR || rank == 0) mbar_expect_tx_a(full0 + 8 * kc, tx);
-                        load_w_chunk((uint32_t)kc, kc, nt * p.BN + (int)rank * bn_cta);
-                    }
+            if (lead == 0 && first < last) {
+                if (p.w_at_rest) {                                       // W of the first tile, or as many of its chunks as the ring holds
+                    int mt, nt;
+                    tile_mn(first, mt, nt);
+                    if (p.wstat) load_w_tile(nt);
+                    else
+                        for (w_ahead = 0; w_ahead < min(p.KC, (int)STAGES); ++w_ahead) {
+                            if (!PAIR || rank == 0) mbar_expect_tx_a(full0 + 8 * w_ahead, tx);
+                            load_w_chunk((uint32_t)w_ahead, w_ahead, nt * p.BN + (int)rank * bn_cta);
+                        }
                 }
+                chain_wait();
             }
-            chain_wait();
+            bool any = lead > 0;
             for (int t = first; t < last && ok; t += step) {
                 int mt, nt;
                 tile_mn(t, mt, nt);
@@ -336,12 +364,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
                 trace(tr, 0, tn);
                 const int m0 = mt * TM + (int)rank * BM, n0 = nt * p.BN + (int)rank * bn_cta;
-                for (int kc = 0; kc < p.KC; ++kc) {
+                const int kc0 = skip;
+                skip = 0;
+                for (int kc = kc0; kc < p.KC; ++kc) {
                     if (!mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag)) { give_up(11); ok = false; break; }
                     const bool whole = w_ahead == 0;            // (otherwise its W chunk is on the way)
                     if (whole && (!PAIR || rank == 0)) mbar_expect_tx_a(full0 + 8 * s, tx);
-                    if (PAIR) tma_load_2d_pair(sA0 + s * a_bytes, &tmA, lead_full0 + 8 * s, kc * p.KCH, m0);
-                    else tma_load_2d_a(sA0 + s * a_bytes, &tmA, full0 + 8 * s, kc * p.KCH, m0);
+                    load_a(s, kc, m0);
                     if (whole) load_w_chunk(s, kc, n0);
                     else --w_ahead;
                     last_s = s; last_ph = ph; any = true;

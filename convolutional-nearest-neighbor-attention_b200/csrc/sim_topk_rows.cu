@@ -94,6 +94,15 @@ __device__ __forceinline__ void conv_rows(const RowsParams& p, float2* list, con
     const int lane = threadIdx.x & 31, b = bh / p.H, h = bh - b * p.H;
     const bool maximum = p.metric != CONVNN_EUCLIDEAN;
     const int vbase = (b * p.T * p.H + h) * p.groups, vstride = p.H * p.groups;      // (B T D < 2^31)
+    // the lane's first neighbour rows are on their way while the weights are made
+    uint4 raw[TAPS];
+    if (lane < n * p.groups) {
+        const int m = lane / p.groups, cg = lane - m * p.groups;
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j)
+            if (j < p.K) raw[j] = __ldg(p.v + vbase + __float_as_int(list[m * p.K + j].y) * vstride + cg);
+    }
+    __syncwarp();                                   // (the entries are rewritten below)
     for (int m0 = 0; m0 < n; m0 += 2) {             // two rows, sixteen lanes each (K <= 17: a lane more holds the last)
         const int j = lane & 15, m = m0 + (lane >> 4);
         const bool in = m < n && j < p.K, last = p.K > 16 && m < n && j == 15;
@@ -125,10 +134,11 @@ __device__ __forceinline__ void conv_rows(const RowsParams& p, float2* list, con
         const float2* l = list + m * p.K;
         f32x2 acc[4] = {0ull, 0ull, 0ull, 0ull};
         for (int j0 = 0; j0 < p.K; j0 += TAPS) {
-            uint4 raw[TAPS];
+            if (e != lane || j0 != 0) {
 #pragma unroll
-            for (int j = 0; j < TAPS; ++j)
-                if (j0 + j < p.K) raw[j] = __ldg(p.v + __float_as_int(l[j0 + j].y) + cg);
+                for (int j = 0; j < TAPS; ++j)
+                    if (j0 + j < p.K) raw[j] = __ldg(p.v + __float_as_int(l[j0 + j].y) + cg);
+            }
 #pragma unroll
             for (int j = 0; j < TAPS; ++j)
                 if (j0 + j < p.K) {
@@ -198,13 +208,28 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
 
     const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty), st0 = smem_u32(smem);
     if (warp == 0) {
-        if (lane < 2) {                              // lane 0: key rows, lane 1: candidate rows (their copies overlap)
-            uint32_t s = 0, ph = 0;
+        // One thread can start a TMA operation only every ~0.3 us, while operations started by different lanes overlap: a lane
+        // per box of the first segment's chunks; from then on lane 0 brings key rows, lane 1 candidate rows.
+        static_assert(MAX_STAGES <= 8, "lanes 8 ... bring the candidate rows");
+        Segment sg(p);
+        const int lead = sg.valid() ? min(p.KC, (int)STAGES) : 0;
+        if (lane < lead) mbar_expect_tx_a(full0 + 8 * lane, landing);
+        __syncwarp();
+        chain_wait();
+        if (lead > 0) {
+            const int b = sg.bh / p.H, h = sg.bh - b * p.H, kc = lane & 7;
+            const uint32_t st = st0 + kc * stage_bytes, fb = full0 + 8 * kc;
+            if (kc < lead && lane < 8) tma_load_4d_a(st, &tmK, fb, kc * p.KCH, h, sg.row, b);
+            else if (kc < lead && lane < 16) tma_load_4d_a(st + a_bytes, &tmQ, fb, kc * p.KCH, h, 0, b);
+        }
+        __syncwarp();
+        if (lane < 2) {
+            uint32_t s = lead == (int)STAGES ? 0u : (uint32_t)lead, ph = lead == (int)STAGES ? 1u : 0u;
+            int kc0 = lead;
             bool ok = true;
-            chain_wait();
-            for (Segment sg(p); sg.valid() && ok; sg.next(p)) {
+            for (; sg.valid() && ok; sg.next(p), kc0 = 0) {
                 const int b = sg.bh / p.H, h = sg.bh - b * p.H;
-                for (int kc = 0; kc < p.KC; ++kc) {
+                for (int kc = kc0; kc < p.KC; ++kc) {
                     ok = mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag);
                     ok = __all_sync(0x3u, ok);
                     if (!ok) { if (lane == 0) fail(abort_flag, 81); break; }
