@@ -321,7 +321,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 template <typename T>
 __global__ void attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                                       T* __restrict__ o, int Tn, int H, int dk, float scale) {
-    chain_begin();
+    chain_begin_for<T>();
     extern __shared__ float sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     float* prob = sm + warp * (Tn + dk);

@@ -43,7 +43,7 @@ __global__ void conv1d_unfold_kernel(const T* __restrict__ y, T* __restrict__ u,
 template <typename T>
 __global__ void conv1d_simt_kernel(const T* __restrict__ y, const T* __restrict__ w, const T* __restrict__ bias,
                                    T* __restrict__ o, int Tn, int H, int dk, int ks, int pad, long long total) {
-    chain_begin();
+    chain_begin_for<T>();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
         const int oc = (int)(i % dk);

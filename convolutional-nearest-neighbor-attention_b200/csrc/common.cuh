@@ -47,6 +47,14 @@ __device__ __forceinline__ void chain_begin() {
     chain_wait();
     chain_next();
 }
+// float32 kernels (and what runs between them) never let their successor start early: it starts as their last CTAs leave.  Their
+// chains end in grids of many small CTAs, which would pile up on the SMs that are free first and wait there (ViT-Tiny
+// float32 1970 -> 2430 us), while a plain launch costs the gap.
+template <typename T>
+__device__ __forceinline__ void chain_begin_for() {
+    chain_wait();
+    if (sizeof(T) != 4) chain_next();
+}
 // Under capture the launch is a plain one: a graph's own launches are cheap, its kernels overlap across branches already
 // (two batches in flight, 128 launches: 2844 us with chained edges, 2831 us without), and instantiating chained edges
 // took the host 0.3 s.
@@ -65,6 +73,13 @@ void launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cuda
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cfg.attrs = attr; cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);   // an error stays the thread's last error (CONVNN_CHECK_LAUNCH)
+}
+
+// A float32 kernel in its chain; the same kernel for bfloat16, whose predecessors let it start early, by a plain launch.
+template <typename T, class... P, class... A>
+void launch_by_type(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+    if (sizeof(T) == 4) launch_chained(kern, grid, block, smem, st, args...);
+    else kern<<<grid, block, smem, st>>>(static_cast<P>(args)...);
 }
 
 // SM count of the current device, asked once per device.

@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const T* __restrict__ x,
                                                         float eps, T* __restrict__ y, long long ldy, long long rows,
                                                         int D, const T* __restrict__ pe, const T* __restrict__ cls,
                                                         int Np, long long cls_rows, float2* __restrict__ moments) {
-    chain_begin();
+    chain_begin_for<T>();
     // moments (or nullptr): (sum, sum of squares) of every STORED output row, indexed by output row: what the
     // pre-norm fold of the first GEMM behind the embedding needs
     constexpr int V = Vec16<T>::N;
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(256, MINB) layernorm_bf16_row256_kernel(
 template <typename T, typename VT>
 __global__ void __launch_bounds__(256) patchify_kernel(const T* __restrict__ img, T* __restrict__ out, int C, int Hh,
                                                        int Ww, int P) {
-    chain_begin();
+    chain_begin_for<T>();
     // One CTA per (image, row of patches): C * P image rows of Ww elements, read in image order
     // (whole rows, coalesced) and stored as the P-element runs of the patches' rows.  The index
     // arithmetic is 32-bit inside the strip; four vectors per thread are in flight.
@@ -439,7 +439,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(256) patchify_u8_kernel(const uint8_t* __restrict__ img, const float* __restrict__ mean,
                                                           const float* __restrict__ inv_std, T* __restrict__ out, int C,
                                                           int Hh, int Ww, int P) {
-    chain_begin();
+    chain_begin_for<T>();
     constexpr int U = VEC == 8 ? 4 : 8;
     const int Hp = Hh / P, Wp = Ww / P;
     const int b = blockIdx.x / Hp, py = blockIdx.x - b * Hp;

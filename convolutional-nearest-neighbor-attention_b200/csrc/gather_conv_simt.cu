@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(THREADS) gather_conv_dw_scalar_kernel(
     const T* __restrict__ v, const int32_t* __restrict__ idx, const float* __restrict__ val,
     const T* __restrict__ wconv, T* __restrict__ o, int T_, int H, int dk, int Cp, int K, int maximum,
     int softmax) {
-    chain_begin();
+    chain_begin_for<T>();
     __shared__ float ps[TT][kMaxK];
     __shared__ int ns[TT][kMaxK];
     const int bh = blockIdx.y;
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(THREADS) gather_conv_mat_kernel(
     const T* __restrict__ v, const int32_t* __restrict__ idx, const float* __restrict__ val,
     const T* __restrict__ wconv, const T* __restrict__ wpw, T* __restrict__ o, int T_, int H, int dk,
     int C, int Cp, int K, int maximum, int softmax, int separable, int TT, int JC) {
-    chain_begin();
+    chain_begin_for<T>();
     extern __shared__ __align__(16) float P[];
     __shared__ float ps[32][kMaxK];
     __shared__ int ns[32][kMaxK];

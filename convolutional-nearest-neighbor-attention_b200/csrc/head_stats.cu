@@ -29,7 +29,7 @@ struct HeadTensors {
 
 template <typename T>
 __global__ void __launch_bounds__(256, 6) head_stats_kernel(const HeadTensors in, int B, int H, int dk, int C, int Cp, int coord, int metric) {
-    chain_begin();
+    chain_begin_for<T>();
     const int which = blockIdx.y;
     T* t = static_cast<T*>(which == 0 ? in.t[0] : which == 1 ? in.t[1] : in.t[2]);
     float* stat = which == 0 ? in.stat[0] : which == 1 ? in.stat[1] : in.stat[2];

@@ -13,7 +13,7 @@ namespace {
 template <typename T>
 __global__ void gather_rows_kernel(const T* __restrict__ x, long long ldx, const int32_t* __restrict__ cand,
                                    T* __restrict__ xq, int Tn, int S, int D, long long total_vec, int vec) {
-    chain_begin();
+    chain_begin_for<T>();
     const int per_row = D / vec;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total_vec;
          i += (long long)gridDim.x * blockDim.x) {
@@ -34,7 +34,7 @@ __global__ void gather_rows_kernel(const T* __restrict__ x, long long ldx, const
 // Sequences of which eight channels exceed shared memory: 32 x 32 tiles.
 template <typename T>
 __global__ void merge_heads_tile_kernel(const T* __restrict__ o, T* __restrict__ y, int Tn, int H, int dk, int D) {
-    chain_begin();
+    chain_begin_for<T>();
     __shared__ T tile[32][33];
     const int bh = blockIdx.z;
     const int b = bh / H, h = bh - b * H;
@@ -57,7 +57,7 @@ __global__ void merge_heads_tile_kernel(const T* __restrict__ o, T* __restrict__
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) merge_heads_kernel(const T* __restrict__ o, T* __restrict__ y, int Tn, int H, int dk,
                                                           int D, int CB) {
-    chain_begin();
+    chain_begin_for<T>();
     extern __shared__ __align__(16) unsigned char mh_smem[];
     T* s = reinterpret_cast<T*>(mh_smem);                 // [CB][Tn]
     constexpr int PER = 16 / sizeof(T);
