@@ -349,7 +349,7 @@ int qkv_proj_impl(const convnn_desc* d, const void* x, int64_t ldx, const void* 
     if ((rc = launch_gemm_simt(d->dtype, p, st))) return rc;
     if (d->sampled) {
         p.cand = cand; p.rows_per_batch = dm.S; p.M = dm.B * dm.S; p.N = dm.D;
-        p.w = static_cast<const char*>(w_qkv) + 2 * wsz; p.c = q; p.c1 = nullptr;
+        p.w = static_cast<const char*>(w_qkv) + 2 * wsz; p.c = q; p.c1 = nullptr; p.chained = 1;
         if ((rc = launch_gemm_simt(d->dtype, p, st))) return rc;
     }
     return launch_head_fill_and_stats(d, dm, q, stats ? qstat : nullptr, k, stats ? kstat : nullptr, v, st);

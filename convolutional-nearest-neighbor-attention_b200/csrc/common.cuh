@@ -75,10 +75,11 @@ void launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cuda
     cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);   // an error stays the thread's last error (CONVNN_CHECK_LAUNCH)
 }
 
-// A float32 kernel in its chain; the same kernel for bfloat16, whose predecessors let it start early, by a plain launch.
-template <typename T, class... P, class... A>
-void launch_by_type(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
-    if (sizeof(T) == 4) launch_chained(kern, grid, block, smem, st, args...);
+// `chained`: the predecessor does not let this kernel start early (float32, and where the caller launched such a one); else, many
+// small CTAs that they are, these kernels are launched plainly.
+template <class... P, class... A>
+void launch_late(bool chained, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+    if (chained) launch_chained(kern, grid, block, smem, st, args...);
     else kern<<<grid, block, smem, st>>>(static_cast<P>(args)...);
 }
 
@@ -168,6 +169,7 @@ struct GemmParams {
     const float* nb_val;
     int taps, C, nb_maximum, nb_softmax;
     int pad;              // A_CONV1D
+    int chained;          // the launch before this one is the caller's and does not let this one start early
     bool a_vec, w_vec, c_vec;   // set by the launcher
 };
 

@@ -106,7 +106,7 @@ template <typename T, typename TO, int TPT> struct DwShape {
 
 template <typename T, typename TO, int VEC, int TPT>
 __global__ void __launch_bounds__(THREADS, DwShape<T, TO, TPT>::MINB) gather_conv_dw_kernel(const DwParams p, const int TT) {
-    chain_begin_for<T>();
+    chain_begin_for<TO>();
     typedef Channels<T, VEC> Ch;
     constexpr int UNROLL = DwShape<T, TO, TPT>::UNROLL;
     extern __shared__ __align__(16) unsigned char dw_smem[];

@@ -246,7 +246,7 @@ int launch_gather_conv_simt(const convnn_desc* d, const Dims& dm, const void* v,
             const int rc = try_launch_gather_conv_dw(d, dm, v, idx, val, w_conv, scratch, true, st);
             if (rc != CONVNN_E_UNSUPPORTED) {
                 if (rc) return rc;
-                p.a = scratch; p.lda = dm.Cp; p.a_mode = A_ROWS; p.a_f32 = 1; p.Kd = dm.C; p.w = w_pw; p.ldw = dm.C;
+                p.a = scratch; p.lda = dm.Cp; p.a_mode = A_ROWS; p.a_f32 = 1; p.chained = 1; p.Kd = dm.C; p.w = w_pw; p.ldw = dm.C;
                 return launch_gemm_simt(d->dtype, p, st);
             }
         }

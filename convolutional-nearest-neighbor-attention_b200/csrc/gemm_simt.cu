@@ -124,7 +124,7 @@ __device__ __forceinline__ void store_outputs(const GemmParams& p, int n0, int s
 // TA: type of the A operand (float32 against bfloat16 weights for the separable conv's unrounded intermediate).
 template <typename TA, typename T, int MODE, int BM, int BN, int BK, int TM, int TN, int MINB>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_kernel(const GemmParams p) {
-    chain_begin_for<T>();
+    chain_wait();                           // (and no early start for the next one, see chain_begin_for())
     constexpr int NT = (BM / TM) * (BN / TN);
     constexpr int VM = TM < 4 ? TM : 4, VN = TN < 4 ? TN : 4;   // rows / columns read with one instruction
     constexpr int RG = TM / VM, CG = TN / VN;               // groups of them per thread
@@ -366,7 +366,7 @@ __device__ __forceinline__ void multiply_step(const float* tile, int ty, int tx,
 template <int MODE, int BM, int BN, int TM, int TN, int MINB>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_copy_kernel(const GemmParams p) {
     static_assert(MODE == A_ROWS || MODE == A_TOKENS, "plain rows");
-    chain_wait();
+    chain_wait();                           // (and no early start for the next one, see chain_begin_for())
     constexpr int NT = (BM / TM) * (BN / TN), BK = 32, ST = 4, PIECES = BK / 4;
     constexpr int WN = BN / TN / 8;
     constexpr int NL = (BM + BN) * PIECES / NT;                 // copies per thread and step
@@ -482,7 +482,7 @@ template <> struct Four<__nv_bfloat16> {
 template <typename TA, typename T, int MODE, int BM, int BN, int TM, int TN, int MINB>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_stage_kernel(const GemmParams p) {
     static_assert(MODE == A_ROWS || MODE == A_TOKENS, "plain rows");
-    chain_begin_for<T>();
+    chain_wait();                           // (and no early start for the next one, see chain_begin_for())
     constexpr int NT = (BM / TM) * (BN / TN), BK = 32, PIECES = BK / 4, STEP = NT / PIECES;   // rows per pass
     constexpr int WN = BN / TN / 8, NA = BM / STEP, NB = BN / STEP;
     static_assert(BM % STEP == 0 && BN % STEP == 0 && NT % 32 == 0 && (BN / TN) % 8 == 0, "tile");
@@ -576,7 +576,7 @@ int launch_tile(const GemmParams& p, cudaStream_t st) {
     const size_t smem = (size_t)2 * BK * (BM + 4 + BN + 4) * 4 + (MODE == A_NEIGHBOURS ? (size_t)BM * p.taps * 8 : 0);
     auto kern = gemm_simt_kernel<TA, T, MODE, BM, BN, BK, TM, TN, MINB>;
     CONVNN_ENSURE_SMEM(kern, smem);
-    launch_by_type<T>(kern, grid, (BM / TM) * (BN / TN), smem, st, p);
+    launch_late(sizeof(T) == 4 || p.chained, kern, grid, (BM / TM) * (BN / TN), smem, st, p);
     return CONVNN_OK;
 }
 
@@ -586,7 +586,7 @@ int launch_stage_tile(const GemmParams& p, cudaStream_t st) {
     const size_t smem = (size_t)2 * (BM + BN) * 32 * 4;
     auto kern = gemm_simt_stage_kernel<TA, T, MODE, BM, BN, TM, TN, MINB>;
     CONVNN_ENSURE_SMEM(kern, smem);
-    launch_by_type<T>(kern, grid, (BM / TM) * (BN / TN), smem, st, p);
+    launch_late(sizeof(T) == 4 || p.chained, kern, grid, (BM / TM) * (BN / TN), smem, st, p);
     return CONVNN_OK;
 }
 

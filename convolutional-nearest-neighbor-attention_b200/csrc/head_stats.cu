@@ -29,7 +29,8 @@ struct HeadTensors {
 
 template <typename T>
 __global__ void __launch_bounds__(256, 6) head_stats_kernel(const HeadTensors in, int B, int H, int dk, int C, int Cp, int coord, int metric) {
-    chain_begin_for<T>();
+    chain_wait();
+    if (sizeof(T) != 4 && !coord) chain_next();      // (with the coordinate channel the fp32 pipes' selection follows, see chain_begin_for())
     const int which = blockIdx.y;
     T* t = static_cast<T*>(which == 0 ? in.t[0] : which == 1 ? in.t[1] : in.t[2]);
     float* stat = which == 0 ? in.stat[0] : which == 1 ? in.stat[1] : in.stat[2];

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(NT) sim_topk_simt_kernel(
     const float* __restrict__ kstat, const int32_t* __restrict__ cand, int32_t* __restrict__ idx,
     float* __restrict__ val, int T_, int S, int H, int Cp, int K, int nsel, int metric, int sampled,
     float sqrt_dk, int vec) {
-    chain_begin_for<T>();
+    chain_wait();               // (and no early start for the next one, see chain_begin_for())
     constexpr int TM = RB / 16, RG = TM / 4;              // 16 x 16 threads, TM x 4 dot products each
     constexpr int LA = RB + 4, LB = CB + 4;
     constexpr int NA = RB * (BK / 4) / NT, TPR = NT / RB; // loads per thread and step; scanning threads per row
@@ -257,7 +257,7 @@ int launch(const convnn_desc* d, const Dims& dm, const void* q, const void* k, c
     auto kern = sim_topk_simt_kernel<T, KCAP, RB>;
     CONVNN_ENSURE_SMEM(kern, smem);
     const int vec = dm.Cp % 4 == 0 && aligned16(q) && aligned16(k);
-    launch_by_type<T>(kern, dim3((dm.T + RB - 1) / RB, dm.B * dm.H), NT, smem, st,
+    launch_late(sizeof(T) == 4 || d->coord, kern, dim3((dm.T + RB - 1) / RB, dm.B * dm.H), NT, smem, st,
         static_cast<const T*>(q), static_cast<const T*>(k), qstat, kstat, cand, idx, val, dm.T, dm.S, dm.H, dm.Cp, dm.K,
         dm.nsel, d->metric, d->sampled, (float)sqrt((double)dm.dk), vec);
     CONVNN_CHECK_LAUNCH("sim_topk_simt");

@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(NT) sim_topk_simt_rows_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const float* __restrict__ qstat, const float* __restrict__ kstat,
     const int32_t* __restrict__ cand, int32_t* __restrict__ idx, float* __restrict__ val, int T_, int S, int H, int Cp, int K,
     int nsel, int metric, int sampled, float sqrt_dk, int vec) {
-    chain_begin_for<T>();
+    chain_wait();               // (and no early start for the next one, see chain_begin_for())
     constexpr int NB = 32 * J, LB = NB + 4;
     extern __shared__ __align__(16) float sm[];
     float* As = sm;                                       // [2][BK][LA]
@@ -153,7 +153,7 @@ int launch(const convnn_desc* d, const Dims& dm, const void* q, const void* k, c
     auto kern = sim_topk_simt_rows_kernel<T, J, NS>;
     CONVNN_ENSURE_SMEM(kern, smem);
     const int vec = dm.Cp % 4 == 0 && aligned16(q) && aligned16(k);
-    launch_by_type<T>(kern, dim3((dm.T + RB - 1) / RB, dm.B * dm.H), NT, smem, st,
+    launch_late(sizeof(T) == 4 || d->coord, kern, dim3((dm.T + RB - 1) / RB, dm.B * dm.H), NT, smem, st,
         static_cast<const T*>(q), static_cast<const T*>(k), qstat, kstat, cand, idx, val, dm.T, dm.S, dm.H, dm.Cp, dm.K,
         dm.nsel, d->metric, d->sampled ? 1 : 0, (float)sqrt((double)dm.dk), vec);
     CONVNN_CHECK_LAUNCH("sim_topk_simt_rows");
