@@ -39,6 +39,7 @@ constexpr int NTHREADS = 192;      // TMA warp, MMA warp, 4 softmax warps
 constexpr int CW = 16;
 
 struct AttnParams {
+    int beside;             // see chain_leave()
     __nv_bfloat16* o;              // (B, T, H * dk)
     int T, H, dk, D;
     int KCH, KC;                   // channels per chunk / chunks of the Q K^T reduction
@@ -112,7 +113,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_begin();
+    chain_wait_unless(p.beside);
+    chain_next();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -314,6 +316,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, ncols);
     }
+    chain_leave(p.beside);
 }
 
 // One warp per query row; scores in shared memory.  float32 (and the fallback for shapes the
@@ -375,7 +378,7 @@ bool attention_tc_ok(int dtype, const void* q, const void* k, const void* v, con
 }
 
 int launch_attention_tc(const void* q, const void* k, const void* v, void* o, int B, int Tn, int D, int H,
-                        cudaStream_t st) {
+                        cudaStream_t st, bool beside) {
     AttnParams p{};
     p.o = static_cast<__nv_bfloat16*>(o);
     p.T = Tn; p.H = H; p.dk = D / H; p.D = D;
@@ -394,6 +397,7 @@ int launch_attention_tc(const void* q, const void* k, const void* v, void* o, in
                         7 * 8 + 16;
     if (smem > 227 * 1024) return set_error(CONVNN_E_UNSUPPORTED, "attention_tc: shape needs %zu bytes of shared memory", smem);
 
+    p.beside = beside;
     CUtensorMap tmQ, tmK, tmV;
     const uint64_t dims[4] = {(uint64_t)p.dk, (uint64_t)H, (uint64_t)Tn, (uint64_t)B};
     const uint64_t str[3] = {(uint64_t)p.dk * 2, (uint64_t)D * 2, (uint64_t)Tn * D * 2};
@@ -437,8 +441,8 @@ int launch_attention_simt_t(const void* q, const void* k, const void* v, void* o
 
 // q, k, v, o: (B, T, H, d_k) = (B*T, D) row-major in `dtype`.
 int launch_attention(int dtype, const void* q, const void* k, const void* v, void* o, int B, int Tn, int D, int H,
-                     cudaStream_t st) {
-    if (attention_tc_ok(dtype, q, k, v, o, Tn, D, H)) return launch_attention_tc(q, k, v, o, B, Tn, D, H, st);
+                     cudaStream_t st, bool beside) {
+    if (attention_tc_ok(dtype, q, k, v, o, Tn, D, H)) return launch_attention_tc(q, k, v, o, B, Tn, D, H, st, beside);
     if (dtype == CONVNN_F32) return launch_attention_simt_t<float>(q, k, v, o, B, Tn, D, H, st);
     return launch_attention_simt_t<__nv_bfloat16>(q, k, v, o, B, Tn, D, H, st);
 }

@@ -395,22 +395,31 @@ int convnn_b200_gather_conv(const convnn_desc* d, const void* v, const int32_t* 
 
 namespace {
 // Neighbours of the workspace's q and k and the conv over its v: in one kernel where that takes the shape (the lists are then
-// not written), else stage by stage.  *merged: o has several heads already in the flat reinterpretation (B, T, D).
+// not written), else stage by stage, with stages 1 and 2 of `other` beside them.  *merged: o has several heads already in the flat reinterpretation (B, T, D).
 int select_and_conv(const convnn_desc* d, const Dims& dm, const Workspace& w, const int32_t* cand, const void* w_conv,
-                    const void* w_pw, void* o, bool* merged, void* stream) {
+                    const void* w_pw, void* o, bool* merged, void* stream, const OtherHalf* other = nullptr) {
     REQUIRE_PTR(w_conv); REQUIRE_PTR(o);
     int rc = CONVNN_E_UNSUPPORTED;
     *merged = false;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (d->conv_type == CONVNN_DEPTHWISE && !force_simt())
-        rc = try_launch_sim_gather(d, dm, w.q, w.k, w.v, w.qstat, w.kstat, cand, w_conv, o, static_cast<cudaStream_t>(stream));
-    if (rc != CONVNN_E_UNSUPPORTED) return rc;
-    if ((rc = convnn_b200_sim_topk(d, w.q, w.k, w.qstat, w.kstat, cand, w.idx, w.val, stream))) return rc;
-    if (dm.H > 1) {
-        rc = try_launch_conv_std_tc(d, dm, w.v, w.idx, w.val, w_conv, o, true, static_cast<cudaStream_t>(stream));
-        *merged = rc == CONVNN_OK;
-        if (rc != CONVNN_E_UNSUPPORTED) return rc;
+        rc = try_launch_sim_gather(d, dm, w.q, w.k, w.v, w.qstat, w.kstat, cand, w_conv, o, st);
+    if (rc != CONVNN_E_UNSUPPORTED) {
+        if (rc || !other) return rc;
+        // (a stage needs the one before it: only the first of them may run beside the layer's kernel)
+        if ((rc = other->stage(1, true, true, stream))) return rc;
+        return other->stage(2, false, true, stream);
     }
-    return convnn_b200_gather_conv(d, w.v, w.idx, w.val, w_conv, w_pw, o, w.conv_scratch, stream);
+    if ((rc = convnn_b200_sim_topk(d, w.q, w.k, w.qstat, w.kstat, cand, w.idx, w.val, stream))) return rc;
+    if (other && (rc = other->stage(1, true, true, stream))) return rc;
+    rc = CONVNN_E_UNSUPPORTED;
+    if (dm.H > 1) {
+        rc = try_launch_conv_std_tc(d, dm, w.v, w.idx, w.val, w_conv, o, true, st);
+        *merged = rc == CONVNN_OK;
+    }
+    if (rc == CONVNN_E_UNSUPPORTED) rc = convnn_b200_gather_conv(d, w.v, w.idx, w.val, w_conv, w_pw, o, w.conv_scratch, stream);
+    if (rc || !other) return rc;
+    return other->stage(2, true, true, stream);
 }
 
 // merged: o is (B, T, D), heads in the flat reinterpretation.
@@ -690,7 +699,7 @@ int convnn::prenorm_mlp(const void* x, int64_t ldx, const float* moments, int32_
 int convnn::layer_forward(const convnn_desc* d, const void* x, int64_t ldx, const void* w_qkv,
                         const void* w_conv, const void* w_pw, const void* w_o, const int32_t* cand,
                         const void* residual, int64_t ldr, void* out, int64_t ldo, void* workspace,
-                        size_t workspace_bytes, bool at_rest, void* stream) {
+                        size_t workspace_bytes, bool at_rest, void* stream, const OtherHalf* other) {
     Dims dm;
     int rc = validate(d, &dm);
     if (rc) return rc;
@@ -700,14 +709,15 @@ int convnn::layer_forward(const convnn_desc* d, const void* x, int64_t ldx, cons
     if (workspace_bytes < w.total)
         return set_error(CONVNN_E_WORKSPACE, "workspace has %zu bytes, %zu needed", workspace_bytes, w.total);
     if ((rc = qkv_proj_impl(d, x, ldx, w_qkv, cand, w.q, w.k, w.v, w.qstat, w.kstat, w.scratch, stream, nullptr, at_rest))) return rc;
+    if (other && (rc = other->stage(0, true, true, stream))) return rc;
     bool merged;
-    if ((rc = select_and_conv(d, dm, w, cand, w_conv, w_pw, w.o, &merged, stream))) return rc;
+    if ((rc = select_and_conv(d, dm, w, cand, w_conv, w_pw, w.o, &merged, stream, other))) return rc;
     return out_proj_impl(d, w.o, w_o, residual, ldr, out, ldo, w.scratch, stream, nullptr, merged, true);
 }
 
 int convnn::linear(int dtype, const void* a, int64_t lda, const void* w, const void* bias, const void* residual,
                        int64_t ldr, void* out, int64_t ldo, int64_t M, int32_t N, int32_t K, int32_t gelu,
-                       bool at_rest, void* stream) {
+                       bool at_rest, void* stream, bool beside) {
     if (dtype != CONVNN_F32 && dtype != CONVNN_BF16) return set_error(CONVNN_E_INVALID, "unknown dtype %d", dtype);
     REQUIRE_PTR(a); REQUIRE_PTR(w); REQUIRE_PTR(out);
     if (M < 0 || N < 1 || K < 1 || lda < K || ldo < N || (residual && ldr < N) || M >= (1ll << 31))
@@ -721,7 +731,7 @@ int convnn::linear(int dtype, const void* a, int64_t lda, const void* w, const v
         const bool extra_ok = (!bias || aligned16(bias)) && (!residual || (aligned16(residual) && ldr % 8 == 0));
         if (extra_ok && gemm_tc_supported(a, lda, w, K, N, 1, cs, ldo)) {
             GemmTcOpts o;
-            o.bias = bias; o.residual = residual; o.ldr = ldr; o.gelu = gelu; o.w_at_rest = at_rest;
+            o.bias = bias; o.residual = residual; o.ldr = ldr; o.gelu = gelu; o.w_at_rest = at_rest; o.beside = beside;
             return launch_gemm_tc(a, lda, w, (int)M, N, K, 1, cs, ldo, o, st);
         }
     }
@@ -783,25 +793,10 @@ int convnn::softmax_attention(int dtype, const void* x, int64_t ldx, const void*
     if (workspace_bytes < need)
         return set_error(CONVNN_E_WORKSPACE, "workspace has %zu bytes, %zu needed", workspace_bytes, need);
     if ((rc = check_device())) return rc;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const size_t elt = dtype == CONVNN_F32 ? 4 : 2, part = up256((size_t)B * T * D * elt);
-    char* ws = static_cast<char*>(workspace);
-    void* qkv[3] = {ws, ws + part, ws + 2 * part};
-    void* o = ws + 3 * part;
-    const long long M = (long long)B * T;
-    // q, k, v: one launch over the packed weight where the tensor-core GEMM takes the shape
-    if (dtype == CONVNN_BF16 && !force_simt() && gemm_tc_supported(x, ldx, w_qkv, D, 3 * D, 3, qkv, D)) {
-        GemmTcOpts go;
-        go.w_at_rest = at_rest;
-        if ((rc = launch_gemm_tc(x, ldx, w_qkv, (int)M, 3 * D, D, 3, qkv, D, go, st))) return rc;
-    } else {
-        for (int i = 0; i < 3; ++i)
-            if ((rc = convnn_b200_linear(dtype, x, ldx, static_cast<const char*>(w_qkv) + (size_t)i * D * D * elt, nullptr,
-                                         nullptr, 0, qkv[i], D, M, D, D, 0, stream)))
-                return rc;
-    }
-    if ((rc = launch_attention(dtype, qkv[0], qkv[1], qkv[2], o, B, T, D, H, st))) return rc;
-    return linear(dtype, o, D, w_o, nullptr, nullptr, 0, out, ldo, M, D, D, 0, true, stream);
+    const OtherHalf half{false, x, w_qkv, nullptr, nullptr, nullptr, w_o, nullptr, out, workspace, ldx, ldo, B, T, D, H, 0, dtype};
+    for (int i = 0; i < 3; ++i)
+        if ((rc = half.stage(i, false, i > 0 || at_rest, stream))) return rc;
+    return CONVNN_OK;
 }
 
 int convnn::conv1d_attention(int dtype, const void* x, int64_t ldx, const void* w_x, const void* b_x,
@@ -817,19 +812,43 @@ int convnn::conv1d_attention(int dtype, const void* x, int64_t ldx, const void* 
     if (workspace_bytes < need)
         return set_error(CONVNN_E_WORKSPACE, "workspace has %zu bytes, %zu needed", workspace_bytes, need);
     if ((rc = check_device())) return rc;
+    const OtherHalf half{true, x, w_x, b_x, w_conv, b_conv, w_o, b_o, out, workspace, ldx, ldo, B, T, D, H, kernel_size, dtype};
+    for (int i = 0; i < 3; ++i)
+        if ((rc = half.stage(i, false, i > 0 || at_rest, stream))) return rc;
+    return CONVNN_OK;
+}
+
+// Softmax attention: q, k, v / the attention / W_o.  Conv1d: the biased Linear / the conv in the reference's flat
+// reinterpretation (it reads the per-head (T, d_k) block back as (d_k, T), layers.py:487-489, 499) / the biased Linear.
+int convnn::OtherHalf::stage(int i, bool beside, bool at_rest, void* stream) const {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t elt = dtype == CONVNN_F32 ? 4 : 2, part = up256((size_t)B * T * D * elt);
     char* ws = static_cast<char*>(workspace);
-    void *y = ws, *o = ws + part, *merged = ws + 2 * part, *unfold = ws + 3 * part;
     const long long M = (long long)B * T;
-    if ((rc = linear(dtype, x, ldx, w_x, b_x, nullptr, 0, y, D, M, D, D, 0, at_rest, stream))) return rc;
-    // the reference reads the per-head (T, d_k) block back as (d_k, T) for every H (layers.py:487-489, 499)
-    rc = dtype == CONVNN_BF16 && !force_simt() ? try_launch_conv1d_tc(y, w_conv, b_conv, merged, B, T, H, D / H, kernel_size, st)
-                                               : (int)CONVNN_E_UNSUPPORTED;
-    if (rc == CONVNN_E_UNSUPPORTED) {
-        if ((rc = launch_conv1d_heads(dtype, y, w_conv, b_conv, o, unfold, B, T, H, D / H, kernel_size, st))) return rc;
-        rc = launch_merge_heads(dtype, o, merged, B, T, H, D / H, st);
+    int rc;
+    if (!conv1d) {
+        void* qkv[3] = {ws, ws + part, ws + 2 * part};
+        void* o = ws + 3 * part;
+        if (i == 1) return launch_attention(dtype, qkv[0], qkv[1], qkv[2], o, B, T, D, H, st, beside);
+        if (i == 2) return linear(dtype, o, D, w_out, nullptr, nullptr, 0, out, ldo, M, D, D, 0, at_rest, stream, beside);
+        // one launch over the packed weight where the tensor-core GEMM takes the shape
+        if (dtype == CONVNN_BF16 && !force_simt() && gemm_tc_supported(x, ldx, w_in, D, 3 * D, 3, qkv, D)) {
+            GemmTcOpts go;
+            go.w_at_rest = at_rest; go.beside = beside;
+            return launch_gemm_tc(x, ldx, w_in, (int)M, 3 * D, D, 3, qkv, D, go, st);
+        }
+        for (int n = 0; n < 3; ++n)
+            if ((rc = linear(dtype, x, ldx, static_cast<const char*>(w_in) + (size_t)n * D * D * elt, nullptr, nullptr, 0, qkv[n],
+                             D, M, D, D, 0, n > 0 || at_rest, stream)))
+                return rc;
+        return CONVNN_OK;
     }
-    if (rc) return rc;
-    return linear(dtype, merged, D, w_o, b_o, nullptr, 0, out, ldo, M, D, D, 0, true, stream);
+    void *y = ws, *o = ws + part, *merged = ws + 2 * part, *unfold = ws + 3 * part;
+    if (i == 0) return linear(dtype, x, ldx, w_in, b_in, nullptr, 0, y, D, M, D, D, 0, at_rest, stream, beside);
+    if (i == 2) return linear(dtype, merged, D, w_out, b_out, nullptr, 0, out, ldo, M, D, D, 0, at_rest, stream, beside);
+    rc = dtype == CONVNN_BF16 && !force_simt()
+             ? try_launch_conv1d_tc(y, w_conv, b_conv, merged, B, T, H, D / H, kernel_size, st, beside) : (int)CONVNN_E_UNSUPPORTED;
+    if (rc != CONVNN_E_UNSUPPORTED) return rc;
+    if ((rc = launch_conv1d_heads(dtype, y, w_conv, b_conv, o, unfold, B, T, H, D / H, kernel_size, st))) return rc;
+    return launch_merge_heads(dtype, o, merged, B, T, H, D / H, st);
 }

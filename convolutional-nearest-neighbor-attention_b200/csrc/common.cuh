@@ -55,6 +55,15 @@ __device__ __forceinline__ void chain_begin_for() {
     chain_wait();
     if (sizeof(T) != 4) chain_next();
 }
+// A kernel launched BESIDE its predecessor does not need that one's results: it starts its work as soon as it is let, and waits
+// at its end instead, so that whoever waits for it has waited for both.  Its predecessor has to be one that waited at its own start
+// (so that everything older has ended), and what it reads and writes must be apart from what that one does.
+__device__ __forceinline__ void chain_wait_unless(bool beside) {
+    if (!beside) chain_wait();
+}
+__device__ __forceinline__ void chain_leave(bool beside) {
+    if (beside && threadIdx.x == 0) chain_wait();
+}
 // Under capture the launch is a plain one: a graph's own launches are cheap, its kernels overlap across branches already
 // (two batches in flight, 128 launches: 2844 us with chained edges, 2831 us without), and instantiating chained edges
 // took the host 0.3 s.
@@ -237,6 +246,7 @@ struct GemmTcOpts {
     // The launch before this one on the stream is this library's own, made by the same call, and does not write W, its
     // extra rows or the bias: they may be read before it has ended (see chain_wait()).
     bool w_at_rest = false;
+    bool beside = false;              // see chain_leave(); takes w_at_rest
     // Row moments of the stored rows, [gemm_tc_moment_planes(N)][gemm_tc_moment_stride(M)][2]; needs a skip connection.
     float* moments_out = nullptr;
 };
@@ -259,6 +269,16 @@ int launch_mlp_tc(const void* x, long long ldx, const float* moments, int planes
                   const void* w1_extra, const void* w2, const void* b2, void* out, long long ldo, int M, int D, int DM,
                   float* moments_out, const void* w_o, const void* resid, long long ldr, bool weights_at_rest, cudaStream_t st);
 int read_mlp_tc_status(int* out);
+// Stages (0, 1, 2) of the other half of a branching block, for layer_forward() to launch beside its own.
+struct OtherHalf {
+    bool conv1d;                                   // else softmax attention
+    const void *x, *w_in, *b_in, *w_conv, *b_conv, *w_out, *b_out;
+    void *out, *workspace;
+    int64_t ldx, ldo;
+    int32_t B, T, D, H, kernel_size;
+    int dtype;
+    int stage(int i, bool beside, bool at_rest, void* stream) const;
+};
 // The entry points of these names; at_rest: as GemmTcOpts::w_at_rest, for the call's first weights.
 int prenorm_mlp(const void* x, int64_t ldx, const float* moments, int32_t planes, float eps, const void* w1_folded,
                 const void* w1_extra, const void* w2, const void* b2, void* out, int64_t ldo, int64_t M, int32_t D, int32_t DM,
@@ -269,9 +289,9 @@ int prenorm_forward(const convnn_desc* d, const void* x, int64_t ldx, const floa
                     size_t workspace_bytes, bool at_rest, void* stream);
 int layer_forward(const convnn_desc* d, const void* x, int64_t ldx, const void* w_qkv, const void* w_conv, const void* w_pw,
                   const void* w_o, const int32_t* cand, const void* residual, int64_t ldr, void* out, int64_t ldo, void*
-                  workspace, size_t workspace_bytes, bool at_rest, void* stream);
+                  workspace, size_t workspace_bytes, bool at_rest, void* stream, const OtherHalf* other = nullptr);
 int linear(int dtype, const void* a, int64_t lda, const void* w, const void* bias, const void* residual, int64_t ldr, void*
-           out, int64_t ldo, int64_t M, int32_t N, int32_t K, int32_t gelu, bool at_rest, void* stream);
+           out, int64_t ldo, int64_t M, int32_t N, int32_t K, int32_t gelu, bool at_rest, void* stream, bool beside = false);
 int prenorm_linear(const void* a, int64_t lda, const float* moments, int32_t planes, float eps, const void* w_folded, const
                    void* w_extra, void* out, int64_t ldo, int64_t M, int32_t N, int32_t K, int32_t gelu, bool at_rest, void*
                    stream);
@@ -293,14 +313,14 @@ int launch_gather_rows(int dtype, const void* x, long long ldx, const int32_t* c
                        int D, cudaStream_t st);
 int launch_merge_heads(int dtype, const void* o, void* y, int B, int Tn, int H, int dk, cudaStream_t st);
 int launch_attention(int dtype, const void* q, const void* k, const void* v, void* o, int B, int Tn, int D, int H,
-                     cudaStream_t st);
+                     cudaStream_t st, bool beside = false);
 int read_attention_status(int* out);
 int launch_conv1d_heads(int dtype, const void* y, const void* w, const void* bias, void* o, void* unfold, int B,
                         int Tn, int H, int dk, int ks, cudaStream_t st);
 // Conv1d half and its flat reinterpretation in one kernel (heads of 16, 32 or 64 channels whose taps fit in shared memory, by a rule
 // on the number and length of the slices).
 int try_launch_conv1d_tc(const void* y, const void* w, const void* bias, void* out, int B, int Tn, int H, int dk, int ks,
-                         cudaStream_t st);
+                         cudaStream_t st, bool beside = false);
 int read_conv1d_tc_status(int* out);
 // Standard conv with its weighted neighbour block kept on the SM (bfloat16 heads of 16, 32 or 64 channels whose taps fit, by a rule on
 // tiles per SM and taps); merged: o is (B, T, D) in the flat reinterpretation.

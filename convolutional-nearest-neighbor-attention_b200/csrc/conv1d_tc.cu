@@ -33,6 +33,7 @@ constexpr int NT = 64 + NEPI;
 constexpr size_t SMEM_MAX = 226 * 1024;
 
 struct Conv1dParams {
+    int beside;             // see chain_leave()
     const __nv_bfloat16* bias;
     __nv_bfloat16* out;
     int T, H, dk, ks, pad, D;
@@ -84,7 +85,7 @@ conv1d_tc_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant_
         tmem_alloc(tmem_slot, ncols);
         tmem_relinquish();
     }
-    chain_wait();
+    chain_wait_unless(p.beside);
     // accumulator := bias by one K = 16 step: rows of `ones` hold 1.0 at the start of both 16-byte halves, a bias row its
     // value at the start of one, so the product picks it up whatever the swizzle
     for (int i = threadIdx.x; i < 1024; i += NT) reinterpret_cast<uint32_t*>(ones)[i] = (i & 3) == 0 ? 0x3f80u : 0u;
@@ -211,6 +212,7 @@ conv1d_tc_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant_
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, ncols);
     }
+    chain_leave(p.beside);
 }
 
 }  // namespace
@@ -236,11 +238,12 @@ static bool conv1d_tc_wanted(int B, int Tn, int H, int dk, int ks) {
 // untouched) where the heads are of another width, the other kernels are faster (above), pointers are unaligned, or a slice
 // does not fit beside the taps and one set of boxes (nine taps: 64 channels up to 21 tokens).
 int try_launch_conv1d_tc(const void* y, const void* w, const void* bias, void* out, int B, int Tn, int H, int dk, int ks,
-                         cudaStream_t st) {
+                         cudaStream_t st, bool beside) {
     if ((dk != 16 && dk != 32 && dk != 64) || ks > 32 || !conv1d_tc_wanted(B, Tn, H, dk, ks) || !aligned16(y) || !aligned16(w) || !aligned16(out)) return CONVNN_E_UNSUPPORTED;
     Conv1dParams p{};
     p.bias = static_cast<const __nv_bfloat16*>(bias); p.out = static_cast<__nv_bfloat16*>(out);
     p.T = Tn; p.H = H; p.dk = dk; p.ks = ks; p.pad = (ks - 1) / 2; p.D = H * dk;
+    p.beside = beside;
     p.n_units = B * H; p.n_tiles = (Tn + BM - 1) / BM;
     p.acc_cols = dk < 32 ? 32 : dk;
     const size_t slab = ((size_t)Tn * dk * 2 + 15) / 16 * 16;

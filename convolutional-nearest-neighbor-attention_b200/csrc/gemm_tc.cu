@@ -79,6 +79,7 @@ struct GemmTcParams {
     int stages;            // depth of the shared-memory ring
     int wstat;             // 1: the whole W tile (BN x Kd) stays in shared memory; the ring holds A only
     int tiles_per_cta;     // wstat: each CTA owns a contiguous range of the n-major tile list
+    int beside;            // see chain_leave()
     int w_at_rest;         // nothing that may still run on the stream writes W, its extra rows or the bias
     // pre-norm fold: the moments of the A rows, [ln_planes][mom_ld] (sum, sum of squares) partial sums,
     // arrive through the tensor map tmM
@@ -320,7 +321,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             };
             if (lane < lead && (!PAIR || rank == 0)) mbar_expect_tx_a(full0 + 8 * lane, tx);
             if (p.w_at_rest) request_w();                                // before the predecessor has ended
-            chain_wait();
+            chain_wait_unless(p.beside);
             if (!p.w_at_rest) request_w();
             if (lane < lead) load_a((uint32_t)lane, lane, m0);
             __syncwarp();
@@ -350,7 +351,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             load_w_chunk((uint32_t)w_ahead, w_ahead, nt * p.BN + (int)rank * bn_cta);
                         }
                 }
-                chain_wait();
+                chain_wait_unless(p.beside);
             }
             bool any = lead > 0;
             for (int t = first; t < last && ok; t += step) {
@@ -463,7 +464,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             mbar_expect_tx(&mfull[slot], slot_bytes);
             tma_load_2d(mring + slot * slot_bytes, &tmM, &mfull[slot], mt * BM * 2, 0);
         };
-        chain_wait();
+        chain_wait_unless(p.beside);
         if (lane == 0)
             for (int k = 0; k < MOM_AHEAD; ++k)
                 if (first + k * step < last) fetch((uint32_t)k, first + k * step);
@@ -538,7 +539,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const bool tr = !PAIR && trace_enabled() && blockIdx.x == 0 && lq == 0 && lane == 0 && chalf == 0;
         const uint32_t lead_tempty0 = PAIR ? map_to_cta(smem_u32(tempty), 0) : 0u;
         int tn = 0;
-        chain_wait();
+        chain_wait_unless(p.beside);
         chain_next();
         for (int t = first + half * step; t < last && ok; t += 2 * step, tile += 2) {
             int mt, nt;
@@ -758,6 +759,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (PAIR) tmem_dealloc_pair(tmem_base, ncols);
         else tmem_dealloc(tmem_base, ncols);
     }
+    chain_leave(p.beside);
 }
 
 int pow2_at_least(int v, int lo) {
@@ -851,7 +853,7 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
     }
     p.ldc = ldc; p.bias = static_cast<const __nv_bfloat16*>(o.bias); p.gelu = o.gelu;
     p.mma_bias = nullptr;
-    p.w_at_rest = o.w_at_rest;
+    p.w_at_rest = o.w_at_rest || o.beside; p.beside = o.beside;
     p.residual = static_cast<const __nv_bfloat16*>(o.residual); p.ldr = o.ldr;
     p.stat_pieces = 1; p.stat_plane = 0;
     p.stat_mode = o.stat_mode; p.dk = o.dk > 0 ? o.dk : 32; p.heads = o.heads; p.rows_per_batch = o.rows_per_batch > 0 ? o.rows_per_batch : 1;

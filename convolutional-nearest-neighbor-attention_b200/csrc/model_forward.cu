@@ -19,6 +19,7 @@ struct Plan {
     size_t x, x1, mom, mom1, scratch, total;      // byte offsets into the workspace
     size_t cols, proj;                             // embedding phase, offsets into scratch
     size_t xn, cat, layer_ws, h;                   // block phases
+    size_t other_ws, least;                        // the other half's own workspace, if it is to run beside; bytes without it
 };
 
 int planes_of(int D) {
@@ -31,7 +32,7 @@ bool plan_of(const convnn_model* m, Plan* p) {
     const size_t patches = (size_t)m->B * (m->T - 1);
     size_t off = 0;
     auto take = [&](size_t n) { const size_t r = off; off += up(n); return r; };
-    size_t h = 0, layer = 0, cat = 0, planes = 1;
+    size_t h = 0, layer = 0, other = 0, cat = 0, planes = 1;
     for (int i = 0; i < m->n_blocks; ++i) {
         const convnn_block& b = m->blocks[i];
         const size_t ws = convnn_b200_workspace_bytes(&b.layer);
@@ -39,9 +40,9 @@ bool plan_of(const convnn_model* m, Plan* p) {
         layer = most(layer, ws);
         const int rest = m->D - b.layer.D;
         if (b.kind == CONVNN_BLOCK_BRANCH_ATTENTION)
-            layer = most(layer, convnn_b200_attention_workspace_bytes(m->dtype, m->B, m->T, rest));
+            other = most(other, convnn_b200_attention_workspace_bytes(m->dtype, m->B, m->T, rest));
         else if (b.kind == CONVNN_BLOCK_BRANCH_CONV1D)
-            layer = most(layer, convnn_b200_conv1d_attention_workspace_bytes(m->dtype, m->B, m->T, rest, b.kernel_size));
+            other = most(other, convnn_b200_conv1d_attention_workspace_bytes(m->dtype, m->B, m->T, rest, b.kernel_size));
         if (b.kind != CONVNN_BLOCK_CONVNN) cat = row_bytes;
         h = most(h, rows * (size_t)b.d_mlp * elt);
         planes = most(planes, (size_t)planes_of(m->D));
@@ -59,19 +60,28 @@ bool plan_of(const convnn_model* m, Plan* p) {
     p->cat = row_bytes;
     p->layer_ws = row_bytes + cat;
     p->h = row_bytes;
-    p->total = off + most(embed, most(p->layer_ws + up(layer), p->h + up(h)));
+    p->least = off + most(embed, most(p->layer_ws + up(most(layer, other)), p->h + up(h)));
+    p->other_ws = p->layer_ws + up(layer);
+    // (float32 kernels are started one after the other whatever the order: nothing to run beside)
+    p->total = m->dtype == CONVNN_BF16 ? most(p->least, off + p->other_ws + up(other)) : p->least;
     return true;
+}
+
+// Whether the other half's entry point would take these arguments (it reports what it refuses, stage() does not look).
+bool half_ok(const convnn_block& b, const OtherHalf& h) {
+    return h.D >= 1 && h.D % h.H == 0 && h.w_in && h.w_out && (!h.conv1d || (h.w_conv && b.kernel_size >= 1)) &&
+           (long long)h.B * h.T * h.D < (1ll << 31);
 }
 
 // One encoder block (vit.py:262-269): rows in x, result in x again, the rows in between in x1.  `mom` / `planes`:
 // moments of x, 0 planes where no kernel has produced them; on return those of the result (if `want_moments`).
-int block_forward(const convnn_model* m, const convnn_block& b, char* ws, const Plan& p, int* planes, bool want_moments,
-                  void* stream) {
+int block_forward(const convnn_model* m, const convnn_block& b, char* ws, const Plan& p, bool beside, int* planes,
+                  bool want_moments, void* stream) {
     const int64_t D = m->D, rows = (int64_t)m->B * m->T;
     const size_t elt = m->dtype == CONVNN_F32 ? 4 : 2;
     char *x = ws + p.x, *x1 = ws + p.x1, *scratch = ws + p.scratch;
     char *xn = scratch + p.xn, *layer_ws = scratch + p.layer_ws;
-    const size_t layer_bytes = p.total - p.scratch - p.layer_ws;
+    const size_t layer_bytes = p.least - p.scratch - p.layer_ws;
     float *mom = reinterpret_cast<float*>(ws + p.mom), *mom1 = reinterpret_cast<float*>(ws + p.mom1);
     const bool fold_mlp = b.fc1_folded != nullptr;
     int planes1 = 0, rc;
@@ -94,12 +104,16 @@ int block_forward(const convnn_model* m, const convnn_block& b, char* ws, const 
             // both branches read their channel slice of xn and write theirs of the concat buffer
             const int64_t dc = b.layer.D, rest = D - dc;
             char* cat = scratch + p.cat;
-            if ((rc = layer_forward(&b.layer, xn, D, b.w_qkv, b.w_conv, b.w_pw, b.w_o, b.cand, nullptr, 0, cat, D, layer_ws,
-                                    layer_bytes, true, stream)))
-                return rc;
             const char* xr = xn + dc * elt;
             char* cr = cat + dc * elt;
-            rc = b.kind == CONVNN_BLOCK_BRANCH_ATTENTION
+            const bool conv1d = b.kind == CONVNN_BLOCK_BRANCH_CONV1D;
+            const OtherHalf half{conv1d, xr, b.branch_w_in, conv1d ? b.branch_b_in : nullptr, b.branch_w_conv, b.branch_b_conv,
+                                 b.branch_w_out, conv1d ? b.branch_b_out : nullptr, cr, scratch + p.other_ws, D, D, m->B, m->T,
+                                 (int32_t)rest, b.layer.H, b.kernel_size, m->dtype};
+            if ((rc = layer_forward(&b.layer, xn, D, b.w_qkv, b.w_conv, b.w_pw, b.w_o, b.cand, nullptr, 0, cat, D, layer_ws,
+                                    layer_bytes, true, stream, beside && half_ok(b, half) ? &half : nullptr)))
+                return rc;
+            if (!(beside && half_ok(b, half))) rc = b.kind == CONVNN_BLOCK_BRANCH_ATTENTION
                      ? softmax_attention(m->dtype, xr, D, b.branch_w_in, b.branch_w_out, cr, D, m->B, m->T, (int32_t)rest,
                                          b.layer.H, layer_ws, layer_bytes, true, stream)
                      : conv1d_attention(m->dtype, xr, D, b.branch_w_in, b.branch_b_in, b.branch_w_conv, b.branch_b_conv,
@@ -174,8 +188,9 @@ int convnn_b200_model_forward(const convnn_model* m, const void* images, void* l
     if (!aligned16(workspace)) return set_error(CONVNN_E_ALIGN, "workspace must be 16-byte aligned");
     Plan p;
     if (!plan_of(m, &p)) return CONVNN_E_INVALID;                 // the layer's own message stands
-    if (workspace_bytes < p.total)
-        return set_error(CONVNN_E_WORKSPACE, "workspace has %zu bytes, %zu needed", workspace_bytes, p.total);
+    if (workspace_bytes < p.least)
+        return set_error(CONVNN_E_WORKSPACE, "workspace has %zu bytes, %zu needed", workspace_bytes, p.least);
+    const bool beside = p.total > p.least && workspace_bytes >= p.total;       // the halves of a block side by side
     char *ws = static_cast<char*>(workspace), *cols = ws + p.scratch + p.cols, *proj = ws + p.scratch + p.proj;
     const int32_t np = m->T - 1, pix = m->channels * m->patch * m->patch;
     if (m->images_u8)
@@ -195,7 +210,7 @@ int convnn_b200_model_forward(const convnn_model* m, const void* images, void* l
     int planes = first_folds ? 1 : 0;
     for (int i = 0; i < m->n_blocks; ++i) {
         const bool want = i + 1 < m->n_blocks && m->blocks[i + 1].w_qkv_folded;
-        if ((rc = block_forward(m, m->blocks[i], ws, p, &planes, want, stream))) return rc;
+        if ((rc = block_forward(m, m->blocks[i], ws, p, beside, &planes, want, stream))) return rc;
     }
     return linear(m->dtype, ws + p.x, (int64_t)m->T * m->D, m->head_w, m->head_b, nullptr, 0, logits, m->classes, m->B,
                   m->classes, m->D, 0, true, stream);

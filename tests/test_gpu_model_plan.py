@@ -137,3 +137,23 @@ def test_weights_written_by_the_launch_before_a_forward(cfg):
             for n, p in m.named_parameters():
                 p.copy_(kept[turn % 3][n])                      # the last of these is the launch before the forward's
             assert torch.equal(m(x), want[turn % 3])
+
+
+@pytest.mark.parametrize("heads,conv", [(3, "depthwise"), (3, "standard"), (1, "depthwise"), (1, "depthwise-separable")])
+@pytest.mark.parametrize("layer", ["BranchConv", "BranchAttention"])
+@pytest.mark.parametrize("B", [1, 5, 40])
+def test_halves_side_by_side_give_the_bits_of_one_after_the_other(layer, heads, conv, B):
+    """A branching block's halves run beside each other where the workspace has room for both; one page less, and they do not."""
+    torch.manual_seed(3)
+    m = convnn_b200.ViT(convnn_b200.make_args(layer=layer, num_layers=4, num_heads=heads, d_hidden=192, d_mlp=768, dropout=0.0,
+                                              attention_dropout=0.0, num_classes=24, convolution_type=conv,
+                                              device=DEV)).to(torch.bfloat16).eval()
+    x = torch.randn(B, 3, 224, 224, device=DEV).bfloat16()
+    with torch.no_grad():
+        want = _op_by_op(m, x)
+        got = [_planned(m, x) for _ in range(20)]
+        plan = model_plan._plans[m][(x.shape, x.dtype, x.device)]
+        plan.workspace_bytes -= 256
+        got += [m(x) for _ in range(3)]
+        assert model_plan._plans[m][(x.shape, x.dtype, x.device)] is plan
+    assert all(torch.equal(y, want) for y in got)
