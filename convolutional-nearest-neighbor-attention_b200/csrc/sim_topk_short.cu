@@ -1,22 +1,31 @@
 // Similarity + top-K for short candidate lists (S <= 256): a row's whole similarity vector is one accumulator in tensor
 // memory, so the selection can read it twice.
 //
-//   pass 1  values only: a sorted list of the best NSEL keys, two columns at a time.  With a >= b the merged list is
-//           v'[s] = max(v[s], min(v[s-1], a), min(v[s-2], b)): three instructions per slot and PAIR of columns, no
-//           branches, no indices, every slot computed from old values.
-//   pass 2  the nsel-th value is now the exact threshold: columns whose key reaches it (nsel of them unless keys tie there)
-//           are appended, in column order, to the row's entries in shared memory.
-//   rank    all pairs of entries are compared once; the earlier column wins ties.
+//   pass 1  a bound.  Lists of up to twelve: the maxima of 32 groups of columns (sixteen per half of a row, column modulo 16)
+//           are sorted by a network; the nsel-th largest of them is a key that at least nsel columns reach.  One maximum per
+//           column and 63 exchanges per sixteen groups, where a sorted list costs three instructions per slot and pair.
+//   pass 2  the columns whose key reaches the bound (about ten of 197 for K = 9) are appended, in column order, to the row's
+//           entries in shared memory, without a branch on how many there are.
+//   rank    the entries are inserted, in column order, into a sorted list in registers: the earlier column wins ties.
+//           A row with more entries than it has room for takes the columns above the bound chunk by chunk.
 //
-// A row with ties at the threshold or too few keys above -inf (NaN inputs) makes its warp repeat the selection with the
-// ordered insertion of the streaming kernels, so results are the same bit for bit.
+// Longer lists take the exact threshold in pass 1: a sorted list of the best NSEL keys, two columns at a time.  With a >= b the
+// merged list is v'[s] = max(v[s], min(v[s-1], a), min(v[s-2], b)), every slot computed from old values.  The entries of pass 2
+// are then nsel unless keys tie, and all pairs of them are compared once; a row with ties at the threshold or too few keys
+// above -inf (NaN inputs) makes its warp repeat the selection with the ordered insertion of the streaming kernels.
+// The results are the streaming kernels' bit for bit.
+//
+// What bounds it (128 images of 12 heads, 197 x 197 x 32, K = 9, 93 us; the streaming kernel 136): instructions, 4400 per 32 rows
+// at 0.47 per cycle and scheduler, and their fetch: a chunk loop unrolled once more 125 for 106, the metric known at compile
+// time 96 for 106, tensor-memory reads one chunk ahead nothing.  us, streaming -> this kernel: 256 images of 197 x 192, K = 9
+// 30.5 -> 20.7 (4: 22.8 -> 16.3), 6 heads of 64 126 -> 84, 65 x 65 x 192 12.5 -> 9.7, 1024 x 65 x 65, 3 heads of 64 94 -> 42,
+// 64 x 1000 x 200 x 256 33 -> 23, 256 x 197 x 64 x 384 17.8 -> 17.2.
 //
 // A persistent CTA per SM: warp 0 TMA producer (128 key rows + all candidate rows of one (batch, head), 64-channel chunks,
 // ring), warp 1 MMA issuer (M = 128, N = S rounded to 16), then selection warps (thread = row).  G accumulators of 512 / G
-// columns, G = 4 for S <= 128, else 2, so the next units' MMAs run under the selection.  With NH = 2 two warps share a row
+// columns, G = 4 for S <= 128 (narrow heads only, lists of up to nine), else 2, so the next units' MMAs run under the selection.  With NH = 2 two warps share a row
 // block of an accumulator, a column half each: the threshold follows from their two sorted lists (the n-th largest of
 // a and b is the largest min(a[i], b[n-2-i])), their entries grow towards each other, and they take turns at ranking.
-// (Eight selection warps, G = 2 and NH = 1, left each scheduler with two: 41 us at 256 images of 197 tokens, now 35.)
 #include "common.cuh"
 #include "sm100.cuh"
 #include "toplist.cuh"
@@ -75,11 +84,30 @@ __device__ __forceinline__ void merge_pair(float (&v)[NSEL], float k0, float k1)
     v[0] = fmaxf(v[0], a);
 }
 
+// Descending sort of 16 values (Batcher's odd-even merge exchange); exchanges that only order unused outputs fall away.
+__device__ __forceinline__ void sort16(float (&v)[16]) {
+#pragma unroll
+    for (int lp = 0; lp < 4; ++lp)
+#pragma unroll
+        for (int lk = lp; lk >= 0; --lk)
+#pragma unroll
+            for (int x = 0; x < 16; ++x) {
+                const int p = 1 << lp, k = 1 << lk, j = k % p;
+                if (x >= j && ((x - j) / k) % 2 == 0 && x + k < 16 && x / (2 * p) == (x + k) / (2 * p)) {
+                    const float a = v[x], b = v[x + k];
+                    v[x] = fmaxf(a, b);
+                    v[x + k] = fminf(a, b);
+                }
+            }
+}
+
 // Ranking keys of W accumulator columns from `col0` on; -inf past the last candidate.
-template <int W>
+// METRIC < 0: p.metric.  CLOSED: the statistics past the last candidate are NaN, and so are the keys (MATMUL has none).
+template <int W, int METRIC = -1, bool CLOSED = false>
 __device__ __forceinline__ void make_keys(float (&key)[W], const uint32_t (&acc)[W], const float* qs, const int* cs, int col0,
                                           const ShortParams& p, int row, float sentinel) {
-    if (p.metric != CONVNN_MATMUL) {
+    const int metric = METRIC < 0 ? p.metric : METRIC;
+    if (metric != CONVNN_MATMUL) {
         const f32x2 two = pack2(2.0f, 2.0f);
 #pragma unroll
         for (int j4 = 0; j4 < W / 4; ++j4) {
@@ -87,7 +115,7 @@ __device__ __forceinline__ void make_keys(float (&key)[W], const uint32_t (&acc)
             const f32x2 d01 = pack2(__uint_as_float(acc[4 * j4]), __uint_as_float(acc[4 * j4 + 1]));
             const f32x2 d23 = pack2(__uint_as_float(acc[4 * j4 + 2]), __uint_as_float(acc[4 * j4 + 3]));
             f32x2 k01, k23;
-            if (p.metric == CONVNN_COSINE) {
+            if (metric == CONVNN_COSINE) {
                 k01 = mul2(d01, pack2(s4.x, s4.y));
                 k23 = mul2(d23, pack2(s4.z, s4.w));
             } else {
@@ -111,6 +139,7 @@ __device__ __forceinline__ void make_keys(float (&key)[W], const uint32_t (&acc)
             if (c4.w == row) key[4 * j4 + 3] = sentinel;
         }
     }
+    if (CLOSED && metric != CONVNN_MATMUL) return;
     const int left = p.S - col0;
     if (left < W) {
 #pragma unroll
@@ -119,23 +148,43 @@ __device__ __forceinline__ void make_keys(float (&key)[W], const uint32_t (&acc)
     }
 }
 
-template <int NSEL, int G, int NH>
+template <int NSEL, int J, class E>
+__device__ __forceinline__ void insert_first(TopList<NSEL>& top, const E& entry, int cnt) {
+    if constexpr (J < NSEL) {
+        if (J < cnt) {
+            const float2 x = entry(J);
+            top.template insert_sorted_first<J>(x.x, __float_as_int(x.y));
+        }
+        insert_first<NSEL, J + 1>(top, entry, cnt);
+    }
+}
+
+// Lists whose rows are bounded by group maxima, and the entries a row has room for then (a side is checked every eight columns).
+template <int NSEL, int NH>
+constexpr bool bounded = NSEL <= 9 || (NSEL <= 12 && NH == 2);
+template <int NSEL, int NH>
+constexpr int slots_of = bounded<NSEL, NH> ? (NH == 2 ? 28 : 32) : NSEL + 2;
+
+template <int NSEL, int G, int NH, int METRIC>
 __global__ void __launch_bounds__(64 + 128 * G * NH, 1)
 sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const ShortParams p) {
     constexpr int MAXC = 512 / G;                  // tensor-memory columns of one accumulator
     constexpr int W = G * NH == 4 ? 16 : 32;       // columns per read (18 warps leave 96 registers per thread)
     constexpr int NT = 128 * G * NH;               // selection threads
     constexpr uint32_t ENTRY = 128 * G * 8;        // bytes between a row's successive entries
+    constexpr bool BOUND = bounded<NSEL, NH>;
+    constexpr int SLOTS = slots_of<NSEL, NH>;
+    constexpr bool LISTS = BOUND || NH == 2;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t pitch = p.KCH * 2;
     const uint32_t a_bytes = BM * pitch, b_bytes = p.BN * pitch, stage_bytes = a_bytes + b_bytes;
     const uint32_t STAGES = p.stages;
-    float2* hits = reinterpret_cast<float2*>(smem + STAGES * stage_bytes);       // [NSEL + 2][128 * G] (key, column)
-    float* statbuf = reinterpret_cast<float*>(hits + (NSEL + 2) * 128 * G);      // [warps][MAXC] column statistics
+    float2* hits = reinterpret_cast<float2*>(smem + STAGES * stage_bytes);       // [SLOTS][128 * G] (key, column)
+    float* statbuf = reinterpret_cast<float*>(hits + SLOTS * 128 * G);      // [warps][MAXC] column statistics
     int* cs = reinterpret_cast<int*>(statbuf + NT / 32 * MAXC);                  // [MAXC] candidate tokens
-    float* lists = reinterpret_cast<float*>(cs + MAXC);                          // NH = 2: [NSEL][NT] sorted keys
-    int* counts = reinterpret_cast<int*>(lists + (NH == 2 ? NSEL * NT : 0));     //         [NT] entries
+    float* lists = reinterpret_cast<float*>(cs + MAXC);                          // LISTS: [NSEL][NT] sorted keys
+    int* counts = reinterpret_cast<int*>(lists + (LISTS ? NSEL * NT : 0));       // NH = 2: [NT] entries
     uint64_t* full = reinterpret_cast<uint64_t*>(counts + (NH == 2 ? NT : 0));
     uint64_t* empty = full + MAX_STAGES;
     uint64_t* tfull = empty + MAX_STAGES;
@@ -250,7 +299,7 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
             if (p.metric != CONVNN_MATMUL) {
                 const float* qrow = p.qstat + (long long)bh * p.S;
 #pragma unroll
-                for (int c = 0; c < MAXC; c += 32) qs[c + lane] = c + lane < p.S ? qrow[c + lane] : 0.f;
+                for (int c = 0; c < MAXC; c += 32) qs[c + lane] = c + lane < p.S ? qrow[c + lane] : (BOUND ? CUDART_NAN_F : 0.f);
             }
             __syncwarp();
             ok = mbar_wait(&tfull[g], use & 1u, abort_flag);
@@ -259,6 +308,146 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
             tc_fence_after_sync();
             bool exact = true;
             int n_low = 0;
+            if constexpr (BOUND) {
+                int cnt = 0;
+                if (warp_live) {
+                    // Pass 1: maxima of column groups, sixteen per half of a row (NH = 1: of the even and the odd chunks).
+                    float v[16], w[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = w[j] = -CUDART_INF_F;
+                    auto into = [&](float (&m)[16], int c) {
+                        uint32_t acc[16];
+                        tmem_ld_x16(taddr + c, acc);
+                        tmem_ld_wait();
+                        float key[16];
+                        make_keys<16, METRIC, true>(key, acc, qs, cs, c, p, row, sentinel);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) m[j] = fmaxf(m[j], key[j]);
+                    };
+#pragma unroll 1
+                    for (int c = c_begin; c < c_end; c += NH == 2 ? 16 : 32) {
+                        into(v, c);
+                        if (NH == 1 && c + 16 < c_end) into(w, c + 16);
+                    }
+                    sort16(v);
+                    if (NH == 1) sort16(w);
+#pragma unroll
+                    for (int s = 0; s < NSEL; ++s) lists[s * NT + tid] = NH == 1 ? w[s] : v[s];
+                    if (NH == 2) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&xlist[xb]);
+                        ok = mbar_wait(&xlist[xb], use_of_pair & 1u, abort_flag);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) { if (lane == 0) fail(abort_flag, 75); break; }
+                    }
+                    // the nsel-th largest of both lists
+                    float thr = v[0];
+#pragma unroll
+                    for (int s = 1; s < NSEL; ++s) thr = fminf(thr, s < p.nsel ? v[s] : CUDART_INF_F);
+                    thr = fmaxf(thr, lists[(p.nsel - 1) * NT + peer]);
+#pragma unroll
+                    for (int i = 0; i < NSEL - 1; ++i)
+                        if (i < p.nsel - 1) thr = fmaxf(thr, fminf(v[i], lists[(p.nsel - 2 - i) * NT + peer]));
+                    // Pass 2: the columns that reach it.
+                    constexpr int ROOM = SLOTS - 8;
+                    const uint32_t first = half ? hit0 + (SLOTS - 1) * ENTRY : hit0;
+                    const uint32_t step = half ? 0u - ENTRY : ENTRY;
+                    uint32_t at = first;
+                    bool over = false;
+#pragma unroll 1
+                    for (int c = c_begin; c < c_end; c += 16) {
+                        uint32_t acc[16];
+                        tmem_ld_x16(taddr + c, acc);
+                        tmem_ld_wait();
+                        float key[16];
+                        make_keys<16, METRIC, true>(key, acc, qs, cs, c, p, row, sentinel);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            if (j % 8 == 0) {
+                                const bool full_up = (half ? first - at : at - first) > ROOM * ENTRY;
+                                over = over || full_up;
+                                at = full_up ? first + ROOM * step : at;
+                            }
+                            if (key[j] >= thr) {
+                                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(__float_as_uint(key[j])), "r"(c + j)
+                                             : "memory");
+                                at += step;
+                            }
+                        }
+                    }
+                    cnt = (int)((half ? first - at : at - first) / ENTRY);
+                    if (over) cnt = SLOTS + 1;
+                    n_low = cnt;
+                    if (NH == 2) {
+                        counts[tid] = cnt;
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&xhits[xb]);
+                        if (ranks) {
+                            ok = mbar_wait(&xhits[xb], use_of_pair & 1u, abort_flag);
+                            ok = __all_sync(0xffffffffu, ok);
+                            if (!ok) { if (lane == 0) fail(abort_flag, 76); break; }
+                            const int other = counts[peer];
+                            n_low = half ? other : cnt;
+                            cnt += other;
+                        }
+                        ++use_of_pair;
+                    }
+                    if (!row_ok) cnt = 0;
+                    exact = cnt <= SLOTS;
+                    if (ranks && !__all_sync(0xffffffffu, exact)) {
+                        // More columns reach the bound than a row has room for: chunk by chunk into the list.
+                        TopList<NSEL> top;
+                        top.init();
+                        const float floor = just_below(thr);
+#pragma unroll 1
+                        for (int c = 0; c < p.S; c += 16) {
+                            uint32_t acc[16];
+                            tmem_ld_x16(taddr + c, acc);
+                            tmem_ld_wait();
+                            float key[16];
+                            make_keys<16, METRIC, true>(key, acc, qs, cs, c, p, row, sentinel);
+                            const float low = fmaxf(top.worst(), floor);
+                            uint32_t mask = 0;
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                mask |= key[j] > low ? 1u << j : 0u;
+                                if (!exact) hits[j * 128 * G + g * 128 + r].x = key[j];
+                            }
+                            if (exact) mask = 0;
+                            const int steps = __reduce_max_sync(0xffffffffu, __popc(mask));
+                            for (int it = 0; it < steps; ++it) {
+                                const int j = mask ? __ffs(mask) - 1 : 0;
+                                const float kc = hits[j * 128 * G + g * 128 + r].x;
+                                if (mask && kc > top.worst()) top.insert_sorted(kc, c + j);
+                                mask &= mask - 1;
+                            }
+                        }
+                        if (!exact) write_selection<NSEL>(top, p, ((long long)bh * p.T + row) * p.K, row, kst);
+                    }
+                }
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&tempty[g]);
+                if (ranks && warp_live) {
+                    // The entries, in column order, into the sorted list.
+                    const float2* e = hits + g * 128 + r;
+                    auto entry = [&](int n) { return e[(NH == 1 || n < n_low ? n : SLOTS - 1 + n_low - n) * 128 * G]; };
+                    if (!exact) cnt = 0;
+                    TopList<NSEL> top;
+                    top.init();
+                    insert_first<NSEL, 0>(top, entry, cnt);
+                    const int most = __reduce_max_sync(0xffffffffu, cnt);
+#pragma unroll 1
+                    for (int n = NSEL; n < most; ++n) {
+                        if (n < cnt) {
+                            const float2 x = entry(n);
+                            top.insert_sorted(x.x, __float_as_int(x.y));
+                        }
+                    }
+                    if (row_ok && exact) write_selection<NSEL>(top, p, ((long long)bh * p.T + row) * p.K, row, kst);
+                }
+                continue;
+            }
             if (warp_live) {
                 float v[NSEL];
 #pragma unroll
@@ -406,36 +595,47 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     }
 }
 
-template <int NSEL, int G, int NH>
-int launch_short(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const CUtensorMap& tmQ, cudaStream_t st) {
+template <int NSEL, int G, int NH, int METRIC>
+int launch_metric(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const CUtensorMap& tmQ, cudaStream_t st) {
     constexpr int MAXC = 512 / G;
     const size_t stage = (size_t)(BM + p.BN) * p.KCH * 2;
     constexpr int NT = 128 * G * NH;
-    const size_t fixed = 1024 + (size_t)(NSEL + 2) * 128 * G * 8 + (size_t)(NT / 32 + 1) * MAXC * 4 +
-                         (NH == 2 ? (size_t)(NSEL + 1) * NT * 4 : 0) + (2 * MAX_STAGES + 10 * G) * 8 + 16;
+    const size_t fixed = 1024 + (size_t)slots_of<NSEL, NH> * 128 * G * 8 + (size_t)(NT / 32 + 1) * MAXC * 4 +
+                         (bounded<NSEL, NH> || NH == 2 ? (size_t)(NSEL + 1) * NT * 4 : 0) + (2 * MAX_STAGES + 10 * G) * 8 + 16;
     p.stages = (int)((226 * 1024 - fixed) / stage);
     if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
     if (p.stages > 2 * p.KC) p.stages = 2 * p.KC;            // deeper than two units' chunks serves nothing
     size_t smem = fixed + p.stages * stage;
     if (smem < 116 * 1024) smem = 116 * 1024;                // a CTA takes all of an SM's TMEM: never two on one SM
     const int sms = device_sms();
-    auto kern = sim_topk_short_kernel<NSEL, G, NH>;
+    auto kern = sim_topk_short_kernel<NSEL, G, NH, METRIC>;
     CONVNN_ENSURE_SMEM(kern, smem);
     launch_chained(kern, p.n_units < sms ? p.n_units : sms, 64 + NT, smem, st, tmK, tmQ, p);
     CONVNN_CHECK_LAUNCH("sim_topk_short");
     return CONVNN_OK;
 }
 
+template <int NSEL, int G, int NH>
+int launch_short(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const CUtensorMap& tmQ, cudaStream_t st) {
+    if constexpr (bounded<NSEL, NH>) {
+        if (p.metric == CONVNN_COSINE) return launch_metric<NSEL, G, NH, CONVNN_COSINE>(dm, p, tmK, tmQ, st);
+        if (p.metric == CONVNN_MATMUL) return launch_metric<NSEL, G, NH, CONVNN_MATMUL>(dm, p, tmK, tmQ, st);
+        return launch_metric<NSEL, G, NH, CONVNN_EUCLIDEAN>(dm, p, tmK, tmQ, st);
+    } else {
+        return launch_metric<NSEL, G, NH, -1>(dm, p, tmK, tmQ, st);
+    }
+}
+
 }  // namespace
 
-// What the warp-per-row kernel leaves to it where the streaming kernel would leave most of the chip idle: up to one unit per SM.  us,
-// streaming -> this kernel: 148 x 100 x 100 x 64, K = 9 11.5 -> 9.5, 74 x 197 x 64 x 384 12.9 -> 9.3, 37 x 197 x 197 x 768 22.8 -> 18.0, 48 x
-// 197 x 197 x 192, K = 25 33.8 -> 23.0.  With several units per SM eight to sixteen streaming warps hide each other's latency (256 images
-// of 197 x 192, K = 9: 30.8, 34.6 here).  Lists of 13 to 16 always: their streaming variant runs one CTA per SM (256 x 577 x 150 x 384,
-// K = 16 129 -> 110; 256 x 197 x 197 x 192 47.0 -> 49.0).
+// What the warp-per-row kernel leaves to it.  Lists of up to twelve, except for up to 32 candidates of sequences that fill more
+// than one of its units, where the streaming kernel's 256-row units are fewer and the bound saves little (us, streaming, this
+// kernel: 512 x 197 x 16 x 192, K = 4 10.8, 14.4; 256 x 197 x 32 x 768, K = 3 19.6, 21.9; 300 images of 17 x 17 x 64 with three
+// heads, K = 5 15.8, 10.8).  Lists of 13 to 16: their streaming variant runs one CTA per SM (256 x 577 x 150 x 384, K = 16 129, 110;
+// 256 x 197 x 197 x 192 47, 49).  Anything of up to one unit per SM (48 x 197 x 197 x 192, K = 25 33.8, 23.0).
 bool sim_topk_short_wanted(const Dims& dm) {
     const long long units = (long long)dm.B * dm.H * ((dm.T + BM - 1) / BM);
-    return dm.S <= 256 && (units <= device_sms() || (dm.nsel > 12 && dm.nsel <= 16));
+    return dm.S <= 256 && (units <= device_sms() || (dm.nsel <= 16 && (dm.nsel > 12 || dm.S > 32 || dm.T <= BM)));
 }
 
 int launch_sim_topk_short(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
@@ -461,16 +661,21 @@ int launch_sim_topk_short(const convnn_desc* d, const Dims& dm, const void* q, c
     if (!encode_tensor_map_bf16(&tmQ, q, 4, dimsQ, strQ, boxQ, p.KCH * 2)) return CONVNN_E_CUDA;
 
     const int n = dm.nsel;
+    // One thread per row and four accumulators for up to 128 candidates, if many units follow one another and the heads are
+    // narrow: its entries leave the ring two stages (us, this form, the other: 256 x 197 x 64, K = 9, three heads of 64 29.3, 33.6;
+    // 1024 x 65 x 65, three heads of 64 42, 58; 256 x 197 x 64 x 384 19.3, 17.2; 1024 x 64 x 64 x 384 37, 25).
+    const bool narrow = dm.S <= 128 && dm.Cp <= 256 && p.n_units > device_sms();
 #define CONVNN_SHORT(N)                                                     \
     do {                                                                    \
-        if (dm.S <= 128) return launch_short<N, 4, 1>(dm, p, tmK, tmQ, st);    \
+        if (narrow) return launch_short<N, 4, 1>(dm, p, tmK, tmQ, st);    \
         return launch_short<N, 2, 2>(dm, p, tmK, tmQ, st);                     \
     } while (0)
     if (n <= 4) CONVNN_SHORT(4);
     if (n <= 8) CONVNN_SHORT(8);
     if (n == 9) CONVNN_SHORT(9);
-    if (n <= 12) CONVNN_SHORT(12);
-    if (n <= 16) CONVNN_SHORT(16);
+    if (n <= 12) return launch_short<12, 2, 2>(dm, p, tmK, tmQ, st);
+    if (n <= 16 && dm.S <= 128) return launch_short<16, 4, 1>(dm, p, tmK, tmQ, st);
+    if (n <= 16) return launch_short<16, 2, 2>(dm, p, tmK, tmQ, st);
     // (longer lists: their exchange buffers would take the ring's shared memory)
     if (n <= 25) return launch_short<25, 2, 1>(dm, p, tmK, tmQ, st);
     return launch_short<32, 2, 1>(dm, p, tmK, tmQ, st);

@@ -167,3 +167,39 @@ def test_warp_per_row_routes(B, T, S, H, dk, K, dtype, rows):
     cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if S != T else None
     names = launches(lambda: ops.sim_topk(spec, q, k, None, None, cand))
     assert len(names) == 1 and any(n in next(iter(names)) for n in ("sim_topk_rows_kernel", "sim_topk_simt_rows_kernel")) == rows
+
+
+# Several 128-row units per SM.  (80 x 197 x 64 with one accumulator in four and one in two; 33 to 48 candidates leave the upper
+# half of a row a chunk or nothing; 208 and 256 end on a whole chunk; "few" values tie, so that most rows overflow their entries;
+# "stripes" puts the best sixteen columns into one group of maxima.)
+@pytest.mark.parametrize("B,T,S,H,dk", [(160, 17, 17, 1, 64), (80, 197, 33, 1, 64), (80, 197, 64, 1, 384), (160, 128, 128, 1, 192),
+                                        (60, 129, 48, 3, 16), (80, 197, 197, 1, 32), (60, 300, 208, 1, 512), (320, 256, 256, 1, 64)])
+@pytest.mark.parametrize("K", [1, 3, 8, 9, 12])
+@pytest.mark.parametrize("values", ["few", "many", "nan", "stripes"])
+def test_exact_lists_of_many_units(B, T, S, H, dk, K, values):
+    sampled = S != T
+    n = K - 1 if sampled else K
+    if n < 1:
+        pytest.skip("the row itself is all of the list")
+    g = torch.Generator(device=DEV).manual_seed(T * 1000 + S + K)
+    top = 1 if values == "few" else 11               # products and sums stay far below 2^24
+    q, k = (torch.randint(-top, top + 1, (B, r, H, dk), device=DEV, generator=g).float() for r in (S, T))
+    if values == "nan":
+        q[:, ::3] = math.nan
+        q[1, 2:] = math.nan
+    if values == "stripes":
+        q[:, ::16] = q[:, ::16].abs() + 12
+        k = k.abs()
+    spec = ops.LayerSpec(H * dk, H, K, "spatial" if sampled else "all", "matmul", "depthwise", True, False, T)
+    cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if sampled else None
+    idx, val = ops.sim_topk(spec, q.bfloat16(), k.bfloat16(), None, None, cand)
+    key = torch.einsum("bthc,bshc->bhts", k.double(), q.double()).float()
+    if sampled:
+        own = cand.view(1, 1, 1, S).long() == torch.arange(T, device=DEV).view(1, 1, T, 1)
+        key = torch.where(own, torch.full_like(key, -0.1) * torch.tensor(math.sqrt(dk), dtype=torch.float32), key)
+    want_idx, want_key = expect(key, n)
+    assert torch.equal(idx.long()[..., K - n:], want_idx if cand is None else cand.long()[want_idx])
+    real = (want_key > -math.inf) & ~((want_key < 0) & (val[..., K - n:] == -0.1))
+    want_val = want_key / torch.tensor(math.sqrt(dk), dtype=torch.float32)
+    # one division: equal up to its rounding
+    assert bool(((val[..., K - n:] - want_val).abs() <= 2.0 ** -22 * want_val.abs())[real].all())
