@@ -42,7 +42,7 @@ def _worker(rank, world, port, total, q):
             model.bias.zero_()
         out = sharded_forward(model, images)
         cand = shared_candidates(65, 16, torch.device("cpu"), seed=3)
-        q.put((rank, out, cand))
+        q.put((rank, out.numpy(), cand.numpy()))        # by value: a tensor would be fetched from a process that may be gone
     finally:
         dist.destroy_process_group()
 
@@ -56,6 +56,7 @@ def test_two_ranks_reproduce_single_process(total):
     for p in procs:
         p.start()
     got = [q.get(timeout=120) for _ in procs]
+    got = [(rank, torch.from_numpy(out), torch.from_numpy(cand)) for rank, out, cand in got]
     for p in procs:
         p.join(timeout=60)
         assert p.exitcode == 0
