@@ -396,6 +396,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             int tn = 0;
             const uint32_t peer_empty0 = PAIR ? map_to_cta(empty0, 1) : 0u;
             const uint32_t peer_tfull0 = PAIR ? map_to_cta(tfull0, 1) : 0u;
+            chain_wait_unless(p.beside);                     // (the budgets of its waits are for this kernel's work)
             for (int t = first; t < last && ok; t += step, ++tile) {
                 const uint32_t buf = tile & 1u, u = tile >> 1;
                 if (!mbar_wait_a(tempty0 + 8 * buf, (u & 1u) ^ 1u, abort_flag)) { give_up(12); ok = false; break; }

@@ -338,6 +338,7 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
                     mtrace(cluster_id == 0, 4, n);
                 }
             };
+            chain_wait();                                          // (the budgets of its waits are for this kernel's work)
             if (OP && my_tiles > 0) mma_wo(0);
             for (int it = 0; it < my_tiles && ok; ++it) {
                 const uint32_t xb = (uint32_t)it & 1u;
@@ -375,6 +376,7 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
             const uint32_t d2 = tmem_base + acc2_col;
             uint32_t s = 0, ph = 0;
             int c = 0, it = 0;
+            chain_wait();
             for (uint32_t g = 0; g < total; ++g) {
                 const uint32_t hb = g & 1u;                       // h chunk = half of its super-chunk
                 if (c == 0 && !mbar_wait_a(lbar(A2EMPTY), ((uint32_t)it & 1u) ^ 1u, abort_flag)) { give_up(58); break; }
@@ -406,8 +408,9 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
             uint32_t s = 0, ph = 0;
             int c = 0;
             const int nch = nsc * 2;
-            if (!p.weights_at_rest) chain_wait();
+            const uint32_t ahead = p.weights_at_rest ? NSW2 : 0u;       // a ring of chunks before the predecessor has ended
             for (uint32_t g = 0; g < total; ++g) {
+                if (g == ahead) chain_wait();
                 if (!mbar_wait_a(lbar(W2EMPTY + s), ph ^ 1u, abort_flag)) { give_up(53); break; }
                 mtrace(cluster_id == 0 && rank == 0, 0, g);
                 if (rank == 0) mbar_expect_tx_a(lbar(W2FULL + s), 2u * (uint32_t)(p.D / 2) * 128u);

@@ -250,6 +250,7 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             const uint32_t tfull0 = smem_u32(tfull), tempty0 = smem_u32(tempty);
             uint32_t s = 0, ph = 0, buf = 0, use = 0;
             bool ok = true;
+            chain_wait();                            // (the budgets of its waits are for this kernel's work)
             for (Segment sg(p); sg.valid() && ok; sg.next(p)) {
                 if (!mbar_wait_a(tempty0 + 8 * buf, (use & 1u) ^ 1u, abort_flag)) { fail(abort_flag, 82); break; }
                 tc_fence_after_sync();

@@ -154,6 +154,7 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
             const uint32_t tfull0 = smem_u32(tfull), tempty0 = smem_u32(tempty);
             uint32_t s = 0, ph = 0, tile = 0;
             bool ok = true;
+            chain_wait();                            // (the budgets of its waits are for this kernel's work)
             for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x) {
                 const int pp = unit % p.n_pairs;
                 const bool has1 = pp * 2 * BM + BM < p.T;

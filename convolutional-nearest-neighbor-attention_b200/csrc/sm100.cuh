@@ -45,9 +45,11 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Bounded wait: gives up once `budget_ns` of wall time (the GPU's nanosecond timer) have passed
 // or as soon as *abort becomes non-zero, and reports failure so the caller can record an error
 // and leave instead of hanging the GPU.  The timer is read once per 256 polls; an extra poll
-// counter backs it up should the timer not advance.  In normal operation no wait of these
-// kernels lasts longer than the epilogue of one tile (tens of microseconds); the budget only has
-// to exceed that under time slicing or a profiler's replay.
+// counter backs it up should the timer not advance.  No role polls for what can only come after
+// the predecessor on the stream has ended (it waits for that first, see chain_wait(), which has no
+// limit), so in normal operation no wait of these kernels lasts longer than the epilogue of one
+// tile (tens of microseconds); the budget only has to exceed that under time slicing or a
+// profiler's replay.
 constexpr unsigned long long kWaitBudgetNs = 250ull * 1000 * 1000;
 constexpr uint32_t kWaitPollLimit = 1u << 28;
 __device__ __forceinline__ unsigned long long global_timer_ns() {
