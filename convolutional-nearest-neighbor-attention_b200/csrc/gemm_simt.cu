@@ -600,43 +600,44 @@ int launch_copy_tile(const GemmParams& p, cudaStream_t st) {
     return CONVNN_OK;
 }
 
-// Plain rows: the tile with the shortest time on the busiest SM, which runs `fit` tiles at a time.  `step` is what a k
-// step takes there with 1, 2, ... tiles side by side, ns.  The numbers are fits to measured times (rms 3 to 7 %).
+// Plain rows: the tile with the shortest time on the busiest SM, which runs `fit` tiles at a time.  `step` is what a value of
+// k takes there with 1, 2, ... tiles side by side, ns, in whole steps of `bk` of them.  The numbers are fits to measured times.
 struct Tile {
-    int bm, bn, fit;
-    double launch, round, step[6];        // us per launch and per round of tiles
+    int bm, bn, bk, fit;
+    double launch, round, step[7];        // us per launch and per round of tiles
 };
 template <int COUNT>
 int cheapest_tile(const Tile (&tiles)[COUNT], const GemmParams& p, int first = 0) {
     const long long sms = device_sms();
-    int best = first;
+    int best = -1;
     double least = 0;
     for (int i = first; i < COUNT; ++i) {
         const Tile& t = tiles[i];
         if (t.bn < 64 && (p.N + t.bn - 1) / t.bn > 65535) continue;      // (grid rows)
         const long long n = (long long)((p.M + t.bm - 1) / t.bm) * ((p.N + t.bn - 1) / t.bn), per_sm = (n + sms - 1) / sms;
         const long long full = per_sm / t.fit, rest = per_sm % t.fit;
-        double cost = t.launch + (full + (rest ? 1 : 0)) * t.round + 1e-3 * p.Kd * full * t.step[t.fit - 1];
-        if (rest) cost += 1e-3 * p.Kd * t.step[rest - 1];
-        if (i == first || cost < least) { least = cost; best = i; }
+        const double k = 1e-3 * t.bk * ((p.Kd + t.bk - 1) / t.bk);
+        double cost = t.launch + (full + (rest ? 1 : 0)) * t.round + k * full * t.step[t.fit - 1];
+        if (rest) cost += k * t.step[rest - 1];
+        if (best < 0 || cost < least) { least = cost; best = i; }
     }
     return best;
 }
 
 // float32 rows that can be copied.  A tile of two warps leaves two of the four schedulers idle, so tiles come in pairs.
-// Over 396 shapes (65 to 25216 rows, 10 to 2304 columns, 64 to 1536 values of k) the choice is within 0.6 % of the
+// Over 396 shapes (65 to 25216 rows, 10 to 2304 columns, 64 to 1536 values of k; rms 3 to 7 %) the choice is within 0.6 % of the
 // best of twelve tiles on average, 12 % at worst.  With the first two tiles alone (and smaller transposed ones, since
 // gone) 2080 rows took 33.0 us at 192 x 768, now 25.8; 20.6 at 576 x 192, now 17.8; 1576 x 384 x 192 15.5, now 11.5; 1050
 // x 384 x 384 18.7, now 15.6.
 template <int MODE>
 int launch_plain_f32(const GemmParams& p, cudaStream_t st) {
     static const Tile tiles[6] = {
-        {128, 64, 3, 5.4, 0.5, {65.4, 107.1, 153.3}},
-        {64, 64, 3, 3.2, 0.7, {38.2, 62.3, 88.9}},
-        {32, 32, 6, 1.7, 1.5, {19.6, 20.9, 33.3, 35.3, 51.4, 48.7}},
-        {40, 32, 6, 2.2, 1.6, {23.5, 25.2, 38.8, 39.7, 61.1, 58.2}},
-        {48, 32, 5, 2.2, 2.3, {26.3, 28.8, 42.9, 46.8, 60.0}},
-        {56, 32, 5, 1.9, 3.1, {30.2, 32.5, 50.4, 53.8, 72.0}},
+        {128, 64, 1, 3, 5.4, 0.5, {65.4, 107.1, 153.3}},
+        {64, 64, 1, 3, 3.2, 0.7, {38.2, 62.3, 88.9}},
+        {32, 32, 1, 6, 1.7, 1.5, {19.6, 20.9, 33.3, 35.3, 51.4, 48.7}},
+        {40, 32, 1, 6, 2.2, 1.6, {23.5, 25.2, 38.8, 39.7, 61.1, 58.2}},
+        {48, 32, 1, 5, 2.2, 2.3, {26.3, 28.8, 42.9, 46.8, 60.0}},
+        {56, 32, 1, 5, 1.9, 3.1, {30.2, 32.5, 50.4, 53.8, 72.0}},
     };
     switch (cheapest_tile(tiles, p)) {
         case 0: return launch_tile<float, float, MODE, 128, 64, 16, 8, 8, 3>(p, st);
@@ -648,24 +649,51 @@ int launch_plain_f32(const GemmParams& p, cudaStream_t st) {
     }
 }
 
-// Other plain rows (bfloat16, float32 against bfloat16 weights, rows of any alignment).  Over 146 bfloat16 shapes within 1 % of the best
-// of nine tiles on average, 18 % at worst, and 0.71 of the time of the transposed tiles that were here (which waited for
-// their operands to be converted and stored value by value), the first tile only where rows are read four values at a time (4039
-// x 768 x 385 135 us, the second 93); us: 2080 x 384 x 388 57.9, now 27.8; 4039 x 384 x 388 51.9, now 44.3; the separable conv with the coordinate channel (rows of d_k + 1 values) of 7 x 577 tokens, 384 channels 89.8, now 68.1; 4 x 197 x 768
-// 130 -> 55; 197 x 192 29.0 -> 16.3.
+// Other plain rows: float32 ones of any alignment, bfloat16, float32 against bfloat16 weights.  Which tiles, and which times, goes by
+// what the operands cost: float32 values need no conversion, so that the transposed tiles wait for little and the largest of
+// them reuses most; bfloat16 values that come one by one are what the transposed tiles wait for.  Narrow outputs of few
+// values of k (the separable conv with the coordinate channel on heads of 8 to 32) end before that counts.  Fits to 209, 98
+// and 98 shapes (30 to 100000 rows, 8 to 2304 columns, 9 to 2048 values of k; rms 9 to 21 %), the choice within 1.2, 1.5 and
+// 0.8 % of the best of seven tiles on average; 0.95, 0.72 and 0.62 of the time of the four transposed tiles alone, at worst 1.08 (4 us).
+// float32, us, staged tiles only -> now: 2813 x 768 x 769 138 -> 102, 56288 x 256 x 257 244 -> 189, 39846 x 8 x 9 9.9 -> 6.7.
+// bfloat16, transposed tiles only -> now: 4 x 197 x 768 x 768 130 -> 55; 2080 x 384 x 388 57.9 -> 27.8.
 template <typename TA, typename T, int MODE>
 int launch_plain_staged(const GemmParams& p, cudaStream_t st) {
-    static const Tile tiles[4] = {
-        {128, 64, 3, 6.4, 0.0, {124.7, 163.2, 198.0}},
-        {64, 64, 3, 0.8, 5.4, {40.2, 64.4, 95.6}},
-        {32, 64, 4, 0.3, 3.6, {26.9, 45.3, 61.7, 77.4}},
-        {40, 32, 6, 0.0, 5.0, {31.9, 33.6, 49.2, 52.1, 70.4, 70.8}},
-    };
-    switch (cheapest_tile(tiles, p, p.a_vec && p.w_vec ? 0 : 1)) {
-        case 0: return launch_tile<TA, T, MODE, 128, 64, 16, 8, 8, 3>(p, st);
-        case 1: return launch_stage_tile<TA, T, MODE, 64, 64, 8, 4, 3>(p, st);
-        case 2: return launch_stage_tile<TA, T, MODE, 32, 64, 4, 4, 4>(p, st);
-        default: return launch_stage_tile<TA, T, MODE, 40, 32, 5, 4, 6>(p, st);
+    if constexpr (sizeof(T) == 4) {
+        static const Tile tiles[4] = {
+            {128, 64, 16, 3, 0.6, 4.8, {75.5, 117.3, 176.8}},
+            {64, 64, 32, 3, 2.9, 1.6, {43.8, 73.6, 105.2}},
+            {32, 32, 32, 7, 2.9, 0.0, {31.1, 35.7, 49.8, 65.0, 81.8, 88.6, 95.5}},
+            {32, 64, 32, 4, 2.0, 1.4, {30.0, 51.2, 66.6, 86.9}},
+        };
+        switch (cheapest_tile(tiles, p)) {
+            case 0: return launch_tile<TA, T, MODE, 128, 64, 16, 8, 8, 3>(p, st);
+            case 1: return launch_tile<TA, T, MODE, 64, 64, 32, 8, 4, 3>(p, st);
+            case 2: return launch_tile<TA, T, MODE, 32, 32, 32, 4, 4, 4>(p, st);
+            default: return launch_stage_tile<TA, T, MODE, 32, 64, 4, 4, 4>(p, st);
+        }
+    } else {
+        static const Tile by_four[5] = {
+            {128, 64, 16, 3, 6.1, 0.1, {114.3, 172.4, 213.5}},
+            {32, 32, 32, 7, 1.7, 0.7, {61.3, 66.3, 69.6, 67.3, 84.9, 69.6, 84.1}},
+            {64, 64, 32, 3, 3.2, 2.9, {40.5, 62.2, 101.5}},
+            {32, 64, 32, 4, 2.2, 1.6, {27.8, 42.1, 59.7, 78.7}},
+            {40, 32, 32, 6, 2.6, 2.5, {31.9, 34.4, 43.8, 46.8, 66.8, 75.5}},
+        };
+        static const Tile by_value[5] = {
+            by_four[0],                                              // (not taken: 4039 x 768 x 385 135 us, the third 93)
+            {32, 32, 32, 7, 1.1, 0.0, {108.4, 122.0, 111.1, 150.7, 131.6, 174.3, 135.2}},
+            {64, 64, 32, 3, 2.6, 3.6, {45.3, 68.7, 102.8}},
+            {32, 64, 32, 4, 2.1, 1.7, {31.9, 48.3, 65.4, 92.7}},
+            {40, 32, 32, 6, 2.3, 2.9, {36.8, 39.8, 54.5, 58.5, 83.1, 87.1}},
+        };
+        switch (p.a_vec && p.w_vec ? cheapest_tile(by_four, p) : cheapest_tile(by_value, p, 1)) {
+            case 0: return launch_tile<TA, T, MODE, 128, 64, 16, 8, 8, 3>(p, st);
+            case 1: return launch_tile<TA, T, MODE, 32, 32, 32, 4, 4, 4>(p, st);
+            case 2: return launch_stage_tile<TA, T, MODE, 64, 64, 8, 4, 3>(p, st);
+            case 3: return launch_stage_tile<TA, T, MODE, 32, 64, 4, 4, 4>(p, st);
+            default: return launch_stage_tile<TA, T, MODE, 40, 32, 5, 4, 6>(p, st);
+        }
     }
 }
 

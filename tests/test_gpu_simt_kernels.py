@@ -271,24 +271,24 @@ def test_three_outputs_of_float32_rows(B, T, S, D, H):
         assert torch.equal(got.reshape(-1, D), ops.linear(rows.reshape(-1, D), w[part]))
 
 
-# Every tile of the rows that come through registers: bfloat16 with k a multiple of four (read four at a time) and not, and
-# float32 rows that are not 16-byte aligned; a sum is the same whichever tile it was computed in.
+# Every tile of the rows that are not copied: bfloat16 with k a multiple of four (read four at a time) and not, and float32 rows
+# that are not 16-byte aligned ("staged" through registers, or transposed); a sum is the same whichever tile it was computed in.
 @on_148_sms
-@pytest.mark.parametrize("M,N,K,tile", [
-    (1, 1, 1, "32x64 4x4"), (65, 193, 385, "32x64 4x4"), (1050, 384, 388, "32x64 4x4"), (788, 768, 772, "40x32 5x4"),
-    (1576, 191, 196, "40x32 5x4"), (4039, 384, 385, "64x64 8x4"), (12001, 384, 197, "64x64 8x4"), (50433, 66, 65, "64x64 8x4"),
-    (50433, 66, 68, "transposed")])
+@pytest.mark.parametrize("M,N,K,bf16,fp32", [
+    (1, 1, 1, "32x32", "32x32"), (65, 193, 385, "32x64 staged", "32x32"), (1050, 384, 388, "32x64 staged", "64x64"),
+    (788, 768, 772, "40x32 staged", "32x64 staged"), (1576, 191, 196, "40x32 staged", "32x32"), (4039, 384, 385, "64x64 staged", "64x64"),
+    (12001, 384, 197, "64x64 staged", "128x64"), (50433, 66, 65, "64x64 staged", "128x64"), (50433, 66, 68, "128x64", "128x64"),
+    (12001, 16, 17, "32x32", "32x32"), (5001, 24, 28, "32x32", "32x32")])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-def test_tiles_of_staged_rows(M, N, K, tile, dtype):
+def test_tiles_of_staged_rows(M, N, K, bf16, fp32, dtype):
     g = torch.Generator(device=DEV).manual_seed(M + N)
     ld = K + (1 if dtype == torch.float32 or K % 4 else 4)           # (odd row strides keep float32 off the copies)
     a, w, b, r = (torch.randn(*s, device=DEV, generator=g).to(dtype) for s in ((M, ld), (N, K), (N,), (M, N)))
     a = a[:, :K]
     call = lambda: ops.linear(a, w, b, residual=r)
-    names = [re.search(r"gemm_simt_stage_kernelI.*?Li\dELi(\d+)ELi(\d+)ELi(\d+)ELi(\d+)E", n) for n in launches(call)]
-    if dtype == torch.float32 and tile == "transposed":
-        tile = "64x64 8x4"
-    assert [("{}x{} {}x{}".format(*m.groups()) if m else "transposed") for m in names] == [tile]
+    names = [re.search(r"gemm_simt_(stage_|copy_|)kernelI.*?Li\dELi(\d+)ELi(\d+)E", n).groups() for n in launches(call)]
+    assert [f"{bm}x{bn}" + {"stage_": " staged", "copy_": " copied", "": ""}[kind] for kind, bm, bn in names] == \
+        [fp32 if dtype == torch.float32 else bf16]
     got = call()
     want = a.double() @ w.double().T + b.double()
     step = 2.0 ** -8 if dtype == torch.bfloat16 else 2 * EPS         # the sum is rounded, then the skip connection added
