@@ -120,7 +120,8 @@ def test_layer_call_follows_changes_and_options():
 
 @pytest.mark.parametrize("cfg", sorted(CONFIGS))
 def test_weights_written_by_the_launch_before_a_forward(cfg):
-    """A forward's kernels may fetch weights early, but never ahead of what the stream did before the call."""
+    """Weights changed in stream order, without a wait, by other kernels than the library's: turn by turn the op-by-op path and a
+    new plan.  (Weights written by a library kernel that lets the next one start early: test_gpu_launch_order.py.)"""
     m = _model(cfg, torch.bfloat16)
     x = torch.randn(3, 3, 224, 224, device=DEV).bfloat16()
     kept = [{n: p.detach() * f for n, p in m.named_parameters()} for f in (0.5, 1.5, 1.0)]
@@ -135,7 +136,7 @@ def test_weights_written_by_the_launch_before_a_forward(cfg):
             m(x)
         for turn in range(12):
             for n, p in m.named_parameters():
-                p.copy_(kept[turn % 3][n])                      # the last of these is the launch before the forward's
+                p.copy_(kept[turn % 3][n])
             assert torch.equal(m(x), want[turn % 3])
 
 
