@@ -39,7 +39,6 @@ constexpr int NTHREADS = 192;      // TMA warp, MMA warp, 4 softmax warps
 constexpr int CW = 16;
 
 struct AttnParams {
-    int beside;             // see chain_leave()
     __nv_bfloat16* o;              // (B, T, H * dk)
     int T, H, dk, D;
     int KCH, KC;                   // channels per chunk / chunks of the Q K^T reduction
@@ -63,6 +62,7 @@ __device__ __forceinline__ void tmem_ld_wait_on(uint32_t (&r)[CW]) {
                  : "memory");
 }
 
+template <bool BESIDE>                    // see chain_leave()
 __global__ void __launch_bounds__(NTHREADS, 2)
 attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
@@ -113,7 +113,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_wait_unless(p.beside);
+    chain_wait_unless(BESIDE);
     chain_next();
 
     if (warp == 0) {
@@ -316,7 +316,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, ncols);
     }
-    chain_leave(p.beside);
+    chain_leave(BESIDE);
 }
 
 // One warp per query row; scores in shared memory.  float32 (and the fallback for shapes the
@@ -397,7 +397,6 @@ int launch_attention_tc(const void* q, const void* k, const void* v, void* o, in
                         7 * 8 + 16;
     if (smem > 227 * 1024) return set_error(CONVNN_E_UNSUPPORTED, "attention_tc: shape needs %zu bytes of shared memory", smem);
 
-    p.beside = beside;
     CUtensorMap tmQ, tmK, tmV;
     const uint64_t dims[4] = {(uint64_t)p.dk, (uint64_t)H, (uint64_t)Tn, (uint64_t)B};
     const uint64_t str[3] = {(uint64_t)p.dk * 2, (uint64_t)D * 2, (uint64_t)Tn * D * 2};
@@ -412,9 +411,13 @@ int launch_attention_tc(const void* q, const void* k, const void* v, void* o, in
     const int per_sm = smem <= 113 * 1024 && p.BNpad <= 256 ? 2 : 1;
     const int ctas = sms * per_sm;
     const int grid = p.n_units < ctas ? p.n_units : ctas;
-    auto kern = attention_tc_kernel;
-    CONVNN_ENSURE_SMEM(kern, smem);
-    launch_chained(kern, grid, NTHREADS, smem, st, tmQ, tmK, tmV, p);
+    if (beside) {
+        CONVNN_ENSURE_SMEM(attention_tc_kernel<true>, smem);
+        launch_chained(attention_tc_kernel<true>, grid, NTHREADS, smem, st, tmQ, tmK, tmV, p);
+    } else {
+        CONVNN_ENSURE_SMEM(attention_tc_kernel<false>, smem);
+        launch_chained(attention_tc_kernel<false>, grid, NTHREADS, smem, st, tmQ, tmK, tmV, p);
+    }
     CONVNN_CHECK_LAUNCH("attention_tc");
     return CONVNN_OK;
 }

@@ -67,12 +67,15 @@ __device__ __forceinline__ void chain_leave(bool beside) {
 // Under capture the launch is a plain one: a graph's own launches are cheap, its kernels overlap across branches already
 // (two batches in flight, 128 launches: 2844 us with chained edges, 2831 us without), and instantiating chained edges
 // took the host 0.3 s.
-static inline cudaLaunchAttribute chained_attribute(cudaStream_t st) {
+static inline bool starts_early(cudaStream_t st) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(st, &capture);
+    return capture == cudaStreamCaptureStatusNone;
+}
+static inline cudaLaunchAttribute chained_attribute(cudaStream_t st) {
     cudaLaunchAttribute a{};
     a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    a.val.programmaticStreamSerializationAllowed = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+    a.val.programmaticStreamSerializationAllowed = starts_early(st);
     return a;
 }
 template <class... P, class... A>

@@ -33,7 +33,6 @@ constexpr int NT = 64 + NEPI;
 constexpr size_t SMEM_MAX = 226 * 1024;
 
 struct Conv1dParams {
-    int beside;             // see chain_leave()
     const __nv_bfloat16* bias;
     __nv_bfloat16* out;
     int T, H, dk, ks, pad, D;
@@ -49,6 +48,7 @@ __device__ __forceinline__ void fail(volatile int* abort_flag, int code) {
 }
 __device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(NEPI) : "memory"); }
 
+template <bool BESIDE>                    // see chain_leave()
 __global__ void __launch_bounds__(NT, 1)
 conv1d_tc_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmW, const Conv1dParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -85,7 +85,7 @@ conv1d_tc_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant_
         tmem_alloc(tmem_slot, ncols);
         tmem_relinquish();
     }
-    chain_wait_unless(p.beside);
+    chain_wait_unless(BESIDE);
     // accumulator := bias by one K = 16 step: rows of `ones` hold 1.0 at the start of both 16-byte halves, a bias row its
     // value at the start of one, so the product picks it up whatever the swizzle
     for (int i = threadIdx.x; i < 1024; i += NT) reinterpret_cast<uint32_t*>(ones)[i] = (i & 3) == 0 ? 0x3f80u : 0u;
@@ -212,7 +212,7 @@ conv1d_tc_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant_
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, ncols);
     }
-    chain_leave(p.beside);
+    chain_leave(BESIDE);
 }
 
 }  // namespace
@@ -243,7 +243,6 @@ int try_launch_conv1d_tc(const void* y, const void* w, const void* bias, void* o
     Conv1dParams p{};
     p.bias = static_cast<const __nv_bfloat16*>(bias); p.out = static_cast<__nv_bfloat16*>(out);
     p.T = Tn; p.H = H; p.dk = dk; p.ks = ks; p.pad = (ks - 1) / 2; p.D = H * dk;
-    p.beside = beside;
     p.n_units = B * H; p.n_tiles = (Tn + BM - 1) / BM;
     p.acc_cols = dk < 32 ? 32 : dk;
     const size_t slab = ((size_t)Tn * dk * 2 + 15) / 16 * 16;
@@ -265,9 +264,14 @@ int try_launch_conv1d_tc(const void* y, const void* w, const void* bias, void* o
         if (!encode_tensor_map_bf16(&tmW, w, 2, dims, str, box, dk * 2)) return CONVNN_E_CUDA;
     }
     size_t smem = fixed + p.nbuf * set;
-    CONVNN_ENSURE_SMEM(conv1d_tc_kernel, smem);
-    const int sms = device_sms();
-    launch_chained(conv1d_tc_kernel, p.n_units < sms ? p.n_units : sms, NT, smem, st, tmY, tmW, p);
+    const int grid = p.n_units < device_sms() ? p.n_units : device_sms();
+    if (beside) {
+        CONVNN_ENSURE_SMEM(conv1d_tc_kernel<true>, smem);
+        launch_chained(conv1d_tc_kernel<true>, grid, NT, smem, st, tmY, tmW, p);
+    } else {
+        CONVNN_ENSURE_SMEM(conv1d_tc_kernel<false>, smem);
+        launch_chained(conv1d_tc_kernel<false>, grid, NT, smem, st, tmY, tmW, p);
+    }
     CONVNN_CHECK_LAUNCH("conv1d_tc");
     return CONVNN_OK;
 }

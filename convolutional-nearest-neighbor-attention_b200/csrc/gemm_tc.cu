@@ -79,8 +79,8 @@ struct GemmTcParams {
     int stages;            // depth of the shared-memory ring
     int wstat;             // 1: the whole W tile (BN x Kd) stays in shared memory; the ring holds A only
     int tiles_per_cta;     // wstat: each CTA owns a contiguous range of the n-major tile list
-    int beside;            // see chain_leave()
-    int w_at_rest;         // nothing that may still run on the stream writes W, its extra rows or the bias
+    int w_at_rest;         // nothing that may still run on the stream writes W, its extra rows or the bias, and this
+                           // kernel may start before its predecessor has ended
     // pre-norm fold: the moments of the A rows, [ln_planes][mom_ld] (sum, sum of squares) partial sums,
     // arrive through the tensor map tmM
     int ln_planes;
@@ -161,7 +161,8 @@ __device__ __forceinline__ float stage_chunk(const uint32_t (&sts)[4], const uin
 // fetches half the W bytes per flop.  The even CTA issues the MMAs; loads of both CTAs credit its
 // "full" barriers, completions are committed to the barriers of both CTAs, and the epilogue
 // warps of both release the accumulator on the leader's "tempty" barriers.  Streaming mode only.
-template <bool STAT, bool BIAS, bool GELU, bool RES, bool WIDE, bool PAIR, bool LNF = false, bool MOM = false>
+// BESIDE: see chain_leave().  (A flag of the launch instead cost every other GEMM 0.2 us.)
+template <bool STAT, bool BIAS, bool GELU, bool RES, bool WIDE, bool PAIR, bool LNF = false, bool MOM = false, bool BESIDE = false>
 __global__ void __launch_bounds__((WIDE ? NTHREADS_WIDE : NTHREADS) + (LNF ? 32 : 0), 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
                const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmM,
@@ -302,11 +303,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         };
         int cur_nt = -1;
         const int lead = first < last && p.KC <= 4 ? min(p.KC, (int)STAGES) : 0;     // chunks of the first tile requested at once
-        int w_ahead = 0;                                                // chunks of W alone that lane 0 requests early
+        int mt = 0, nt = 0;
+        if (first < last) tile_mn(first, mt, nt);
+        int m0 = mt * TM + (int)rank * BM, n0 = nt * p.BN + (int)rank * bn_cta;
         if (lead > 0) {
-            int mt, nt;
-            tile_mn(first, mt, nt);
-            const int m0 = mt * TM + (int)rank * BM, n0 = nt * p.BN + (int)rank * bn_cta;
             auto request_w = [&]() {                                     // W of the first tile, or its chunks in the ring
                 if (p.wstat) {
                     if (lane == 0) mbar_expect_tx_a(wfull_a, p.KC * b_bytes + (LNF ? (uint32_t)bn_cta * 32u : 0u));
@@ -321,62 +321,60 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             };
             if (lane < lead && (!PAIR || rank == 0)) mbar_expect_tx_a(full0 + 8 * lane, tx);
             if (p.w_at_rest) request_w();                                // before the predecessor has ended
-            chain_wait_unless(p.beside);
+            chain_wait_unless(BESIDE);
             if (!p.w_at_rest) request_w();
             if (lane < lead) load_a((uint32_t)lane, lane, m0);
             __syncwarp();
         }
-        if (lane == 0) {
-            uint32_t s = lead == (int)STAGES ? 0u : (uint32_t)lead, ph = lead == (int)STAGES ? 1u : 0u;   // ring slot and its phase
-            uint32_t last_s = lead > 0 ? (uint32_t)lead - 1u : 0u, last_ph = 0;
-            int skip = lead;                                             // chunks of the first tile that are on the way
+        if (lane == 0 && first < last) {
             bool ok = true;
             const bool tr = !PAIR && trace_enabled() && blockIdx.x == 0;
             int tn = 0;
             trace(tr, 0, tn);
-            auto load_w_tile = [&](int nt) {
+            auto load_w_tile = [&](int n) {
                 mbar_expect_tx_a(wfull_a, p.KC * b_bytes + (LNF ? (uint32_t)bn_cta * 32u : 0u));
-                for (int kc = 0; kc < p.KC; ++kc) tma_load_2d_a(sB0 + kc * b_bytes, &tmW, wfull_a, kc * p.KCH, nt * p.BN);
-                if (LNF) tma_load_2d_a(smem_u32(xb), &tmX, wfull_a, 0, nt * p.BN);
-                cur_nt = nt;
+                for (int kc = 0; kc < p.KC; ++kc) tma_load_2d_a(sB0 + kc * b_bytes, &tmW, wfull_a, kc * p.KCH, n * p.BN);
+                if (LNF) tma_load_2d_a(smem_u32(xb), &tmX, wfull_a, 0, n * p.BN);
+                cur_nt = n;
             };
-            if (lead == 0 && first < last) {
+            int sent = lead;                                             // chunks of the first tile that are on the way
+            if (lead == 0) {
                 if (p.w_at_rest) {                                       // W of the first tile, or as many of its chunks as the ring holds
-                    int mt, nt;
-                    tile_mn(first, mt, nt);
                     if (p.wstat) load_w_tile(nt);
                     else
-                        for (w_ahead = 0; w_ahead < min(p.KC, (int)STAGES); ++w_ahead) {
-                            if (!PAIR || rank == 0) mbar_expect_tx_a(full0 + 8 * w_ahead, tx);
-                            load_w_chunk((uint32_t)w_ahead, w_ahead, nt * p.BN + (int)rank * bn_cta);
+                        for (; sent < min(p.KC, (int)STAGES); ++sent) {
+                            if (!PAIR || rank == 0) mbar_expect_tx_a(full0 + 8 * sent, tx);
+                            load_w_chunk((uint32_t)sent, sent, n0);
                         }
                 }
-                chain_wait_unless(p.beside);
+                chain_wait_unless(BESIDE);
+                if (p.wstat && cur_nt < 0) load_w_tile(nt);
+                for (int kc = 0; kc < sent; ++kc) load_a((uint32_t)kc, kc, m0);
             }
-            bool any = lead > 0;
-            for (int t = first; t < last && ok; t += step) {
-                int mt, nt;
+            uint32_t s = sent == (int)STAGES ? 0u : (uint32_t)sent, ph = sent == (int)STAGES ? 1u : 0u;   // ring slot and its phase
+            uint32_t last_s = sent > 0 ? (uint32_t)sent - 1u : 0u, last_ph = 0;
+            for (int t = first;;) {
+                for (int kc = sent; kc < p.KC; ++kc) {
+                    if (!mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag)) { give_up(11); ok = false; break; }
+                    if (!PAIR || rank == 0) mbar_expect_tx_a(full0 + 8 * s, tx);
+                    load_a(s, kc, m0);
+                    load_w_chunk(s, kc, n0);
+                    last_s = s; last_ph = ph;
+                    if (++s == STAGES) { s = 0; ph ^= 1u; }
+                }
+                sent = 0;
+                t += step;
+                if (t >= last || !ok) break;
                 tile_mn(t, mt, nt);
                 if (p.wstat && nt != cur_nt) {
                     // every MMA that reads the old W tile has completed once the most recently
                     // filled ring stage has been released
-                    if (any && !mbar_wait_a(empty0 + 8 * last_s, last_ph, abort_flag)) { give_up(15); ok = false; break; }
+                    if (!mbar_wait_a(empty0 + 8 * last_s, last_ph, abort_flag)) { give_up(15); break; }
                     load_w_tile(nt);
                 }
                 trace(tr, 0, tn);
-                const int m0 = mt * TM + (int)rank * BM, n0 = nt * p.BN + (int)rank * bn_cta;
-                const int kc0 = skip;
-                skip = 0;
-                for (int kc = kc0; kc < p.KC; ++kc) {
-                    if (!mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag)) { give_up(11); ok = false; break; }
-                    const bool whole = w_ahead == 0;            // (otherwise its W chunk is on the way)
-                    if (whole && (!PAIR || rank == 0)) mbar_expect_tx_a(full0 + 8 * s, tx);
-                    load_a(s, kc, m0);
-                    if (whole) load_w_chunk(s, kc, n0);
-                    else --w_ahead;
-                    last_s = s; last_ph = ph; any = true;
-                    if (++s == STAGES) { s = 0; ph ^= 1u; }
-                }
+                m0 = mt * TM + (int)rank * BM;
+                n0 = nt * p.BN + (int)rank * bn_cta;
             }
         }
     } else if (warp == 1) {
@@ -396,7 +394,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             int tn = 0;
             const uint32_t peer_empty0 = PAIR ? map_to_cta(empty0, 1) : 0u;
             const uint32_t peer_tfull0 = PAIR ? map_to_cta(tfull0, 1) : 0u;
-            chain_wait_unless(p.beside);                     // (the budgets of its waits are for this kernel's work)
+            chain_wait_unless(BESIDE);                     // (the budgets of its waits are for this kernel's work)
             for (int t = first; t < last && ok; t += step, ++tile) {
                 const uint32_t buf = tile & 1u, u = tile >> 1;
                 if (!mbar_wait_a(tempty0 + 8 * buf, (u & 1u) ^ 1u, abort_flag)) { give_up(12); ok = false; break; }
@@ -465,7 +463,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             mbar_expect_tx(&mfull[slot], slot_bytes);
             tma_load_2d(mring + slot * slot_bytes, &tmM, &mfull[slot], mt * BM * 2, 0);
         };
-        chain_wait_unless(p.beside);
+        chain_wait_unless(BESIDE);
         if (lane == 0)
             for (int k = 0; k < MOM_AHEAD; ++k)
                 if (first + k * step < last) fetch((uint32_t)k, first + k * step);
@@ -540,7 +538,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const bool tr = !PAIR && trace_enabled() && blockIdx.x == 0 && lq == 0 && lane == 0 && chalf == 0;
         const uint32_t lead_tempty0 = PAIR ? map_to_cta(smem_u32(tempty), 0) : 0u;
         int tn = 0;
-        chain_wait_unless(p.beside);
+        chain_wait_unless(BESIDE);
         chain_next();
         for (int t = first + half * step; t < last && ok; t += 2 * step, tile += 2) {
             int mt, nt;
@@ -760,7 +758,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (PAIR) tmem_dealloc_pair(tmem_base, ncols);
         else tmem_dealloc(tmem_base, ncols);
     }
-    chain_leave(p.beside);
+    chain_leave(BESIDE);
 }
 
 int pow2_at_least(int v, int lo) {
@@ -854,7 +852,7 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
     }
     p.ldc = ldc; p.bias = static_cast<const __nv_bfloat16*>(o.bias); p.gelu = o.gelu;
     p.mma_bias = nullptr;
-    p.w_at_rest = o.w_at_rest || o.beside; p.beside = o.beside;
+    p.w_at_rest = o.w_at_rest && starts_early(st);
     p.residual = static_cast<const __nv_bfloat16*>(o.residual); p.ldr = o.ldr;
     p.stat_pieces = 1; p.stat_plane = 0;
     p.stat_mode = o.stat_mode; p.dk = o.dk > 0 ? o.dk : 32; p.heads = o.heads; p.rows_per_batch = o.rows_per_batch > 0 ? o.rows_per_batch : 1;
@@ -1011,9 +1009,9 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
     if (has_stat && (p.bias || p.residual || p.gelu))
         return set_error(CONVNN_E_UNSUPPORTED, "gemm_tc: statistics cannot be combined with bias / GELU / residual");
     if (p.gelu && p.residual) return set_error(CONVNN_E_UNSUPPORTED, "gemm_tc: GELU with a residual is not built");
-#define CONVNN_GEMM_LAUNCH1(S, B, G, R, W)                                                                  \
+#define CONVNN_GEMM_LAUNCH1(S, B, G, R, W, ...)                                                             \
     do {                                                                                                    \
-        auto kern = gemm_tc_kernel<S, B, G, R, W, false>;                                                   \
+        auto kern = gemm_tc_kernel<S, B, G, R, W, false, ##__VA_ARGS__>;                                    \
         CONVNN_ENSURE_SMEM(kern, smem);                                                            \
         launch_chained(kern, grid, W ? NTHREADS_WIDE : NTHREADS, smem, st, tmA, tmW, tmX, tmM, p);                           \
     } while (0)
@@ -1061,7 +1059,9 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
         else if (p.residual) CONVNN_GEMM_LAUNCH_PAIR(false, true, true);
         else CONVNN_GEMM_LAUNCH_PAIR(false, false, false);
     } else
-    if (has_stat) CONVNN_GEMM_LAUNCH1(true, false, false, false, false);
+    // (with another epilogue, or as a pair, it waits at its start, which is as right)
+    if (o.beside && !has_stat && !wide) CONVNN_GEMM_LAUNCH1(false, false, false, false, false, false, false, true);
+    else if (has_stat) CONVNN_GEMM_LAUNCH1(true, false, false, false, false);
     else if (p.gelu) { if (p.bias) CONVNN_GEMM_LAUNCH(false, true, true, false); else CONVNN_GEMM_LAUNCH(false, false, true, false); }
     else if (p.bias && p.residual) CONVNN_GEMM_LAUNCH(false, true, false, true);
     else if (p.bias) CONVNN_GEMM_LAUNCH(false, true, false, false);

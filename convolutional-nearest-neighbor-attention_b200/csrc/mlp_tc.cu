@@ -751,7 +751,7 @@ int launch_mlp_tc(const void* x, long long ldx, const float* moments, int planes
     p.planes = planes; p.eps = eps; p.inv_d = 1.0f / (float)D;
     p.bias2 = static_cast<const __nv_bfloat16*>(b2);
     p.resid = static_cast<const __nv_bfloat16*>(resid); p.ldr = ldr;
-    p.weights_at_rest = weights_at_rest;
+    p.weights_at_rest = weights_at_rest && starts_early(st);
     p.moments_out = reinterpret_cast<float2*>(moments_out);
     CUtensorMap tmX, tmO, tmW1, tmWX, tmW2, tmWO;
     {
