@@ -53,27 +53,35 @@ __device__ __forceinline__ void store_group(float* o, const f32x2 (&a)[N]) {
 
 // (neighbour row in units of VEC channels, weight) pairs of tokens m0 ... m0 + nt - 1 into shared memory, the TPT tokens of
 // a set side by side per tap.  The exponentials are taken by all threads; a token's maximum and its sum in tap order by
-// one, so the weights are those of a serial loop.  The places behind the last token hold its rows again.
+// one, so the weights are those of a serial loop.  Threads go along shared memory (along a token's taps, with four tokens per
+// set, their stores met in the same banks: 830000 tokens of 16 float32 channels, 25 taps 250 us).  The places behind the last
+// token hold its pairs again.
 template <int VEC, int TPT>
 __device__ __forceinline__ void token_pairs(const DwParams& p, int m0, int nt, int2* pairs, float* red) {
-    const int n = nt * p.K, n_up = (nt + TPT - 1) / TPT * TPT * p.K;
+    const int n_up = (nt + TPT - 1) / TPT * TPT * p.K;
     const long long nbase = (long long)m0 * p.K;
-    auto at = [&](int t, int j) { return TPT == 1 ? t * p.K + j : ((t / TPT) * p.K + j) * TPT + t % TPT; };
+    auto at = [&](int t, int j) { return ((t / TPT) * p.K + j) * TPT + t % TPT; };
+    // token and tap of place e
+    auto whose = [&](int e, int& t, int& j) {
+        const int per_set = p.K * TPT, set = e / per_set, in = e - set * per_set;
+        t = min(set * TPT + in % TPT, nt - 1);
+        j = in / TPT;
+    };
     for (int e = threadIdx.x; e < n_up; e += THREADS) {
-        const int slot = e / p.K, t = TPT == 1 ? slot : min(slot, nt - 1);
-        const long long ne = nbase + (e - (slot - t) * p.K);
+        int t, j;
+        whose(e, t, j);
+        const long long ne = nbase + t * p.K + j;
         const int bh = (m0 + t) / p.T, b = bh / p.H, h = bh - b * p.H;
         const float x = p.val[ne];
-        pairs[TPT == 1 ? e : at(slot, e - slot * p.K)] =
-            make_int2(((b * p.T + p.idx[ne]) * p.H + h) * (p.Cp / VEC), __float_as_int(p.maximum ? x : -x));
+        pairs[e] = make_int2(((b * p.T + p.idx[ne]) * p.H + h) * (p.Cp / VEC), __float_as_int(p.maximum ? x : -x));
     }
     __syncthreads();
     // f(weight, token) over all of them
     auto each = [&](auto f) {
-        for (int e = threadIdx.x; e < n; e += THREADS) {
-            const int t = e / p.K;
-            int& y = pairs[TPT == 1 ? e : at(t, e - t * p.K)].y;
-            y = __float_as_int(f(__int_as_float(y), t));
+        for (int e = threadIdx.x; e < n_up; e += THREADS) {
+            int t, j;
+            whose(e, t, j);
+            pairs[e].y = __float_as_int(f(__int_as_float(pairs[e].y), t));
         }
     };
     if (p.softmax) {
@@ -99,16 +107,10 @@ __device__ __forceinline__ void token_pairs(const DwParams& p, int m0, int nt, i
 }
 
 // Rows in flight: TPT tokens side by side per tap, UNROLL taps; more of either leaves fewer warps (MINB CTAs per SM).
-template <typename T, typename TO, int TPT> struct DwShape {
-    static constexpr bool wider = sizeof(TO) > sizeof(T);
-    static constexpr int UNROLL = TPT == 4 ? 1 : (wider ? 2 : 4), MINB = TPT == 4 ? 3 : (wider ? 5 : 4);
-};
-
-template <typename T, typename TO, int VEC, int TPT>
-__global__ void __launch_bounds__(THREADS, DwShape<T, TO, TPT>::MINB) gather_conv_dw_kernel(const DwParams p, const int TT) {
+template <typename T, typename TO, int VEC, int TPT, int UNROLL, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) gather_conv_dw_kernel(const DwParams p, const int TT) {
     chain_begin_for<TO>();
     typedef Channels<T, VEC> Ch;
-    constexpr int UNROLL = DwShape<T, TO, TPT>::UNROLL;
     extern __shared__ __align__(16) unsigned char dw_smem[];
     int2* pairs = reinterpret_cast<int2*>(dw_smem);           // [TT / TPT][K][TPT]
     float* red = reinterpret_cast<float*>(pairs + TT * p.K);  // [TT]
@@ -228,8 +230,17 @@ int launch(const DwParams& p, cudaStream_t st) {
     if (TT < tpt) TT = tpt;
     const size_t smem = (size_t)TT * p.K * 8 + TT * 4;
     const int grid = (p.M + TT - 1) / TT;
-    if (tpt == 4) launch_chained(gather_conv_dw_kernel<T, TO, VEC, 4>, grid, THREADS, smem, st, p, TT);
-    else launch_chained(gather_conv_dw_kernel<T, TO, VEC, 1>, grid, THREADS, smem, st, p, TT);
+    // The form by the rounds of CTAs per SM it needs: with four tokens per thread three CTAs of one tap in flight, or two of two
+    // taps where both need two rounds (3 x 1611 tokens x 10, 96 channels, 25 taps 36.1, 32.7 us); with one token four CTAs of four
+    // taps while that is one round, then five or six of two taps, which fit in one (71 x 34 x 2 heads of 128, float32, 3 taps
+    // 5.4, 4.1; 9 x 701 x 2 heads of 64 6.6, 5.3).
+    const int sms = device_sms(), per_sm = (grid + sms - 1) / sms;
+    auto go = [&](auto kern) { launch_chained(kern, grid, THREADS, smem, st, p, TT); };
+    if (tpt == 4 && per_sm != 4) go(gather_conv_dw_kernel<T, TO, VEC, 4, 1, 3>);
+    else if (tpt == 4) go(gather_conv_dw_kernel<T, TO, VEC, 4, 2, 2>);
+    else if (per_sm <= 4) go(gather_conv_dw_kernel<T, TO, VEC, 1, 4, 4>);
+    else if (per_sm == 6) go(gather_conv_dw_kernel<T, TO, VEC, 1, 2, 6>);
+    else go(gather_conv_dw_kernel<T, TO, VEC, 1, 2, 5>);
     CONVNN_CHECK_LAUNCH("gather_conv_dw");
     return CONVNN_OK;
 }

@@ -139,3 +139,20 @@ def test_standard_conv_in_the_flat_reinterpretation(B, T, H, dk, K, fused, metri
 def test_sets_of_four_tokens(B, T, H, dk, K, dtype):
     test_depthwise_against_float64(B, T, H, dk, K, dtype, "cosine", True)
     test_depthwise_against_float64(B, T, H, dk, K, dtype, "euclidean", False)
+
+
+# Every form by the rounds of CTAs per SM (tokens per thread, taps in flight, CTAs per SM that fit), as the dispatch picks them.
+@on_148_sms
+@pytest.mark.parametrize("B,T,H,dk,K,dtype,form", [
+    (3, 33, 1, 64, 9, torch.float32, "1, 4, 4"), (71, 34, 2, 128, 3, torch.float32, "1, 2, 5"), (9, 701, 2, 64, 5, torch.float32, "1, 2, 6"),
+    (12, 158, 1, 768, 5, torch.float32, "4, 2, 2"), (7, 3098, 2, 96, 9, torch.float32, "4, 1, 3"), (2, 473, 12, 128, 3, torch.bfloat16, "1, 2, 5"),
+    (5, 660, 1, 256, 9, torch.bfloat16, "1, 4, 4"), (10, 1611, 3, 96, 25, torch.bfloat16, "4, 2, 2"), (76, 518, 6, 16, 3, torch.bfloat16, "4, 2, 2"),
+    (40, 1024, 4, 16, 25, torch.bfloat16, "4, 1, 3")])
+def test_forms_of_the_depthwise_gather(B, T, H, dk, K, dtype, form):
+    spec = ops.LayerSpec(H * dk, H, K, "all", "cosine", "depthwise", True, False, T)
+    v, w = torch.zeros(B, T, H, dk, device=DEV, dtype=dtype), torch.zeros(K, dk, device=DEV, dtype=dtype)
+    idx, val = torch.zeros(B, H, T, K, device=DEV, dtype=torch.int32), torch.zeros(B, H, T, K, device=DEV)
+    name, = launches(lambda: ops.gather_conv(spec, v, idx, val, w))
+    assert "gather_conv_dw_kernel" in name and "Li{}ELi{}ELi{}EE".format(*form.split(", ")) in name
+    test_depthwise_against_float64(B, T, H, dk, K, dtype, "cosine", True)
+    test_depthwise_against_float64(B, T, H, dk, K, dtype, "euclidean", False)
