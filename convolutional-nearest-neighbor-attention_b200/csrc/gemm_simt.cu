@@ -652,10 +652,12 @@ int launch_plain_f32(const GemmParams& p, cudaStream_t st) {
 // Other plain rows: float32 ones of any alignment, bfloat16, float32 against bfloat16 weights.  Which tiles, and which times, goes by
 // what the operands cost: float32 values need no conversion, so that the transposed tiles wait for little and the largest of
 // them reuses most; bfloat16 values that come one by one are what the transposed tiles wait for.  Narrow outputs of few
-// values of k (the separable conv with the coordinate channel on heads of 8 to 32) end before that counts.  Fits to 209, 98
-// and 98 shapes (30 to 100000 rows, 8 to 2304 columns, 9 to 2048 values of k; rms 9 to 21 %), the choice within 1.2, 1.5 and
-// 0.8 % of the best of seven tiles on average; 0.95, 0.72 and 0.62 of the time of the four transposed tiles alone, at worst 1.08 (4 us).
-// float32, us, staged tiles only -> now: 2813 x 768 x 769 138 -> 102, 56288 x 256 x 257 244 -> 189, 39846 x 8 x 9 9.9 -> 6.7.
+// values of k (the separable conv with the coordinate channel on heads of 8 to 32) end before that counts.  Fits to 209, 98, 98
+// and 90 shapes (30 to 1000000 rows, 8 to 2304 columns, 9 to 2048 values of k; rms 3 to 21 %), the choice within 1.2, 1.5, 0.8
+// and 0.9 % of the best of seven tiles on average; 0.95, 0.72, 0.55 and 0.71 of the time of the four transposed tiles alone, at worst
+// 1.09 (kernels of 4 us).
+// float32, us, staged tiles only -> now: 2813 x 768 x 769 138 -> 102, 56288 x 256 x 257 244 -> 189, 39846 x 8 x 9 9.9 -> 6.7; mixed 650981 x
+// 64 x 65 277 -> 233, 109615 x 16 x 17 18.7 -> 12.3.
 // bfloat16, transposed tiles only -> now: 4 x 197 x 768 x 768 130 -> 55; 2080 x 384 x 388 57.9 -> 27.8.
 template <typename TA, typename T, int MODE>
 int launch_plain_staged(const GemmParams& p, cudaStream_t st) {
@@ -687,7 +689,14 @@ int launch_plain_staged(const GemmParams& p, cudaStream_t st) {
             {32, 64, 32, 4, 2.1, 1.7, {31.9, 48.3, 65.4, 92.7}},
             {40, 32, 32, 6, 2.3, 2.9, {36.8, 39.8, 54.5, 58.5, 83.1, 87.1}},
         };
-        switch (p.a_vec && p.w_vec ? cheapest_tile(by_four, p) : cheapest_tile(by_value, p, 1)) {
+        static const Tile mixed[5] = {                               // float32 rows against bfloat16 weights
+            {128, 64, 16, 3, 2.0, 0.0, {157.9, 182.8, 200.0}},
+            {32, 32, 32, 7, 0.9, 0.0, {90.3, 100.6, 98.8, 99.2, 114.6, 113.0, 102.3}},
+            {64, 64, 32, 3, 2.1, 2.6, {42.7, 67.6, 95.9}},
+            {32, 64, 32, 4, 1.9, 1.0, {31.5, 47.1, 66.7, 82.2}},
+            {40, 32, 32, 6, 1.8, 2.2, {32.9, 37.0, 45.6, 55.8, 70.9, 74.7}},
+        };
+        switch (sizeof(TA) == 4 ? cheapest_tile(mixed, p) : p.a_vec && p.w_vec ? cheapest_tile(by_four, p) : cheapest_tile(by_value, p, 1)) {
             case 0: return launch_tile<TA, T, MODE, 128, 64, 16, 8, 8, 3>(p, st);
             case 1: return launch_tile<TA, T, MODE, 32, 32, 32, 4, 4, 4>(p, st);
             case 2: return launch_stage_tile<TA, T, MODE, 64, 64, 8, 4, 3>(p, st);
