@@ -628,14 +628,29 @@ int launch_short(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const C
 
 }  // namespace
 
-// What the warp-per-row kernel leaves to it.  Lists of up to twelve, except for up to 32 candidates of sequences that fill more
-// than one of its units, where the streaming kernel's 256-row units are fewer and the bound saves little (us, streaming, this
-// kernel: 512 x 197 x 16 x 192, K = 4 10.8, 14.4; 256 x 197 x 32 x 768, K = 3 19.6, 21.9; 300 images of 17 x 17 x 64 with three
-// heads, K = 5 15.8, 10.8).  Lists of 13 to 16: their streaming variant runs one CTA per SM (256 x 577 x 150 x 384, K = 16 129, 110;
-// 256 x 197 x 197 x 192 47, 49).  Anything of up to one unit per SM (48 x 197 x 197 x 192, K = 25 33.8, 23.0).
+// What the warp-per-row kernel leaves to it.  Anything of up to one unit per SM (48 x 197 x 197 x 192, K = 25 33.8, 23.0); lists of 13 to
+// 16, whose streaming variant runs one CTA per SM (256 x 577 x 150 x 384, K = 16 129, 110; 256 x 197 x 197 x 192 47, 49); lists of up to
+// twelve except where the streaming kernel's 256-row units are fewer and the bound saves little (us, streaming, this kernel):
+//   * few candidates: of sequences that fill more than one unit here (512 x 197 x 16 x 192, K = 4 10.8, 14.4; 256 x 197 x 32 x 768, K = 3
+//     19.6, 21.9), and of others where heads are wide, lists long or the second round of units thin (1000 x 17 x 17 x 512, K = 2 19.5, 23.6;
+//     200 x 100 x 20 x 384, K = 5 8.6, 9.6; 163 x 65 x 65 x 128, K = 12 13.4, 14.6; but 1000 x 17 x 17 x 64 0.65 of the time, 340 x 25 x 25 x 192 0.85, and
+//     heads above 512 channels, which leave the streaming kernel one CTA per SM, 0.85)
+//   * heads above 640 channels with so many candidates that the ring has two stages, while the streaming kernel's units fill most of
+//     one round (141 x 256 x 256 x 768, K = 5 26.2, 32.6; 100 images 25.2, 22.1; 200 50.6, 42.6)
 bool sim_topk_short_wanted(const Dims& dm) {
-    const long long units = (long long)dm.B * dm.H * ((dm.T + BM - 1) / BM);
-    return dm.S <= 256 && (units <= device_sms() || (dm.nsel <= 16 && (dm.nsel > 12 || dm.S > 32 || dm.T <= BM)));
+    if (dm.S > 256) return false;
+    const long long sms = device_sms(), bh = (long long)dm.B * dm.H, units = bh * ((dm.T + BM - 1) / BM);
+    if (units <= sms) return true;
+    if (dm.nsel > 12) return dm.nsel <= 16;
+    if (dm.T > BM && dm.S <= 32) return false;
+    if (dm.T <= BM && dm.S <= 40) {
+        if (dm.Cp > 512) return true;
+        if (dm.nsel > 9) return false;
+        return dm.Cp <= 128 || (units > 2 * sms && dm.Cp <= (dm.nsel > 4 ? 384 : dm.S > 32 ? 256 : 192));
+    }
+    if (dm.T <= BM && dm.S <= 80 && dm.nsel > 9 && dm.Cp <= 128 && 2 * units <= 3 * sms) return false;
+    const long long streaming = bh * ((dm.T + 2 * BM - 1) / (2 * BM));
+    return !(dm.Cp > 640 && dm.S > 224 && streaming <= sms && 5 * streaming > 4 * sms);
 }
 
 int launch_sim_topk_short(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,

@@ -169,6 +169,23 @@ def test_warp_per_row_routes(B, T, S, H, dk, K, dtype, rows):
     assert len(names) == 1 and any(n in next(iter(names)) for n in ("sim_topk_rows_kernel", "sim_topk_simt_rows_kernel")) == rows
 
 
+@on_148_sms
+@pytest.mark.parametrize("B,T,S,H,dk,K,two_pass", [
+    # few candidates: narrow heads, several rounds of units, wide heads, long lists
+    (1000, 17, 17, 1, 64, 5, True), (1000, 17, 17, 1, 512, 2, False), (340, 25, 25, 1, 192, 9, True), (200, 100, 20, 1, 384, 5, False),
+    (340, 25, 25, 1, 768, 5, True), (281, 48, 33, 1, 128, 5, True), (281, 48, 33, 3, 64, 12, False), (512, 197, 16, 1, 192, 4, False),
+    (163, 65, 65, 1, 128, 12, False), (281, 65, 65, 1, 128, 12, True),
+    # the widest heads, most candidates, streaming units that fill most of a round
+    (141, 256, 256, 1, 768, 5, False), (100, 256, 256, 1, 768, 5, True), (200, 256, 256, 1, 768, 5, True), (141, 224, 224, 1, 768, 5, True)])
+def test_two_pass_routes(B, T, S, H, dk, K, two_pass):
+    g = torch.Generator(device=DEV).manual_seed(1)
+    spec = ops.LayerSpec(H * dk, H, K, "spatial" if S != T else "all", "matmul", "depthwise", True, False, T)
+    q, k = (torch.randn(B, r, H, dk, device=DEV, generator=g).bfloat16() for r in (S, T))
+    cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if S != T else None
+    name, = launches(lambda: ops.sim_topk(spec, q, k, None, None, cand))
+    assert ("sim_topk_short_kernel" in name) == two_pass and ("sim_topk_tc_kernel" in name) != two_pass
+
+
 # Several 128-row units per SM.  (80 x 197 x 64 with one accumulator in four and one in two; 33 to 48 candidates leave the upper
 # half of a row a chunk or nothing; 208 and 256 end on a whole chunk; "few" values tie, so that most rows overflow their entries;
 # "stripes" puts the best sixteen columns into one group of maxima.)
