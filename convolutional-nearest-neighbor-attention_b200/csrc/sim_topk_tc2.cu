@@ -193,7 +193,9 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         // value after every 32 columns, with the number of its unit, and reads the other's, which may be older (a rank's
         // value only grows within a unit) or of another unit (then it is not used).  Equal keys stay: the order among them
         // goes by column, and the other half may hold the higher ones.  768 channels: 16384 x 4096, K = 25 1184 -> 1119 us; 4096 x
-        // 4096, K = 9 198.4 -> 196.5 (the products bound it); 384 channels, K = 16 204 -> 197; 3000 x 1500 x 128, K = 12 104 -> 98.
+        // 4096, K = 9 198.4 -> 196.5 (the products bound it); 384 channels, K = 16 204 -> 197; 3000 x 1500 x 128, K = 12 104 -> 98.  Lists
+        // of up to four make too few insertions for it (2269 x 2269 x 256, K = 4 44.9, 46.8 with it).
+        constexpr bool SHARE = NSEL > 4;
         constexpr int R0 = (NSEL + 1) / 2, R1 = NSEL / 2;
         volatile unsigned long long* own_rank = ranks + chalf * kSelGroup + r;
         volatile unsigned long long* their_rank = ranks + (chalf ^ 1) * kSelGroup + r;
@@ -244,15 +246,19 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
                         if (cbase + c4 * 32 < p.S) {             // otherwise the rest of the tile is padding
                             uint32_t acc[32];
                             tmem_ld_x32(taddr + c4 * 32, acc);
-                            const unsigned long long other = *their_rank;
-                            const float floor = (uint32_t)(other >> 32) == it + 1
-                                                    ? just_below(fminf(my_rank, __uint_as_float((uint32_t)other)))
-                                                    : -CUDART_INF_F;
+                            float floor = -CUDART_INF_F;
+                            if constexpr (SHARE) {
+                                const unsigned long long other = *their_rank;
+                                if ((uint32_t)(other >> 32) == it + 1)
+                                    floor = just_below(fminf(my_rank, __uint_as_float((uint32_t)other)));
+                            }
                             tmem_ld_wait();
-                            consume<NSEL, 32, true>(top, acc, cbase + c4 * 32, 0, sq + c4 * 32, cv[c4], p, row, row_ok,
+                            consume<NSEL, 32, SHARE>(top, acc, cbase + c4 * 32, 0, sq + c4 * 32, cv[c4], p, row, row_ok,
                                                     sentinel, ks, floor);
-                            my_rank = chalf == 0 ? top.v[R0 - 1] : top.v[R1 - 1];
-                            *own_rank = ((unsigned long long)(it + 1) << 32) | __float_as_uint(my_rank);
+                            if constexpr (SHARE) {
+                                my_rank = chalf == 0 ? top.v[R0 - 1] : top.v[R1 - 1];
+                                *own_rank = ((unsigned long long)(it + 1) << 32) | __float_as_uint(my_rank);
+                            }
                         }
                     }
                 }
