@@ -41,3 +41,39 @@ def test_ties_go_to_the_lower_column(T, S, dk, K, order):
     col = key.sort(dim=1, descending=True, stable=True).indices[:, :n]
     want = col if cand is None else cand.long()[col]
     assert torch.equal(idx[0, 0, :, first:].long(), want)
+
+
+# Columns that are no number, columns whose keys are +inf for some rows and -inf or no number for others, and rows with fewer
+# usable columns than the list is long: NaN and -inf are never picked, an empty slot holds the first token.
+@pytest.mark.parametrize("T,S,dk,K", [(1100, 1100, 128, 9), (1030, 1153, 192, 16), (2048, 2048, 64, 4), (8200, 4225, 128, 26)])
+@pytest.mark.parametrize("columns", ["nan", "inf", "few left"])
+def test_unusable_keys(T, S, dk, K, columns):
+    T = max(T, S)
+    g = torch.Generator(device=DEV).manual_seed(T + S + K)
+    spec = ops.LayerSpec(dk, 1, K, "all" if S == T else "spatial", "matmul", "depthwise", True, False, T)
+    q = torch.randint(-3, 4, (1, S, 1, dk), device=DEV, generator=g).float()
+    k = torch.randint(-3, 4, (1, T, 1, dk), device=DEV, generator=g).float()
+    if columns == "nan":
+        q[:, ::3] = float("nan")
+    elif columns == "inf":
+        q[:, 7::50, :, 0] = float("inf")                       # times k's channel 0: both infinities, or no number at 0
+        q[:, 100::200, :, 1] = float("-inf")
+    else:
+        q[:, 3:S - 2] = float("nan")
+    cand = None if S == T else torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32)
+    qb, kb = q.bfloat16(), k.bfloat16()
+    call = lambda: ops.sim_topk(spec, qb, kb, None, None, cand)
+    assert any("sim_topk_tc2_kernel" in name for name in launches(call))
+    idx, val = call()
+    dot = torch.zeros(T, S, device=DEV)
+    for c in range(dk):                                        # (term by term: no infinity meets one that a sum made)
+        dot += k[0, :, 0, c:c + 1] * q[0, :, 0, c]
+    n, first = K, 0
+    if cand is not None:
+        own = cand.view(1, S).long() == torch.arange(T, device=DEV).view(T, 1)
+        dot = dot.masked_fill(own, -0.1 * dk ** 0.5)
+        n, first = K - 1, 1
+    dot = torch.where(dot.isnan(), torch.full_like(dot, -float("inf")), dot)
+    ranked = dot.sort(dim=1, descending=True, stable=True)
+    col = torch.where(ranked.values[:, :n] > -float("inf"), ranked.indices[:, :n], 0)
+    assert torch.equal(idx[0, 0, :, first:].long(), col if cand is None else cand.long()[col])

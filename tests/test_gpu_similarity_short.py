@@ -220,3 +220,52 @@ def test_exact_lists_of_many_units(B, T, S, H, dk, K, values):
     want_val = want_key / torch.tensor(math.sqrt(dk), dtype=torch.float32)
     # one division: equal up to its rounding
     assert bool(((val[..., K - n:] - want_val).abs() <= 2.0 ** -22 * want_val.abs())[real].all())
+
+
+# The same kernel for the other metrics, whose rows end on a NaN statistic instead of -inf: whole numbers with statistics that are
+# powers of two (cosine) or exact squared norms (euclidean), so that every key is exact.
+@on_148_sms
+@pytest.mark.parametrize("B,T,S,H,dk", [(160, 17, 17, 1, 64), (80, 197, 33, 1, 64), (80, 197, 64, 1, 384), (160, 128, 128, 1, 192),
+                                        (60, 129, 48, 3, 16), (80, 197, 197, 3, 32), (60, 300, 208, 1, 512), (320, 256, 256, 1, 64)])
+@pytest.mark.parametrize("K", [3, 9, 12])
+@pytest.mark.parametrize("values", ["few", "many", "nan", "stripes"])
+@pytest.mark.parametrize("metric", ["cosine", "euclidean"])
+def test_exact_lists_of_the_other_metrics(B, T, S, H, dk, K, values, metric):
+    sampled = S != T
+    n = K - 1 if sampled else K
+    g = torch.Generator(device=DEV).manual_seed(T * 1000 + S + K)
+    top = 1 if values == "few" else 11               # products and sums stay far below 2^24
+    q, k = (torch.randint(-top, top + 1, (B, r, H, dk), device=DEV, generator=g).float() for r in (S, T))
+    if values == "stripes":
+        q[:, ::16] = q[:, ::16].abs() + 12
+        k = k.abs()
+    if metric == "cosine":
+        qs, ks = (2.0 ** torch.randint(-2, 3, (B, H, r), device=DEV, generator=g).float() for r in (S, T))
+    else:
+        qs, ks = (t.pow(2).sum(-1).permute(0, 2, 1).contiguous() for t in (q, k))
+    if values == "nan":
+        q[:, ::3] = math.nan
+        q[1, 2:] = math.nan
+        qs[:, :, 1::5] = math.nan
+    spec = ops.LayerSpec(H * dk, H, K, "spatial" if sampled else "all", metric, "depthwise", True, False, T)
+    cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if sampled else None
+    call = lambda: ops.sim_topk(spec, q.bfloat16(), k.bfloat16(), qs, ks, cand)
+    if S > 40 or n <= 9:
+        assert any("sim_topk_short_kernel" in name for name in launches(call))
+    idx, val = call()
+    dot = torch.einsum("bthc,bshc->bhts", k.double(), q.double()).float()
+    col, row = qs.unsqueeze(2), ks.unsqueeze(3)
+    key = dot * col if metric == "cosine" else 2 * dot - col
+    if sampled:
+        own = cand.view(1, 1, 1, S).long() == torch.arange(T, device=DEV).view(1, 1, T, 1)
+        key = torch.where(own, torch.tensor(-0.1, device=DEV) / row if metric == "cosine" else row - torch.tensor(1.21, device=DEV), key)
+    want_idx, want_key = expect(key, n)
+    token = want_idx if cand is None else cand.long()[want_idx]
+    assert torch.equal(idx.long()[..., K - n:], token)
+    want = want_key * row if metric == "cosine" else (row - want_key).clamp_min(0).sqrt()
+    if sampled:
+        self = token == torch.arange(T, device=DEV).view(1, 1, T, 1)
+        want = torch.where(self, torch.tensor(-0.1 if metric == "cosine" else 1.1, device=DEV), want)
+    real = want_key > -math.inf
+    # one product, or a difference of whole numbers and its root: equal up to the root's rounding
+    assert bool(((val[..., K - n:] - want).abs() <= 2.0 ** -22 * want.abs())[real].all())
