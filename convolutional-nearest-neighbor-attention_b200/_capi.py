@@ -113,6 +113,7 @@ SIGNATURES = {
                                                     c_void, c_void, c_i64, c_i32, c_i32, c_i32, c_i32, c_i32, c_void,
                                                     c_size, c_void]),
     "convnn_b200_model_workspace_bytes": (c_size, [ctypes.POINTER(ConvnnModel)]),
+    "convnn_b200_model_workspace_least_bytes": (c_size, [ctypes.POINTER(ConvnnModel)]),
     "convnn_b200_model_forward": (ctypes.c_int, [ctypes.POINTER(ConvnnModel), c_void, c_void, c_void, c_size, c_void]),
 }
 

@@ -180,6 +180,12 @@ size_t convnn_b200_model_workspace_bytes(const convnn_model* m) {
     return p.total;
 }
 
+size_t convnn_b200_model_workspace_least_bytes(const convnn_model* m) {
+    Plan p;
+    if (check(m) || !plan_of(m, &p)) return 0;
+    return p.least;
+}
+
 int convnn_b200_model_forward(const convnn_model* m, const void* images, void* logits, void* workspace,
                               size_t workspace_bytes, void* stream) {
     int rc = check(m);

@@ -74,6 +74,7 @@ class Plan:
         L = _capi.lib()
         self.call, self.arg = L.convnn_b200_model_forward, ctypes.byref(m)
         self.workspace_bytes = L.convnn_b200_model_workspace_bytes(self.arg)
+        self.least_bytes = L.convnn_b200_model_workspace_least_bytes(self.arg)
 
     def unchanged(self, model) -> bool:
         return (self.watch.unchanged(model) and not any(self.watch.hooks) and
@@ -155,8 +156,15 @@ class Plan:
             x = x.contiguous()
         dev = x.device
         out = torch.empty(self.out_shape, dtype=self.act, device=dev)
-        ws = torch.empty(self.workspace_bytes, dtype=torch.uint8, device=dev)
-        args = (self.arg, x.data_ptr(), out.data_ptr(), ws.data_ptr(), self.workspace_bytes, ops._stream(x))
+        try:
+            ws = torch.empty(self.workspace_bytes, dtype=torch.uint8, device=dev)
+        except torch.cuda.OutOfMemoryError:
+            # room for one half of a branching block at a time is enough: they run in turn then
+            if self.workspace_bytes <= self.least_bytes:
+                raise
+            self.workspace_bytes = self.least_bytes
+            ws = torch.empty(self.least_bytes, dtype=torch.uint8, device=dev)
+        args = (self.arg, x.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel(), ops._stream(x))
         if self.sampled:
             sets = self._candidates(dev)
             if sets is None:

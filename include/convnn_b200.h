@@ -376,8 +376,9 @@ typedef struct convnn_model {
 } convnn_model;
 
 /* With branching blocks the size has a region of its own for the second half, so that the halves run beside each other; a
- * workspace that holds one half at a time is accepted too, and the halves then run in turn (same results). */
+ * workspace that holds one half at a time (..._least_bytes) is accepted too, and the halves then run in turn (same results). */
 size_t convnn_b200_model_workspace_bytes(const convnn_model* m);
+size_t convnn_b200_model_workspace_least_bytes(const convnn_model* m);
 /* images (B, C, H, W) -> logits (B, classes).  The structs are read during the call only. */
 int convnn_b200_model_forward(const convnn_model* m, const void* images, void* logits, void* workspace,
                               size_t workspace_bytes, void* stream);

@@ -158,3 +158,28 @@ def test_halves_side_by_side_give_the_bits_of_one_after_the_other(layer, heads, 
         got += [m(x) for _ in range(3)]
         assert model_plan._plans[m][(x.shape, x.dtype, x.device)] is plan
     assert all(torch.equal(y, want) for y in got)
+
+
+@pytest.mark.parametrize("layer", ["BranchConv", "BranchAttention"])
+def test_no_room_for_both_halves(layer, monkeypatch):
+    """Memory for one half of a branching block at a time is enough, as before the halves ran side by side."""
+    torch.manual_seed(3)
+    m = convnn_b200.ViT(convnn_b200.make_args(layer=layer, num_layers=3, num_heads=3, d_hidden=192, d_mlp=768, dropout=0.0,
+                                              attention_dropout=0.0, num_classes=24, device=DEV)).to(torch.bfloat16).eval()
+    x = torch.randn(5, 3, 224, 224, device=DEV).bfloat16()
+    allocate = torch.empty
+
+    def limited(*size, **kw):
+        if kw.get("dtype") is torch.uint8 and size[0] > plan.least_bytes:
+            raise torch.cuda.OutOfMemoryError("out of memory")
+        return allocate(*size, **kw)
+
+    with torch.no_grad():
+        want = _planned(m, x)
+        plan = model_plan._plans[m][(x.shape, x.dtype, x.device)]
+        assert 0 < plan.least_bytes < plan.workspace_bytes
+        monkeypatch.setattr(torch, "empty", limited)
+        got = [m(x) for _ in range(3)]
+        monkeypatch.undo()
+        assert model_plan._plans[m][(x.shape, x.dtype, x.device)] is plan
+    assert all(torch.equal(y, want) for y in got)
