@@ -29,13 +29,20 @@ void count_launch();
 // Kernels of a chain: each is launched while its predecessor on the stream still runs (programmatic stream
 // serialization), so that its launch, barrier set-up and TMEM allocation overlap the predecessor's tail.  The rule that
 // makes this safe: EVERY thread of a kernel launched with launch_chained() calls chain_wait() before its first access to
-// global memory, read or write (one exception below).  The wait ends when the predecessor has completed and its writes are visible; the
-// predecessor has waited likewise, so completion is transitive along the stream.  chain_next() lets the successor start;
-// it comes after the wait (nothing older than the predecessor can still run when a successor starts) and, in kernels that
-// allocate TMEM, after the allocation (a successor's CTA may take only what is left, and gives it back).
-// The exception: weights, where the predecessor is a kernel of this library that the same call has launched and that does not write
-// them ("at rest").  That kernel let this one start only after its own wait, so all that came before it on the stream, a
-// kernel of the caller's that wrote the weights included, has ended.  The first kernel of a call never does this.
+// global memory, read or write, and chain_next() comes after that.  The wait ends when the predecessor has completed and its
+// writes are visible; the predecessor has waited likewise, so completion is transitive along the stream and nothing older than the
+// predecessor can still run when a kernel starts.  In kernels that allocate TMEM chain_next() also comes after the allocation (a
+// successor's CTA may take only what is left, and gives it back).
+// Two exceptions, both only inside one call of this library:
+//   * Beside: a kernel that does not need its predecessor's results lets the next one start and does its work without waiting, and
+//     waits for the predecessor at its own end (chain_leave()), so that whoever waits for it has waited for both.  When the next
+//     kernel starts, two may still run: this one and its predecessor, which therefore has to be one that waited at its own start.
+//     So never two of them in a row: OtherHalf::stage() with `beside` follows a launch of the layer's own each time
+//     (layer_forward(), select_and_conv()), and a launcher that has no such form ignores the flag and waits.  What it reads was
+//     complete before that predecessor started, what it writes is apart from what that one reads or writes.
+//   * Weights at rest may be read before chain_wait() where none of the kernels that may still run writes them: the call's own earlier
+//     launches, the predecessor and, behind a kernel beside it, that one's.  The call's first kernel has waited for all that came
+//     before it on the stream, a kernel of the caller's that wrote the weights included, and never does this itself.
 // A ViT-Tiny forward is 64 kernels (52 up to 21 images) with gaps of ~1.9 us and prologues of ~2 us.  One image 827 -> 712 us, 37 images
 // 923 -> 808 us, 256 images 1757 -> 1673 us, BranchConv 64 images 1788 -> 1500 us, ViT-Small 256 images 4588 -> 4441 us.
 // The GEMM and MLP kernels' roles each wait for themselves, after their set-up (in the MLP block of one image 4.7 us passed
@@ -55,9 +62,7 @@ __device__ __forceinline__ void chain_begin_for() {
     chain_wait();
     if (sizeof(T) != 4) chain_next();
 }
-// A kernel launched BESIDE its predecessor does not need that one's results: it starts its work as soon as it is let, and waits
-// at its end instead, so that whoever waits for it has waited for both.  Its predecessor has to be one that waited at its own start
-// (so that everything older has ended), and what it reads and writes must be apart from what that one does.
+// A kernel launched beside its predecessor, see above.
 __device__ __forceinline__ void chain_wait_unless(bool beside) {
     if (!beside) chain_wait();
 }
@@ -246,10 +251,10 @@ struct GemmTcOpts {
     int ln_planes = 0;
     float ln_eps = 0.f;
     const void* ln_wextra = nullptr;
-    // The launch before this one on the stream is this library's own, made by the same call, and does not write W, its
-    // extra rows or the bias: they may be read before it has ended (see chain_wait()).
+    // What may still run on the stream is this library's own, launched by the same call, and does not write W, its extra
+    // rows or the bias: they may be read before the predecessor has ended (see chain_wait()).
     bool w_at_rest = false;
-    bool beside = false;              // see chain_leave(); takes w_at_rest
+    bool beside = false;              // see chain_leave(); where the epilogue has no such form, the kernel waits at its start
     // Row moments of the stored rows, [gemm_tc_moment_planes(N)][gemm_tc_moment_stride(M)][2]; needs a skip connection.
     float* moments_out = nullptr;
 };

@@ -10,7 +10,8 @@
 // 0.2 GB of values.  There L2 is 42 % busy and the ALU, which unpacks, 50 %: bound by the latency of the neighbour rows, so
 // what counts is how many of them an SM has in flight: four tokens side by side, one tap at a time and three CTAs (80
 // registers), whose (row, weight) pairs of a tap lie together: 131072 x 768 x 25 501 -> 477 us (two taps and two CTAs, 104
-// registers, before), 32768 x 768 x 9 66.2 -> 58.4, 32768 x 384 x 9 35.4 -> 32.6; one token: four taps, four CTAs.
+// registers, before), 32768 x 768 x 9 66.2 -> 58.4, 32768 x 384 x 9 35.4 -> 32.6; one token: four taps, four CTAs.  (The bounds
+// leave the bfloat16 forms spills of 4 to 20 bytes.)
 #include "common.cuh"
 #include "f32x2.cuh"
 

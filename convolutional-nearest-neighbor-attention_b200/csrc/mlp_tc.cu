@@ -222,8 +222,8 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         // ---- TMA producers (each CTA fetches its own rows of x and its half of every weight chunk).
         // One thread can start a TMA operation only every ~0.3 us, whatever its size, while operations
         // started by different lanes overlap: lanes 0 .. KC issue the sub-chunks of a W1 super-chunk (and
-        // the x tiles) with one instruction of the warp; lane KC + 2 stores finished tiles and refills their
-        // buffers.  The W2 stream, whose slots are released by MMA 2, has warp 20.
+        // the x tiles) with one instruction of the warp; lanes 8 .. 8 + KC - 1 store finished tiles and refill
+        // their buffers.  The W2 stream, whose slots are released by MMA 2, has warp 20.
         const uint32_t w1_mask = (2u << p.KC) - 1u;              // lanes 0 .. KC
         // one W1 super-chunk into slot b
         auto load_w1 = [&](uint32_t b, int sc) {

@@ -437,8 +437,9 @@ static Ranges ranges_of(const Dims& dm) {
 //   197 x 197, K = 25        1 image 23.5 -> 8.2    16: 24.1 -> 21.0    48: 24.4 -> 28.3 (not taken)
 //   (two batches in flight lose 0.6 % with it at 256 images: a CTA of this kernel fills its SM)
 //   1000 x 256 x 768, K = 5  1 image 18.0 -> 9.9    4: 18.2 -> 11.1     16: 18.9 -> 21.5 (not taken)
-// (Against the streaming kernel and the two-pass kernel's sorted lists.  With its bound from group maxima the two-pass kernel is
-// ahead from about 64 rows per SM on: 197 x 197, K = 9 48 images 9.8, here 9.7; 72: 9.9, 11.3; 132: 12.7, 18.7; 220: 20, 28.)
+// These figures and the lines below are against the streaming kernel and the two-pass kernel's sorted lists.  Since the two-pass
+// kernel bounds lists of up to twelve by group maxima it is ahead from about 64 rows per SM on with 197 candidates (K = 9, 48
+// images 9.8 us there, 9.7 here; 72: 9.9, 11.3; 132: 12.7, 18.7; 220: 20, 28): the lines for such lists have yet to be drawn again.
 // Where others win, and the lines of the rule (R rows per SM, rounds u of 256-row units per SM, w the share of their warps that
 // has rows: two units of the streaming kernel share an SM and slow each other down by about w / 2):
 //   * up to 128 candidates, and heads above 384 channels, only ranges that stay inside a head: a range across heads is cut into

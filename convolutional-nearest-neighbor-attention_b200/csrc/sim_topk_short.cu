@@ -17,7 +17,7 @@
 //
 // What bounds it (128 images of 12 heads, 197 x 197 x 32, K = 9, 93 us; the streaming kernel 136): instructions, 4400 per 32 rows
 // at 0.47 per cycle and scheduler, and their fetch: a chunk loop unrolled once more 125 for 106, the metric known at compile
-// time 96 for 106, tensor-memory reads one chunk ahead nothing.  us, streaming -> this kernel: 256 images of 197 x 192, K = 9
+// time 96 for 106, tensor-memory reads one chunk ahead nothing.  (18 warps of 96 registers: one thread per row spills 12 to 52 bytes.)  us, streaming -> this kernel: 256 images of 197 x 192, K = 9
 // 30.5 -> 20.7 (4: 22.8 -> 16.3), 6 heads of 64 126 -> 84, 65 x 65 x 192 12.5 -> 9.7, 1024 x 65 x 65, 3 heads of 64 94 -> 42,
 // 64 x 1000 x 200 x 256 33 -> 23, 256 x 197 x 64 x 384 17.8 -> 17.2.
 //
@@ -276,8 +276,9 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         const int tid = threadIdx.x - 64, peer = NH == 2 ? (tid ^ 128) : tid;   // the other half's thread of this row
         const int xb = g * 4 + lq;
         float* qs = statbuf + (warp - 2) * MAXC;
-        // entries of a row: the lower half's upwards from slot 0, the upper half's downwards from slot NSEL + 1; a count
-        // stops at nsel + 1 (more than nsel in all is repeated below, whatever the slots hold then)
+        // entries of a row: the lower half's upwards from slot 0, the upper half's downwards from the last.  Behind an exact
+        // threshold a count stops at nsel + 1 (more than nsel in all is repeated below, whatever the slots hold then); behind the
+        // bound of shorter lists it may reach all slots, more are marked with a count that no row has room for.
         const uint32_t hit0 = smem_u32(hits) + (uint32_t)(g * 128 + r) * 8u;
         const int c_begin = half ? ((p.S + 1) / 2 + 15) / 16 * 16 : 0;
         const int c_end = NH == 2 && !half ? min(((p.S + 1) / 2 + 15) / 16 * 16, p.S) : p.S;
