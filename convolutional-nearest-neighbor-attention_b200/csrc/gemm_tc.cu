@@ -303,10 +303,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         };
         int cur_nt = -1;
         const int lead = first < last && p.KC <= 4 ? min(p.KC, (int)STAGES) : 0;     // chunks of the first tile requested at once
-        int mt = 0, nt = 0;
-        if (first < last) tile_mn(first, mt, nt);
-        int m0 = mt * TM + (int)rank * BM, n0 = nt * p.BN + (int)rank * bn_cta;
+        int w_ahead = 0;                                                // chunks of W alone that lane 0 requests early
         if (lead > 0) {
+            int mt, nt;
+            tile_mn(first, mt, nt);
+            const int m0 = mt * TM + (int)rank * BM, n0 = nt * p.BN + (int)rank * bn_cta;
             auto request_w = [&]() {                                     // W of the first tile, or its chunks in the ring
                 if (p.wstat) {
                     if (lane == 0) mbar_expect_tx_a(wfull_a, p.KC * b_bytes + (LNF ? (uint32_t)bn_cta * 32u : 0u));
@@ -326,55 +327,57 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (lane < lead) load_a((uint32_t)lane, lane, m0);
             __syncwarp();
         }
-        if (lane == 0 && first < last) {
+        if (lane == 0) {
+            uint32_t s = lead == (int)STAGES ? 0u : (uint32_t)lead, ph = lead == (int)STAGES ? 1u : 0u;   // ring slot and its phase
+            uint32_t last_s = lead > 0 ? (uint32_t)lead - 1u : 0u, last_ph = 0;
+            int skip = lead;                                             // chunks of the first tile that are on the way
             bool ok = true;
             const bool tr = !PAIR && trace_enabled() && blockIdx.x == 0;
             int tn = 0;
             trace(tr, 0, tn);
-            auto load_w_tile = [&](int n) {
+            auto load_w_tile = [&](int nt) {
                 mbar_expect_tx_a(wfull_a, p.KC * b_bytes + (LNF ? (uint32_t)bn_cta * 32u : 0u));
-                for (int kc = 0; kc < p.KC; ++kc) tma_load_2d_a(sB0 + kc * b_bytes, &tmW, wfull_a, kc * p.KCH, n * p.BN);
-                if (LNF) tma_load_2d_a(smem_u32(xb), &tmX, wfull_a, 0, n * p.BN);
-                cur_nt = n;
+                for (int kc = 0; kc < p.KC; ++kc) tma_load_2d_a(sB0 + kc * b_bytes, &tmW, wfull_a, kc * p.KCH, nt * p.BN);
+                if (LNF) tma_load_2d_a(smem_u32(xb), &tmX, wfull_a, 0, nt * p.BN);
+                cur_nt = nt;
             };
-            int sent = lead;                                             // chunks of the first tile that are on the way
-            if (lead == 0) {
+            if (lead == 0 && first < last) {
                 if (p.w_at_rest) {                                       // W of the first tile, or as many of its chunks as the ring holds
+                    int mt, nt;
+                    tile_mn(first, mt, nt);
                     if (p.wstat) load_w_tile(nt);
                     else
-                        for (; sent < min(p.KC, (int)STAGES); ++sent) {
-                            if (!PAIR || rank == 0) mbar_expect_tx_a(full0 + 8 * sent, tx);
-                            load_w_chunk((uint32_t)sent, sent, n0);
+                        for (w_ahead = 0; w_ahead < min(p.KC, (int)STAGES); ++w_ahead) {
+                            if (!PAIR || rank == 0) mbar_expect_tx_a(full0 + 8 * w_ahead, tx);
+                            load_w_chunk((uint32_t)w_ahead, w_ahead, nt * p.BN + (int)rank * bn_cta);
                         }
                 }
                 chain_wait_unless(BESIDE);
-                if (p.wstat && cur_nt < 0) load_w_tile(nt);
-                for (int kc = 0; kc < sent; ++kc) load_a((uint32_t)kc, kc, m0);
             }
-            uint32_t s = sent == (int)STAGES ? 0u : (uint32_t)sent, ph = sent == (int)STAGES ? 1u : 0u;   // ring slot and its phase
-            uint32_t last_s = sent > 0 ? (uint32_t)sent - 1u : 0u, last_ph = 0;
-            for (int t = first;;) {
-                for (int kc = sent; kc < p.KC; ++kc) {
-                    if (!mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag)) { give_up(11); ok = false; break; }
-                    if (!PAIR || rank == 0) mbar_expect_tx_a(full0 + 8 * s, tx);
-                    load_a(s, kc, m0);
-                    load_w_chunk(s, kc, n0);
-                    last_s = s; last_ph = ph;
-                    if (++s == STAGES) { s = 0; ph ^= 1u; }
-                }
-                sent = 0;
-                t += step;
-                if (t >= last || !ok) break;
+            bool any = lead > 0;
+            for (int t = first; t < last && ok; t += step) {
+                int mt, nt;
                 tile_mn(t, mt, nt);
                 if (p.wstat && nt != cur_nt) {
                     // every MMA that reads the old W tile has completed once the most recently
                     // filled ring stage has been released
-                    if (!mbar_wait_a(empty0 + 8 * last_s, last_ph, abort_flag)) { give_up(15); break; }
+                    if (any && !mbar_wait_a(empty0 + 8 * last_s, last_ph, abort_flag)) { give_up(15); ok = false; break; }
                     load_w_tile(nt);
                 }
                 trace(tr, 0, tn);
-                m0 = mt * TM + (int)rank * BM;
-                n0 = nt * p.BN + (int)rank * bn_cta;
+                const int m0 = mt * TM + (int)rank * BM, n0 = nt * p.BN + (int)rank * bn_cta;
+                const int kc0 = skip;
+                skip = 0;
+                for (int kc = kc0; kc < p.KC; ++kc) {
+                    if (!mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag)) { give_up(11); ok = false; break; }
+                    const bool whole = w_ahead == 0;            // (otherwise its W chunk is on the way)
+                    if (whole && (!PAIR || rank == 0)) mbar_expect_tx_a(full0 + 8 * s, tx);
+                    load_a(s, kc, m0);
+                    if (whole) load_w_chunk(s, kc, n0);
+                    else --w_ahead;
+                    last_s = s; last_ph = ph; any = true;
+                    if (++s == STAGES) { s = 0; ph ^= 1u; }
+                }
             }
         }
     } else if (warp == 1) {
@@ -394,7 +397,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             int tn = 0;
             const uint32_t peer_empty0 = PAIR ? map_to_cta(empty0, 1) : 0u;
             const uint32_t peer_tfull0 = PAIR ? map_to_cta(tfull0, 1) : 0u;
-            chain_wait_unless(BESIDE);                     // (the budgets of its waits are for this kernel's work)
+            // The first tile's operands may take as long as the predecessor.  (Waiting for that one here as well, which the
+            // producer does, cost each GEMM 0.1 to 0.2 us.)
+            unsigned long long budget = kStartBudgetNs;
             for (int t = first; t < last && ok; t += step, ++tile) {
                 const uint32_t buf = tile & 1u, u = tile >> 1;
                 if (!mbar_wait_a(tempty0 + 8 * buf, (u & 1u) ^ 1u, abort_flag)) { give_up(12); ok = false; break; }
@@ -403,7 +408,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (p.wstat || mbias) tile_mn(t, mt, nt);
                 if (p.wstat) {
                     if (nt != cur_nt) {
-                        if (!mbar_wait_a(wfull_a, wloads & 1u, abort_flag)) { give_up(16); ok = false; break; }
+                        if (!mbar_wait_a(wfull_a, wloads & 1u, abort_flag, budget)) { give_up(16); ok = false; break; }
                         cur_nt = nt;
                         ++wloads;
                     }
@@ -416,7 +421,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     else mma_bf16_ss(d_tmem, ones_desc, bias_desc, idesc, 0);
                 }
                 for (int kc = 0; kc < p.KC; ++kc) {
-                    if (!mbar_wait_a(full0 + 8 * s, ph, abort_flag)) { give_up(13); ok = false; break; }
+                    if (!mbar_wait_a(full0 + 8 * s, ph, abort_flag, budget)) { give_up(13); ok = false; break; }
                     tc_fence_after_sync();
                     const uint64_t adesc = dhi | (uint64_t)(((sA0 + s * a_bytes) & 0x3FFFFu) >> 4);
                     const uint64_t bdesc = dhi | (uint64_t)(((sB0 + (p.wstat ? (uint32_t)kc : s) * b_bytes) & 0x3FFFFu) >> 4);
@@ -437,13 +442,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
                 if (LNF && ok) {
                     // accumulator += [-mean, sigma] x [c, b']: the chunk the extra warp wrote for this buffer
-                    if (!mbar_wait_a(smem_u32(&xfull[buf]), u & 1u, abort_flag)) { give_up(17); ok = false; break; }
+                    if (!mbar_wait_a(smem_u32(&xfull[buf]), u & 1u, abort_flag, budget)) { give_up(17); ok = false; break; }
                     tc_fence_after_sync();
                     const uint64_t xa_desc = dhi32 | (uint64_t)(((smem_u32(xa) + buf * 4096u) & 0x3FFFFu) >> 4);
                     const uint64_t xb_desc = dhi32 | (uint64_t)((smem_u32(xb) & 0x3FFFFu) >> 4);
                     mma_bf16_ss(d_tmem, xa_desc, xb_desc, idesc, 1);
                     mma_commit_a(empty0 + 8 * last_stage);
                 }
+                budget = kWaitBudgetNs;
                 if (ok) {
                     if (PAIR) { mma_commit_pair(tfull0 + 8 * buf); mma_commit_pair(peer_tfull0 + 8 * buf); }
                     else mma_commit_a(tfull0 + 8 * buf);

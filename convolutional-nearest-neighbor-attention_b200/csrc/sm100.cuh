@@ -45,13 +45,16 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Bounded wait: gives up once `budget_ns` of wall time (the GPU's nanosecond timer) have passed
 // or as soon as *abort becomes non-zero, and reports failure so the caller can record an error
 // and leave instead of hanging the GPU.  The timer is read once per 256 polls; an extra poll
-// counter backs it up should the timer not advance.  No role polls for what can only come after
-// the predecessor on the stream has ended (it waits for that first, see chain_wait(), which has no
-// limit), so in normal operation no wait of these kernels lasts longer than the epilogue of one
-// tile (tens of microseconds); the budget only has to exceed that under time slicing or a
-// profiler's replay.
+// counter backs it up should the timer not advance.  A role that needs what can only come after
+// the predecessor on the stream has ended waits for that first (chain_wait(), which has no limit) or
+// polls for it with the start budget, so in normal operation no other wait of these kernels lasts
+// longer than the epilogue of one tile (tens of microseconds); the budget only has to exceed that
+// under time slicing or a profiler's replay.
 constexpr unsigned long long kWaitBudgetNs = 250ull * 1000 * 1000;
 constexpr uint32_t kWaitPollLimit = 1u << 28;
+// What may follow in the time of a whole predecessor: longer than any kernel.
+constexpr unsigned long long kStartBudgetNs = 60ull * 1000 * 1000 * 1000;
+constexpr uint32_t kStartPollLimit = 1u << 31;
 __device__ __forceinline__ unsigned long long global_timer_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -84,14 +87,15 @@ __device__ __forceinline__ bool mbar_try_wait_a(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ bool mbar_wait_a(uint32_t bar, uint32_t parity, volatile int* abort) {
+__device__ __forceinline__ bool mbar_wait_a(uint32_t bar, uint32_t parity, volatile int* abort,
+                                            unsigned long long budget_ns = kWaitBudgetNs) {
     if (mbar_try_wait_a(bar, parity)) return true;          // common case: already complete
     const unsigned long long t0 = global_timer_ns();
-    for (uint32_t i = 0; i < kWaitPollLimit; ++i) {
+    for (uint32_t i = 0; i < kStartPollLimit; ++i) {
         if (mbar_try_wait_a(bar, parity)) return true;
         if ((i & 255u) == 255u) {
             if (*abort) return false;
-            if (global_timer_ns() - t0 > kWaitBudgetNs) return false;
+            if (global_timer_ns() - t0 > budget_ns) return false;
         }
     }
     return false;
