@@ -6,8 +6,8 @@ MLP kernel's 197 row tiles on 74 CTA pairs leave a third of the pairs idle for t
 kernel, the output projection's 394 tiles on 148 CTAs likewise, and between two kernels of a chain the
 GPU is empty for a launch latency.  A second batch that runs the same chain beside the first fills
 those gaps with its own kernels' CTAs.  Measured on a B200, ViT-Tiny ConvNN-Attention, 256 images per
-batch: 1.61 ms per batch one after another, 1.41-1.43 ms with two forwards as the two branches of ONE
-CUDA graph.  (Two graphs replayed on two streams gave 1.52 ms in some runs and 1.62 ms in others: how
+batch: 1.45 ms per batch one after another, 1.27-1.30 ms with two forwards as the two branches of ONE
+CUDA graph.  (Two graphs replayed on two streams gave, when one after another took 1.61, 1.52 ms in some runs and 1.62 in others: how
 the two chains interleave then depends on the phase they happen to fall into; branches of one graph
 start together at every replay.)  The reference runs one batch at a time (main.py's evaluation loop);
 the results per batch are the same bits either way.
