@@ -629,8 +629,15 @@ int cheapest_tile(const Tile (&tiles)[COUNT], const GemmParams& p, int first = 0
 // best of twelve tiles on average, 12 % at worst.  With the first two tiles alone (and smaller transposed ones, since
 // gone) 2080 rows took 33.0 us at 192 x 768, now 25.8; 20.6 at 576 x 192, now 17.8; 1576 x 384 x 192 15.5, now 11.5; 1050
 // x 384 x 384 18.7, now 15.6.
+// Few values of k give the copies nothing to run ahead of, and their start costs 0.3 to 0.6 us: the smallest transposed tile then, up to
+// 32 values while an SM runs few of them (24853 x 28 x 16 5.5 us with a copy tile, 4.3; 99 x 39 x 4 5.4, 4.8), up to 96 while it runs one
+// (500 x 64 x 96 4.8, 4.6; with two to four 2000 x 192 x 96 6.1, 6.4), and up to 64 where columns are stored one by one (28216 x 10 x
+// 44 10.3, 8.3; 3196 x 659 x 40 19.6, 17.2; with whole vectors 4100 x 384 x 64 9.9, 12.1).
 template <int MODE>
 int launch_plain_f32(const GemmParams& p, cudaStream_t st) {
+    const int few = p.Kd <= 32 ? 14 : p.Kd <= 64 && !p.c_vec ? 21 : p.Kd <= 96 ? 1 : 0;       // tiles per SM
+    if ((long long)((p.M + 31) / 32) * ((p.N + 31) / 32) <= (long long)few * device_sms() && (p.N + 31) / 32 <= 65535)
+        return launch_tile<float, float, MODE, 32, 32, 32, 4, 4, 4>(p, st);
     static const Tile tiles[6] = {
         {128, 64, 1, 3, 5.4, 0.5, {65.4, 107.1, 153.3}},
         {64, 64, 1, 3, 3.2, 0.7, {38.2, 62.3, 88.9}},

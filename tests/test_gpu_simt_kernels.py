@@ -242,8 +242,9 @@ def test_statistics_of_all_tensors_in_one_launch(B, T, S, H, dk, coord, dtype, m
 # columns and k; a sum is the same whichever tile it was computed in.
 @on_148_sms
 @pytest.mark.parametrize("M,N,K,tile", [
-    (2081, 190, 100, "32x32 4x4"), (1, 1, 4, "32x32 4x4"), (33, 65, 768, "32x32 4x4"), (3121, 190, 764, "32x32 4x4"),
-    (5003, 193, 36, "40x32 5x4"), (1576, 385, 100, "40x32 5x4"), (1001, 1003, 192, "40x32 5x4"), (2081, 190, 768, "48x32 6x4"),
+    (2081, 190, 100, "32x32 4x4"), (1, 1, 4, "transposed"), (1, 1, 132, "32x32 4x4"), (33, 65, 768, "32x32 4x4"), (3121, 190, 764, "32x32 4x4"),
+    (5003, 193, 36, "transposed"), (1576, 385, 100, "40x32 5x4"), (1001, 1003, 192, "40x32 5x4"), (500, 64, 96, "transposed"),
+    (5003, 192, 36, "40x32 5x4"), (1301, 64, 96, "transposed"), (3200, 64, 96, "32x32 4x4"), (5003, 192, 20, "transposed"), (2081, 190, 768, "48x32 6x4"),
     (1050, 383, 388, "48x32 6x4"), (5203, 190, 768, "56x32 7x4"), (2081, 577, 32, "transposed"), (50432, 190, 8, "transposed")])
 def test_tiles_of_float32_rows(M, N, K, tile):
     g = torch.Generator(device=DEV).manual_seed(M + N)
