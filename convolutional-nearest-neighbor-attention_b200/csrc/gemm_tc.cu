@@ -1047,11 +1047,6 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
         const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmW, tmX, tmM, p);                                                    \
         if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "gemm_tc pair launch: %s", cudaGetErrorString(e)); \
     } while (0)
-#define CONVNN_GEMM_LAUNCH(S, B, G, R)                          \
-    do {                                                        \
-        if (wide) CONVNN_GEMM_LAUNCH1(false, B, G, R, true);    \
-        else CONVNN_GEMM_LAUNCH1(S, B, G, R, false);            \
-    } while (0)
     if (lnf) {
         if (has_stat && wide) CONVNN_GEMM_LAUNCH_X(true, false, false, true, true, false);
         else if (has_stat) CONVNN_GEMM_LAUNCH_X(true, false, false, false, true, false);
@@ -1068,12 +1063,11 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
     // (with another epilogue, or as a pair, it waits at its start, which is as right)
     if (o.beside && !has_stat && !wide) CONVNN_GEMM_LAUNCH1(false, false, false, false, false, false, false, true);
     else if (has_stat) CONVNN_GEMM_LAUNCH1(true, false, false, false, false);
-    else if (p.gelu) { if (p.bias) CONVNN_GEMM_LAUNCH(false, true, true, false); else CONVNN_GEMM_LAUNCH(false, false, true, false); }
-    else if (p.bias && p.residual) CONVNN_GEMM_LAUNCH(false, true, false, true);
-    else if (p.bias) CONVNN_GEMM_LAUNCH(false, true, false, false);
-    else if (p.residual) CONVNN_GEMM_LAUNCH(false, false, false, true);
-    else CONVNN_GEMM_LAUNCH(false, false, false, false);
-#undef CONVNN_GEMM_LAUNCH
+    else if (p.gelu) { if (p.bias) CONVNN_GEMM_LAUNCH1(false, true, true, false, true); else CONVNN_GEMM_LAUNCH1(false, false, true, false, true); }
+    else if (p.bias && p.residual) CONVNN_GEMM_LAUNCH1(false, true, false, true, true);
+    else if (p.bias) CONVNN_GEMM_LAUNCH1(false, true, false, false, true);
+    else if (p.residual) CONVNN_GEMM_LAUNCH1(false, false, false, true, true);
+    else CONVNN_GEMM_LAUNCH1(false, false, false, false, false);
 #undef CONVNN_GEMM_LAUNCH1
 #undef CONVNN_GEMM_LAUNCH_PAIR
 #undef CONVNN_GEMM_LAUNCH_X
