@@ -659,8 +659,8 @@ int launch_plain_f32(const GemmParams& p, cudaStream_t st) {
 // Other plain rows: float32 ones of any alignment, bfloat16, float32 against bfloat16 weights.  Which tiles, and which times, goes by
 // what the operands cost: float32 values need no conversion, so that the transposed tiles wait for little and the largest of
 // them reuses most; bfloat16 values that come one by one are what the transposed tiles wait for.  Narrow outputs of few
-// values of k (the separable conv with the coordinate channel on heads of 8 to 32) end before that counts.  Fits to 209, 98, 98
-// and 90 shapes (30 to 1000000 rows, 8 to 2304 columns, 9 to 2048 values of k; rms 3 to 21 %), the choice within 1.2, 1.5, 0.8
+// values of k (the separable conv with the coordinate channel on heads of 8 to 32) end before that counts.  Fits to 209, 90, 98
+// and 90 shapes (30 to 1000000 rows, 8 to 2304 columns, 9 to 2048 values of k; rms 3 to 21 %), the choice within 1.2, 1.0, 0.8
 // and 0.9 % of the best of seven tiles on average; 0.95, 0.72, 0.55 and 0.71 of the time of the four transposed tiles alone, at worst
 // 1.09 (kernels of 4 us).
 // float32, us, staged tiles only -> now: 2813 x 768 x 769 138 -> 102, 56288 x 256 x 257 244 -> 189, 39846 x 8 x 9 9.9 -> 6.7; mixed 650981 x
@@ -683,11 +683,11 @@ int launch_plain_staged(const GemmParams& p, cudaStream_t st) {
         }
     } else {
         static const Tile by_four[5] = {
-            {128, 64, 16, 3, 6.1, 0.1, {114.3, 172.4, 213.5}},
-            {32, 32, 32, 7, 1.7, 0.7, {61.3, 66.3, 69.6, 67.3, 84.9, 69.6, 84.1}},
-            {64, 64, 32, 3, 3.2, 2.9, {40.5, 62.2, 101.5}},
-            {32, 64, 32, 4, 2.2, 1.6, {27.8, 42.1, 59.7, 78.7}},
-            {40, 32, 32, 6, 2.6, 2.5, {31.9, 34.4, 43.8, 46.8, 66.8, 75.5}},
+            {128, 64, 16, 3, 0.0, 4.1, {122.5, 162.1, 187.0}},
+            {32, 32, 32, 7, 2.1, 0.0, {62.1, 67.9, 72.2, 82.4, 84.4, 93.8, 81.1}},
+            {64, 64, 32, 3, 2.4, 2.9, {41.0, 62.8, 91.7}},
+            {32, 64, 32, 4, 1.5, 1.8, {27.3, 43.1, 59.2, 76.9}},
+            {40, 32, 32, 6, 1.8, 2.5, {32.2, 34.5, 46.8, 51.2, 60.2, 70.8}},
         };
         static const Tile by_value[5] = {
             by_four[0],                                              // (not taken: 4039 x 768 x 385 135 us, the third 93)
