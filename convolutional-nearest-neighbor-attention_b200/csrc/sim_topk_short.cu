@@ -30,6 +30,7 @@
 #include "sm100.cuh"
 #include "toplist.cuh"
 #include "sim_topk_select.cuh"
+#include "packed_rank.cuh"
 
 namespace convnn {
 
@@ -62,44 +63,6 @@ __device__ __forceinline__ void fail(volatile int* abort_flag, int code) {
 
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld_x32(taddr, r); }
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld_x16(taddr, r); }
-
-// (NaN stays out of the list: min propagates it, max drops it)
-__device__ __forceinline__ float min_nan(float a, float b) {
-    float r;
-    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-    float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-
-template <int NSEL>
-__device__ __forceinline__ void merge_pair(float (&v)[NSEL], float k0, float k1) {
-    const float a = fmaxf(k0, k1), b = min_nan(k0, k1);
-#pragma unroll
-    for (int s = NSEL - 1; s >= 2; --s) v[s] = max3(v[s], min_nan(v[s - 1], a), min_nan(v[s - 2], b));
-    if (NSEL > 1) v[1] = max3(v[1], min_nan(v[0], a), b);
-    v[0] = fmaxf(v[0], a);
-}
-
-// Descending sort of 16 values (Batcher's odd-even merge exchange); exchanges that only order unused outputs fall away.
-__device__ __forceinline__ void sort16(float (&v)[16]) {
-#pragma unroll
-    for (int lp = 0; lp < 4; ++lp)
-#pragma unroll
-        for (int lk = lp; lk >= 0; --lk)
-#pragma unroll
-            for (int x = 0; x < 16; ++x) {
-                const int p = 1 << lp, k = 1 << lk, j = k % p;
-                if (x >= j && ((x - j) / k) % 2 == 0 && x + k < 16 && x / (2 * p) == (x + k) / (2 * p)) {
-                    const float a = v[x], b = v[x + k];
-                    v[x] = fmaxf(a, b);
-                    v[x + k] = fminf(a, b);
-                }
-            }
-}
 
 // Ranking keys of W accumulator columns from `col0` on; -inf past the last candidate.
 // METRIC < 0: p.metric.  CLOSED: the statistics past the last candidate are NaN, and so are the keys (MATMUL has none).
@@ -159,22 +122,22 @@ __device__ __forceinline__ void insert_first(TopList<NSEL>& top, const E& entry,
     }
 }
 
-// Lists whose rows are bounded by group maxima, and the entries a row has room for then (a side is checked every eight columns).
+// Lists of more than twelve are ranked by a network (one thread per row); the entries a row has room for (checked every eight columns).
+template <int NSEL>
+constexpr bool networked = NSEL > 12;
 template <int NSEL, int NH>
-constexpr bool bounded = NSEL <= 9 || (NSEL <= 12 && NH == 2);
-template <int NSEL, int NH>
-constexpr int slots_of = bounded<NSEL, NH> ? (NH == 2 ? 28 : 32) : NSEL + 2;
+constexpr int slots_of = NSEL <= 12 ? (NH == 2 ? 28 : 32) : NSEL <= 16 ? 32 : NSEL <= 25 ? 48 : 60;
 
 template <int NSEL, int G, int NH, int METRIC>
 __global__ void __launch_bounds__(64 + 128 * G * NH, 1)
 sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const ShortParams p) {
     constexpr int MAXC = 512 / G;                  // tensor-memory columns of one accumulator
-    constexpr int W = G * NH == 4 ? 16 : 32;       // columns per read (18 warps leave 96 registers per thread)
     constexpr int NT = 128 * G * NH;               // selection threads
+    constexpr int W = G == 4 ? 16 : 32;            // columns per read of a long list's first pass (18 warps leave 96 registers per thread)
     constexpr uint32_t ENTRY = 128 * G * 8;        // bytes between a row's successive entries
-    constexpr bool BOUND = bounded<NSEL, NH>;
     constexpr int SLOTS = slots_of<NSEL, NH>;
-    constexpr bool LISTS = BOUND || NH == 2;
+    constexpr bool NETWORK = networked<NSEL>;
+    static_assert(!NETWORK || NH == 1, "rows of long lists are one thread's");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t pitch = p.KCH * 2;
@@ -183,8 +146,8 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     float2* hits = reinterpret_cast<float2*>(smem + STAGES * stage_bytes);       // [SLOTS][128 * G] (key, column)
     float* statbuf = reinterpret_cast<float*>(hits + SLOTS * 128 * G);      // [warps][MAXC] column statistics
     int* cs = reinterpret_cast<int*>(statbuf + NT / 32 * MAXC);                  // [MAXC] candidate tokens
-    float* lists = reinterpret_cast<float*>(cs + MAXC);                          // LISTS: [NSEL][NT] sorted keys
-    int* counts = reinterpret_cast<int*>(lists + (LISTS ? NSEL * NT : 0));       // NH = 2: [NT] entries
+    float* lists = reinterpret_cast<float*>(cs + MAXC);                          // short lists: [NSEL][NT] sorted keys
+    int* counts = reinterpret_cast<int*>(lists + (NETWORK ? 0 : NSEL * NT));       // NH = 2: [NT] entries
     uint64_t* full = reinterpret_cast<uint64_t*>(counts + (NH == 2 ? NT : 0));
     uint64_t* empty = full + MAX_STAGES;
     uint64_t* tfull = empty + MAX_STAGES;
@@ -276,9 +239,8 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         const int tid = threadIdx.x - 64, peer = NH == 2 ? (tid ^ 128) : tid;   // the other half's thread of this row
         const int xb = g * 4 + lq;
         float* qs = statbuf + (warp - 2) * MAXC;
-        // entries of a row: the lower half's upwards from slot 0, the upper half's downwards from the last.  Behind an exact
-        // threshold a count stops at nsel + 1 (more than nsel in all is repeated below, whatever the slots hold then); behind the
-        // bound of shorter lists it may reach all slots, more are marked with a count that no row has room for.
+        // entries of a row: the lower half's upwards from slot 0, the upper half's downwards from the last; more than there are
+        // slots are marked with a count that no row has room for.
         const uint32_t hit0 = smem_u32(hits) + (uint32_t)(g * 128 + r) * 8u;
         const int c_begin = half ? ((p.S + 1) / 2 + 15) / 16 * 16 : 0;
         const int c_end = NH == 2 && !half ? min(((p.S + 1) / 2 + 15) / 16 * 16, p.S) : p.S;
@@ -300,17 +262,16 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
             if (p.metric != CONVNN_MATMUL) {
                 const float* qrow = p.qstat + (long long)bh * p.S;
 #pragma unroll
-                for (int c = 0; c < MAXC; c += 32) qs[c + lane] = c + lane < p.S ? qrow[c + lane] : (BOUND ? CUDART_NAN_F : 0.f);
+                for (int c = 0; c < MAXC; c += 32) qs[c + lane] = c + lane < p.S ? qrow[c + lane] : CUDART_NAN_F;
             }
             __syncwarp();
             ok = mbar_wait(&tfull[g], use & 1u, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) { if (lane == 0) fail(abort_flag, 74); break; }
             tc_fence_after_sync();
-            bool exact = true;
-            int n_low = 0;
-            if constexpr (BOUND) {
-                int cnt = 0;
+            if constexpr (!NETWORK) {
+                bool exact = true;
+                int n_low = 0, cnt = 0;
                 if (warp_live) {
                     // Pass 1: maxima of column groups, sixteen per half of a row (NH = 1: of the even and the odd chunks).
                     float v[16], w[16];
@@ -330,8 +291,8 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
                         into(v, c);
                         if (NH == 1 && c + 16 < c_end) into(w, c + 16);
                     }
-                    sort16(v);
-                    if (NH == 1) sort16(w);
+                    sort_descending(v);
+                    if (NH == 1) sort_descending(w);
 #pragma unroll
                     for (int s = 0; s < NSEL; ++s) lists[s * NT + tid] = NH == 1 ? w[s] : v[s];
                     if (NH == 2) {
@@ -447,137 +408,123 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
                     }
                     if (row_ok && exact) write_selection<NSEL>(top, p, ((long long)bh * p.T + row) * p.K, row, kst);
                 }
-                continue;
-            }
-            if (warp_live) {
-                float v[NSEL];
-#pragma unroll
-                for (int s = 0; s < NSEL; ++s) v[s] = -CUDART_INF_F;
+            } else {
+                uint32_t at = hit0;
+                bool redo = false;
+                if (warp_live) {
+                    // Pass 1: maxima of 64 column groups, 32 of the even chunks of 32 columns and 32 of the odd ones.
+                    float thr = -CUDART_INF_F, largest = -CUDART_INF_F;
+                    {
+                        float v[32];
 #pragma unroll 1
-                for (int c = c_begin; c < c_end; c += W) {
-                    uint32_t acc[W];
-                    tmem_ld(taddr + c, acc);
-                    tmem_ld_wait();
-                    float key[W];
-                    make_keys<W>(key, acc, qs, cs, c, p, row, sentinel);
+                        for (int odd = 0; odd < 2; ++odd) {
 #pragma unroll
-                    for (int j = 0; j < W; j += 2) merge_pair<NSEL>(v, key[j], key[j + 1]);
-                }
-                float thr = v[0];                    // v[nsel - 1] = the smallest of the first nsel
-#pragma unroll
-                for (int s = 1; s < NSEL; ++s) thr = fminf(thr, s < p.nsel ? v[s] : CUDART_INF_F);
-                if (NH == 2) {
-#pragma unroll
-                    for (int s = 0; s < NSEL; ++s) lists[s * NT + tid] = v[s];
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&xlist[xb]);
-                    ok = mbar_wait(&xlist[xb], use_of_pair & 1u, abort_flag);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) { if (lane == 0) fail(abort_flag, 75); break; }
-                    thr = fmaxf(thr, lists[(p.nsel - 1) * NT + peer]);
-#pragma unroll
-                    for (int i = 0; i < NSEL - 1; ++i)
-                        if (i < p.nsel - 1) thr = fmaxf(thr, fminf(v[i], lists[(p.nsel - 2 - i) * NT + peer]));
-                }
-                int cnt = 0;
-                const uint32_t first = half ? hit0 + (NSEL + 1) * ENTRY : hit0;
-                uint32_t at = first;
+                            for (int j = 0; j < 32; ++j) v[j] = -CUDART_INF_F;
 #pragma unroll 1
-                for (int c = c_begin; c < c_end; c += W) {
-                    uint32_t acc[W];
-                    tmem_ld(taddr + c, acc);
-                    tmem_ld_wait();
-                    float key[W];
-                    make_keys<W>(key, acc, qs, cs, c, p, row, sentinel);
+                            for (int c = 32 * odd; c < p.S; c += 64) {
 #pragma unroll
-                    for (int j = 0; j < W; ++j) {
-                        if (key[j] >= thr) {
-                            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(__float_as_uint(key[j])), "r"(c + j)
-                                         : "memory");
-                            at = half ? max(at - ENTRY, hit0 + (uint32_t)(NSEL - p.nsel) * ENTRY)
-                                      : min(at + ENTRY, hit0 + (uint32_t)(p.nsel + 1) * ENTRY);
+                                for (int w = 0; w < 32; w += W) {
+                                    uint32_t acc[W];
+                                    tmem_ld(taddr + c + w, acc);
+                                    tmem_ld_wait();
+                                    float key[W];
+                                    make_keys<W, METRIC, true>(key, acc, qs, cs, c + w, p, row, sentinel);
+#pragma unroll
+                                    for (int j = 0; j < W; ++j) v[w + j] = fmaxf(v[w + j], key[j]);
+                                }
+                            }
+                            sort_descending(v);
+                            largest = fmaxf(largest, v[0]);
+                            if (odd) break;
+#pragma unroll
+                            for (int s = 0; s < NSEL; ++s)       // (into the row's own, still empty slots)
+                                asm volatile("st.shared.f32 [%0], %1;" ::"r"(hit0 + s * ENTRY), "f"(v[s]) : "memory");
+                        }
+                        // the nsel-th largest of both
+                        thr = v[0];
+#pragma unroll
+                        for (int s = 1; s < NSEL; ++s) thr = fminf(thr, s < p.nsel ? v[s] : CUDART_INF_F);
+                        auto of_even = [&](int s) {
+                            float x;
+                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(hit0 + s * ENTRY) : "memory");
+                            return x;
+                        };
+                        thr = fmaxf(thr, of_even(p.nsel - 1));
+#pragma unroll
+                        for (int i = 0; i < NSEL - 1; ++i)
+                            if (i < p.nsel - 1) thr = fmaxf(thr, fminf(v[i], of_even(p.nsel - 2 - i)));
+                    }
+                    // Pass 2: the columns that reach it.
+                    constexpr uint32_t ROOM = (SLOTS - 8) * ENTRY;
+                    bool over = false;
+#pragma unroll 1
+                    for (int c = 0; c < p.S; c += 16) {
+                        uint32_t acc[16];
+                        tmem_ld_x16(taddr + c, acc);
+                        tmem_ld_wait();
+                        float key[16];
+                        make_keys<16, METRIC, true>(key, acc, qs, cs, c, p, row, sentinel);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            if (j % 8 == 0) {
+                                over = over || at > hit0 + ROOM;
+                                at = min(at, hit0 + ROOM);
+                            }
+                            if (key[j] >= thr) {
+                                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(__float_as_uint(key[j])), "r"(c + j)
+                                             : "memory");
+                                at += ENTRY;
+                            }
                         }
                     }
-                }
-                cnt = (int)((half ? first - at : at - first) / ENTRY);
-                n_low = cnt;
-                if (NH == 2) {
-                    counts[tid] = cnt;
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&xhits[xb]);
-                    if (ranks) {
-                        ok = mbar_wait(&xhits[xb], use_of_pair & 1u, abort_flag);
-                        ok = __all_sync(0xffffffffu, ok);
-                        if (!ok) { if (lane == 0) fail(abort_flag, 76); break; }
-                        const int other = counts[peer];
-                        n_low = half ? other : cnt;
-                        cnt += other;
-                    }
-                    ++use_of_pair;
-                }
-                if (ranks) {
-                    exact = !row_ok || (cnt == p.nsel && thr > -CUDART_INF_F);
-                    if (!__all_sync(0xffffffffu, exact)) {
+                    // Too many of them (ties), fewer than nsel keys above -inf (NaN inputs), keys of +inf: the row takes the columns
+                    // above the bound chunk by chunk.
+                    redo = row_ok && (over || !(thr > -CUDART_INF_F) || !(largest < CUDART_INF_F));
+                    if (!row_ok) at = hit0;
+                    if (__any_sync(0xffffffffu, redo)) {
                         TopList<NSEL> top;
                         top.init();
+                        const float floor = just_below(thr);
 #pragma unroll 1
                         for (int c = 0; c < p.S; c += 16) {
                             uint32_t acc[16];
                             tmem_ld_x16(taddr + c, acc);
                             tmem_ld_wait();
                             float key[16];
-                            make_keys<16>(key, acc, qs, cs, c, p, row, sentinel);
+                            make_keys<16, METRIC, true>(key, acc, qs, cs, c, p, row, sentinel);
+                            const float low = fmaxf(top.worst(), floor);
+                            uint32_t mask = 0;
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) top.insert_sorted(key[j], c + j);
+                            for (int j = 0; j < 16; ++j) {
+                                mask |= key[j] > low ? 1u << j : 0u;
+                                if (redo) hits[j * 128 * G + g * 128 + r].x = key[j];
+                            }
+                            if (!redo) mask = 0;
+                            const int steps = __reduce_max_sync(0xffffffffu, __popc(mask));
+                            for (int it = 0; it < steps; ++it) {
+                                const int j = mask ? __ffs(mask) - 1 : 0;
+                                const float kc = hits[j * 128 * G + g * 128 + r].x;
+                                if (mask && kc > top.worst()) top.insert_sorted(kc, c + j);
+                                mask &= mask - 1;
+                            }
                         }
-                        if (row_ok && !exact)
-                            write_selection<NSEL>(top, p, ((long long)bh * p.T + row) * p.K, row, kst);
-                    }
-                }
-            }
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty[g]);
-            if (ranks && row_ok && exact) {
-                const float2* e = hits + g * 128 + r;
-                // n-th entry in column order
-                auto entry = [&](int n) { return (NH == 1 || n < n_low ? n : NSEL + 1 + n_low - n) * 128 * G; };
-                float key[NSEL];
-                int slot[NSEL];
+                        if (redo) {                  // its list is its entries
 #pragma unroll
-                for (int n = 0; n < NSEL; ++n) {
-                    key[n] = n < p.nsel ? e[entry(n)].x : -CUDART_INF_F;
-                    slot[n] = 0;
-                }
-#pragma unroll
-                for (int n = 1; n < NSEL; ++n)
-#pragma unroll
-                    for (int m = 0; m < n; ++m) {
-                        const int first = key[m] >= key[n] ? 1 : 0;
-                        slot[n] += first;
-                        slot[m] += 1 - first;
-                    }
-                long long obase = ((long long)bh * p.T + row) * p.K;
-                if (p.sampled) {
-                    p.idx[obase] = row;
-                    p.val[obase] = 1.0f;
-                    ++obase;
-                }
-#pragma unroll
-                for (int n = 0; n < NSEL; ++n) {
-                    if (n < p.nsel) {
-                        int tok = __float_as_int(e[entry(n)].y);
-                        float s;
-                        if (p.metric == CONVNN_COSINE) s = key[n] * kst;
-                        else if (p.metric == CONVNN_MATMUL) s = key[n] / p.sqrt_dk;
-                        else s = sqrtf(fmaxf(kst - key[n], 0.f));
-                        if (p.sampled) {
-                            tok = cs[tok];
-                            if (tok == row) s = (p.metric == CONVNN_EUCLIDEAN) ? 1.1f : -0.1f;
+                            for (int s = 0; s < NSEL; ++s)
+                                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(hit0 + s * ENTRY),
+                                             "r"(__float_as_uint(top.v[s])), "r"(top.i[s]) : "memory");
+                            at = hit0 + p.nsel * ENTRY;
                         }
-                        p.idx[obase + slot[n]] = tok;
-                        p.val[obase + slot[n]] = s;
                     }
+                }
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&tempty[g]);
+                if (warp_live) {
+                    TopList<NSEL> top;
+                    rank_entries<NSEL, SLOTS>(top, hit0, ENTRY, (int)((at - hit0) / ENTRY), p.nsel, redo);
+                    write_rows<NSEL>(top, p, cs, smem_u32(hits) + (uint32_t)(g * 128 + lq * 32) * 8u, ENTRY,
+                                     ((long long)bh * p.T + rt * BM + lq * 32) * p.K, min(32, p.T - rt * BM - lq * 32), row, kst);
                 }
             }
         }
@@ -602,7 +549,7 @@ int launch_metric(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const 
     const size_t stage = (size_t)(BM + p.BN) * p.KCH * 2;
     constexpr int NT = 128 * G * NH;
     const size_t fixed = 1024 + (size_t)slots_of<NSEL, NH> * 128 * G * 8 + (size_t)(NT / 32 + 1) * MAXC * 4 +
-                         (bounded<NSEL, NH> || NH == 2 ? (size_t)(NSEL + 1) * NT * 4 : 0) + (2 * MAX_STAGES + 10 * G) * 8 + 16;
+                         (networked<NSEL> ? 0 : (size_t)(NSEL + 1) * NT * 4) + (2 * MAX_STAGES + 10 * G) * 8 + 16;
     p.stages = (int)((226 * 1024 - fixed) / stage);
     if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
     if (p.stages > 2 * p.KC) p.stages = 2 * p.KC;            // deeper than two units' chunks serves nothing
@@ -618,13 +565,9 @@ int launch_metric(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const 
 
 template <int NSEL, int G, int NH>
 int launch_short(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const CUtensorMap& tmQ, cudaStream_t st) {
-    if constexpr (bounded<NSEL, NH>) {
-        if (p.metric == CONVNN_COSINE) return launch_metric<NSEL, G, NH, CONVNN_COSINE>(dm, p, tmK, tmQ, st);
-        if (p.metric == CONVNN_MATMUL) return launch_metric<NSEL, G, NH, CONVNN_MATMUL>(dm, p, tmK, tmQ, st);
-        return launch_metric<NSEL, G, NH, CONVNN_EUCLIDEAN>(dm, p, tmK, tmQ, st);
-    } else {
-        return launch_metric<NSEL, G, NH, -1>(dm, p, tmK, tmQ, st);
-    }
+    if (p.metric == CONVNN_COSINE) return launch_metric<NSEL, G, NH, CONVNN_COSINE>(dm, p, tmK, tmQ, st);
+    if (p.metric == CONVNN_MATMUL) return launch_metric<NSEL, G, NH, CONVNN_MATMUL>(dm, p, tmK, tmQ, st);
+    return launch_metric<NSEL, G, NH, CONVNN_EUCLIDEAN>(dm, p, tmK, tmQ, st);
 }
 
 }  // namespace
@@ -642,7 +585,7 @@ bool sim_topk_short_wanted(const Dims& dm) {
     if (dm.S > 256) return false;
     const long long sms = device_sms(), bh = (long long)dm.B * dm.H, units = bh * ((dm.T + BM - 1) / BM);
     if (units <= sms) return true;
-    if (dm.nsel > 12) return dm.nsel <= 16;
+    if (dm.nsel > 12) return true;
     if (dm.T > BM && dm.S <= 32) return false;
     if (dm.T <= BM && dm.S <= 40) {
         if (dm.Cp > 512) return true;
@@ -691,8 +634,7 @@ int launch_sim_topk_short(const convnn_desc* d, const Dims& dm, const void* q, c
     if (n == 9) CONVNN_SHORT(9);
     if (n <= 12) return launch_short<12, 2, 2>(dm, p, tmK, tmQ, st);
     if (n <= 16 && dm.S <= 128) return launch_short<16, 4, 1>(dm, p, tmK, tmQ, st);
-    if (n <= 16) return launch_short<16, 2, 2>(dm, p, tmK, tmQ, st);
-    // (longer lists: their exchange buffers would take the ring's shared memory)
+    if (n <= 16) return launch_short<16, 2, 1>(dm, p, tmK, tmQ, st);
     if (n <= 25) return launch_short<25, 2, 1>(dm, p, tmK, tmQ, st);
     return launch_short<32, 2, 1>(dm, p, tmK, tmQ, st);
 #undef CONVNN_SHORT
