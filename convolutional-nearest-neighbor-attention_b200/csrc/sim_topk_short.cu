@@ -1,30 +1,28 @@
 // Similarity + top-K for short candidate lists (S <= 256): a row's whole similarity vector is one accumulator in tensor
 // memory, so the selection can read it twice.
 //
-//   pass 1  a bound.  Lists of up to twelve: the maxima of 32 groups of columns (sixteen per half of a row, column modulo 16)
-//           are sorted by a network; the nsel-th largest of them is a key that at least nsel columns reach.  One maximum per
-//           column and 63 exchanges per sixteen groups, where a sorted list costs three instructions per slot and pair.
-//   pass 2  the columns whose key reaches the bound (about ten of 197 for K = 9) are appended, in column order, to the row's
-//           entries in shared memory, without a branch on how many there are.
-//   rank    the entries are inserted, in column order, into a sorted list in registers: the earlier column wins ties.
+//   pass 1  a bound: the maxima of 32 groups of columns (lists of up to twelve: sixteen per half of a row, column modulo 16) or 64
+//           (longer lists) are sorted by networks; the nsel-th largest of them is a key that at least nsel columns reach.
+//   pass 2  the columns whose key reaches the bound (of 197 about 10 for K = 9, 29 for K = 25) are appended, in column order, to the
+//           row's entries in shared memory, without a branch on how many there are.
+//   rank    a network sorts the entries (packed_rank.cuh); the earlier column wins ties.
 //           A row with more entries than it has room for takes the columns above the bound chunk by chunk.
 //
-// Longer lists take the exact threshold in pass 1: a sorted list of the best NSEL keys, two columns at a time.  With a >= b the
-// merged list is v'[s] = max(v[s], min(v[s-1], a), min(v[s-2], b)), every slot computed from old values.  The entries of pass 2
-// are then nsel unless keys tie, and all pairs of them are compared once; a row with ties at the threshold or too few keys
-// above -inf (NaN inputs) makes its warp repeat the selection with the ordered insertion of the streaming kernels.
 // The results are the streaming kernels' bit for bit.
 //
-// What bounds it (128 images of 12 heads, 197 x 197 x 32, K = 9, 93 us; the streaming kernel 136): instructions, 4400 per 32 rows
-// at 0.47 per cycle and scheduler, and their fetch: a chunk loop unrolled once more 125 for 106, the metric known at compile
-// time 96 for 106, tensor-memory reads one chunk ahead nothing.  (18 warps of 96 registers: one thread per row spills 12 to 52 bytes.)  us, streaming -> this kernel: 256 images of 197 x 192, K = 9
-// 30.5 -> 20.7 (4: 22.8 -> 16.3), 6 heads of 64 126 -> 84, 65 x 65 x 192 12.5 -> 9.7, 1024 x 65 x 65, 3 heads of 64 94 -> 42,
-// 64 x 1000 x 200 x 256 33 -> 23, 256 x 197 x 64 x 384 17.8 -> 17.2.
+// What bounds it (128 images of 12 heads, 197 x 197 x 32, K = 9, 83 us; with the entries inserted into a sorted list and written a word at
+// a time 93; the streaming kernel 136): instructions, half of them on the half-rate pipe, and their fetch: a chunk loop unrolled once
+// more 125 for 106, the metric known at compile time 96 for 106, tensor-memory reads one chunk ahead nothing.  (18 warps of 96 registers:
+// one thread per row spills 16 to 64 bytes.)  Lists of more than twelve have one thread per row, eight warps, and wait as much as they
+// issue (0.31 instructions per cycle and scheduler); us, a sorted list of values as the bound or the streaming kernel -> groups and a
+// network: 57 x 12 heads of 197 x 197 x 32, K = 25 171 -> 84; 256 x 197 x 197 x 192, K = 25 70 -> 41, K = 16 50 -> 30; 256 x 577 x 150 x 384,
+// K = 16 107 -> 67.  Streaming -> this kernel, K = 9: 256 images of 197 x 192 30.5 -> 20.5 (K = 4: 22.8 -> 16.3), 6 heads of 64 126 -> 84,
+// 65 x 65 x 192 12.5 -> 9.7, 1024 x 65 x 65, 3 heads of 64 94 -> 43, 64 x 1000 x 200 x 256 33 -> 25, 256 x 197 x 64 x 384 17.8 -> 17.6.
 //
 // A persistent CTA per SM: warp 0 TMA producer (128 key rows + all candidate rows of one (batch, head), 64-channel chunks,
 // ring), warp 1 MMA issuer (M = 128, N = S rounded to 16), then selection warps (thread = row).  G accumulators of 512 / G
 // columns, G = 4 for S <= 128 (narrow heads only, lists of up to nine), else 2, so the next units' MMAs run under the selection.  With NH = 2 two warps share a row
-// block of an accumulator, a column half each: the threshold follows from their two sorted lists (the n-th largest of
+// block of an accumulator, a column half each: the bound follows from their two sorted lists (the n-th largest of
 // a and b is the largest min(a[i], b[n-2-i])), their entries grow towards each other, and they take turns at ranking.
 #include "common.cuh"
 #include "sm100.cuh"
@@ -128,13 +126,13 @@ constexpr bool networked = NSEL > 12;
 template <int NSEL, int NH>
 constexpr int slots_of = NSEL <= 12 ? (NH == 2 ? 28 : 32) : NSEL <= 16 ? 32 : NSEL <= 25 ? 48 : 60;
 
-template <int NSEL, int G, int NH, int METRIC>
+template <int NSEL, int G, int NH, int METRIC, Way WAY>
 __global__ void __launch_bounds__(64 + 128 * G * NH, 1)
 sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ, const ShortParams p) {
     constexpr int MAXC = 512 / G;                  // tensor-memory columns of one accumulator
     constexpr int NT = 128 * G * NH;               // selection threads
     constexpr int W = G == 4 ? 16 : 32;            // columns per read of a long list's first pass (18 warps leave 96 registers per thread)
-    constexpr uint32_t ENTRY = 128 * G * 8;        // bytes between a row's successive entries
+    constexpr uint32_t ENTRY = 32 * 8;             // bytes between a row's successive entries
     constexpr int SLOTS = slots_of<NSEL, NH>;
     constexpr bool NETWORK = networked<NSEL>;
     static_assert(!NETWORK || NH == 1, "rows of long lists are one thread's");
@@ -143,7 +141,7 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     const uint32_t pitch = p.KCH * 2;
     const uint32_t a_bytes = BM * pitch, b_bytes = p.BN * pitch, stage_bytes = a_bytes + b_bytes;
     const uint32_t STAGES = p.stages;
-    float2* hits = reinterpret_cast<float2*>(smem + STAGES * stage_bytes);       // [SLOTS][128 * G] (key, column)
+    float2* hits = reinterpret_cast<float2*>(smem + STAGES * stage_bytes);       // [4 G blocks of rows][SLOTS][32] (key, column)
     float* statbuf = reinterpret_cast<float*>(hits + SLOTS * 128 * G);      // [warps][MAXC] column statistics
     int* cs = reinterpret_cast<int*>(statbuf + NT / 32 * MAXC);                  // [MAXC] candidate tokens
     float* lists = reinterpret_cast<float*>(cs + MAXC);                          // short lists: [NSEL][NT] sorted keys
@@ -241,7 +239,8 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         float* qs = statbuf + (warp - 2) * MAXC;
         // entries of a row: the lower half's upwards from slot 0, the upper half's downwards from the last; more than there are
         // slots are marked with a count that no row has room for.
-        const uint32_t hit0 = smem_u32(hits) + (uint32_t)(g * 128 + r) * 8u;
+        float2* own = hits + (g * 4 + lq) * (SLOTS * 32) + lane;
+        const uint32_t hit0 = smem_u32(own), block0 = hit0 - lane * 8u;
         const int c_begin = half ? ((p.S + 1) / 2 + 15) / 16 * 16 : 0;
         const int c_end = NH == 2 && !half ? min(((p.S + 1) / 2 + 15) / 16 * 16, p.S) : p.S;
         const uint32_t taddr = tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)g * MAXC;
@@ -270,7 +269,7 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
             if (!ok) { if (lane == 0) fail(abort_flag, 74); break; }
             tc_fence_after_sync();
             if constexpr (!NETWORK) {
-                bool exact = true;
+                bool insert = false;
                 int n_low = 0, cnt = 0;
                 if (warp_live) {
                     // Pass 1: maxima of column groups, sixteen per half of a row (NH = 1: of the even and the odd chunks).
@@ -310,6 +309,7 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 #pragma unroll
                     for (int i = 0; i < NSEL - 1; ++i)
                         if (i < p.nsel - 1) thr = fmaxf(thr, fminf(v[i], lists[(p.nsel - 2 - i) * NT + peer]));
+                    insert = !(thr > -CUDART_INF_F) || !(fmaxf(v[0], lists[peer]) < CUDART_INF_F);
                     // Pass 2: the columns that reach it.
                     constexpr int ROOM = SLOTS - 8;
                     const uint32_t first = half ? hit0 + (SLOTS - 1) * ENTRY : hit0;
@@ -355,8 +355,8 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
                         ++use_of_pair;
                     }
                     if (!row_ok) cnt = 0;
-                    exact = cnt <= SLOTS;
-                    if (ranks && !__all_sync(0xffffffffu, exact)) {
+                    const bool redo = cnt > SLOTS;
+                    if (ranks && __any_sync(0xffffffffu, redo)) {
                         // More columns reach the bound than a row has room for: chunk by chunk into the list.
                         TopList<NSEL> top;
                         top.init();
@@ -373,40 +373,37 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 #pragma unroll
                             for (int j = 0; j < 16; ++j) {
                                 mask |= key[j] > low ? 1u << j : 0u;
-                                if (!exact) hits[j * 128 * G + g * 128 + r].x = key[j];
+                                if (redo) own[j * 32].x = key[j];
                             }
-                            if (exact) mask = 0;
+                            if (!redo) mask = 0;
                             const int steps = __reduce_max_sync(0xffffffffu, __popc(mask));
                             for (int it = 0; it < steps; ++it) {
                                 const int j = mask ? __ffs(mask) - 1 : 0;
-                                const float kc = hits[j * 128 * G + g * 128 + r].x;
+                                const float kc = own[j * 32].x;
                                 if (mask && kc > top.worst()) top.insert_sorted(kc, c + j);
                                 mask &= mask - 1;
                             }
                         }
-                        if (!exact) write_selection<NSEL>(top, p, ((long long)bh * p.T + row) * p.K, row, kst);
+                        if (redo) {                  // its list is its entries
+#pragma unroll
+                            for (int s = 0; s < NSEL; ++s)
+                                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(hit0 + s * ENTRY),
+                                             "r"(__float_as_uint(top.v[s])), "r"(top.i[s]) : "memory");
+                            n_low = cnt = p.nsel;
+                            insert = true;
+                        }
                     }
                 }
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&tempty[g]);
                 if (ranks && warp_live) {
-                    // The entries, in column order, into the sorted list.
-                    const float2* e = hits + g * 128 + r;
-                    auto entry = [&](int n) { return e[(NH == 1 || n < n_low ? n : SLOTS - 1 + n_low - n) * 128 * G]; };
-                    if (!exact) cnt = 0;
+                    // The n-th entry in column order.
+                    auto entry = [&](int n) { return hit0 + (NH == 1 || n < n_low ? n : SLOTS - 1 + n_low - n) * ENTRY; };
                     TopList<NSEL> top;
-                    top.init();
-                    insert_first<NSEL, 0>(top, entry, cnt);
-                    const int most = __reduce_max_sync(0xffffffffu, cnt);
-#pragma unroll 1
-                    for (int n = NSEL; n < most; ++n) {
-                        if (n < cnt) {
-                            const float2 x = entry(n);
-                            top.insert_sorted(x.x, __float_as_int(x.y));
-                        }
-                    }
-                    if (row_ok && exact) write_selection<NSEL>(top, p, ((long long)bh * p.T + row) * p.K, row, kst);
+                    rank_entries<NSEL>(top, entry, cnt, p.nsel, insert);
+                    write_rows<NSEL, WAY>(top, p, cs, block0, ((long long)bh * p.T + rt * BM + lq * 32) * p.K,
+                                     min(32, p.T - rt * BM - lq * 32), row, kst);
                 }
             } else {
                 uint32_t at = hit0;
@@ -497,13 +494,13 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 #pragma unroll
                             for (int j = 0; j < 16; ++j) {
                                 mask |= key[j] > low ? 1u << j : 0u;
-                                if (redo) hits[j * 128 * G + g * 128 + r].x = key[j];
+                                if (redo) own[j * 32].x = key[j];
                             }
                             if (!redo) mask = 0;
                             const int steps = __reduce_max_sync(0xffffffffu, __popc(mask));
                             for (int it = 0; it < steps; ++it) {
                                 const int j = mask ? __ffs(mask) - 1 : 0;
-                                const float kc = hits[j * 128 * G + g * 128 + r].x;
+                                const float kc = own[j * 32].x;
                                 if (mask && kc > top.worst()) top.insert_sorted(kc, c + j);
                                 mask &= mask - 1;
                             }
@@ -522,9 +519,9 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
                 if (lane == 0) mbar_arrive(&tempty[g]);
                 if (warp_live) {
                     TopList<NSEL> top;
-                    rank_entries<NSEL, SLOTS>(top, hit0, ENTRY, (int)((at - hit0) / ENTRY), p.nsel, redo);
-                    write_rows<NSEL>(top, p, cs, smem_u32(hits) + (uint32_t)(g * 128 + lq * 32) * 8u, ENTRY,
-                                     ((long long)bh * p.T + rt * BM + lq * 32) * p.K, min(32, p.T - rt * BM - lq * 32), row, kst);
+                    rank_entries<NSEL>(top, [&](int n) { return hit0 + n * ENTRY; }, (int)((at - hit0) / ENTRY), p.nsel, redo);
+                    write_rows<NSEL, WAY>(top, p, cs, block0, ((long long)bh * p.T + rt * BM + lq * 32) * p.K,
+                                     min(32, p.T - rt * BM - lq * 32), row, kst);
                 }
             }
         }
@@ -543,7 +540,7 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     }
 }
 
-template <int NSEL, int G, int NH, int METRIC>
+template <int NSEL, int G, int NH, int METRIC, Way WAY>
 int launch_metric(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const CUtensorMap& tmQ, cudaStream_t st) {
     constexpr int MAXC = 512 / G;
     const size_t stage = (size_t)(BM + p.BN) * p.KCH * 2;
@@ -556,25 +553,40 @@ int launch_metric(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const 
     size_t smem = fixed + p.stages * stage;
     if (smem < 116 * 1024) smem = 116 * 1024;                // a CTA takes all of an SM's TMEM: never two on one SM
     const int sms = device_sms();
-    auto kern = sim_topk_short_kernel<NSEL, G, NH, METRIC>;
+    auto kern = sim_topk_short_kernel<NSEL, G, NH, METRIC, WAY>;
     CONVNN_ENSURE_SMEM(kern, smem);
     launch_chained(kern, p.n_units < sms ? p.n_units : sms, 64 + NT, smem, st, tmK, tmQ, p);
     CONVNN_CHECK_LAUNCH("sim_topk_short");
     return CONVNN_OK;
 }
 
+template <int NSEL, int G, int NH, Way WAY>
+int launch_way(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const CUtensorMap& tmQ, cudaStream_t st) {
+    if (p.metric == CONVNN_COSINE) return launch_metric<NSEL, G, NH, CONVNN_COSINE, WAY>(dm, p, tmK, tmQ, st);
+    if (p.metric == CONVNN_MATMUL) return launch_metric<NSEL, G, NH, CONVNN_MATMUL, WAY>(dm, p, tmK, tmQ, st);
+    return launch_metric<NSEL, G, NH, CONVNN_EUCLIDEAN, WAY>(dm, p, tmK, tmQ, st);
+}
+
+// Short lists a word at a time cost a sector per word, by lines a pass through shared memory and code that few rows do not repay:
+// K = 9, 128 x 12 x 197 x 197 x 32 91.5 -> 82.8 us, 64 x 1000 x 200 x 256 27.3 -> 24.8, 1024 x 3 x 65 x 65 x 64 46.7 -> 43.6; but 256 x 197 x
+// 197 x 192 20.2 -> 20.4, 256 x 65 x 65 x 192 9.8 -> 10.3, K = 5, 700 x 197 x 197 x 32 35.4 -> 37.3.  Long ones, skewed: K = 25, 64 x 3 x 197 x 197 x 64 33.5 -> 29.4; 57 x 12 x 197 x
+// 197 x 32 84 (by lines 85 to 87); K = 16, 256 x 577 x 150 x 384 75.7 -> 67.
 template <int NSEL, int G, int NH>
 int launch_short(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const CUtensorMap& tmQ, cudaStream_t st) {
-    if (p.metric == CONVNN_COSINE) return launch_metric<NSEL, G, NH, CONVNN_COSINE>(dm, p, tmK, tmQ, st);
-    if (p.metric == CONVNN_MATMUL) return launch_metric<NSEL, G, NH, CONVNN_MATMUL>(dm, p, tmK, tmQ, st);
-    return launch_metric<NSEL, G, NH, CONVNN_EUCLIDEAN>(dm, p, tmK, tmQ, st);
+    if constexpr (networked<NSEL>) {
+        return launch_way<NSEL, G, NH, SKEWED>(dm, p, tmK, tmQ, st);
+    } else {
+        if constexpr (NSEL == 8 || NSEL == 9)
+            if (dm.K % 2 == 1 && dm.K >= 9 && (long long)dm.B * dm.H * dm.T >= 384ll * device_sms())
+                return launch_way<NSEL, G, NH, LINES>(dm, p, tmK, tmQ, st);
+        return launch_way<NSEL, G, NH, WORDS>(dm, p, tmK, tmQ, st);
+    }
 }
 
 }  // namespace
 
-// What the warp-per-row kernel leaves to it.  Anything of up to one unit per SM (48 x 197 x 197 x 192, K = 25 33.8, 23.0); lists of 13 to
-// 16, whose streaming variant runs one CTA per SM (256 x 577 x 150 x 384, K = 16 129, 110; 256 x 197 x 197 x 192 47, 49); lists of up to
-// twelve except where the streaming kernel's 256-row units are fewer and the bound saves little (us, streaming, this kernel):
+// What the warp-per-row kernel leaves to it.  Anything of up to one unit per SM (48 x 197 x 197 x 192, K = 25 33.8, 23.0); lists of more
+// than twelve (streaming 256 x 577 x 150 x 384, K = 16 129, here 67; 57 x 12 x 197 x 197 x 32, K = 25 171, 84); lists of up to twelve except where the streaming kernel's 256-row units are fewer and the bound saves little (us, streaming, this kernel):
 //   * few candidates: of sequences that fill more than one unit here (512 x 197 x 16 x 192, K = 4 10.8, 14.4; 256 x 197 x 32 x 768, K = 3
 //     19.6, 21.9), and of others where heads are wide, lists long or the second round of units thin (1000 x 17 x 17 x 512, K = 2 19.5, 23.6;
 //     200 x 100 x 20 x 384, K = 5 8.6, 9.6; 163 x 65 x 65 x 128, K = 12 13.4, 14.6; but 1000 x 17 x 17 x 64 0.65 of the time, 340 x 25 x 25 x 192 0.85, and
