@@ -18,18 +18,13 @@ __device__ __forceinline__ void prefix_insert(TopList<NSEL>& top, const float (&
     }
 }
 
-// One chunk of W accumulator columns of this thread's row: keys, then either plain inserts
-// (the first 32 columns of a row, where most values enter the list anyway) or a threshold
-// mask followed by a drain loop that only visits the survivors.
+// Ranking keys of W accumulator columns of this thread's row.
 // qs points at the W column statistics of this chunk in shared memory (16-byte aligned, the same
 // for every lane: broadcast loads); cv holds the candidate token of column (32-aligned base +
-// lane).  P needs the fields metric, sampled and S (number of candidate columns).
-// FLOOR: keys at or below `floor` are known to lie outside the row's final list.
-template <int NSEL, int W, bool FLOOR = false, class P>
-__device__ __forceinline__ void consume(TopList<NSEL>& top, const uint32_t (&acc)[W], int col0, int lane_off,
-                                        const float* qs, int cv, const P& p, int row, bool row_ok, float sentinel,
-                                        float* ks, float floor = 0.f) {
-    float key[W];
+// lane).  P needs the fields metric and sampled.
+template <int W, class P>
+__device__ __forceinline__ void keys_of(float (&key)[W], const uint32_t (&acc)[W], int lane_off, const float* qs, int cv, const P& p,
+                                        int row, float sentinel) {
     if (p.metric != CONVNN_MATMUL) {
         const f32x2 two = pack2(2.0f, 2.0f);
 #pragma unroll
@@ -52,13 +47,29 @@ __device__ __forceinline__ void consume(TopList<NSEL>& top, const uint32_t (&acc
 #pragma unroll
         for (int j = 0; j < W; ++j) key[j] = __uint_as_float(acc[j]);
     }
-    if (p.sampled) {
+    // (the warp's rows follow one another: most chunks hold none of them)
+    if (p.sampled && __any_sync(0xffffffffu, (uint32_t)(cv - (row - (int)(threadIdx.x & 31))) < 32u)) {
 #pragma unroll
         for (int j = 0; j < W; ++j) {
             const int cj = __shfl_sync(0xffffffffu, cv, lane_off + j);
             if (cj == row) key[j] = sentinel;
         }
     }
+}
+
+// One chunk of W accumulator columns of this thread's row: keys, then either plain inserts
+// (the first 32 columns of a row, where most values enter the list anyway) or a threshold
+// mask followed by a drain loop that only visits the survivors.
+// qs points at the W column statistics of this chunk in shared memory (16-byte aligned, the same
+// for every lane: broadcast loads); cv holds the candidate token of column (32-aligned base +
+// lane).  P needs the fields metric, sampled and S (number of candidate columns).
+// FLOOR: keys at or below `floor` are known to lie outside the row's final list.
+template <int NSEL, int W, bool FLOOR = false, class P>
+__device__ __forceinline__ void consume(TopList<NSEL>& top, const uint32_t (&acc)[W], int col0, int lane_off,
+                                        const float* qs, int cv, const P& p, int row, bool row_ok, float sentinel,
+                                        float* ks, float floor = 0.f) {
+    float key[W];
+    keys_of<W>(key, acc, lane_off, qs, cv, p, row, sentinel);
     const int left = p.S - col0;                       // valid columns from col0 on
     if (col0 < 32) {
         if (col0 == 0) {                               // the list is still filling up
