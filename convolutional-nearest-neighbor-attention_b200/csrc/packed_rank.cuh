@@ -2,8 +2,8 @@
 //
 // A sorted list takes five instructions per slot and insertion, all on the half-rate pipe.  Here the low bits of a key are
 // replaced by the number of its entry, so that a sorting network moves one word per entry, two instructions per exchange.
-// Keys that agree in the bits that are left are put in order afterwards, by what the entries hold; where such keys meet at the
-// end of the list, the entries are inserted one by one.  The order is the ordered insertion's: larger key first, then lower column.
+// Keys that agree in the bits that are left are put in order afterwards, by what the entries hold; where more than two such keys
+// meet at the end of the list, the entries are inserted one by one.  The order is the ordered insertion's: larger key first, then lower column.
 #pragma once
 #include <math_constants.h>
 
@@ -55,7 +55,7 @@ __device__ __forceinline__ void insert_entries(TopList<NSEL>& top, const At& at,
 // What the network takes; more entries than that are inserted.  (Ten to twelve: all of them, 256 x 6 heads of 197 x 197 x 64, K = 12
 // 111.6 us, 113.8 with a network of 24.)
 template <int NSEL>
-constexpr int network_of = NSEL <= 4 ? 8 : NSEL <= 8 ? 12 : NSEL <= 9 ? 16 : NSEL <= 12 ? 0 : NSEL <= 16 ? 24 : NSEL <= 25 ? 40 : 52;
+constexpr int network_of = NSEL <= 4 ? 8 : NSEL <= 8 ? 12 : NSEL <= 9 ? 16 : NSEL <= 12 ? 0 : NSEL <= 16 ? 28 : NSEL <= 25 ? 44 : 52;
 
 // The best nsel <= NSEL of `cnt` <= 64 entries, entry n at the address at(n); all lanes of a warp call it.  Rows whose keys are
 // not all finite ask for the insertion (`insert`), which leaves out -inf.
@@ -92,14 +92,15 @@ __device__ __forceinline__ void rank_entries(TopList<NSEL>& top, const At& at, i
         for (int i = 0; i < NSEL; ++i) {
             const bool c = close(i) && i < nsel && i + 1 < cnt;
             near_any |= c;
-            insert |= c && (NSEL <= 12 || i == nsel - 1);
+            // (the last place and the first beyond change places like any two, unless a third is as close)
+            insert |= c && (NSEL <= 12 || (i == nsel - 1 && close(i + 1) && i + 2 < cnt));
         }
         near_any = near_any && !insert;
         while (NSEL > 12 && __any_sync(0xffffffffu, near_any)) {
             bool moved = false;
 #pragma unroll
-            for (int i = 0; i + 1 < NSEL; ++i) {
-                if (near_any && i + 1 < nsel && close(i)) {
+            for (int i = 0; i < NSEL; ++i) {
+                if (near_any && i < nsel && i + 1 < cnt && close(i)) {
                     const uint32_t a = __float_as_uint(q[i]) & LOW, b = __float_as_uint(q[i + 1]) & LOW;
                     const float ka = lds_key(at((int)a)), kb = lds_key(at((int)b));
                     if (kb > ka || (kb == ka && b < a)) {

@@ -124,7 +124,7 @@ __device__ __forceinline__ void insert_first(TopList<NSEL>& top, const E& entry,
 template <int NSEL>
 constexpr bool networked = NSEL > 12;
 template <int NSEL, int NH>
-constexpr int slots_of = NSEL <= 12 ? (NH == 2 ? 28 : 32) : NSEL <= 16 ? 32 : NSEL <= 25 ? 48 : 60;
+constexpr int slots_of = NSEL <= 12 ? (NH == 2 ? 28 : 32) : NSEL <= 16 ? 36 : NSEL <= 25 ? 52 : 60;
 
 template <int NSEL, int G, int NH, int METRIC, Way WAY>
 __global__ void __launch_bounds__(64 + 128 * G * NH, 1)

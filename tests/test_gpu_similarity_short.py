@@ -269,3 +269,43 @@ def test_exact_lists_of_the_other_metrics(B, T, S, H, dk, K, values, metric):
     real = want_key > -math.inf
     # one product, or a difference of whole numbers and its root: equal up to the root's rounding
     assert bool(((val[..., K - n:] - want).abs() <= 2.0 ** -22 * want.abs())[real].all())
+
+
+# Lists of more than twelve, ranked by one thread per row, with several units per SM, and short ones written by lines (K = 9, 384 rows
+# per SM, ragged ends).  "close" keys agree in all but their last bits, so that neighbours in the list and at its end are told
+# apart by what the entries hold; "few" values tie and overflow the entries; "stripes" puts the best columns into few groups of maxima.
+@on_148_sms
+@pytest.mark.parametrize("B,T,S,H,dk", [(160, 40, 40, 1, 64), (100, 197, 64, 1, 384), (160, 128, 128, 1, 192), (60, 129, 48, 3, 16),
+                                        (80, 197, 197, 3, 32), (60, 300, 208, 1, 512), (160, 256, 256, 1, 64), (325, 197, 197, 1, 32)])
+@pytest.mark.parametrize("K", [9, 13, 16, 17, 25, 32])
+@pytest.mark.parametrize("values", ["few", "many", "nan", "stripes", "close", "inf"])
+def test_ranked_entries(B, T, S, H, dk, K, values):
+    sampled = S != T
+    n = K - 1 if sampled else K
+    g = torch.Generator(device=DEV).manual_seed(T * 1000 + S + K)
+    top = 1 if values == "few" else 11               # products and sums stay below 2^24
+    q, k = (torch.randint(-top, top + 1, (B, r, H, dk), device=DEV, generator=g).float() for r in (S, T))
+    if values == "nan":
+        q[:, ::3] = math.nan
+        q[1, 2:] = math.nan
+    if values == "stripes":
+        q[:, ::16] = q[:, ::16].abs() + 12
+        k = k.abs()
+    if values == "close":
+        q[..., 0], k[..., 0] = 2048.0, 2048.0
+    if values == "inf":
+        q[:, 5], k[..., 0] = 1.0, 3.0
+        q[:, 5, :, 0] = math.inf
+    spec = ops.LayerSpec(H * dk, H, K, "spatial" if sampled else "all", "matmul", "depthwise", True, False, T)
+    cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if sampled else None
+    idx, val = ops.sim_topk(spec, q.bfloat16(), k.bfloat16(), None, None, cand)
+    key = torch.einsum("bthc,bshc->bhts", k.double(), q.double()).float()
+    if sampled:
+        own = cand.view(1, 1, 1, S).long() == torch.arange(T, device=DEV).view(1, 1, T, 1)
+        key = torch.where(own, torch.full_like(key, -0.1) * torch.tensor(math.sqrt(dk), dtype=torch.float32, device=DEV), key)
+    want_idx, want_key = expect(key, n)
+    assert torch.equal(idx.long()[..., K - n:], want_idx if cand is None else cand.long()[want_idx])
+    real = (want_key.abs() < math.inf) & ~((want_key < 0) & (val[..., K - n:] == -0.1))
+    want_val = want_key / torch.tensor(math.sqrt(dk), dtype=torch.float32, device=DEV)
+    # one division: equal up to its rounding
+    assert bool(((val[..., K - n:] - want_val).abs() <= 2.0 ** -22 * want_val.abs())[real].all())
