@@ -393,11 +393,13 @@ template <int J>
 int launch_rows_j(RowsParams& p, size_t smem, int grid, const CUtensorMap& tmK, const CUtensorMap& tmQ, cudaStream_t st) {
     if (p.o) {
         if (p.nsel == 9) return launch_rows<J, 9, true>(p, smem, grid, tmK, tmQ, st);
-        return launch_rows<J, 0, true>(p, smem, grid, tmK, tmQ, st);
+        if (p.nsel <= 12) return launch_rows<J, 0, true>(p, smem, grid, tmK, tmQ, st);
+        return launch_rows<J, -3, true>(p, smem, grid, tmK, tmQ, st);
     }
     if (p.nsel == 8) return launch_rows<J, 8, false>(p, smem, grid, tmK, tmQ, st);
     if (p.nsel == 9) return launch_rows<J, 9, false>(p, smem, grid, tmK, tmQ, st);
-    if (p.nsel <= 16) return launch_rows<J, 0, false>(p, smem, grid, tmK, tmQ, st);
+    if (p.nsel <= 12) return launch_rows<J, 0, false>(p, smem, grid, tmK, tmQ, st);
+    if (p.nsel <= 16) return launch_rows<J, -3, false>(p, smem, grid, tmK, tmQ, st);
     if (p.nsel <= 25) return launch_rows<J, -1, false>(p, smem, grid, tmK, tmQ, st);
     return launch_rows<J, -2, false>(p, smem, grid, tmK, tmQ, st);
 }
@@ -434,12 +436,14 @@ static Ranges ranges_of(const Dims& dm) {
 //   197 x 197, K = 9         1 image 14.9 -> 6.5    37: 15.2 -> 8.8    148: 21.9 -> 17.1    220: 30.4 -> 26.2    256: 30.4 -> 30.2 (not taken)
 //   12 heads of 64           1 image 14.8 -> 6.6    16: 27.5 -> 22.3    32: 40.4 -> 37.8 (not taken)
 //   197 x 64 x 384, K = 9    1 image 9.2 -> 6.5     16: 9.5 -> 7.1      74: 9.8 -> 12.2 (not taken)
-//   197 x 197, K = 25        1 image 23.5 -> 8.2    16: 24.1 -> 21.0    48: 24.4 -> 28.3 (not taken)
 //   (two batches in flight lose 0.6 % with it at 256 images: a CTA of this kernel fills its SM)
 //   1000 x 256 x 768, K = 5  1 image 18.0 -> 9.9    4: 18.2 -> 11.1     16: 18.9 -> 21.5 (not taken)
-// These figures and the lines below are against the streaming kernel and the two-pass kernel's sorted lists.  Since the two-pass
-// kernel bounds lists of up to twelve by group maxima it is ahead from about 64 rows per SM on with 197 candidates (K = 9, 48
-// images 9.8 us there, 9.7 here; 72: 9.9, 11.3; 132: 12.7, 18.7; 220: 20, 28): the lines for such lists have yet to be drawn again.
+// These figures are against the two-pass kernel's sorted lists of values.  Since that bounds its rows by group maxima, and this kernel
+// bounds lists of more than twelve by two maxima per lane (two-pass, this kernel, us):
+//   197 x 197, one head of 96, K = 9   20 images 9.3, 7.1   38: 9.4, 9.2   64: 9.7, 10.6   150: 17.6, 21.0;  3 heads of 32   64: 17.4, 22.1
+//   K = 5   20: 8.4, 7.0   38: 8.6, 8.8   64: 8.8, 10.2        K = 16   20: 12.7, 8.1   38: 13.3, 12.0   64 x 3 heads of 64: 23.5, 36.6
+//   197 x 197 x 192, K = 25   1 image 16.8, 8.2   20: 16.8, 10.0   34: 17.8, 13.9      65 x 65 x 192   80: 13.0, 13.5   100: 14.2, 13.5
+// The line of lists of five to twelve with one head of 129 to 192 channels has not been drawn again (132 images 12.3, 18.8).
 // Where others win, and the lines of the rule (R rows per SM, rounds u of 256-row units per SM, w the share of their warps that
 // has rows: two units of the streaming kernel share an SM and slow each other down by about w / 2):
 //   * up to 128 candidates, and heads above 384 channels, only ranges that stay inside a head: a range across heads is cut into
@@ -447,17 +451,16 @@ static Ranges ranges_of(const Dims& dm) {
 //   * lists of up to four are cheap elsewhere (256 x 130 x 130 x 16, K = 3 12.9 -> 17.3; 192 x 197 x 197 x 192, K = 3 1.08 times)
 //   * up to 175 candidates the streaming kernel's 64-column tiles fit better (236 x 130 x 130 x 16, K = 5 1.08 times)
 //   * many wide candidates are fetched again for every segment (30 x 1000 x 250 x 384, K = 9 1.13 times; 120 x 256 x 256 x 384 0.91)
-//   * sixteen: in most batches a row or two overflow the survivors' buffer, which adds 6 us (64 x 197 x 197 x 192 14.4 without, 19.5 to
-//     20.7 with, two-pass 19.7; room for 64 costs every batch 5 to 8 %); the two-pass kernel's own slow path, a tie at its threshold, costs
-//     15 us (74 x 224 x 224 x 16 20 or 35).  More candidates or longer sequences lose more (37 x 1000 x 250 x 192 33.7 -> 36.9)
 bool sim_topk_rows_wanted(const Dims& dm) {
     if (dm.S > 256) return false;
     const int R = rows_per_sm(dm);
-    if (dm.nsel > 16) return R <= 32;
+    if (dm.nsel > 16) return R <= 48;
     if (dm.S <= 128 || dm.Cp > 384) return R <= 48 && ranges_of(dm).per_head;
-    if (dm.nsel == 16) return R <= (dm.S <= 208 && dm.T <= 256 ? 304 : 64);
-    if (dm.Cp > 192 && dm.S > 208 && (dm.T > 256 || dm.nsel > 12)) return R <= 96;
-    if (dm.nsel > 12 || (dm.nsel > 4 && dm.S >= 176)) return R <= 304;
+    const bool other_width = dm.Cp <= 128 || dm.Cp > 192;
+    if (dm.nsel > 12) return R <= (other_width || dm.S < 176 ? 64 : 96);
+    if (dm.Cp > 192 && dm.S > 208 && dm.T > 256) return R <= 96;
+    if (dm.nsel >= 4 && dm.S >= 176 && other_width && (dm.Cp <= 128 || dm.S <= 208)) return R <= (dm.S > 208 ? 80 : 64);
+    if (dm.nsel > 4 && dm.S >= 176) return R <= 304;
     const int units_of = (dm.T + 255) / 256;
     const double u = (double)dm.B * dm.H * units_of / device_sms(), w = (double)((dm.T + 31) / 32) / (8 * units_of);
     if (dm.nsel <= 4) return R <= (dm.S < 144 ? 110 : dm.S < 176 ? 150 : 165) * (u <= 1 ? 1 : u <= 2 ? 1 + 0.4 * w : 2);

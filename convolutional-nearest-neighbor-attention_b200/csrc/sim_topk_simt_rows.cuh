@@ -195,7 +195,8 @@ template <typename T, int J>
 int launch_ns(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat, const float* kstat,
               const int32_t* cand, int32_t* idx, float* val, cudaStream_t st) {
     if (dm.nsel == 9) return launch<T, J, 9>(d, dm, q, k, qstat, kstat, cand, idx, val, st);
-    if (dm.nsel <= 16) return launch<T, J, 0>(d, dm, q, k, qstat, kstat, cand, idx, val, st);
+    if (dm.nsel <= 12) return launch<T, J, 0>(d, dm, q, k, qstat, kstat, cand, idx, val, st);
+    if (dm.nsel <= 16) return launch<T, J, -3>(d, dm, q, k, qstat, kstat, cand, idx, val, st);
     return launch<T, J, -2>(d, dm, q, k, qstat, kstat, cand, idx, val, st);
 }
 

@@ -34,7 +34,7 @@ struct RowsTask {
 // e / K = e * inverse_of(K) >> 16 for e < 16 K, K <= 32
 __host__ __device__ constexpr int inverse_of(int K) { return (65536 + K - 1) / K; }
 // survivors of a warp: R rows of 32 (64: lists of more than 16) pairs
-__host__ __device__ constexpr int found_pairs(int NS) { return R * (NS < 0 ? 64 : 32); }
+__host__ __device__ constexpr int found_pairs(int NS) { return R * (NS == -1 || NS == -2 ? 64 : 32); }
 
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float r;
@@ -234,11 +234,14 @@ __device__ __forceinline__ uint32_t select_rows(const RowsTask& p, const float* 
 
 // The rows w, w + NW, ... below n_rows of a key buffer (tokens row0 + r of their sequence): lists through `list` (room for K
 // pairs per row of the warp), then sink(row of the warp, slot, token, value) for every entry.  Returns the rows of the warp.
-// NS: number of neighbours where it is fixed, 0: any up to 16, -1: up to 25, -2: up to 32.
+// NS: number of neighbours where it is fixed, 0: any up to 12, -3: 13 to 16, -1: up to 25, -2: up to 32.  From 13 on (up to 16: of more
+// than 128 keys) two maxima per lane give the bound: of 197 keys 48 reach the 25th of 32 maxima, so that a row in two hundred overflowed the buffer and the
+// batch waited for its ordered list, but 29 reach the 25th of 64 (us, one maximum, two: 3 x 197 x 197 x 32, K = 25 18.0, 8.2; 20 x 197 x
+// 197 x 96 20.9, 10.8; 64 x 197 x 197 x 192, K = 16 20.5, 15.6).
 template <int J, int NS, int NW, class Sink>
 __device__ __forceinline__ int select_lists(const RowsTask& p, const float* keybuf, float2* list, uint32_t found0, int w,
                                             int n_rows, int row0, Sink sink) {
-    constexpr int E = NS < 0 ? 2 : 1, GR = NS == -2 && J > 1 ? 2 : 1;
+    constexpr int E = NS == -1 || NS == -2 ? 2 : 1, GR = NS < 0 && J > (NS == -3 ? 4 : 1) ? 2 : 1;
     const int lane = threadIdx.x & 31;
     const uint32_t list0 = static_cast<uint32_t>(__cvta_generic_to_shared(list + p.sampled)), list_stride = p.K * 8;
     uint32_t redo = 0;                       // bit n: row w + n NW
