@@ -18,8 +18,7 @@
 // CTAs fit on an SM at ViT shapes and cover each other's serial phases.
 // Every mbarrier wait is bounded; on expiry the CTA latches a code and drains.
 //
-// Anything else (float32, longer sequences, other head widths) takes a plain SIMT kernel, one warp
-// per query row.
+// Anything else (float32, longer sequences, other head widths) is computed on the fp32 pipes, a tile of rows per CTA.
 #include <math_constants.h>
 
 #include "common.cuh"
@@ -319,8 +318,223 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     chain_leave(BESIDE);
 }
 
-// One warp per query row; scores in shared memory.  float32 (and the fallback for shapes the
-// tensor-core kernel does not take).
+// R query rows of one (batch, head) per CTA, for float32 and head widths that the tensor-core kernel does not take.
+//
+//   scores   a thread owns R / 8 rows x 4 keys; K passes through shared memory in chunks of 32 channels x 128 keys, the next chunk in
+//            registers meanwhile
+//   softmax  a warp per row
+//   output   a thread owns R / 8 rows x 4 channels; V passes in chunks of 32 tokens x 128 channels
+//
+// Every sum runs in the order of the kernel for longer sequences below (channels, tokens and the lanes' partial sums ascending), so
+// that both give the same bits.  What bounds it: shared-memory reads, two 16-byte ones per 16 multiply-adds, and at few rows the chain of
+// chunks.  us with the four projections, one warp per row reading K a word at a time -> this kernel: 6 x 65 x 192, one head, bfloat16 98 ->
+// 30; 64 x 197 x 192 2090 -> 170; 8 x 197 x 384 806 -> 91; float32, 8 x 197, 3 heads of 32 171 -> 52; 16 x 197, 12 heads of 32 1113 -> 290.
+constexpr int AT_KEYS = 128, AT_CH = 32, AT_THREADS = 256;
+
+// The chunk of 32 x 128 values that a thread holds 16 of: values 8 i .. 8 i + 7 of row `line(i)`, i = 0, 1, zeros past the ends.
+template <typename T>
+__device__ __forceinline__ void load_eight(float (&x)[8], const T* row, int first, int n, bool vec) {
+    if (vec && first + 8 <= n) {
+        if constexpr (sizeof(T) == 2) {
+            const uint4 u = *reinterpret_cast<const uint4*>(row + first);
+            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                x[2 * e] = __uint_as_float(w[e] << 16);
+                x[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+            }
+        } else {
+            const float4 u = *reinterpret_cast<const float4*>(row + first), v = *reinterpret_cast<const float4*>(row + first + 4);
+            x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
+            x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = first + e < n ? to_f32(row[first + e]) : 0.f;
+    }
+}
+
+// acc[r][e] += a[r][i] * tile[i][e] for i = 0 .. n - 1, in that order.
+template <int TR>
+__device__ __forceinline__ void times_tile(float (&acc)[TR][4], const float* a, int pitch, const float* tile, int n) {
+    auto step = [&](int r, float x, const float4& t) {
+        acc[r][0] = fmaf(x, t.x, acc[r][0]);
+        acc[r][1] = fmaf(x, t.y, acc[r][1]);
+        acc[r][2] = fmaf(x, t.z, acc[r][2]);
+        acc[r][3] = fmaf(x, t.w, acc[r][3]);
+    };
+    int i = 0;
+#pragma unroll 2
+    for (; i + 4 <= n; i += 4) {
+        float4 x[TR], t[4];
+#pragma unroll
+        for (int r = 0; r < TR; ++r) x[r] = *reinterpret_cast<const float4*>(a + r * pitch + i);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) t[u] = *reinterpret_cast<const float4*>(tile + (i + u) * AT_KEYS);
+#pragma unroll
+        for (int r = 0; r < TR; ++r) {
+            step(r, x[r].x, t[0]);
+            step(r, x[r].y, t[1]);
+            step(r, x[r].z, t[2]);
+            step(r, x[r].w, t[3]);
+        }
+    }
+    for (; i < n; ++i) {
+        const float4 t = *reinterpret_cast<const float4*>(tile + i * AT_KEYS);
+#pragma unroll
+        for (int r = 0; r < TR; ++r) step(r, a[r * pitch + i], t);
+    }
+}
+
+template <typename T, int R>
+__global__ void __launch_bounds__(AT_THREADS)
+attention_tile_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o, int Tn, int H, int dk,
+                      float scale, int vec) {
+    constexpr int TR = R / 8;
+    chain_begin_for<T>();
+    extern __shared__ float sm[];
+    const int pitch = (Tn + 3) / 4 * 4 + 4;              // of a row of scores
+    const int qpitch = (dk + 3) / 4 * 4;
+    float* qs = sm;                                      // [R][qpitch]
+    float* prob = qs + R * qpitch;                       // [R][pitch]
+    float* tile = prob + R * pitch;                      // [32][128], scores: channel, key; output: token, channel
+    float* inv = tile + AT_CH * AT_KEYS;                 // [R]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int bh = blockIdx.y, b = bh / H, h = bh - b * H, row0 = blockIdx.x * R;
+    const long long D = (long long)H * dk, base = (long long)b * Tn * D + h * dk;
+    const int n_rows = min(R, Tn - row0);
+    const int rg = warp * TR;                            // first row of this warp (its lanes read their values as broadcasts)
+#pragma unroll
+    for (int r = 0; r < TR; ++r)
+#pragma unroll 4
+        for (int c = lane; c < dk; c += 32)
+            qs[(rg + r) * qpitch + c] = rg + r < n_rows ? to_f32(q[base + (row0 + rg + r) * D + c]) * scale : 0.f;
+    // ---- scores ----
+    const T* kb = k + base;
+    const int n_ch = (dk + AT_CH - 1) / AT_CH, n_kt = (Tn + AT_KEYS - 1) / AT_KEYS;
+    // this thread's part of a chunk: key tid % 128, channels 16 (tid / 128) .. + 15
+    const int lk = tid & 127, lc = (tid >> 7) * 16;
+    float next[16];
+    auto fetch_k = [&](int step) {
+        const int kt = step / n_ch, key = kt * AT_KEYS + lk, c = (step - kt * n_ch) * AT_CH + lc;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            float x[8];
+            load_eight<T>(x, kb + (long long)min(key, Tn - 1) * D, min(c + 8 * i, dk), dk, vec);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) next[8 * i + e] = x[e];
+        }
+    };
+    fetch_k(0);
+    float acc[TR][4];
+    for (int step = 0; step < n_kt * n_ch; ++step) {
+        const int kt = step / n_ch, ch = step - kt * n_ch;
+        __syncthreads();                                 // the chunk before has been read
+#pragma unroll
+        for (int e = 0; e < 16; ++e) tile[(lc + e) * AT_KEYS + lk] = next[e];
+        __syncthreads();
+        if (step + 1 < n_kt * n_ch) fetch_k(step + 1);
+        if (ch == 0) {
+#pragma unroll
+            for (int r = 0; r < TR; ++r)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[r][e] = 0.f;
+        }
+        if (kt * AT_KEYS + 4 * lane < Tn) {
+            const int nc = min(AT_CH, dk - ch * AT_CH);
+            times_tile<TR>(acc, qs + rg * qpitch + ch * AT_CH, qpitch, tile + 4 * lane, nc);
+            if (ch == n_ch - 1) {
+#pragma unroll
+                for (int r = 0; r < TR; ++r)
+                    *reinterpret_cast<float4*>(prob + (rg + r) * pitch + kt * AT_KEYS + 4 * lane) =
+                        make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+            }
+        }
+    }
+    // ---- softmax: the rows of this warp, whose scores it has written itself ----
+    const T* vb = v + base;
+    const int n_vt = (dk + AT_KEYS - 1) / AT_KEYS, n_jt = (Tn + AT_CH - 1) / AT_CH;
+    // this thread's part of a chunk: token tid / 8, channels 16 (tid % 8) .. + 15
+    const int lj = tid >> 3, lv = (tid & 7) * 16;
+    auto fetch_v = [&](int step) {
+        const int vt = step / n_jt, j = (step - vt * n_jt) * AT_CH + lj, c = vt * AT_KEYS + lv;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            float x[8];
+            load_eight<T>(x, vb + (long long)min(j, Tn - 1) * D, min(c + 8 * i, dk), dk, vec);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) next[8 * i + e] = x[e];
+        }
+    };
+    fetch_v(0);
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < TR; ++r) {
+        float* pr = prob + (rg + r) * pitch;
+        float m = -3.402823466e38f;
+        for (int j = lane; j < Tn; j += 32) m = fmaxf(m, pr[j]);
+        for (int off = 16; off; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+        float sum = 0.f;
+        for (int j = lane; j < Tn; j += 32) {
+            const float e = expf(pr[j] - m);
+            pr[j] = e;
+            sum += e;
+        }
+        for (int off = 16; off; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        if (lane == 0) inv[rg + r] = 1.0f / sum;
+    }
+    // ---- output ----
+    for (int step = 0; step < n_vt * n_jt; ++step) {
+        const int vt = step / n_jt, jt = step - vt * n_jt, c0 = vt * AT_KEYS + 4 * lane;
+        __syncthreads();
+#pragma unroll
+        for (int e4 = 0; e4 < 4; ++e4)
+            *reinterpret_cast<float4*>(tile + lj * AT_KEYS + lv + 4 * e4) =
+                make_float4(next[4 * e4], next[4 * e4 + 1], next[4 * e4 + 2], next[4 * e4 + 3]);
+        __syncthreads();
+        if (step + 1 < n_vt * n_jt) fetch_v(step + 1);
+        if (jt == 0) {
+#pragma unroll
+            for (int r = 0; r < TR; ++r)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[r][e] = 0.f;
+        }
+        if (c0 < dk) {
+            const int nj = min(AT_CH, Tn - jt * AT_CH);
+            times_tile<TR>(acc, prob + rg * pitch + jt * AT_CH, pitch, tile + 4 * lane, nj);
+            if (jt == n_jt - 1) {
+#pragma unroll
+                for (int r = 0; r < TR; ++r) {
+                    if (rg + r < n_rows) {
+                        T* to = o + base + (row0 + rg + r) * D + c0;
+                        const float s = inv[rg + r];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (c0 + e < dk) to[e] = from_f32<T>(acc[r][e] * s);
+                    }
+                }
+            }
+        }
+    }
+}
+
+size_t tile_smem(int Tn, int dk, int R) {
+    return ((size_t)R * ((dk + 3) / 4 * 4) + (size_t)R * ((Tn + 3) / 4 * 4 + 4) + AT_CH * AT_KEYS + R) * sizeof(float);
+}
+
+template <typename T, int R>
+int launch_tile(const void* q, const void* k, const void* v, void* o, int B, int Tn, int H, int dk, float scale, cudaStream_t st) {
+    const size_t smem = tile_smem(Tn, dk, R);
+    auto kern = attention_tile_kernel<T, R>;
+    CONVNN_ENSURE_SMEM(kern, smem);
+    const int vec = dk % 8 == 0 && aligned16(k) && aligned16(v);         // (rows of a multiple of eight values)
+    launch_chained(kern, dim3((Tn + R - 1) / R, B * H), AT_THREADS, smem, st, static_cast<const T*>(q), static_cast<const T*>(k),
+                   static_cast<const T*>(v), static_cast<T*>(o), Tn, H, dk, scale, vec);
+    CONVNN_CHECK_LAUNCH("attention_tile");
+    return CONVNN_OK;
+}
+
+// One warp per query row; scores in shared memory.  Sequences too long for a tile of rows.
 template <typename T>
 __global__ void attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                                       T* __restrict__ o, int Tn, int H, int dk, float scale) {
@@ -426,6 +640,16 @@ template <typename T>
 int launch_attention_simt_t(const void* q, const void* k, const void* v, void* o, int B, int Tn, int D, int H,
                             cudaStream_t st) {
     const int dk = D / H, nw = 4;
+    const float scale = (float)(1.0 / sqrt((double)dk));
+    // Fewer rows per CTA where more leave SMs without one (all read every chunk, so that they are fewer multiply-adds per read: 6 x 65 x 192
+    // 22 us with 16 rows, 19 with 8; 6 x 197 x 192 46, 57).
+    auto ctas = [&](int R) { return (long long)B * H * ((Tn + R - 1) / R); };
+    const int R = 3 * ctas(16) < device_sms() ? 8 : ctas(32) < 2 * device_sms() ? 16 : 32;
+    if (tile_smem(Tn, dk, R) <= 200 * 1024) {
+        if (R == 8) return launch_tile<T, 8>(q, k, v, o, B, Tn, H, dk, scale, st);
+        if (R == 16) return launch_tile<T, 16>(q, k, v, o, B, Tn, H, dk, scale, st);
+        return launch_tile<T, 32>(q, k, v, o, B, Tn, H, dk, scale, st);
+    }
     const size_t smem = (size_t)nw * (Tn + dk) * sizeof(float);
     if (smem > 200 * 1024)
         return set_error(CONVNN_E_UNSUPPORTED, "softmax attention over %d tokens is outside this build", Tn);
@@ -434,8 +658,7 @@ int launch_attention_simt_t(const void* q, const void* k, const void* v, void* o
     int gx = (Tn + nw - 1) / nw;
     if (gx > 64) gx = 64;
     launch_chained(kern, dim3(gx, B * H), nw * 32, smem, st, static_cast<const T*>(q), static_cast<const T*>(k),
-                                                 static_cast<const T*>(v), static_cast<T*>(o), Tn, H, dk,
-                                                 (float)(1.0 / sqrt((double)dk)));
+                                                 static_cast<const T*>(v), static_cast<T*>(o), Tn, H, dk, scale);
     CONVNN_CHECK_LAUNCH("attention_simt");
     return CONVNN_OK;
 }
