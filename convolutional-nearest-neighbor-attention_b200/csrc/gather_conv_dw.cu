@@ -88,6 +88,7 @@ __device__ __forceinline__ void token_pairs(const DwParams& p, int m0, int nt, i
     if (p.softmax) {
         for (int t = threadIdx.x; t < nt; t += THREADS) {
             float m = -3.402823466e38f;
+#pragma unroll 8
             for (int j = 0; j < p.K; ++j) m = fmaxf(m, __int_as_float(pairs[at(t, j)].y));
             red[t] = m;
         }
@@ -96,6 +97,7 @@ __device__ __forceinline__ void token_pairs(const DwParams& p, int m0, int nt, i
         __syncthreads();
         for (int t = threadIdx.x; t < nt; t += THREADS) {
             float s = 0.f;
+#pragma unroll 8
             for (int j = 0; j < p.K; ++j) s += __int_as_float(pairs[at(t, j)].y);
             red[t] = s;
         }
@@ -226,6 +228,10 @@ int launch(const DwParams& p, cudaStream_t st) {
     int TT = (THREADS * tpt + p.groups - 1) / p.groups;
     const long long mult = p.M / ((long long)TT * device_sms() * 6);
     if (mult > 1) TT *= mult < 8 ? (int)mult : 8;
+    // A grid that leaves SMs idle: fewer tokens per CTA, whose weights come first, at the price of idle threads (us; 2 x 65 x 96, 25 taps
+    // 7.4 -> 4.7, 10 x 197 x 192 8.4 -> 6.3, 14 x 65 x 192, 16 taps 6.5 -> 4.2, 3 x 65 x 96, 9 taps 5.0 -> 3.9).
+    const int spread = (p.M + 2 * device_sms() - 1) / (2 * device_sms());
+    if (tpt == 1 && TT > spread) TT = spread;
     if (TT > 4096 / p.K) TT = 4096 / p.K;                 // 32 KB of (row, weight) pairs
     TT = TT / tpt * tpt;
     if (TT < tpt) TT = tpt;
@@ -233,12 +239,13 @@ int launch(const DwParams& p, cudaStream_t st) {
     const int grid = (p.M + TT - 1) / TT;
     // The form by the rounds of CTAs per SM it needs: with four tokens per thread three CTAs of one tap in flight, or two of two
     // taps where both need two rounds (3 x 1611 tokens x 10, 96 channels, 25 taps 36.1, 32.7 us); with one token four CTAs of four
-    // taps while that is one round, then five or six of two taps, which fit in one (71 x 34 x 2 heads of 128, float32, 3 taps
-    // 5.4, 4.1; 9 x 701 x 2 heads of 64 6.6, 5.3).
+    // taps while that is one round (two CTAs of eight, of more than twelve taps: 2 x 65 x 96, 25 taps 8.9, 7.4), then five or six of
+    // two taps, which fit in one (71 x 34 x 2 heads of 128, float32, 3 taps 5.4, 4.1; 9 x 701 x 2 heads of 64 6.6, 5.3).
     const int sms = device_sms(), per_sm = (grid + sms - 1) / sms;
     auto go = [&](auto kern) { launch_chained(kern, grid, THREADS, smem, st, p, TT); };
     if (tpt == 4 && per_sm != 4) go(gather_conv_dw_kernel<T, TO, VEC, 4, 1, 3>);
     else if (tpt == 4) go(gather_conv_dw_kernel<T, TO, VEC, 4, 2, 2>);
+    else if (per_sm <= 2 && p.K > 12) go(gather_conv_dw_kernel<T, TO, VEC, 1, 8, 2>);
     else if (per_sm <= 4) go(gather_conv_dw_kernel<T, TO, VEC, 1, 4, 4>);
     else if (per_sm == 6) go(gather_conv_dw_kernel<T, TO, VEC, 1, 2, 6>);
     else go(gather_conv_dw_kernel<T, TO, VEC, 1, 2, 5>);
