@@ -327,18 +327,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (lane < lead) load_a((uint32_t)lane, lane, m0);
             __syncwarp();
         }
-        if (lane == 0) {
+        {
             uint32_t s = lead == (int)STAGES ? 0u : (uint32_t)lead, ph = lead == (int)STAGES ? 1u : 0u;   // ring slot and its phase
             uint32_t last_s = lead > 0 ? (uint32_t)lead - 1u : 0u, last_ph = 0;
             int skip = lead;                                             // chunks of the first tile that are on the way
             bool ok = true;
-            const bool tr = !PAIR && trace_enabled() && blockIdx.x == 0;
+            const bool tr = !PAIR && trace_enabled() && blockIdx.x == 0 && lane == 0;
             int tn = 0;
             trace(tr, 0, tn);
             auto load_w_tile = [&](int nt) {
-                mbar_expect_tx_a(wfull_a, p.KC * b_bytes + (LNF ? (uint32_t)bn_cta * 32u : 0u));
-                for (int kc = 0; kc < p.KC; ++kc) tma_load_2d_a(sB0 + kc * b_bytes, &tmW, wfull_a, kc * p.KCH, nt * p.BN);
-                if (LNF) tma_load_2d_a(smem_u32(xb), &tmX, wfull_a, 0, nt * p.BN);
+                if (elect_one()) {
+                    mbar_expect_tx_a(wfull_a, p.KC * b_bytes + (LNF ? (uint32_t)bn_cta * 32u : 0u));
+                    for (int kc = 0; kc < p.KC; ++kc) tma_load_2d_a(sB0 + kc * b_bytes, &tmW, wfull_a, kc * p.KCH, nt * p.BN);
+                    if (LNF) tma_load_2d_a(smem_u32(xb), &tmX, wfull_a, 0, nt * p.BN);
+                }
                 cur_nt = nt;
             };
             if (lead == 0 && first < last) {
@@ -348,8 +350,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     if (p.wstat) load_w_tile(nt);
                     else
                         for (w_ahead = 0; w_ahead < min(p.KC, (int)STAGES); ++w_ahead) {
-                            if (!PAIR || rank == 0) mbar_expect_tx_a(full0 + 8 * w_ahead, tx);
-                            load_w_chunk((uint32_t)w_ahead, w_ahead, nt * p.BN + (int)rank * bn_cta);
+                            if (elect_one()) {
+                                if (!PAIR || rank == 0) mbar_expect_tx_a(full0 + 8 * w_ahead, tx);
+                                load_w_chunk((uint32_t)w_ahead, w_ahead, nt * p.BN + (int)rank * bn_cta);
+                            }
                         }
                 }
                 chain_wait_unless(BESIDE);
@@ -361,7 +365,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (p.wstat && nt != cur_nt) {
                     // every MMA that reads the old W tile has completed once the most recently
                     // filled ring stage has been released
-                    if (any && !mbar_wait_a(empty0 + 8 * last_s, last_ph, abort_flag)) { give_up(15); ok = false; break; }
+                    if (any && !mbar_wait_warp(empty0 + 8 * last_s, last_ph, abort_flag)) { give_up(15); ok = false; break; }
                     load_w_tile(nt);
                 }
                 trace(tr, 0, tn);
@@ -369,19 +373,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 const int kc0 = skip;
                 skip = 0;
                 for (int kc = kc0; kc < p.KC; ++kc) {
-                    if (!mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag)) { give_up(11); ok = false; break; }
+                    if (!mbar_wait_warp(empty0 + 8 * s, ph ^ 1u, abort_flag)) { give_up(11); ok = false; break; }
                     const bool whole = w_ahead == 0;            // (otherwise its W chunk is on the way)
-                    if (whole && (!PAIR || rank == 0)) mbar_expect_tx_a(full0 + 8 * s, tx);
-                    load_a(s, kc, m0);
-                    if (whole) load_w_chunk(s, kc, n0);
-                    else --w_ahead;
+                    if (elect_one()) {
+                        if (whole && (!PAIR || rank == 0)) mbar_expect_tx_a(full0 + 8 * s, tx);
+                        load_a(s, kc, m0);
+                        if (whole) load_w_chunk(s, kc, n0);
+                    }
+                    if (!whole) --w_ahead;
                     last_s = s; last_ph = ph; any = true;
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             const uint32_t idesc = make_idesc_bf16_f32(TM, p.BN);
             const uint64_t dhi = kmajor_desc_hi(pitch);
             const int nk16 = p.KCH / 16;
@@ -393,7 +399,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             uint32_t s = 0, ph = 0, tile = 0, wloads = 0, last_stage = 0;
             int cur_nt = -1;
             bool ok = true;
-            const bool tr = !PAIR && trace_enabled() && blockIdx.x == 0;
+            const bool tr = !PAIR && trace_enabled() && blockIdx.x == 0 && lane == 0;
             int tn = 0;
             const uint32_t peer_empty0 = PAIR ? map_to_cta(empty0, 1) : 0u;
             const uint32_t peer_tfull0 = PAIR ? map_to_cta(tfull0, 1) : 0u;
@@ -402,13 +408,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             unsigned long long budget = kStartBudgetNs;
             for (int t = first; t < last && ok; t += step, ++tile) {
                 const uint32_t buf = tile & 1u, u = tile >> 1;
-                if (!mbar_wait_a(tempty0 + 8 * buf, (u & 1u) ^ 1u, abort_flag)) { give_up(12); ok = false; break; }
+                if (!mbar_wait_warp(tempty0 + 8 * buf, (u & 1u) ^ 1u, abort_flag)) { give_up(12); ok = false; break; }
                 trace(tr, 1, tn);                           // accumulator buffer free
                 int mt = 0, nt = 0;
                 if (p.wstat || mbias) tile_mn(t, mt, nt);
                 if (p.wstat) {
                     if (nt != cur_nt) {
-                        if (!mbar_wait_a(wfull_a, wloads & 1u, abort_flag, budget)) { give_up(16); ok = false; break; }
+                        if (!mbar_wait_warp(wfull_a, wloads & 1u, abort_flag, budget)) { give_up(16); ok = false; break; }
                         cur_nt = nt;
                         ++wloads;
                     }
@@ -417,15 +423,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 const uint32_t d_tmem = tmem_base + buf * p.BNpad;
                 if (mbias) {                                 // accumulator := bias, the chunks add to it
                     const uint64_t bias_desc = dhi32 | (uint64_t)((btile0 + (uint32_t)nt * bn_cta * 32u) >> 4);
-                    if (PAIR) mma_bf16_ss_pair(d_tmem, ones_desc, bias_desc, idesc, 0);
-                    else mma_bf16_ss(d_tmem, ones_desc, bias_desc, idesc, 0);
+                    if (elect_one()) {
+                        if (PAIR) mma_bf16_ss_pair(d_tmem, ones_desc, bias_desc, idesc, 0);
+                        else mma_bf16_ss(d_tmem, ones_desc, bias_desc, idesc, 0);
+                    }
                 }
                 for (int kc = 0; kc < p.KC; ++kc) {
-                    if (!mbar_wait_a(full0 + 8 * s, ph, abort_flag, budget)) { give_up(13); ok = false; break; }
+                    if (!mbar_wait_warp(full0 + 8 * s, ph, abort_flag, budget)) { give_up(13); ok = false; break; }
                     tc_fence_after_sync();
                     const uint64_t adesc = dhi | (uint64_t)(((sA0 + s * a_bytes) & 0x3FFFFu) >> 4);
                     const uint64_t bdesc = dhi | (uint64_t)(((sB0 + (p.wstat ? (uint32_t)kc : s) * b_bytes) & 0x3FFFFu) >> 4);
-                    if (PAIR) {
+                    if (LNF && kc == p.KC - 1) last_stage = s;
+                    if (!elect_one()) {
+                    } else if (PAIR) {
                         mma_chunk_pair(d_tmem, adesc, bdesc, idesc, nk16, (kc != 0) | mbias);
                         mma_commit_pair(empty0 + 8 * s);
                         mma_commit_pair(peer_empty0 + 8 * s);
@@ -435,22 +445,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         // the release of the most recently filled stage as "every MMA that reads the resident W
                         // tile has completed" before it loads the next W tile, and the extra MMA reads the
                         // extra rows that travel with that tile.
-                        if (LNF && kc == p.KC - 1) last_stage = s;
-                        else mma_commit_a(empty0 + 8 * s);
+                        if (!LNF || kc != p.KC - 1) mma_commit_a(empty0 + 8 * s);
                     }
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
                 if (LNF && ok) {
                     // accumulator += [-mean, sigma] x [c, b']: the chunk the extra warp wrote for this buffer
-                    if (!mbar_wait_a(smem_u32(&xfull[buf]), u & 1u, abort_flag, budget)) { give_up(17); ok = false; break; }
+                    if (!mbar_wait_warp(smem_u32(&xfull[buf]), u & 1u, abort_flag, budget)) { give_up(17); ok = false; break; }
                     tc_fence_after_sync();
                     const uint64_t xa_desc = dhi32 | (uint64_t)(((smem_u32(xa) + buf * 4096u) & 0x3FFFFu) >> 4);
                     const uint64_t xb_desc = dhi32 | (uint64_t)((smem_u32(xb) & 0x3FFFFu) >> 4);
-                    mma_bf16_ss(d_tmem, xa_desc, xb_desc, idesc, 1);
-                    mma_commit_a(empty0 + 8 * last_stage);
+                    if (elect_one()) {
+                        mma_bf16_ss(d_tmem, xa_desc, xb_desc, idesc, 1);
+                        mma_commit_a(empty0 + 8 * last_stage);
+                    }
                 }
                 budget = kWaitBudgetNs;
-                if (ok) {
+                if (ok && elect_one()) {
                     if (PAIR) { mma_commit_pair(tfull0 + 8 * buf); mma_commit_pair(peer_tfull0 + 8 * buf); }
                     else mma_commit_a(tfull0 + 8 * buf);
                 }
@@ -816,6 +827,16 @@ static int tile_width(int N, int parts, bool has_stat) {
     return (((N + nt - 1) / nt) + 15) / 16 * 16;
 }
 
+// A grid that leaves most SMs idle: narrower tiles of the same sums, as long as there is at most one per SM.
+static int narrower(int bn, int M, int part_cols, int parts) {
+    const long long m_tiles = (M + BM - 1) / BM, sms = device_sms();
+    for (int half = bn / 2; half >= 32 && half % 16 == 0 && (parts == 1 || part_cols % half == 0); half /= 2) {
+        if (m_tiles * parts * ((part_cols + half - 1) / half) > sms) break;
+        bn = half;
+    }
+    return bn;
+}
+
 // Planes of partial row moments a GEMM with `moments_out` writes for N output columns.
 int gemm_tc_moment_planes(int N) { return 2 * ((N + tile_width(N, 1, false) - 1) / tile_width(N, 1, false)); }
 
@@ -868,6 +889,7 @@ int launch_gemm_tc(const void* a, long long lda, const void* w, int M, int N, in
     p.KC = Kd / p.KCH;
     p.BN = tile_width(N, parts, o.stat[0] != nullptr);
     const bool lnf = o.ln_moments != nullptr;
+    if (!lnf && !o.moments_out && !o.stat[0] && !o.stat[1] && !o.stat[2]) p.BN = narrower(p.BN, M, N / parts, parts);
     p.ln_planes = o.ln_planes; p.ln_eps = o.ln_eps; p.ln_inv_k = 1.0f / (float)Kd;
     p.moments_out = static_cast<float2*>(static_cast<void*>(o.moments_out));
     p.mom_ld = gemm_tc_moment_stride(M);

@@ -194,6 +194,19 @@ __device__ __forceinline__ uint64_t make_kmajor_desc(uint32_t smem_addr, uint32_
 __host__ __device__ constexpr uint32_t make_idesc_bf16_f32(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+// One lane of a converged warp, the same every time.  A role that issues MMAs is walked by its whole warp, so that addresses and
+// descriptors are the warp's and not a lane's (uniform registers), and only the issue itself belongs to this lane: a loop
+// inside `if (lane == 0)` moves every operand of every instruction over, 26 ns per MMA and 0.2 us per wait, commit and address of a chunk.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
+// A wait of a converged warp, with one answer for all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort,
+                                               unsigned long long budget_ns = kWaitBudgetNs) {
+    return __all_sync(0xffffffffu, mbar_wait_a(bar, parity, abort, budget_ns));
+}
 // D[tmem] (+)= A[smem] * B[smem]^T; issued by one thread.
 __device__ __forceinline__ void mma_bf16_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                             uint32_t accumulate) {
@@ -366,16 +379,6 @@ __device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t (&r)[
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ bool elect_one() {
-    uint32_t pred;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "elect.sync _|p, 0xffffffff;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(pred));
-    return pred != 0;
-}
 
 }  // namespace sm100
 
