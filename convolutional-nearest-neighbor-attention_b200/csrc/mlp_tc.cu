@@ -313,7 +313,7 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
         // ---- issuer of MMA 1 (leader only): acc1[n & 1] = x W1'[super-chunk]^T, N = 128.  A tcgen05.mma
         // costs its issuing thread ~35-50 ns whatever its size, so the steps are as wide as the pipeline
         // allows and MMA 2 has an issuing thread of its own; the barriers order the two streams.
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             const uint32_t idesc1 = make_idesc_bf16_f32(2 * BM, SC);
             const uint64_t dhi = kmajor_desc_hi(128), dhi32 = kmajor_desc_hi(32);
             auto desc = [&](uint64_t hi, uint32_t addr) { return hi | (uint64_t)((addr & 0x3FFFFu) >> 4); };
@@ -323,19 +323,21 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
             // the two output-projection items of tile `it`: acc1[n & 1] = o W_o[item]^T, N = D / 2
             auto mma_wo = [&](int it) {
                 const uint32_t xb = (uint32_t)it & 1u;
-                if (!mbar_wait_a(lbar(XFULL + xb), (uint32_t)(it >> 1) & 1u, abort_flag)) { give_up(54); ok = false; return; }
+                if (!mbar_wait_warp(lbar(XFULL + xb), (uint32_t)(it >> 1) & 1u, abort_flag)) { give_up(54); ok = false; return; }
                 for (int item = 0; item < 2; ++item, ++n) {
                     const uint32_t b = n & 1u;
-                    if (!mbar_wait_a(lbar(A1EMPTY + b), ((n >> 1) & 1u) ^ 1u, abort_flag)) { give_up(56); ok = false; return; }
-                    mtrace(cluster_id == 0, 2, n);
-                    if (!mbar_wait_a(lbar(W1FULL + b), (n >> 1) & 1u, abort_flag)) { give_up(57); ok = false; return; }
-                    mtrace(cluster_id == 0, 3, n);
+                    if (!mbar_wait_warp(lbar(A1EMPTY + b), ((n >> 1) & 1u) ^ 1u, abort_flag)) { give_up(56); ok = false; return; }
+                    mtrace(cluster_id == 0 && lane == 0, 2, n);
+                    if (!mbar_wait_warp(lbar(W1FULL + b), (n >> 1) & 1u, abort_flag)) { give_up(57); ok = false; return; }
+                    mtrace(cluster_id == 0 && lane == 0, 3, n);
                     tc_fence_after_sync();
                     const uint32_t xs0 = base + L.x + xb * x_tile_bytes, w0s = base + L.w1 + b * L.w1_slot;
-                    for (int kc = 0; kc < p.KC; ++kc)
-                        mma_chunk_pair(tmem_base + b * SC, desc(dhi, xs0 + kc * 16384u), desc(dhi, w0s + kc * 8192u), idesc0, 4, kc != 0);
-                    mma_commit_pair_both(lbar(A1FULL + b));
-                    mtrace(cluster_id == 0, 4, n);
+                    if (elect_one()) {
+                        for (int kc = 0; kc < p.KC; ++kc)
+                            mma_chunk_pair(tmem_base + b * SC, desc(dhi, xs0 + kc * 16384u), desc(dhi, w0s + kc * 8192u), idesc0, 4, kc != 0);
+                        mma_commit_pair_both(lbar(A1FULL + b));
+                    }
+                    mtrace(cluster_id == 0 && lane == 0, 4, n);
                 }
             };
             chain_wait();                                          // (the budgets of its waits are for this kernel's work)
@@ -346,28 +348,30 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
                     if (OP && sc == kp && it + 1 < my_tiles) { mma_wo(it + 1); if (!ok) break; }
                     const uint32_t b = n & 1u;
                     if (sc == 0) {
-                        if (!OP && !mbar_wait_a(lbar(XFULL + xb), (uint32_t)(it >> 1) & 1u, abort_flag)) { give_up(54); ok = false; break; }
-                        if (!mbar_wait_a(lbar(XAFULL + xb), (uint32_t)(it >> 1) & 1u, abort_flag)) { give_up(55); ok = false; break; }
+                        if (!OP && !mbar_wait_warp(lbar(XFULL + xb), (uint32_t)(it >> 1) & 1u, abort_flag)) { give_up(54); ok = false; break; }
+                        if (!mbar_wait_warp(lbar(XAFULL + xb), (uint32_t)(it >> 1) & 1u, abort_flag)) { give_up(55); ok = false; break; }
                     }
-                    if (!mbar_wait_a(lbar(A1EMPTY + b), ((n >> 1) & 1u) ^ 1u, abort_flag)) { give_up(56); ok = false; break; }
-                    mtrace(cluster_id == 0, 2, n);
-                    if (!mbar_wait_a(lbar(W1FULL + b), (n >> 1) & 1u, abort_flag)) { give_up(57); ok = false; break; }
-                    mtrace(cluster_id == 0, 3, n);
+                    if (!mbar_wait_warp(lbar(A1EMPTY + b), ((n >> 1) & 1u) ^ 1u, abort_flag)) { give_up(56); ok = false; break; }
+                    mtrace(cluster_id == 0 && lane == 0, 2, n);
+                    if (!mbar_wait_warp(lbar(W1FULL + b), (n >> 1) & 1u, abort_flag)) { give_up(57); ok = false; break; }
+                    mtrace(cluster_id == 0 && lane == 0, 3, n);
                     tc_fence_after_sync();
                     const uint32_t d1 = tmem_base + b * SC;
                     const uint32_t xs = base + L.x + xb * x_tile_bytes, w1s = base + L.w1 + b * L.w1_slot;
-                    for (int kc = 0; kc < p.KC; ++kc)
-                        mma_chunk_pair(d1, desc(dhi, xs + kc * 16384u), desc(dhi, w1s + kc * 8192u), idesc1, 4, kc != 0);
-                    // the pre-norm fold's extra step: [-mean, sigma] x [c, b']
-                    mma_bf16_ss_pair(d1, desc(dhi32, base + L.xa + xb * 4096u), desc(dhi32, w1s + p.KC * 8192u), idesc1, 1);
-                    mma_commit_pair_both(lbar(A1FULL + b));
-                    mtrace(cluster_id == 0, 4, n);
+                    if (elect_one()) {
+                        for (int kc = 0; kc < p.KC; ++kc)
+                            mma_chunk_pair(d1, desc(dhi, xs + kc * 16384u), desc(dhi, w1s + kc * 8192u), idesc1, 4, kc != 0);
+                        // the pre-norm fold's extra step: [-mean, sigma] x [c, b']
+                        mma_bf16_ss_pair(d1, desc(dhi32, base + L.xa + xb * 4096u), desc(dhi32, w1s + p.KC * 8192u), idesc1, 1);
+                        mma_commit_pair_both(lbar(A1FULL + b));
+                    }
+                    mtrace(cluster_id == 0 && lane == 0, 4, n);
                 }
             }
         }
     } else if (warp == 19) {
         // ---- issuer of MMA 2 (leader only): acc2 (+)= h[chunk] W2[:, chunk]^T, N = D
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             const uint32_t idesc2 = make_idesc_bf16_f32(2 * BM, p.D);
             const uint64_t dhi = kmajor_desc_hi(128);
             auto desc = [&](uint64_t hi, uint32_t addr) { return hi | (uint64_t)((addr & 0x3FFFFu) >> 4); };
@@ -379,23 +383,25 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
             chain_wait();
             for (uint32_t g = 0; g < total; ++g) {
                 const uint32_t hb = g & 1u;                       // h chunk = half of its super-chunk
-                if (c == 0 && !mbar_wait_a(lbar(A2EMPTY), ((uint32_t)it & 1u) ^ 1u, abort_flag)) { give_up(58); break; }
-                if (!mbar_wait_a(lbar(HFULL + hb), (g >> 1) & 1u, abort_flag)) { give_up(59); break; }
-                mtrace(cluster_id == 0, 5, g);
-                if (!mbar_wait_a(lbar(W2FULL + s), ph, abort_flag)) { give_up(60); break; }
-                mtrace(cluster_id == 0, 6, g);
+                if (c == 0 && !mbar_wait_warp(lbar(A2EMPTY), ((uint32_t)it & 1u) ^ 1u, abort_flag)) { give_up(58); break; }
+                if (!mbar_wait_warp(lbar(HFULL + hb), (g >> 1) & 1u, abort_flag)) { give_up(59); break; }
+                mtrace(cluster_id == 0 && lane == 0, 5, g);
+                if (!mbar_wait_warp(lbar(W2FULL + s), ph, abort_flag)) { give_up(60); break; }
+                mtrace(cluster_id == 0 && lane == 0, 6, g);
                 tc_fence_after_sync();
                 // h straight from tensor memory, where the epilogue warps put it: 8 columns per K = 16 step
                 const uint64_t w2d = desc(dhi, base + L.w2 + s * L.w2_slot);
                 const uint32_t ha = tmem_base + h_col + hb * 32u;
-                mma_bf16_ts_pair(d2, ha, w2d, idesc2, c != 0);
-                mma_bf16_ts_pair(d2, ha + 8, w2d + 2, idesc2, 1);
-                mma_bf16_ts_pair(d2, ha + 16, w2d + 4, idesc2, 1);
-                mma_bf16_ts_pair(d2, ha + 24, w2d + 6, idesc2, 1);
-                mma_commit_pair_both(lbar(W2EMPTY + s));
-                mma_commit_pair_both(lbar(HEMPTY + hb));
-                if (c == nch - 1) mma_commit_pair_both(lbar(A2FULL));
-                mtrace(cluster_id == 0, 7, g);
+                if (elect_one()) {
+                    mma_bf16_ts_pair(d2, ha, w2d, idesc2, c != 0);
+                    mma_bf16_ts_pair(d2, ha + 8, w2d + 2, idesc2, 1);
+                    mma_bf16_ts_pair(d2, ha + 16, w2d + 4, idesc2, 1);
+                    mma_bf16_ts_pair(d2, ha + 24, w2d + 6, idesc2, 1);
+                    mma_commit_pair_both(lbar(W2EMPTY + s));
+                    mma_commit_pair_both(lbar(HEMPTY + hb));
+                    if (c == nch - 1) mma_commit_pair_both(lbar(A2FULL));
+                }
+                mtrace(cluster_id == 0 && lane == 0, 7, g);
                 if (++s == NSW2) { s = 0; ph ^= 1u; }
                 if (++c == nch) { c = 0; ++it; }
             }
@@ -403,7 +409,7 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
     } else if (warp == 20) {
         // ---- the W2 stream, a warp of its own: lanes of one warp that wait in different loops take turns, and
         // a W2 lane next to the W1 lanes only advanced when those came out of their (long) waits
-        if (lane == 0) {
+        {
             const uint32_t total = (uint32_t)my_tiles * (uint32_t)nsc * 2u;   // h chunks
             uint32_t s = 0, ph = 0;
             int c = 0;
@@ -411,10 +417,12 @@ mlp_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ C
             const uint32_t ahead = p.weights_at_rest ? NSW2 : 0u;       // a ring of chunks before the predecessor has ended
             for (uint32_t g = 0; g < total; ++g) {
                 if (g == ahead) chain_wait();
-                if (!mbar_wait_a(lbar(W2EMPTY + s), ph ^ 1u, abort_flag)) { give_up(53); break; }
-                mtrace(cluster_id == 0 && rank == 0, 0, g);
-                if (rank == 0) mbar_expect_tx_a(lbar(W2FULL + s), 2u * (uint32_t)(p.D / 2) * 128u);
-                tma_load_2d_pair(base + L.w2 + s * L.w2_slot, &tmW2, leadbar(W2FULL + s), c * CH, (int)rank * (p.D / 2));
+                if (!mbar_wait_warp(lbar(W2EMPTY + s), ph ^ 1u, abort_flag)) { give_up(53); break; }
+                mtrace(cluster_id == 0 && rank == 0 && lane == 0, 0, g);
+                if (elect_one()) {
+                    if (rank == 0) mbar_expect_tx_a(lbar(W2FULL + s), 2u * (uint32_t)(p.D / 2) * 128u);
+                    tma_load_2d_pair(base + L.w2 + s * L.w2_slot, &tmW2, leadbar(W2FULL + s), c * CH, (int)rank * (p.D / 2));
+                }
                 if (++s == NSW2) { s = 0; ph ^= 1u; }
                 if (++c == nch) c = 0;
             }
