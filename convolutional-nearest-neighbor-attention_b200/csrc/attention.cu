@@ -116,7 +116,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     chain_next();
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
             uint32_t it = 0;
             bool ok = true;
             for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x, ++it) {
@@ -124,19 +124,23 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 const int bh = unit / p.n_row_tiles, rt = unit - bh * p.n_row_tiles;
                 const int b = bh / p.H, h = bh - b * p.H;
                 // Q / K land where the previous unit's P was: MMA 2 must have finished reading it
-                if (it > 0 && !mbar_wait(o_full, ph ^ 1u, abort_flag)) { fail(abort_flag, 61); ok = false; break; }
-                mbar_expect_tx(qk_full, p.KC * (a_bytes + b_bytes));
-                for (int kc = 0; kc < p.KC; ++kc) {
-                    tma_load_4d(sQ + kc * a_bytes, &tmQ, qk_full, kc * p.KCH, h, rt * BM, b);
-                    tma_load_4d(sK + kc * b_bytes, &tmK, qk_full, kc * p.KCH, h, 0, b);
+                if (it > 0 && !mbar_wait_warp(smem_u32(o_full), ph ^ 1u, abort_flag)) { fail(abort_flag, 61); ok = false; break; }
+                if (elect_one()) {
+                    mbar_expect_tx(qk_full, p.KC * (a_bytes + b_bytes));
+                    for (int kc = 0; kc < p.KC; ++kc) {
+                        tma_load_4d(sQ + kc * a_bytes, &tmQ, qk_full, kc * p.KCH, h, rt * BM, b);
+                        tma_load_4d(sK + kc * b_bytes, &tmK, qk_full, kc * p.KCH, h, 0, b);
+                    }
                 }
-                if (!mbar_wait(v_empty, ph ^ 1u, abort_flag)) { fail(abort_flag, 62); ok = false; break; }
-                mbar_expect_tx(v_full, v_bytes);
-                tma_load_4d(sV, &tmV, v_full, 0, h, 0, b);
+                if (!mbar_wait_warp(smem_u32(v_empty), ph ^ 1u, abort_flag)) { fail(abort_flag, 62); ok = false; break; }
+                if (elect_one()) {
+                    mbar_expect_tx(v_full, v_bytes);
+                    tma_load_4d(sV, &tmV, v_full, 0, h, 0, b);
+                }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             const uint32_t idesc1 = make_idesc_bf16_f32(BM, p.BN);
             const uint32_t idesc2 = make_idesc_bf16_f32(BM, p.dk);
             const uint64_t dhi = kmajor_desc_hi(pitch), dhi128 = kmajor_desc_hi(128);
@@ -146,28 +150,32 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             bool ok = true;
             for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x, ++it) {
                 const uint32_t ph = it & 1u;
-                if (!mbar_wait(t_empty, ph ^ 1u, abort_flag)) { fail(abort_flag, 63); ok = false; break; }
-                if (!mbar_wait(qk_full, ph, abort_flag)) { fail(abort_flag, 64); ok = false; break; }
+                if (!mbar_wait_warp(smem_u32(t_empty), ph ^ 1u, abort_flag)) { fail(abort_flag, 63); ok = false; break; }
+                if (!mbar_wait_warp(smem_u32(qk_full), ph, abort_flag)) { fail(abort_flag, 64); ok = false; break; }
                 tc_fence_after_sync();
-                for (int kc = 0; kc < p.KC; ++kc) {
-                    const uint64_t ad = dhi | (uint64_t)(((sQ0 + kc * a_bytes) & 0x3FFFFu) >> 4);
-                    const uint64_t bd = dhi | (uint64_t)(((sK0 + kc * b_bytes) & 0x3FFFFu) >> 4);
-                    mma_chunk(tmem_base, ad, bd, idesc1, nk16, kc != 0);
-                }
-                mma_commit(s_full);
-                if (!mbar_wait(p_ready, ph, abort_flag)) { fail(abort_flag, 65); ok = false; break; }
-                tc_fence_after_sync();
-                uint32_t acc = 0;
-                for (int kc2 = 0; kc2 < p.NKC2; ++kc2) {
-                    const uint64_t ad = dhi128 | (uint64_t)(((sP0 + kc2 * 16384u) & 0x3FFFFu) >> 4);
-                    const uint64_t bd = dhi128 | (uint64_t)(((sVt0 + kc2 * vt_chunk) & 0x3FFFFu) >> 4);
-                    for (int k16 = 0; k16 < 4; ++k16) {
-                        if (kc2 * 64 + k16 * 16 >= p.BN) break;
-                        mma_bf16_ss(tmem_base, ad + 2 * k16, bd + 2 * k16, idesc2, acc);
-                        acc = 1;
+                if (elect_one()) {
+                    for (int kc = 0; kc < p.KC; ++kc) {
+                        const uint64_t ad = dhi | (uint64_t)(((sQ0 + kc * a_bytes) & 0x3FFFFu) >> 4);
+                        const uint64_t bd = dhi | (uint64_t)(((sK0 + kc * b_bytes) & 0x3FFFFu) >> 4);
+                        mma_chunk(tmem_base, ad, bd, idesc1, nk16, kc != 0);
                     }
+                    mma_commit(s_full);
                 }
-                mma_commit(o_full);
+                if (!mbar_wait_warp(smem_u32(p_ready), ph, abort_flag)) { fail(abort_flag, 65); ok = false; break; }
+                tc_fence_after_sync();
+                if (elect_one()) {
+                    uint32_t acc = 0;
+                    for (int kc2 = 0; kc2 < p.NKC2; ++kc2) {
+                        const uint64_t ad = dhi128 | (uint64_t)(((sP0 + kc2 * 16384u) & 0x3FFFFu) >> 4);
+                        const uint64_t bd = dhi128 | (uint64_t)(((sVt0 + kc2 * vt_chunk) & 0x3FFFFu) >> 4);
+                        for (int k16 = 0; k16 < 4; ++k16) {
+                            if (kc2 * 64 + k16 * 16 >= p.BN) break;
+                            mma_bf16_ss(tmem_base, ad + 2 * k16, bd + 2 * k16, idesc2, acc);
+                            acc = 1;
+                        }
+                    }
+                    mma_commit(o_full);
+                }
             }
         }
     } else {

@@ -123,31 +123,34 @@ conv1d_tc_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             const uint32_t idesc = make_idesc_bf16_f32(BM, p.dk);
             const uint64_t dhi = kmajor_desc_hi(pitch), dhi32 = kmajor_desc_hi(32);
             auto desc = [&](uint64_t hi, const void* at) { return hi | (uint64_t)((smem_u32(at) & 0x3FFFFu) >> 4); };
             const uint64_t ones_desc = desc(dhi32, ones), bias_desc = desc(dhi32, btile);
             const int nk16 = p.dk / 16;
-            bool ok = mbar_wait(wfull, 0, abort_flag);
+            bool ok = mbar_wait_warp(smem_u32(wfull), 0, abort_flag);
             if (!ok) fail(abort_flag, 102);
             uint32_t buf = 0, ph = 0, n = 0;
             for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x) {
                 for (int i = 0; i < p.n_tiles; ++i, ++n) {
                     const uint32_t a = n & 1u;
-                    if (!mbar_wait(&tempty[a], ((n >> 1) & 1u) ^ 1u, abort_flag) || !mbar_wait(&full[buf], ph, abort_flag)) {
+                    if (!mbar_wait_warp(smem_u32(&tempty[a]), ((n >> 1) & 1u) ^ 1u, abort_flag) ||
+                        !mbar_wait_warp(smem_u32(&full[buf]), ph, abort_flag)) {
                         fail(abort_flag, 103);
                         ok = false;
                         break;
                     }
                     tc_fence_after_sync();
                     const uint32_t d = tmem_base + a * p.acc_cols;
-                    if (p.bias) mma_bf16_ss(d, ones_desc, bias_desc, idesc, 0);
-                    for (int j = 0; j < p.ks; ++j)
-                        mma_chunk(d, desc(dhi, smem + buf * set_bytes + j * a_bytes), desc(dhi, sW + j * w_tap), idesc, nk16,
-                                  j != 0 || p.bias);
-                    mma_commit(&empty[buf]);
-                    mma_commit(&tfull[a]);
+                    if (elect_one()) {
+                        if (p.bias) mma_bf16_ss(d, ones_desc, bias_desc, idesc, 0);
+                        for (int j = 0; j < p.ks; ++j)
+                            mma_chunk(d, desc(dhi, smem + buf * set_bytes + j * a_bytes), desc(dhi, sW + j * w_tap), idesc, nk16,
+                                      j != 0 || p.bias);
+                        mma_commit(&empty[buf]);
+                        mma_commit(&tfull[a]);
+                    }
                     if (++buf == (uint32_t)p.nbuf) { buf = 0; ph ^= 1u; }
                 }
             }

@@ -208,42 +208,28 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
 
     const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty), st0 = smem_u32(smem);
     if (warp == 0) {
-        // One thread can start a TMA operation only every ~0.3 us, while operations started by different lanes overlap: a lane
-        // per box of the first segment's chunks; from then on lane 0 brings key rows, lane 1 candidate rows.
-        static_assert(MAX_STAGES <= 8, "lanes 8 ... bring the candidate rows");
         Segment sg(p);
-        const int lead = sg.valid() ? min(p.KC, (int)STAGES) : 0;
-        if (lane < lead) mbar_expect_tx_a(full0 + 8 * lane, landing);
-        __syncwarp();
         chain_wait();
-        if (lead > 0) {
-            const int b = sg.bh / p.H, h = sg.bh - b * p.H, kc = lane & 7;
-            const uint32_t st = st0 + kc * stage_bytes, fb = full0 + 8 * kc;
-            if (kc < lead && lane < 8) tma_load_4d_a(st, &tmK, fb, kc * p.KCH, h, sg.row, b);
-            else if (kc < lead && lane < 16) tma_load_4d_a(st + a_bytes, &tmQ, fb, kc * p.KCH, h, 0, b);
-        }
-        __syncwarp();
-        if (lane < 2) {
-            uint32_t s = lead == (int)STAGES ? 0u : (uint32_t)lead, ph = lead == (int)STAGES ? 1u : 0u;
-            int kc0 = lead;
+        {
+            uint32_t s = 0, ph = 0;
             bool ok = true;
-            for (; sg.valid() && ok; sg.next(p), kc0 = 0) {
+            for (; sg.valid() && ok; sg.next(p)) {
                 const int b = sg.bh / p.H, h = sg.bh - b * p.H;
-                for (int kc = kc0; kc < p.KC; ++kc) {
-                    ok = mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag);
-                    ok = __all_sync(0x3u, ok);
+                for (int kc = 0; kc < p.KC; ++kc) {
+                    ok = mbar_wait_warp(empty0 + 8 * s, ph ^ 1u, abort_flag);
                     if (!ok) { if (lane == 0) fail(abort_flag, 81); break; }
                     const uint32_t st = st0 + s * stage_bytes, fb = full0 + 8 * s;
-                    if (lane == 0) mbar_expect_tx_a(fb, landing);
-                    __syncwarp(0x3u);
-                    if (lane == 0) tma_load_4d_a(st, &tmK, fb, kc * p.KCH, h, sg.row, b);
-                    else tma_load_4d_a(st + a_bytes, &tmQ, fb, kc * p.KCH, h, 0, b);
+                    if (elect_one()) {
+                        mbar_expect_tx_a(fb, landing);
+                        tma_load_4d_a(st, &tmK, fb, kc * p.KCH, h, sg.row, b);
+                        tma_load_4d_a(st + a_bytes, &tmQ, fb, kc * p.KCH, h, 0, b);
+                    }
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             const uint32_t idesc = make_idesc_bf16_f32(BM, p.BN);
             const uint64_t dhi = kmajor_desc_hi(pitch);
             const int nk16 = p.KCH / 16;
@@ -252,18 +238,20 @@ sim_topk_rows_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
             bool ok = true;
             chain_wait();                            // (the budgets of its waits are for this kernel's work)
             for (Segment sg(p); sg.valid() && ok; sg.next(p)) {
-                if (!mbar_wait_a(tempty0 + 8 * buf, (use & 1u) ^ 1u, abort_flag)) { fail(abort_flag, 82); break; }
+                if (!mbar_wait_warp(tempty0 + 8 * buf, (use & 1u) ^ 1u, abort_flag)) { fail(abort_flag, 82); break; }
                 tc_fence_after_sync();
                 for (int kc = 0; kc < p.KC; ++kc) {
-                    if (!mbar_wait_a(full0 + 8 * s, ph, abort_flag)) { fail(abort_flag, 83); ok = false; break; }
+                    if (!mbar_wait_warp(full0 + 8 * s, ph, abort_flag)) { fail(abort_flag, 83); ok = false; break; }
                     tc_fence_after_sync();
                     const uint32_t sa = st0 + s * stage_bytes;
-                    mma_chunk(tmem_base + buf * p.acc_cols, dhi | (uint64_t)(sa >> 4),
-                              dhi | (uint64_t)((sa + a_bytes) >> 4), idesc, nk16, kc != 0);
-                    mma_commit_a(empty0 + 8 * s);
+                    if (elect_one()) {
+                        mma_chunk(tmem_base + buf * p.acc_cols, dhi | (uint64_t)(sa >> 4),
+                                  dhi | (uint64_t)((sa + a_bytes) >> 4), idesc, nk16, kc != 0);
+                        mma_commit_a(empty0 + 8 * s);
+                    }
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
-                if (ok) mma_commit_a(tfull0 + 8 * buf);
+                if (ok && elect_one()) mma_commit_a(tfull0 + 8 * buf);
                 if (++buf == 2) { buf = 0; ++use; }
             }
         }

@@ -186,27 +186,27 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 
     const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty), st0 = smem_u32(smem);
     if (warp == 0) {
-        if (lane < 2) {                              // lane 0: key rows, lane 1: candidate rows (their copies overlap)
+        {
             uint32_t s = 0, ph = 0;
             bool ok = true;
             for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x) {
                 const int bh = unit / p.n_row_tiles, rt = unit - bh * p.n_row_tiles;
                 const int b = bh / p.H, h = bh - b * p.H;
                 for (int kc = 0; kc < p.KC; ++kc) {
-                    ok = mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag);
-                    ok = __all_sync(0x3u, ok);
+                    ok = mbar_wait_warp(empty0 + 8 * s, ph ^ 1u, abort_flag);
                     if (!ok) { if (lane == 0) fail(abort_flag, 71); break; }
                     const uint32_t st = st0 + s * stage_bytes, fb = full0 + 8 * s;
-                    if (lane == 0) mbar_expect_tx_a(fb, stage_bytes);
-                    __syncwarp(0x3u);
-                    if (lane == 0) tma_load_4d_a(st, &tmK, fb, kc * p.KCH, h, rt * BM, b);
-                    else tma_load_4d_a(st + a_bytes, &tmQ, fb, kc * p.KCH, h, 0, b);
+                    if (elect_one()) {
+                        mbar_expect_tx_a(fb, stage_bytes);
+                        tma_load_4d_a(st, &tmK, fb, kc * p.KCH, h, rt * BM, b);
+                        tma_load_4d_a(st + a_bytes, &tmQ, fb, kc * p.KCH, h, 0, b);
+                    }
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             const uint32_t idesc = make_idesc_bf16_f32(BM, p.BN);
             const uint64_t dhi = kmajor_desc_hi(pitch);
             const int nk16 = p.KCH / 16;
@@ -214,18 +214,20 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
             uint32_t s = 0, ph = 0, buf = 0, use = 0;
             bool ok = true;
             for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x) {
-                if (!mbar_wait_a(tempty0 + 8 * buf, (use & 1u) ^ 1u, abort_flag)) { fail(abort_flag, 72); break; }
+                if (!mbar_wait_warp(tempty0 + 8 * buf, (use & 1u) ^ 1u, abort_flag)) { fail(abort_flag, 72); break; }
                 tc_fence_after_sync();
                 for (int kc = 0; kc < p.KC; ++kc) {
-                    if (!mbar_wait_a(full0 + 8 * s, ph, abort_flag)) { fail(abort_flag, 73); ok = false; break; }
+                    if (!mbar_wait_warp(full0 + 8 * s, ph, abort_flag)) { fail(abort_flag, 73); ok = false; break; }
                     tc_fence_after_sync();
                     const uint32_t sa = st0 + s * stage_bytes;
-                    mma_chunk(tmem_base + buf * MAXC, dhi | (uint64_t)(sa >> 4), dhi | (uint64_t)((sa + a_bytes) >> 4), idesc, nk16,
-                              kc != 0);
-                    mma_commit_a(empty0 + 8 * s);
+                    if (elect_one()) {
+                        mma_chunk(tmem_base + buf * MAXC, dhi | (uint64_t)(sa >> 4), dhi | (uint64_t)((sa + a_bytes) >> 4), idesc, nk16,
+                                  kc != 0);
+                        mma_commit_a(empty0 + 8 * s);
+                    }
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
-                if (ok) mma_commit_a(tfull0 + 8 * buf);
+                if (ok && elect_one()) mma_commit_a(tfull0 + 8 * buf);
                 if (++buf == G) { buf = 0; ++use; }
             }
         }

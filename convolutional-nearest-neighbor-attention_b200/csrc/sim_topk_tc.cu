@@ -115,11 +115,7 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     const uint32_t st0 = smem_u32(stages);
 
     if (warp == 0) {
-        // One thread can start a TMA operation only every ~0.3 us whatever its size, while operations started
-        // by different lanes overlap: the three boxes of a stage (two key tiles, one query tile) are issued by
-        // lanes 0, 1 and 2 with one instruction of the warp (a unit of the ViT shape has 36 of them).
-        if (lane < 3) {
-            const uint32_t m3 = 0x7u;
+        {
             uint32_t s = 0, ph = 0;                  // ring slot and phase, advanced incrementally
             bool ok = true;
             chain_wait();
@@ -132,22 +128,22 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
                 for (int ct = 0; ct < p.n_col_tiles && ok; ++ct) {
                     const int col0 = ct * p.BN;
                     for (int kc = 0; kc < p.KC; ++kc) {
-                        ok = mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag);
-                        ok = __all_sync(m3, ok);
+                        ok = mbar_wait_warp(empty0 + 8 * s, ph ^ 1u, abort_flag);
                         if (!ok) { if (lane == 0) fail(abort_flag, 1); break; }
                         const uint32_t st = st0 + s * stage_bytes, fb = full0 + 8 * s;
-                        if (lane == 0) mbar_expect_tx_a(fb, tx);
-                        __syncwarp(m3);
-                        if (lane == 0) tma_load_4d_a(st, &tmK, fb, kc * p.KCH, h, row0, b);
-                        else if (lane == 1) { if (has1) tma_load_4d_a(st + a_bytes, &tmK, fb, kc * p.KCH, h, row0 + BM, b); }
-                        else tma_load_4d_a(st + 2 * a_bytes, &tmQ, fb, kc * p.KCH, h, col0, b);
+                        if (elect_one()) {
+                            mbar_expect_tx_a(fb, tx);
+                            tma_load_4d_a(st, &tmK, fb, kc * p.KCH, h, row0, b);
+                            tma_load_4d_a(st + 2 * a_bytes, &tmQ, fb, kc * p.KCH, h, col0, b);
+                            if (has1) tma_load_4d_a(st + a_bytes, &tmK, fb, kc * p.KCH, h, row0 + BM, b);
+                        }
                         if (++s == STAGES) { s = 0; ph ^= 1u; }
                     }
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             const uint32_t idesc = make_idesc_bf16_f32(BM, p.BN);
             const uint64_t dhi = kmajor_desc_hi(pitch);
             const int nk16 = p.KCH / 16;
@@ -160,23 +156,25 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
                 const bool has1 = pp * 2 * BM + BM < p.T;
                 for (int ct = 0; ct < p.n_col_tiles && ok; ++ct, ++tile) {
                     const uint32_t par = tile & 1u, u = tile >> 1;
-                    if (!mbar_wait_a(tempty0 + 8 * par, (u & 1u) ^ 1u, abort_flag)) { fail(abort_flag, 2); ok = false; break; }
+                    if (!mbar_wait_warp(tempty0 + 8 * par, (u & 1u) ^ 1u, abort_flag)) { fail(abort_flag, 2); ok = false; break; }
                     tc_fence_after_sync();
                     const uint32_t d0 = tmem_base + par * p.BNpad;
                     const uint32_t d1 = tmem_base + (2 + par) * p.BNpad;
                     for (int kc = 0; kc < p.KC; ++kc) {
-                        if (!mbar_wait_a(full0 + 8 * s, ph, abort_flag)) { fail(abort_flag, 3); ok = false; break; }
+                        if (!mbar_wait_warp(full0 + 8 * s, ph, abort_flag)) { fail(abort_flag, 3); ok = false; break; }
                         tc_fence_after_sync();
                         const uint32_t sa = st0 + s * stage_bytes;
                         const uint64_t a0 = dhi | (uint64_t)(sa >> 4);
                         const uint64_t a1 = dhi | (uint64_t)((sa + a_bytes) >> 4);
                         const uint64_t bd = dhi | (uint64_t)((sa + 2 * a_bytes) >> 4);
-                        mma_chunk(d0, a0, bd, idesc, nk16, kc != 0);
-                        if (has1) mma_chunk(d1, a1, bd, idesc, nk16, kc != 0);
-                        mma_commit_a(empty0 + 8 * s);
+                        if (elect_one()) {
+                            mma_chunk(d0, a0, bd, idesc, nk16, kc != 0);
+                            if (has1) mma_chunk(d1, a1, bd, idesc, nk16, kc != 0);
+                            mma_commit_a(empty0 + 8 * s);
+                        }
                         if (++s == STAGES) { s = 0; ph ^= 1u; }
                     }
-                    if (ok) mma_commit_a(tfull0 + 8 * par);
+                    if (ok && elect_one()) mma_commit_a(tfull0 + 8 * par);
                 }
             }
         }

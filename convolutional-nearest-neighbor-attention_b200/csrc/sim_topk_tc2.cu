@@ -125,7 +125,7 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     const uint32_t peer_abort = map_to_cta(smem_u32(const_cast<int*>(abort_flag)), peer);
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
             const uint32_t lead_full0 = map_to_cta(full0, 0);
             uint32_t s = 0, ph = 0;
             bool ok = true;
@@ -136,18 +136,20 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
                 for (int ct = 0; ct < p.n_col_tiles && ok; ++ct) {
                     const int col0 = ct * BN + (int)rank * BNH;
                     for (int kc = 0; kc < p.KC; ++kc) {
-                        if (!mbar_wait_a(empty0 + 8 * s, ph ^ 1u, abort_flag)) { fail(abort_flag, peer_abort, 21); ok = false; break; }
+                        if (!mbar_wait_warp(empty0 + 8 * s, ph ^ 1u, abort_flag)) { fail(abort_flag, peer_abort, 21); ok = false; break; }
                         const uint32_t st = st0 + s * STAGE_BYTES;
-                        if (rank == 0) mbar_expect_tx_a(full0 + 8 * s, 2 * STAGE_BYTES);
-                        tma_load_4d_pair(st, &tmK, lead_full0 + 8 * s, kc * KCH, h, row0, b);
-                        tma_load_4d_pair(st + A_BYTES, &tmQ, lead_full0 + 8 * s, kc * KCH, h, col0, b);
+                        if (elect_one()) {
+                            if (rank == 0) mbar_expect_tx_a(full0 + 8 * s, 2 * STAGE_BYTES);
+                            tma_load_4d_pair(st, &tmK, lead_full0 + 8 * s, kc * KCH, h, row0, b);
+                            tma_load_4d_pair(st + A_BYTES, &tmQ, lead_full0 + 8 * s, kc * KCH, h, col0, b);
+                        }
                         if (++s == NST) { s = 0; ph ^= 1u; }
                     }
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             const uint32_t idesc = make_idesc_bf16_f32(2 * BM, BN);
             const uint64_t dhi = kmajor_desc_hi(KCH * 2);
             const uint32_t peer_empty0 = map_to_cta(empty0, 1), peer_tfull0 = map_to_cta(tfull0, 1);
@@ -156,24 +158,26 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
             for (int unit = cluster_id; unit < p.n_units && ok; unit += n_clusters) {
                 for (int ct = 0; ct < p.n_col_tiles && ok; ++ct, ++tile) {
                     const uint32_t par = tile & 1u, u = tile >> 1;
-                    if (!mbar_wait_a(tempty0 + 8 * par, (u & 1u) ^ 1u, abort_flag)) { fail(abort_flag, peer_abort, 22); ok = false; break; }
+                    if (!mbar_wait_warp(tempty0 + 8 * par, (u & 1u) ^ 1u, abort_flag)) { fail(abort_flag, peer_abort, 22); ok = false; break; }
                     tc_fence_after_sync();
                     const uint32_t d = tmem_base + par * BN;
                     for (int kc = 0; kc < p.KC; ++kc) {
-                        if (!mbar_wait_a(full0 + 8 * s, ph, abort_flag)) { fail(abort_flag, peer_abort, 23); ok = false; break; }
+                        if (!mbar_wait_warp(full0 + 8 * s, ph, abort_flag)) { fail(abort_flag, peer_abort, 23); ok = false; break; }
                         tc_fence_after_sync();
                         const uint32_t sa = st0 + s * STAGE_BYTES;
                         const uint64_t ad = dhi | (uint64_t)((sa & 0x3FFFFu) >> 4);
                         const uint64_t bd = dhi | (uint64_t)(((sa + A_BYTES) & 0x3FFFFu) >> 4);
-                        mma_bf16_ss_pair(d, ad, bd, idesc, kc != 0);
-                        mma_bf16_ss_pair(d, ad + 2, bd + 2, idesc, 1);
-                        mma_bf16_ss_pair(d, ad + 4, bd + 4, idesc, 1);
-                        mma_bf16_ss_pair(d, ad + 6, bd + 6, idesc, 1);
-                        mma_commit_pair(empty0 + 8 * s);
-                        mma_commit_pair(peer_empty0 + 8 * s);
+                        if (elect_one()) {
+                            mma_bf16_ss_pair(d, ad, bd, idesc, kc != 0);
+                            mma_bf16_ss_pair(d, ad + 2, bd + 2, idesc, 1);
+                            mma_bf16_ss_pair(d, ad + 4, bd + 4, idesc, 1);
+                            mma_bf16_ss_pair(d, ad + 6, bd + 6, idesc, 1);
+                            mma_commit_pair(empty0 + 8 * s);
+                            mma_commit_pair(peer_empty0 + 8 * s);
+                        }
                         if (++s == NST) { s = 0; ph ^= 1u; }
                     }
-                    if (ok) {
+                    if (ok && elect_one()) {
                         mma_commit_pair(tfull0 + 8 * par);
                         mma_commit_pair(peer_tfull0 + 8 * par);
                     }
