@@ -9,12 +9,12 @@ namespace convnn {
 
 constexpr int kSelGroup = 128;    // threads per epilogue group = stride of the key staging buffer
 
-// Columns 0 .. W-1 of a row: insertion number j only touches the first j + 1 slots.
+// The first W columns of a row, from col0 on: insertion number j only touches the first j + 1 slots.
 template <int NSEL, int W, int J>
-__device__ __forceinline__ void prefix_insert(TopList<NSEL>& top, const float (&key)[W], bool row_ok, int left) {
+__device__ __forceinline__ void prefix_insert(TopList<NSEL>& top, const float (&key)[W], bool row_ok, int left, int col0) {
     if constexpr (J < W) {
-        if (row_ok && J < left) top.template insert_sorted_first<J>(key[J], J);
-        prefix_insert<NSEL, W, J + 1>(top, key, row_ok, left);
+        if (row_ok && J < left) top.template insert_sorted_first<J>(key[J], col0 + J);
+        prefix_insert<NSEL, W, J + 1>(top, key, row_ok, left, col0);
     }
 }
 
@@ -63,17 +63,17 @@ __device__ __forceinline__ void keys_of(float (&key)[W], const uint32_t (&acc)[W
 // qs points at the W column statistics of this chunk in shared memory (16-byte aligned, the same
 // for every lane: broadcast loads); cv holds the candidate token of column (32-aligned base +
 // lane).  P needs the fields metric, sampled and S (number of candidate columns).
-// FLOOR: keys at or below `floor` are known to lie outside the row's final list.
+// FLOOR: keys at or below `floor` are known to lie outside the row's final list.  first: the list's first column.
 template <int NSEL, int W, bool FLOOR = false, class P>
 __device__ __forceinline__ void consume(TopList<NSEL>& top, const uint32_t (&acc)[W], int col0, int lane_off,
                                         const float* qs, int cv, const P& p, int row, bool row_ok, float sentinel,
-                                        float* ks, float floor = 0.f) {
+                                        float* ks, float floor = 0.f, int first = 0) {
     float key[W];
     keys_of<W>(key, acc, lane_off, qs, cv, p, row, sentinel);
     const int left = p.S - col0;                       // valid columns from col0 on
-    if (col0 < 32) {
-        if (col0 == 0) {                               // the list is still filling up
-            prefix_insert<NSEL, W, 0>(top, key, row_ok, left);
+    if (col0 - first < 32) {
+        if (col0 == first) {                           // the list is still filling up
+            prefix_insert<NSEL, W, 0>(top, key, row_ok, left, col0);
         } else {
 #pragma unroll
             for (int j = 0; j < W; ++j)

@@ -20,6 +20,9 @@
 // keep the lower candidate column.  bfloat16 products are exact in fp32 and accumulation
 // is fp32, so the selection is as accurate as the float32 SIMT kernel on the same q, k.
 // Every mbarrier wait is bounded; on expiry the CTA latches a code and drains.
+//
+// Few units: up to eight CTAs of a cluster take a share of a unit's column tiles each, hand their rows' lists to one another through
+// distributed shared memory and merge 256 / split rows apiece.
 #include "common.cuh"
 #include "sm100.cuh"
 #include "toplist.cuh"
@@ -55,6 +58,9 @@ struct TcParams {
     int BNpad;        // TMEM columns per accumulator (power of two >= BN)
     int stages;       // shared-memory ring depth (<= MAX_STAGES)
     int n_pairs, n_col_tiles, n_units;
+    int split;        // CTAs of a cluster that share a unit's column tiles (then every cluster has one unit)
+    int tiles_each;   // column tiles per CTA
+    uint32_t ring_bytes;   // the ring's space, in which a split unit's lists are merged
     float sqrt_dk;
 };
 
@@ -74,7 +80,7 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     const uint32_t stage_bytes = 2 * a_bytes + b_bytes;
     const uint32_t STAGES = p.stages;
     uint8_t* stages = smem;                                            // [STAGES][A0 | A1 | B]
-    float* keybuf = reinterpret_cast<float*>(smem + STAGES * stage_bytes);   // [2 groups][CW][GROUP]
+    float* keybuf = reinterpret_cast<float*>(smem + p.ring_bytes);   // [2 groups][CW][GROUP]
     float* statbuf = keybuf + 2 * CW * GROUP;                                 // [8 warps][128] column statistics of the tile
     uint64_t* bars = reinterpret_cast<uint64_t*>(statbuf + 8 * 128);
     uint64_t* full = bars;
@@ -113,19 +119,23 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 
     const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty);
     const uint32_t st0 = smem_u32(stages);
+    const int rank = p.split > 1 ? (int)cluster_ctarank() : 0;
+    const int unit0 = (int)blockIdx.x / p.split, unit_step = (int)gridDim.x / p.split;
+    const int ct0 = rank * p.tiles_each, ct1 = min(p.n_col_tiles, ct0 + p.tiles_each);
+    float2* lists = reinterpret_cast<float2*>(stages);
 
     if (warp == 0) {
         {
             uint32_t s = 0, ph = 0;                  // ring slot and phase, advanced incrementally
             bool ok = true;
             chain_wait();
-            for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x) {
+            for (int unit = unit0; unit < p.n_units && ok; unit += unit_step) {
                 const int bh = unit / p.n_pairs, pp = unit - bh * p.n_pairs;
                 const int b = bh / p.H, h = bh - b * p.H;
                 const int row0 = pp * 2 * BM;
                 const bool has1 = row0 + BM < p.T;
                 const uint32_t tx = (has1 ? 2u : 1u) * a_bytes + b_bytes;
-                for (int ct = 0; ct < p.n_col_tiles && ok; ++ct) {
+                for (int ct = ct0; ct < ct1 && ok; ++ct) {
                     const int col0 = ct * p.BN;
                     for (int kc = 0; kc < p.KC; ++kc) {
                         ok = mbar_wait_warp(empty0 + 8 * s, ph ^ 1u, abort_flag);
@@ -151,10 +161,10 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
             uint32_t s = 0, ph = 0, tile = 0;
             bool ok = true;
             chain_wait();                            // (the budgets of its waits are for this kernel's work)
-            for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x) {
+            for (int unit = unit0; unit < p.n_units && ok; unit += unit_step) {
                 const int pp = unit % p.n_pairs;
                 const bool has1 = pp * 2 * BM + BM < p.T;
-                for (int ct = 0; ct < p.n_col_tiles && ok; ++ct, ++tile) {
+                for (int ct = ct0; ct < ct1 && ok; ++ct, ++tile) {
                     const uint32_t par = tile & 1u, u = tile >> 1;
                     if (!mbar_wait_warp(tempty0 + 8 * par, (u & 1u) ^ 1u, abort_flag)) { fail(abort_flag, 2); ok = false; break; }
                     tc_fence_after_sync();
@@ -188,7 +198,7 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         bool ok = true;
         chain_wait();
         chain_next();
-        for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x) {
+        for (int unit = unit0; unit < p.n_units && ok; unit += unit_step) {
             const int bh = unit / p.n_pairs, pp = unit - bh * p.n_pairs;
             const int row = pp * 2 * BM + grp * BM + r;
             const bool row_ok = row < p.T;
@@ -209,10 +219,10 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
                     fc[c4] = (p.sampled && c4 * 32 < p.BN) ? p.cand[cl] : -1;
                 }
             };
-            fetch(0, qv, cv);
-            for (int ct = 0; ct < p.n_col_tiles && ok; ++ct, ++tile) {
+            fetch(ct0, qv, cv);
+            for (int ct = ct0; ct < ct1 && ok; ++ct, ++tile) {
                 const uint32_t par = tile & 1u, u = tile >> 1;
-                if (ct + 1 < p.n_col_tiles) fetch(ct + 1, qn, cn);
+                if (ct + 1 < ct1) fetch(ct + 1, qn, cn);
                 ok = mbar_wait(&tfull[par], u & 1u, abort_flag);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) { if (lane == 0) fail(abort_flag, 4); break; }
@@ -238,12 +248,12 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
                             uint32_t acc[32];
                             tmem_ld_x32(taddr + c, acc);
                             tmem_ld_wait();
-                            consume<NSEL, 32>(top, acc, ct * p.BN + c, 0, sq + c, c1, p, row, row_ok, sentinel, ks);
+                            consume<NSEL, 32>(top, acc, ct * p.BN + c, 0, sq + c, c1, p, row, row_ok, sentinel, ks, 0.f, ct0 * p.BN);
                         } else {
                             uint32_t acc[16];
                             tmem_ld_x16(taddr + c, acc);
                             tmem_ld_wait();
-                            consume<NSEL, 16>(top, acc, ct * p.BN + c, c & 31, sq + c, c1, p, row, row_ok, sentinel, ks);
+                            consume<NSEL, 16>(top, acc, ct * p.BN + c, c & 31, sq + c, c1, p, row, row_ok, sentinel, ks, 0.f, ct0 * p.BN);
                         }
                     }
                 }
@@ -253,10 +263,82 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 #pragma unroll
                 for (int c4 = 0; c4 < 4; ++c4) { qv[c4] = qn[c4]; cv[c4] = cn[c4]; }
             }
-            if (ok && row_ok) {
+            if (p.split > 1) {                       // to the cluster: [slot][256 rows], where the operands were
+#pragma unroll
+                for (int s = 0; s < NSEL; ++s)
+                    lists[s * 2 * BM + grp * BM + r] = make_float2(top.v[s], __int_as_float(top.i[s]));
+            } else if (ok && row_ok) {
                 write_selection<NSEL>(top, p, ((long long)bh * p.T + row) * p.K, row, kst);
             }
         }
+    }
+
+    if (p.split > 1) {
+        // Every CTA takes 256 / split rows of the unit: their lists come over from the whole cluster, and a thread merges a row's.
+        // The lists' columns ascend with the rank, so that of equal keys the lower rank's goes first.
+        __syncthreads();
+        cluster_sync_all();
+        const int rows = 2 * BM / p.split, tid = (int)threadIdx.x - 64;
+        float2* all = lists + NSEL * 2 * BM;         // [rank][slot][rows]
+        if (tid >= 0) {
+            const int from = tid / rows, rr = tid - from * rows;
+            const uint32_t theirs = map_to_cta(smem_u32(lists + rank * rows + rr), (uint32_t)from);
+            float2 e[NSEL];
+#pragma unroll
+            for (int s = 0; s < NSEL; ++s)
+                asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(e[s].x), "=f"(e[s].y) : "r"(theirs + s * 2 * BM * 8) : "memory");
+#pragma unroll
+            for (int s = 0; s < NSEL; ++s) all[(from * NSEL + s) * rows + rr] = e[s];
+        }
+        __syncthreads();
+        const int bh = unit0 / p.n_pairs, pp = unit0 - bh * p.n_pairs, row = pp * 2 * BM + rank * rows + tid;
+        if (tid >= 0 && tid < rows && row < p.T && !*abort_flag) {
+            const float kst = p.metric != CONVNN_MATMUL ? p.kstat[(long long)bh * p.T + row] : 1.0f;
+            long long at = ((long long)bh * p.T + row) * p.K;
+            if (p.sampled) {
+                p.idx[at] = row;
+                p.val[at++] = 1.0f;
+            }
+            constexpr int MAX_SPLIT = 8;
+            float2 head[MAX_SPLIT];
+            int next[MAX_SPLIT];
+#pragma unroll
+            for (int l = 0; l < MAX_SPLIT; ++l) {
+                next[l] = 1;
+                head[l] = l < p.split ? all[l * NSEL * rows + tid] : make_float2(-CUDART_INF_F, 0.f);
+            }
+#pragma unroll 1
+            for (int s = 0; s < p.nsel; ++s, ++at) {
+                float2 best = head[0];
+                int from = 0;
+#pragma unroll
+                for (int l = 1; l < MAX_SPLIT; ++l)
+                    if (head[l].x > best.x) { best = head[l]; from = l; }
+                // (the last place of a list is taken by the last round at the earliest)
+                int pos = 0;
+#pragma unroll
+                for (int l = 0; l < MAX_SPLIT; ++l) pos = l == from ? next[l] : pos;
+                const float2 after = all[(from * NSEL + min(pos, NSEL - 1)) * rows + tid];
+#pragma unroll
+                for (int l = 0; l < MAX_SPLIT; ++l) {
+                    head[l] = l == from ? after : head[l];
+                    next[l] += l == from ? 1 : 0;
+                }
+                int tok = __float_as_int(best.y);
+                float v;
+                if (p.metric == CONVNN_COSINE) v = best.x * kst;
+                else if (p.metric == CONVNN_MATMUL) v = best.x / p.sqrt_dk;
+                else v = sqrtf(fmaxf(kst - best.x, 0.f));
+                if (p.sampled) {
+                    tok = p.cand[tok];
+                    if (tok == row) v = (p.metric == CONVNN_EUCLIDEAN) ? 1.1f : -0.1f;
+                }
+                p.idx[at] = tok;
+                p.val[at] = v;
+            }
+        }
+        __syncthreads();
+        cluster_sync_all();                          // nobody reads this CTA's lists any more
     }
 
     tc_fence_before_sync();
@@ -289,11 +371,23 @@ bool sim_topk_tc_supported(const convnn_desc* d, const Dims& dm, const void* q, 
     return d->dtype == CONVNN_BF16 && dm.Cp % 16 == 0 && aligned16(q) && aligned16(k);
 }
 
+// CTAs that share the columns of a unit where the units alone leave most SMs idle (a unit's time goes with its columns; us, one CTA per
+// unit, a cluster): 2 x 2048 x 2048 x 256, K = 25 125, 85; 4 x 1366 x 632 x 192, K = 9 47, 23; 577 x 577 x 384 34, 15; 14 x 624 x 624 x 256, K = 16
+// 47, 36; 2048 x 2048 x 256, K = 32 149, 53.  Lists and their merge cost about 3 us: not for less than 128 columns each.
+static int split_of(const Dims& dm, int n_units) {
+    int split = 1;
+    while (split < 8 && n_units * 2 * split <= device_sms() && dm.S >= 128 * split) split *= 2;
+    return split;
+}
+
 int launch_sim_topk_tc(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
                        const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st) {
     if (sim_topk_rows_wanted(dm)) return launch_sim_topk_rows(d, dm, q, k, qstat, kstat, cand, idx, val, st);
     if (sim_topk_short_wanted(dm)) return launch_sim_topk_short(d, dm, q, k, qstat, kstat, cand, idx, val, st);
-    if (sim_topk_tc2_wanted(d, dm)) return launch_sim_topk_tc2(d, dm, q, k, qstat, kstat, cand, idx, val, st);
+    // (a pair of SMs per unit against a cluster of up to eight: 4096 x 4096 x 768, K = 9 85, 71 us; 2 x 4168 x 4168 x 256 83, 89; K = 16, 2 x
+    // 4042 x 4042 x 384 87, 63; heads of up to 192 channels stay with the pairs)
+    const bool few = dm.Cp > 192 && (dm.nsel > 12 ? 4ll : 8ll) * dm.B * dm.H * ((dm.T + 2 * BM - 1) / (2 * BM)) <= device_sms();
+    if (!few && sim_topk_tc2_wanted(d, dm)) return launch_sim_topk_tc2(d, dm, q, k, qstat, kstat, cand, idx, val, st);
     TcParams p{};
     p.qstat = qstat; p.kstat = kstat; p.cand = cand; p.idx = idx; p.val = val;
     p.T = dm.T; p.S = dm.S; p.H = dm.H; p.K = dm.K; p.nsel = dm.nsel; p.metric = d->metric; p.sampled = d->sampled;
@@ -307,12 +401,14 @@ int launch_sim_topk_tc(const convnn_desc* d, const Dims& dm, const void* q, cons
     const bool small_cfg = dm.nsel <= 12 && (dm.Cp <= 256 || (dm.Cp <= 512 && dm.T <= 512));
     const int bn_cap = small_cfg ? 64 : 128;
     p.stages = small_cfg ? 2 : 3;
-    const int ntile = (dm.S + bn_cap - 1) / bn_cap;
+    p.n_pairs = (dm.T + 2 * BM - 1) / (2 * BM);
+    p.n_units = dm.B * dm.H * p.n_pairs;
+    p.split = split_of(dm, p.n_units);
+    const int ntile = ((dm.S + bn_cap - 1) / bn_cap + p.split - 1) / p.split * p.split;
     p.BN = (((dm.S + ntile - 1) / ntile) + 15) / 16 * 16;
     p.BNpad = pow2_at_least(p.BN, 32);
-    p.n_pairs = (dm.T + 2 * BM - 1) / (2 * BM);
     p.n_col_tiles = (dm.S + p.BN - 1) / p.BN;
-    p.n_units = dm.B * dm.H * p.n_pairs;
+    p.tiles_each = (p.n_col_tiles + p.split - 1) / p.split;
     p.sqrt_dk = (float)sqrt((double)dm.dk);
 
     const int pitch = p.KCH * 2;
@@ -327,7 +423,8 @@ int launch_sim_topk_tc(const convnn_desc* d, const Dims& dm, const void* q, cons
     if (!encode_tensor_map_bf16(&tmQ, q, 4, dimsQ, strQ, boxQ, pitch)) return CONVNN_E_CUDA;
 
     const int cw = small_cfg ? 16 : 32;
-    const size_t smem = 1024 + (size_t)p.stages * (2 * BM + p.BN) * pitch + 2 * cw * GROUP * sizeof(float) +
+    const size_t ring = (size_t)p.stages * (2 * BM + p.BN) * pitch;
+    const size_t smem = 1024 + ring + 2 * cw * GROUP * sizeof(float) +
                         8 * 128 * sizeof(float) + (2 * MAX_STAGES + 4) * 8 + 16;
     const int sms = device_sms();
     const int ctas = sms * (small_cfg ? 2 : 1);
@@ -336,8 +433,24 @@ int launch_sim_topk_tc(const convnn_desc* d, const Dims& dm, const void* q, cons
 #define CONVNN_TC_LAUNCH2(N, MINB, CWV)                                                                \
     do {                                                                                               \
         auto kern = sim_topk_tc_kernel<N, MINB, CWV>;                                                  \
-        CONVNN_ENSURE_SMEM(kern, smem);                                                            \
-        launch_chained(kern, grid, NTHREADS, smem, st, tmK, tmQ, p);                                               \
+        /* (the merge's lists and their gathered copy lie where the ring was) */                       \
+        constexpr size_t merge = 2 * (size_t)N * 2 * BM * 8;                                           \
+        const size_t need = p.split > 1 && merge > ring ? smem + merge - ring : smem;                  \
+        p.ring_bytes = (uint32_t)(ring + need - smem);                                                 \
+        CONVNN_ENSURE_SMEM(kern, need);                                                            \
+        if (p.split > 1) {                                                                             \
+            cudaLaunchConfig_t cfg{};                                                                  \
+            cudaLaunchAttribute attr[2];                                                               \
+            attr[0].id = cudaLaunchAttributeClusterDimension;                                          \
+            attr[0].val.clusterDim.x = p.split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1; \
+            attr[1] = chained_attribute(st);                                                           \
+            cfg.gridDim = dim3(p.n_units * p.split); cfg.blockDim = dim3(NTHREADS);                    \
+            cfg.dynamicSmemBytes = need; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 2;          \
+            const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmK, tmQ, p);                         \
+            if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "sim_topk_tc launch: %s", cudaGetErrorString(e)); \
+        } else {                                                                                       \
+            launch_chained(kern, grid, NTHREADS, need, st, tmK, tmQ, p);                               \
+        }                                                                                              \
     } while (0)
 #define CONVNN_TC_LAUNCH(N)                            \
     do {                                               \

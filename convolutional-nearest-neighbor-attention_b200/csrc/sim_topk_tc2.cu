@@ -258,7 +258,7 @@ sim_topk_tc2_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
                             }
                             tmem_ld_wait();
                             consume<NSEL, 32, SHARE>(top, acc, cbase + c4 * 32, 0, sq + c4 * 32, cv[c4], p, row, row_ok,
-                                                    sentinel, ks, floor);
+                                                    sentinel, ks, floor, NSEL > 12 ? chalf * BNH : 0);
                             if constexpr (SHARE) {
                                 my_rank = chalf == 0 ? top.v[R0 - 1] : top.v[R1 - 1];
                                 *own_rank = ((unsigned long long)(it + 1) << 32) | __float_as_uint(my_rank);

@@ -77,3 +77,37 @@ def test_unusable_keys(T, S, dk, K, columns):
     ranked = dot.sort(dim=1, descending=True, stable=True)
     col = torch.where(ranked.values[:, :n] > -float("inf"), ranked.indices[:, :n], 0)
     assert torch.equal(idx[0, 0, :, first:].long(), col if cand is None else cand.long()[col])
+
+
+# Few units: two, four and eight CTAs per unit, some without a column tile, ragged last tiles, rows that end inside a CTA's share of the
+# merge, lists longer than a CTA's share of good columns ("rising": all of the best lie in the last CTA's), ties and NaN.
+@pytest.mark.parametrize("B,T,S,H,dk", [(1, 300, 300, 1, 64), (2, 577, 577, 1, 384), (1, 1040, 1040, 1, 256), (3, 1020, 344, 1, 512), (5, 700, 700, 2, 16),
+                                        (1, 2600, 1100, 1, 256), (1, 2048, 2048, 1, 32)])
+@pytest.mark.parametrize("K", [2, 5, 9, 12, 16, 25, 32])
+@pytest.mark.parametrize("values", ["ties", "many", "rising", "nan"])
+def test_columns_shared_by_a_cluster(B, T, S, H, dk, K, values):
+    g = torch.Generator(device=DEV).manual_seed(T + S + K)
+    sampled = S != T
+    top = 1 if values == "ties" else 11
+    q, k = (torch.randint(-top, top + 1, (B, r, H, dk), device=DEV, generator=g).float() for r in (S, T))
+    if values == "rising":
+        q[..., 0] = (torch.arange(S, device=DEV) // 8).float().view(1, S, 1)
+        k[..., 0] = 16.0
+    if values == "nan":
+        q[:, ::3] = float("nan")
+        q[0, 3:S - 2] = float("nan")
+    spec = ops.LayerSpec(H * dk, H, K, "spatial" if sampled else "all", "matmul", "depthwise", True, False, T)
+    cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if sampled else None
+    qb, kb = q.bfloat16(), k.bfloat16()
+    call = lambda: ops.sim_topk(spec, qb, kb, None, None, cand)
+    assert any("sim_topk_tc_kernel" in name for name in launches(call))
+    idx, val = call()
+    key = torch.einsum("bthc,bshc->bhts", kb.double(), qb.double()).float()        # whole numbers below 2^24: exact
+    n = K - 1 if sampled else K
+    if sampled:
+        own = cand.view(1, S).long() == torch.arange(T, device=DEV).view(T, 1)
+        key = key.masked_fill(own, -0.1 * dk ** 0.5)
+    key = torch.where(key.isnan(), torch.full_like(key, -float("inf")), key)
+    ranked = key.sort(dim=-1, descending=True, stable=True)
+    col = torch.where(ranked.values[..., :n] > -float("inf"), ranked.indices[..., :n], 0)
+    assert torch.equal(idx.long()[..., K - n:], col if cand is None else cand.long()[col])
