@@ -9,7 +9,7 @@
 // never exists in memory, and exact ties go to the lower candidate column.
 //
 // Bound by the shared-memory reads that feed the fp32 pipes (64 images of 197 x 192: L1 68 % busy, warps wait for shared
-// memory most).  One thread per row with its 64 columns in registers, before, read every operand value of a column from
+// memory most), and by the insertions of long lists.  One thread per row with its 64 columns in registers, before, read every operand value of a column from
 // shared memory once per row: 97 us per layer at 32 x 65 tokens x 192 channels.
 //
 // Ranking keys (larger is better) and the values reported for the survivors:
@@ -28,6 +28,7 @@
 #include "common.cuh"
 #include "f32x2.cuh"
 #include "toplist.cuh"
+#include "cluster_lists.cuh"
 
 namespace convnn {
 namespace simt_topk {
@@ -37,11 +38,12 @@ constexpr int CB = 64;      // candidate columns per tile
 constexpr int BK = 16;      // channels per step
 constexpr int LK = CB + 4;  // row stride of the key tile: 16-byte rows that fall into different banks
 
-__host__ __device__ constexpr int tile_floats(int rb) { return 2 * BK * (rb + 4) + 2 * BK * (CB + 4) + rb * LK; }
+__host__ __device__ constexpr int tile_floats(int rb) { return 2 * BK * (rb + 4) + 2 * BK * (CB + 4) + rb * LK + NT; }
 __host__ __device__ constexpr int merge_floats(int rb, int kcap) { return 2 * kcap * rb * (NT / rb - 1); }
-__host__ __device__ constexpr int smem_bytes(int rb, int kcap) {
-    const int a = tile_floats(rb), b = merge_floats(rb, kcap);
-    return 4 * (a > b ? a : b);
+__host__ __device__ constexpr int cluster_floats(int rb, int kcap) { return 4 * kcap * rb; }
+__host__ __device__ constexpr int smem_bytes(int rb, int kcap, bool split) {
+    const int a = tile_floats(rb), b = merge_floats(rb, kcap), c = split ? cluster_floats(rb, kcap) : 0;
+    return 4 * (a > b ? (a > c ? a : c) : (b > c ? b : c));
 }
 
 __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -65,7 +67,7 @@ __global__ void __launch_bounds__(NT) sim_topk_simt_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const float* __restrict__ qstat,
     const float* __restrict__ kstat, const int32_t* __restrict__ cand, int32_t* __restrict__ idx,
     float* __restrict__ val, int T_, int S, int H, int Cp, int K, int nsel, int metric, int sampled,
-    float sqrt_dk, int vec) {
+    float sqrt_dk, int vec, int split) {
     chain_wait();               // (and no early start for the next one, see chain_begin_for())
     constexpr int TM = RB / 16, RG = TM / 4;              // 16 x 16 threads, TM x 4 dot products each
     constexpr int LA = RB + 4, LB = CB + 4;
@@ -75,6 +77,8 @@ __global__ void __launch_bounds__(NT) sim_topk_simt_kernel(
     float* As = sm;                                       // [2][BK][LA]
     float* Bs = As + 2 * BK * LA;                         // [2][BK][LB]
     float* keys = Bs + 2 * BK * LB;                       // [RB][LK]
+    volatile float* ranks = keys + RB * LK;               // [TPR][RB]: the RANK-th key of every list, see below
+    constexpr int RANK = (KCAP + TPR - 1) / TPR;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int bh = blockIdx.y, b = bh / H, h = bh - b * H;
@@ -105,7 +109,9 @@ __global__ void __launch_bounds__(NT) sim_topk_simt_kernel(
     TopList<KCAP> top;
     top.init();
 
-    const int ksteps = (Cp + BK - 1) / BK, ntiles = (S + CB - 1) / CB;
+    // (a cluster of `split` CTAs shares the tiles: blockIdx.z is the rank)
+    const int ksteps = (Cp + BK - 1) / BK, all_tiles = (S + CB - 1) / CB, each = (all_tiles + split - 1) / split;
+    const int first = (int)blockIdx.z * each, ntiles = min(all_tiles, first + each);
     float4 av[NA], bv;
     auto fetch = [&](int ct, int ks) {
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -127,11 +133,12 @@ __global__ void __launch_bounds__(NT) sim_topk_simt_kernel(
         d[0] = bv.x; d[LB] = bv.y; d[2 * LB] = bv.z; d[3 * LB] = bv.w;
     };
 
-    fetch(0, 0);
+    ranks[tid] = -CUDART_INF_F;
+    fetch(first, 0);
     stage(0);
     __syncthreads();
     int buf = 0;
-    for (int ct = 0; ct < ntiles; ++ct) {
+    for (int ct = first; ct < ntiles; ++ct) {
         f32x2 acc[TM][2];
 #pragma unroll
         for (int i = 0; i < TM; ++i) acc[i][0] = acc[i][1] = 0ull;
@@ -186,16 +193,45 @@ __global__ void __launch_bounds__(NT) sim_topk_simt_kernel(
                 }
                 __syncthreads();
                 const int s0 = ct * CB + sq * CW;
-                if (row_ok) {
+                const float* kr = keys + srow * LK + sq * CW;
+                if (ct == first) {                            // the list is filling up
+                    if (row_ok) {
 #pragma unroll 4
+                        for (int j4 = 0; j4 < CW; j4 += 4) {
+                            const float4 v = *reinterpret_cast<const float4*>(kr + j4);
+                            const float kv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (s0 + j4 + j < S && kv[j] > top.worst()) top.insert_sorted(kv[j], s0 + j4 + j);
+                        }
+                    }
+                } else {
+                    // The columns that enter: those above this list's last key and not below the smallest of the lists' RANK-th keys,
+                    // which at least KCAP keys of the row reach (the others' may be a tile old: they only grow).  They are taken one per
+                    // lane and step, whichever columns the lanes are at.
+                    float floor = ranks[srow];
+#pragma unroll
+                    for (int l = 1; l < TPR; ++l) floor = fminf(floor, ranks[l * RB + srow]);
+                    uint32_t mask = 0;
+#pragma unroll
                     for (int j4 = 0; j4 < CW; j4 += 4) {
-                        const float4 v = *reinterpret_cast<const float4*>(keys + srow * LK + sq * CW + j4);
+                        const float4 v = *reinterpret_cast<const float4*>(kr + j4);
                         const float kv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            if (s0 + j4 + j < S && kv[j] > top.worst()) top.insert_sorted(kv[j], s0 + j4 + j);
+                        for (int j = 0; j < 4; ++j) mask |= kv[j] > top.worst() && kv[j] >= floor ? 1u << (j4 + j) : 0u;
+                    }
+                    if (S - s0 < CW) mask &= S > s0 ? (1u << (S - s0)) - 1u : 0u;
+                    if (!row_ok) mask = 0;
+                    const int steps = __reduce_max_sync(0xffffffffu, __popc(mask));
+#pragma unroll 1
+                    for (int n = 0; n < steps; ++n) {
+                        const int j = mask ? __ffs(mask) - 1 : 0;
+                        const float key = kr[j];
+                        if (mask && key > top.worst()) top.insert_sorted(key, s0 + j);
+                        mask &= mask - 1;
                     }
                 }
+                ranks[tid] = top.v[RANK - 1];
             }
             if (more) {
                 stage(buf ^ 1);
@@ -216,11 +252,24 @@ __global__ void __launch_bounds__(NT) sim_topk_simt_kernel(
         }
     }
     __syncthreads();
-    if (sq > 0 || !row_ok) return;
-    for (int l = 0; l < (TPR - 1) * KCAP; ++l) {
-        const float key = mk[l * RB + srow];
-        if (key >= top.worst() && key > -CUDART_INF_F) top.insert_ordered(key, mc[l * RB + srow]);
+    if (sq == 0 && row_ok) {
+        for (int l = 0; l < (TPR - 1) * KCAP; ++l) {
+            const float key = mk[l * RB + srow];
+            if (key >= top.worst() && key > -CUDART_INF_F) top.insert_ordered(key, mc[l * RB + srow]);
+        }
     }
+    if (split > 1) {
+        float2* lists = reinterpret_cast<float2*>(sm);
+        __syncthreads();
+        if (sq == 0) {
+#pragma unroll
+            for (int s = 0; s < KCAP; ++s) lists[s * RB + srow] = make_float2(top.v[s], __int_as_float(top.i[s]));
+        }
+        const ListOutput o{kst_row, cand, idx, val, T_, K, nsel, metric, sampled, sqrt_dk};
+        merge_cluster_lists<KCAP>(lists, lists + KCAP * RB, RB, split, (int)blockIdx.z, tid, row0, ((long long)b * H + h) * T_ + row0, true, o);
+        return;
+    }
+    if (sq > 0 || !row_ok) return;
 
     const float kst = kst_row ? kst_row[row] : 0.f;
     const long long obase = (((long long)b * H + h) * T_ + row) * K;
@@ -250,16 +299,40 @@ __global__ void __launch_bounds__(NT) sim_topk_simt_kernel(
     }
 }
 
+// CTAs that share a block's columns where the blocks alone leave room: one CTA of 128 rows fits an SM, two of 64 (us, float32, one CTA per block, a cluster: 577 x
+// 577 x 384 209, 75; 8 x 500 x 500 x 64 48, 33; 5000 x 5000 x 193, K = 25 1196, 880; 9363 x 9363 x 192 1467, 1228 with 64 rows).
+inline int split_of(const Dims& dm, int rb) {
+    const long long ctas = (long long)dm.B * dm.H * ((dm.T + rb - 1) / rb);
+    int split = 1;
+    while (split < MAX_SPLIT && ctas * 2 * split <= (rb == 128 ? 1ll : 2ll) * device_sms() && dm.S >= 2 * CB * 2 * split) split *= 2;
+    return split;
+}
+
 template <typename T, int KCAP, int RB>
 int launch(const convnn_desc* d, const Dims& dm, const void* q, const void* k, const float* qstat,
            const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st) {
-    const size_t smem = smem_bytes(RB, KCAP);
+    const int split = split_of(dm, RB);
+    const size_t smem = smem_bytes(RB, KCAP, split > 1);
     auto kern = sim_topk_simt_kernel<T, KCAP, RB>;
     CONVNN_ENSURE_SMEM(kern, smem);
     const int vec = dm.Cp % 4 == 0 && aligned16(q) && aligned16(k);
+    if (split > 1) {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = split;
+        attr[1] = chained_attribute(st);
+        cfg.gridDim = dim3((dm.T + RB - 1) / RB, dm.B * dm.H, split); cfg.blockDim = dim3(NT);
+        cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 2;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<const T*>(q), static_cast<const T*>(k), qstat, kstat, cand, idx, val,
+                                                 dm.T, dm.S, dm.H, dm.Cp, dm.K, dm.nsel, (int)d->metric, (int)d->sampled,
+                                                 (float)sqrt((double)dm.dk), vec, split);
+        if (e != cudaSuccess) return set_error(CONVNN_E_CUDA, "sim_topk_simt launch: %s", cudaGetErrorString(e));
+        return CONVNN_OK;
+    }
     launch_late(sizeof(T) == 4 || d->coord, kern, dim3((dm.T + RB - 1) / RB, dm.B * dm.H), NT, smem, st,
         static_cast<const T*>(q), static_cast<const T*>(k), qstat, kstat, cand, idx, val, dm.T, dm.S, dm.H, dm.Cp, dm.K,
-        dm.nsel, d->metric, d->sampled, (float)sqrt((double)dm.dk), vec);
+        dm.nsel, d->metric, d->sampled, (float)sqrt((double)dm.dk), vec, 1);
     CONVNN_CHECK_LAUNCH("sim_topk_simt");
     return CONVNN_OK;
 }
@@ -272,7 +345,8 @@ struct Blocks {
 };
 inline Blocks blocks_of(const Dims& dm) {
     const long long bh = (long long)dm.B * dm.H, wide = (dm.T + 127) / 128 * bh;
-    if (wide >= device_sms() && ((dm.T + 127) / 128) * 128 <= ((dm.T + 63) / 64) * 64 * 5 / 4) return {128, wide};
+    const long long shares = dm.S > 256 ? split_of(dm, 128) : 1;
+    if (wide * shares * (shares > 1 ? 2 : 1) >= device_sms() && ((dm.T + 127) / 128) * 128 <= ((dm.T + 63) / 64) * 64 * 5 / 4) return {128, wide};
     return {64, (dm.T + 63) / 64 * bh};
 }
 

@@ -27,6 +27,7 @@
 #include "sm100.cuh"
 #include "toplist.cuh"
 #include "sim_topk_select.cuh"
+#include "cluster_lists.cuh"
 
 namespace convnn {
 
@@ -274,71 +275,10 @@ sim_topk_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     }
 
     if (p.split > 1) {
-        // Every CTA takes 256 / split rows of the unit: their lists come over from the whole cluster, and a thread merges a row's.
-        // The lists' columns ascend with the rank, so that of equal keys the lower rank's goes first.
-        __syncthreads();
-        cluster_sync_all();
-        const int rows = 2 * BM / p.split, tid = (int)threadIdx.x - 64;
-        float2* all = lists + NSEL * 2 * BM;         // [rank][slot][rows]
-        if (tid >= 0) {
-            const int from = tid / rows, rr = tid - from * rows;
-            const uint32_t theirs = map_to_cta(smem_u32(lists + rank * rows + rr), (uint32_t)from);
-            float2 e[NSEL];
-#pragma unroll
-            for (int s = 0; s < NSEL; ++s)
-                asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(e[s].x), "=f"(e[s].y) : "r"(theirs + s * 2 * BM * 8) : "memory");
-#pragma unroll
-            for (int s = 0; s < NSEL; ++s) all[(from * NSEL + s) * rows + rr] = e[s];
-        }
-        __syncthreads();
-        const int bh = unit0 / p.n_pairs, pp = unit0 - bh * p.n_pairs, row = pp * 2 * BM + rank * rows + tid;
-        if (tid >= 0 && tid < rows && row < p.T && !*abort_flag) {
-            const float kst = p.metric != CONVNN_MATMUL ? p.kstat[(long long)bh * p.T + row] : 1.0f;
-            long long at = ((long long)bh * p.T + row) * p.K;
-            if (p.sampled) {
-                p.idx[at] = row;
-                p.val[at++] = 1.0f;
-            }
-            constexpr int MAX_SPLIT = 8;
-            float2 head[MAX_SPLIT];
-            int next[MAX_SPLIT];
-#pragma unroll
-            for (int l = 0; l < MAX_SPLIT; ++l) {
-                next[l] = 1;
-                head[l] = l < p.split ? all[l * NSEL * rows + tid] : make_float2(-CUDART_INF_F, 0.f);
-            }
-#pragma unroll 1
-            for (int s = 0; s < p.nsel; ++s, ++at) {
-                float2 best = head[0];
-                int from = 0;
-#pragma unroll
-                for (int l = 1; l < MAX_SPLIT; ++l)
-                    if (head[l].x > best.x) { best = head[l]; from = l; }
-                // (the last place of a list is taken by the last round at the earliest)
-                int pos = 0;
-#pragma unroll
-                for (int l = 0; l < MAX_SPLIT; ++l) pos = l == from ? next[l] : pos;
-                const float2 after = all[(from * NSEL + min(pos, NSEL - 1)) * rows + tid];
-#pragma unroll
-                for (int l = 0; l < MAX_SPLIT; ++l) {
-                    head[l] = l == from ? after : head[l];
-                    next[l] += l == from ? 1 : 0;
-                }
-                int tok = __float_as_int(best.y);
-                float v;
-                if (p.metric == CONVNN_COSINE) v = best.x * kst;
-                else if (p.metric == CONVNN_MATMUL) v = best.x / p.sqrt_dk;
-                else v = sqrtf(fmaxf(kst - best.x, 0.f));
-                if (p.sampled) {
-                    tok = p.cand[tok];
-                    if (tok == row) v = (p.metric == CONVNN_EUCLIDEAN) ? 1.1f : -0.1f;
-                }
-                p.idx[at] = tok;
-                p.val[at] = v;
-            }
-        }
-        __syncthreads();
-        cluster_sync_all();                          // nobody reads this CTA's lists any more
+        const int bh = unit0 / p.n_pairs, pp = unit0 - bh * p.n_pairs;
+        const ListOutput o{p.kstat ? p.kstat + (long long)bh * p.T : nullptr, p.cand, p.idx, p.val, p.T, p.K, p.nsel, p.metric, p.sampled, p.sqrt_dk};
+        merge_cluster_lists<NSEL>(lists, lists + NSEL * 2 * BM, 2 * BM, p.split, rank, (int)threadIdx.x - 64, pp * 2 * BM,
+                                  (long long)bh * p.T + pp * 2 * BM, !*abort_flag, o);
     }
 
     tc_fence_before_sync();
@@ -376,7 +316,7 @@ bool sim_topk_tc_supported(const convnn_desc* d, const Dims& dm, const void* q, 
 // 47, 36; 2048 x 2048 x 256, K = 32 149, 53.  Lists and their merge cost about 3 us: not for less than 128 columns each.
 static int split_of(const Dims& dm, int n_units) {
     int split = 1;
-    while (split < 8 && n_units * 2 * split <= device_sms() && dm.S >= 128 * split) split *= 2;
+    while (split < MAX_SPLIT && n_units * 2 * split <= device_sms() && dm.S >= 128 * split) split *= 2;
     return split;
 }
 

@@ -85,7 +85,7 @@ def test_unusable_keys(T, S, dk, K, columns):
                                         (1, 2600, 1100, 1, 256), (1, 2048, 2048, 1, 32)])
 @pytest.mark.parametrize("K", [2, 5, 9, 12, 16, 25, 32])
 @pytest.mark.parametrize("values", ["ties", "many", "rising", "nan"])
-def test_columns_shared_by_a_cluster(B, T, S, H, dk, K, values):
+def test_columns_shared_by_a_cluster(B, T, S, H, dk, K, values, dtype=torch.bfloat16, kernel="sim_topk_tc_kernel"):
     g = torch.Generator(device=DEV).manual_seed(T + S + K)
     sampled = S != T
     top = 1 if values == "ties" else 11
@@ -98,9 +98,9 @@ def test_columns_shared_by_a_cluster(B, T, S, H, dk, K, values):
         q[0, 3:S - 2] = float("nan")
     spec = ops.LayerSpec(H * dk, H, K, "spatial" if sampled else "all", "matmul", "depthwise", True, False, T)
     cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if sampled else None
-    qb, kb = q.bfloat16(), k.bfloat16()
+    qb, kb = q.to(dtype), k.to(dtype)
     call = lambda: ops.sim_topk(spec, qb, kb, None, None, cand)
-    assert any("sim_topk_tc_kernel" in name for name in launches(call))
+    assert any(kernel in name for name in launches(call))
     idx, val = call()
     key = torch.einsum("bthc,bshc->bhts", kb.double(), qb.double()).float()        # whole numbers below 2^24: exact
     n = K - 1 if sampled else K
@@ -111,3 +111,11 @@ def test_columns_shared_by_a_cluster(B, T, S, H, dk, K, values):
     ranked = key.sort(dim=-1, descending=True, stable=True)
     col = torch.where(ranked.values[..., :n] > -float("inf"), ranked.indices[..., :n], 0)
     assert torch.equal(idx.long()[..., K - n:], col if cand is None else cand.long()[col])
+
+
+# The same on the fp32 pipes: blocks of 64 and of 128 rows, two to eight CTAs each, widths that are no multiple of four.
+@pytest.mark.parametrize("B,T,S,H,dk", [(1, 300, 300, 1, 33), (2, 577, 577, 1, 64), (1, 1040, 1040, 1, 48), (1, 2100, 700, 1, 20), (2, 1300, 1300, 1, 64)])
+@pytest.mark.parametrize("K", [4, 9, 16, 25, 32])
+@pytest.mark.parametrize("values", ["ties", "many", "rising", "nan"])
+def test_columns_shared_by_a_cluster_float32(B, T, S, H, dk, K, values):
+    test_columns_shared_by_a_cluster(B, T, S, H, dk, K, values, torch.float32, "sim_topk_simt_kernel")
