@@ -288,9 +288,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t sA0 = smem_u32(sA), sB0 = smem_u32(sB);
 
     if (warp == 0) {
-        // One thread can start a TMA operation only every ~0.3 us, while operations started by different lanes overlap: a first
-        // tile of few chunks, all of which its products wait for, is requested by as many lanes (a small GEMM is little more
-        // than that), the rest by lane 0.  With more chunks the first would land later (K = 384 0.6 us per launch).
+        // A first tile of few chunks, all of which its products wait for, is requested by as many lanes, whose requests overlap (a small
+        // GEMM is little more than that; by one lane 1 to 4 % of a ViT-Tiny forward), the rest by an elected one.  With more
+        // chunks the first would land later (K = 384 0.6 us per launch).
         const uint32_t tx = (a_bytes + (p.wstat ? 0u : b_bytes)) * (PAIR ? 2u : 1u);
         const uint32_t lead_full0 = PAIR ? map_to_cta(full0, 0) : full0;
         auto load_a = [&](uint32_t slot, int kc, int m0) {
