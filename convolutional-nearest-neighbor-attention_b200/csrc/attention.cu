@@ -326,20 +326,21 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     chain_leave(BESIDE);
 }
 
-// R query rows of one (batch, head) per CTA, for float32 and head widths that the tensor-core kernel does not take.
+// R = 8 TR query rows of one (batch, head) per CTA, for float32 and head widths that the tensor-core kernel does not take.
 //
-//   scores   a thread owns R / 8 rows x 4 keys; K passes through shared memory in chunks of 32 channels x 128 keys, the next chunk in
-//            registers meanwhile
+//   scores   a thread owns TR rows x up to seven keys (lane, lane + 32, ...); q and K pass through shared memory in chunks of 32
+//            channels, the next chunk in registers meanwhile
 //   softmax  a warp per row
-//   output   a thread owns R / 8 rows x 4 channels; V passes in chunks of 32 tokens x 128 channels
+//   output   a thread owns TR rows x up to seven channels; V passes in chunks of 32 tokens
 //
-// Every sum runs in the order of the kernel for longer sequences below (channels, tokens and the lanes' partial sums ascending), so
-// that both give the same bits.  What bounds it: shared-memory reads, two 16-byte ones per 16 multiply-adds, and at few rows the chain of
-// chunks.  us with the four projections, one warp per row reading K a word at a time -> this kernel: 6 x 65 x 192, one head, bfloat16 98 ->
-// 30; 64 x 197 x 192 2090 -> 170; 8 x 197 x 384 806 -> 91; float32, 8 x 197, 3 heads of 32 171 -> 52; 16 x 197, 12 heads of 32 1113 -> 290.
-constexpr int AT_KEYS = 128, AT_CH = 32, AT_THREADS = 256;
+// Columns (keys, channels) that one pass has no room for are spread evenly over several.  Every sum runs in the order of the kernel for
+// longer sequences below (channels, tokens and the lanes' partial sums ascending), so that both give the same bits.  What bounds it:
+// shared-memory reads, a word per column and a broadcast per row for TR multiply-adds each, and at few rows the chain of chunks.
+// us with the four projections, one warp per row reading K a word at a time -> this kernel: 6 x 65 x 192, one head, bfloat16 98 -> 26; 64
+// x 197 x 192 2090 -> 115; 8 x 197 x 384 806 -> 84; float32, 8 x 197, 3 heads of 32 171 -> 39; 16 x 197, 12 heads of 32 1113 -> 229.
+constexpr int AT_CH = 32, AT_THREADS = 256, AT_COLS = 7, AT_QP = AT_CH + 4;
 
-// The chunk of 32 x 128 values that a thread holds 16 of: values 8 i .. 8 i + 7 of row `line(i)`, i = 0, 1, zeros past the ends.
+// Values first .. first + 7 of a row of n, zeros past its end.
 template <typename T>
 __device__ __forceinline__ void load_eight(float (&x)[8], const T* row, int first, int n, bool vec) {
     if (vec && first + 8 <= n) {
@@ -362,121 +363,155 @@ __device__ __forceinline__ void load_eight(float (&x)[8], const T* row, int firs
     }
 }
 
-// acc[r][e] += a[r][i] * tile[i][e] for i = 0 .. n - 1, in that order.
-template <int TR>
-__device__ __forceinline__ void times_tile(float (&acc)[TR][4], const float* a, int pitch, const float* tile, int n) {
-    auto step = [&](int r, float x, const float4& t) {
-        acc[r][0] = fmaf(x, t.x, acc[r][0]);
-        acc[r][1] = fmaf(x, t.y, acc[r][1]);
-        acc[r][2] = fmaf(x, t.z, acc[r][2]);
-        acc[r][3] = fmaf(x, t.w, acc[r][3]);
-    };
+// acc[r][g] += a[r][i] * tile[i][32 g + lane] for i = 0 .. n - 1, in that order, G groups of columns; rows of the tile are 32 G + PAD apart.
+template <int TR, int G, int PAD>
+__device__ __forceinline__ void times_tile(float (&acc)[TR][AT_COLS], const float* a, int pitch, const float* tile, int n) {
+    constexpr int V = TR > 5 ? 2 : 4;                // values of a row at once (registers)
     int i = 0;
-#pragma unroll 2
-    for (; i + 4 <= n; i += 4) {
-        float4 x[TR], t[4];
-#pragma unroll
-        for (int r = 0; r < TR; ++r) x[r] = *reinterpret_cast<const float4*>(a + r * pitch + i);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) t[u] = *reinterpret_cast<const float4*>(tile + (i + u) * AT_KEYS);
+#pragma unroll 1
+    for (; i + V <= n; i += V) {
+        float x[TR][V];
 #pragma unroll
         for (int r = 0; r < TR; ++r) {
-            step(r, x[r].x, t[0]);
-            step(r, x[r].y, t[1]);
-            step(r, x[r].z, t[2]);
-            step(r, x[r].w, t[3]);
+            if (V == 4) {
+                const float4 w = *reinterpret_cast<const float4*>(a + r * pitch + i);
+                x[r][0] = w.x; x[r][1] = w.y; x[r][V - 2] = w.z; x[r][V - 1] = w.w;
+            } else {
+                const float2 w = *reinterpret_cast<const float2*>(a + r * pitch + i);
+                x[r][0] = w.x; x[r][1] = w.y;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < V; ++u) {
+            float t[G];
+#pragma unroll
+            for (int g = 0; g < G; ++g) t[g] = tile[(i + u) * (32 * G + PAD) + 32 * g];
+#pragma unroll
+            for (int r = 0; r < TR; ++r)
+#pragma unroll
+                for (int g = 0; g < G; ++g) acc[r][g] = fmaf(x[r][u], t[g], acc[r][g]);
         }
     }
+#pragma unroll 1
     for (; i < n; ++i) {
-        const float4 t = *reinterpret_cast<const float4*>(tile + i * AT_KEYS);
 #pragma unroll
-        for (int r = 0; r < TR; ++r) step(r, a[r * pitch + i], t);
+        for (int g = 0; g < G; ++g) {
+            const float t = tile[i * (32 * G + PAD) + 32 * g];
+#pragma unroll
+            for (int r = 0; r < TR; ++r) acc[r][g] = fmaf(a[r * pitch + i], t, acc[r][g]);
+        }
+    }
+}
+template <int TR, int PAD>
+__device__ __forceinline__ void times_groups(float (&acc)[TR][AT_COLS], const float* a, int pitch, const float* tile, int n, int groups) {
+    switch (groups) {
+        case 1: times_tile<TR, 1, PAD>(acc, a, pitch, tile, n); break;
+        case 2: times_tile<TR, 2, PAD>(acc, a, pitch, tile, n); break;
+        case 3: times_tile<TR, 3, PAD>(acc, a, pitch, tile, n); break;
+        case 4: times_tile<TR, 4, PAD>(acc, a, pitch, tile, n); break;
+        case 5: times_tile<TR, 5, PAD>(acc, a, pitch, tile, n); break;
+        case 6: times_tile<TR, 6, PAD>(acc, a, pitch, tile, n); break;
+        default: times_tile<TR, 7, PAD>(acc, a, pitch, tile, n); break;
     }
 }
 
-template <typename T, int R>
-__global__ void __launch_bounds__(AT_THREADS)
+// Passes over `cols` columns and groups of 32 per pass.
+__host__ __device__ inline int tile_passes(int cols) { return (cols + 32 * AT_COLS - 1) / (32 * AT_COLS); }
+__host__ __device__ inline int tile_groups(int cols) { return ((cols + 31) / 32 + tile_passes(cols) - 1) / tile_passes(cols); }
+
+template <typename T, int TR>
+__global__ void __launch_bounds__(AT_THREADS, 2)
 attention_tile_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ o, int Tn, int H, int dk,
                       float scale, int vec) {
-    constexpr int TR = R / 8;
+    constexpr int R = 8 * TR;
     chain_begin_for<T>();
     extern __shared__ float sm[];
+    const int kp = tile_passes(Tn), kg = tile_groups(Tn), vp = tile_passes(dk), vg = tile_groups(dk);
     const int pitch = (Tn + 3) / 4 * 4 + 4;              // of a row of scores
-    const int qpitch = (dk + 3) / 4 * 4;
-    float* qs = sm;                                      // [R][qpitch]
-    float* prob = qs + R * qpitch;                       // [R][pitch]
-    float* tile = prob + R * pitch;                      // [32][128], scores: channel, key; output: token, channel
-    float* inv = tile + AT_CH * AT_KEYS;                 // [R]
+    float* qs = sm;                                      // [R][AT_QP]
+    float* prob = qs + R * AT_QP;                        // [R][pitch]
+    float* inv = prob + R * pitch;                       // [R]
+    float* tile = inv + R;                               // scores: [32 channels][32 kg + 1 keys], output: [32 tokens][32 vg channels]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int bh = blockIdx.y, b = bh / H, h = bh - b * H, row0 = blockIdx.x * R;
     const long long D = (long long)H * dk, base = (long long)b * Tn * D + h * dk;
     const int n_rows = min(R, Tn - row0);
     const int rg = warp * TR;                            // first row of this warp (its lanes read their values as broadcasts)
+    float acc[TR][AT_COLS];
+    auto clear = [&] {
 #pragma unroll
-    for (int r = 0; r < TR; ++r)
-#pragma unroll 4
-        for (int c = lane; c < dk; c += 32)
-            qs[(rg + r) * qpitch + c] = rg + r < n_rows ? to_f32(q[base + (row0 + rg + r) * D + c]) * scale : 0.f;
+        for (int r = 0; r < TR; ++r)
+#pragma unroll
+            for (int g = 0; g < AT_COLS; ++g) acc[r][g] = 0.f;
+    };
     // ---- scores ----
     const T* kb = k + base;
-    const int n_ch = (dk + AT_CH - 1) / AT_CH, n_kt = (Tn + AT_KEYS - 1) / AT_KEYS;
-    // this thread's part of a chunk: key tid % 128, channels 16 (tid / 128) .. + 15
-    const int lk = tid & 127, lc = (tid >> 7) * 16;
-    float next[16];
-    auto fetch_k = [&](int step) {
-        const int kt = step / n_ch, key = kt * AT_KEYS + lk, c = (step - kt * n_ch) * AT_CH + lc;
+    const int n_ch = (dk + AT_CH - 1) / AT_CH, keys = 32 * kg;
+    // a thread's part of a chunk: eight channels 8 (tid % 4) .. of keys tid / 4, + 64, ... (four lanes read 64 or 128 bytes of a row; the
+    // tile's rows are a word longer than they need be, so that they meet in no bank)
+    const int lk = tid >> 2, lc = (tid & 3) * 8;
+    float next[(32 * AT_COLS + 63) / 64][8], qnext[(R + 31) / 32 * 4];
+    auto fetch_k = [&](int pass, int ch) {
+        const int c = min(ch * AT_CH + lc, dk);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            float x[8];
-            load_eight<T>(x, kb + (long long)min(key, Tn - 1) * D, min(c + 8 * i, dk), dk, vec);
+        for (int i = 0; i < (32 * AT_COLS + 63) / 64; ++i)
+            if (lk + 64 * i < keys) load_eight<T>(next[i], kb + (long long)min(pass * keys + lk + 64 * i, Tn - 1) * D, c, dk, vec);
+        // (four channels 4 (tid % 8) .. of rows tid / 8, + 32)
 #pragma unroll
-            for (int e = 0; e < 8; ++e) next[8 * i + e] = x[e];
+        for (int i = 0; i < (R + 31) / 32; ++i) {
+            const int r = (tid >> 3) + 32 * i, c4 = ch * AT_CH + (tid & 7) * 4;
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                qnext[4 * i + e] = r < n_rows && c4 + e < dk ? to_f32(q[base + (row0 + r) * D + c4 + e]) * scale : 0.f;
         }
     };
-    fetch_k(0);
-    float acc[TR][4];
-    for (int step = 0; step < n_kt * n_ch; ++step) {
-        const int kt = step / n_ch, ch = step - kt * n_ch;
-        __syncthreads();                                 // the chunk before has been read
+    fetch_k(0, 0);
+    for (int pass = 0; pass < kp; ++pass) {
+        clear();
+        for (int ch = 0; ch < n_ch; ++ch) {
+            __syncthreads();                             // the chunk before has been read
 #pragma unroll
-        for (int e = 0; e < 16; ++e) tile[(lc + e) * AT_KEYS + lk] = next[e];
-        __syncthreads();
-        if (step + 1 < n_kt * n_ch) fetch_k(step + 1);
-        if (ch == 0) {
+            for (int i = 0; i < (32 * AT_COLS + 63) / 64; ++i)
+                if (lk + 64 * i < keys) {
 #pragma unroll
-            for (int r = 0; r < TR; ++r)
+                    for (int e = 0; e < 8; ++e) tile[(lc + e) * (keys + 1) + lk + 64 * i] = next[i][e];
+                }
 #pragma unroll
-                for (int e = 0; e < 4; ++e) acc[r][e] = 0.f;
-        }
-        if (kt * AT_KEYS + 4 * lane < Tn) {
-            const int nc = min(AT_CH, dk - ch * AT_CH);
-            times_tile<TR>(acc, qs + rg * qpitch + ch * AT_CH, qpitch, tile + 4 * lane, nc);
-            if (ch == n_ch - 1) {
-#pragma unroll
-                for (int r = 0; r < TR; ++r)
-                    *reinterpret_cast<float4*>(prob + (rg + r) * pitch + kt * AT_KEYS + 4 * lane) =
-                        make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+            for (int i = 0; i < (R + 31) / 32; ++i) {
+                const int r = (tid >> 3) + 32 * i;
+                if (r < R)
+                    *reinterpret_cast<float4*>(qs + r * AT_QP + (tid & 7) * 4) =
+                        make_float4(qnext[4 * i], qnext[4 * i + 1], qnext[4 * i + 2], qnext[4 * i + 3]);
             }
+            __syncthreads();
+            if (ch + 1 < n_ch) fetch_k(pass, ch + 1);
+            else if (pass + 1 < kp) fetch_k(pass + 1, 0);
+            times_groups<TR, 1>(acc, qs + rg * AT_QP, AT_QP, tile + lane, min(AT_CH, dk - ch * AT_CH), kg);
         }
+#pragma unroll
+        for (int r = 0; r < TR; ++r)
+#pragma unroll
+            for (int g = 0; g < AT_COLS; ++g) {
+                const int key = pass * keys + 32 * g + lane;
+                if (g < kg && key < Tn) prob[(rg + r) * pitch + key] = acc[r][g];
+            }
     }
     // ---- softmax: the rows of this warp, whose scores it has written itself ----
     const T* vb = v + base;
-    const int n_vt = (dk + AT_KEYS - 1) / AT_KEYS, n_jt = (Tn + AT_CH - 1) / AT_CH;
-    // this thread's part of a chunk: token tid / 8, channels 16 (tid % 8) .. + 15
-    const int lj = tid >> 3, lv = (tid & 7) * 16;
-    auto fetch_v = [&](int step) {
-        const int vt = step / n_jt, j = (step - vt * n_jt) * AT_CH + lj, c = vt * AT_KEYS + lv;
+    const int n_jt = (Tn + AT_CH - 1) / AT_CH, chans = 32 * vg;
+    // a thread's part of a chunk: eight channels 8 (tid % 8 + 8 i) .. of token tid / 8
+    const int lj = tid >> 3;
+    auto fetch_v = [&](int pass, int jt) {
+        const T* vr = vb + (long long)min(jt * AT_CH + lj, Tn - 1) * D;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            float x[8];
-            load_eight<T>(x, vb + (long long)min(j, Tn - 1) * D, min(c + 8 * i, dk), dk, vec);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) next[8 * i + e] = x[e];
+        for (int i = 0; i < (32 * AT_COLS + 63) / 64; ++i) {
+            const int c = 8 * ((tid & 7) + 8 * i);
+            if (c < chans) load_eight<T>(next[i], vr, min(pass * chans + c, dk), dk, vec);
         }
     };
-    fetch_v(0);
+    fetch_v(0, 0);
     __syncwarp();
-#pragma unroll
+#pragma unroll 1
     for (int r = 0; r < TR; ++r) {
         float* pr = prob + (rg + r) * pitch;
         float m = -3.402823466e38f;
@@ -492,34 +527,33 @@ attention_tile_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
         if (lane == 0) inv[rg + r] = 1.0f / sum;
     }
     // ---- output ----
-    for (int step = 0; step < n_vt * n_jt; ++step) {
-        const int vt = step / n_jt, jt = step - vt * n_jt, c0 = vt * AT_KEYS + 4 * lane;
-        __syncthreads();
+    for (int pass = 0; pass < vp; ++pass) {
+        clear();
+        for (int jt = 0; jt < n_jt; ++jt) {
+            __syncthreads();
 #pragma unroll
-        for (int e4 = 0; e4 < 4; ++e4)
-            *reinterpret_cast<float4*>(tile + lj * AT_KEYS + lv + 4 * e4) =
-                make_float4(next[4 * e4], next[4 * e4 + 1], next[4 * e4 + 2], next[4 * e4 + 3]);
-        __syncthreads();
-        if (step + 1 < n_vt * n_jt) fetch_v(step + 1);
-        if (jt == 0) {
-#pragma unroll
-            for (int r = 0; r < TR; ++r)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) acc[r][e] = 0.f;
+            for (int i = 0; i < (32 * AT_COLS + 63) / 64; ++i) {
+                const int c = 8 * ((tid & 7) + 8 * i);
+                if (c < chans) {
+                    float* to = tile + lj * chans + c;
+                    *reinterpret_cast<float4*>(to) = make_float4(next[i][0], next[i][1], next[i][2], next[i][3]);
+                    *reinterpret_cast<float4*>(to + 4) = make_float4(next[i][4], next[i][5], next[i][6], next[i][7]);
+                }
+            }
+            __syncthreads();
+            if (jt + 1 < n_jt) fetch_v(pass, jt + 1);
+            else if (pass + 1 < vp) fetch_v(pass + 1, 0);
+            times_groups<TR, 0>(acc, prob + rg * pitch + jt * AT_CH, pitch, tile + lane, min(AT_CH, Tn - jt * AT_CH), vg);
         }
-        if (c0 < dk) {
-            const int nj = min(AT_CH, Tn - jt * AT_CH);
-            times_tile<TR>(acc, prob + rg * pitch + jt * AT_CH, pitch, tile + 4 * lane, nj);
-            if (jt == n_jt - 1) {
 #pragma unroll
-                for (int r = 0; r < TR; ++r) {
-                    if (rg + r < n_rows) {
-                        T* to = o + base + (row0 + rg + r) * D + c0;
-                        const float s = inv[rg + r];
+        for (int r = 0; r < TR; ++r) {
+            if (rg + r < n_rows) {
+                T* to = o + base + (row0 + rg + r) * D;
+                const float s = inv[rg + r];
 #pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            if (c0 + e < dk) to[e] = from_f32<T>(acc[r][e] * s);
-                    }
+                for (int g = 0; g < AT_COLS; ++g) {
+                    const int c = pass * chans + 32 * g + lane;
+                    if (g < vg && c < dk) to[c] = from_f32<T>(acc[r][g] * s);
                 }
             }
         }
@@ -527,17 +561,18 @@ attention_tile_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
 }
 
 size_t tile_smem(int Tn, int dk, int R) {
-    return ((size_t)R * ((dk + 3) / 4 * 4) + (size_t)R * ((Tn + 3) / 4 * 4 + 4) + AT_CH * AT_KEYS + R) * sizeof(float);
+    const int groups = tile_groups(Tn) > tile_groups(dk) ? tile_groups(Tn) : tile_groups(dk);
+    return ((size_t)R * AT_QP + (size_t)R * ((Tn + 3) / 4 * 4 + 4) + R + (size_t)AT_CH * (32 * groups + 1)) * sizeof(float);
 }
 
-template <typename T, int R>
+template <typename T, int TR>
 int launch_tile(const void* q, const void* k, const void* v, void* o, int B, int Tn, int H, int dk, float scale, cudaStream_t st) {
-    const size_t smem = tile_smem(Tn, dk, R);
-    auto kern = attention_tile_kernel<T, R>;
+    const size_t smem = tile_smem(Tn, dk, 8 * TR);
+    auto kern = attention_tile_kernel<T, TR>;
     CONVNN_ENSURE_SMEM(kern, smem);
     const int vec = dk % 8 == 0 && aligned16(k) && aligned16(v);         // (rows of a multiple of eight values)
-    launch_chained(kern, dim3((Tn + R - 1) / R, B * H), AT_THREADS, smem, st, static_cast<const T*>(q), static_cast<const T*>(k),
-                   static_cast<const T*>(v), static_cast<T*>(o), Tn, H, dk, scale, vec);
+    launch_chained(kern, dim3((Tn + 8 * TR - 1) / (8 * TR), B * H), AT_THREADS, smem, st, static_cast<const T*>(q),
+                   static_cast<const T*>(k), static_cast<const T*>(v), static_cast<T*>(o), Tn, H, dk, scale, vec);
     CONVNN_CHECK_LAUNCH("attention_tile");
     return CONVNN_OK;
 }
@@ -649,15 +684,21 @@ int launch_attention_simt_t(const void* q, const void* k, const void* v, void* o
                             cudaStream_t st) {
     const int dk = D / H, nw = 4;
     const float scale = (float)(1.0 / sqrt((double)dk));
-    // Fewer rows per CTA where more leave SMs without one (all read every chunk, so that they are fewer multiply-adds per read: 6 x 65 x 192
-    // 22 us with 16 rows, 19 with 8; 6 x 197 x 192 46, 57).
-    auto ctas = [&](int R) { return (long long)B * H * ((Tn + R - 1) / R); };
-    const int R = 3 * ctas(16) < device_sms() ? 8 : ctas(32) < 2 * device_sms() ? 16 : 32;
-    if (tile_smem(Tn, dk, R) <= 200 * 1024) {
-        if (R == 8) return launch_tile<T, 8>(q, k, v, o, B, Tn, H, dk, scale, st);
-        if (R == 16) return launch_tile<T, 16>(q, k, v, o, B, Tn, H, dk, scale, st);
-        return launch_tile<T, 32>(q, k, v, o, B, Tn, H, dk, scale, st);
+    // Rows per CTA: the fewest multiply-adds on the busiest SM, where a CTA costs its rows and, staging its chunks, twelve more, and a
+    // round of two CTAs their chain of chunks.
+    int rows = 0;
+    long long least = 0;
+    for (const int R : {56, 40, 16, 8}) {
+        const long long n = ((long long)B * H * ((Tn + R - 1) / R) + device_sms() - 1) / device_sms(), cost = n * (R + 12) + (n + 1) / 2 * 32;
+        if (tile_smem(Tn, dk, R) <= 200 * 1024 && (!rows || cost < least)) {
+            rows = R;
+            least = cost;
+        }
     }
+    if (rows == 8) return launch_tile<T, 1>(q, k, v, o, B, Tn, H, dk, scale, st);
+    if (rows == 16) return launch_tile<T, 2>(q, k, v, o, B, Tn, H, dk, scale, st);
+    if (rows == 40) return launch_tile<T, 5>(q, k, v, o, B, Tn, H, dk, scale, st);
+    if (rows == 56) return launch_tile<T, 7>(q, k, v, o, B, Tn, H, dk, scale, st);
     const size_t smem = (size_t)nw * (Tn + dk) * sizeof(float);
     if (smem > 200 * 1024)
         return set_error(CONVNN_E_UNSUPPORTED, "softmax attention over %d tokens is outside this build", Tn);

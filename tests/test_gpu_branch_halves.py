@@ -156,7 +156,7 @@ def test_branching_modules_fold_the_skip_connection():
 @pytest.mark.parametrize("B,T,D,H,dtype", [
     (2, 1, 8, 1, torch.float32), (2, 15, 33, 1, torch.float32), (1, 129, 60, 2, torch.float32), (3, 65, 192, 1, torch.bfloat16),
     (1, 128, 384, 1, torch.bfloat16), (2, 257, 136, 1, torch.bfloat16), (40, 257, 64, 2, torch.bfloat16), (50, 197, 160, 1, torch.float32),
-    (1, 4000, 16, 1, torch.float32), (1, 33, 30, 2, torch.bfloat16)])
+    (1, 7000, 16, 1, torch.float32), (60, 197, 48, 1, torch.float32), (1, 33, 30, 2, torch.bfloat16)])
 def test_softmax_attention_tiles(B, T, D, H, dtype):
     g = torch.Generator().manual_seed(T + D)
     w = {f"W_{n}.weight": _uni((D, D), D, g) * (3.0 if n in "qk" else 1.0) for n in "qkvo"}
@@ -167,5 +167,5 @@ def test_softmax_attention_tiles(B, T, D, H, dtype):
     w_qkv = torch.stack([w[f"W_{n}.weight"] for n in "qkv"]).to(DEV, dtype)
     x_dev, w_o = x.to(DEV, dtype), w["W_o.weight"].to(DEV, dtype)
     call = lambda: ops.softmax_attention(x_dev, w_qkv, w_o, H)
-    assert any("attention_tile_kernel" in n for n in launches(call)) == (T < 3000)
+    assert any("attention_tile_kernel" in n for n in launches(call)) == (T < 6000)
     assert rel_err(call(), softmax_attention(x, w, H)) < (1e-4 if dtype == torch.float32 else 2e-2)
