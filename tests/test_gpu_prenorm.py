@@ -79,6 +79,23 @@ def test_prenorm_linear_against_float64(M, N, K, shift, gelu):
     assert _capi.device_status() == 0
 
 
+@pytest.mark.parametrize("gelu", [False, True])
+@pytest.mark.parametrize("N,K", [(576, 192), (192, 192), (360, 64), (96, 128)])
+def test_prenorm_linear_of_few_rows_has_the_bits_of_many(N, K, gelu):
+    """Few row tiles are cut into narrower column tiles of the same sums: the rows keep their bits on
+    either side of the line (256 rows) and as the head of a matrix that fills the chip."""
+    x = rnd(24000, K, seed=16)
+    w, b = rnd(N, K, seed=17, scale=K ** -0.5), rnd(N, seed=18, scale=0.3)
+    wf, wx = ops.fold_layernorm(w, b, rnd(K, seed=19, scale=0.2, shift=1.0), rnd(K, seed=20, scale=0.2))
+    want = ops.prenorm_linear(x, ops.row_moments(x), 1e-5, wf, wx, gelu=gelu)
+    for M in (256, 257, 385, 1111):
+        got = ops.prenorm_linear(x[:M], ops.row_moments(x[:M]), 1e-5, wf, wx, gelu=gelu)
+        assert torch.equal(got, want[:M]), M
+    x, wide = rnd(300, 768, seed=21), torch.zeros(3072, 768, dtype=BF, device=DEV)
+    with pytest.raises(_capi.ConvnnError):                         # refused with 300 rows as with 64
+        ops.prenorm_linear(x, ops.row_moments(x), 1e-5, wide, torch.zeros(3072, 16, dtype=BF, device=DEV), gelu=gelu)
+
+
 def test_prenorm_linear_takes_moments_in_several_planes():
     """The consumer adds the planes up: moments split arbitrarily over three planes give the same bits."""
     M, N, K = 500, 768, 192
