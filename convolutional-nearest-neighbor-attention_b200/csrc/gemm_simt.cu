@@ -120,6 +120,41 @@ __device__ __forceinline__ void store_outputs(const GemmParams& p, int n0, int s
     }
 }
 
+// Four values of an operand row as they came from memory, made float32 when they are stored to shared memory, a step later.
+template <typename T> struct Four;
+template <> struct Four<float> {
+    float4 v;
+    __device__ __forceinline__ void none() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ __forceinline__ void load(const float* p, int n, bool vec) { v = load_upto4(p, n, vec); }
+    __device__ __forceinline__ float4 get() const { return v; }
+};
+template <> struct Four<__nv_bfloat16> {
+    uint32_t r[4];             // two pairs, or four values one by one (`vec` tells)
+    bool pairs;
+    __device__ __forceinline__ void none() {
+        pairs = true;
+        r[0] = r[1] = 0u;
+    }
+    __device__ __forceinline__ void load(const __nv_bfloat16* p, int n, bool vec) {
+        pairs = vec && n >= 4;
+        if (pairs) {
+            const uint2 w = *reinterpret_cast<const uint2*>(p);
+            r[0] = w.x;
+            r[1] = w.y;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r[i] = i < n ? reinterpret_cast<const unsigned short*>(p)[i] : 0u;
+        }
+    }
+    __device__ __forceinline__ float4 get() const {
+        if (pairs)
+            return make_float4(__uint_as_float(r[0] << 16), __uint_as_float(r[0] & 0xffff0000u), __uint_as_float(r[1] << 16),
+                               __uint_as_float(r[1] & 0xffff0000u));
+        return make_float4(__uint_as_float(r[0] << 16), __uint_as_float(r[1] << 16), __uint_as_float(r[2] << 16),
+                           __uint_as_float(r[3] << 16));
+    }
+};
+
 // Tile BM x BN, NT = (BM / TM) * (BN / TN) threads in warps of 4 (rows) x 8 (columns).
 // TA: type of the A operand (float32 against bfloat16 weights for the separable conv's unrounded intermediate).
 template <typename TA, typename T, int MODE, int BM, int BN, int BK, int TM, int TN, int MINB>
@@ -191,16 +226,23 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_kernel(
     }
     const bool avec = p.a_vec, wvec = p.w_vec;
 
-    float4 av[NA], bv[NB];
+    // Plain rows stay as they came until they are stored to shared memory, a step later: converted here, a bfloat16 load is waited
+    // for before the products it should hide behind (7 x 577 x 384 with the coordinate channel, k and v 80.5 -> 69.4 us).
+    constexpr bool PLAIN = MODE == A_ROWS || MODE == A_TOKENS;
+    std::conditional_t<PLAIN, Four<TA>, Four<float>> av[NA];
+    std::conditional_t<PLAIN, Four<T>, Four<float>> bv[NB];
     auto fetch = [&](int k0) {
 #pragma unroll
         for (int i = 0; i < NA; ++i) {
             const int kk = k0 + akq[i] * 4;
+            if constexpr (PLAIN) {
+                av[i].none();
+                if (ar[i].base && kk < p.Kd) av[i].load(ar[i].base + kk, p.Kd - kk, avec);
+                continue;
+            }
             float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
             if (ar[i].base && kk < p.Kd) {
-                if (MODE == A_ROWS || MODE == A_TOKENS) {
-                    r = load_upto4<TA>(ar[i].base + kk, p.Kd - kk, avec);
-                } else if (MODE == A_HEAD_QUIRK) {
+                if (MODE == A_HEAD_QUIRK) {
                     float e[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
@@ -221,11 +263,16 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_kernel(
                     if (tt >= 0 && tt < p.T) r = load_upto4<TA>(ar[i].base + (long long)tt * p.H * p.Cp + c, 4, avec);
                 }
             }
-            av[i] = r;
+            if constexpr (!PLAIN) av[i].v = r;
         }
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
             const int kk = k0 + bkq[i] * 4;
+            if constexpr (PLAIN) {
+                bv[i].none();
+                if (wbase[i] && kk < p.Kd) bv[i].load(wbase[i] + kk, p.Kd - kk, wvec);
+                continue;
+            }
             float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
             if (wbase[i] && kk < p.Kd) {
                 if (MODE == A_NEIGHBOURS && p.C != p.Cp) {        // taps of C values against C + padding stored channels
@@ -235,19 +282,21 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_kernel(
                     r = load_upto4<T>(wbase[i] + kk, p.Kd - kk, wvec);
                 }
             }
-            bv[i] = r;
+            if constexpr (!PLAIN) bv[i].v = r;
         }
     };
     auto stage = [&](int buf) {
 #pragma unroll
         for (int i = 0; i < NA; ++i) {
             float* d = As + (buf * BK + akq[i] * 4) * LA + arow[i];
-            d[0] = av[i].x; d[LA] = av[i].y; d[2 * LA] = av[i].z; d[3 * LA] = av[i].w;
+            const float4 v = av[i].get();
+            d[0] = v.x; d[LA] = v.y; d[2 * LA] = v.z; d[3 * LA] = v.w;
         }
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
             float* d = Bs + (buf * BK + bkq[i] * 4) * LB + brow[i];
-            d[0] = bv[i].x; d[LB] = bv[i].y; d[2 * LB] = bv[i].z; d[3 * LB] = bv[i].w;
+            const float4 v = bv[i].get();
+            d[0] = v.x; d[LB] = v.y; d[2 * LB] = v.z; d[3 * LB] = v.w;
         }
     };
 
@@ -442,41 +491,6 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_copy_ke
         });
 }
 
-// Four values of an operand row as they came from memory, made float32 when they are stored to shared memory, a step later.
-template <typename T> struct Four;
-template <> struct Four<float> {
-    float4 v;
-    __device__ __forceinline__ void none() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
-    __device__ __forceinline__ void load(const float* p, int n, bool vec) { v = load_upto4(p, n, vec); }
-    __device__ __forceinline__ float4 get() const { return v; }
-};
-template <> struct Four<__nv_bfloat16> {
-    uint32_t r[4];             // two pairs, or four values one by one (`vec` tells)
-    bool pairs;
-    __device__ __forceinline__ void none() {
-        pairs = true;
-        r[0] = r[1] = 0u;
-    }
-    __device__ __forceinline__ void load(const __nv_bfloat16* p, int n, bool vec) {
-        pairs = vec && n >= 4;
-        if (pairs) {
-            const uint2 w = *reinterpret_cast<const uint2*>(p);
-            r[0] = w.x;
-            r[1] = w.y;
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) r[i] = i < n ? reinterpret_cast<const unsigned short*>(p)[i] : 0u;
-        }
-    }
-    __device__ __forceinline__ float4 get() const {
-        if (pairs)
-            return make_float4(__uint_as_float(r[0] << 16), __uint_as_float(r[0] & 0xffff0000u), __uint_as_float(r[1] << 16),
-                               __uint_as_float(r[1] & 0xffff0000u));
-        return make_float4(__uint_as_float(r[0] << 16), __uint_as_float(r[1] << 16), __uint_as_float(r[2] << 16),
-                           __uint_as_float(r[3] << 16));
-    }
-};
-
 // The same tiles for rows that have to be converted, or that cannot be copied 16 bytes at a time: they come through
 // registers, a step ahead.
 template <typename TA, typename T, int MODE, int BM, int BN, int TM, int TN, int MINB>
@@ -657,8 +671,7 @@ int launch_plain_f32(const GemmParams& p, cudaStream_t st) {
 }
 
 // Other plain rows: float32 ones of any alignment, bfloat16, float32 against bfloat16 weights.  Which tiles, and which times, goes by
-// what the operands cost: float32 values need no conversion, so that the transposed tiles wait for little and the largest of
-// them reuses most; bfloat16 values that come one by one are what the transposed tiles wait for.  Narrow outputs of few
+// what the operands cost: rows that come one value at a time cost every tile more, the small ones most.  Narrow outputs of few
 // values of k (the separable conv with the coordinate channel on heads of 8 to 32) end before that counts.  Fits to 209, 90, 98
 // and 90 shapes (30 to 1000000 rows, 8 to 2304 columns, 9 to 2048 values of k; rms 3 to 21 %), the choice within 1.2, 1.0, 0.8
 // and 0.9 % of the best of seven tiles on average; 0.95, 0.72, 0.55 and 0.71 of the time of the four transposed tiles alone, at worst
@@ -666,6 +679,8 @@ int launch_plain_f32(const GemmParams& p, cudaStream_t st) {
 // float32, us, staged tiles only -> now: 2813 x 768 x 769 138 -> 102, 56288 x 256 x 257 244 -> 189, 39846 x 8 x 9 9.9 -> 6.7; mixed 650981 x
 // 64 x 65 277 -> 233, 109615 x 16 x 17 18.7 -> 12.3.
 // bfloat16, transposed tiles only -> now: 4 x 197 x 768 x 768 130 -> 55; 2080 x 384 x 388 57.9 -> 27.8.
+// The 128 x 64 tile, once it waits for no conversion, is the best of five on most large outputs of bfloat16 rows read four at a time and of mixed ones (27 shapes; the fits
+// hold within 10 %), us: 4925 x 2304 x 768 468 -> 399, 25216 x 192 x 192 64 -> 54, mixed 4925 x 768 x 769 215 -> 176.
 template <typename TA, typename T, int MODE>
 int launch_plain_staged(const GemmParams& p, cudaStream_t st) {
     if constexpr (sizeof(T) == 4) {
@@ -683,21 +698,21 @@ int launch_plain_staged(const GemmParams& p, cudaStream_t st) {
         }
     } else {
         static const Tile by_four[5] = {
-            {128, 64, 16, 3, 0.0, 4.1, {122.5, 162.1, 187.0}},
-            {32, 32, 32, 7, 2.1, 0.0, {62.1, 67.9, 72.2, 82.4, 84.4, 93.8, 81.1}},
+            {128, 64, 16, 3, 7.5, 2.0, {65.0, 113.0, 156.0}},
+            {32, 32, 32, 7, 1.5, 1.2, {45.0, 51.0, 66.0, 68.0, 72.0, 78.0, 73.0}},
             {64, 64, 32, 3, 2.4, 2.9, {41.0, 62.8, 91.7}},
             {32, 64, 32, 4, 1.5, 1.8, {27.3, 43.1, 59.2, 76.9}},
             {40, 32, 32, 6, 1.8, 2.5, {32.2, 34.5, 46.8, 51.2, 60.2, 70.8}},
         };
         static const Tile by_value[5] = {
-            by_four[0],                                              // (not taken: 4039 x 768 x 385 135 us, the third 93)
+            by_four[0],          // (not among the choices: no layer has such rows on both sides.  4039 x 768 x 385 87 us, the third 98)
             {32, 32, 32, 7, 1.1, 0.0, {108.4, 122.0, 111.1, 150.7, 131.6, 174.3, 135.2}},
             {64, 64, 32, 3, 2.6, 3.6, {45.3, 68.7, 102.8}},
             {32, 64, 32, 4, 2.1, 1.7, {31.9, 48.3, 65.4, 92.7}},
             {40, 32, 32, 6, 2.3, 2.9, {36.8, 39.8, 54.5, 58.5, 83.1, 87.1}},
         };
         static const Tile mixed[5] = {                               // float32 rows against bfloat16 weights
-            {128, 64, 16, 3, 2.0, 0.0, {157.9, 182.8, 200.0}},
+            {128, 64, 16, 3, 7.5, 2.0, {64.0, 113.0, 148.0}},
             {32, 32, 32, 7, 0.9, 0.0, {90.3, 100.6, 98.8, 99.2, 114.6, 113.0, 102.3}},
             {64, 64, 32, 3, 2.1, 2.6, {42.7, 67.6, 95.9}},
             {32, 64, 32, 4, 1.9, 1.0, {31.5, 47.1, 66.7, 82.2}},

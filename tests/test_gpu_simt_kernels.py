@@ -297,3 +297,24 @@ def test_tiles_of_staged_rows(M, N, K, bf16, fp32, dtype):
     assert bool(((got.double() - want - r.double()).abs() <= bound).all())
     some = torch.randperm(M, device=DEV, generator=g)[:20]
     assert torch.equal(ops.linear(a[some], w, b, residual=r[some]), got[some])
+
+
+# The 128 x 64 tile on bfloat16 and mixed rows, which stay as they came until they are stored to shared memory: ragged rows, columns
+# and k, by fours and one by one (the separable conv's intermediate with the coordinate channel: dk + 1 values).
+@on_148_sms
+@pytest.mark.parametrize("B,T,dk", [(32, 197, 384), (25, 197, 768), (65, 577, 96), (48, 577, 96)])
+def test_large_tile_of_mixed_rows(B, T, dk):
+    g = torch.Generator(device=DEV).manual_seed(dk)
+    spec = ops.LayerSpec(dk, 1, 5, "all", "cosine", "depthwise-separable", True, True, T)
+    C, Cp = dk + 1, (dk + 8) // 8 * 8
+    v = torch.zeros(B, T, 1, Cp, device=DEV)
+    v[..., :C] = torch.randn(B, T, 1, C, device=DEV, generator=g)
+    v = v.to(torch.bfloat16)
+    idx = torch.randint(0, T, (B, 1, T, 5), device=DEV, generator=g, dtype=torch.int32)
+    val = torch.randn(B, 1, T, 5, device=DEV, generator=g)
+    dw = (torch.randn(5, C, device=DEV, generator=g) / 2).to(torch.bfloat16)
+    pw = (torch.randn(dk, C, device=DEV, generator=g) / C ** 0.5).to(torch.bfloat16)
+    call = lambda n=B: ops.gather_conv(spec, v[:n], idx[:n], val[:n], dw, pw)
+    assert any(re.search(r"gemm_simt_kernelIf13__nv_bfloat16Li\dELi128ELi64E", n) for n in launches(call))
+    got = call()
+    assert torch.equal(call(2), got[:2])                             # (two images take smaller tiles: the same sums)
