@@ -226,23 +226,23 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_kernel(
     }
     const bool avec = p.a_vec, wvec = p.w_vec;
 
-    // Plain rows stay as they came until they are stored to shared memory, a step later: converted here, a bfloat16 load is waited
-    // for before the products it should hide behind (7 x 577 x 384 with the coordinate channel, k and v 80.5 -> 69.4 us).
-    constexpr bool PLAIN = MODE == A_ROWS || MODE == A_TOKENS;
-    std::conditional_t<PLAIN, Four<TA>, Four<float>> av[NA];
-    std::conditional_t<PLAIN, Four<T>, Four<float>> bv[NB];
+    // Operands stay as they came until they are stored to shared memory, a step later: converted or weighted here, a load is waited
+    // for before the products it should hide behind (bfloat16, 7 x 577 x 384 with the coordinate channel, k and v 80.5 -> 69.4 us;
+    // standard conv, 9 taps, float32 8 x 197 x 192 104 -> 91, 32 x 197 x 384 678 -> 592, 1 x 197 x 3 heads of 64 28.2 -> 23.0; bfloat16 with the
+    // coordinate channel 8 x 197 x 192 150 -> 110, 32 x 197 x 384 893 -> 783).
+    std::conditional_t<MODE == A_HEAD_QUIRK, Four<float>, Four<TA>> av[NA];
+    Four<T> bv[NB];
+    float aw[MODE == A_NEIGHBOURS ? NA : 1];                // the neighbours' weights
     auto fetch = [&](int k0) {
 #pragma unroll
         for (int i = 0; i < NA; ++i) {
             const int kk = k0 + akq[i] * 4;
-            if constexpr (PLAIN) {
-                av[i].none();
-                if (ar[i].base && kk < p.Kd) av[i].load(ar[i].base + kk, p.Kd - kk, avec);
-                continue;
-            }
-            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+            av[i].none();
+            if constexpr (MODE == A_NEIGHBOURS) aw[i] = 0.f;
             if (ar[i].base && kk < p.Kd) {
-                if (MODE == A_HEAD_QUIRK) {
+                if constexpr (MODE == A_ROWS || MODE == A_TOKENS) {
+                    av[i].load(ar[i].base + kk, p.Kd - kk, avec);
+                } else if constexpr (MODE == A_HEAD_QUIRK) {
                     float e[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
@@ -250,46 +250,39 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB) gemm_simt_kernel(
                             const int h = (kk + j) / p.dk, c = kk + j - h * p.dk;
                             e[j] = to_f32<TA>(ar[i].base[((long long)h * p.dk + c) * p.T]);
                         }
-                    r = make_float4(e[0], e[1], e[2], e[3]);
-                } else if (MODE == A_NEIGHBOURS) {
+                    av[i].v = make_float4(e[0], e[1], e[2], e[3]);
+                } else if constexpr (MODE == A_NEIGHBOURS) {
                     // k = (tap, stored channel): Cp is a multiple of four, so the four values share a tap
                     const int j = kk / p.Cp, c = kk - j * p.Cp;
                     const int e = ar[i].m_local * p.taps + j;
-                    const float w = ps[e];
-                    r = load_upto4<TA>(ar[i].base + ns[e] + c, 4, avec);
-                    r.x *= w; r.y *= w; r.z *= w; r.w *= w;
+                    aw[i] = ps[e];
+                    av[i].load(ar[i].base + ns[e] + c, 4, avec);
                 } else {                                          // A_CONV1D: k = (tap, channel)
                     const int j = kk / p.Cp, c = kk - j * p.Cp, tt = ar[i].t + j - p.pad;
-                    if (tt >= 0 && tt < p.T) r = load_upto4<TA>(ar[i].base + (long long)tt * p.H * p.Cp + c, 4, avec);
+                    if (tt >= 0 && tt < p.T) av[i].load(ar[i].base + (long long)tt * p.H * p.Cp + c, 4, avec);
                 }
             }
-            if constexpr (!PLAIN) av[i].v = r;
         }
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
             const int kk = k0 + bkq[i] * 4;
-            if constexpr (PLAIN) {
-                bv[i].none();
-                if (wbase[i] && kk < p.Kd) bv[i].load(wbase[i] + kk, p.Kd - kk, wvec);
-                continue;
-            }
-            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+            bv[i].none();
             if (wbase[i] && kk < p.Kd) {
                 if (MODE == A_NEIGHBOURS && p.C != p.Cp) {        // taps of C values against C + padding stored channels
                     const int j = kk / p.Cp, c = kk - j * p.Cp;
-                    r = load_upto4<T>(wbase[i] + (long long)j * p.C + c, p.C - c, false);
+                    bv[i].load(wbase[i] + (long long)j * p.C + c, p.C - c, false);
                 } else {
-                    r = load_upto4<T>(wbase[i] + kk, p.Kd - kk, wvec);
+                    bv[i].load(wbase[i] + kk, p.Kd - kk, wvec);
                 }
             }
-            if constexpr (!PLAIN) bv[i].v = r;
         }
     };
     auto stage = [&](int buf) {
 #pragma unroll
         for (int i = 0; i < NA; ++i) {
             float* d = As + (buf * BK + akq[i] * 4) * LA + arow[i];
-            const float4 v = av[i].get();
+            float4 v = av[i].get();
+            if constexpr (MODE == A_NEIGHBOURS) { v.x *= aw[i]; v.y *= aw[i]; v.z *= aw[i]; v.w *= aw[i]; }
             d[0] = v.x; d[LA] = v.y; d[2 * LA] = v.z; d[3 * LA] = v.w;
         }
 #pragma unroll
@@ -746,7 +739,8 @@ int launch_other_mode(const GemmParams& p, cudaStream_t st) {
     // An implicit operand is fetched with divisions and dependent reads per value.  While an SM has few tiles that, not the
     // products, is what a step waits for, and a tile with twice the threads wins; with more of them the tiles hide each other's
     // waits, and its extra shared-memory reads per product lose.  It keeps two tiles on an SM (four of the smallest) where
-    // the other form keeps three (seven), so it is taken where that takes no more passes.  Weighted neighbours, us, other form -> twice the
+    // the other form keeps three (seven), so it is taken where that takes no more passes.  (Times from before the operands were weighted
+    // and converted as late as they are now, which took both forms to 0.64 to 0.96 of them.)  Weighted neighbours, us, other form -> twice the
     // threads, float32, 9 taps unless noted; rounds of tiles per SM first:
     //   128 x 64   1: 32 x 197 x 3 heads of 64 84.9 -> 60.0   2: 64 x 197 x 3 x 64 107 -> 87   3: 256 x 65 x 192 380 -> 388 (not taken)   4: 128 x 197 x 3 x 64 194 -> 170
     //   64 x 64    1: 8 x 197 x 192 133 -> 103   3: 20 x 577 x 100 113 -> 128 (not taken)   4: 64 x 197 x 192 314 -> 301   5: 32 x 197 x 384 675 -> 706 (not taken)
