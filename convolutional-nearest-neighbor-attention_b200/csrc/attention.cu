@@ -577,7 +577,7 @@ int launch_tile(const void* q, const void* k, const void* v, void* o, int B, int
     return CONVNN_OK;
 }
 
-// One warp per query row; scores in shared memory.  Sequences too long for a tile of rows.
+// One warp per query row; scores in shared memory.  Sequences too long for a tile of rows, and short ones of many heads.
 template <typename T>
 __global__ void attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                                       T* __restrict__ o, int Tn, int H, int dk, float scale) {
@@ -679,6 +679,25 @@ int launch_attention_tc(const void* q, const void* k, const void* v, void* o, in
     return CONVNN_OK;
 }
 
+// Sequences of up to 20 tokens (28 of many narrow bfloat16 heads): a tile of `rows` rows takes its chain of chunks whatever it holds,
+// two at a time on an SM, while a warp per row waits for one row's dot products and shares the SM with many.  us of both, fits to 190
+// and 221 shapes of 2 to 40 tokens (rms 10 %) and 150 of up to 26 (18 %); the choice costs 0.3 % over the better of the two on average.
+// Tile -> row per warp, us of the attention alone: 4854 heads of 2 tokens x 8 70.9 -> 6.9, 1551 x 2 x 24 24.9 -> 4.1, 5904 x 2 x 192 225 -> 39,
+// 3730 x 4 x 40 71 -> 13.7, 3978 x 7 x 24 60 -> 22, 4608 x 9 x 24 91 -> 37; few heads, 120 x 2 x 8 5.0 -> 2.9; bfloat16 with the projections 4205 x 20 x
+// 24 170 -> 114, 1188 x 26 x 8 55 -> 43.  The other way 108 x 9 x 256 29 -> 18, 1440 x 10 x 160 115 -> 60, 585 x 15 x 160 116 -> 25, float32 3600 x 20
+// x 32 190 -> 105.  (One token of few heads has the tile whatever it costs: 4 us.)
+bool row_per_warp(int heads, int Tn, int dk, int rows, bool bf16) {
+    if (rows == 0) return false;
+    const long long tiles = (long long)heads * ((Tn + rows - 1) / rows), at_once = 2ll * device_sms();
+    const bool narrow = bf16 && dk <= 64;
+    if (Tn > (narrow && tiles > 3 * at_once ? 28 : 20) || (Tn == 1 && tiles <= at_once)) return false;
+    const double round = rows == 8 ? 3.9 + 0.042 * dk : rows == 16 ? 4.5 + 0.048 * dk + 0.04 * Tn : 6.5 + 0.059 * dk + 0.077 * Tn;
+    const double tile = round * ((tiles + at_once - 1) / at_once);
+    const double chain = 2.7 + dk * (0.017 + 0.0077 * Tn);
+    const double work = (narrow ? 0.65 : 1.0) * heads * Tn / device_sms() * (0.03 + dk * (0.0021 + 0.0004 * Tn));
+    return chain * chain + work * work < (tiles <= at_once ? 0.8 : 1.1) * tile * tile;
+}
+
 template <typename T>
 int launch_attention_simt_t(const void* q, const void* k, const void* v, void* o, int B, int Tn, int D, int H,
                             cudaStream_t st) {
@@ -695,6 +714,7 @@ int launch_attention_simt_t(const void* q, const void* k, const void* v, void* o
             least = cost;
         }
     }
+    if (row_per_warp(B * H, Tn, dk, rows, sizeof(T) == 2)) rows = 0;
     if (rows == 8) return launch_tile<T, 1>(q, k, v, o, B, Tn, H, dk, scale, st);
     if (rows == 16) return launch_tile<T, 2>(q, k, v, o, B, Tn, H, dk, scale, st);
     if (rows == 40) return launch_tile<T, 5>(q, k, v, o, B, Tn, H, dk, scale, st);

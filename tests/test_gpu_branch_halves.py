@@ -169,3 +169,26 @@ def test_softmax_attention_tiles(B, T, D, H, dtype):
     call = lambda: ops.softmax_attention(x_dev, w_qkv, w_o, H)
     assert any("attention_tile_kernel" in n for n in launches(call)) == (T < 6000)
     assert rel_err(call(), softmax_attention(x, w, H)) < (1e-4 if dtype == torch.float32 else 2e-2)
+
+
+# Short sequences of many heads: a warp per row; the same sequences by themselves: a tile of rows.  Both give the same bits.
+@on_148_sms
+@pytest.mark.parametrize("B,T,D,H,few,dtype", [
+    (4854, 2, 8, 1, 16, torch.bfloat16), (500, 7, 192, 3, 2, torch.float32), (1500, 9, 48, 2, 2, torch.bfloat16),
+    (700, 11, 24, 1, 16, torch.float32), (800, 20, 8, 1, 16, torch.float32), (1000, 1, 40, 1, 16, torch.float32)])
+def test_softmax_attention_of_short_sequences(B, T, D, H, few, dtype):
+    g = torch.Generator().manual_seed(T + D)
+    w = {f"W_{n}.weight": _uni((D, D), D, g) * (3.0 if n in "qk" else 1.0) for n in "qkvo"}
+    x = torch.randn(B, T, D, generator=g)
+    if dtype == torch.bfloat16:
+        w = {n: bf16_round(t) for n, t in w.items()}
+        x = bf16_round(x)
+    w_qkv = torch.stack([w[f"W_{n}.weight"] for n in "qkv"]).to(DEV, dtype)
+    x_dev, w_o = x.to(DEV, dtype), w["W_o.weight"].to(DEV, dtype)
+    call = lambda n=B: ops.softmax_attention(x_dev[:n], w_qkv, w_o, H)
+    assert any("attention_simt_kernel" in n for n in launches(call))
+    got = call()
+    assert rel_err(got[:64], softmax_attention(x[:64], w, H)) < (1e-4 if dtype == torch.float32 else 2e-2)
+    if T > 8 or T == 1:
+        assert any("attention_tile_kernel" in n for n in launches(lambda: call(few)))
+        assert torch.equal(call(few), got[:few])
