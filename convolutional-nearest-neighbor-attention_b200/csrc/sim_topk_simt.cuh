@@ -62,8 +62,10 @@ __device__ __forceinline__ float4 load_upto4(const T* p, int n, bool vec) {
     return make_float4(r[0], r[1], r[2], r[3]);
 }
 
+// (Two CTAs of 64 rows fit an SM: the other lists keep to 128 registers by themselves, 26 to 32 neighbours took 160 and ran one at a time:
+// us, so -> bounded, bfloat16 20 x 439 x 439 x 97 242 -> 143, 17 x 570 x 570 x 8 201 -> 123, float32 21 x 624 x 624 x 8 209 -> 132.  0: not stated.)
 template <typename T, int KCAP, int RB>
-__global__ void __launch_bounds__(NT) sim_topk_simt_kernel(
+__global__ void __launch_bounds__(NT, RB == 64 && KCAP > 25 ? 2 : 0) sim_topk_simt_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const float* __restrict__ qstat,
     const float* __restrict__ kstat, const int32_t* __restrict__ cand, int32_t* __restrict__ idx,
     float* __restrict__ val, int T_, int S, int H, int Cp, int K, int nsel, int metric, int sampled,

@@ -48,8 +48,9 @@ def rel_err(a, b):
     return float((a - b).norm() / b.norm().clamp_min(1e-30))
 
 
-def launches(fn):
-    """{kernel name (mangled): bytes of local memory per thread} of what fn() launches, read from a captured graph."""
+def launches(fn, attribute="LOCAL_SIZE_BYTES"):
+    """{kernel name (mangled): bytes of local memory per thread, or another attribute} of what fn() launches, read from a
+    captured graph."""
     from cuda.bindings import driver
 
     def ok(r):
@@ -70,6 +71,6 @@ def launches(fn):
         p = ok(driver.cuGraphKernelNodeGetParams(node))[0]
         func = p.func if int(p.func) else ok(driver.cuKernelGetFunction(p.kern))[0]
         found[ok(driver.cuFuncGetName(func))[0].decode()] = ok(driver.cuFuncGetAttribute(
-            driver.CUfunction_attribute.CU_FUNC_ATTRIBUTE_LOCAL_SIZE_BYTES, func))[0]
+            getattr(driver.CUfunction_attribute, "CU_FUNC_ATTRIBUTE_" + attribute), func))[0]
     graph.reset()
     return found

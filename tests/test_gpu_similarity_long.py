@@ -119,3 +119,15 @@ def test_columns_shared_by_a_cluster(B, T, S, H, dk, K, values, dtype=torch.bflo
 @pytest.mark.parametrize("values", ["ties", "many", "rising", "nan"])
 def test_columns_shared_by_a_cluster_float32(B, T, S, H, dk, K, values):
     test_columns_shared_by_a_cluster(B, T, S, H, dk, K, values, torch.float32, "sim_topk_simt_kernel")
+
+
+# 64 rows per CTA: the rule that shares columns counts on two CTAs per SM, also with the longest lists.
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("K", [4, 9, 16, 25, 32])
+def test_two_blocks_of_64_rows_fit_an_sm(K, dtype):
+    spec = ops.LayerSpec(97, 1, K, "all", "matmul", "depthwise", True, False, 439)
+    q, k = (torch.ones(20, 439, 1, 97, device=DEV, dtype=dtype) for _ in "qk")
+    regs = launches(lambda: ops.sim_topk(spec, q, k, None, None), "NUM_REGS")
+    assert len(regs) == 1
+    name, n = regs.popitem()
+    assert "sim_topk_simt_kernel" in name and "Li64EEE" in name and 2 * 256 * ((n + 7) // 8 * 8) <= 65536
