@@ -674,6 +674,8 @@ int launch_plain_f32(const GemmParams& p, cudaStream_t st) {
 // bfloat16, transposed tiles only -> now: 4 x 197 x 768 x 768 130 -> 55; 2080 x 384 x 388 57.9 -> 27.8.
 // The 128 x 64 tile, once it waits for no conversion, is the best of five on most large outputs of bfloat16 rows read four at a time and of mixed ones (27 shapes; the fits
 // hold within 10 %), us: 4925 x 2304 x 768 468 -> 399, 25216 x 192 x 192 64 -> 54, mixed 4925 x 768 x 769 215 -> 176.
+// Six 32 x 32 tiles fit an SM with the 136 to 138 registers that rows kept as they came take, eight with 128: bounded where there are more than
+// six, 36230 x 96 x 9 14.1 -> 12.4 us, 21446 x 192 x 9 16.1 -> 14.5, 15506 x 64 x 196 22.3 -> 19.8; few lose a little (785 x 192 x 12 3.9 -> 4.1).
 template <typename TA, typename T, int MODE>
 int launch_plain_staged(const GemmParams& p, cudaStream_t st) {
     if constexpr (sizeof(T) == 4) {
@@ -713,7 +715,10 @@ int launch_plain_staged(const GemmParams& p, cudaStream_t st) {
         };
         switch (sizeof(TA) == 4 ? cheapest_tile(mixed, p) : p.a_vec && p.w_vec ? cheapest_tile(by_four, p) : cheapest_tile(by_value, p, 1)) {
             case 0: return launch_tile<TA, T, MODE, 128, 64, 16, 8, 8, 3>(p, st);
-            case 1: return launch_tile<TA, T, MODE, 32, 32, 32, 4, 4, 4>(p, st);
+            case 1:
+                if ((long long)((p.M + 31) / 32) * ((p.N + 31) / 32) > 6ll * device_sms())
+                    return launch_tile<TA, T, MODE, 32, 32, 32, 4, 4, 8>(p, st);
+                return launch_tile<TA, T, MODE, 32, 32, 32, 4, 4, 4>(p, st);
             case 2: return launch_stage_tile<TA, T, MODE, 64, 64, 8, 4, 3>(p, st);
             case 3: return launch_stage_tile<TA, T, MODE, 32, 64, 4, 4, 4>(p, st);
             default: return launch_stage_tile<TA, T, MODE, 40, 32, 5, 4, 6>(p, st);

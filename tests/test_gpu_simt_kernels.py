@@ -318,3 +318,13 @@ def test_large_tile_of_mixed_rows(B, T, dk):
     assert any(re.search(r"gemm_simt_kernelIf13__nv_bfloat16Li\dELi128ELi64E", n) for n in launches(call))
     got = call()
     assert torch.equal(call(2), got[:2])                             # (two images take smaller tiles: the same sums)
+
+
+# The smallest tile on bfloat16 and mixed rows: its times are for eight of them on an SM.
+@pytest.mark.parametrize("M,N,K", [(37529, 32, 9), (4880, 192, 20)])
+def test_eight_small_tiles_fit_an_sm(M, N, K):
+    a, w = torch.ones(M, K, dtype=torch.bfloat16, device=DEV), torch.ones(N, K, dtype=torch.bfloat16, device=DEV)
+    regs = {n: r for n, r in launches(lambda: ops.linear(a, w), "NUM_REGS").items() if "gemm_simt_kernel" in n}
+    (name, r), = regs.items()
+    assert "Li32ELi32ELi32ELi4ELi4E" in name and 8 * 64 * ((r + 7) // 8 * 8) <= 65536
+    assert bool((ops.linear(a, w) == K).all())
