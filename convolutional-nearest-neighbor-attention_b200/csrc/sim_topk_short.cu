@@ -6,7 +6,9 @@
 //   pass 2  the columns whose key reaches the bound (of 197 about 10 for K = 9, 29 for K = 25) are appended, in column order, to the
 //           row's entries in shared memory, without a branch on how many there are.
 //   rank    a network sorts the entries (packed_rank.cuh); the earlier column wins ties.
-//           A row with more entries than it has room for takes the columns above the bound chunk by chunk.
+//           A row with more entries than it has room for takes, if its list is long, the nsel-th largest of those it has as its bound
+//           and repeats pass 2 (some 47 of 256 columns reach the first bound for K = 32, 3 more or less, where there is room for 51);
+//           where that does not do either (ties), and short lists at once, the columns above the bound chunk by chunk, 15 us more.
 //
 // The results are the streaming kernels' bit for bit.
 //
@@ -121,10 +123,13 @@ __device__ __forceinline__ void insert_first(TopList<NSEL>& top, const E& entry,
 }
 
 // Lists of more than twelve are ranked by a network (one thread per row); the entries a row has room for (checked every eight columns).
+// 59 leave the ring two stages of 64 channels with 256 candidates, 60 one (us, one stage and no second bound -> two and a second bound:
+// 87 images of 256 x 256 x 128, K = 30 38.8 -> 25.4, 105 x 2 x 242 x 242 x 192, K = 26 45 -> 41; 68 x 243 x 243 x 192, K = 32 40 -> 27, 10 x 6 heads of 239 x
+// 239 x 128 38 -> 26; sorted lists of values 33).
 template <int NSEL>
 constexpr bool networked = NSEL > 12;
 template <int NSEL, int NH>
-constexpr int slots_of = NSEL <= 12 ? (NH == 2 ? 28 : 32) : NSEL <= 16 ? 36 : NSEL <= 25 ? 52 : 60;
+constexpr int slots_of = NSEL <= 12 ? (NH == 2 ? 28 : 32) : NSEL <= 16 ? 36 : NSEL <= 25 ? 52 : 59;
 
 template <int NSEL, int G, int NH, int METRIC, Way WAY>
 __global__ void __launch_bounds__(64 + 128 * G * NH, 1)
@@ -453,28 +458,45 @@ sim_topk_short_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
                         for (int i = 0; i < NSEL - 1; ++i)
                             if (i < p.nsel - 1) thr = fmaxf(thr, fminf(v[i], of_even(p.nsel - 2 - i)));
                     }
-                    // Pass 2: the columns that reach it.
-                    constexpr uint32_t ROOM = (SLOTS - 8) * ENTRY;
-                    bool over = false;
+                    // Pass 2: the columns that reach it.  A row that has no room for them all takes the nsel-th largest of those it has
+                    // room for as its bound, which nsel columns reach too, and once more the columns that reach that.
+                    constexpr int FULL = SLOTS - 8;
+                    constexpr uint32_t ROOM = FULL * ENTRY;
+                    bool over;
 #pragma unroll 1
-                    for (int c = 0; c < p.S; c += 16) {
-                        uint32_t acc[16];
-                        tmem_ld_x16(taddr + c, acc);
-                        tmem_ld_wait();
-                        float key[16];
-                        make_keys<16, METRIC, true>(key, acc, qs, cs, c, p, row, sentinel);
+                    for (int attempt = 0;; ++attempt) {
+                        over = false;
+                        at = hit0;
+#pragma unroll 1
+                        for (int c = 0; c < p.S; c += 16) {
+                            uint32_t acc[16];
+                            tmem_ld_x16(taddr + c, acc);
+                            tmem_ld_wait();
+                            float key[16];
+                            make_keys<16, METRIC, true>(key, acc, qs, cs, c, p, row, sentinel);
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            if (j % 8 == 0) {
-                                over = over || at > hit0 + ROOM;
-                                at = min(at, hit0 + ROOM);
-                            }
-                            if (key[j] >= thr) {
-                                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(__float_as_uint(key[j])), "r"(c + j)
-                                             : "memory");
-                                at += ENTRY;
+                            for (int j = 0; j < 16; ++j) {
+                                if (j % 8 == 0) {
+                                    over = over || at > hit0 + ROOM;
+                                    at = min(at, hit0 + ROOM);
+                                }
+                                if (key[j] >= thr) {
+                                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(__float_as_uint(key[j])), "r"(c + j)
+                                                 : "memory");
+                                    at += ENTRY;
+                                }
                             }
                         }
+                        over = over || at > hit0 + ROOM;
+                        if (attempt == 1 || !__any_sync(0xffffffffu, over && row_ok)) break;
+                        float q[FULL];
+#pragma unroll
+                        for (int n = 0; n < FULL; ++n) q[n] = lds_key(hit0 + n * ENTRY);
+                        sort_descending(q);
+                        float tight = q[0];
+#pragma unroll
+                        for (int s = 1; s < NSEL; ++s) tight = fminf(tight, s < p.nsel ? q[s] : CUDART_INF_F);
+                        if (over) thr = fmaxf(thr, tight);
                     }
                     // Too many of them (ties), fewer than nsel keys above -inf (NaN inputs), keys of +inf: the row takes the columns
                     // above the bound chunk by chunk.

@@ -309,3 +309,41 @@ def test_ranked_entries(B, T, S, H, dk, K, values):
     want_val = want_key / torch.tensor(math.sqrt(dk), dtype=torch.float32, device=DEV)
     # one division: equal up to its rounding
     assert bool(((val[..., K - n:] - want_val).abs() <= 2.0 ** -22 * want_val.abs())[real].all())
+
+
+# Lists of more than twelve whose first bound more columns reach than a row has entries: the best columns lie in few groups of maxima
+# ("few groups"), the good ones come last ("rising"), so that the tighter bound is no help either, or first ("falling"), or tie there ("steps").
+@on_148_sms
+@pytest.mark.parametrize("B,T,S,dk", [(60, 256, 256, 64), (50, 300, 241, 96), (100, 128, 128, 64), (200, 65, 65, 32), (70, 255, 255, 384)])
+@pytest.mark.parametrize("K", [13, 16, 17, 25, 31, 32])
+@pytest.mark.parametrize("values", ["few groups", "rising", "falling", "steps", "nan", "inf"])
+def test_more_columns_at_the_bound_than_entries(B, T, S, dk, K, values):
+    sampled = S != T
+    n = K - 1 if sampled else K
+    g = torch.Generator(device=DEV).manual_seed(T * 1000 + S + K)
+    q, k = (torch.randint(-2, 3, (B, r, 1, dk), device=DEV, generator=g).float() for r in (S, T))
+    c = torch.arange(S, device=DEV)
+    worth = {"rising": c, "falling": S - c, "steps": c // 8 * 8}.get(values, torch.randperm(S, device=DEV, generator=g))
+    if values not in ("rising", "falling", "steps"):
+        worth = worth + 256 * (c % 64 < 16)
+    q[..., 0], k[..., 0] = (worth // 16).float().view(1, S, 1), 256.0     # 16 worth, and noise of up to 4 per other channel
+    q[..., 1], k[..., 1] = (worth % 16).float().view(1, S, 1), 16.0
+    if values == "nan":
+        q[:, ::5] = math.nan
+    if values == "inf":
+        q[::2, 7, :, 2], k[..., 2] = math.inf, 1.0
+    spec = ops.LayerSpec(dk, 1, K, "spatial" if sampled else "all", "matmul", "depthwise", True, False, T)
+    cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if sampled else None
+    call = lambda: ops.sim_topk(spec, q.bfloat16(), k.bfloat16(), None, None, cand)
+    assert any("sim_topk_short_kernel" in name for name in launches(call))
+    idx, val = call()
+    key = torch.einsum("bthc,bshc->bhts", k.double(), q.double()).float()
+    if sampled:
+        own = cand.view(1, 1, 1, S).long() == torch.arange(T, device=DEV).view(1, 1, T, 1)
+        key = torch.where(own, torch.full_like(key, -0.1) * torch.tensor(math.sqrt(dk), dtype=torch.float32, device=DEV), key)
+    want_idx, want_key = expect(key, n)
+    assert torch.equal(idx.long()[..., K - n:], want_idx if cand is None else cand.long()[want_idx])
+    real = (want_key.abs() < math.inf) & ~((want_key < 0) & (val[..., K - n:] == -0.1))
+    want_val = want_key / torch.tensor(math.sqrt(dk), dtype=torch.float32, device=DEV)
+    # one division: equal up to its rounding
+    assert bool(((val[..., K - n:] - want_val).abs() <= 2.0 ** -22 * want_val.abs())[real].all())
