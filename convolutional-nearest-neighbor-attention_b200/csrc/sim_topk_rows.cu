@@ -431,6 +431,12 @@ static Ranges ranges_of(const Dims& dm) {
 //   197 x 197, one head of 96, K = 9   20 images 9.3, 7.1   38: 9.4, 9.2   64: 9.7, 10.6   150: 17.6, 21.0;  3 heads of 32   64: 17.4, 22.1
 //   K = 5   20: 8.4, 7.0   38: 8.6, 8.8   64: 8.8, 10.2        K = 16   20: 12.7, 8.1   38: 13.3, 12.0   64 x 3 heads of 64: 23.5, 36.6
 //   197 x 197 x 192, K = 25   1 image 16.8, 8.2   20: 16.8, 10.0   34: 17.8, 13.9      65 x 65 x 192   80: 13.0, 13.5   100: 14.2, 13.5
+// Row tiles of 128 pad longer sequences, and candidates that are not the rows themselves cost the two-pass kernel more: lists of up to twelve
+// keep this kernel longer beyond 256 tokens (two-pass, this kernel, us).
+//   K = 9    13 x 969 x 254 x 64 13.3, 9.9   35 x 330 x 206 x 32 12.0, 9.4   18 x 893 x 253 x 32 13.0, 10.6   14 x 677 x 210, two heads of 64 12.0, 13.5
+//            12 x 843 x 188 x 256 11.5, 9.6   20 x 680 x 207 x 256 12.5, 14.7
+// (Rows whose survivors overflow cost this kernel 5 us and a launch has them or not.  For lists of 13 to 16 that decides between 64 and 112
+// rows per SM, 150 shapes 0.7 to 1.5 times the two-pass kernel's time and as often the one as the other: left at 64.)
 // The line of lists of five to twelve with one head of 129 to 192 channels has not been drawn again (132 images 12.3, 18.8).
 // Where others win, and the lines of the rule (R rows per SM, rounds u of 256-row units per SM, w the share of their warps that
 // has rows: two units of the streaming kernel share an SM and slow each other down by about w / 2):
@@ -447,7 +453,7 @@ bool sim_topk_rows_wanted(const Dims& dm) {
     const bool other_width = dm.Cp <= 128 || dm.Cp > 192;
     if (dm.nsel > 12) return R <= (other_width || dm.S < 176 ? 64 : 96);
     if (dm.Cp > 192 && dm.S > 208 && dm.T > 256) return R <= 96;
-    if (dm.nsel >= 4 && dm.S >= 176 && other_width && (dm.Cp <= 128 || dm.S <= 208)) return R <= (dm.S > 208 ? 80 : 64);
+    if (dm.nsel >= 4 && dm.S >= 176 && other_width && (dm.Cp <= 128 || dm.S <= 208)) return R <= (dm.T > 256 && dm.Cp <= 128 ? 112 : dm.S > 208 || (dm.T > 256 && dm.nsel > 4) ? 80 : 64);
     if (dm.nsel > 4 && dm.S >= 176) return R <= 304;
     const int units_of = (dm.T + 255) / 256;
     const double u = (double)dm.B * dm.H * units_of / device_sms(), w = (double)((dm.T + 31) / 32) / (8 * units_of);

@@ -314,7 +314,7 @@ def test_ranked_entries(B, T, S, H, dk, K, values):
 # Lists of more than twelve whose first bound more columns reach than a row has entries: the best columns lie in few groups of maxima
 # ("few groups"), the good ones come last ("rising"), so that the tighter bound is no help either, or first ("falling"), or tie there ("steps").
 @on_148_sms
-@pytest.mark.parametrize("B,T,S,dk", [(60, 256, 256, 64), (50, 300, 241, 96), (100, 128, 128, 64), (200, 65, 65, 32), (70, 255, 255, 384)])
+@pytest.mark.parametrize("B,T,S,dk", [(60, 256, 256, 64), (60, 300, 241, 96), (100, 128, 128, 64), (200, 65, 65, 32), (70, 255, 255, 384)])
 @pytest.mark.parametrize("K", [13, 16, 17, 25, 31, 32])
 @pytest.mark.parametrize("values", ["few groups", "rising", "falling", "steps", "nan", "inf"])
 def test_more_columns_at_the_bound_than_entries(B, T, S, dk, K, values):
@@ -347,3 +347,12 @@ def test_more_columns_at_the_bound_than_entries(B, T, S, dk, K, values):
     want_val = want_key / torch.tensor(math.sqrt(dk), dtype=torch.float32, device=DEV)
     # one division: equal up to its rounding
     assert bool(((val[..., K - n:] - want_val).abs() <= 2.0 ** -22 * want_val.abs())[real].all())
+
+
+# Lines between the two-pass and the warp-per-row kernel: either side of each.
+@on_148_sms
+@pytest.mark.parametrize("B,T,S,dk,K,rows", [
+    (13, 900, 250, 64, 9, True), (20, 900, 250, 64, 9, False), (18, 900, 190, 32, 6, True), (20, 900, 190, 32, 6, False),
+    (13, 860, 190, 256, 9, True), (16, 860, 190, 256, 9, False)])
+def test_warp_per_row_or_two_passes(B, T, S, dk, K, rows):
+    test_warp_per_row_routes(B, T, S, 1, dk, K, torch.bfloat16, rows)
