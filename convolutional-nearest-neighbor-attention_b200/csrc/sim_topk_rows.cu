@@ -437,6 +437,10 @@ static Ranges ranges_of(const Dims& dm) {
 //            12 x 843 x 188 x 256 11.5, 9.6   20 x 680 x 207 x 256 12.5, 14.7
 // (Rows whose survivors overflow cost this kernel 5 us and a launch has them or not.  For lists of 13 to 16 that decides between 64 and 112
 // rows per SM, 150 shapes 0.7 to 1.5 times the two-pass kernel's time and as often the one as the other: left at 64.)
+// Long lists among up to 64 candidates, where most of them are listed (K = 17 to 32; two-pass, this kernel): up to one unit of the two-pass
+// kernel per SM   27 x 281 x 30 x 64 13.5, 9.6   12 x 822 x 32 x 128 16.5, 12.5   37 x 272 x 49 x 64 14.7, 12.3   39 x 341 x 58 x 768 16.5, 19.4 (90 rows per SM, not
+// taken);  short sequences, whose units are mostly padding   174 x 50, six heads of 768 122, 76   1144 x 22, three heads of 64 131, 83   28 x 131,
+// three heads of 128 21.9, 14.6;  but 195 x 57 x 23, six heads of 192 47, 57   175 x 58, six heads of 768 63, 68   186 x 45 x 192 12.6, 13.5.
 // The line of lists of five to twelve with one head of 129 to 192 channels has not been drawn again (132 images 12.3, 18.8).
 // Where others win, and the lines of the rule (R rows per SM, rounds u of 256-row units per SM, w the share of their warps that
 // has rows: two units of the streaming kernel share an SM and slow each other down by about w / 2):
@@ -448,7 +452,11 @@ static Ranges ranges_of(const Dims& dm) {
 bool sim_topk_rows_wanted(const Dims& dm) {
     if (dm.S > 256) return false;
     const int R = rows_per_sm(dm);
-    if (dm.nsel > 16) return R <= 48;
+    if (dm.nsel > 16) {
+        const long long two_pass_units = (long long)dm.B * dm.H * ((dm.T + 127) / 128);
+        if ((dm.T <= 40 && dm.S <= 32) || (dm.T <= 56 && dm.Cp >= 512)) return R <= 512;
+        return R <= (dm.S <= 64 && two_pass_units <= device_sms() ? 80 : 48);
+    }
     if (dm.S <= 128 || dm.Cp > 384) return R <= 48 && ranges_of(dm).per_head;
     const bool other_width = dm.Cp <= 128 || dm.Cp > 192;
     if (dm.nsel > 12) return R <= (other_width || dm.S < 176 ? 64 : 96);

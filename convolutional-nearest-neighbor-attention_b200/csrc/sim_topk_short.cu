@@ -610,7 +610,10 @@ int launch_short(const Dims& dm, ShortParams& p, const CUtensorMap& tmK, const C
 }  // namespace
 
 // What the warp-per-row kernel leaves to it.  Anything of up to one unit per SM (48 x 197 x 197 x 192, K = 25 33.8, 23.0); lists of more
-// than twelve (streaming 256 x 577 x 150 x 384, K = 16 129, here 67; 57 x 12 x 197 x 197 x 32, K = 25 171, 84); lists of up to twelve except where the streaming kernel's 256-row units are fewer and the bound saves little (us, streaming, this kernel):
+// than twelve (streaming 256 x 577 x 150 x 384, K = 16 129, here 67; 57 x 12 x 197 x 197 x 32, K = 25 171, 84) except, beyond sixteen, where they hold most of up
+// to 40 candidates and about half as many rounds of units stream (streaming, this kernel: 94 x 153 x 23 x 768, K = 20 13.8, 21.5; 143 x 172 x 38 x 32, K =
+// 28 16.4, 19.4; 20 x 187 x 28 x 6 x 96, K = 28 14.5, 18.7; 32 x 574 x 18 x 3 x 512, K = 18 22.6, 30.7; 32 x 175 x 39 x 12 x 384, K = 27 44.7, 69.3; 316 x 131 x 27 x
+// 256, K = 27 30, 36; but 77 x 685 x 47 x 32, K = 17 25.3, 15.8; 84 x 654 x 31 x 64, K = 17 21.1, 15.9; 47 x 886 x 36 x 256, K = 25 32, 28); lists of up to twelve except where the streaming kernel's 256-row units are fewer and the bound saves little (us, streaming, this kernel):
 //   * few candidates: of sequences that fill more than one unit here (512 x 197 x 16 x 192, K = 4 10.8, 14.4; 256 x 197 x 32 x 768, K = 3
 //     19.6, 21.9), and of others where heads are wide, lists long or the second round of units thin (1000 x 17 x 17 x 512, K = 2 19.5, 23.6;
 //     200 x 100 x 20 x 384, K = 5 8.6, 9.6; 163 x 65 x 65 x 128, K = 12 13.4, 14.6; but 1000 x 17 x 17 x 64 0.65 of the time, 340 x 25 x 25 x 192 0.85, and
@@ -621,7 +624,12 @@ bool sim_topk_short_wanted(const Dims& dm) {
     if (dm.S > 256) return false;
     const long long sms = device_sms(), bh = (long long)dm.B * dm.H, units = bh * ((dm.T + BM - 1) / BM);
     if (units <= sms) return true;
-    if (dm.nsel > 12) return true;
+    if (dm.nsel > 12) {
+        const long long streaming = bh * ((dm.T + 2 * BM - 1) / (2 * BM));
+        const long long here = (units + sms - 1) / sms, there = (streaming + sms - 1) / sms;
+        const bool half = here >= 2 * there || (dm.T <= BM + 32 && 5 * here >= 8 * there);
+        return !(dm.nsel > 16 && dm.S <= 40 && dm.T > BM && half && (there == 1 ? 2 : 1) * dm.nsel * 3 >= 2 * dm.S);
+    }
     if (dm.T > BM && dm.S <= 32) return false;
     if (dm.T <= BM && dm.S <= 40) {
         if (dm.Cp > 512) return true;

@@ -356,3 +356,27 @@ def test_more_columns_at_the_bound_than_entries(B, T, S, dk, K, values):
     (13, 860, 190, 256, 9, True), (16, 860, 190, 256, 9, False)])
 def test_warp_per_row_or_two_passes(B, T, S, dk, K, rows):
     test_warp_per_row_routes(B, T, S, 1, dk, K, torch.bfloat16, rows)
+
+
+# The same for long lists among few candidates, with the streaming kernel where it takes half the rounds.
+@on_148_sms
+@pytest.mark.parametrize("B,T,S,H,dk,K,kernel", [
+    (27, 281, 30, 1, 64, 24, "rows"), (29, 385, 64, 1, 64, 18, "rows"), (37, 385, 64, 1, 64, 18, "short"),
+    (50, 40, 20, 6, 32, 18, "rows"), (50, 41, 20, 6, 32, 18, "short"), (50, 50, 50, 6, 512, 30, "rows"), (50, 50, 50, 6, 496, 30, "short"),
+    (148, 172, 40, 1, 32, 28, "tc"), (149, 172, 40, 1, 32, 28, "short"), (148, 172, 41, 1, 32, 28, "short"), (135, 132, 28, 2, 16, 28, "tc"),
+    (300, 140, 28, 1, 16, 28, "tc"), (300, 161, 28, 1, 16, 28, "short"), (148, 172, 40, 1, 32, 18, "tc"), (135, 172, 31, 2, 16, 18, "short"), (32, 574, 18, 3, 512, 18, "tc"), (94, 153, 23, 1, 768, 17, "short")])
+def test_long_lists_among_few_candidates(B, T, S, H, dk, K, kernel):
+    g = torch.Generator(device=DEV).manual_seed(T + S + K)
+    sampled, n = S != T, K - (S != T)
+    spec = ops.LayerSpec(H * dk, H, K, "spatial" if sampled else "all", "matmul", "depthwise", True, False, T)
+    q, k = (torch.randint(-11, 12, (B, r, H, dk), device=DEV, generator=g).bfloat16() for r in (S, T))
+    cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if sampled else None
+    call = lambda: ops.sim_topk(spec, q, k, None, None, cand)
+    name, = launches(call)
+    assert f"sim_topk_{kernel}_kernel" in name
+    key = torch.einsum("bthc,bshc->bhts", k.double(), q.double()).float()        # whole numbers: exact
+    if sampled:
+        own = cand.view(1, 1, 1, S).long() == torch.arange(T, device=DEV).view(1, 1, T, 1)
+        key = torch.where(own, torch.full_like(key, -0.1) * torch.tensor(math.sqrt(dk), dtype=torch.float32, device=DEV), key)
+    want_idx, _ = expect(key, n)
+    assert torch.equal(call()[0].long()[..., K - n:], want_idx if cand is None else cand.long()[want_idx])
