@@ -311,12 +311,36 @@ bool sim_topk_tc_supported(const convnn_desc* d, const Dims& dm, const void* q, 
     return d->dtype == CONVNN_BF16 && dm.Cp % 16 == 0 && aligned16(q) && aligned16(k);
 }
 
+// A cluster stays within a GPC: of CTAs that fill an SM each 15 clusters of eight run at once on 148 SMs, 33 of four, 74 of two.
+static int clusters_at_once(int split) {
+    static ClusterLimit fit[MAX_SPLIT + 1]{};
+    auto kern = sim_topk_tc_kernel<32, 1, 32>;
+    const size_t smem = 160 * 1024;
+    static SmemLimit limit{};
+    if (limit.ensure(reinterpret_cast<const void*>(kern), smem) != CONVNN_OK) return 0;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(split); cfg.blockDim = dim3(NTHREADS); cfg.dynamicSmemBytes = smem; cfg.attrs = attr; cfg.numAttrs = 1;
+    int n = 0;
+    return fit[split].query(reinterpret_cast<const void*>(kern), &cfg, &n) == CONVNN_OK ? n : 0;
+}
+
+// The small shape: two CTAs of 64-column tiles per SM.  (Heads of 257-512 channels on short sequences: 19.3 against 22.8 us at B=256, T=197,
+// S=64, d_k=384; with 768 channels it measured slower.)
+static bool small_shape(const Dims& dm) { return dm.nsel <= 12 && (dm.Cp <= 256 || (dm.Cp <= 512 && dm.T <= 512)); }
+
 // CTAs that share the columns of a unit where the units alone leave most SMs idle (a unit's time goes with its columns; us, one CTA per
-// unit, a cluster): 2 x 2048 x 2048 x 256, K = 25 125, 85; 4 x 1366 x 632 x 192, K = 9 47, 23; 577 x 577 x 384 34, 15; 14 x 624 x 624 x 256, K = 16
-// 47, 36; 2048 x 2048 x 256, K = 32 149, 53.  Lists and their merge cost about 3 us: not for less than 128 columns each.
+// unit, a cluster): 2 x 2011 x 2011 x 256, K = 25 130, 60; 4 x 1366 x 632 x 192, K = 9 47, 23; 577 x 577 x 384 34, 15; 14 x 624 x 624 x 256, K = 16
+// 47, 36; 2048 x 2048 x 256, K = 32 149, 53.  At least 64 columns each (fewer are faster still: 283 x 283 x 64, K = 3, four
+// CTAs 11.5, eight 8.9).  All clusters have to run at once, a second round costs as much as the first: eight CTAs, four: 2 x 1929 x
+// 1929 x 384, K = 16 60, 45; 4416 x 4416 x 384, K = 5 67, 54; four, two: 2 x 3722 x 4440 x 384, K = 25 167, 119.
 static int split_of(const Dims& dm, int n_units) {
     int split = 1;
-    while (split < MAX_SPLIT && n_units * 2 * split <= device_sms() && dm.S >= 128 * split) split *= 2;
+    while (split < MAX_SPLIT && n_units * 2 * split <= device_sms() && dm.S >= 128 * split &&
+           (small_shape(dm) || n_units <= clusters_at_once(2 * split)))
+        split *= 2;
     return split;
 }
 
@@ -324,9 +348,10 @@ int launch_sim_topk_tc(const convnn_desc* d, const Dims& dm, const void* q, cons
                        const float* kstat, const int32_t* cand, int32_t* idx, float* val, cudaStream_t st) {
     if (sim_topk_rows_wanted(dm)) return launch_sim_topk_rows(d, dm, q, k, qstat, kstat, cand, idx, val, st);
     if (sim_topk_short_wanted(dm)) return launch_sim_topk_short(d, dm, q, k, qstat, kstat, cand, idx, val, st);
-    // (a pair of SMs per unit against a cluster of up to eight: 4096 x 4096 x 768, K = 9 85, 71 us; 2 x 4168 x 4168 x 256 83, 89; K = 16, 2 x
-    // 4042 x 4042 x 384 87, 63; heads of up to 192 channels stay with the pairs)
-    const bool few = dm.Cp > 192 && (dm.nsel > 12 ? 4ll : 8ll) * dm.B * dm.H * ((dm.T + 2 * BM - 1) / (2 * BM)) <= device_sms();
+    // A pair of SMs per unit against a cluster of four (eight of the small shape) or more: 4973 x 4744 x 768, K = 12 96, 71 us; 2 x 3396 x 3396 x 512, K = 5 70, 46; 2 x 2606 x 2606
+    // x 384, K = 12 63, 46; K = 16, 2 x 4042 x 4042 x 384 87, 63; against one of two, 2 x 4451 x 4451 x 320, K = 16 100, 111, 3 x 3029 x 3029 x 768, K = 13 83,
+    // 91; small shape, four, 2 x 4168 x 4168 x 256 83, 89.  Heads of up to 192 channels stay with the pairs.
+    const bool few = dm.Cp > 192 && split_of(dm, dm.B * dm.H * ((dm.T + 2 * BM - 1) / (2 * BM))) >= (small_shape(dm) ? 8 : 4);
     if (!few && sim_topk_tc2_wanted(d, dm)) return launch_sim_topk_tc2(d, dm, q, k, qstat, kstat, cand, idx, val, st);
     TcParams p{};
     p.qstat = qstat; p.kstat = kstat; p.cand = cand; p.idx = idx; p.val = val;
@@ -336,9 +361,7 @@ int launch_sim_topk_tc(const convnn_desc* d, const Dims& dm, const void* q, cons
     // one).
     p.KCH = dm.Cp <= 16 ? 16 : (dm.Cp <= 32 ? 32 : 64);
     p.KC = (dm.Cp + p.KCH - 1) / p.KCH;
-    // (heads of 257-512 channels on short sequences: 19.3 against 22.8 us at B=256, T=197, S=64, d_k=384;
-    // with 768 channels the small shape measured slower)
-    const bool small_cfg = dm.nsel <= 12 && (dm.Cp <= 256 || (dm.Cp <= 512 && dm.T <= 512));
+    const bool small_cfg = small_shape(dm);
     const int bn_cap = small_cfg ? 64 : 128;
     p.stages = small_cfg ? 2 : 3;
     p.n_pairs = (dm.T + 2 * BM - 1) / (2 * BM);

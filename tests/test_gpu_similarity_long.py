@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from convnn_b200 import ops
-from gpu_util import DEV, launches
+from gpu_util import DEV, launches, on_148_sms
 
 pytestmark = pytest.mark.gpu
 
@@ -131,3 +131,12 @@ def test_two_blocks_of_64_rows_fit_an_sm(K, dtype):
     assert len(regs) == 1
     name, n = regs.popitem()
     assert "sim_topk_simt_kernel" in name and "Li64EEE" in name and 2 * 256 * ((n + 7) // 8 * 8) <= 65536
+
+
+# Clusters that run at once: 15 of eight CTAs, 33 of four; beyond that fewer CTAs per unit, and a pair of SMs where it would be two.
+@on_148_sms
+@pytest.mark.parametrize("B,T,dk,K,kernel", [
+    (1, 3840, 256, 9, "sim_topk_tc_kernel"), (1, 4096, 256, 16, "sim_topk_tc_kernel"), (3, 2816, 320, 12, "sim_topk_tc_kernel"), (3, 2816, 208, 12, "sim_topk_tc2_kernel"), (2, 4352, 256, 9, "sim_topk_tc2_kernel"),
+    (2, 4352, 256, 16, "sim_topk_tc2_kernel"), (2, 4352, 256, 25, "sim_topk_tc_kernel")])
+def test_clusters_that_run_at_once(B, T, dk, K, kernel):
+    test_columns_shared_by_a_cluster(B, T, T, 1, dk, K, "many", kernel=kernel)
