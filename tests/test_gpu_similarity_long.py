@@ -140,3 +140,55 @@ def test_two_blocks_of_64_rows_fit_an_sm(K, dtype):
     (2, 4352, 256, 16, "sim_topk_tc2_kernel"), (2, 4352, 256, 25, "sim_topk_tc_kernel")])
 def test_clusters_that_run_at_once(B, T, dk, K, kernel):
     test_columns_shared_by_a_cluster(B, T, T, 1, dk, K, "many", kernel=kernel)
+
+
+# What the merged lists are written as: values of the three metrics, the sampled rows' own entry, rows that pick themselves (every euclidean
+# one, and the others where all products are negative), keys of +inf.  Whole numbers with statistics that are powers of two (cosine) or
+# exact squared norms (euclidean), so that every key is exact.
+@on_148_sms
+@pytest.mark.parametrize("B,T,S,H,dk,dtype", [
+    (1, 300, 300, 1, 64, torch.bfloat16), (3, 1020, 344, 1, 512, torch.bfloat16), (1, 2600, 1100, 1, 256, torch.bfloat16), (5, 700, 500, 2, 16, torch.bfloat16),
+    (2, 577, 577, 1, 64, torch.float32), (1, 2100, 700, 1, 20, torch.float32), (1, 333, 270, 1, 33, torch.float32)])
+@pytest.mark.parametrize("K", [4, 9, 13, 26])
+@pytest.mark.parametrize("metric,values", [("cosine", "many"), ("cosine", "negative"), ("euclidean", "many"), ("matmul", "many"), ("matmul", "negative"),
+                                           ("matmul", "inf")])
+def test_values_of_lists_shared_by_a_cluster(B, T, S, H, dk, dtype, K, metric, values):
+    g = torch.Generator(device=DEV).manual_seed(T + S + K)
+    sampled, n = S != T, K - (S != T)
+    q, k = (torch.randint(-11, 12, (B, r, H, dk), device=DEV, generator=g).float() for r in (S, T))
+    if values == "negative":
+        q, k = q.abs() + 1, -k.abs() - 1
+    if values == "inf":
+        q[:, 7::50, :, 2] = float("inf")
+        k[..., 2] = torch.where(k[..., 2] < 0, -1.0, 1.0)
+    qs, ks = (2.0 ** torch.randint(-2, 3, (B, H, r), device=DEV, generator=g).float() for r in (S, T))
+    if metric == "euclidean":
+        qs, ks = (t.pow(2).sum(-1).permute(0, 2, 1).contiguous() for t in (q, k))
+    spec = ops.LayerSpec(H * dk, H, K, "spatial" if sampled else "all", metric, "depthwise", True, False, T)
+    cand = torch.randperm(T, device=DEV, generator=g)[:S].to(torch.int32) if sampled else None
+    call = lambda: ops.sim_topk(spec, q.to(dtype), k.to(dtype), qs, ks, cand)
+    kernel = "sim_topk_tc_kernel" if dtype == torch.bfloat16 else "sim_topk_simt_kernel"
+    assert any(kernel in name for name in launches(call))
+    idx, val = call()
+    root = torch.tensor(dk, dtype=torch.float32, device=DEV).sqrt()
+    dot = torch.einsum("bthc,bshc->bhts", k.double(), q.double()).float()
+    col, row = qs.unsqueeze(2), ks.unsqueeze(3)
+    key = {"cosine": dot * col, "euclidean": 2 * dot - col, "matmul": dot}[metric]
+    if sampled:
+        own = cand.view(1, 1, 1, S).long() == torch.arange(T, device=DEV).view(1, 1, T, 1)
+        tenth = torch.tensor(-0.1, device=DEV)
+        key = torch.where(own, {"cosine": tenth / row, "euclidean": row - torch.tensor(1.21, device=DEV), "matmul": tenth * root}[metric], key)
+    ranked = torch.where(key.isnan(), -float("inf"), key).sort(dim=-1, descending=True, stable=True)
+    want_key = ranked.values[..., :n]
+    want_idx = torch.where(want_key > -float("inf"), ranked.indices[..., :n], 0)
+    token = want_idx if cand is None else cand.long()[want_idx]
+    assert torch.equal(idx.long()[..., K - n:], token)
+    want = {"cosine": want_key * row, "euclidean": (row - want_key).clamp_min(0).sqrt(), "matmul": want_key / root}[metric]
+    if sampled:
+        here = torch.arange(T, device=DEV).view(1, 1, T, 1)
+        want = torch.where(token == here, torch.tensor(1.1 if metric == "euclidean" else -0.1, device=DEV), want)
+        assert torch.equal(idx.long()[..., :1], here.expand(B, H, T, 1)) and bool((val[..., 0] == 1).all())
+        assert values != "negative" and metric != "euclidean" or bool((token == here).any())
+    real = want_key.abs() < float("inf")
+    # one product or quotient, or a difference of whole numbers and its root: equal up to that rounding
+    assert bool(((val[..., K - n:] - want).abs() <= 2.0 ** -22 * want.abs())[real].all())
