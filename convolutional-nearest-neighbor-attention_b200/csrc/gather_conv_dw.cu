@@ -239,13 +239,14 @@ int launch(const DwParams& p, cudaStream_t st) {
     const int grid = (p.M + TT - 1) / TT;
     // The form by the rounds of CTAs per SM it needs: with four tokens per thread three CTAs of one tap in flight, or two of two
     // taps where both need two rounds (3 x 1611 tokens x 10, 96 channels, 25 taps 36.1, 32.7 us); with one token four CTAs of four
-    // taps while that is one round (two CTAs of eight, of more than twelve taps: 2 x 65 x 96, 25 taps 8.9, 7.4), then five or six of
+    // taps while that is one round (two CTAs of eight, of more than twelve taps: 2 x 65 x 96, 25 taps 8.9, 7.4; unless that leaves four or
+    // more to be taken one by one: 17 x 65 x 2 heads of 64, float32, 13 taps 4.1, 4.6, 115 x 79 x 16, 20 taps 4.2, 4.7), then five or six of
     // two taps, which fit in one (71 x 34 x 2 heads of 128, float32, 3 taps 5.4, 4.1; 9 x 701 x 2 heads of 64 6.6, 5.3).
     const int sms = device_sms(), per_sm = (grid + sms - 1) / sms;
     auto go = [&](auto kern) { launch_chained(kern, grid, THREADS, smem, st, p, TT); };
     if (tpt == 4 && per_sm != 4) go(gather_conv_dw_kernel<T, TO, VEC, 4, 1, 3>);
     else if (tpt == 4) go(gather_conv_dw_kernel<T, TO, VEC, 4, 2, 2>);
-    else if (per_sm <= 2 && p.K > 12) go(gather_conv_dw_kernel<T, TO, VEC, 1, 8, 2>);
+    else if (per_sm <= 2 && p.K > 12 && p.K % 8 < 4) go(gather_conv_dw_kernel<T, TO, VEC, 1, 8, 2>);
     else if (per_sm <= 4) go(gather_conv_dw_kernel<T, TO, VEC, 1, 4, 4>);
     else if (per_sm == 6) go(gather_conv_dw_kernel<T, TO, VEC, 1, 2, 6>);
     else go(gather_conv_dw_kernel<T, TO, VEC, 1, 2, 5>);

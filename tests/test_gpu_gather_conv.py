@@ -164,3 +164,11 @@ def test_forms_of_the_depthwise_gather(B, T, H, dk, K, dtype, form):
 def test_small_grids(B, T, H, dk, K, dtype):
     test_depthwise_against_float64(B, T, H, dk, K, dtype, "cosine", True)
     test_depthwise_against_float64(B, T, H, dk, K, dtype, "euclidean", False)
+
+
+# Eight taps in flight on small grids only where they leave at most three.
+@on_148_sms
+@pytest.mark.parametrize("K,form", [(13, "1, 4, 4"), (16, "1, 8, 2"), (19, "1, 8, 2"), (20, "1, 4, 4"), (25, "1, 8, 2"), (31, "1, 4, 4")])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_taps_in_flight_on_small_grids(K, form, dtype):
+    test_forms_of_the_depthwise_gather(2, 65, 1, 96, K, dtype, form)
