@@ -56,6 +56,7 @@ SIGNATURES = {
     "convnn_b200_status_string": (ctypes.c_char_p, [ctypes.c_int]),
     "convnn_b200_last_error": (ctypes.c_char_p, []),
     "convnn_b200_launch_count": (ctypes.c_uint64, []),
+    "convnn_b200_forwards_in_flight": (ctypes.c_int, [ctypes.c_int32]),
     "convnn_b200_device_status": (ctypes.c_int, [ctypes.POINTER(ctypes.c_int)]),
     "convnn_b200_selftest_wait_timeout": (ctypes.c_int, [ctypes.c_uint32, c_void, c_void, c_void]),
     "convnn_b200_head_channels": (ctypes.c_int, [ctypes.POINTER(ConvnnDesc)]),

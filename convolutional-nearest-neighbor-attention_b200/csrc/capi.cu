@@ -75,6 +75,12 @@ int ClusterLimit::query(const void* kern, const cudaLaunchConfig_t* cfg, int* cl
     return CONVNN_OK;
 }
 
+static thread_local int t_in_flight = 1;
+int sms_of_a_forward() {
+    const int n = device_sms() / t_in_flight;
+    return n > 0 ? n : 1;
+}
+
 static std::atomic<unsigned long long> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
@@ -238,6 +244,13 @@ int convnn_b200_device_status(int* code) {
     if (!c && (rc = read_conv1d_tc_status(&c))) return rc;
     *code = a ? a : (b ? b : c);
     return CONVNN_OK;
+}
+
+int convnn_b200_forwards_in_flight(int32_t n) {
+    if (n < 0) return set_error(CONVNN_E_INVALID, "convnn_b200_forwards_in_flight: %d forwards", n);
+    const int before = t_in_flight;
+    if (n > 0) t_in_flight = n;
+    return before;
 }
 
 uint64_t convnn_b200_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }

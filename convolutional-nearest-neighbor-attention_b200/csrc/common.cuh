@@ -102,6 +102,8 @@ void launch_late(bool chained, void (*kern)(P...), dim3 grid, dim3 block, size_t
 
 // SM count of the current device, asked once per device.
 int device_sms();
+// Its share of them where several forwards are in flight (convnn_b200_forwards_in_flight(), the calling thread's).
+int sms_of_a_forward();
 
 // Raises a kernel's dynamic shared-memory limit.  cudaFuncSetAttribute costs a launch about as much host time as
 // building a tensor map, so a call site keeps one of these per kernel and calls the runtime only when the size grows.

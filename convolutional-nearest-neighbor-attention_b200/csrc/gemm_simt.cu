@@ -744,19 +744,18 @@ int launch_other_mode(const GemmParams& p, cudaStream_t st) {
     // An implicit operand is fetched with divisions and dependent reads per value.  While an SM has few tiles that, not the
     // products, is what a step waits for, and a tile with twice the threads wins; with more of them the tiles hide each other's
     // waits, and its extra shared-memory reads per product lose.  It keeps two tiles on an SM (four of the smallest) where
-    // the other form keeps three (seven), so it is taken where that takes no more passes.  (Times from before the operands were weighted
-    // and converted as late as they are now, which took both forms to 0.64 to 0.96 of them.)  Weighted neighbours, us, other form -> twice the
+    // the other form keeps three (seven), so it is taken where that takes no more passes.  Weighted neighbours, us, other form -> twice the
     // threads, float32, 9 taps unless noted; rounds of tiles per SM first:
-    //   128 x 64   1: 32 x 197 x 3 heads of 64 84.9 -> 60.0   2: 64 x 197 x 3 x 64 107 -> 87   3: 256 x 65 x 192 380 -> 388 (not taken)   4: 128 x 197 x 3 x 64 194 -> 170
-    //   64 x 64    1: 8 x 197 x 192 133 -> 103   3: 20 x 577 x 100 113 -> 128 (not taken)   4: 64 x 197 x 192 314 -> 301   5: 32 x 197 x 384 675 -> 706 (not taken)
-    //   32 x 64    1: 8 x 197 x 3 x 64 32.4 -> 27.7   4: 32 x 197 x 192 206 -> 212
-    //   32 x 32    1: 1 x 65 x 192 104 -> 67   6: 64 x 197 x 2 heads of 20 21.9 -> 28.1 (not taken)
-    // Shifted rows cost one division less and gain less: 16 x 197 x 192 209 -> 177 (1), 64 x 197 x 192 312 -> 342 (4, not taken), 32 x 197 x 72
-    // bfloat16 32 x 32 tiles 0.83 of the time (4).
-    // Tap rows of C values against more stored channels (the coordinate channel) come value by value: in bfloat16 they gain longest, longer
-    // still where an odd number of taps leaves every other row of them at an odd address.  64 x 64, 4: 64 x 197 x 192 617 -> 375; 3: 24 x 197 x
-    // 384, 9 taps 726 -> 615, 24 x 577 x 96, 8 taps 123 -> 151 (not taken); 32 x 32, 7: 159 x 65 x 96, 25 taps 741 -> 391, 6 and one column
-    // of tiles: 48 x 577 x 20, 16 taps 58 -> 63 (not taken).
+    //   128 x 64   1: 32 x 197 x 3 heads of 64 66.2 -> 50.0   2: 64 x 197 x 3 x 64 91 -> 82   3: 256 x 65 x 192 337 -> 354 (not taken)   4: 128 x 197 x 3 x 64 165 -> 160
+    //   64 x 64    1: 8 x 197 x 192 105 -> 89   3: 20 x 577 x 100 101 -> 119 (not taken)   4: 64 x 197 x 192 267 -> 289   5: 32 x 197 x 384 592 -> 687 (not taken)
+    //   32 x 64    1: 8 x 197 x 3 x 64 26.5 -> 25.3   4: 32 x 197 x 192 208 -> 198
+    //   32 x 32    1: 1 x 65 x 192 79 -> 53   6: 64 x 197 x 2 heads of 20 19.8 -> 25.1 (not taken)
+    // The lines were drawn when operands were weighted and converted as they were fetched, 1.04 to 1.6 times these: since then the other form
+    // is ahead at four rounds of 64 x 64, and of bfloat16 tap rows of C values against more stored channels (the coordinate channel, value
+    // by value), which gained longest from twice the threads: 64 x 64, 4: 64 x 197 x 192 323 -> 332; 3: 24 x 197 x 384, 9 taps 423 -> 503, 24 x 577 x 96, 8
+    // taps 99 -> 118 (not taken); 32 x 32, 7: 159 x 65 x 96, 25 taps 295 -> 308, 6 and one column of tiles: 48 x 577 x 20, 16 taps 44 -> 50 (not taken).
+    // Shifted rows cost one division less and gain less (times of before): 16 x 197 x 192 209 -> 177 (1), 64 x 197 x 192 312 -> 342 (4, not taken),
+    // 32 x 197 x 72 bfloat16 32 x 32 tiles 0.83 of the time (4).
     if constexpr (MODE == A_NEIGHBOURS || MODE == A_CONV1D) {
         const long long per_sm = (tiles_of[best] + sms - 1) / sms, here = best == 3 ? 4 : 2, other = best == 3 ? 7 : 3;
         bool twice = (per_sm + here - 1) / here <= (per_sm + other - 1) / other;

@@ -12,14 +12,14 @@
 //
 // The results are the streaming kernels' bit for bit.
 //
-// What bounds it (128 images of 12 heads, 197 x 197 x 32, K = 9, 83 us; with the entries inserted into a sorted list and written a word at
-// a time 93; the streaming kernel 136): instructions, half of them on the half-rate pipe, and their fetch: a chunk loop unrolled once
-// more 125 for 106, the metric known at compile time 96 for 106, tensor-memory reads one chunk ahead nothing.  (18 warps of 96 registers:
+// What bounds it (128 images of 12 heads, 197 x 197 x 32, K = 9, 79 us; the streaming kernel 136): instructions, half of them on the half-rate
+// pipe, and their fetch: with the entries inserted into a sorted list and written a word at a time 93; a chunk loop unrolled once more 125 for 106,
+// the metric known at compile time 96 for 106, tensor-memory reads one chunk ahead nothing.  (18 warps of 96 registers:
 // one thread per row spills 16 to 64 bytes.)  Lists of more than twelve have one thread per row, eight warps, and wait as much as they
 // issue (0.31 instructions per cycle and scheduler); us, a sorted list of values as the bound or the streaming kernel -> groups and a
-// network: 57 x 12 heads of 197 x 197 x 32, K = 25 171 -> 84; 256 x 197 x 197 x 192, K = 25 70 -> 41, K = 16 50 -> 30; 256 x 577 x 150 x 384,
-// K = 16 107 -> 67.  Streaming -> this kernel, K = 9: 256 images of 197 x 192 30.5 -> 20.5 (K = 4: 22.8 -> 16.3), 6 heads of 64 126 -> 84,
-// 65 x 65 x 192 12.5 -> 9.7, 1024 x 65 x 65, 3 heads of 64 94 -> 43, 64 x 1000 x 200 x 256 33 -> 25, 256 x 197 x 64 x 384 17.8 -> 17.6.
+// network: 57 x 12 heads of 197 x 197 x 32, K = 25 171 -> 85; 256 x 197 x 197 x 192, K = 25 70 -> 36, K = 16 50 -> 26; 256 x 577 x 150 x 384,
+// K = 16 107 -> 67.  Streaming -> this kernel, K = 9: 256 images of 197 x 192 30.5 -> 20.9 (K = 4: 22.8 -> 15.8), 6 heads of 64 126 -> 82,
+// 65 x 65 x 192 12.5 -> 9.2, 1024 x 65 x 65, 3 heads of 64 94 -> 41, 64 x 1000 x 200 x 256 33 -> 25, 256 x 197 x 64 x 384 17.8 -> 15.9.
 //
 // A persistent CTA per SM: warp 0 TMA producer (128 key rows + all candidate rows of one (batch, head), 64-channel chunks,
 // ring), warp 1 MMA issuer (M = 128, N = S rounded to 16), then selection warps (thread = row).  G accumulators of 512 / G
@@ -108,17 +108,6 @@ __device__ __forceinline__ void make_keys(float (&key)[W], const uint32_t (&acc)
 #pragma unroll
         for (int j = 0; j < W; ++j)
             if (j >= left) key[j] = -CUDART_INF_F;
-    }
-}
-
-template <int NSEL, int J, class E>
-__device__ __forceinline__ void insert_first(TopList<NSEL>& top, const E& entry, int cnt) {
-    if constexpr (J < NSEL) {
-        if (J < cnt) {
-            const float2 x = entry(J);
-            top.template insert_sorted_first<J>(x.x, __float_as_int(x.y));
-        }
-        insert_first<NSEL, J + 1>(top, entry, cnt);
     }
 }
 

@@ -74,8 +74,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     return false;
 }
 
-// Variants on raw shared-memory addresses for the single-thread producer / MMA loops, whose
-// instruction count per pipeline step is what bounds the whole kernel's issue rate.
+// Variants on raw shared-memory addresses for the loops that issue copies and products, whose instruction count per
+// pipeline step is what bounds the whole kernel's issue rate.
 __device__ __forceinline__ bool mbar_try_wait_a(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(

@@ -18,6 +18,8 @@ from typing import List, Optional, Sequence
 
 import torch
 
+from . import _capi
+
 
 class ForwardLanes:
     """CUDA graphs of ``model``'s forward over fixed input buffers, ``lanes`` forwards per graph.
@@ -53,16 +55,20 @@ class ForwardLanes:
             pool = None
             for group in self.groups:
                 g = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(g, pool=pool):
-                    cur = torch.cuda.current_stream()
-                    for st in side[: len(group) - 1]:
-                        st.wait_stream(cur)                # the branches start together
-                    self.outputs[group[0]] = model(inputs[group[0]])
-                    for st, k in zip(side, group[1:]):
-                        with torch.cuda.stream(st):
-                            self.outputs[k] = model(inputs[k])
-                    for st in side[: len(group) - 1]:
-                        cur.wait_stream(st)
+                before = _capi.lib().convnn_b200_forwards_in_flight(len(group))
+                try:
+                    with torch.cuda.graph(g, pool=pool):
+                        cur = torch.cuda.current_stream()
+                        for st in side[: len(group) - 1]:
+                            st.wait_stream(cur)                # the branches start together
+                        self.outputs[group[0]] = model(inputs[group[0]])
+                        for st, k in zip(side, group[1:]):
+                            with torch.cuda.stream(st):
+                                self.outputs[k] = model(inputs[k])
+                        for st in side[: len(group) - 1]:
+                            cur.wait_stream(st)
+                finally:
+                    _capi.lib().convnn_b200_forwards_in_flight(before)
                 pool = pool or g.pool()
                 self.graphs.append(g)
         torch.cuda.synchronize(dev)

@@ -100,6 +100,10 @@ const char* convnn_b200_last_error(void);
 /* No reference counterpart: number of kernels this library has launched in the process so
  * far (a monotonically increasing statistic; the only process-wide state it keeps). */
 uint64_t convnn_b200_launch_count(void);
+/* What this thread launches from now on runs beside as much again of n - 1 other forwards (two batches in
+ * flight: 2): grids that would spread over idle SMs leave the others theirs.  The results are the same bits.
+ * Returns the number before, 1 at a thread's start; n = 0 leaves it as it is, n < 0 is CONVNN_E_INVALID. */
+int convnn_b200_forwards_in_flight(int32_t n);
 
 /* No reference counterpart: reads the device-side error latch (synchronises the device).
  * 0 = no kernel gave up; otherwise the code of the first bounded wait that expired inside

@@ -49,8 +49,8 @@ def rel_err(a, b):
 
 
 def launches(fn, attribute="LOCAL_SIZE_BYTES"):
-    """{kernel name (mangled): bytes of local memory per thread, or another attribute} of what fn() launches, read from a
-    captured graph."""
+    """{kernel name (mangled): bytes of local memory per thread, or another attribute, or its CTAs ("GRID")} of what fn() launches,
+    read from a captured graph."""
     from cuda.bindings import driver
 
     def ok(r):
@@ -70,7 +70,8 @@ def launches(fn, attribute="LOCAL_SIZE_BYTES"):
             continue
         p = ok(driver.cuGraphKernelNodeGetParams(node))[0]
         func = p.func if int(p.func) else ok(driver.cuKernelGetFunction(p.kern))[0]
-        found[ok(driver.cuFuncGetName(func))[0].decode()] = ok(driver.cuFuncGetAttribute(
+        name = ok(driver.cuFuncGetName(func))[0].decode()
+        found[name] = p.gridDimX * p.gridDimY * p.gridDimZ if attribute == "GRID" else ok(driver.cuFuncGetAttribute(
             getattr(driver.CUfunction_attribute, "CU_FUNC_ATTRIBUTE_" + attribute), func))[0]
     graph.reset()
     return found

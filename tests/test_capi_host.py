@@ -196,3 +196,15 @@ def test_separable_workspace_with_the_coordinate_channel(B, T, S, D, H, dtype, e
     assert 0 < got <= total or dk > 1024
     if (B, dtype) == (83, _capi.BF16):
         assert got <= 32 << 20
+
+
+def test_forwards_in_flight_are_the_threads_own():
+    import threading
+    L = _capi.lib()
+    assert L.convnn_b200_forwards_in_flight(0) == 1 and L.convnn_b200_forwards_in_flight(3) == 1
+    other = []
+    t = threading.Thread(target=lambda: other.append(L.convnn_b200_forwards_in_flight(0)))
+    t.start()
+    t.join()
+    assert other == [1] and L.convnn_b200_forwards_in_flight(-1) < 0
+    assert L.convnn_b200_forwards_in_flight(1) == 3 and L.convnn_b200_forwards_in_flight(0) == 1

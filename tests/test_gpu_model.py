@@ -7,7 +7,7 @@ from convnn_b200 import _capi, ops
 from oracle.convnn_oracle import ConvNNConfig, bf16_round, make_input, make_layer_weights
 from oracle.vit_oracle import vit_forward
 from golden_util import VIT_NAMES, vit_case
-from gpu_util import DEV, pack, rel_err, spec_of
+from gpu_util import DEV, launches, on_148_sms, pack, rel_err, spec_of
 
 pytestmark = pytest.mark.gpu
 
@@ -356,3 +356,35 @@ def test_forward_lanes_reproduce_the_eager_forward():
     for j in range(10):
         assert torch.equal(logits[j], want[j % 5])
     assert _capi.device_status() == 0
+
+
+@on_148_sms
+@pytest.mark.parametrize("M,N,K,alone,beside", [(1430, 1536, 192, 144, 72), (390, 768, 768, 96, 48), (1950, 768, 384, 96, 48)])
+def test_forwards_in_flight_leave_each_other_their_sms(M, N, K, alone, beside):
+    """A grid that leaves SMs idle takes narrower tiles up to the forward's share of the SMs; the bits are the same."""
+    L = _capi.lib()
+    g = torch.Generator(device=DEV).manual_seed(M)
+    a, w = (torch.randn(r, K, device=DEV, generator=g).to(torch.bfloat16) for r in (M, N))
+    call = lambda: ops.linear(a, w)
+    want, (grid,) = call(), launches(call, "GRID").values()
+    assert L.convnn_b200_forwards_in_flight(2) == 1
+    try:
+        assert torch.equal(call(), want)
+        assert (grid, *launches(call, "GRID").values()) == (alone, beside)
+    finally:
+        assert L.convnn_b200_forwards_in_flight(1) == 2
+
+
+def test_forward_lanes_give_the_sms_back():
+    """The number of forwards in flight holds while a group is captured, by its length, and no longer."""
+    seen, L = [], _capi.lib()
+
+    class Model(torch.nn.Module):
+        def forward(self, x):
+            if torch.cuda.is_current_stream_capturing():
+                seen.append(L.convnn_b200_forwards_in_flight(0))
+            return x + 1
+
+    xs = [torch.zeros(2, device=DEV) for _ in range(3)]
+    convnn_b200.ForwardLanes(Model(), xs, lanes=2)
+    assert seen == [2, 2, 1] and L.convnn_b200_forwards_in_flight(0) == 1
